@@ -111,6 +111,7 @@ struct SearchCtx {
     uint64_t vis_stride = 0;
     size_t vis_slots = 0;
     DevBuf d_qtables, d_qcodes, d_q, d_out_ids, d_out_dist, d_stats;
+    DevBuf d_seeds, d_cand;  // entry scan -> walk: seed keys; walk -> rerank: ids
     DevBuf d_probe_codes, d_probe_ids, d_probe_dist;  // search_multiprobe
     ~SearchCtx() {
         if (done) cudaEventDestroy(done);
@@ -156,6 +157,7 @@ struct cphnsw_b200_index {
     // index contents
     uint64_t n = 0;
     cpb::DevBuf d_vectors, d_codes, d_adj, d_entry, d_entry_codes;
+    cpb::DevBuf d_entry_scan;   // the entry nodes' codes as the entry scan reads them (gather_entry_codes)
     cpb::DevBuf d_packed;       // binary-code mode: the sign bits of every node packed 32 per word, uint32 [n][packed_words],
     int packed_words = 0;       // which is what the walk reads (popcount of an XOR); 0 outside that mode
     bool codes_released = false;  // binary-code mode between build stages: d_codes is freed, the packed bits are the stored

@@ -418,6 +418,19 @@ __global__ void adjacency_dup_kernel(const uint32_t* __restrict__ adj, uint64_t 
     if (__ballot_sync(kFull, dup) && lane == 0) atomicOr(flag, 1u);
 }
 
+// The entry nodes' codes as the entry scan of the asymmetric metric reads them: per block of 32 rotations, component
+// (j + e) & 31 of entry e at place j (zero for rotations past K)
+template <typename CompT>
+__global__ void rotate_entry_codes_kernel(const CompT* __restrict__ codes /* [n_entry][K] */, uint32_t n_entry, int K, int padded,
+                                          CompT* __restrict__ out /* [n_entry][padded] */) {
+    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= uint64_t(n_entry) * padded) return;
+    const uint32_t e = uint32_t(t / padded);
+    const int j = int(t % padded);
+    const int r = (j & ~31) | ((j + int(e & 31u)) & 31);
+    out[t] = r < K ? codes[uint64_t(e) * K + r] : CompT(0);
+}
+
 struct LaunchCfg {
     uint32_t cap;
     int warps;
@@ -451,9 +464,8 @@ LaunchCfg pick_cfg(const cphnsw_b200_index* h, uint32_t beam, bool sym) {
 
 }  // namespace
 
-// two-warps-per-query kernel (search_team.cu)
-size_t search_team_extra_smem();
-int launch_search_team(cphnsw_b200_index* h, SearchArgs a, size_t per_team, int narrow_blocks, cudaStream_t st);
+// several expansions per step (search_walk.cu)
+int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, bool table_smem, cudaStream_t st);
 
 // sign bits of every node, 32 per word: bit b of word w = bit 0 of component 32 * w + b (binary-code mode)
 __global__ void pack_walk_codes_kernel(const unsigned char* __restrict__ codes, uint64_t n, int K, int comp_bytes, int words,
@@ -522,6 +534,23 @@ int gather_entry_codes(cphnsw_b200_index* h, cudaStream_t st) {
             h->d_entry_codes.as<unsigned char>());
         h->launches++;
         CPB_CUDA(cudaGetLastError());
+        if (h->packed_words) {
+            CPB_TRY(h->d_entry_scan.reserve(size_t(h->n_entry) * h->packed_words * 4 + 16));
+            CPB_TRY(gather_rows(h, h->d_packed.p, size_t(h->packed_words) * 4, h->d_entry.as<uint32_t>(), h->n_entry, h->d_entry_scan.p, st));
+        } else {
+            const int padded = int((h->K + 31) / 32 * 32);
+            const uint64_t cells = uint64_t(h->n_entry) * padded;
+            CPB_TRY(h->d_entry_scan.reserve(cells * h->comp_bytes + 16));
+            const unsigned grid = unsigned((cells + 255) / 256);
+            if (h->comp_bytes == 2)
+                rotate_entry_codes_kernel<uint16_t><<<grid, 256, 0, st>>>(h->d_entry_codes.as<uint16_t>(), h->n_entry, int(h->K), padded,
+                                                                         h->d_entry_scan.as<uint16_t>());
+            else
+                rotate_entry_codes_kernel<uint8_t><<<grid, 256, 0, st>>>(h->d_entry_codes.as<uint8_t>(), h->n_entry, int(h->K), padded,
+                                                                        h->d_entry_scan.as<uint8_t>());
+            h->launches++;
+            CPB_CUDA(cudaGetLastError());
+        }
     }
     return 0;
 }
@@ -596,7 +625,6 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
         set_error("search: internal error (a narrow context was given %llu queries)", (unsigned long long)nq);
         return CPHNSW_B200_E_STATE;
     }
-    CPB_TRY(prepare_search_scratch(h, cx, st));
     LaunchCfg c = pick_cfg(h, beam, sym);
     SearchArgs a;
     a.qcodes = d_qcodes;
@@ -625,9 +653,6 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
     a.per_warp_smem = uint32_t(c.per_warp);
     a.k = k;
     a.rerank_k = rerank_k;
-    a.visited = cx.d_visited.as<uint8_t>();
-    a.vis_stride = cx.vis_stride;
-    a.epochs = cx.d_epochs.as<uint32_t>();
     a.out_ids = d_ids;
     a.out_dist = d_dists;
     a.stats = d_stats;
@@ -650,27 +675,17 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
     const bool u16 = h->comp_bytes == 2;
     LaunchTimer timer(h, kKernelSearch, st);
 
-    // two warps per query: asymmetric metric, table in shared memory, one adjacency row per warp
-    // (beams over 1,024 up to 2,048 in its wide form, which exists for tables in shared memory; under the symmetric
-    // metric only on packed sign bits, i.e. in binary-code mode)
-    const bool team_ok = !scan_only && h->M <= 32 && h->k_entry <= 128 &&
-                         (sym ? (a.packed != nullptr && beam <= 1024)
-                              : ((beam <= 1024 || (beam <= 2048 && c.table_smem)) && (c.table_smem || h->K <= 32)));
-    a.table_in_smem = c.table_smem ? 1 : 0;
-    if (h->search_kernel == 2 && !team_ok && !sym) {
-        set_error("search_kernel=2 needs the asymmetric metric, M <= 32, K*P*4 <= 32 KB or K <= 32, and a beam of at most 1024 (2048 with the table in shared memory)");
+    // several expansions per step: rows of up to 32 links, any metric and beam
+    const bool walk_ok = !scan_only && h->M <= 32;
+    if (h->search_kernel == 2 && !walk_ok && !scan_only) {
+        set_error("search_kernel=2 needs M <= 32");
         return CPHNSW_B200_E_UNSUPPORTED;
     }
-    // (Also for a table too large for shared memory, read in place: on 1M x 960 clustered vectors the two-warp kernel
-    // does 301 k queries/s against 237 k for one warp per query; only on vectors with independent coordinates, where an
-    // expansion scores ~26 neighbours instead of ~2, one warp per query was 3-7 % ahead.)
-    if (team_ok && h->search_kernel != 1) {
-        const size_t per_team = (c.per_warp + search_team_extra_smem() + 15) & ~size_t(15);
-        CPB_TRY(launch_search_team(h, a, per_team, narrow ? int(nq) : 0, st));
-        h->launches++;
-        CPB_CUDA(cudaGetLastError());
-        return 0;
-    }
+    if (walk_ok && h->search_kernel != 1) return launch_search_walk(h, cx, a, sym, c.table_smem, st);
+    CPB_TRY(prepare_search_scratch(h, cx, st));
+    a.visited = cx.d_visited.as<uint8_t>();
+    a.vis_stride = cx.vis_stride;
+    a.epochs = cx.d_epochs.as<uint32_t>();
 
 #define CPB_SEARCH(U, T, S)                                                                                \
     do {                                                                                                   \

@@ -1,0 +1,878 @@
+// Beam search, one warp per query, several expansions per step: same algorithm and same results as search_kernel
+// (search.cu) for adjacency rows of up to 32 links.
+//
+// What bounds a walk is its chain of dependent steps: select the closest unexpanded member of W, read its links, ask
+// which are new, fetch and score their codes, rank them into W.  The next member to expand is the next unexpanded one
+// unless this expansion admitted something closer, which is rare (3 % of the steps on 1M clustered vectors at beam
+// 500).  A step therefore takes the first kRows unexpanded members of W at once: their rows are looked up together,
+// their new neighbours are scored together, and then the longest prefix of the rows is committed that the sequential
+// walk would have expanded in this order: row t is left for the next step when a neighbour of an earlier row is
+// closer than member t.  Candidates are ordered by the total order (distance, id), so W after the committed rows does
+// not depend on the order in which their neighbours are admitted, and a row that was not committed has left no trace.
+//
+// Visited nodes.  W itself decides what is admitted: a node seen before is either a member of W (found there by its
+// key when it is ranked) or was turned away or pushed out by members that are closer, and would be again, since the
+// worst member of a full W only gets closer.  Remembering visited nodes only saves the scoring, so a filter that may
+// forget is enough: 16-bit tags in shared memory, 8 to a bucket (one 128-bit read), the tag and the bucket together
+// being a bijection of the id, so that a hit is never wrong.  When the caller asks for statistics (the number of
+// distance evaluations counts every node once) or the index is too large for exact tags, the exact set is kept
+// instead: one byte per node and slot in global memory holding the number of the slot's last query that visited it.
+//
+// W is one sorted array of 64-bit keys (ordered distance bits, id, expanded flag) in shared memory.  A step's
+// admitted candidates are merged in one pass from the highest position down: the final positions of the candidates
+// are marked in a bit set (one word per lane), and the member that moves to position j is the one at j minus the
+// marks below it.
+//
+// The exact rerank (-<q,x> of the best rerank_k, replacing GPUBruteForce::rerank, src/cuda/gpu_encoder.cu:605-664) is
+// a kernel of its own, one block per query: inside the walk a single warp would have to read all the vectors.
+#include "search_common.cuh"
+
+namespace cpb {
+namespace {
+
+using namespace srch;
+
+constexpr int kRows = 4;          // members of W taken per step
+constexpr int kBucketLog2 = 9;    // tag filter: 512 buckets of 8 tags = 8 KB per query
+constexpr uint32_t kTagBytes = (1u << kBucketLog2) * 16;
+constexpr uint64_t kFiller = ~0ull;
+constexpr int kScanKeep = 32;     // most seeds the entry-scan kernel keeps per query
+constexpr int kScanWarps = 8;
+
+// metrics: asymmetric CP score with the query table in shared memory / read in place, symmetric code distance on
+// whole components / on packed sign bits
+enum { kAsymSmem = 0, kAsymGlobal = 1, kSymBytes = 2, kSymPacked = 3 };
+
+struct WalkArgs {
+    SearchArgs s;
+    const uint64_t* seeds;  // [nq][kScanKeep] keys of the entry scan's best, ascending (nullptr: scanned by the walk itself)
+    uint32_t* cand;         // [nq][rerank_k] ids handed to the rerank kernel (nullptr: no rerank)
+    uint32_t smem_per_warp;
+    uint32_t wcap_slots;    // slots of W's array (multiple of 32)
+    int exact_visited;      // bytes in global memory instead of the tag filter
+    uint32_t tag_bits;      // id bits below the bucket index after mixing
+    uint32_t id_bits_mask;  // (1 << id bits) - 1
+};
+
+__device__ __forceinline__ uint32_t float_order(float d) {
+    const uint32_t u = __float_as_uint(d);
+    return u ^ (uint32_t(int32_t(u) >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float float_unorder(uint32_t u) {
+    return __uint_as_float(u ^ ((u & 0x80000000u) ? 0x80000000u : 0xffffffffu));
+}
+// key of an unexpanded member; bit 0 is the expanded flag
+__device__ __forceinline__ uint64_t make_key(float d, uint32_t id) { return (uint64_t(float_order(d)) << 32) | (id << 1); }
+__device__ __forceinline__ uint32_t key_id(uint64_t k) { return uint32_t(k) >> 1; }
+
+// ---- tag filter -----------------------------------------------------------------------------------------
+struct TagSpot {
+    uint32_t bucket, tag;  // tag 0: not cacheable
+};
+__device__ __forceinline__ TagSpot tag_spot(uint32_t id, uint32_t id_mask, uint32_t tag_bits) {
+    const uint32_t x = (id * 0x9E3779B1u) & id_mask;  // an odd multiplier is a bijection on the low bits
+    TagSpot s;
+    s.bucket = x >> tag_bits;
+    s.tag = ((x & ((1u << tag_bits) - 1u)) + 1u) & 0xffffu;
+    return s;
+}
+// non-zero when one of the two halfwords of w is zero; the lowest flag set is that of a zero halfword
+__device__ __forceinline__ uint32_t zero_half(uint32_t w) { return (w - 0x00010001u) & ~w & 0x80008000u; }
+
+__device__ __forceinline__ bool tag_seen(const uint4* tags, const TagSpot& s) {
+    const uint4 b = tags[s.bucket];
+    const uint32_t p = s.tag | (s.tag << 16);
+    return ((zero_half(b.x ^ p) | zero_half(b.y ^ p) | zero_half(b.z ^ p) | zero_half(b.w ^ p)) != 0u) && s.tag != 0u;
+}
+// first empty place of the bucket, or a victim; two lanes that meet in one place lose one of the tags
+__device__ __forceinline__ void tag_store(uint4* tags, const TagSpot& s) {
+    if (s.tag == 0u) return;
+    const uint4 b = tags[s.bucket];
+    const uint32_t z0 = zero_half(b.x), z1 = zero_half(b.y), z2 = zero_half(b.z), z3 = zero_half(b.w);
+    uint32_t pos = s.tag & 7u;
+    if (z0) pos = (z0 & 0x8000u) ? 0u : 1u;
+    else if (z1) pos = (z1 & 0x8000u) ? 2u : 3u;
+    else if (z2) pos = (z2 & 0x8000u) ? 4u : 5u;
+    else if (z3) pos = (z3 & 0x8000u) ? 6u : 7u;
+    reinterpret_cast<uint16_t*>(tags + s.bucket)[pos] = uint16_t(s.tag);
+}
+
+// ---- W -----------------------------------------------------------------------------------------------------
+// Members of W below `key` (binary search, every lane its own key); flags do not matter: a candidate's flag is 0.
+// (An eight-ary search, three rounds for 512 members, has the shorter chain of reads but issues 60 instructions a
+// round, and was slower: 2,040 against 1,020 cycles where ten lanes search at once.)
+__device__ __forceinline__ uint32_t lower_bound(const uint64_t* W, uint32_t count, uint64_t key) {
+    uint32_t lo = 0, len = count;
+    while (len) {
+        const uint32_t half = len >> 1;
+        const bool right = W[lo + half] < key;
+        lo = right ? lo + half + 1 : lo;
+        len = right ? len - half - 1 : half;
+    }
+    return lo;
+}
+
+// Scratch of the merge, per warp: the step's keys and, for every 32 positions of W, {marks, marks before}.
+// Merges the keys of the lanes in `m` (distinct, none of them in W, rank p = members below the key) into W, which
+// keeps the `cap` best.  Returns the lowest position taken.
+template <int WORDS>
+__device__ __forceinline__ uint32_t merge_into(uint64_t* W, uint32_t& count, uint32_t cap, uint32_t m, uint64_t key, uint32_t p,
+                                               uint64_t* kbuf, uint2* marks, int lane) {
+    const bool mine = (m >> lane) & 1u;
+    const int k = __popc(m);
+    if (mine) kbuf[__popc(m & ((1u << lane) - 1u))] = key;
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) marks[w * 32 + lane].x = 0;
+    __syncwarp();
+    uint32_t o = 0;  // candidates of the step below this one
+    for (int i = 0; i < k; ++i) o += kbuf[i] < key;
+    const uint32_t f = p + o;  // final position
+    if (mine && (f >> 5) < uint32_t(WORDS * 32)) atomicOr(&marks[f >> 5].x, 1u << (f & 31));
+    const uint32_t fmin = __reduce_min_sync(kFull, mine ? f : 0xffffffffu);
+    __syncwarp();
+    uint32_t carry = 0;
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        const uint32_t own = __popc(marks[w * 32 + lane].x);
+        uint32_t x = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, d);
+            if (lane >= d) x += y;
+        }
+        marks[w * 32 + lane].y = carry + x - own;
+        if (WORDS > 1) carry += __shfl_sync(kFull, x, 31);
+    }
+    __syncwarp();
+    const uint32_t newcount = min(cap, count + uint32_t(k));
+    // four chunks of 32 positions at a time, highest first: all reads of a group precede its writes
+    constexpr int G = 4;
+    for (int c = int((newcount + 31) >> 5) - 1; c >= int(fmin >> 5); c -= G) {
+        uint64_t e[G];
+        bool move[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const int cc = max(c - g, 0);
+            const uint2 t = marks[cc];
+            const uint32_t j = uint32_t(cc) * 32 + lane;
+            move[g] = c - g >= 0 && j >= fmin && j < newcount && !((t.x >> lane) & 1u);
+            e[g] = 0;
+            if (move[g]) e[g] = W[j - t.y - __popc(t.x & ((1u << lane) - 1u))];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            if (move[g]) W[uint32_t(c - g) * 32 + lane] = e[g];
+        __syncwarp();
+    }
+    if (mine && f < cap) W[f] = key;
+    count = newcount;
+    __syncwarp();
+    return fmin;
+}
+
+// ---- scoring -------------------------------------------------------------------------------------------------
+// Distances of up to 32 nodes under the asymmetric metric; lane c receives that of node c.  Their code rows are in
+// shared memory, `stride` bytes apart.  Eight nodes at a time: lane r owns rotation r, and the tree sum over the
+// rotations (pairs 16 apart, then 8, 4, 2, 1) halves the number of nodes a lane carries at each of its first three
+// steps, 9 shuffles for 8 nodes; the pairs added are the ones asym_distance_lane adds.
+template <bool U16, bool SMEM>
+__device__ __forceinline__ float score_asym(const float* table, const unsigned char* rows, int stride, int K, int P, int total,
+                                            int lane) {
+    float mine = 0.0f;
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+    for (int g = 0; g < total; g += 8) {
+        float acc = 0.0f;
+        for (int c0 = 0; c0 < K; c0 += 32) {
+            const bool own = c0 + lane < K;
+            const int r = own ? c0 + lane : K - 1;
+            const float* at = table + r * P;
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {  // rows past `total` hold anything: read within the table (P is a power of two), not used
+                const uint32_t comp = load_component<U16>(rows + (g + i) * stride, r);
+                const uint32_t index = (comp >> 1) & uint32_t(P - 1);
+                const float val = SMEM ? at[index] : __ldg(at + index);
+                v[i] = own ? __uint_as_float(__float_as_uint(val) ^ (comp << 31)) : 0.0f;
+            }
+            float v4[4], v2[2], t;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float send = h16 ? v[i] : v[i + 4], keep = h16 ? v[i + 4] : v[i];
+                v4[i] = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 16));
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float send = h8 ? v4[i] : v4[i + 2], keep = h8 ? v4[i + 2] : v4[i];
+                v2[i] = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 8));
+            }
+            {
+                const float send = h4 ? v2[0] : v2[1], keep = h4 ? v2[1] : v2[0];
+                t = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 4));
+            }
+            t = __fadd_rn(t, __shfl_xor_sync(kFull, t, 2));
+            t = __fadd_rn(t, __shfl_xor_sync(kFull, t, 1));
+            acc = __fadd_rn(acc, t);
+        }
+        const float d = __shfl_sync(kFull, -acc, ((lane - g) & 7) * 4);  // lanes 4i .. 4i+3 hold node g + i
+        if (lane >= g && lane < g + 8) mine = d;
+    }
+    return mine;
+}
+
+// The code row of every lane's own node to shared memory (rows `stride` bytes apart, 16-byte aligned).
+__device__ __forceinline__ void stage_codes(unsigned char* rows, int stride, const unsigned char* codes, int row_bytes,
+                                            const uint32_t* ids, uint32_t id, int total, int lane) {
+    if ((row_bytes & 15) == 0) {
+        if (lane < total) {
+            const uint4* src = reinterpret_cast<const uint4*>(codes + size_t(id) * row_bytes);
+            uint4* dst = reinterpret_cast<uint4*>(rows + lane * stride);
+            if (row_bytes == 32) {
+                const uint4 x = __ldg(src), y = __ldg(src + 1);
+                dst[0] = x;
+                dst[1] = y;
+            } else {
+#pragma unroll 4
+                for (int i = 0; i < row_bytes / 16; ++i) dst[i] = __ldg(src + i);
+            }
+        }
+    } else {
+        for (int c = 0; c < total; ++c)
+            for (int i = lane; i < row_bytes; i += 32) rows[c * stride + i] = __ldg(codes + size_t(ids[c]) * row_bytes + i);
+    }
+    __syncwarp();
+}
+
+// ---- entry scan ------------------------------------------------------------------------------------------------
+// The n_seed best entry nodes of every query (n_seed <= 32), QG queries per block, the entries dealt to its warps in
+// batches of 32, one entry per lane.  Every query reads every entry node, so the scan is bound by table lookups:
+// n_entry * K per query, 4 bytes of shared-memory bandwidth each.
+//   * The tables of the block's queries are interleaved [block of 32 rotations][index][rotation][query]: one address
+//     and one 16-byte read serve four queries.
+//   * At step j lane l looks up rotation (j + l) & 31 of its entry, so the lanes of a read sit in different banks; the
+//     entries' codes are stored with the components in that order (gather_entry_codes).  The balanced tree pairs
+//     rotations 16, 8, 4, 2, 1 apart, and pairing j with j + 16 (mod 32) pairs the same rotations whatever l is, so
+//     the sums keep their bits.
+//   * Each warp keeps its 32 best per query, one per lane.  A candidate has to beat the warp's own n_seed-th and the
+//     largest of all warps' (n_seed / warps)-th distances, below which n_seed entries are known to lie, so the warps
+//     admit about as little as one list would.
+struct ScanArgs {
+    const float* tables;          // asymmetric: [nq][K][P]
+    const unsigned char* qcodes;  // symmetric: [nq][row_bytes]
+    const unsigned char* entry_scan;  // asymmetric: rotated codes [n_entry][nblk * 32]; symmetric: code rows / packed words
+    const uint32_t* entry;
+    uint32_t n_entry, n_seed, nq;
+    int K, P, row_bytes, packed_words, resid_kp, resid_mul;
+    uint64_t* seeds;  // [nq][kScanKeep]
+};
+
+template <int QG>
+struct Vals {
+    float v[QG];
+};
+
+// S(step, j) of the tree over rotations (j + lane) & 31; w: the entry's components in that order
+template <bool U16, int QG, int STEP, int J>
+__device__ __forceinline__ Vals<QG> scan_tree(const unsigned char* table, const uint32_t (&w)[U16 ? 16 : 8], uint32_t lane_at,
+                                              uint32_t index2_mask) {
+    Vals<QG> r;
+    if constexpr (STEP == 32) {
+        constexpr int PER = U16 ? 2 : 4, BITS = U16 ? 16 : 8;
+        constexpr int SH = (J % PER) * BITS;  // the component's position in its word
+        constexpr int ROW = 32 * QG * 4;      // bytes of one index of the table
+        const uint32_t word = w[J / PER];
+        const uint32_t sign = word << (31 - SH);
+        const uint32_t comp2 = (word >> SH) & index2_mask;  // twice the index, kept inside the table
+        const uint32_t at = comp2 * uint32_t(ROW / 2) + ((lane_at + uint32_t(J * QG * 4)) & uint32_t(ROW - 1));
+        float x[QG];
+        if constexpr (QG == 4) {
+            const float4 f = *reinterpret_cast<const float4*>(table + at);
+            x[0] = f.x, x[1] = f.y, x[2] = f.z, x[3] = f.w;
+        } else if constexpr (QG == 2) {
+            const float2 f = *reinterpret_cast<const float2*>(table + at);
+            x[0] = f.x, x[1] = f.y;
+        } else {
+            x[0] = *reinterpret_cast<const float*>(table + at);
+        }
+#pragma unroll
+        for (int i = 0; i < QG; ++i) r.v[i] = __uint_as_float(__float_as_uint(x[i]) ^ (sign & 0x80000000u));
+    } else {
+        const Vals<QG> a = scan_tree<U16, QG, STEP * 2, J>(table, w, lane_at, index2_mask);
+        const Vals<QG> b = scan_tree<U16, QG, STEP * 2, J + STEP>(table, w, lane_at, index2_mask);
+#pragma unroll
+        for (int i = 0; i < QG; ++i) r.v[i] = __fadd_rn(a.v[i], b.v[i]);
+    }
+    return r;
+}
+
+template <bool U16, int METRIC, int QG>
+__global__ void __launch_bounds__(kScanWarps * 32)
+entry_scan_kernel(ScanArgs a) {
+    extern __shared__ __align__(16) unsigned char scan_smem[];
+    __shared__ uint64_t lists[kScanWarps][QG][kScanKeep];
+    __shared__ uint32_t bound[QG][kScanWarps];  // ordered distance of each warp's (n_seed / warps)-th best
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t q0 = blockIdx.x * QG;
+    const int nblk = (a.K + 31) / 32;
+    if (threadIdx.x < QG * kScanWarps) bound[threadIdx.x / kScanWarps][threadIdx.x % kScanWarps] = 0xffffffffu;
+    if constexpr (METRIC == kAsymSmem) {
+        // lane = rotation; four indices of QG queries per pass
+        float* tab = reinterpret_cast<float*>(scan_smem);
+        const int quads = a.P / 4;
+        for (int u = warp; u < nblk * quads; u += kScanWarps) {
+            const int blk = u / quads, i4 = (u % quads) * 4, r = blk * 32 + lane;
+            float x[QG][4];
+#pragma unroll
+            for (int g = 0; g < QG; ++g) {
+                float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (r < a.K && q0 + g < a.nq)
+                    f = __ldg(reinterpret_cast<const float4*>(a.tables + (size_t(q0 + g) * a.K + r) * a.P + i4));
+                x[g][0] = f.x, x[g][1] = f.y, x[g][2] = f.z, x[g][3] = f.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float* dst = tab + ((size_t(blk) * a.P + i4 + i) * 32 + lane) * QG;
+                if constexpr (QG == 4) *reinterpret_cast<float4*>(dst) = make_float4(x[0][i], x[1][i], x[2][i], x[3][i]);
+                else if constexpr (QG == 2) *reinterpret_cast<float2*>(dst) = make_float2(x[0][i], x[1][i]);
+                else *dst = x[0][i];
+            }
+        }
+    } else {  // the queries' codes, as bytes or packed sign bits
+        for (int g = 0; g < QG; ++g) {
+            const unsigned char* src = a.qcodes + size_t(min(q0 + g, a.nq - 1)) * a.row_bytes;
+            if (METRIC == kSymBytes) {
+                for (int i = threadIdx.x; i < a.row_bytes; i += kScanWarps * 32) scan_smem[size_t(g) * ((a.row_bytes + 15) / 16 * 16) + i] = src[i];
+            } else if (warp == 0) {
+                for (int i = 0; i < a.packed_words; ++i) {
+                    const int r = 32 * i + lane;
+                    const uint32_t word = __ballot_sync(kFull, r < a.K && (src[r * (U16 ? 2 : 1)] & 1u));
+                    if (lane == 0) reinterpret_cast<uint32_t*>(scan_smem)[g * a.packed_words + i] = word;
+                }
+            }
+        }
+    }
+    __syncthreads();
+
+    uint64_t best[QG];
+    uint32_t thr[QG];  // ordered distance a candidate must not exceed
+#pragma unroll
+    for (int g = 0; g < QG; ++g) best[g] = kFiller, thr[g] = 0xffffffffu;
+    const int pub = (int(a.n_seed) + kScanWarps - 1) / kScanWarps - 1;
+    for (uint32_t e0 = warp * 32; e0 < a.n_entry; e0 += kScanWarps * 32) {
+        const uint32_t e = e0 + lane;
+        const bool ok = e < a.n_entry;
+        const uint32_t ee = ok ? e : a.n_entry - 1;
+        const uint32_t id = __ldg(a.entry + ee);
+        float d[QG];
+        if constexpr (METRIC == kAsymSmem) {
+            constexpr int WORDS = U16 ? 16 : 8;
+            const uint4* row = reinterpret_cast<const uint4*>(a.entry_scan + size_t(ee) * nblk * (U16 ? 64 : 32));
+#pragma unroll
+            for (int g = 0; g < QG; ++g) d[g] = 0.0f;
+            for (int blk = 0; blk < nblk; ++blk) {
+                uint32_t w[WORDS];
+#pragma unroll
+                for (int i = 0; i < WORDS / 4; ++i) {
+                    const uint4 v = __ldg(row + blk * (WORDS / 4) + i);
+                    w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+                }
+                const Vals<QG> s = scan_tree<U16, QG, 1, 0>(scan_smem + size_t(blk) * a.P * 32 * QG * 4, w, uint32_t(lane * QG * 4),
+                                                               uint32_t(2 * a.P - 2));
+#pragma unroll
+                for (int g = 0; g < QG; ++g) d[g] = __fadd_rn(d[g], s.v[g]);
+            }
+#pragma unroll
+            for (int g = 0; g < QG; ++g) d[g] = -d[g];
+        } else {
+#pragma unroll
+            for (int g = 0; g < QG; ++g) {
+                if (METRIC == kSymPacked)
+                    d[g] = packed_distance_lane(reinterpret_cast<const uint32_t*>(scan_smem) + g * a.packed_words,
+                                                reinterpret_cast<const uint32_t*>(a.entry_scan), ee, a.packed_words, a.resid_kp, a.resid_mul);
+                else
+                    d[g] = sym_distance_lane<U16>(scan_smem + size_t(g) * ((a.row_bytes + 15) / 16 * 16), a.entry_scan, ee, a.K, a.resid_kp,
+                                                  a.resid_mul);
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < QG; ++g) {
+            const uint64_t key = make_key(d[g], id);
+            const uint32_t others = lane < kScanWarps ? *reinterpret_cast<volatile uint32_t*>(&bound[g][lane]) : 0u;
+            const uint32_t lim = min(thr[g], __reduce_max_sync(kFull, others));
+            uint32_t m = __ballot_sync(kFull, ok && uint32_t(key >> 32) <= lim);
+            if (m == 0) continue;
+            while (m) {
+                const int src = __ffs(m) - 1;
+                m &= m - 1;
+                const uint64_t k = __shfl_sync(kFull, key, src);
+                const int r = __popc(__ballot_sync(kFull, best[g] < k));
+                const uint64_t up = __shfl_up_sync(kFull, best[g], 1);
+                best[g] = lane < r ? best[g] : (lane == r ? k : up);
+            }
+            const uint32_t hi = uint32_t(best[g] >> 32);
+            thr[g] = __shfl_sync(kFull, hi, int(a.n_seed) - 1);
+            if (lane == pub) *reinterpret_cast<volatile uint32_t*>(&bound[g][warp]) = hi;
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < QG; ++g) lists[warp][g][lane] = best[g];
+    __syncthreads();
+    // one warp per query joins the sorted lists: the lower half of (own, other reversed) is bitonic
+    for (int g = warp; g < QG; g += kScanWarps) {
+        if (q0 + g >= a.nq) continue;
+        uint64_t x = lists[0][g][lane];
+        for (int o = 1; o < kScanWarps; ++o) {
+            const uint64_t y = lists[o][g][31 - lane];
+            x = y < x ? y : x;
+#pragma unroll
+            for (int s = 16; s >= 1; s >>= 1) {
+                const uint64_t z = __shfl_xor_sync(kFull, x, s);
+                const bool low = (lane & s) == 0;
+                x = (z < x) == low ? z : x;
+            }
+        }
+        a.seeds[size_t(q0 + g) * kScanKeep + lane] = x;
+    }
+}
+
+template <bool U16, int METRIC, int WORDS>
+__global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    const SearchArgs& a = w.s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
+    const size_t table_floats = METRIC == kAsymSmem ? size_t(a.K) * a.P : 0;
+    const int row_bytes = a.K * (U16 ? 2 : 1);
+    unsigned char* area = walk_smem + size_t(w.smem_per_warp) * warp;
+    float* table_sm = reinterpret_cast<float*>(area);
+    uint64_t* W = reinterpret_cast<uint64_t*>(area + table_floats * 4);
+    uint4* tags = reinterpret_cast<uint4*>(W + w.wcap_slots);
+    uint64_t* kbuf = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(tags) + (w.exact_visited ? 0 : kTagBytes));
+    uint2* marks = reinterpret_cast<uint2*>(kbuf + 32);
+    uint32_t* cid = reinterpret_cast<uint32_t*>(marks + WORDS * 32);
+    uint32_t* front = cid + 32;  // the first unexpanded members of W
+    unsigned char* qcode = reinterpret_cast<unsigned char*>(front + 8);  // symmetric metric: code bytes or packed words
+    unsigned char* rows_sm = qcode;                                      // asymmetric: the candidates' code rows
+    const int stride = (row_bytes + 15) / 16 * 16;
+    uint32_t* qpacked = reinterpret_cast<uint32_t*>(qcode);
+
+    const uint32_t slot = blockIdx.x * warps + warp;
+    uint8_t* vis = w.exact_visited ? a.visited + size_t(slot) * a.vis_stride : nullptr;
+    uint32_t epoch = w.exact_visited ? a.epochs[slot] : 0u;
+    const unsigned char* codes = static_cast<const unsigned char*>(a.codes);
+
+    while (true) {
+        uint32_t q = 0;
+        if (lane == 0) q = atomicAdd(a.next_query, 1u);
+        q = __shfl_sync(kFull, q, 0);
+        if (q >= a.nq) break;
+        __syncwarp();
+        const float* table = METRIC == kAsymSmem ? table_sm : (METRIC == kAsymGlobal ? a.tables + size_t(q) * a.K * a.P : nullptr);
+        if (METRIC == kAsymSmem) {
+            const float4* src = reinterpret_cast<const float4*>(a.tables + size_t(q) * table_floats);
+            float4* dst = reinterpret_cast<float4*>(table_sm);
+#pragma unroll 8
+            for (int i = lane; i < int(table_floats / 4); i += 32) dst[i] = __ldg(src + i);
+        }
+        if (SYM) {
+            const unsigned char* src = static_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes;
+            if (METRIC == kSymBytes) {
+                for (int i = lane; i < row_bytes; i += 32) qcode[i] = src[i];
+            } else {
+                for (int i = 0; i < a.packed_words; ++i) {
+                    const int r = 32 * i + lane;
+                    const uint32_t word = __ballot_sync(kFull, r < a.K && (src[r * (U16 ? 2 : 1)] & 1u));
+                    if (lane == 0) qpacked[i] = word;
+                }
+            }
+        }
+        if (!w.exact_visited) {
+            for (int i = lane; i < int(kTagBytes / 16); i += 32) tags[i] = make_uint4(0u, 0u, 0u, 0u);
+        } else if (++epoch == 256) {  // the 8-bit epoch wraps: forget every earlier query
+            uint4* v4 = reinterpret_cast<uint4*>(vis);
+            for (uint64_t i = lane; i < a.vis_stride / 16; i += 32) v4[i] = make_uint4(0u, 0u, 0u, 0u);
+            epoch = 1;
+        }
+        __syncwarp();
+
+        uint32_t count = 0, cur = 0, nexp = 0, nevals = 0;
+
+        // distance of node `id` of lane `lane` < total (ids also in cid[])
+        auto score = [&](int total, uint32_t id) -> float {
+            if (METRIC == kSymPacked)
+                return lane < total ? packed_distance_lane(qpacked, a.packed, id, a.packed_words, a.resid_kp, a.resid_mul) : 0.0f;
+            if (METRIC == kSymBytes)
+                return lane < total ? sym_distance_lane<U16>(qcode, a.codes, id, a.K, a.resid_kp, a.resid_mul) : 0.0f;
+            stage_codes(rows_sm, stride, codes, row_bytes, cid, id, total, lane);
+            return score_asym<U16, METRIC == kAsymSmem>(table, rows_sm, stride, a.K, a.P, total, lane);
+        };
+        auto remember = [&](bool mine, uint32_t id) {
+            if (w.exact_visited) {
+                if (mine) vis[id] = uint8_t(epoch);
+            } else if (mine) {
+                tag_store(tags, tag_spot(id, w.id_bits_mask, w.tag_bits));
+            }
+        };
+
+        // ---- entry nodes (search_engine.hpp:105-115): all of them are offered, or the n_seed best of a scan
+        const bool scan = a.n_seed < a.n_entry;
+        const uint32_t cap0 = scan ? a.n_seed : a.beam;
+        if (w.seeds) {
+            const uint64_t k = w.seeds[size_t(q) * kScanKeep + lane];
+            count = __popc(__ballot_sync(kFull, k != kFiller && uint32_t(lane) < cap0));
+            if (uint32_t(lane) < count) W[lane] = k;
+            nevals += a.n_entry;
+            __syncwarp();
+        }
+        for (uint32_t e0 = w.seeds ? a.n_entry : 0u; e0 < a.n_entry; e0 += 32) {
+            const uint32_t e = e0 + lane;
+            const uint32_t id = e < a.n_entry ? __ldg(a.entry + e) : kInvalidNode;
+            const bool ok = id < a.n;
+            const uint32_t m = __ballot_sync(kFull, ok);  // (entry ids are distinct and valid up to the end of the list)
+            const int total = 32 - __clz(int(m));
+            if (total == 0) continue;
+            float d;
+            if (METRIC == kSymPacked || METRIC == kSymBytes) {
+                d = ok ? sym_distance_lane<U16>(METRIC == kSymBytes ? qcode : reinterpret_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes,
+                                                a.entry_codes, e, a.K, a.resid_kp, a.resid_mul) : 0.0f;
+            } else {
+                d = ok ? asym_distance_lane<U16>(table, a.entry_codes, e, a.K, a.P) : 0.0f;
+            }
+            nevals += __popc(m);
+            const uint64_t key = make_key(d, id);
+            const bool adm = ok && (count < cap0 || key < W[count - 1]);
+            const uint32_t am = __ballot_sync(kFull, adm);
+            if (am) merge_into<WORDS>(W, count, cap0, am, key, adm ? lower_bound(W, count, key) : 0u, kbuf, marks, lane);
+            if (!scan) remember(ok, id);
+        }
+        if (scan) {  // the seeds are offered to the walk: marked visited, scored once more (a beam narrower than the
+                     // seed set keeps the best `beam` of them)
+            nevals += count;
+            for (uint32_t p = lane; p < count; p += 32) remember(true, key_id(W[p]));
+            if (count > a.beam) count = a.beam;
+        }
+        __syncwarp();
+
+        // ---- walk
+        uint32_t pre_node[kRows], pre_row[kRows];  // links loaded one step ahead for the members expected next
+#pragma unroll
+        for (int b = 0; b < kRows; ++b) pre_node[b] = kInvalidNode, pre_row[b] = kInvalidNode;
+        while (true) {
+            // the first kRows unexpanded members of the first window of 32 that has any (search_engine.hpp:121-123)
+            uint64_t ek = kFiller;
+            uint32_t un = 0;
+            while (cur < count) {
+                const uint32_t p = cur + lane;
+                ek = p < count ? W[p] : kFiller;
+                un = __ballot_sync(kFull, !(uint32_t(ek) & 1u));
+                if (un) break;
+                cur += 32;
+            }
+            if (!un) break;
+            const uint32_t below = (1u << lane) - 1u;
+            const uint32_t order = __popc(un & below);
+            const bool open_member = (un >> lane) & 1u;
+            if (open_member && order < 2 * kRows) front[order] = uint32_t(ek) >> 1;
+            const uint32_t sel = __ballot_sync(kFull, open_member && order < kRows);  // the members taken
+            const int have = __popc(un);
+            __syncwarp();
+            uint32_t row[kRows], node[kRows];
+#pragma unroll
+            for (int b = 0; b < kRows; ++b) {
+                node[b] = b < have ? front[b] : kInvalidNode;
+                row[b] = pre_row[b];
+                if (node[b] != pre_node[b])
+                    row[b] = (node[b] != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(node[b]) * a.M + lane) : kInvalidNode;
+            }
+            // the members behind them are the next step's unless this one changes the front of W
+#pragma unroll
+            for (int b = 0; b < kRows; ++b) {
+                pre_node[b] = kRows + b < have ? front[kRows + b] : kInvalidNode;
+                pre_row[b] = (pre_node[b] != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(pre_node[b]) * a.M + lane) : kInvalidNode;
+            }
+            // neighbours not seen before, row by row
+            uint32_t fresh[kRows];
+            if (w.exact_visited) {
+                uint32_t vb[kRows];
+#pragma unroll
+                for (int b = 0; b < kRows; ++b) vb[b] = row[b] < a.n ? uint32_t(__ldcg(vis + row[b])) : epoch;
+#pragma unroll
+                for (int b = 0; b < kRows; ++b) fresh[b] = __ballot_sync(kFull, vb[b] != epoch);
+            } else {
+#pragma unroll
+                for (int b = 0; b < kRows; ++b)
+                    fresh[b] = __ballot_sync(kFull, row[b] < a.n && !tag_seen(tags, tag_spot(row[b], w.id_bits_mask, w.tag_bits)));
+            }
+            // as many leading rows as bring at most 32 candidates; lane c owns candidate c
+            int total = 0, rows = 0, first_of[kRows];
+            bool open = true;
+#pragma unroll
+            for (int b = 0; b < kRows; ++b) {
+                const int nf = __popc(fresh[b]);
+                open = open && node[b] != kInvalidNode && total + nf <= 32;
+                first_of[b] = total;
+                if (open) {
+                    if ((fresh[b] >> lane) & 1u) cid[total + __popc(fresh[b] & below)] = row[b];
+                    total += nf;
+                    ++rows;
+                }
+            }
+            __syncwarp();
+            uint32_t commit = uint32_t(rows);
+            uint32_t id = kInvalidNode, my_row = 0, p = 0xffffffffu;
+            uint64_t key = kFiller;
+            bool own = false;
+            if (total) {
+                own = lane < total;
+                id = own ? cid[lane] : kInvalidNode;
+#pragma unroll
+                for (int b = 1; b < kRows; ++b)
+                    if (b < rows && lane >= first_of[b]) my_row = b;
+                const float d = score(total, id);
+                // a node listed by two rows (or twice in one) belongs to the first
+                const uint32_t grp = __match_any_sync(kFull, id);
+                own = own && (__ffs(grp) - 1) == lane;
+                key = make_key(d, id);
+                bool adm = own && (count < a.beam || key < W[count - 1]);
+                uint32_t am = __ballot_sync(kFull, adm);
+                if (am) {
+                    if (adm) {
+                        p = lower_bound(W, count, key);
+                        // a forgotten node that is a member of W
+                        if (p < count && (W[p] >> 1) == (key >> 1)) adm = false;
+                    }
+                    if (adm) {
+                        // rows t with member t below this candidate stay in order; the row that found it is done by then
+                        const uint32_t rel = p - cur;  // cur <= position of every selected member
+                        const uint32_t bl = p <= cur ? 0u : (rel >= 32u ? sel : sel & ((1u << rel) - 1u));
+                        commit = max(my_row + 1u, uint32_t(__popc(bl)));
+                    }
+                    commit = min(uint32_t(rows), __reduce_min_sync(kFull, commit));
+                    am = __ballot_sync(kFull, adm && my_row < commit);
+                }
+                own = own && my_row < commit;
+                remember(own, id);
+                nevals += __popc(__ballot_sync(kFull, own));
+                // the committed members carry their flag before positions move
+                if (open_member && order < commit) W[cur + lane] = ek | 1u;
+                __syncwarp();
+                if (am) {
+                    const uint32_t f = merge_into<WORDS>(W, count, a.beam, am, key, p, kbuf, marks, lane);
+                    cur = min(cur, f);
+                }
+            } else {
+                if (open_member && order < commit) W[cur + lane] = ek | 1u;
+                __syncwarp();
+            }
+            nexp += commit;
+        }
+
+        // ---- results: the ids the rerank kernel scores, or the k best with their distances
+        if (w.cand) {
+            uint32_t* out = w.cand + size_t(q) * a.rerank_k;
+            for (uint32_t p = lane; p < a.rerank_k; p += 32) out[p] = p < count ? key_id(W[p]) : kInvalidNode;
+        } else {
+            for (uint32_t p = lane; p < a.k; p += 32) {
+                const uint64_t e = p < count ? W[p] : 0;
+                a.out_ids[size_t(q) * a.k + p] = p < count ? key_id(e) : kInvalidNode;
+                a.out_dist[size_t(q) * a.k + p] = p < count ? float_unorder(uint32_t(e >> 32)) : INFINITY;
+            }
+        }
+        if (a.stats && lane == 0) {
+            a.stats[2 * size_t(q)] = nexp;
+            a.stats[2 * size_t(q) + 1] = nevals;
+        }
+        __syncwarp();
+    }
+    if (w.exact_visited && lane == 0) a.epochs[slot] = epoch;
+}
+
+// ---- exact rerank: one block per query -------------------------------------------------------------------------
+// 8 lanes per candidate row (128-bit loads), 32 rows of a block in flight per pass; the dot product is accumulated
+// with fmaf per lane and folded 4, 2, 1, as the fused rerank of search_kernel does.  The keys are then sorted in
+// shared memory and the k best written out.
+constexpr int kRerankThreads = 256;
+
+__global__ void __launch_bounds__(kRerankThreads)
+search_rerank_kernel(const float* __restrict__ vectors, const float* __restrict__ queries, const uint32_t* __restrict__ cand,
+                     uint32_t rr, uint32_t slots /* power of two >= rr */, int dim, uint32_t k, uint32_t* __restrict__ out_ids,
+                     float* __restrict__ out_dist) {
+    extern __shared__ __align__(16) unsigned char rr_smem[];
+    uint64_t* keys = reinterpret_cast<uint64_t*>(rr_smem);
+    float* qsm = reinterpret_cast<float*>(keys + slots);
+    const size_t q = blockIdx.x;
+    const uint32_t* ids = cand + q * rr;
+    for (int i = threadIdx.x; i < dim; i += kRerankThreads) qsm[i] = __ldg(queries + q * dim + i);
+    __syncthreads();
+    const int g = threadIdx.x >> 3, j = threadIdx.x & 7;
+    const bool vec4 = (dim & 3) == 0;
+#pragma unroll 4
+    for (uint32_t c0 = 0; c0 < slots; c0 += kRerankThreads / 8) {
+        const uint32_t c = c0 + g;
+        const uint32_t id = c < rr ? __ldg(ids + c) : kInvalidNode;
+        float acc = 0.0f;
+        if (id != kInvalidNode) {
+            const float* x = vectors + size_t(id) * dim;
+            if (vec4) {
+                for (int i = 4 * j; i < dim; i += 32) {
+                    const float4 xv = __ldg(reinterpret_cast<const float4*>(x + i));
+                    const float4 qv = *reinterpret_cast<const float4*>(qsm + i);
+                    acc = fmaf(xv.x, qv.x, acc);
+                    acc = fmaf(xv.y, qv.y, acc);
+                    acc = fmaf(xv.z, qv.z, acc);
+                    acc = fmaf(xv.w, qv.w, acc);
+                }
+            } else {
+                for (int i = j; i < dim; i += 8) acc = fmaf(__ldg(x + i), qsm[i], acc);
+            }
+        }
+        acc += __shfl_xor_sync(kFull, acc, 4);
+        acc += __shfl_xor_sync(kFull, acc, 2);
+        acc += __shfl_xor_sync(kFull, acc, 1);
+        if (j == 0 && c < slots) keys[c] = id != kInvalidNode ? make_key(-acc, id) : kFiller;
+    }
+    __syncthreads();
+    for (uint32_t k2 = 2; k2 <= slots; k2 <<= 1) {
+        for (uint32_t jj = k2 >> 1; jj > 0; jj >>= 1) {
+            for (uint32_t t = threadIdx.x; t < slots / 2; t += kRerankThreads) {
+                const uint32_t lo = ((t & ~(jj - 1)) << 1) | (t & (jj - 1)), hi = lo | jj;
+                const uint64_t x = keys[lo], y = keys[hi];
+                if ((y < x) == ((lo & k2) == 0)) {
+                    keys[lo] = y;
+                    keys[hi] = x;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (uint32_t p = threadIdx.x; p < k; p += kRerankThreads) {
+        const uint64_t e = p < slots ? keys[p] : kFiller;
+        out_ids[q * k + p] = e != kFiller ? key_id(e) : kInvalidNode;
+        out_dist[q * k + p] = e != kFiller ? float_unorder(uint32_t(e >> 32)) : INFINITY;
+    }
+}
+
+template <bool U16, int METRIC, int QG>
+int launch_scan_t(cphnsw_b200_index* h, const ScanArgs& a, size_t smem, cudaStream_t st) {
+    CPB_CUDA(allow_max_dynamic_smem(entry_scan_kernel<U16, METRIC, QG>));
+    entry_scan_kernel<U16, METRIC, QG><<<(a.nq + QG - 1) / QG, kScanWarps * 32, smem, st>>>(a);
+    h->launches++;
+    CPB_CUDA(cudaGetLastError());
+    return 0;
+}
+
+template <bool U16>
+int launch_scan(cphnsw_b200_index* h, const ScanArgs& a, int metric, cudaStream_t st) {
+    const size_t row = (size_t(a.row_bytes) + 15) / 16 * 16;
+    // several queries share a block's reads of the entry codes once every SM has a block of its own
+    const bool many = a.nq > uint32_t(h->sm_count);
+    if (metric == kSymBytes)
+        return many ? launch_scan_t<U16, kSymBytes, 4>(h, a, 4 * row, st) : launch_scan_t<U16, kSymBytes, 1>(h, a, row, st);
+    if (metric == kSymPacked)
+        return many ? launch_scan_t<U16, kSymPacked, 4>(h, a, size_t(16) * a.packed_words, st)
+                    : launch_scan_t<U16, kSymPacked, 1>(h, a, size_t(4) * a.packed_words, st);
+    const size_t table = size_t((a.K + 31) / 32) * 32 * a.P * 4;
+    if (many && a.nq > 2 * uint32_t(h->sm_count) && 4 * table <= 72 * 1024) return launch_scan_t<U16, kAsymSmem, 4>(h, a, 4 * table, st);
+    if (many && 2 * table <= 72 * 1024) return launch_scan_t<U16, kAsymSmem, 2>(h, a, 2 * table, st);
+    return launch_scan_t<U16, kAsymSmem, 1>(h, a, table, st);
+}
+
+template <bool U16, int METRIC>
+int launch_walk_t(cphnsw_b200_index* h, const WalkArgs& w, int blocks, int warps, cudaStream_t st) {
+    const size_t smem = size_t(w.smem_per_warp) * warps;
+    auto go = [&](auto kernel) -> int {
+        CPB_CUDA(allow_max_dynamic_smem(kernel));
+        kernel<<<unsigned(blocks), unsigned(warps) * 32, smem, st>>>(w);
+        return 0;
+    };
+    if (w.wcap_slots <= 1024) return go(search_walk_kernel<U16, METRIC, 1>);
+    return go(search_walk_kernel<U16, METRIC, 4>);  // beams up to 4,096: four words of the merge's bit set per lane
+}
+
+}  // namespace
+
+// Fills in the launch shape and runs walk and rerank.  a.next_query is zero on entry.
+int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, bool table_smem, cudaStream_t st) {
+    WalkArgs w;
+    w.s = a;
+    w.cand = nullptr;
+    if (a.rerank_k) {
+        CPB_TRY(cx.d_cand.reserve(size_t(a.nq) * a.rerank_k * 4 + 16));
+        w.cand = cx.d_cand.as<uint32_t>();
+    }
+    uint32_t top = a.beam > a.n_seed ? a.beam : a.n_seed;
+    w.wcap_slots = (top + 31) & ~31u;
+    // exact tags: the id bits above the bucket index have to fit 16 bits
+    uint32_t id_bits = kBucketLog2;
+    while ((uint64_t(1) << id_bits) < a.n) ++id_bits;
+    w.tag_bits = id_bits - kBucketLog2;
+    w.id_bits_mask = uint32_t((uint64_t(1) << id_bits) - 1);
+    w.exact_visited = (a.stats != nullptr || w.tag_bits > 16) ? 1 : 0;
+    if (w.exact_visited) {
+        CPB_TRY(prepare_search_scratch(h, cx, st));
+        w.s.visited = cx.d_visited.as<uint8_t>();
+        w.s.vis_stride = cx.vis_stride;
+        w.s.epochs = cx.d_epochs.as<uint32_t>();
+    }
+    const int metric = sym ? (a.packed ? kSymPacked : kSymBytes) : (table_smem ? kAsymSmem : kAsymGlobal);
+    const size_t table = metric == kAsymSmem ? size_t(a.K) * a.P * 4 : 0;
+    const size_t row = (size_t(a.K) * a.comp_bytes + 15) / 16 * 16;
+    const size_t words = w.wcap_slots <= 1024 ? 1 : 4;
+    // table, W, tags, merge scratch (keys, marks), candidate ids, front, then the query's code or the candidates' codes
+    w.smem_per_warp = uint32_t((table + size_t(w.wcap_slots) * 8 + (w.exact_visited ? 0 : kTagBytes) + 256 + words * 256 + 128 + 32 +
+                                (sym ? row : 32 * row) + 15) / 16 * 16);
+    int warps = int((226 * 1024) / w.smem_per_warp);
+    if (warps > 16) warps = 16;
+    const int per_sm = int((a.nq + h->sm_count - 1) / h->sm_count);  // a small batch spreads over all SMs
+    if (warps > per_sm) warps = per_sm;
+    if (warps < 1) warps = 1;
+    if (!cx.wide) warps = 1;
+    const uint64_t want = (uint64_t(a.nq) + warps - 1) / warps;
+    const int blocks = int(want < uint64_t(h->sm_count) ? want : uint64_t(h->sm_count));
+    const bool u16 = a.comp_bytes == 2;
+    w.seeds = nullptr;
+    const size_t scan_table = size_t((a.K + 31) / 32) * 32 * a.P * 4;
+    if (a.n_seed < a.n_entry && a.n_seed <= uint32_t(kScanKeep) && (sym || (a.P >= 4 && scan_table <= 200 * 1024))) {
+        ScanArgs sc;
+        sc.tables = a.tables;
+        sc.qcodes = static_cast<const unsigned char*>(a.qcodes);
+        sc.entry_scan = metric == kSymBytes ? static_cast<const unsigned char*>(a.entry_codes) : h->d_entry_scan.as<unsigned char>();
+        sc.entry = a.entry;
+        sc.n_entry = a.n_entry;
+        sc.n_seed = a.n_seed;
+        sc.nq = a.nq;
+        sc.K = a.K;
+        sc.P = a.P;
+        sc.row_bytes = a.K * a.comp_bytes;
+        sc.packed_words = a.packed_words;
+        sc.resid_kp = a.resid_kp;
+        sc.resid_mul = a.resid_mul;
+        CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * kScanKeep * 8));
+        sc.seeds = cx.d_seeds.as<uint64_t>();
+        w.seeds = sc.seeds;
+        CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
+    }
+#define CPB_WALK(X) (u16 ? launch_walk_t<true, X>(h, w, blocks, warps, st) : launch_walk_t<false, X>(h, w, blocks, warps, st))
+    switch (metric) {
+        case kAsymSmem: CPB_TRY(CPB_WALK(kAsymSmem)); break;
+        case kAsymGlobal: CPB_TRY(CPB_WALK(kAsymGlobal)); break;
+        case kSymBytes: CPB_TRY(CPB_WALK(kSymBytes)); break;
+        default: CPB_TRY(CPB_WALK(kSymPacked)); break;
+    }
+#undef CPB_WALK
+    h->launches++;
+    CPB_CUDA(cudaGetLastError());
+    if (a.rerank_k) {
+        uint32_t slots = 32;
+        while (slots < a.rerank_k) slots <<= 1;
+        const size_t smem = size_t(slots) * 8 + (size_t(a.dim) * 4 + 15) / 16 * 16;
+        CPB_CUDA(allow_max_dynamic_smem(search_rerank_kernel));
+        search_rerank_kernel<<<a.nq, kRerankThreads, smem, st>>>(a.vectors, a.queries, w.cand, a.rerank_k, slots, a.dim, a.k,
+                                                                a.out_ids, a.out_dist);
+        h->launches++;
+        CPB_CUDA(cudaGetLastError());
+    }
+    return 0;
+}
+
+}  // namespace cpb
