@@ -465,7 +465,7 @@ LaunchCfg pick_cfg(const cphnsw_b200_index* h, uint32_t beam, bool sym) {
 }  // namespace
 
 // several expansions per step (search_walk.cu)
-int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, bool table_smem, cudaStream_t st);
+int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, cudaStream_t st);
 
 // sign bits of every node, 32 per word: bit b of word w = bit 0 of component 32 * w + b (binary-code mode)
 __global__ void pack_walk_codes_kernel(const unsigned char* __restrict__ codes, uint64_t n, int K, int comp_bytes, int words,
@@ -681,7 +681,7 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
         set_error("search_kernel=2 needs M <= 32");
         return CPHNSW_B200_E_UNSUPPORTED;
     }
-    if (walk_ok && h->search_kernel != 1) return launch_search_walk(h, cx, a, sym, c.table_smem, st);
+    if (walk_ok && h->search_kernel != 1) return launch_search_walk(h, cx, a, sym, st);
     CPB_TRY(prepare_search_scratch(h, cx, st));
     a.visited = cx.d_visited.as<uint8_t>();
     a.vis_stride = cx.vis_stride;

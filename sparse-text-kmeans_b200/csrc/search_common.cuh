@@ -68,7 +68,7 @@ __device__ __forceinline__ uint32_t load_component(const unsigned char* row, int
 __device__ __forceinline__ float signed_term(const float* table, int r, int K, int P, uint32_t comp) {
     if (r >= K) return 0.0f;
     const float val = table[r * P + int(comp >> 1)];
-    return (comp & 1u) ? -val : val;
+    return __uint_as_float(__float_as_uint(val) ^ (comp << 31));
 }
 
 // One lane scores one node: the 32 terms of each block are combined in the balanced-tree order

@@ -33,15 +33,22 @@ namespace {
 using namespace srch;
 
 constexpr int kRows = 4;          // members of W taken per step
-constexpr int kBucketLog2 = 9;    // tag filter: 512 buckets of 8 tags = 8 KB per query
-constexpr uint32_t kTagBytes = (1u << kBucketLog2) * 16;
+constexpr int kBucketLog2 = 9;    // tag filter: 512 buckets of 4 tags = 4 KB per query
+constexpr uint32_t kTagBytes = (1u << kBucketLog2) * 8;
+constexpr uint64_t kTagNodes = uint64_t(0xffff) << kBucketLog2;  // ids below this have exact tags
 constexpr uint64_t kFiller = ~0ull;
 constexpr int kScanKeep = 32;     // most seeds the entry-scan kernel keeps per query
 constexpr int kScanWarps = 8;
+// Warps (queries) per SM.  A step is about 900 instructions with a chain of memory and shuffle latencies between them,
+// so what counts is how many walks an SM has in flight: the query table (16 KB) is therefore read in place, through L1
+// and L2, and not held in shared memory, where 7 to 9 walks would fit (1M x 128, 10,000 queries: 5.9 ms with the tables
+// in shared memory, 4.3 ms in place with 16 walks per SM, 3.4 ms with 24; 28 at 64 registers: 3.5 ms).
+constexpr int kWalkWarps = 24;
+constexpr int kFewRanked = 4;     // up to this many candidates are ranked by the whole warp, one after the other
 
-// metrics: asymmetric CP score with the query table in shared memory / read in place, symmetric code distance on
-// whole components / on packed sign bits
-enum { kAsymSmem = 0, kAsymGlobal = 1, kSymBytes = 2, kSymPacked = 3 };
+// metrics: asymmetric CP score (kAsym128: its most frequent shape, one-byte codes of 32 rotations at padded dim 128, as
+// compile-time facts), symmetric code distance on whole components / on packed sign bits
+enum { kAsym = 0, kAsym128 = 1, kSymBytes = 2, kSymPacked = 3 };
 
 struct WalkArgs {
     SearchArgs s;
@@ -50,8 +57,6 @@ struct WalkArgs {
     uint32_t smem_per_warp;
     uint32_t wcap_slots;    // slots of W's array (multiple of 32)
     int exact_visited;      // bytes in global memory instead of the tag filter
-    uint32_t tag_bits;      // id bits below the bucket index after mixing
-    uint32_t id_bits_mask;  // (1 << id bits) - 1
 };
 
 __device__ __forceinline__ uint32_t float_order(float d) {
@@ -66,35 +71,25 @@ __device__ __forceinline__ uint64_t make_key(float d, uint32_t id) { return (uin
 __device__ __forceinline__ uint32_t key_id(uint64_t k) { return uint32_t(k) >> 1; }
 
 // ---- tag filter -----------------------------------------------------------------------------------------
-struct TagSpot {
-    uint32_t bucket, tag;  // tag 0: not cacheable
-};
-__device__ __forceinline__ TagSpot tag_spot(uint32_t id, uint32_t id_mask, uint32_t tag_bits) {
-    const uint32_t x = (id * 0x9E3779B1u) & id_mask;  // an odd multiplier is a bijection on the low bits
-    TagSpot s;
-    s.bucket = x >> tag_bits;
-    s.tag = ((x & ((1u << tag_bits) - 1u)) + 1u) & 0xffffu;
-    return s;
-}
-// non-zero when one of the two halfwords of w is zero; the lowest flag set is that of a zero halfword
+// The low bits of an id name its bucket, the high bits plus one are its tag (zero: an empty place).
+__device__ __forceinline__ uint32_t tag_of(uint32_t id) { return (id >> kBucketLog2) + 1u; }
+__device__ __forceinline__ uint32_t bucket_of(uint32_t id) { return id & ((1u << kBucketLog2) - 1u); }
+// flags the halfwords of w that are zero; the lowest flag set is always that of a zero halfword
 __device__ __forceinline__ uint32_t zero_half(uint32_t w) { return (w - 0x00010001u) & ~w & 0x80008000u; }
 
-__device__ __forceinline__ bool tag_seen(const uint4* tags, const TagSpot& s) {
-    const uint4 b = tags[s.bucket];
-    const uint32_t p = s.tag | (s.tag << 16);
-    return ((zero_half(b.x ^ p) | zero_half(b.y ^ p) | zero_half(b.z ^ p) | zero_half(b.w ^ p)) != 0u) && s.tag != 0u;
+__device__ __forceinline__ bool tag_seen(const uint2* tags, uint32_t id) {
+    const uint2 b = tags[bucket_of(id)];
+    const uint32_t p = tag_of(id) * 0x00010001u;
+    return (zero_half(b.x ^ p) | zero_half(b.y ^ p)) != 0u;
 }
 // first empty place of the bucket, or a victim; two lanes that meet in one place lose one of the tags
-__device__ __forceinline__ void tag_store(uint4* tags, const TagSpot& s) {
-    if (s.tag == 0u) return;
-    const uint4 b = tags[s.bucket];
-    const uint32_t z0 = zero_half(b.x), z1 = zero_half(b.y), z2 = zero_half(b.z), z3 = zero_half(b.w);
-    uint32_t pos = s.tag & 7u;
+__device__ __forceinline__ void tag_store(uint2* tags, uint32_t id) {
+    const uint2 b = tags[bucket_of(id)];
+    const uint32_t tag = tag_of(id), z0 = zero_half(b.x), z1 = zero_half(b.y);
+    uint32_t pos = tag & 3u;
     if (z0) pos = (z0 & 0x8000u) ? 0u : 1u;
     else if (z1) pos = (z1 & 0x8000u) ? 2u : 3u;
-    else if (z2) pos = (z2 & 0x8000u) ? 4u : 5u;
-    else if (z3) pos = (z3 & 0x8000u) ? 6u : 7u;
-    reinterpret_cast<uint16_t*>(tags + s.bucket)[pos] = uint16_t(s.tag);
+    reinterpret_cast<uint16_t*>(tags + bucket_of(id))[pos] = uint16_t(tag);
 }
 
 // ---- W -----------------------------------------------------------------------------------------------------
@@ -112,6 +107,23 @@ __device__ __forceinline__ uint32_t lower_bound(const uint64_t* W, uint32_t coun
     return lo;
 }
 
+// Members of W below a key known to every lane: two rounds of a 32-ary search (beams up to 1,024; more passes of 32 in
+// the second round beyond).
+__device__ __forceinline__ uint32_t lower_bound_warp(const uint64_t* W, uint32_t count, uint64_t key, int lane) {
+    if (count == 0) return 0;
+    const uint32_t stride = (count + 31) >> 5;
+    const uint32_t last = min(count, (uint32_t(lane) + 1) * stride) - 1;  // last member of this lane's block
+    const bool less = uint32_t(lane) * stride < count && W[last] < key;
+    const uint32_t base = __popc(__ballot_sync(kFull, less)) * stride;    // the blocks entirely below
+    if (base >= count) return count;
+    uint32_t inside = 0;
+    for (uint32_t o = 0; o < stride; o += 32) {
+        const uint32_t j = base + o + lane;
+        inside += __popc(__ballot_sync(kFull, o + lane < stride && j < count && W[min(j, count - 1)] < key));
+    }
+    return base + inside;
+}
+
 // Scratch of the merge, per warp: the step's keys and, for every 32 positions of W, {marks, marks before}.
 // Merges the keys of the lanes in `m` (distinct, none of them in W, rank p = members below the key) into W, which
 // keeps the `cap` best.  Returns the lowest position taken.
@@ -120,6 +132,32 @@ __device__ __forceinline__ uint32_t merge_into(uint64_t* W, uint32_t& count, uin
                                                uint64_t* kbuf, uint2* marks, int lane) {
     const bool mine = (m >> lane) & 1u;
     const int k = __popc(m);
+    const uint32_t newcount = min(cap, count + uint32_t(k));
+    constexpr int G = 8;  // chunks of 32 positions moved at a time, highest first: all reads of a group precede its writes
+    if (k == 1) {         // one candidate: everything from its position on moves up by one
+        const int src = __ffs(m) - 1;
+        const uint32_t f = __shfl_sync(kFull, p, src);
+        for (int c = int((newcount + 31) >> 5) - 1; c >= int(f >> 5); c -= G) {
+            uint64_t e[G];
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int j = (c - g) * 32 + lane;
+                e[g] = 0;
+                if (j > int(f) && j < int(newcount)) e[g] = W[j - 1];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int j = (c - g) * 32 + lane;
+                if (j > int(f) && j < int(newcount)) W[j] = e[g];
+            }
+            __syncwarp();
+        }
+        if (mine) W[f] = key;
+        count = newcount;
+        __syncwarp();
+        return f;
+    }
     if (mine) kbuf[__popc(m & ((1u << lane) - 1u))] = key;
 #pragma unroll
     for (int w = 0; w < WORDS; ++w) marks[w * 32 + lane].x = 0;
@@ -144,9 +182,6 @@ __device__ __forceinline__ uint32_t merge_into(uint64_t* W, uint32_t& count, uin
         if (WORDS > 1) carry += __shfl_sync(kFull, x, 31);
     }
     __syncwarp();
-    const uint32_t newcount = min(cap, count + uint32_t(k));
-    // four chunks of 32 positions at a time, highest first: all reads of a group precede its writes
-    constexpr int G = 4;
     for (int c = int((newcount + 31) >> 5) - 1; c >= int(fmin >> 5); c -= G) {
         uint64_t e[G];
         bool move[G];
@@ -172,75 +207,68 @@ __device__ __forceinline__ uint32_t merge_into(uint64_t* W, uint32_t& count, uin
 }
 
 // ---- scoring -------------------------------------------------------------------------------------------------
-// Distances of up to 32 nodes under the asymmetric metric; lane c receives that of node c.  Their code rows are in
-// shared memory, `stride` bytes apart.  Eight nodes at a time: lane r owns rotation r, and the tree sum over the
-// rotations (pairs 16 apart, then 8, 4, 2, 1) halves the number of nodes a lane carries at each of its first three
-// steps, 9 shuffles for 8 nodes; the pairs added are the ones asym_distance_lane adds.
-template <bool U16, bool SMEM>
-__device__ __forceinline__ float score_asym(const float* table, const unsigned char* rows, int stride, int K, int P, int total,
+// Distances of the nodes ids[0, total) (total <= 32) under the asymmetric metric; lane c receives that of node c.
+// Four lanes share a node: lane part owns rotations part + 4 i, so the tree's first three levels (16, 8 and 4 apart)
+// stay in the lane and the last two are shuffles.  Eight nodes take 8 lookups a lane, against 32 for a lane alone
+// (most steps bring fewer than eight) and 13 dependent stages for a warp that shares each node.
+template <bool U16, bool FIXED /* one-byte codes, K = 32, P = 128 */>
+__device__ __forceinline__ float score_asym(const float* table, const unsigned char* codes, int K_, int P_, const uint32_t* ids, int total,
                                             int lane) {
+    const int K = FIXED ? 32 : K_, P = FIXED ? 128 : P_;
+    const int row_bytes = K * (U16 ? 2 : 1);
     float mine = 0.0f;
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+    const int part = lane & 3;
+    const bool vec = FIXED || (row_bytes & 15) == 0;
+    const float* part_table = table + part * P;
     for (int g = 0; g < total; g += 8) {
+        const uint32_t id = ids[min(g + (lane >> 2), total - 1)];
+        const unsigned char* row = codes + size_t(id) * row_bytes;
         float acc = 0.0f;
         for (int c0 = 0; c0 < K; c0 += 32) {
-            const bool own = c0 + lane < K;
-            const int r = own ? c0 + lane : K - 1;
-            const float* at = table + r * P;
+            uint32_t comp[8];
+            if (vec && c0 + 32 <= K) {
+                constexpr int WORDS = U16 ? 16 : 8;
+                const uint4* r4 = reinterpret_cast<const uint4*>(row + c0 * (U16 ? 2 : 1));
+                uint32_t x[WORDS];
+#pragma unroll
+                for (int i = 0; i < WORDS / 4; ++i) {
+                    const uint4 v = __ldg(r4 + i);
+                    x[4 * i] = v.x, x[4 * i + 1] = v.y, x[4 * i + 2] = v.z, x[4 * i + 3] = v.w;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (U16) comp[i] = ((part & 2) ? x[2 * i + 1] : x[2 * i]) >> (16 * (part & 1)) & 0xffffu;
+                    else comp[i] = __byte_perm(x[i], 0u, 0x4440u | uint32_t(part));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = c0 + part + 4 * i;
+                    comp[i] = r < K ? load_component<U16>(row, r) : 0u;
+                }
+            }
             float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {  // rows past `total` hold anything: read within the table (P is a power of two), not used
-                const uint32_t comp = load_component<U16>(rows + (g + i) * stride, r);
-                const uint32_t index = (comp >> 1) & uint32_t(P - 1);
-                const float val = SMEM ? at[index] : __ldg(at + index);
-                v[i] = own ? __uint_as_float(__float_as_uint(val) ^ (comp << 31)) : 0.0f;
-            }
-            float v4[4], v2[2], t;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float send = h16 ? v[i] : v[i + 4], keep = h16 ? v[i + 4] : v[i];
-                v4[i] = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 16));
+            for (int i = 0; i < 8; ++i) {
+                const int r = c0 + part + 4 * i;
+                v[i] = 0.0f;
+                if (FIXED || r < K)
+                    v[i] = __uint_as_float(__float_as_uint(__ldg(part_table + (c0 + 4 * i) * P + (comp[i] >> 1))) ^ (comp[i] << 31));
             }
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const float send = h8 ? v4[i] : v4[i + 2], keep = h8 ? v4[i + 2] : v4[i];
-                v2[i] = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 8));
+            for (int h = 4; h >= 1; h >>= 1) {
+#pragma unroll
+                for (int i = 0; i < h; ++i) v[i] = __fadd_rn(v[i], v[i + h]);
             }
-            {
-                const float send = h4 ? v2[0] : v2[1], keep = h4 ? v2[1] : v2[0];
-                t = __fadd_rn(keep, __shfl_xor_sync(kFull, send, 4));
-            }
+            float t = v[0];
             t = __fadd_rn(t, __shfl_xor_sync(kFull, t, 2));
             t = __fadd_rn(t, __shfl_xor_sync(kFull, t, 1));
             acc = __fadd_rn(acc, t);
         }
-        const float d = __shfl_sync(kFull, -acc, ((lane - g) & 7) * 4);  // lanes 4i .. 4i+3 hold node g + i
+        const float d = __shfl_sync(kFull, -acc, ((lane - g) & 7) * 4);
         if (lane >= g && lane < g + 8) mine = d;
     }
     return mine;
-}
-
-// The code row of every lane's own node to shared memory (rows `stride` bytes apart, 16-byte aligned).
-__device__ __forceinline__ void stage_codes(unsigned char* rows, int stride, const unsigned char* codes, int row_bytes,
-                                            const uint32_t* ids, uint32_t id, int total, int lane) {
-    if ((row_bytes & 15) == 0) {
-        if (lane < total) {
-            const uint4* src = reinterpret_cast<const uint4*>(codes + size_t(id) * row_bytes);
-            uint4* dst = reinterpret_cast<uint4*>(rows + lane * stride);
-            if (row_bytes == 32) {
-                const uint4 x = __ldg(src), y = __ldg(src + 1);
-                dst[0] = x;
-                dst[1] = y;
-            } else {
-#pragma unroll 4
-                for (int i = 0; i < row_bytes / 16; ++i) dst[i] = __ldg(src + i);
-            }
-        }
-    } else {
-        for (int c = 0; c < total; ++c)
-            for (int i = lane; i < row_bytes; i += 32) rows[c * stride + i] = __ldg(codes + size_t(ids[c]) * row_bytes + i);
-    }
-    __syncwarp();
 }
 
 // ---- entry scan ------------------------------------------------------------------------------------------------
@@ -265,6 +293,21 @@ struct ScanArgs {
     int K, P, row_bytes, packed_words, resid_kp, resid_mul;
     uint64_t* seeds;  // [nq][kScanKeep]
 };
+
+// compare-exchange across lanes s apart: the lane keeps the smaller key when `low`
+__device__ __forceinline__ uint64_t keep_order(uint64_t x, int s, bool low) {
+    const uint64_t z = __shfl_xor_sync(kFull, x, s);
+    return (z < x) == low ? z : x;
+}
+// the 32 smallest of two ascending lists, ascending: the smaller of (own, other reversed) is a bitonic sequence
+__device__ __forceinline__ uint64_t join_sorted(uint64_t x, uint64_t other, int lane) {
+    const uint64_t y = __shfl_sync(kFull, other, 31 - lane);
+    x = y < x ? y : x;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) x = keep_order(x, s, (lane & s) == 0);
+    return x;
+}
+constexpr int kSortAdmit = 8;  // from here on sorting a batch (120 instructions) costs less than inserting one by one (14 each)
 
 template <int QG>
 struct Vals {
@@ -306,7 +349,7 @@ __device__ __forceinline__ Vals<QG> scan_tree(const unsigned char* table, const 
 }
 
 template <bool U16, int METRIC, int QG>
-__global__ void __launch_bounds__(kScanWarps * 32)
+__global__ void __launch_bounds__(kScanWarps * 32, 3)
 entry_scan_kernel(ScanArgs a) {
     extern __shared__ __align__(16) unsigned char scan_smem[];
     __shared__ uint64_t lists[kScanWarps][QG][kScanKeep];
@@ -315,7 +358,7 @@ entry_scan_kernel(ScanArgs a) {
     const uint32_t q0 = blockIdx.x * QG;
     const int nblk = (a.K + 31) / 32;
     if (threadIdx.x < QG * kScanWarps) bound[threadIdx.x / kScanWarps][threadIdx.x % kScanWarps] = 0xffffffffu;
-    if constexpr (METRIC == kAsymSmem) {
+    if constexpr (METRIC == kAsym) {
         // lane = rotation; four indices of QG queries per pass
         float* tab = reinterpret_cast<float*>(scan_smem);
         const int quads = a.P / 4;
@@ -364,7 +407,7 @@ entry_scan_kernel(ScanArgs a) {
         const uint32_t ee = ok ? e : a.n_entry - 1;
         const uint32_t id = __ldg(a.entry + ee);
         float d[QG];
-        if constexpr (METRIC == kAsymSmem) {
+        if constexpr (METRIC == kAsym) {
             constexpr int WORDS = U16 ? 16 : 8;
             const uint4* row = reinterpret_cast<const uint4*>(a.entry_scan + size_t(ee) * nblk * (U16 ? 64 : 32));
 #pragma unroll
@@ -401,13 +444,22 @@ entry_scan_kernel(ScanArgs a) {
             const uint32_t lim = min(thr[g], __reduce_max_sync(kFull, others));
             uint32_t m = __ballot_sync(kFull, ok && uint32_t(key >> 32) <= lim);
             if (m == 0) continue;
-            while (m) {
-                const int src = __ffs(m) - 1;
-                m &= m - 1;
-                const uint64_t k = __shfl_sync(kFull, key, src);
-                const int r = __popc(__ballot_sync(kFull, best[g] < k));
-                const uint64_t up = __shfl_up_sync(kFull, best[g], 1);
-                best[g] = lane < r ? best[g] : (lane == r ? k : up);
+            if (__popc(m) > kSortAdmit) {  // many: sorted and joined as one list
+                uint64_t x = ((m >> lane) & 1u) ? key : kFiller;
+#pragma unroll
+                for (int k2 = 2; k2 <= 32; k2 <<= 1)
+#pragma unroll
+                    for (int s = k2 >> 1; s >= 1; s >>= 1) x = keep_order(x, s, ((lane & s) == 0) == ((lane & k2) == 0 || k2 == 32));
+                best[g] = join_sorted(best[g], x, lane);
+            } else {
+                while (m) {
+                    const int src = __ffs(m) - 1;
+                    m &= m - 1;
+                    const uint64_t k = __shfl_sync(kFull, key, src);
+                    const int r = __popc(__ballot_sync(kFull, best[g] < k));
+                    const uint64_t up = __shfl_up_sync(kFull, best[g], 1);
+                    best[g] = lane < r ? best[g] : (lane == r ? k : up);
+                }
             }
             const uint32_t hi = uint32_t(best[g] >> 32);
             thr[g] = __shfl_sync(kFull, hi, int(a.n_seed) - 1);
@@ -417,49 +469,37 @@ entry_scan_kernel(ScanArgs a) {
 #pragma unroll
     for (int g = 0; g < QG; ++g) lists[warp][g][lane] = best[g];
     __syncthreads();
-    // one warp per query joins the sorted lists: the lower half of (own, other reversed) is bitonic
+    // one warp per query joins the sorted lists
     for (int g = warp; g < QG; g += kScanWarps) {
         if (q0 + g >= a.nq) continue;
         uint64_t x = lists[0][g][lane];
         for (int o = 1; o < kScanWarps; ++o) {
-            const uint64_t y = lists[o][g][31 - lane];
-            x = y < x ? y : x;
-#pragma unroll
-            for (int s = 16; s >= 1; s >>= 1) {
-                const uint64_t z = __shfl_xor_sync(kFull, x, s);
-                const bool low = (lane & s) == 0;
-                x = (z < x) == low ? z : x;
-            }
+            x = join_sorted(x, lists[o][g][lane], lane);
         }
         a.seeds[size_t(q0 + g) * kScanKeep + lane] = x;
     }
 }
 
 template <bool U16, int METRIC, int WORDS>
-__global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
+__global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     const SearchArgs& a = w.s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
-    const size_t table_floats = METRIC == kAsymSmem ? size_t(a.K) * a.P : 0;
     const int row_bytes = a.K * (U16 ? 2 : 1);
-    unsigned char* area = walk_smem + size_t(w.smem_per_warp) * warp;
-    float* table_sm = reinterpret_cast<float*>(area);
-    uint64_t* W = reinterpret_cast<uint64_t*>(area + table_floats * 4);
-    uint4* tags = reinterpret_cast<uint4*>(W + w.wcap_slots);
+    uint64_t* W = reinterpret_cast<uint64_t*>(walk_smem + size_t(w.smem_per_warp) * warp);
+    uint2* tags = reinterpret_cast<uint2*>(W + w.wcap_slots);
     uint64_t* kbuf = reinterpret_cast<uint64_t*>(reinterpret_cast<unsigned char*>(tags) + (w.exact_visited ? 0 : kTagBytes));
     uint2* marks = reinterpret_cast<uint2*>(kbuf + 32);
     uint32_t* cid = reinterpret_cast<uint32_t*>(marks + WORDS * 32);
     uint32_t* front = cid + 32;  // the first unexpanded members of W
     unsigned char* qcode = reinterpret_cast<unsigned char*>(front + 8);  // symmetric metric: code bytes or packed words
-    unsigned char* rows_sm = qcode;                                      // asymmetric: the candidates' code rows
-    const int stride = (row_bytes + 15) / 16 * 16;
     uint32_t* qpacked = reinterpret_cast<uint32_t*>(qcode);
 
+    const uint32_t n = uint32_t(a.n);  // below 2^31
     const uint32_t slot = blockIdx.x * warps + warp;
     uint8_t* vis = w.exact_visited ? a.visited + size_t(slot) * a.vis_stride : nullptr;
     uint32_t epoch = w.exact_visited ? a.epochs[slot] : 0u;
-    const unsigned char* codes = static_cast<const unsigned char*>(a.codes);
 
     while (true) {
         uint32_t q = 0;
@@ -467,13 +507,7 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
         q = __shfl_sync(kFull, q, 0);
         if (q >= a.nq) break;
         __syncwarp();
-        const float* table = METRIC == kAsymSmem ? table_sm : (METRIC == kAsymGlobal ? a.tables + size_t(q) * a.K * a.P : nullptr);
-        if (METRIC == kAsymSmem) {
-            const float4* src = reinterpret_cast<const float4*>(a.tables + size_t(q) * table_floats);
-            float4* dst = reinterpret_cast<float4*>(table_sm);
-#pragma unroll 8
-            for (int i = lane; i < int(table_floats / 4); i += 32) dst[i] = __ldg(src + i);
-        }
+        const float* table = SYM ? nullptr : a.tables + size_t(q) * a.K * a.P;
         if (SYM) {
             const unsigned char* src = static_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes;
             if (METRIC == kSymBytes) {
@@ -487,7 +521,7 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
             }
         }
         if (!w.exact_visited) {
-            for (int i = lane; i < int(kTagBytes / 16); i += 32) tags[i] = make_uint4(0u, 0u, 0u, 0u);
+            for (int i = lane; i < int(kTagBytes / 16); i += 32) reinterpret_cast<uint4*>(tags)[i] = make_uint4(0u, 0u, 0u, 0u);
         } else if (++epoch == 256) {  // the 8-bit epoch wraps: forget every earlier query
             uint4* v4 = reinterpret_cast<uint4*>(vis);
             for (uint64_t i = lane; i < a.vis_stride / 16; i += 32) v4[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -503,14 +537,13 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
                 return lane < total ? packed_distance_lane(qpacked, a.packed, id, a.packed_words, a.resid_kp, a.resid_mul) : 0.0f;
             if (METRIC == kSymBytes)
                 return lane < total ? sym_distance_lane<U16>(qcode, a.codes, id, a.K, a.resid_kp, a.resid_mul) : 0.0f;
-            stage_codes(rows_sm, stride, codes, row_bytes, cid, id, total, lane);
-            return score_asym<U16, METRIC == kAsymSmem>(table, rows_sm, stride, a.K, a.P, total, lane);
+            return score_asym<U16, METRIC == kAsym128>(table, static_cast<const unsigned char*>(a.codes), a.K, a.P, cid, total, lane);
         };
         auto remember = [&](bool mine, uint32_t id) {
             if (w.exact_visited) {
                 if (mine) vis[id] = uint8_t(epoch);
             } else if (mine) {
-                tag_store(tags, tag_spot(id, w.id_bits_mask, w.tag_bits));
+                tag_store(tags, id);
             }
         };
 
@@ -527,7 +560,7 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
         for (uint32_t e0 = w.seeds ? a.n_entry : 0u; e0 < a.n_entry; e0 += 32) {
             const uint32_t e = e0 + lane;
             const uint32_t id = e < a.n_entry ? __ldg(a.entry + e) : kInvalidNode;
-            const bool ok = id < a.n;
+            const bool ok = id < n;
             const uint32_t m = __ballot_sync(kFull, ok);  // (entry ids are distinct and valid up to the end of the list)
             const int total = 32 - __clz(int(m));
             if (total == 0) continue;
@@ -559,19 +592,27 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
         for (int b = 0; b < kRows; ++b) pre_node[b] = kInvalidNode, pre_row[b] = kInvalidNode;
         while (true) {
             // the first kRows unexpanded members of the first window of 32 that has any (search_engine.hpp:121-123)
-            uint64_t ek = kFiller;
             uint32_t un = 0;
-            while (cur < count) {
-                const uint32_t p = cur + lane;
-                ek = p < count ? W[p] : kFiller;
-                un = __ballot_sync(kFull, !(uint32_t(ek) & 1u));
-                if (un) break;
-                cur += 32;
+            while (cur < count) {  // four windows at a time: an admission near the front sends the cursor back to it
+                uint32_t u[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t p = cur + 32 * i + lane;
+                    u[i] = __ballot_sync(kFull, p < count && !(uint32_t(W[min(p, count - 1)]) & 1u));
+                }
+                if (u[0] | u[1] | u[2] | u[3]) {
+                    const int i = u[0] ? 0 : (u[1] ? 1 : (u[2] ? 2 : 3));
+                    un = u[0] ? u[0] : (u[1] ? u[1] : (u[2] ? u[2] : u[3]));
+                    cur += 32 * i;
+                    break;
+                }
+                cur += 128;
             }
             if (!un) break;
             const uint32_t below = (1u << lane) - 1u;
             const uint32_t order = __popc(un & below);
             const bool open_member = (un >> lane) & 1u;
+            const uint64_t ek = W[min(cur + lane, count - 1)];
             if (open_member && order < 2 * kRows) front[order] = uint32_t(ek) >> 1;
             const uint32_t sel = __ballot_sync(kFull, open_member && order < kRows);  // the members taken
             const int have = __popc(un);
@@ -595,13 +636,13 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
             if (w.exact_visited) {
                 uint32_t vb[kRows];
 #pragma unroll
-                for (int b = 0; b < kRows; ++b) vb[b] = row[b] < a.n ? uint32_t(__ldcg(vis + row[b])) : epoch;
+                for (int b = 0; b < kRows; ++b) vb[b] = row[b] < n ? uint32_t(__ldcg(vis + row[b])) : epoch;
 #pragma unroll
                 for (int b = 0; b < kRows; ++b) fresh[b] = __ballot_sync(kFull, vb[b] != epoch);
             } else {
 #pragma unroll
                 for (int b = 0; b < kRows; ++b)
-                    fresh[b] = __ballot_sync(kFull, row[b] < a.n && !tag_seen(tags, tag_spot(row[b], w.id_bits_mask, w.tag_bits)));
+                    fresh[b] = __ballot_sync(kFull, row[b] < n && !tag_seen(tags, row[b]));
             }
             // as many leading rows as bring at most 32 candidates; lane c owns candidate c
             int total = 0, rows = 0, first_of[kRows];
@@ -636,8 +677,17 @@ __global__ void __launch_bounds__(512) search_walk_kernel(WalkArgs w) {
                 bool adm = own && (count < a.beam || key < W[count - 1]);
                 uint32_t am = __ballot_sync(kFull, adm);
                 if (am) {
-                    if (adm) {
+                    if (__popc(am) <= kFewRanked) {  // the warp ranks one key after the other
+                        for (uint32_t r = am; r;) {
+                            const int src = __ffs(r) - 1;
+                            r &= r - 1;
+                            const uint32_t at = lower_bound_warp(W, count, __shfl_sync(kFull, key, src), lane);
+                            if (lane == src) p = at;
+                        }
+                    } else if (adm) {
                         p = lower_bound(W, count, key);
+                    }
+                    if (adm) {
                         // a forgotten node that is a member of W
                         if (p < count && (W[p] >> 1) == (key >> 1)) adm = false;
                     }
@@ -772,9 +822,9 @@ int launch_scan(cphnsw_b200_index* h, const ScanArgs& a, int metric, cudaStream_
         return many ? launch_scan_t<U16, kSymPacked, 4>(h, a, size_t(16) * a.packed_words, st)
                     : launch_scan_t<U16, kSymPacked, 1>(h, a, size_t(4) * a.packed_words, st);
     const size_t table = size_t((a.K + 31) / 32) * 32 * a.P * 4;
-    if (many && a.nq > 2 * uint32_t(h->sm_count) && 4 * table <= 72 * 1024) return launch_scan_t<U16, kAsymSmem, 4>(h, a, 4 * table, st);
-    if (many && 2 * table <= 72 * 1024) return launch_scan_t<U16, kAsymSmem, 2>(h, a, 2 * table, st);
-    return launch_scan_t<U16, kAsymSmem, 1>(h, a, table, st);
+    if (many && a.nq > 2 * uint32_t(h->sm_count) && 4 * table <= 72 * 1024) return launch_scan_t<U16, kAsym, 4>(h, a, 4 * table, st);
+    if (many && 2 * table <= 72 * 1024) return launch_scan_t<U16, kAsym, 2>(h, a, 2 * table, st);
+    return launch_scan_t<U16, kAsym, 1>(h, a, table, st);
 }
 
 template <bool U16, int METRIC>
@@ -792,7 +842,7 @@ int launch_walk_t(cphnsw_b200_index* h, const WalkArgs& w, int blocks, int warps
 }  // namespace
 
 // Fills in the launch shape and runs walk and rerank.  a.next_query is zero on entry.
-int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, bool table_smem, cudaStream_t st) {
+int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool sym, cudaStream_t st) {
     WalkArgs w;
     w.s = a;
     w.cand = nullptr;
@@ -802,34 +852,29 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     }
     uint32_t top = a.beam > a.n_seed ? a.beam : a.n_seed;
     w.wcap_slots = (top + 31) & ~31u;
-    // exact tags: the id bits above the bucket index have to fit 16 bits
-    uint32_t id_bits = kBucketLog2;
-    while ((uint64_t(1) << id_bits) < a.n) ++id_bits;
-    w.tag_bits = id_bits - kBucketLog2;
-    w.id_bits_mask = uint32_t((uint64_t(1) << id_bits) - 1);
-    w.exact_visited = (a.stats != nullptr || w.tag_bits > 16) ? 1 : 0;
+    w.exact_visited = (a.stats != nullptr || a.n > kTagNodes) ? 1 : 0;
     if (w.exact_visited) {
         CPB_TRY(prepare_search_scratch(h, cx, st));
         w.s.visited = cx.d_visited.as<uint8_t>();
         w.s.vis_stride = cx.vis_stride;
         w.s.epochs = cx.d_epochs.as<uint32_t>();
     }
-    const int metric = sym ? (a.packed ? kSymPacked : kSymBytes) : (table_smem ? kAsymSmem : kAsymGlobal);
-    const size_t table = metric == kAsymSmem ? size_t(a.K) * a.P * 4 : 0;
+    const bool u16 = a.comp_bytes == 2;
+    const int metric = sym ? (a.packed ? kSymPacked : kSymBytes) : (!u16 && a.K == 32 && a.P == 128 ? kAsym128 : kAsym);
     const size_t row = (size_t(a.K) * a.comp_bytes + 15) / 16 * 16;
     const size_t words = w.wcap_slots <= 1024 ? 1 : 4;
-    // table, W, tags, merge scratch (keys, marks), candidate ids, front, then the query's code or the candidates' codes
-    w.smem_per_warp = uint32_t((table + size_t(w.wcap_slots) * 8 + (w.exact_visited ? 0 : kTagBytes) + 256 + words * 256 + 128 + 32 +
-                                (sym ? row : 32 * row) + 15) / 16 * 16);
+    // W, tags, merge scratch (keys, marks), candidate ids, front, the query's code
+    w.smem_per_warp = uint32_t((size_t(w.wcap_slots) * 8 + (w.exact_visited ? 0 : kTagBytes) + 256 + words * 256 + 128 + 32 +
+                                (sym ? row : 0) + 15) / 16 * 16);
     int warps = int((226 * 1024) / w.smem_per_warp);
-    if (warps > 16) warps = 16;
+    const int most = w.exact_visited && warps > 16 ? 16 : kWalkWarps;  // visited arrays: 16 per SM
+    if (warps > most) warps = most;
     const int per_sm = int((a.nq + h->sm_count - 1) / h->sm_count);  // a small batch spreads over all SMs
     if (warps > per_sm) warps = per_sm;
     if (warps < 1) warps = 1;
     if (!cx.wide) warps = 1;
     const uint64_t want = (uint64_t(a.nq) + warps - 1) / warps;
     const int blocks = int(want < uint64_t(h->sm_count) ? want : uint64_t(h->sm_count));
-    const bool u16 = a.comp_bytes == 2;
     w.seeds = nullptr;
     const size_t scan_table = size_t((a.K + 31) / 32) * 32 * a.P * 4;
     if (a.n_seed < a.n_entry && a.n_seed <= uint32_t(kScanKeep) && (sym || (a.P >= 4 && scan_table <= 200 * 1024))) {
@@ -854,8 +899,8 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     }
 #define CPB_WALK(X) (u16 ? launch_walk_t<true, X>(h, w, blocks, warps, st) : launch_walk_t<false, X>(h, w, blocks, warps, st))
     switch (metric) {
-        case kAsymSmem: CPB_TRY(CPB_WALK(kAsymSmem)); break;
-        case kAsymGlobal: CPB_TRY(CPB_WALK(kAsymGlobal)); break;
+        case kAsym: CPB_TRY(CPB_WALK(kAsym)); break;
+        case kAsym128: CPB_TRY((launch_walk_t<false, kAsym128>(h, w, blocks, warps, st))); break;
         case kSymBytes: CPB_TRY(CPB_WALK(kSymBytes)); break;
         default: CPB_TRY(CPB_WALK(kSymPacked)); break;
     }
