@@ -28,65 +28,84 @@ namespace {
 
 constexpr int kP128 = 128;
 constexpr int kTileVecs = 128;          // vectors per block = threads per block
-// Padded row of the staged tile: thread t reads bank (t + i) & 31.  (Measured and dropped: a 132-float stride with
-// 128-bit reloads, 3.875 ms per 1M vectors against 3.835 ms, and on top of it the diagonal applied as a sign-bit XOR
-// on the integer pipe with plain first-stage butterflies, 3.883 ms.  Also measured and dropped: the diagonal folded
-// into every stage - block multipliers t = s[i] * s[i + h], butterflies fma(+-t, y, x), one overall sign per layer
-// left for the end - which is bit-equal and saves the 64 multiplies per layer, 3.894 ms: the three-operand
-// instructions cost what the saved ones gave.)
-constexpr int kTileStride = kP128 + 1;
+// Padded row of the staged tile: 64-bit reads of 16 threads hit distinct banks.  (Measured and dropped with scalar
+// arithmetic: the diagonal applied as a sign-bit XOR on the integer pipe, 3.883 ms per 1M vectors against 3.835 ms; the
+// diagonal folded into every stage as block multipliers, 3.894 ms.)
+constexpr int kTileStride = kP128 + 2;
 
-template <int H>
-__device__ __forceinline__ void butterfly_stage(float (&v)[kP128]) {
+// ---- packed fp32 pairs (two IEEE operations per instruction, each rounded as the scalar one) -----------------------
+// The transform is bound by fp32 adds; packing leaves the add pipe as busy but halves the issue slots they take, which
+// scalar code shared with the argmax and the table reads.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// butterflies between pairs H apart (elements 2 * H apart)
+template <int H, int N>
+__device__ __forceinline__ void butterfly_pairs(f32x2 (&v)[N]) {
 #pragma unroll
-    for (int i = 0; i < kP128; i += 2 * H) {
+    for (int i = 0; i < N; i += 2 * H) {
 #pragma unroll
         for (int j = i; j < i + H; ++j) {
-            float x = v[j], y = v[j + H];
-            v[j] = __fadd_rn(x, y);
-            v[j + H] = __fsub_rn(x, y);
+            const f32x2 x = v[j], y = v[j + H];
+            v[j] = add2(x, y);
+            v[j + H] = sub2(x, y);
         }
     }
 }
 
-// D then H on 128 registers.  `sg` points at 128 +-1 floats in shared memory, read by every
-// thread at the same address (broadcast).
-__device__ __forceinline__ void diag_fht128(float (&v)[kP128], const float* __restrict__ sg) {
-    const float4* s4 = reinterpret_cast<const float4*>(sg);
+// D then H on 128 values held as 64 pairs of neighbours.  `sg` points at 128 +-1 floats in shared memory, read by
+// every thread at the same address (broadcast).  The products with +-1 are exact.
+__device__ __forceinline__ void diag_fht128(f32x2 (&v)[kP128 / 2], const float* __restrict__ sg) {
+    const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(sg);
 #pragma unroll
     for (int c = 0; c < kP128 / 4; ++c) {
-        float4 s = s4[c];
-        {
-            float t = __fmul_rn(s.x, v[4 * c]);
-            float y = v[4 * c + 1];
-            v[4 * c] = __fmaf_rn(s.y, y, t);
-            v[4 * c + 1] = __fmaf_rn(-s.y, y, t);
-        }
-        {
-            float t = __fmul_rn(s.z, v[4 * c + 2]);
-            float y = v[4 * c + 3];
-            v[4 * c + 2] = __fmaf_rn(s.w, y, t);
-            v[4 * c + 3] = __fmaf_rn(-s.w, y, t);
-        }
+        const ulonglong2 s = s2[c];
+        float a, b;
+        unpack2(mul2(v[2 * c], s.x), a, b);
+        v[2 * c] = pack2(__fadd_rn(a, b), __fsub_rn(a, b));
+        unpack2(mul2(v[2 * c + 1], s.y), a, b);
+        v[2 * c + 1] = pack2(__fadd_rn(a, b), __fsub_rn(a, b));
     }
-    butterfly_stage<2>(v);
-    butterfly_stage<4>(v);
-    butterfly_stage<8>(v);
-    butterfly_stage<16>(v);
-    butterfly_stage<32>(v);
-    butterfly_stage<64>(v);
+    butterfly_pairs<1>(v);
+    butterfly_pairs<2>(v);
+    butterfly_pairs<4>(v);
+    butterfly_pairs<8>(v);
+    butterfly_pairs<16>(v);
+    butterfly_pairs<32>(v);
 }
 
 // Lowest-index argmax of |v| by a left-biased tournament: the right operand wins only when it is
 // strictly larger, so among equal magnitudes the lowest index survives every round
 // (same answer as the strict `>` scan of cp_encoder.hpp:82-88).
-__device__ __forceinline__ void argmax128(const float (&v)[kP128], float& win, int& idx) {
+__device__ __forceinline__ void argmax128(const f32x2 (&v)[kP128 / 2], float& win, int& idx) {
     float w[64];
     int id[64];
 #pragma unroll
     for (int j = 0; j < 64; ++j) {
-        bool r = fabsf(v[2 * j + 1]) > fabsf(v[2 * j]);
-        w[j] = r ? v[2 * j + 1] : v[2 * j];
+        float a, b;
+        unpack2(v[j], a, b);
+        bool r = fabsf(b) > fabsf(a);
+        w[j] = r ? b : a;
         id[j] = r ? 2 * j + 1 : 2 * j;
     }
 #pragma unroll
@@ -113,13 +132,14 @@ __device__ __forceinline__ uint32_t component_of(float win, int idx, int flip_ma
 // QUERY = true additionally writes the rotated vectors and winning magnitudes (CPQuery).
 template <typename CompT, bool QUERY>
 __global__ void __launch_bounds__(kTileVecs, QUERY ? 2 : 3)
-encode_p128_kernel(const float* __restrict__ x, uint64_t n, int dim, int K,
+encode_p128_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb /* rotations per block */,
                    const float* __restrict__ signs /*[K][3][128]*/, int flip_mask,
                    CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
     extern __shared__ float smem[];
     float* tile = smem;                                                 // [kTileVecs][kTileStride]
     float* sign_sm = tile + kTileVecs * kTileStride;                              // [2][3][128], double buffer
-    CompT* code_tile = reinterpret_cast<CompT*>(sign_sm + 2 * 3 * kP128);         // [kTileVecs][K]
+    CompT* code_tile = reinterpret_cast<CompT*>(sign_sm + 2 * 3 * kP128);         // [kTileVecs][rotations of this block]
+    const int r0 = blockIdx.y * rpb, r1 = min(K, r0 + rpb), nr = r1 - r0;
 
     const uint64_t row0 = uint64_t(blockIdx.x) * kTileVecs;
     const int rows = int(min(uint64_t(kTileVecs), n - row0));
@@ -153,46 +173,52 @@ encode_p128_kernel(const float* __restrict__ x, uint64_t n, int dim, int K,
     // the three diagonals of one rotation are staged in shared memory one rotation ahead
     const int t = threadIdx.x;
     if (t < 3 * kP128 / 4)
-        reinterpret_cast<float4*>(sign_sm)[t] = __ldg(reinterpret_cast<const float4*>(signs) + t);
+        reinterpret_cast<float4*>(sign_sm)[t] = __ldg(reinterpret_cast<const float4*>(signs + size_t(r0) * 3 * kP128) + t);
     __syncthreads();
 
-    const float* mine = tile + t * kTileStride;
+    const f32x2* mine = reinterpret_cast<const f32x2*>(tile + t * kTileStride);
     const uint64_t row = row0 + t;
-    for (int r = 0; r < K; ++r) {
-        if (r + 1 < K && t < 3 * kP128 / 4)
-            reinterpret_cast<float4*>(sign_sm + ((r + 1) & 1) * 3 * kP128)[t] =
+    for (int r = r0; r < r1; ++r) {
+        if (r + 1 < r1 && t < 3 * kP128 / 4)
+            reinterpret_cast<float4*>(sign_sm + ((r + 1 - r0) & 1) * 3 * kP128)[t] =
                 __ldg(reinterpret_cast<const float4*>(signs + size_t(r + 1) * 3 * kP128) + t);
-        float v[kP128];
+        f32x2 v[kP128 / 2];
 #pragma unroll
-        for (int i = 0; i < kP128; ++i) v[i] = mine[i];
-        const float* sg = sign_sm + (r & 1) * 3 * kP128;
+        for (int i = 0; i < kP128 / 2; ++i) v[i] = mine[i];
+        const float* sg = sign_sm + ((r - r0) & 1) * 3 * kP128;
 #pragma unroll 1
         for (int layer = 0; layer < 3; ++layer) diag_fht128(v, sg + layer * kP128);
         float win;
         int idx;
         argmax128(v, win, idx);
-        code_tile[t * K + r] = CompT(component_of(win, idx, flip_mask));
+        code_tile[t * nr + (r - r0)] = CompT(component_of(win, idx, flip_mask));
         if (QUERY && t < rows) {
             if (mags) mags[row * K + r] = fabsf(win);
             if (rotated) {
                 float4* out = reinterpret_cast<float4*>(rotated + (row * K + r) * kP128);
 #pragma unroll
                 for (int c = 0; c < kP128 / 4; ++c) {
+                    float a0, a1, a2, a3;
+                    unpack2(v[2 * c], a0, a1);
+                    unpack2(v[2 * c + 1], a2, a3);
                     float4 o;
-                    o.x = (__popc((4 * c) & flip_mask) & 1) ? -v[4 * c] : v[4 * c];
-                    o.y = (__popc((4 * c + 1) & flip_mask) & 1) ? -v[4 * c + 1] : v[4 * c + 1];
-                    o.z = (__popc((4 * c + 2) & flip_mask) & 1) ? -v[4 * c + 2] : v[4 * c + 2];
-                    o.w = (__popc((4 * c + 3) & flip_mask) & 1) ? -v[4 * c + 3] : v[4 * c + 3];
+                    o.x = (__popc((4 * c) & flip_mask) & 1) ? -a0 : a0;
+                    o.y = (__popc((4 * c + 1) & flip_mask) & 1) ? -a1 : a1;
+                    o.z = (__popc((4 * c + 2) & flip_mask) & 1) ? -a2 : a2;
+                    o.w = (__popc((4 * c + 3) & flip_mask) & 1) ? -a3 : a3;
                     out[c] = o;
                 }
             }
         }
         __syncthreads();  // the next rotation's diagonals are in place, this rotation's are free
     }
-    // the tile's codes are contiguous in the output: write them back coalesced
-    const int total = rows * K;
+    // the tile's codes are contiguous in the output (a row of K at a time when the rotations are split over blocks)
     CompT* dst = codes + row0 * uint64_t(K);
-    for (int i = threadIdx.x; i < total; i += kTileVecs) dst[i] = code_tile[i];
+    if (nr == K) {
+        for (int i = threadIdx.x; i < rows * K; i += kTileVecs) dst[i] = code_tile[i];
+    } else {
+        for (int i = threadIdx.x; i < rows * nr; i += kTileVecs) dst[uint64_t(i / nr) * K + r0 + i % nr] = code_tile[i];
+    }
 }
 
 // ---- padded dim 1024 (d in 513..1024): one warp per vector, 32 elements per lane -------------------
@@ -207,17 +233,18 @@ constexpr int kP1024 = 1024;
 constexpr int kWarps1024 = 4;
 
 __device__ __forceinline__ void fht32_regs(float (&v)[32]) {
+    f32x2 p[16];
 #pragma unroll
-    for (int h = 1; h < 32; h <<= 1) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            if ((j & h) == 0) {
-                const float x = v[j], y = v[j + h];
-                v[j] = __fadd_rn(x, y);
-                v[j + h] = __fsub_rn(x, y);
-            }
-        }
+    for (int j = 0; j < 16; ++j) {
+        const float x = v[2 * j], y = v[2 * j + 1];
+        p[j] = pack2(__fadd_rn(x, y), __fsub_rn(x, y));
     }
+    butterfly_pairs<1>(p);
+    butterfly_pairs<2>(p);
+    butterfly_pairs<4>(p);
+    butterfly_pairs<8>(p);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) unpack2(p[j], v[2 * j], v[2 * j + 1]);
 }
 
 __device__ __forceinline__ void flip_signs32(float (&v)[32], uint32_t word) {
@@ -228,7 +255,7 @@ __device__ __forceinline__ void flip_signs32(float (&v)[32], uint32_t word) {
 
 template <typename CompT, bool QUERY>
 __global__ void __launch_bounds__(kWarps1024 * 32)
-encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K,
+encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb,
                     const uint32_t* __restrict__ signbits /*[K][3][32]*/, int flip_mask,
                     CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
     __shared__ float tiles[kWarps1024][32 * 33];
@@ -254,7 +281,7 @@ encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K,
                 xin[j] = i < dim ? __ldg(src + i) : 0.0f;
             }
         }
-        for (int r = 0; r < K; ++r) {
+        for (int r = blockIdx.y * rpb; r < min(K, int(blockIdx.y + 1) * rpb); ++r) {
             const uint32_t* sb = signbits + size_t(r) * 3 * 32;
             float v[32];
 #pragma unroll
@@ -326,7 +353,7 @@ encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K,
 // bit-identical.  Nothing goes through shared memory.
 template <typename CompT, bool QUERY, int E>
 __global__ void __launch_bounds__(128)
-encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, const float* __restrict__ signs /*[K][3][P]*/,
+encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb, const float* __restrict__ signs /*[K][3][P]*/,
                    int flip_mask, CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
     constexpr int P = 32 * E;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -336,7 +363,7 @@ encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, cons
         float in[E];
 #pragma unroll
         for (int j = 0; j < E; ++j) in[j] = first + j < dim ? __ldg(src + first + j) : 0.0f;
-        for (int r = 0; r < K; ++r) {
+        for (int r = blockIdx.y * rpb; r < min(K, int(blockIdx.y + 1) * rpb); ++r) {
             float v[E];
 #pragma unroll
             for (int j = 0; j < E; ++j) v[j] = in[j];
@@ -481,6 +508,14 @@ __global__ void sign_only_bytes_kernel(unsigned char* __restrict__ codes, uint64
     if (i < bytes) codes[i] &= (comp_bytes == 2 && (i & 1)) ? 0u : 1u;  // little-endian halfwords: the high byte is cleared
 }
 
+// The rotations of a vector are independent, so few vectors spread them over blocks until `want` blocks are in flight
+// (a lone vector of padded dim 128: one thread's 32 rotations in sequence took 115 us, one rotation a block 7 us).
+static int rotations_per_block(uint64_t blocks, uint64_t want, int K) {
+    uint64_t split = (want + blocks - 1) / blocks;
+    if (split > uint64_t(K)) split = K;
+    return int((K + split - 1) / split);
+}
+
 int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_codes, float* d_rot,
                   float* d_mag, cudaStream_t st) {
     if (n == 0) return 0;
@@ -497,12 +532,15 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     if (P == kP128) {
         size_t smem = size_t(kTileVecs) * kTileStride * sizeof(float) + size_t(2) * 3 * kP128 * sizeof(float) +
                       size_t(kTileVecs) * K * h->comp_bytes;
-        unsigned grid = unsigned((n + kTileVecs - 1) / kTileVecs);
+        const uint64_t tiles = (n + kTileVecs - 1) / kTileVecs;
+        const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * 6, K);
+        smem -= size_t(kTileVecs) * (K - rpb) * h->comp_bytes;
+        const dim3 grid(unsigned(tiles), unsigned((K + rpb - 1) / rpb));
         const bool query = d_rot || d_mag;
 #define CPB_LAUNCH_P128(T, Q)                                                                              \
     do {                                                                                                   \
         CPB_CUDA(allow_max_dynamic_smem(encode_p128_kernel<T, Q>));                                        \
-        encode_p128_kernel<T, Q><<<grid, kTileVecs, smem, st>>>(d_x, n, dim, K, signs, flip_mask,           \
+        encode_p128_kernel<T, Q><<<grid, kTileVecs, smem, st>>>(d_x, n, dim, K, rpb, signs, flip_mask,           \
                                                                (T*)d_codes, d_rot, d_mag);                  \
     } while (0)
         if (h->comp_bytes == 1) {
@@ -516,10 +554,11 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     } else if (P == kP1024 && h->d_signbits.p) {
         const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + kWarps1024 - 1) / kWarps1024;
-        const unsigned grid = unsigned(blocks < uint64_t(h->sm_count) * 16 ? blocks : uint64_t(h->sm_count) * 16);
+        const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 16, K);
+        const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 16 ? blocks : uint64_t(h->sm_count) * 16), unsigned((K + rpb - 1) / rpb));
         const uint32_t* sb = h->d_signbits.as<uint32_t>();
 #define CPB_LAUNCH_P1024(T, Q)                                                                              \
-    encode_p1024_kernel<T, Q><<<grid, kWarps1024 * 32, 0, st>>>(d_x, n, dim, K, sb, flip_mask, (T*)d_codes, d_rot, d_mag)
+    encode_p1024_kernel<T, Q><<<grid, kWarps1024 * 32, 0, st>>>(d_x, n, dim, K, rpb, sb, flip_mask, (T*)d_codes, d_rot, d_mag)
         if (h->comp_bytes == 1) {  // (a 1-byte component cannot hold a 1024-wide index; kept for symmetry)
             if (query) CPB_LAUNCH_P1024(uint8_t, true);
             else CPB_LAUNCH_P1024(uint8_t, false);
@@ -531,9 +570,10 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     } else if (P == 32 || P == 64 || P == 256 || P == 512) {
         const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + 3) / 4;
-        const unsigned grid = unsigned(blocks < uint64_t(h->sm_count) * 32 ? blocks : uint64_t(h->sm_count) * 32);
+        const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 32, K);
+        const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 32 ? blocks : uint64_t(h->sm_count) * 32), unsigned((K + rpb - 1) / rpb));
 #define CPB_LAUNCH_WARP(T, Q, EE) \
-    encode_warp_kernel<T, Q, EE><<<grid, 128, 0, st>>>(d_x, n, dim, K, signs, flip_mask, (T*)d_codes, d_rot, d_mag)
+    encode_warp_kernel<T, Q, EE><<<grid, 128, 0, st>>>(d_x, n, dim, K, rpb, signs, flip_mask, (T*)d_codes, d_rot, d_mag)
 #define CPB_LAUNCH_WARP_E(T, Q)                      \
     do {                                             \
         if (P == 32) CPB_LAUNCH_WARP(T, Q, 1);       \
