@@ -648,7 +648,7 @@ int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double v) {
     if (s == "prune") { h->prune = v != 0.0; return 0; }
     if (s == "profile") { h->profile = v != 0.0; return 0; }
     if (s == "knn_kernel") {
-        if (v != 0 && v != 1 && v != 2) { set_error("knn_kernel must be 0 (pick), 1 (byte-wise) or 2 (bit-sliced)"); return CPHNSW_B200_E_INVALID; }
+        if (v != 0 && v != 1 && v != 2 && v != 3) { set_error("knn_kernel must be 0 (pick), 1 (byte-wise), 2 (bit-sliced) or 3 (tensor-core filter)"); return CPHNSW_B200_E_INVALID; }
         h->knn_kernel = int(v);
         return 0;
     }

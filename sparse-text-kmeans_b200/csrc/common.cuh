@@ -131,7 +131,7 @@ struct cphnsw_b200_index {
     int keep_pruned = 1;
     int prune = 1;  // 0: the bulk build keeps the M nearest kNN candidates instead of running select_neighbors
     uint32_t k_entry = 4, knn_k = 0, entry_scan = 0;
-    int knn_kernel = 0;  // 0 = pick, 1 = byte-wise distance, 2 = bit-sliced distance
+    int knn_kernel = 0;  // 0 = pick, 1 = byte-wise distance, 2 = bit-sliced distance, 3 = tensor-core filter
     int search_kernel = 0;  // 0 = pick, 1 = one warp per query, 2 = two warps per query
     int search_table_smem = 1;  // 0: the query table is read in place even when it would fit shared memory
     int binary_codes = 0;  // 1: components keep only the sign bit (Hamming metric), search walks under the code distance
@@ -208,6 +208,10 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
 bool knn_sliced_supported(const cphnsw_b200_index* h);
 int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
                             uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
+// tensor-core filter and exact distances of the pairs that pass (knn_mma.cu); padded: code rows of `words` 32-bit words
+bool knn_mma_supported(const cphnsw_b200_index* h);
+int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,
+                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
 int launch_select_neighbors(cphnsw_b200_index* h, const void* d_codes, uint64_t n, const uint32_t* d_cand,
                             uint32_t k, uint64_t row_begin, uint64_t row_end, uint32_t M, int keep_pruned,
                             uint32_t* d_adj, cudaStream_t st, const uint32_t* d_row_ids = nullptr);

@@ -587,6 +587,9 @@ static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_
     return launch_knn_t<WC, U16, 4, Q>(h, codes, n, k, rb, re, nbrs, dist, st);
 }
 
+// From this many nodes on the tensor-core kernel is taken; below it the launches around it cost more than the sweep.
+constexpr uint64_t kMmaMinNodes = 4096;
+
 int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
                      uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
     if (row_end <= row_begin) return 0;
@@ -607,6 +610,17 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
     if (h->knn_kernel == 2 && !knn_sliced_supported(h)) {
         set_error("knn_kernel=2 (bit-sliced) needs K = 16, 32 or 64 with uint8 components, K = 16 / 32 with padded dim 1024, or one-byte sign-bit codes of whole blocks of 8 components (K <= 120)");
         return CPHNSW_B200_E_UNSUPPORTED;
+    }
+    if (h->knn_kernel == 3 && !knn_mma_supported(h)) {
+        set_error("knn_kernel=3 (tensor-core filter) needs plain codes of 2 to 74 components");
+        return CPHNSW_B200_E_UNSUPPORTED;
+    }
+    // (rows of whole 16-byte words are read in place and have to be aligned then)
+    const bool readable = (reinterpret_cast<uintptr_t>(d_codes) & 15) == 0 || size_t(h->K) * h->comp_bytes != size_t(WC) * 4;
+    if (h->knn_kernel == 3 || (h->knn_kernel == 0 && n >= kMmaMinNodes && readable && knn_mma_supported(h))) {
+        const uint32_t* pc;
+        CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
+        return launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist, st);
     }
     if (h->knn_kernel != 1 && knn_sliced_supported(h))
         return launch_knn_graph_sliced(h, d_codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);

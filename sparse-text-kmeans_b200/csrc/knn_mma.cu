@@ -1,0 +1,734 @@
+// Brute-force code-distance kNN graph with the tensor cores as a filter.
+//
+// Same result as the two other kNN kernels (k smallest under (distance, id), self excluded).  The distance of two codes
+// is K minus the number of components they share.  Every component is hashed to one of S = 8 (K <= 32) or 4 symbols and a
+// symbol is written as a row of the S-point Hadamard matrix without its constant column: S - 1 values of +-1 whose dot
+// product is S - 1 for equal symbols and -1 for different ones.  The dot product of two such rows of (S - 1) K values is
+// S m - K, m the number of components with equal symbols, and m is at least the number of equal components: a pair whose
+// dot product is below S (K - t) - K differs in more than t components.  The products run on tcgen05 in fp8 with fp16
+// accumulators (+-1 and integers up to 224 are exact in both), so all n^2 pairs cost 2 * 224 tensor operations and one
+// instruction of the epilogue each; only pairs that reach the row's threshold t have their exact distance computed.
+//
+// Row thresholds.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie
+// beside rows that share both, and the k-th smallest exact distance in a window of 256 of them (the row itself aside),
+// the least over four such orders, bounds the row's final t from above.  On clustered data this leaves some 600 passing
+// pairs per row, 250 of them truly within t.  The pairs found are kept in a buffer; when it runs full its k best are
+// kept and t falls below the worst of them for the pairs still to come, which have higher ids.  On data without clusters
+// the bound says nothing and t is lowered by this alone.
+//
+// Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the candidates
+// in tiles of 256, two stages of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
+// halves of tensor memory; while one half is computed the eight epilogue warps of the other read it.  The operand is laid
+// out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a tile is one
+// contiguous copy and no tensor map is needed.  Blocks that take whole rows of tiles sweep them in step, so that a tile
+// comes from L2; only the rows left over by the last full wave are split between blocks along the candidates.
+#include <cuda_fp16.h>
+
+#include "knn_common.cuh"
+
+namespace cpb {
+namespace {
+
+using knn::kFull;
+using knn::kWaitLimit;
+using knn::mbar_wait_bounded;
+using knn::smem_u32;
+
+constexpr int kMmaRows = 256;             // rows per block and candidates per tile
+constexpr int kMmaCap = 288;              // entries of a buffer: at most 128 before a tile, 32 still queued and 128 from it
+constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
+constexpr uint32_t kMmaKeep = 128;
+constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, a half of the columns
+constexpr int kMmaThreads = (kEpiWarps + 2) * 32;  // and one that copies, one that issues the products
+constexpr uint32_t kTmemCols = 512;
+constexpr int kQueue = 64;                // pairs a warp collects before it computes the distances of 32
+constexpr int kBoundOrders = 4;           // orders of likely neighbours
+constexpr int kBoundWindow = 256;         // rows looked at per order
+constexpr uint32_t kKeys = 65536;
+
+// symbols and values of a code shape; 0 symbols: not served
+struct HashShape {
+    int symbols, chunks;  // chunks: 16-byte pieces of a row's operand, an even number
+};
+__host__ __device__ inline HashShape hash_shape(int K) {
+    HashShape s;
+    s.symbols = K <= 32 ? 8 : (K <= 74 ? 4 : 0);
+    const int values = K * (s.symbols - 1);
+    s.chunks = (values + 31) / 32 * 2;
+    return s;
+}
+
+__device__ __forceinline__ uint32_t symbol_of(uint32_t comp, uint32_t symbols) {
+    return (comp ^ (comp >> 3) ^ (comp >> 6) ^ (comp >> 9)) & (symbols - 1);
+}
+
+// ---- operand: [tile of 256 rows][chunk][row][16 values] ------------------------------------------------------------
+template <typename CompT>
+__global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n, int K, int symbols, int chunks,
+                                    uint4* __restrict__ out, uint64_t tiles) {
+    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= tiles * chunks * kMmaRows) return;
+    const int r = int(t % kMmaRows), c = int(t / kMmaRows % chunks);
+    const uint64_t row = t / (uint64_t(kMmaRows) * chunks) * kMmaRows + r;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (row < n) {
+        int comp = c * 16 / (symbols - 1), j = c * 16 % (symbols - 1) + 1;
+        uint32_t h = comp < K ? symbol_of(codes[row * K + comp], uint32_t(symbols)) : 0u;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const uint32_t e4m3 = (__popc(h & uint32_t(j)) & 1) ? 0xB8u : 0x38u;  // -1 : +1
+            if (comp < K) w[i / 4] |= e4m3 << (8 * (i % 4));
+            if (++j == symbols) {
+                j = 1;
+                ++comp;
+                if (comp < K) h = symbol_of(codes[row * K + comp], uint32_t(symbols));
+            }
+        }
+    }
+    out[t] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// ---- exact distance: differing bytes / halfwords of two padded rows -------------------------------------------------
+template <bool U16>
+__device__ __forceinline__ uint32_t exact_distance(const uint4* __restrict__ codes, int quads, uint32_t a, uint32_t b) {
+    constexpr uint32_t LO = U16 ? 0x7fff7fffu : 0x7f7f7f7fu;
+    const uint4* pa = codes + size_t(a) * quads;
+    const uint4* pb = codes + size_t(b) * quads;
+    uint32_t d = 0;
+#pragma unroll 2
+    for (int i = 0; i < quads; ++i) {
+        const uint4 x = __ldg(pa + i), y = __ldg(pb + i);
+        const uint32_t v[4] = {x.x ^ y.x, x.y ^ y.y, x.z ^ y.z, x.w ^ y.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d += __popc((((v[j] & LO) + LO) | v[j]) & ~LO);
+    }
+    return d;
+}
+
+// Smallest T with at least `need` of the lanes' entries at distance <= T (entries without a node hold kFull); K when
+// there are fewer.
+template <int SLOTS>
+__device__ __forceinline__ uint32_t kth_distance(const uint32_t (&dist)[SLOTS], uint32_t need, int K) {
+    uint32_t lo = 0, hi = uint32_t(K);
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        uint32_t c = 0;
+#pragma unroll
+        for (int s = 0; s < SLOTS; ++s) c += dist[s] <= mid;
+        if (__reduce_add_sync(kFull, c) >= need) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
+
+// ---- bounds from likely neighbours ---------------------------------------------------------------------------------
+// the low 8 bits of two components (the sign and the low index bits; all of a one-byte component)
+template <typename CompT>
+__device__ __forceinline__ uint32_t row_key(const CompT* codes, int K, uint64_t row, int order) {
+    return (uint32_t(codes[row * K + (2 * order) % K]) & 0xffu) << 8 | (uint32_t(codes[row * K + (2 * order + 1) % K]) & 0xffu);
+}
+template <typename CompT>
+__global__ void key_count_kernel(const CompT* __restrict__ codes, uint64_t n, int K, uint32_t* __restrict__ hist) {
+    const uint64_t row = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (row < n) atomicAdd(hist + size_t(blockIdx.y) * kKeys + row_key(codes, K, row, blockIdx.y), 1u);
+}
+__global__ void __launch_bounds__(1024) key_scan_kernel(uint32_t* __restrict__ hist) {  // exclusive, one block per order
+    __shared__ uint32_t sums[32];
+    uint4* h = reinterpret_cast<uint4*>(hist + size_t(blockIdx.x) * kKeys + threadIdx.x * (kKeys / 1024));
+    uint32_t own = 0;
+#pragma unroll 8
+    for (int i = 0; i < int(kKeys / 4096); ++i) {
+        const uint4 v = h[i];
+        own += v.x + v.y + v.z + v.w;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = own;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, d);
+        if (lane >= d) x += y;
+    }
+    if (lane == 31) sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t s = sums[lane];
+        const uint32_t o = s;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, s, d);
+            if (lane >= d) s += y;
+        }
+        sums[lane] = s - o;
+    }
+    __syncthreads();
+    uint32_t at = sums[warp] + x - own;
+#pragma unroll 4
+    for (int i = 0; i < int(kKeys / 4096); ++i) {
+        const uint4 c = h[i];
+        h[i] = make_uint4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
+        at += c.x + c.y + c.z + c.w;
+    }
+}
+template <typename CompT>
+__global__ void key_scatter_kernel(const CompT* __restrict__ codes, uint64_t n, int K, uint32_t* __restrict__ hist,
+                                   uint32_t* __restrict__ order /* [orders][n] */) {
+    const uint64_t row = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (row >= n) return;
+    const uint32_t at = atomicAdd(hist + size_t(blockIdx.y) * kKeys + row_key(codes, K, row, blockIdx.y), 1u);
+    order[size_t(blockIdx.y) * n + at] = uint32_t(row);
+}
+// A warp takes the row at one place of one order: the k-th smallest distance in the window around it, itself aside.
+template <bool U16>
+__global__ void bound_kernel(const uint4* __restrict__ codes, int quads, int K, uint64_t n, const uint32_t* __restrict__ order,
+                             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t at = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    if (at >= n) return;
+    const uint32_t* ord = order + size_t(blockIdx.y) * n;
+    const uint32_t row = ord[at];
+    if (row < row_begin || row >= row_end) return;
+    uint64_t first = at < kBoundWindow / 2 ? 0 : at - kBoundWindow / 2;
+    if (first + kBoundWindow > n) first = n > kBoundWindow ? n - kBoundWindow : 0;
+    uint32_t dist[kBoundWindow / 32];
+#pragma unroll
+    for (int s = 0; s < kBoundWindow / 32; ++s) {
+        const uint64_t p = first + s * 32 + lane;
+        const uint32_t id = p < n ? ord[p] : row;
+        dist[s] = id != row ? exact_distance<U16>(codes, quads, row, id) : kFull;
+    }
+    const uint32_t T = kth_distance(dist, k, K);  // (K when the window holds fewer than k others)
+    if (lane == 0) atomicMin(bound + row, T);
+}
+
+// ---- tcgen05 pieces ------------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
+    // K-major, no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes apart along the rows (stride offset) and
+    // 256 * 16 bytes apart along K (leading offset); version 1
+    uint64_t d = (smem_addr >> 4) & 0x3fffu;
+    d |= uint64_t((kMmaRows * 16) >> 4) << 16;
+    d |= uint64_t(128 >> 4) << 32;
+    d |= uint64_t(1) << 46;
+    return d;
+}
+// D fp16, A and B e4m3, both K-major, M = 128, N = 256
+constexpr uint32_t kIdesc = (uint32_t(256 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+
+__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a, uint64_t b, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(kIdesc), "r"(uint32_t(accumulate))
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// 32 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
+__device__ __forceinline__ void tmem_load32(uint32_t (&r)[16], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+        "%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr)
+        : "memory");
+}
+// (the registers are operands so that no use of them moves in front of the wait)
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+// A bounded wait that also ends when another role of the block has given up.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* aborted) {
+    for (uint32_t i = 0; i < limit; ++i) {
+        if (knn::mbar_try_wait(bar, parity)) return true;
+        if ((i & 63) == 63 && *aborted) return false;
+    }
+    return false;
+}
+
+// ---- work split -----------------------------------------------------------------------------------------------------
+// A launch takes `rts` row tiles against all `cts` candidate tiles: rts * cts steps in row-major order, an equal run of
+// them for every block.  When rts is a multiple of the blocks a block takes whole row tiles, and all blocks read the same
+// candidate tiles at the same time; otherwise a row tile may be shared by blocks.  Along the runs block + row tile only
+// grows, so it names a segment (one block's part of one row tile) and its buffers.
+struct Split {
+    uint64_t steps;
+    uint32_t cts, blocks;
+    __host__ __device__ uint64_t first_step(uint32_t block) const { return uint64_t(block) * steps / blocks; }
+    __host__ __device__ uint32_t block_of(uint64_t step) const { return uint32_t(((step + 1) * blocks - 1) / steps); }
+};
+
+struct KnnMmaArgs {
+    const uint4* operand;  // [tiles][chunks][256]
+    const uint4* codes;    // padded rows
+    int quads;             // 16-byte words of a padded row
+    int K, symbols, chunks;
+    uint64_t n;
+    uint32_t k;
+    Split split;
+    uint32_t tile0;               // first row tile of the launch
+    uint32_t row_begin, row_end;  // rows wanted
+    const uint32_t* bound;        // [n] bounds on the final thresholds
+    uint32_t* ids;                // [segments][256 rows][2 sides][kMmaCap]
+    uint8_t* dists;               // the same
+    uint32_t* counts;             // [segments][256][2]
+    uint32_t* status;
+    uint32_t first_wait_polls;
+};
+
+// the dot product a pair at distance <= t reaches at least (t < 0: none does), twice
+__device__ __forceinline__ __half2 dot_of_distance(int symbols, int K, int t) {
+    return t < 0 ? __half2half2(__ushort_as_half(0x7c00)) : __float2half2_rn(float(symbols * (K - t) - K));
+}
+
+// The row's buffer shrinks to its k best (or all that are no worse than the k-th, up to kMmaKeep).  By the whole warp;
+// returns the k-th distance and the new count.
+__device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, uint32_t& count, uint32_t k, int K, int lane) {
+    uint32_t id[kMmaSlots], dist[kMmaSlots];
+#pragma unroll
+    for (int s = 0; s < kMmaSlots; ++s) {
+        const uint32_t e = uint32_t(s * 32 + lane);
+        id[s] = e < count ? ids[e] : kInvalidNode;
+        dist[s] = e < count ? dists[e] : kFull;
+    }
+    const uint32_t T = kth_distance(dist, k, K);
+    uint32_t below = 0, upto = 0;
+#pragma unroll
+    for (int s = 0; s < kMmaSlots; ++s) below += dist[s] < T, upto += dist[s] <= T;
+    below = __reduce_add_sync(kFull, below);
+    upto = __reduce_add_sync(kFull, upto);
+    uint32_t last = kInvalidNode;  // largest id kept at distance T
+    if (upto > kMmaKeep) {
+        uint32_t lo = 0, hi = kInvalidNode;
+        while (lo < hi) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            uint32_t c = 0;
+#pragma unroll
+            for (int s = 0; s < kMmaSlots; ++s) c += dist[s] == T && id[s] <= mid;
+            if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
+            else lo = mid + 1;
+        }
+        last = lo;
+    }
+    __syncwarp();
+    uint32_t at = 0;
+#pragma unroll
+    for (int s = 0; s < kMmaSlots; ++s) {
+        const bool keep = dist[s] < T || (dist[s] == T && id[s] <= last);
+        const uint32_t m = __ballot_sync(kFull, keep);
+        if (keep) {
+            const uint32_t to = at + __popc(m & ((1u << lane) - 1u));
+            ids[to] = id[s];
+            dists[to] = uint8_t(dist[s]);
+        }
+        at += __popc(m);
+    }
+    __syncwarp();
+    count = at;
+    return T;
+}
+
+template <bool U16>
+__global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
+    extern __shared__ __align__(1024) unsigned char mma_smem[];
+    __shared__ __align__(8) uint64_t full_bar[2], empty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
+    __shared__ uint2 queue[kEpiWarps][kQueue];      // {candidate, lane of the row}
+    __shared__ int limit[2][2][kMmaRows];           // [segment parity][side][row]: largest distance still of use
+    __shared__ uint32_t filled[2][kMmaRows];        // [side][row]: entries of the buffer
+    __shared__ uint32_t tmem_base_sm;
+    __shared__ int abort_flag;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t operand_bytes = uint32_t(a.chunks) * kMmaRows * 16;
+    unsigned char* a_sm = mma_smem;
+    unsigned char* b_sm = mma_smem + operand_bytes;  // two stages
+    const uint64_t s0 = a.split.first_step(blockIdx.x);
+    const uint32_t steps = uint32_t(a.split.first_step(blockIdx.x + 1) - s0);
+    const uint32_t rt0 = uint32_t(s0 / a.split.cts), ct0 = uint32_t(s0 % a.split.cts);  // first row and candidate tile
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) {
+            knn::mbar_init(&full_bar[i], 1);
+            knn::mbar_init(&empty_bar[i], 1);
+            knn::mbar_init(&tfull_bar[i], 1);
+            knn::mbar_init(&tempty_bar[i], kEpiWarps / 2);
+        }
+        knn::mbar_init(&drain_bar, 1);
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kEpiWarps + 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sm)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base_sm;
+    volatile int* aborted = &abort_flag;
+
+    uint32_t loads = 0;  // steps whose copies were issued
+    if (warp == kEpiWarps) {
+        if (lane == 0) {
+            uint32_t rt = rt0, ct = ct0;
+            bool fresh = true;  // the row tile's own operand has to come too
+            for (uint32_t i = 0; i < steps && !*aborted; ++i) {
+                const uint32_t s = i & 1;
+                bool ok = wait_or_abort(&empty_bar[s], ((i >> 1) & 1) ^ 1, kWaitLimit, aborted);
+                // it replaces the one that the step before still reads
+                if (ok && fresh && i) ok = wait_or_abort(&empty_bar[s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted);
+                if (!ok) {
+                    *aborted = 1;
+                    break;
+                }
+                knn::mbar_expect_tx(&full_bar[s], fresh ? 2 * operand_bytes : operand_bytes);
+                const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
+                if (fresh) knn::bulk_g2s(a_sm, op + size_t(a.tile0 + rt) * operand_bytes, operand_bytes, &full_bar[s]);
+                knn::bulk_g2s(b_sm + s * operand_bytes, op + size_t(ct) * operand_bytes, operand_bytes, &full_bar[s]);
+                ++loads;
+                fresh = ++ct == a.split.cts;
+                if (fresh) ct = 0, ++rt;
+            }
+        }
+    } else if (warp == kEpiWarps + 1) {
+        if (lane == 0) {
+            const uint64_t a_desc = operand_desc(smem_u32(a_sm));
+            const uint64_t b_desc[2] = {operand_desc(smem_u32(b_sm)), operand_desc(smem_u32(b_sm + operand_bytes))};
+            const int ksteps = a.chunks / 2;
+            bool ok = true;
+            for (uint32_t i = 0; i < steps && ok && !*aborted; ++i) {
+                const uint32_t s = i & 1;
+                ok = wait_or_abort(&full_bar[s], (i >> 1) & 1, i == 0 ? a.first_wait_polls : kWaitLimit, aborted);
+                for (int h = 0; h < 2 && ok; ++h) {
+                    ok = wait_or_abort(&tempty_bar[h], (i & 1) ^ 1, kWaitLimit, aborted);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    for (int ks = 0; ks < ksteps; ++ks)  // 32 values of K a step: two 16-byte chunks
+                        mma_f8(tmem + h * 256, a_desc + uint64_t((h * 128 * 16 + ks * 2 * kMmaRows * 16) >> 4),
+                               b_desc[s] + uint64_t((ks * 2 * kMmaRows * 16) >> 4), ks != 0);
+                    mma_commit(&tfull_bar[h]);
+                }
+                if (ok) mma_commit(&empty_bar[s]);
+            }
+            if (!ok) *aborted = 1;
+            mma_commit(&drain_bar);  // everything issued above has finished when this completes
+        }
+    } else {
+        const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
+        const uint32_t base = uint32_t(half * 128 + quarter * 32), local = base + lane;  // rows of the warp, of the lane
+        const uint32_t n = uint32_t(a.n);
+        const uint32_t below = (1u << lane) - 1u;
+        const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256 + side * 128;
+        uint2* mine = queue[warp];
+        uint32_t rt = rt0, ct = ct0, queued = 0, parity = 0;
+        bool ok = true, fresh = true;
+        for (uint32_t i = 0; i < steps; ++i) {
+            const uint32_t row0 = (a.tile0 + rt) * kMmaRows + base;  // the warp's first row
+            const size_t buf0 = ((size_t(blockIdx.x + rt) * kMmaRows + base) * 2 + side) * kMmaCap;  // and its buffer
+            if (fresh) {
+                const uint32_t row = row0 + lane;
+                const bool wanted = row >= a.row_begin && row < a.row_end;
+                limit[parity][side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
+                filled[side][local] = 0;
+                __syncwarp();
+            }
+            // distances of the last `m` queued pairs; those of use go to their row's buffer
+            auto drain = [&](uint32_t m) {
+                __syncwarp();
+                queued -= m;
+                if (uint32_t(lane) < m) {
+                    const uint2 e = mine[queued + lane];
+                    const uint32_t row = row0 + e.y;
+                    const int d = int(exact_distance<U16>(a.codes, a.quads, row, e.x));
+                    if (e.x != row && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + e.y])) {
+                        const uint32_t at = atomicAdd(&filled[side][base + e.y], 1u);
+                        const size_t to = buf0 + size_t(e.y) * (2 * kMmaCap) + at;
+                        a.ids[to] = e.x;
+                        a.dists[to] = uint8_t(d);
+                    }
+                }
+                __syncwarp();
+            };
+            ok = wait_or_abort(&tfull_bar[half], i & 1, kWaitLimit, aborted);
+            if (__ballot_sync(kFull, !ok || *aborted)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[parity][side][local]));
+            // pairs that pass, bit j of a word: column 2 j for j < 16, else column 2 (j - 16) + 1; one load is in flight
+            // while the columns of the one before are compared
+            uint32_t pass[4], r[2][16];
+            tmem_load32(r[0], addr);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tmem_wait(r[c & 1]);
+                if (c < 3) tmem_load32(r[(c + 1) & 1], addr + (c + 1) * 32);
+                uint32_t m = 0;
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    m |= __hge2_mask(*reinterpret_cast<const __half2*>(&r[c & 1][j]), thr) & (0x00010001u << j);
+                pass[c] = m;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty_bar[half]);
+
+            const uint32_t col0 = ct * kMmaRows + side * 128;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t any;
+                while ((any = __ballot_sync(kFull, pass[c] != 0)) != 0) {
+                    const uint32_t b = __ffs(pass[c]) - 1;  // (of an empty word: not used)
+                    const uint32_t col = col0 + c * 32 + 2 * (b & 15) + (b >> 4);
+                    bool take = pass[c] != 0 && col < n;
+                    pass[c] &= pass[c] - 1;
+                    const uint32_t m = __ballot_sync(kFull, take);
+                    if (take) mine[queued + __popc(m & below)] = make_uint2(col, uint32_t(lane));
+                    queued += __popc(m);
+                    if (queued >= 32) drain(32);
+                }
+            }
+            // a row whose buffer could overflow in the next tile
+            uint32_t full = __ballot_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&filled[side][local]) > kMmaKeep);
+            const bool last_of_segment = ct + 1 == a.split.cts || i + 1 == steps;
+            if (full || last_of_segment) {
+                drain(queued);
+                full = __ballot_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&filled[side][local]) > kMmaKeep);
+                while (full) {
+                    const int src = __ffs(full) - 1;
+                    full &= full - 1;
+                    uint32_t count = filled[side][base + src];
+                    const size_t b = buf0 + size_t(src) * (2 * kMmaCap);
+                    const uint32_t T = compact_row(a.ids + b, a.dists + b, count, a.k, a.K, lane);
+                    if (lane == 0) {
+                        filled[side][base + src] = count;
+                        // this side's later candidates have higher ids and must be strictly closer
+                        atomicMin(&limit[parity][side][base + src], int(T) - 1);
+                        atomicMin(&limit[parity][side ^ 1][base + src], int(T));
+                    }
+                    __syncwarp();
+                }
+            }
+            fresh = last_of_segment;
+            if (fresh) {
+                a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = filled[side][local];
+                // the row's other warp may be a tile behind and still lower the old limits
+                parity ^= 1;
+            }
+            if (++ct == a.split.cts) ct = 0, ++rt;
+        }
+        if (!ok) *aborted = 1;
+    }
+    __syncthreads();
+    // copies and products in flight after a lost wait end before the block's memory goes away
+    if (warp == kEpiWarps && lane == 0 && *aborted) {
+        atomicExch(a.status, kStatusWaitTimeout);
+        for (uint32_t i = loads > 2 ? loads - 2 : 0; i < loads; ++i) mbar_wait_bounded(&full_bar[i & 1], (i >> 1) & 1, kWaitLimit);
+    }
+    if (warp == kEpiWarps + 1) {
+        if (lane == 0) mbar_wait_bounded(&drain_bar, 0, kWaitLimit);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    }
+    __syncthreads();
+}
+
+// ---- results: the k best of a row's buffers by (distance, id) ---------------------------------------------------------
+constexpr int kFinishWarps = 4;
+constexpr int kFinishKeys = 512;
+
+__global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
+                                                                       uint16_t* __restrict__ dists, uint32_t out_row0) {
+    __shared__ uint64_t keys_sm[kFinishWarps][kFinishKeys];
+    __shared__ uint32_t hist_sm[kFinishWarps][96];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t local = blockIdx.x * kFinishWarps + warp;
+    if (local >= rows) return;
+    const uint32_t row = a.tile0 * kMmaRows + local;
+    if (row < a.row_begin || row >= a.row_end) return;
+    uint64_t* keys = keys_sm[warp];
+    uint32_t* hist = hist_sm[warp];
+    const uint32_t rt = local / kMmaRows, in_tile = local % kMmaRows;
+    const uint32_t seg0 = a.split.block_of(uint64_t(rt) * a.split.cts) + rt;
+    const uint32_t seg1 = a.split.block_of(uint64_t(rt + 1) * a.split.cts - 1) + rt;
+    // every buffer of the row, 32 entries at a time
+    auto each = [&](auto&& f) {
+        for (uint32_t b = seg0 * 2; b <= seg1 * 2 + 1; ++b) {
+            const size_t slot = (size_t(b >> 1) * kMmaRows + in_tile) * 2 + (b & 1);
+            const uint32_t count = a.counts[slot];
+            for (uint32_t e = 0; e < count; e += 32) {
+                const bool have = e + lane < count;
+                f(have ? uint32_t(a.dists[slot * kMmaCap + e + lane]) : kFull, slot * kMmaCap + e + lane);
+            }
+        }
+    };
+    for (int i = lane; i < 96; i += 32) hist[i] = 0;
+    __syncwarp();
+    each([&](uint32_t d, size_t) {
+        if (d != kFull) atomicAdd(hist + d, 1u);
+    });
+    __syncwarp();
+    // T: the k-th distance (K when there are fewer); lane l owns bins 3 l .. 3 l + 2
+    const uint32_t h0 = hist[3 * lane], h1 = hist[3 * lane + 1], h2 = hist[3 * lane + 2];
+    uint32_t x = h0 + h1 + h2;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    const uint32_t total = __shfl_sync(kFull, x, 31), lower = x - h0 - h1 - h2;  // entries in the bins of earlier lanes
+    uint32_t T = kFull, below = 0;
+    if (lower < a.k && x >= a.k) {
+        T = 3 * lane, below = lower;
+        if (below + h0 < a.k) {
+            ++T, below += h0;
+            if (below + h1 < a.k) ++T, below += h1;
+        }
+    }
+    const uint32_t owner = __ballot_sync(kFull, T != kFull);
+    uint32_t last = kInvalidNode, kept = total;  // largest id of use at distance T; entries collected
+    if (owner) {
+        const int src = __ffs(owner) - 1;
+        T = __shfl_sync(kFull, T, src);
+        below = __shfl_sync(kFull, below, src);
+        kept = below + hist[T];
+        if (kept > uint32_t(kFinishKeys)) {  // a great many ties: the id that bounds the ones wanted
+            uint32_t lo = 0, hi = kInvalidNode;
+            while (lo < hi) {
+                const uint32_t mid = lo + ((hi - lo) >> 1);
+                uint32_t c = 0;
+                each([&](uint32_t d, size_t at) { c += d == T && a.ids[at] <= mid; });
+                if (__reduce_add_sync(kFull, c) >= a.k - below) hi = mid;
+                else lo = mid + 1;
+            }
+            last = lo;
+        }
+    }
+    uint32_t m = 0;
+    each([&](uint32_t d, size_t at) {
+        const uint32_t id = d <= T && d != kFull ? a.ids[at] : kInvalidNode;
+        const bool take = id != kInvalidNode && (d < T || id <= last);
+        const uint32_t b = __ballot_sync(kFull, take);
+        if (take) keys[m + __popc(b & ((1u << lane) - 1u))] = (uint64_t(d) << 32) | id;
+        m += __popc(b);
+    });
+    __syncwarp();
+    uint32_t* out_n = nbrs + size_t(row - out_row0) * a.k;
+    uint16_t* out_d = dists ? dists + size_t(row - out_row0) * a.k : nullptr;
+    for (uint32_t e = lane; e < m; e += 32) {  // rank by counting: keys are distinct
+        const uint64_t key = keys[e];
+        uint32_t rank = 0;
+#pragma unroll 4
+        for (uint32_t i = 0; i < m; ++i) rank += keys[i] < key;
+        if (rank < a.k) {
+            out_n[rank] = uint32_t(key);
+            if (out_d) out_d[rank] = uint16_t(key >> 32);
+        }
+    }
+    for (uint32_t o = m + lane; o < a.k; o += 32) {
+        out_n[o] = kInvalidNode;
+        if (out_d) out_d[o] = 0xFFFF;
+    }
+}
+
+template <typename CompT>
+int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k, uint64_t row_begin,
+                 uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
+    constexpr bool U16 = sizeof(CompT) == 2;
+    const CompT* codes = static_cast<const CompT*>(d_codes);
+    const HashShape shape = hash_shape(int(h->K));
+    const uint64_t tiles = (n + kMmaRows - 1) / kMmaRows;
+    const size_t operand_bytes = size_t(shape.chunks) * kMmaRows * 16;
+    const uint64_t sms = uint64_t(h->sm_count);
+    // row tiles go in launches of whole waves (the buffers of a segment take 720 KB) and a last one that splits the rest
+    constexpr uint64_t kWaves = 4;
+    const uint64_t first_tile = row_begin / kMmaRows, end_tile = (row_end - 1) / kMmaRows + 1;
+    const uint64_t most = end_tile - first_tile < kWaves * sms ? end_tile - first_tile : kWaves * sms;
+    const size_t segments = size_t(most + sms);
+
+    auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
+    const size_t op_b = up(size_t(tiles) * operand_bytes), hist_b = up(size_t(kBoundOrders) * kKeys * 4);
+    const size_t order_b = up(size_t(kBoundOrders) * n * 4), bound_b = up(size_t(n) * 4);
+    const size_t slots = segments * kMmaRows * 2;
+    const size_t ids_b = up(slots * kMmaCap * 4), dists_b = up(slots * kMmaCap), counts_b = up(slots * 4);
+    CPB_TRY(h->s_sliced.reserve(op_b + hist_b + order_b + bound_b + ids_b + dists_b + counts_b));
+    unsigned char* p = h->s_sliced.as<unsigned char>();
+    auto take = [&](size_t b) {
+        unsigned char* r = p;
+        p += b;
+        return r;
+    };
+    uint4* operand = reinterpret_cast<uint4*>(take(op_b));
+    uint32_t* hist = reinterpret_cast<uint32_t*>(take(hist_b));
+    uint32_t* order = reinterpret_cast<uint32_t*>(take(order_b));
+    uint32_t* bound = reinterpret_cast<uint32_t*>(take(bound_b));
+
+    KnnMmaArgs a;
+    a.operand = operand;
+    a.codes = reinterpret_cast<const uint4*>(padded);
+    a.quads = words / 4;
+    a.K = int(h->K);
+    a.symbols = shape.symbols;
+    a.chunks = shape.chunks;
+    a.n = n;
+    a.k = k;
+    a.row_begin = uint32_t(row_begin);
+    a.row_end = uint32_t(row_end);
+    a.bound = bound;
+    a.ids = reinterpret_cast<uint32_t*>(take(ids_b));
+    a.dists = reinterpret_cast<uint8_t*>(take(dists_b));
+    a.counts = reinterpret_cast<uint32_t*>(take(counts_b));
+    a.status = h->d_status.as<uint32_t>();
+    a.first_wait_polls = h->first_wait_polls;
+
+    LaunchTimer timer(h, kKernelKnn, st);
+    const uint64_t cells = tiles * shape.chunks * kMmaRows;
+    expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(codes, n, int(h->K), shape.symbols, shape.chunks, operand, tiles);
+    CPB_CUDA(cudaMemsetAsync(hist, 0, size_t(kBoundOrders) * kKeys * 4, st));
+    CPB_CUDA(cudaMemsetAsync(bound, 0xff, size_t(n) * 4, st));
+    const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
+    key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
+    key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
+    key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order);
+    bound_kernel<U16><<<dim3(unsigned((n + 7) / 8), kBoundOrders), 256, 0, st>>>(a.codes, a.quads, a.K, n, order, k, a.row_begin, a.row_end,
+                                                                               bound);
+    h->launches += 5;
+    CPB_CUDA(cudaGetLastError());
+    CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16>));
+    for (uint64_t t0 = first_tile; t0 < end_tile;) {
+        const uint64_t left = end_tile - t0;
+        const uint64_t rts = left >= kWaves * sms ? kWaves * sms : (left >= sms ? left / sms * sms : left);
+        a.tile0 = uint32_t(t0);
+        a.split.cts = uint32_t(tiles);
+        a.split.steps = rts * tiles;
+        a.split.blocks = uint32_t(a.split.steps < sms ? a.split.steps : sms);
+        knn_mma_kernel<U16><<<a.split.blocks, kMmaThreads, 3 * operand_bytes, st>>>(a);
+        const uint32_t rows = uint32_t(rts) * kMmaRows;
+        knn_finish_kernel<<<(rows + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, rows, d_nbrs, d_dist, uint32_t(row_begin));
+        h->launches += 2;
+        CPB_CUDA(cudaGetLastError());
+        t0 += rts;
+    }
+    return 0;
+}
+
+}  // namespace
+
+// Plain K-component codes of up to 74 components (the operand of 256 rows has to fit shared memory three times).
+bool knn_mma_supported(const cphnsw_b200_index* h) {
+    return !h->binary_codes && !h->residual_bits && h->K >= 2 && hash_shape(int(h->K)).symbols != 0;
+}
+
+int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,
+                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
+    if (h->comp_bytes == 2) return launch_mma_t<uint16_t>(h, d_codes, padded, words, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+    return launch_mma_t<uint8_t>(h, d_codes, padded, words, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+}
+
+}  // namespace cpb

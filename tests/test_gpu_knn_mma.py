@@ -1,0 +1,92 @@
+"""The kNN graph with the tensor cores as a filter (csrc/knn_mma.cu, knn_kernel = 3) against the CPU oracle: neighbour
+ids and distances are integers with ties broken by id, so every comparison is exact."""
+import numpy as np
+import pytest
+
+from cphnsw_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cp():
+    import cphnsw_b200
+    return cphnsw_b200
+
+
+@pytest.fixture(scope="module")
+def oracle():
+    import oracle
+    return oracle
+
+
+def index(cp, dim, K, cb):
+    idx = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
+    idx.set_param("knn_kernel", 3)
+    return idx
+
+
+def check(idx, oracle, codes, k, rows=None):
+    n = codes.shape[0]
+    rb, re = rows or (0, n)
+    nbrs, dist = idx.knn_graph(codes, k, rb, re)
+    wn, wd = oracle.knn_graph(codes, k, rb, re)
+    assert np.array_equal(nbrs, wn) and np.array_equal(dist, wd)
+
+
+# tiles are 256 rows by 256 candidates; 8 symbols up to K = 32, 4 up to K = 74
+@pytest.mark.parametrize("n,k,K,cb,dim", [(1, 4, 32, 1, 128), (255, 64, 32, 1, 128), (256, 127, 32, 1, 128), (257, 1, 16, 1, 100),
+                                          (513, 40, 2, 1, 64), (3000, 64, 32, 1, 128), (2999, 32, 24, 1, 96), (2049, 64, 33, 1, 128),
+                                          (4100, 64, 64, 1, 128), (1500, 127, 74, 1, 128), (2300, 64, 32, 2, 960), (1200, 20, 64, 2, 300)])
+def test_shapes(cp, oracle, n, k, K, cb, dim):
+    base, _ = synthetic.gaussian_mixture(n, 1, dim, max(1, n // 400), 0.3, n + K)
+    codes = oracle.encode(base, K, cb, oracle.sign_tables(dim, K, 42))
+    idx = index(cp, dim, K, cb)
+    check(idx, oracle, codes, k)
+    if n > 600:
+        check(idx, oracle, codes, k, (n // 3, n // 3 + 300))  # a row block across a tile edge
+
+
+# the row buffers overflow many times: unclustered rows, identical rows, rows that differ in one component only
+@pytest.mark.parametrize("kind", ["random", "equal", "near"])
+def test_full_buffers_and_ties(cp, oracle, kind):
+    rng = np.random.default_rng(7)
+    n, K = 6000, 32
+    codes = rng.integers(0, 256, (n, K)).astype(np.uint8)
+    if kind == "equal":
+        codes[:] = codes[0]
+    if kind == "near":
+        codes[:] = codes[0]
+        codes[np.arange(n), rng.integers(0, K, n)] = rng.integers(0, 256, n)
+    idx = index(cp, 128, K, 1)
+    check(idx, oracle, codes, 64, (0, 700))
+    check(idx, oracle, codes, 127, (n - 300, n))
+
+
+def test_many_clusters_against_the_bit_sliced_kernel(cp):
+    # row tiles in a full wave of blocks and in a split one; both kernels are exact, so they agree
+    base, _ = synthetic.gaussian_mixture(70_001, 1, 128, 70, 0.3, 11)
+    idx = index(cp, 128, 32, 1)
+    codes = idx.encode(base)
+    a = idx.knn_graph(codes, 64)
+    idx.set_param("knn_kernel", 2)
+    b = idx.knn_graph(codes, 64)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+def test_lost_wait_is_reported(cp, oracle):
+    # the first wait gets no polls: every role of the block ends and the call reports it; the handle stays usable
+    codes = np.random.default_rng(3).integers(0, 256, (3000, 32)).astype(np.uint8)
+    idx = index(cp, 128, 32, 1)
+    idx.set_param("first_wait_polls", 0)
+    with pytest.raises(cp.CPHNSWError) as err:
+        idx.knn_graph(codes, 16)
+    assert "[%d]" % cp.E_DEVICE_WAIT in str(err.value)
+    idx.set_param("first_wait_polls", 1 << 22)
+    check(idx, oracle, codes, 16)
+
+
+def test_unsupported_codes_are_refused(cp):
+    idx = index(cp, 128, 100, 1)
+    with pytest.raises(cp.CPHNSWError):
+        idx.knn_graph(np.zeros((10, 100), np.uint8), 4)
