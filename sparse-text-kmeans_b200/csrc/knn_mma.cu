@@ -10,11 +10,11 @@
 // instruction of the epilogue each; only pairs that reach the row's threshold t have their exact distance computed.
 //
 // Row thresholds.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie
-// beside rows that share both, and the k-th smallest exact distance in a window of 256 of them (the row itself aside),
-// the least over four such orders, bounds the row's final t from above.  On clustered data this leaves some 600 passing
-// pairs per row, 250 of them truly within t.  The pairs found are kept in a buffer; when it runs full its k best are
-// kept and t falls below the worst of them for the pairs still to come, which have higher ids.  On data without clusters
-// the bound says nothing and t is lowered by this alone.
+// beside rows that share both, and the k-th smallest exact distance in the windows of 128 around a row in eight such
+// orders, every row counted once, bounds its final t from above.  On clustered data t is mostly right or one too high, and
+// some 450 pairs per row pass, 140 of them truly within t.  The pairs found are kept in a buffer; when it runs full its k
+// best are kept and t falls below the worst of them for the pairs still to come, which have higher ids.  On data without
+// clusters the bound says nothing and t is lowered by this alone.
 //
 // Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the candidates
 // in tiles of 256, two stages of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
@@ -35,15 +35,15 @@ using knn::mbar_wait_bounded;
 using knn::smem_u32;
 
 constexpr int kMmaRows = 256;             // rows per block and candidates per tile
-constexpr int kMmaCap = 288;              // entries of a buffer: at most 128 before a tile, 32 still queued and 128 from it
+constexpr int kMmaCap = 384;              // entries of a buffer: at most 256 before a tile and 128 from it
 constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
-constexpr uint32_t kMmaKeep = 128;
+constexpr uint32_t kMmaKeep = 256;
 constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, a half of the columns
 constexpr int kMmaThreads = (kEpiWarps + 2) * 32;  // and one that copies, one that issues the products
 constexpr uint32_t kTmemCols = 512;
-constexpr int kQueue = 64;                // pairs a warp collects before it computes the distances of 32
-constexpr int kBoundOrders = 4;           // orders of likely neighbours
-constexpr int kBoundWindow = 256;         // rows looked at per order
+constexpr int kMaxCodeStages = 4;
+constexpr int kBoundOrders = 8;           // orders of likely neighbours
+constexpr int kBoundWindow = 128;         // rows looked at per order
 constexpr uint32_t kKeys = 65536;
 
 // symbols and values of a code shape; 0 symbols: not served
@@ -89,18 +89,25 @@ __global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n,
 }
 
 // ---- exact distance: differing bytes / halfwords of two padded rows -------------------------------------------------
-template <bool U16>
-__device__ __forceinline__ uint32_t exact_distance(const uint4* __restrict__ codes, int quads, uint32_t a, uint32_t b) {
+// a flag in the top bit of every differing byte (halfword), the flags of 8 (16) words packed for one popcount
+template <bool U16, int QUADS>
+__device__ __forceinline__ uint32_t code_distance(const uint4 (&a)[QUADS], const uint4* b) {
     constexpr uint32_t LO = U16 ? 0x7fff7fffu : 0x7f7f7f7fu;
-    const uint4* pa = codes + size_t(a) * quads;
-    const uint4* pb = codes + size_t(b) * quads;
-    uint32_t d = 0;
-#pragma unroll 2
-    for (int i = 0; i < quads; ++i) {
-        const uint4 x = __ldg(pa + i), y = __ldg(pb + i);
-        const uint32_t v[4] = {x.x ^ y.x, x.y ^ y.y, x.z ^ y.z, x.w ^ y.w};
+    constexpr int G = U16 ? 16 : 8;
+    uint32_t d = 0, acc = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) d += __popc((((v[j] & LO) + LO) | v[j]) & ~LO);
+    for (int i = 0; i < QUADS; ++i) {
+        const uint4 y = b[i];
+        const uint32_t v[4] = {a[i].x ^ y.x, a[i].y ^ y.y, a[i].z ^ y.z, a[i].w ^ y.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int sh = (i * 4 + j) % G;
+            acc |= ((((v[j] & LO) + LO) | v[j]) >> sh) & (~LO >> sh);
+        }
+        if ((i + 1) * 4 % G == 0 || i + 1 == QUADS) {
+            d += __popc(acc);
+            acc = 0;
+        }
     }
     return d;
 }
@@ -169,33 +176,75 @@ __global__ void __launch_bounds__(1024) key_scan_kernel(uint32_t* __restrict__ h
 }
 template <typename CompT>
 __global__ void key_scatter_kernel(const CompT* __restrict__ codes, uint64_t n, int K, uint32_t* __restrict__ hist,
-                                   uint32_t* __restrict__ order /* [orders][n] */) {
+                                   uint32_t* __restrict__ order /* [orders][n] */, uint32_t* __restrict__ place /* [n][orders] */) {
     const uint64_t row = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (row >= n) return;
     const uint32_t at = atomicAdd(hist + size_t(blockIdx.y) * kKeys + row_key(codes, K, row, blockIdx.y), 1u);
     order[size_t(blockIdx.y) * n + at] = uint32_t(row);
+    place[row * kBoundOrders + blockIdx.y] = at;
 }
-// A warp takes the row at one place of one order: the k-th smallest distance in the window around it, itself aside.
-template <bool U16>
-__global__ void bound_kernel(const uint4* __restrict__ codes, int quads, int K, uint64_t n, const uint32_t* __restrict__ order,
-                             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t at = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+// A warp takes a row: the k-th smallest distance among the rows in the windows around it in all orders, each counted
+// once.  (The least of the orders' own k-th distances is 0.4 to 1 higher, which lets half as many pairs again through.)
+// Rows are taken as the first order has them, whose neighbours share much of their windows.
+constexpr int kBoundWarps = 8;
+constexpr uint32_t kSeenSlots = 1024;
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kBoundWarps * 32)
+bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t* __restrict__ order, const uint32_t* __restrict__ place,
+             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound) {
+    constexpr int S = kBoundWindow / 32, N = kBoundOrders * S;
+    __shared__ uint32_t seen_sm[kBoundWarps][kSeenSlots];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t at = uint64_t(blockIdx.x) * kBoundWarps + warp;
     if (at >= n) return;
-    const uint32_t* ord = order + size_t(blockIdx.y) * n;
-    const uint32_t row = ord[at];
+    const uint32_t row = order[at];
     if (row < row_begin || row >= row_end) return;
-    uint64_t first = at < kBoundWindow / 2 ? 0 : at - kBoundWindow / 2;
-    if (first + kBoundWindow > n) first = n > kBoundWindow ? n - kBoundWindow : 0;
-    uint32_t dist[kBoundWindow / 32];
+    uint32_t* seen = seen_sm[warp];
+    for (uint32_t i = lane; i < kSeenSlots / 4; i += 32) reinterpret_cast<uint4*>(seen)[i] = make_uint4(kFull, kFull, kFull, kFull);
+    const uint32_t where = lane < kBoundOrders ? place[uint64_t(row) * kBoundOrders + lane] : 0u;
+    uint32_t id[N], dist[N];
+    uint4 own[QUADS];
 #pragma unroll
-    for (int s = 0; s < kBoundWindow / 32; ++s) {
-        const uint64_t p = first + s * 32 + lane;
-        const uint32_t id = p < n ? ord[p] : row;
-        dist[s] = id != row ? exact_distance<U16>(codes, quads, row, id) : kFull;
+    for (int w = 0; w < QUADS; ++w) own[w] = __ldg(codes + size_t(row) * QUADS + w);
+#pragma unroll
+    for (int o = 0; o < kBoundOrders; ++o) {
+        const uint64_t pos = __shfl_sync(kFull, where, o);
+        uint64_t first = pos < kBoundWindow / 2 ? 0 : pos - kBoundWindow / 2;
+        if (first + kBoundWindow > n) first = n > kBoundWindow ? n - kBoundWindow : 0;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {
+            const uint64_t p = first + s * 32 + lane;
+            id[o * S + s] = p < n ? __ldg(order + size_t(o) * n + p) : row;
+        }
     }
-    const uint32_t T = kth_distance(dist, k, K);  // (K when the window holds fewer than k others)
-    if (lane == 0) atomicMin(bound + row, T);
+#pragma unroll
+    for (int i = 0; i < N; ++i) dist[i] = id[i] != row ? code_distance<U16, QUADS>(own, codes + size_t(id[i]) * QUADS) : kFull;
+    // enough of the closest, repeats included, to hold k different rows in most cases; half the table at most
+    const uint32_t reach = kth_distance(dist, kSeenSlots / 2 < 4 * k ? kSeenSlots / 2 : 4 * k, K);
+    uint32_t upto = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) upto += dist[i] <= reach;
+    const bool all = __reduce_add_sync(kFull, upto) <= kSeenSlots * 3 / 4;  // else the farthest of them would crowd the table
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (dist[i] < reach + (all ? 1u : 0u)) {
+            uint32_t slot = (id[i] * 0x9E3779B1u) >> 22;
+            while (true) {
+                const uint32_t was = atomicCAS(seen + slot, kFull, id[i]);
+                if (was == kFull) break;
+                if (was == id[i]) {
+                    dist[i] = kFull;  // a repeat
+                    break;
+                }
+                slot = (slot + 1) & (kSeenSlots - 1);
+            }
+        } else {
+            dist[i] = kFull;
+        }
+    }
+    const uint32_t T = kth_distance(dist, k, K);  // (K when fewer than k were found)
+    if (lane == 0) bound[row] = T;
 }
 
 // ---- tcgen05 pieces ------------------------------------------------------------------------------------------------
@@ -266,7 +315,7 @@ struct Split {
 struct KnnMmaArgs {
     const uint4* operand;  // [tiles][chunks][256]
     const uint4* codes;    // padded rows
-    int quads;             // 16-byte words of a padded row
+    int code_stages;       // candidate tiles whose codes are held in shared memory
     int K, symbols, chunks;
     uint64_t n;
     uint32_t k;
@@ -333,19 +382,22 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
     return T;
 }
 
-template <bool U16>
+template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     extern __shared__ __align__(1024) unsigned char mma_smem[];
     __shared__ __align__(8) uint64_t full_bar[2], empty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
-    __shared__ uint2 queue[kEpiWarps][kQueue];      // {candidate, lane of the row}
-    __shared__ int limit[2][2][kMmaRows];           // [segment parity][side][row]: largest distance still of use
+    __shared__ __align__(8) uint64_t cfull_bar[kMaxCodeStages], cempty_bar[kMaxCodeStages];
+    __shared__ uint16_t queue[kEpiWarps][64];       // pairs a warp has collected: column | lane of the row << 7
     __shared__ uint32_t filled[2][kMmaRows];        // [side][row]: entries of the buffer
+    __shared__ int limit[2][2][kMmaRows];           // [segment parity][side][row]: largest distance still of use
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t operand_bytes = uint32_t(a.chunks) * kMmaRows * 16;
     unsigned char* a_sm = mma_smem;
-    unsigned char* b_sm = mma_smem + operand_bytes;  // two stages
+    unsigned char* b_sm = mma_smem + operand_bytes;      // two stages
+    unsigned char* c_sm = mma_smem + 3 * operand_bytes;  // the candidates' codes, code_stages of them
+    constexpr uint32_t kCodeBytes = kMmaRows * QUADS * 16;
     const uint64_t s0 = a.split.first_step(blockIdx.x);
     const uint32_t steps = uint32_t(a.split.first_step(blockIdx.x + 1) - s0);
     const uint32_t rt0 = uint32_t(s0 / a.split.cts), ct0 = uint32_t(s0 % a.split.cts);  // first row and candidate tile
@@ -356,6 +408,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
             knn::mbar_init(&empty_bar[i], 1);
             knn::mbar_init(&tfull_bar[i], 1);
             knn::mbar_init(&tempty_bar[i], kEpiWarps / 2);
+        }
+        for (int i = 0; i < kMaxCodeStages; ++i) {
+            knn::mbar_init(&cfull_bar[i], 1);
+            knn::mbar_init(&cempty_bar[i], kEpiWarps);
         }
         knn::mbar_init(&drain_bar, 1);
         abort_flag = 0;
@@ -376,15 +432,21 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         if (lane == 0) {
             uint32_t rt = rt0, ct = ct0;
             bool fresh = true;  // the row tile's own operand has to come too
+            uint32_t cs = 0, cparity = 1;
             for (uint32_t i = 0; i < steps && !*aborted; ++i) {
                 const uint32_t s = i & 1;
                 bool ok = wait_or_abort(&empty_bar[s], ((i >> 1) & 1) ^ 1, kWaitLimit, aborted);
                 // it replaces the one that the step before still reads
                 if (ok && fresh && i) ok = wait_or_abort(&empty_bar[s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted);
+                if (ok) ok = wait_or_abort(&cempty_bar[cs], cparity, kWaitLimit, aborted);
                 if (!ok) {
                     *aborted = 1;
                     break;
                 }
+                const uint32_t code_rows = uint32_t(a.n - uint64_t(ct) * kMmaRows < kMmaRows ? a.n - uint64_t(ct) * kMmaRows : kMmaRows);
+                knn::mbar_expect_tx(&cfull_bar[cs], code_rows * QUADS * 16);
+                knn::bulk_g2s(c_sm + cs * kCodeBytes, a.codes + size_t(ct) * kMmaRows * QUADS, code_rows * QUADS * 16, &cfull_bar[cs]);
+                if (++cs == uint32_t(a.code_stages)) cs = 0, cparity ^= 1;
                 knn::mbar_expect_tx(&full_bar[s], fresh ? 2 * operand_bytes : operand_bytes);
                 const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
                 if (fresh) knn::bulk_g2s(a_sm, op + size_t(a.tile0 + rt) * operand_bytes, operand_bytes, &full_bar[s]);
@@ -421,10 +483,11 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
         const uint32_t base = uint32_t(half * 128 + quarter * 32), local = base + lane;  // rows of the warp, of the lane
         const uint32_t n = uint32_t(a.n);
-        const uint32_t below = (1u << lane) - 1u;
         const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256 + side * 128;
-        uint2* mine = queue[warp];
-        uint32_t rt = rt0, ct = ct0, queued = 0, parity = 0;
+        uint32_t rt = rt0, ct = ct0, parity = 0, cs = 0, cparity = 0;
+        const uint32_t below = (1u << lane) - 1u;
+        uint16_t* mine = queue[warp];
+        uint4 own[QUADS];    // the code of the lane's row
         bool ok = true, fresh = true;
         for (uint32_t i = 0; i < steps; ++i) {
             const uint32_t row0 = (a.tile0 + rt) * kMmaRows + base;  // the warp's first row
@@ -434,25 +497,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                 const bool wanted = row >= a.row_begin && row < a.row_end;
                 limit[parity][side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
                 filled[side][local] = 0;
+#pragma unroll
+                for (int w = 0; w < QUADS; ++w) own[w] = wanted ? __ldg(a.codes + size_t(row) * QUADS + w) : make_uint4(0u, 0u, 0u, 0u);
                 __syncwarp();
             }
-            // distances of the last `m` queued pairs; those of use go to their row's buffer
-            auto drain = [&](uint32_t m) {
-                __syncwarp();
-                queued -= m;
-                if (uint32_t(lane) < m) {
-                    const uint2 e = mine[queued + lane];
-                    const uint32_t row = row0 + e.y;
-                    const int d = int(exact_distance<U16>(a.codes, a.quads, row, e.x));
-                    if (e.x != row && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + e.y])) {
-                        const uint32_t at = atomicAdd(&filled[side][base + e.y], 1u);
-                        const size_t to = buf0 + size_t(e.y) * (2 * kMmaCap) + at;
-                        a.ids[to] = e.x;
-                        a.dists[to] = uint8_t(d);
-                    }
-                }
-                __syncwarp();
-            };
             ok = wait_or_abort(&tfull_bar[half], i & 1, kWaitLimit, aborted);
             if (__ballot_sync(kFull, !ok || *aborted)) {
                 ok = false;
@@ -478,47 +526,86 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
             __syncwarp();
             if (lane == 0) mbar_arrive(&tempty_bar[half]);
 
+            // their exact distances, 32 pairs at a time, a lane each
+            ok = wait_or_abort(&cfull_bar[cs], cparity, kWaitLimit, aborted);
+            if (__ballot_sync(kFull, !ok)) {
+                ok = false;
+                break;
+            }
+            const uint4* cand = reinterpret_cast<const uint4*>(c_sm + cs * kCodeBytes) + side * 128 * QUADS;
             const uint32_t col0 = ct * kMmaRows + side * 128;
+            if (col0 + 128 > n) {  // columns past the last node
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                uint32_t any;
-                while ((any = __ballot_sync(kFull, pass[c] != 0)) != 0) {
-                    const uint32_t b = __ffs(pass[c]) - 1;  // (of an empty word: not used)
-                    const uint32_t col = col0 + c * 32 + 2 * (b & 15) + (b >> 4);
-                    bool take = pass[c] != 0 && col < n;
-                    pass[c] &= pass[c] - 1;
-                    const uint32_t m = __ballot_sync(kFull, take);
-                    if (take) mine[queued + __popc(m & below)] = make_uint2(col, uint32_t(lane));
-                    queued += __popc(m);
-                    if (queued >= 32) drain(32);
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t first = col0 + c * 32, have = first >= n ? 0u : (n - first < 32 ? n - first : 32u);
+                    const uint32_t even = (1u << ((have + 1) / 2)) - 1u, odd = (1u << (have / 2)) - 1u;
+                    pass[c] &= even | odd << 16;
                 }
             }
-            // a row whose buffer could overflow in the next tile
-            uint32_t full = __ballot_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&filled[side][local]) > kMmaKeep);
-            const bool last_of_segment = ct + 1 == a.split.cts || i + 1 == steps;
-            if (full || last_of_segment) {
-                drain(queued);
-                full = __ballot_sync(kFull, *reinterpret_cast<volatile uint32_t*>(&filled[side][local]) > kMmaKeep);
-                while (full) {
-                    const int src = __ffs(full) - 1;
-                    full &= full - 1;
-                    uint32_t count = filled[side][base + src];
-                    const size_t b = buf0 + size_t(src) * (2 * kMmaCap);
-                    const uint32_t T = compact_row(a.ids + b, a.dists + b, count, a.k, a.K, lane);
-                    if (lane == 0) {
-                        filled[side][base + src] = count;
-                        // this side's later candidates have higher ids and must be strictly closer
-                        atomicMin(&limit[parity][side][base + src], int(T) - 1);
-                        atomicMin(&limit[parity][side ^ 1][base + src], int(T));
-                    }
-                    __syncwarp();
+            uint32_t queued = 0;
+            auto drain = [&](uint32_t m) {
+                __syncwarp();
+                queued -= m;
+                const bool act = uint32_t(lane) < m;
+                const uint32_t e = act ? mine[queued + lane] : 0u;
+                const uint32_t col = e & 127u, src = e >> 7;
+                uint4 theirs[QUADS];
+#pragma unroll
+                for (int w = 0; w < QUADS; ++w) {
+                    theirs[w].x = __shfl_sync(kFull, own[w].x, src);
+                    theirs[w].y = __shfl_sync(kFull, own[w].y, src);
+                    theirs[w].z = __shfl_sync(kFull, own[w].z, src);
+                    theirs[w].w = __shfl_sync(kFull, own[w].w, src);
                 }
+                const int d = int(code_distance<U16, QUADS>(theirs, cand + col * QUADS));
+                const uint32_t id = col0 + col;
+                if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + src])) {
+                    const size_t to = buf0 + size_t(src) * (2 * kMmaCap) + atomicAdd(&filled[side][base + src], 1u);
+                    a.ids[to] = id;
+                    a.dists[to] = uint8_t(d);
+                }
+                __syncwarp();
+            };
+            // a lane's next pair: the lowest bit of its first word that has any (the lanes stay together)
+            while (true) {
+                const uint32_t word = pass[0] ? pass[0] : (pass[1] ? pass[1] : (pass[2] ? pass[2] : pass[3]));
+                const uint32_t any = __ballot_sync(kFull, word != 0);
+                if (any == 0) break;
+                const uint32_t c = pass[0] ? 0u : (pass[1] ? 32u : (pass[2] ? 64u : 96u));
+                const uint32_t b = __ffs(word) - 1, rest = word & (word - 1);
+                if (word) mine[queued + __popc(any & below)] = uint16_t(c + 2 * (b & 15) + (b >> 4) + (lane << 7));
+                pass[0] = c == 0 ? rest : pass[0];
+                pass[1] = c == 32 ? rest : pass[1];
+                pass[2] = c == 64 ? rest : pass[2];
+                pass[3] = c == 96 ? rest : pass[3];
+                queued += __popc(any);
+                if (queued >= 32) drain(32);
             }
-            fresh = last_of_segment;
+            if (queued) drain(queued);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&cempty_bar[cs]);
+            if (++cs == uint32_t(a.code_stages)) cs = 0, cparity ^= 1;
+
+            // rows whose buffer could overflow in the next tile
+            uint32_t full = __ballot_sync(kFull, filled[side][local] > kMmaKeep);
+            while (full) {
+                const int src = __ffs(full) - 1;
+                full &= full - 1;
+                uint32_t count = filled[side][base + src];
+                const size_t at = buf0 + size_t(src) * (2 * kMmaCap);
+                const uint32_t T = compact_row(a.ids + at, a.dists + at, count, a.k, a.K, lane);
+                if (lane == 0) {
+                    filled[side][base + src] = count;
+                    // this side's later candidates have higher ids and must be strictly closer
+                    atomicMin(&limit[parity][side][base + src], int(T) - 1);
+                    atomicMin(&limit[parity][side ^ 1][base + src], int(T));
+                }
+                __syncwarp();
+            }
+            fresh = ct + 1 == a.split.cts || i + 1 == steps;
             if (fresh) {
                 a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = filled[side][local];
-                // the row's other warp may be a tile behind and still lower the old limits
-                parity ^= 1;
+                parity ^= 1;  // the row's other warp may be a tile behind and still lower the old limits
             }
             if (++ct == a.split.cts) ct = 0, ++rt;
         }
@@ -529,6 +616,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     if (warp == kEpiWarps && lane == 0 && *aborted) {
         atomicExch(a.status, kStatusWaitTimeout);
         for (uint32_t i = loads > 2 ? loads - 2 : 0; i < loads; ++i) mbar_wait_bounded(&full_bar[i & 1], (i >> 1) & 1, kWaitLimit);
+        const uint32_t stages = uint32_t(a.code_stages);
+        for (uint32_t i = loads > stages ? loads - stages : 0; i < loads; ++i)
+            mbar_wait_bounded(&cfull_bar[i % stages], (i / stages) & 1, kWaitLimit);
     }
     if (warp == kEpiWarps + 1) {
         if (lane == 0) mbar_wait_bounded(&drain_bar, 0, kWaitLimit);
@@ -637,8 +727,8 @@ __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArg
     }
 }
 
-template <typename CompT>
-int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k, uint64_t row_begin,
+template <typename CompT, int QUADS>
+int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, uint64_t n, uint32_t k, uint64_t row_begin,
                  uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
     constexpr bool U16 = sizeof(CompT) == 2;
     const CompT* codes = static_cast<const CompT*>(d_codes);
@@ -646,18 +736,18 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const uint64_t tiles = (n + kMmaRows - 1) / kMmaRows;
     const size_t operand_bytes = size_t(shape.chunks) * kMmaRows * 16;
     const uint64_t sms = uint64_t(h->sm_count);
-    // row tiles go in launches of whole waves (the buffers of a segment take 720 KB) and a last one that splits the rest
-    constexpr uint64_t kWaves = 4;
+    // row tiles go in launches of whole waves (the buffers of a segment take 960 KB) and a last one that splits the rest
+    constexpr uint64_t kWaves = 2;
     const uint64_t first_tile = row_begin / kMmaRows, end_tile = (row_end - 1) / kMmaRows + 1;
     const uint64_t most = end_tile - first_tile < kWaves * sms ? end_tile - first_tile : kWaves * sms;
     const size_t segments = size_t(most + sms);
 
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t op_b = up(size_t(tiles) * operand_bytes), hist_b = up(size_t(kBoundOrders) * kKeys * 4);
-    const size_t order_b = up(size_t(kBoundOrders) * n * 4), bound_b = up(size_t(n) * 4);
+    const size_t order_b = up(size_t(kBoundOrders) * n * 4), place_b = order_b, bound_b = up(size_t(n) * 4);
     const size_t slots = segments * kMmaRows * 2;
     const size_t ids_b = up(slots * kMmaCap * 4), dists_b = up(slots * kMmaCap), counts_b = up(slots * 4);
-    CPB_TRY(h->s_sliced.reserve(op_b + hist_b + order_b + bound_b + ids_b + dists_b + counts_b));
+    CPB_TRY(h->s_sliced.reserve(op_b + hist_b + order_b + place_b + bound_b + ids_b + dists_b + counts_b));
     unsigned char* p = h->s_sliced.as<unsigned char>();
     auto take = [&](size_t b) {
         unsigned char* r = p;
@@ -667,12 +757,14 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     uint4* operand = reinterpret_cast<uint4*>(take(op_b));
     uint32_t* hist = reinterpret_cast<uint32_t*>(take(hist_b));
     uint32_t* order = reinterpret_cast<uint32_t*>(take(order_b));
+    uint32_t* place = reinterpret_cast<uint32_t*>(take(place_b));
     uint32_t* bound = reinterpret_cast<uint32_t*>(take(bound_b));
 
     KnnMmaArgs a;
     a.operand = operand;
     a.codes = reinterpret_cast<const uint4*>(padded);
-    a.quads = words / 4;
+    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, room = 210 * 1024 - 3 * operand_bytes;
+    a.code_stages = int(room / code_bytes < size_t(kMaxCodeStages) ? room / code_bytes : size_t(kMaxCodeStages));
     a.K = int(h->K);
     a.symbols = shape.symbols;
     a.chunks = shape.chunks;
@@ -691,16 +783,15 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const uint64_t cells = tiles * shape.chunks * kMmaRows;
     expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(codes, n, int(h->K), shape.symbols, shape.chunks, operand, tiles);
     CPB_CUDA(cudaMemsetAsync(hist, 0, size_t(kBoundOrders) * kKeys * 4, st));
-    CPB_CUDA(cudaMemsetAsync(bound, 0xff, size_t(n) * 4, st));
     const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
     key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
     key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
-    key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order);
-    bound_kernel<U16><<<dim3(unsigned((n + 7) / 8), kBoundOrders), 256, 0, st>>>(a.codes, a.quads, a.K, n, order, k, a.row_begin, a.row_end,
-                                                                               bound);
+    key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order, place);
+    bound_kernel<U16, QUADS><<<unsigned((n + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(a.codes, a.K, n, order, place, k,
+                                                                                                       a.row_begin, a.row_end, bound);
     h->launches += 5;
     CPB_CUDA(cudaGetLastError());
-    CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16>));
+    CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS>));
     for (uint64_t t0 = first_tile; t0 < end_tile;) {
         const uint64_t left = end_tile - t0;
         const uint64_t rts = left >= kWaves * sms ? kWaves * sms : (left >= sms ? left / sms * sms : left);
@@ -708,7 +799,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         a.split.cts = uint32_t(tiles);
         a.split.steps = rts * tiles;
         a.split.blocks = uint32_t(a.split.steps < sms ? a.split.steps : sms);
-        knn_mma_kernel<U16><<<a.split.blocks, kMmaThreads, 3 * operand_bytes, st>>>(a);
+        knn_mma_kernel<U16, QUADS><<<a.split.blocks, kMmaThreads, 3 * operand_bytes + a.code_stages * code_bytes, st>>>(a);
         const uint32_t rows = uint32_t(rts) * kMmaRows;
         knn_finish_kernel<<<(rows + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, rows, d_nbrs, d_dist, uint32_t(row_begin));
         h->launches += 2;
@@ -727,8 +818,15 @@ bool knn_mma_supported(const cphnsw_b200_index* h) {
 
 int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,
                          uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
-    if (h->comp_bytes == 2) return launch_mma_t<uint16_t>(h, d_codes, padded, words, n, k, row_begin, row_end, d_nbrs, d_dist, st);
-    return launch_mma_t<uint8_t>(h, d_codes, padded, words, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+#define CPB_MMA(T, Q) return launch_mma_t<T, Q>(h, d_codes, padded, n, k, row_begin, row_end, d_nbrs, d_dist, st)
+    const bool u16 = h->comp_bytes == 2;
+    switch (words) {
+        case 4: if (u16) CPB_MMA(uint16_t, 1); CPB_MMA(uint8_t, 1);
+        case 8: if (u16) CPB_MMA(uint16_t, 2); CPB_MMA(uint8_t, 2);
+        case 16: if (u16) CPB_MMA(uint16_t, 4); CPB_MMA(uint8_t, 4);
+        default: if (u16) CPB_MMA(uint16_t, 8); CPB_MMA(uint8_t, 8);
+    }
+#undef CPB_MMA
 }
 
 }  // namespace cpb
