@@ -612,7 +612,7 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
         return CPHNSW_B200_E_UNSUPPORTED;
     }
     if (h->knn_kernel == 3 && !knn_mma_supported(h)) {
-        set_error("knn_kernel=3 (tensor-core filter) needs plain codes of 2 to 74 components");
+        set_error("knn_kernel=3 (tensor-core filter) needs plain codes of 2 to 64 components");
         return CPHNSW_B200_E_UNSUPPORTED;
     }
     // (rows of whole 16-byte words are read in place and have to be aligned then)

@@ -18,10 +18,11 @@
 //
 // Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the candidates
 // in tiles of 256, two stages of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
-// halves of tensor memory; while one half is computed the eight epilogue warps of the other read it.  The operand is laid
-// out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a tile is one
-// contiguous copy and no tensor map is needed.  Blocks that take whole rows of tiles sweep them in step, so that a tile
-// comes from L2; only the rows left over by the last full wave are split between blocks along the candidates.
+// halves of tensor memory; while one half is computed the other is read.  A row has two epilogue threads, which take the
+// tiles in turn (a buffer and a limit each): one reads a tile while the other still deals with the pairs of the one before.
+// The operand is laid out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a
+// tile is one contiguous copy and no tensor map is needed.  Blocks that take whole rows of tiles sweep them in step, so
+// that a tile comes from L2; only the rows left over by the last full wave are split between blocks along the candidates.
 #include <cuda_fp16.h>
 
 #include "knn_common.cuh"
@@ -35,13 +36,14 @@ using knn::mbar_wait_bounded;
 using knn::smem_u32;
 
 constexpr int kMmaRows = 256;             // rows per block and candidates per tile
-constexpr int kMmaCap = 384;              // entries of a buffer: at most 256 before a tile and 128 from it
+constexpr int kMmaCap = 384;              // entries of a buffer: at most 128 before a tile and 256 from it
 constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
-constexpr uint32_t kMmaKeep = 256;
-constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, a half of the columns
-constexpr int kMmaThreads = (kEpiWarps + 2) * 32;  // and one that copies, one that issues the products
+constexpr uint32_t kMmaKeep = 128;
+constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, every second tile
+constexpr int kMmaThreads = (kEpiWarps + 3) * 32;  // and one each for the operands' copies, the products, the codes' copies
 constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxCodeStages = 4;
+constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 9 KB of static
 constexpr int kBoundOrders = 8;           // orders of likely neighbours
 constexpr int kBoundWindow = 128;         // rows looked at per order
 constexpr uint32_t kKeys = 65536;
@@ -52,7 +54,7 @@ struct HashShape {
 };
 __host__ __device__ inline HashShape hash_shape(int K) {
     HashShape s;
-    s.symbols = K <= 32 ? 8 : (K <= 74 ? 4 : 0);
+    s.symbols = K <= 32 ? 8 : (K <= 64 ? 4 : 0);
     const int values = K * (s.symbols - 1);
     s.chunks = (values + 31) / 32 * 2;
     return s;
@@ -91,14 +93,14 @@ __global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n,
 // ---- exact distance: differing bytes / halfwords of two padded rows -------------------------------------------------
 // a flag in the top bit of every differing byte (halfword), the flags of 8 (16) words packed for one popcount
 template <bool U16, int QUADS>
-__device__ __forceinline__ uint32_t code_distance(const uint4 (&a)[QUADS], const uint4* b) {
+__device__ __forceinline__ uint32_t code_distance(const uint4* a, const uint4* b) {
     constexpr uint32_t LO = U16 ? 0x7fff7fffu : 0x7f7f7f7fu;
     constexpr int G = U16 ? 16 : 8;
     uint32_t d = 0, acc = 0;
 #pragma unroll
     for (int i = 0; i < QUADS; ++i) {
-        const uint4 y = b[i];
-        const uint32_t v[4] = {a[i].x ^ y.x, a[i].y ^ y.y, a[i].z ^ y.z, a[i].w ^ y.w};
+        const uint4 x = a[i], y = b[i];
+        const uint32_t v[4] = {x.x ^ y.x, x.y ^ y.y, x.z ^ y.z, x.w ^ y.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int sh = (i * 4 + j) % G;
@@ -267,35 +269,48 @@ __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a, uint64_t b, 
         "l"(a), "l"(b), "r"(kIdesc), "r"(uint32_t(accumulate))
         : "memory");
 }
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// 32 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
-__device__ __forceinline__ void tmem_load32(uint32_t (&r)[16], uint32_t addr) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(addr)
-        : "memory");
+// 16 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
+__device__ __forceinline__ void tmem_load16(uint32_t (&r)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(addr)
+                 : "memory");
 }
 // (the registers are operands so that no use of them moves in front of the wait)
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
-                   "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                  :
                  : "memory");
 }
-// A bounded wait that also ends when another role of the block has given up.
+// A bounded wait that also ends when another role of the block has given up.  A poll may sleep for a microsecond: warps
+// that spin take the issue slots of those that work.
+__device__ __forceinline__ bool mbar_try_wait_us(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* aborted) {
     for (uint32_t i = 0; i < limit; ++i) {
-        if (knn::mbar_try_wait(bar, parity)) return true;
-        if ((i & 63) == 63 && *aborted) return false;
+        if (mbar_try_wait_us(bar, parity)) return true;
+        if ((i & 15) == 15 && *aborted) return false;
     }
     return false;
 }
@@ -338,11 +353,10 @@ __device__ __forceinline__ __half2 dot_of_distance(int symbols, int K, int t) {
 // The row's buffer shrinks to its k best (or all that are no worse than the k-th, up to kMmaKeep).  By the whole warp;
 // returns the k-th distance and the new count.
 __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, uint32_t& count, uint32_t k, int K, int lane) {
-    uint32_t id[kMmaSlots], dist[kMmaSlots];
+    uint32_t dist[kMmaSlots];
 #pragma unroll
     for (int s = 0; s < kMmaSlots; ++s) {
         const uint32_t e = uint32_t(s * 32 + lane);
-        id[s] = e < count ? ids[e] : kInvalidNode;
         dist[s] = e < count ? dists[e] : kFull;
     }
     const uint32_t T = kth_distance(dist, k, K);
@@ -357,8 +371,8 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
         while (lo < hi) {
             const uint32_t mid = lo + ((hi - lo) >> 1);
             uint32_t c = 0;
-#pragma unroll
-            for (int s = 0; s < kMmaSlots; ++s) c += dist[s] == T && id[s] <= mid;
+#pragma unroll 1
+            for (uint32_t e = lane; e < count; e += 32) c += dists[e] == T && ids[e] <= mid;
             if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
             else lo = mid + 1;
         }
@@ -366,18 +380,19 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
     }
     __syncwarp();
     uint32_t at = 0;
-#pragma unroll
-    for (int s = 0; s < kMmaSlots; ++s) {
-        const bool keep = dist[s] < T || (dist[s] == T && id[s] <= last);
+#pragma unroll 1
+    for (uint32_t e = lane; e < (count + 31u) / 32 * 32; e += 32) {  // (an entry moves down or stays)
+        const uint32_t d = e < count ? dists[e] : kFull, id = e < count ? ids[e] : kInvalidNode;
+        const bool keep = d < T || (d == T && id <= last);
         const uint32_t m = __ballot_sync(kFull, keep);
         if (keep) {
             const uint32_t to = at + __popc(m & ((1u << lane) - 1u));
-            ids[to] = id[s];
-            dists[to] = uint8_t(dist[s]);
+            ids[to] = id;
+            dists[to] = uint8_t(d);
         }
         at += __popc(m);
+        __syncwarp();
     }
-    __syncwarp();
     count = at;
     return T;
 }
@@ -385,33 +400,38 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
 template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     extern __shared__ __align__(1024) unsigned char mma_smem[];
-    __shared__ __align__(8) uint64_t full_bar[2], empty_bar[2], tfull_bar[2], tempty_bar[2], drain_bar;
-    __shared__ __align__(8) uint64_t cfull_bar[kMaxCodeStages], cempty_bar[kMaxCodeStages];
-    __shared__ uint16_t queue[kEpiWarps][64];       // pairs a warp has collected: column | lane of the row << 7
+    __shared__ __align__(8) uint64_t full_bar[2][2], empty_bar[2][2];    // [stage][part of K]
+    __shared__ __align__(8) uint64_t tfull_bar[2][2], tempty_bar[2][2];  // [half of the rows][side]
+    __shared__ __align__(8) uint64_t cfull_bar[kMaxCodeStages], cempty_bar[kMaxCodeStages], drain_bar;
+    __shared__ uint16_t queue[kEpiWarps][64];       // pairs a warp has collected: column | lane of the row << 8
     __shared__ uint32_t filled[2][kMmaRows];        // [side][row]: entries of the buffer
     __shared__ int limit[2][2][kMmaRows];           // [segment parity][side][row]: largest distance still of use
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
     const uint32_t operand_bytes = uint32_t(a.chunks) * kMmaRows * 16;
+    const int ksteps = a.chunks / 2, split_k = (ksteps + 1) / 2;  // 32 values of K a step: two 16-byte chunks
     unsigned char* a_sm = mma_smem;
     unsigned char* b_sm = mma_smem + operand_bytes;      // two stages
     unsigned char* c_sm = mma_smem + 3 * operand_bytes;  // the candidates' codes, code_stages of them
     constexpr uint32_t kCodeBytes = kMmaRows * QUADS * 16;
+    constexpr uint32_t kStepBytes = 2 * kMmaRows * 16;
+    constexpr bool kOwnInSmem = QUADS <= 2;  // the rows' own codes, once per side (wider codes: read from L2)
     const uint64_t s0 = a.split.first_step(blockIdx.x);
     const uint32_t steps = uint32_t(a.split.first_step(blockIdx.x + 1) - s0);
     const uint32_t rt0 = uint32_t(s0 / a.split.cts), ct0 = uint32_t(s0 % a.split.cts);  // first row and candidate tile
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
-            knn::mbar_init(&full_bar[i], 1);
-            knn::mbar_init(&empty_bar[i], 1);
-            knn::mbar_init(&tfull_bar[i], 1);
-            knn::mbar_init(&tempty_bar[i], kEpiWarps / 2);
-        }
+        for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < 2; ++j) {
+                knn::mbar_init(&full_bar[i][j], 1);
+                knn::mbar_init(&empty_bar[i][j], 1);
+                knn::mbar_init(&tfull_bar[i][j], 1);
+                knn::mbar_init(&tempty_bar[i][j], 4);
+            }
         for (int i = 0; i < kMaxCodeStages; ++i) {
             knn::mbar_init(&cfull_bar[i], 1);
-            knn::mbar_init(&cempty_bar[i], kEpiWarps);
+            knn::mbar_init(&cempty_bar[i], kEpiWarps / 2);
         }
         knn::mbar_init(&drain_bar, 1);
         abort_flag = 0;
@@ -427,185 +447,218 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     const uint32_t tmem = tmem_base_sm;
     volatile int* aborted = &abort_flag;
 
-    uint32_t loads = 0;  // steps whose copies were issued
+    uint32_t loads = 0;  // copies issued by this warp: parts of operands, or code tiles
     if (warp == kEpiWarps) {
         if (lane == 0) {
             uint32_t rt = rt0, ct = ct0;
-            bool fresh = true;  // the row tile's own operand has to come too
-            uint32_t cs = 0, cparity = 1;
-            for (uint32_t i = 0; i < steps && !*aborted; ++i) {
+            bool fresh = true, ok = true;  // fresh: the row tile's own operand has to come too
+            const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
+            for (uint32_t i = 0; i < steps && ok && !*aborted; ++i) {
                 const uint32_t s = i & 1;
-                bool ok = wait_or_abort(&empty_bar[s], ((i >> 1) & 1) ^ 1, kWaitLimit, aborted);
-                // it replaces the one that the step before still reads
-                if (ok && fresh && i) ok = wait_or_abort(&empty_bar[s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted);
-                if (ok) ok = wait_or_abort(&cempty_bar[cs], cparity, kWaitLimit, aborted);
-                if (!ok) {
-                    *aborted = 1;
-                    break;
+                // a new row operand replaces the one that the step before still reads
+                if (fresh && i) ok = wait_or_abort(&empty_bar[s ^ 1][1], ((i - 1) >> 1) & 1, kWaitLimit, aborted);
+                for (int part = 0; part < 2 && ok; ++part) {
+                    const uint32_t from = part ? split_k * kStepBytes : 0u;
+                    const uint32_t bytes = (part ? ksteps - split_k : split_k) * kStepBytes;
+                    ok = wait_or_abort(&empty_bar[s][part], ((i >> 1) & 1) ^ 1, kWaitLimit, aborted);
+                    if (!ok) break;
+                    const uint32_t own = fresh && part == 0 ? operand_bytes : 0u;
+                    knn::mbar_expect_tx(&full_bar[s][part], bytes + own);
+                    if (own) knn::bulk_g2s(a_sm, op + size_t(a.tile0 + rt) * operand_bytes, own, &full_bar[s][part]);
+                    if (bytes) knn::bulk_g2s(b_sm + s * operand_bytes + from, op + size_t(ct) * operand_bytes + from, bytes, &full_bar[s][part]);
+                    ++loads;
                 }
-                const uint32_t code_rows = uint32_t(a.n - uint64_t(ct) * kMmaRows < kMmaRows ? a.n - uint64_t(ct) * kMmaRows : kMmaRows);
-                knn::mbar_expect_tx(&cfull_bar[cs], code_rows * QUADS * 16);
-                knn::bulk_g2s(c_sm + cs * kCodeBytes, a.codes + size_t(ct) * kMmaRows * QUADS, code_rows * QUADS * 16, &cfull_bar[cs]);
-                if (++cs == uint32_t(a.code_stages)) cs = 0, cparity ^= 1;
-                knn::mbar_expect_tx(&full_bar[s], fresh ? 2 * operand_bytes : operand_bytes);
-                const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
-                if (fresh) knn::bulk_g2s(a_sm, op + size_t(a.tile0 + rt) * operand_bytes, operand_bytes, &full_bar[s]);
-                knn::bulk_g2s(b_sm + s * operand_bytes, op + size_t(ct) * operand_bytes, operand_bytes, &full_bar[s]);
-                ++loads;
                 fresh = ++ct == a.split.cts;
                 if (fresh) ct = 0, ++rt;
             }
+            if (!ok) *aborted = 1;
+        }
+    } else if (warp == kEpiWarps + 2) {
+        if (lane == 0) {
+            uint32_t ct = ct0, cs = 0, parity = 1;
+            for (uint32_t i = 0; i < steps && !*aborted; ++i) {
+                if (!wait_or_abort(&cempty_bar[cs], parity, kWaitLimit, aborted)) {
+                    *aborted = 1;
+                    break;
+                }
+                const uint64_t left = a.n - uint64_t(ct) * kMmaRows;
+                const uint32_t bytes = uint32_t(left < kMmaRows ? left : kMmaRows) * QUADS * 16;
+                knn::mbar_expect_tx(&cfull_bar[cs], bytes);
+                knn::bulk_g2s(c_sm + cs * kCodeBytes, a.codes + size_t(ct) * kMmaRows * QUADS, bytes, &cfull_bar[cs]);
+                ++loads;
+                if (++cs == uint32_t(a.code_stages)) cs = 0, parity ^= 1;
+                if (++ct == a.split.cts) ct = 0;
+            }
         }
     } else if (warp == kEpiWarps + 1) {
-        if (lane == 0) {
-            const uint64_t a_desc = operand_desc(smem_u32(a_sm));
-            const uint64_t b_desc[2] = {operand_desc(smem_u32(b_sm)), operand_desc(smem_u32(b_sm + operand_bytes))};
-            const int ksteps = a.chunks / 2;
-            bool ok = true;
-            for (uint32_t i = 0; i < steps && ok && !*aborted; ++i) {
-                const uint32_t s = i & 1;
-                ok = wait_or_abort(&full_bar[s], (i >> 1) & 1, i == 0 ? a.first_wait_polls : kWaitLimit, aborted);
-                for (int h = 0; h < 2 && ok; ++h) {
-                    ok = wait_or_abort(&tempty_bar[h], (i & 1) ^ 1, kWaitLimit, aborted);
-                    if (!ok) break;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int ks = 0; ks < ksteps; ++ks)  // 32 values of K a step: two 16-byte chunks
-                        mma_f8(tmem + h * 256, a_desc + uint64_t((h * 128 * 16 + ks * 2 * kMmaRows * 16) >> 4),
-                               b_desc[s] + uint64_t((ks * 2 * kMmaRows * 16) >> 4), ks != 0);
-                    mma_commit(&tfull_bar[h]);
+        // The whole warp goes along and one lane issues: descriptors then stay in uniform registers.  (One thread in a
+        // branch of its own took 270 cycles a product, twice what the product does.)
+        const uint32_t elected = elect_one();
+        const uint64_t a_desc = operand_desc(smem_u32(a_sm));
+        const uint64_t b_desc[2] = {operand_desc(smem_u32(b_sm)), operand_desc(smem_u32(b_sm + operand_bytes))};
+        constexpr uint64_t kStep = kStepBytes >> 4;
+        bool ok = true;
+        for (uint32_t i = 0; i < steps && ok; ++i) {
+            const uint32_t s = i & 1;
+            ok = __all_sync(kFull, wait_or_abort(&full_bar[s][0], (i >> 1) & 1, i == 0 ? a.first_wait_polls : kWaitLimit, aborted) && !*aborted);
+            for (int h = 0; h < 2 && ok; ++h) {
+                // the half was read for the step before by the other side
+                if (i) ok = __all_sync(kFull, wait_or_abort(&tempty_bar[h][s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted));
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d = tmem + h * 256;
+                uint64_t ad = a_desc + h * ((128 * 16) >> 4), bd = b_desc[s];
+                if (elected) {
+#pragma unroll 4
+                    for (int ks = 0; ks < split_k; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, ks != 0);
+                    if (h == 1) mma_commit(&empty_bar[s][0]);
                 }
-                if (ok) mma_commit(&empty_bar[s]);
+                if (h == 0) {
+                    ok = __all_sync(kFull, wait_or_abort(&full_bar[s][1], (i >> 1) & 1, kWaitLimit, aborted));
+                    if (!ok) break;
+                }
+                ad = a_desc + h * ((128 * 16) >> 4) + split_k * kStep, bd = b_desc[s] + split_k * kStep;
+                if (elected) {
+#pragma unroll 4
+                    for (int ks = split_k; ks < ksteps; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, true);
+                    mma_commit(&tfull_bar[h][s]);
+                    if (h == 1) mma_commit(&empty_bar[s][1]);
+                }
             }
-            if (!ok) *aborted = 1;
-            mma_commit(&drain_bar);  // everything issued above has finished when this completes
         }
+        if (!ok) *aborted = 1;
+        if (elected) mma_commit(&drain_bar);  // everything issued above has finished when this completes
     } else {
         const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
         const uint32_t base = uint32_t(half * 128 + quarter * 32), local = base + lane;  // rows of the warp, of the lane
         const uint32_t n = uint32_t(a.n);
-        const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256 + side * 128;
-        uint32_t rt = rt0, ct = ct0, parity = 0, cs = 0, cparity = 0;
         const uint32_t below = (1u << lane) - 1u;
+        const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256;
         uint16_t* mine = queue[warp];
-        uint4 own[QUADS];    // the code of the lane's row
-        bool ok = true, fresh = true;
+        uint4* own = reinterpret_cast<uint4*>(c_sm + size_t(a.code_stages) * kCodeBytes) + base * QUADS;  // the rows' codes
+        uint32_t rt = rt0, ct = ct0, parity = 0;
+        bool ok = true, begun = false;  // begun: this side has had a tile of the segment
         for (uint32_t i = 0; i < steps; ++i) {
             const uint32_t row0 = (a.tile0 + rt) * kMmaRows + base;  // the warp's first row
-            const size_t buf0 = ((size_t(blockIdx.x + rt) * kMmaRows + base) * 2 + side) * kMmaCap;  // and its buffer
-            if (fresh) {
-                const uint32_t row = row0 + lane;
-                const bool wanted = row >= a.row_begin && row < a.row_end;
-                limit[parity][side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
-                filled[side][local] = 0;
+            const bool last = ct + 1 == a.split.cts || i + 1 == steps;  // of the segment
+            if ((i & 1) == uint32_t(side)) {
+                const size_t buf0 = ((size_t(blockIdx.x + rt) * kMmaRows + base) * 2 + side) * kMmaCap;
+                ok = wait_or_abort(&tfull_bar[half][side], (i >> 1) & 1, kWaitLimit, aborted);
+                if (__ballot_sync(kFull, !ok || *aborted)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (!begun) {
+                    // (the row's other warp is past the segment before by now and lowers no limit of that parity any more)
+                    begun = true;
+                    const uint32_t row = row0 + lane;
+                    const bool wanted = row >= a.row_begin && row < a.row_end;
+                    limit[parity][side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
+                    filled[side][local] = 0;
+                    if (kOwnInSmem && wanted)
 #pragma unroll
-                for (int w = 0; w < QUADS; ++w) own[w] = wanted ? __ldg(a.codes + size_t(row) * QUADS + w) : make_uint4(0u, 0u, 0u, 0u);
+                        for (int w = 0; w < QUADS; ++w) own[side * kMmaRows * QUADS + lane * QUADS + w] = __ldg(a.codes + size_t(row) * QUADS + w);
+                    __syncwarp();
+                }
+                const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[parity][side][local]));
+                // pairs that pass, bit j of a word: column 2 j for j < 16, else column 2 (j - 16) + 1; one load is in flight
+                // while the columns of the one before are compared
+                uint32_t pass[8], r[2][8];
+                tmem_load16(r[0], addr);
+#pragma unroll
+                for (int c = 0; c < 16; ++c) {
+                    tmem_wait(r[c & 1]);
+                    if (c < 15) tmem_load16(r[(c + 1) & 1], addr + (c + 1) * 16);
+                    uint32_t m = c & 1 ? pass[c >> 1] : 0u;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        m |= __hge2_mask(*reinterpret_cast<const __half2*>(&r[c & 1][j]), thr) & (0x00010001u << (j + (c & 1) * 8));
+                    pass[c >> 1] = m;
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
-            }
-            ok = wait_or_abort(&tfull_bar[half], i & 1, kWaitLimit, aborted);
-            if (__ballot_sync(kFull, !ok || *aborted)) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[parity][side][local]));
-            // pairs that pass, bit j of a word: column 2 j for j < 16, else column 2 (j - 16) + 1; one load is in flight
-            // while the columns of the one before are compared
-            uint32_t pass[4], r[2][16];
-            tmem_load32(r[0], addr);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                tmem_wait(r[c & 1]);
-                if (c < 3) tmem_load32(r[(c + 1) & 1], addr + (c + 1) * 32);
-                uint32_t m = 0;
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    m |= __hge2_mask(*reinterpret_cast<const __half2*>(&r[c & 1][j]), thr) & (0x00010001u << j);
-                pass[c] = m;
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty_bar[half]);
+                if (lane == 0) mbar_arrive(&tempty_bar[half][side]);
 
-            // their exact distances, 32 pairs at a time, a lane each
-            ok = wait_or_abort(&cfull_bar[cs], cparity, kWaitLimit, aborted);
-            if (__ballot_sync(kFull, !ok)) {
-                ok = false;
-                break;
-            }
-            const uint4* cand = reinterpret_cast<const uint4*>(c_sm + cs * kCodeBytes) + side * 128 * QUADS;
-            const uint32_t col0 = ct * kMmaRows + side * 128;
-            if (col0 + 128 > n) {  // columns past the last node
+                // their exact distances, 32 pairs at a time, a lane each
+                const uint32_t cs = i % uint32_t(a.code_stages);
+                ok = wait_or_abort(&cfull_bar[cs], (i / uint32_t(a.code_stages)) & 1, kWaitLimit, aborted);
+                if (__ballot_sync(kFull, !ok)) {
+                    ok = false;
+                    break;
+                }
+                const uint4* cand = reinterpret_cast<const uint4*>(c_sm + cs * kCodeBytes);
+                const uint32_t col0 = ct * kMmaRows;
+                uint32_t queued = 0;
+                auto drain = [&](uint32_t m) {
+                    __syncwarp();
+                    queued -= m;
+                    const bool act = uint32_t(lane) < m;
+                    const uint32_t e = act ? mine[queued + lane] : 0u;
+                    const uint32_t col = e & 255u, src = e >> 8;
+                    const uint4* theirs = kOwnInSmem ? own + (side * kMmaRows + src) * QUADS : a.codes + size_t(min(row0 + src, n - 1)) * QUADS;
+                    const int d = int(code_distance<U16, QUADS>(theirs, cand + col * QUADS));
+                    const uint32_t id = col0 + col;
+                    if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + src])) {
+                        const size_t to = buf0 + size_t(src) * (2 * kMmaCap) + atomicAdd(&filled[side][base + src], 1u);
+                        a.ids[to] = id;
+                        a.dists[to] = uint8_t(d);
+                    }
+                    __syncwarp();
+                };
+                if (col0 + kMmaRows > n) {  // columns past the last node
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const uint32_t first = col0 + c * 32, have = first >= n ? 0u : (n - first < 32 ? n - first : 32u);
-                    const uint32_t even = (1u << ((have + 1) / 2)) - 1u, odd = (1u << (have / 2)) - 1u;
-                    pass[c] &= even | odd << 16;
+                    for (int c = 0; c < 8; ++c) {
+                        const uint32_t from = col0 + c * 32, have = from >= n ? 0u : (n - from < 32 ? n - from : 32u);
+                        pass[c] &= ((1u << ((have + 1) / 2)) - 1u) | ((1u << (have / 2)) - 1u) << 16;
+                    }
                 }
-            }
-            uint32_t queued = 0;
-            auto drain = [&](uint32_t m) {
-                __syncwarp();
-                queued -= m;
-                const bool act = uint32_t(lane) < m;
-                const uint32_t e = act ? mine[queued + lane] : 0u;
-                const uint32_t col = e & 127u, src = e >> 7;
-                uint4 theirs[QUADS];
+                uint32_t words = 0;  // the words that have a pair left, beside the current one
 #pragma unroll
-                for (int w = 0; w < QUADS; ++w) {
-                    theirs[w].x = __shfl_sync(kFull, own[w].x, src);
-                    theirs[w].y = __shfl_sync(kFull, own[w].y, src);
-                    theirs[w].z = __shfl_sync(kFull, own[w].z, src);
-                    theirs[w].w = __shfl_sync(kFull, own[w].w, src);
+                for (int c = 0; c < 8; ++c) words |= pass[c] ? 1u << c : 0u;
+                uint32_t word = 0, at = 0;
+                while (true) {
+                    if (word == 0 && words) {
+                        at = __ffs(words) - 1;
+                        words &= words - 1;
+                        const uint32_t w0 = at & 1 ? pass[1] : pass[0], w1 = at & 1 ? pass[3] : pass[2];
+                        const uint32_t w2 = at & 1 ? pass[5] : pass[4], w3 = at & 1 ? pass[7] : pass[6];
+                        const uint32_t lo = at & 2 ? w1 : w0, hi = at & 2 ? w3 : w2;
+                        word = at & 4 ? hi : lo;
+                    }
+                    const uint32_t any = __ballot_sync(kFull, word != 0);
+                    if (any == 0) break;
+                    const uint32_t b = __ffs(word) - 1;
+                    if (word) mine[queued + __popc(any & below)] = uint16_t(at * 32 + 2 * (b & 15) + (b >> 4) + (lane << 8));
+                    word &= word - 1;
+                    queued += __popc(any);
+                    if (queued >= 32) drain(32);
                 }
-                const int d = int(code_distance<U16, QUADS>(theirs, cand + col * QUADS));
-                const uint32_t id = col0 + col;
-                if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + src])) {
-                    const size_t to = buf0 + size_t(src) * (2 * kMmaCap) + atomicAdd(&filled[side][base + src], 1u);
-                    a.ids[to] = id;
-                    a.dists[to] = uint8_t(d);
-                }
+                if (queued) drain(queued);
                 __syncwarp();
-            };
-            // a lane's next pair: the lowest bit of its first word that has any (the lanes stay together)
-            while (true) {
-                const uint32_t word = pass[0] ? pass[0] : (pass[1] ? pass[1] : (pass[2] ? pass[2] : pass[3]));
-                const uint32_t any = __ballot_sync(kFull, word != 0);
-                if (any == 0) break;
-                const uint32_t c = pass[0] ? 0u : (pass[1] ? 32u : (pass[2] ? 64u : 96u));
-                const uint32_t b = __ffs(word) - 1, rest = word & (word - 1);
-                if (word) mine[queued + __popc(any & below)] = uint16_t(c + 2 * (b & 15) + (b >> 4) + (lane << 7));
-                pass[0] = c == 0 ? rest : pass[0];
-                pass[1] = c == 32 ? rest : pass[1];
-                pass[2] = c == 64 ? rest : pass[2];
-                pass[3] = c == 96 ? rest : pass[3];
-                queued += __popc(any);
-                if (queued >= 32) drain(32);
-            }
-            if (queued) drain(queued);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&cempty_bar[cs]);
-            if (++cs == uint32_t(a.code_stages)) cs = 0, cparity ^= 1;
+                if (lane == 0) mbar_arrive(&cempty_bar[cs]);
 
-            // rows whose buffer could overflow in the next tile
-            uint32_t full = __ballot_sync(kFull, filled[side][local] > kMmaKeep);
-            while (full) {
-                const int src = __ffs(full) - 1;
-                full &= full - 1;
-                uint32_t count = filled[side][base + src];
-                const size_t at = buf0 + size_t(src) * (2 * kMmaCap);
-                const uint32_t T = compact_row(a.ids + at, a.dists + at, count, a.k, a.K, lane);
-                if (lane == 0) {
-                    filled[side][base + src] = count;
-                    // this side's later candidates have higher ids and must be strictly closer
-                    atomicMin(&limit[parity][side][base + src], int(T) - 1);
-                    atomicMin(&limit[parity][side ^ 1][base + src], int(T));
+                // rows whose buffer could overflow in the next tile
+                uint32_t full = __ballot_sync(kFull, filled[side][local] > kMmaKeep);
+                while (full) {
+                    const int src = __ffs(full) - 1;
+                    full &= full - 1;
+                    uint32_t count = filled[side][base + src];
+                    const size_t at = buf0 + size_t(src) * (2 * kMmaCap);
+                    const uint32_t T = compact_row(a.ids + at, a.dists + at, count, a.k, a.K, lane);
+                    if (lane == 0) {
+                        filled[side][base + src] = count;
+                        // this side's later candidates have higher ids and must be strictly closer
+                        atomicMin(&limit[parity][side][base + src], int(T) - 1);
+                        atomicMin(&limit[parity][side ^ 1][base + src], int(T));
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
             }
-            fresh = ct + 1 == a.split.cts || i + 1 == steps;
-            if (fresh) {
-                a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = filled[side][local];
-                parity ^= 1;  // the row's other warp may be a tile behind and still lower the old limits
+            if (last) {
+                a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = begun ? filled[side][local] : 0u;
+                begun = false;
+                parity ^= 1;  // the row's other warp may still lower limits of the segment before
             }
             if (++ct == a.split.cts) ct = 0, ++rt;
         }
@@ -613,12 +666,14 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     }
     __syncthreads();
     // copies and products in flight after a lost wait end before the block's memory goes away
-    if (warp == kEpiWarps && lane == 0 && *aborted) {
-        atomicExch(a.status, kStatusWaitTimeout);
-        for (uint32_t i = loads > 2 ? loads - 2 : 0; i < loads; ++i) mbar_wait_bounded(&full_bar[i & 1], (i >> 1) & 1, kWaitLimit);
-        const uint32_t stages = uint32_t(a.code_stages);
-        for (uint32_t i = loads > stages ? loads - stages : 0; i < loads; ++i)
-            mbar_wait_bounded(&cfull_bar[i % stages], (i / stages) & 1, kWaitLimit);
+    if (*aborted && lane == 0) {
+        if (warp == kEpiWarps) {
+            atomicExch(a.status, kStatusWaitTimeout);
+            for (uint32_t l = loads > 4 ? loads - 4 : 0; l < loads; ++l) mbar_wait_bounded(&full_bar[(l >> 1) & 1][l & 1], (l >> 2) & 1, kWaitLimit);
+        } else if (warp == kEpiWarps + 2) {
+            const uint32_t stages = uint32_t(a.code_stages);
+            for (uint32_t l = loads > stages ? loads - stages : 0; l < loads; ++l) mbar_wait_bounded(&cfull_bar[l % stages], (l / stages) & 1, kWaitLimit);
+        }
     }
     if (warp == kEpiWarps + 1) {
         if (lane == 0) mbar_wait_bounded(&drain_bar, 0, kWaitLimit);
@@ -763,8 +818,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     KnnMmaArgs a;
     a.operand = operand;
     a.codes = reinterpret_cast<const uint4*>(padded);
-    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, room = 210 * 1024 - 3 * operand_bytes;
-    a.code_stages = int(room / code_bytes < size_t(kMaxCodeStages) ? room / code_bytes : size_t(kMaxCodeStages));
+    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, own_bytes = QUADS <= 2 ? 2 * code_bytes : 0;
+    a.code_stages = 3 * operand_bytes + 4 * code_bytes + own_bytes <= kMmaSmem ? 4 : 2;  // even: a stage serves one side
     a.K = int(h->K);
     a.symbols = shape.symbols;
     a.chunks = shape.chunks;
@@ -799,7 +854,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         a.split.cts = uint32_t(tiles);
         a.split.steps = rts * tiles;
         a.split.blocks = uint32_t(a.split.steps < sms ? a.split.steps : sms);
-        knn_mma_kernel<U16, QUADS><<<a.split.blocks, kMmaThreads, 3 * operand_bytes + a.code_stages * code_bytes, st>>>(a);
+        knn_mma_kernel<U16, QUADS><<<a.split.blocks, kMmaThreads, 3 * operand_bytes + a.code_stages * code_bytes + own_bytes, st>>>(a);
         const uint32_t rows = uint32_t(rts) * kMmaRows;
         knn_finish_kernel<<<(rows + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, rows, d_nbrs, d_dist, uint32_t(row_begin));
         h->launches += 2;
@@ -811,7 +866,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
 
 }  // namespace
 
-// Plain K-component codes of up to 74 components (the operand of 256 rows has to fit shared memory three times).
+// Plain K-component codes of up to 64 components (the operand of 256 rows has to fit shared memory three times).
 bool knn_mma_supported(const cphnsw_b200_index* h) {
     return !h->binary_codes && !h->residual_bits && h->K >= 2 && hash_shape(int(h->K)).symbols != 0;
 }

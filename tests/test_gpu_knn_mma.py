@@ -34,10 +34,10 @@ def check(idx, oracle, codes, k, rows=None):
     assert np.array_equal(nbrs, wn) and np.array_equal(dist, wd)
 
 
-# tiles are 256 rows by 256 candidates; 8 symbols up to K = 32, 4 up to K = 74
+# tiles are 256 rows by 256 candidates; 8 symbols up to K = 32, 4 up to K = 64
 @pytest.mark.parametrize("n,k,K,cb,dim", [(1, 4, 32, 1, 128), (255, 64, 32, 1, 128), (256, 127, 32, 1, 128), (257, 1, 16, 1, 100),
                                           (513, 40, 2, 1, 64), (3000, 64, 32, 1, 128), (2999, 32, 24, 1, 96), (2049, 64, 33, 1, 128),
-                                          (4100, 64, 64, 1, 128), (1500, 127, 74, 1, 128), (2300, 64, 32, 2, 960), (1200, 20, 64, 2, 300)])
+                                          (4100, 64, 64, 1, 128), (1500, 127, 61, 1, 128), (2300, 64, 32, 2, 960), (1200, 20, 64, 2, 300)])
 def test_shapes(cp, oracle, n, k, K, cb, dim):
     base, _ = synthetic.gaussian_mixture(n, 1, dim, max(1, n // 400), 0.3, n + K)
     codes = oracle.encode(base, K, cb, oracle.sign_tables(dim, K, 42))
