@@ -405,7 +405,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     __shared__ __align__(8) uint64_t cfull_bar[kMaxCodeStages], cempty_bar[kMaxCodeStages], drain_bar;
     __shared__ uint16_t queue[kEpiWarps][64];       // pairs a warp has collected: column | lane of the row << 8
     __shared__ uint32_t filled[2][kMmaRows];        // [side][row]: entries of the buffer
-    __shared__ int limit[2][2][kMmaRows];           // [segment parity][side][row]: largest distance still of use
+    __shared__ int limit[2][kMmaRows];              // [side][row]: largest distance still of use
+    __shared__ uint32_t finished[kEpiWarps];        // segments the epilogue warps are done with
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
     const int lane = threadIdx.x & 31, warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     unsigned char* c_sm = mma_smem + 3 * operand_bytes;  // the candidates' codes, code_stages of them
     constexpr uint32_t kCodeBytes = kMmaRows * QUADS * 16;
     constexpr uint32_t kStepBytes = 2 * kMmaRows * 16;
-    constexpr bool kOwnInSmem = QUADS <= 2;  // the rows' own codes, once per side (wider codes: read from L2)
+    constexpr bool kOwnInSmem = QUADS <= 4;  // the rows' own codes (wider ones: read from L2)
     const uint64_t s0 = a.split.first_step(blockIdx.x);
     const uint32_t steps = uint32_t(a.split.first_step(blockIdx.x + 1) - s0);
     const uint32_t rt0 = uint32_t(s0 / a.split.cts), ct0 = uint32_t(s0 % a.split.cts);  // first row and candidate tile
@@ -434,6 +435,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
             knn::mbar_init(&cempty_bar[i], kEpiWarps / 2);
         }
         knn::mbar_init(&drain_bar, 1);
+        for (int i = 0; i < kEpiWarps; ++i) finished[i] = 0;
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -536,7 +538,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256;
         uint16_t* mine = queue[warp];
         uint4* own = reinterpret_cast<uint4*>(c_sm + size_t(a.code_stages) * kCodeBytes) + base * QUADS;  // the rows' codes
-        uint32_t rt = rt0, ct = ct0, parity = 0;
+        uint32_t rt = rt0, ct = ct0, segment = 0;
         bool ok = true, begun = false;  // begun: this side has had a tile of the segment
         for (uint32_t i = 0; i < steps; ++i) {
             const uint32_t row0 = (a.tile0 + rt) * kMmaRows + base;  // the warp's first row
@@ -550,18 +552,21 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (!begun) {
-                    // (the row's other warp is past the segment before by now and lowers no limit of that parity any more)
+                    // the rows' other warp has to be done with the segment before, whose codes and limits are replaced
                     begun = true;
+                    for (uint32_t polls = 0; *reinterpret_cast<volatile uint32_t*>(&finished[warp ^ 8]) < segment && polls < kWaitLimit && !*aborted;)
+                        ++polls;
+                    __syncwarp();
                     const uint32_t row = row0 + lane;
                     const bool wanted = row >= a.row_begin && row < a.row_end;
-                    limit[parity][side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
+                    limit[side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
                     filled[side][local] = 0;
                     if (kOwnInSmem && wanted)
 #pragma unroll
-                        for (int w = 0; w < QUADS; ++w) own[side * kMmaRows * QUADS + lane * QUADS + w] = __ldg(a.codes + size_t(row) * QUADS + w);
+                        for (int w = 0; w < QUADS; ++w) own[lane * QUADS + w] = __ldg(a.codes + size_t(row) * QUADS + w);
                     __syncwarp();
                 }
-                const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[parity][side][local]));
+                const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[side][local]));
                 // pairs that pass, bit j of a word: column 2 j for j < 16, else column 2 (j - 16) + 1; one load is in flight
                 // while the columns of the one before are compared
                 uint32_t pass[8], r[2][8];
@@ -596,10 +601,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                     const bool act = uint32_t(lane) < m;
                     const uint32_t e = act ? mine[queued + lane] : 0u;
                     const uint32_t col = e & 255u, src = e >> 8;
-                    const uint4* theirs = kOwnInSmem ? own + (side * kMmaRows + src) * QUADS : a.codes + size_t(min(row0 + src, n - 1)) * QUADS;
+                    const uint4* theirs = kOwnInSmem ? own + src * QUADS : a.codes + size_t(min(row0 + src, n - 1)) * QUADS;
                     const int d = int(code_distance<U16, QUADS>(theirs, cand + col * QUADS));
                     const uint32_t id = col0 + col;
-                    if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[parity][side][base + src])) {
+                    if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[side][base + src])) {
                         const size_t to = buf0 + size_t(src) * (2 * kMmaCap) + atomicAdd(&filled[side][base + src], 1u);
                         a.ids[to] = id;
                         a.dists[to] = uint8_t(d);
@@ -649,8 +654,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                     if (lane == 0) {
                         filled[side][base + src] = count;
                         // this side's later candidates have higher ids and must be strictly closer
-                        atomicMin(&limit[parity][side][base + src], int(T) - 1);
-                        atomicMin(&limit[parity][side ^ 1][base + src], int(T));
+                        atomicMin(&limit[side][base + src], int(T) - 1);
+                        atomicMin(&limit[side ^ 1][base + src], int(T));
                     }
                     __syncwarp();
                 }
@@ -658,7 +663,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
             if (last) {
                 a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = begun ? filled[side][local] : 0u;
                 begun = false;
-                parity ^= 1;  // the row's other warp may still lower limits of the segment before
+                __syncwarp();
+                ++segment;
+                if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&finished[warp]) = segment;
             }
             if (++ct == a.split.cts) ct = 0, ++rt;
         }
@@ -818,7 +825,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     KnnMmaArgs a;
     a.operand = operand;
     a.codes = reinterpret_cast<const uint4*>(padded);
-    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, own_bytes = QUADS <= 2 ? 2 * code_bytes : 0;
+    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, own_bytes = QUADS <= 4 ? code_bytes : 0;
     a.code_stages = 3 * operand_bytes + 4 * code_bytes + own_bytes <= kMmaSmem ? 4 : 2;  // even: a stage serves one side
     a.K = int(h->K);
     a.symbols = shape.symbols;
