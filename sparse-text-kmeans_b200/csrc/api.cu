@@ -255,6 +255,22 @@ struct CtxLease {
     }
 };
 
+// Host-pointer calls with queries and results of up to this size go through page-locked memory: a copy from or to
+// pageable memory blocks for 10 us or more, and a call on one query had three of them.
+constexpr size_t kStagedBytes = 256 * 1024;
+
+// `bytes` of host input to the device buffer dst, through the context's staging area when small
+int copy_in(SearchCtx& cx, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    if (bytes > kStagedBytes) {
+        CPB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+        return 0;
+    }
+    CPB_TRY(cx.h_in.reserve(kStagedBytes));
+    std::memcpy(cx.h_in.p, src, bytes);
+    CPB_CUDA(cudaMemcpyAsync(dst, cx.h_in.p, bytes, cudaMemcpyHostToDevice, st));
+    return 0;
+}
+
 // scan_only: brute_force_search (every node scored, no walk); calibrated: distances mapped through the fit;
 // q_codes: the walk runs under the symmetric code distance to these query codes ([nq][K], same place as q).
 // `st` is the caller's stream for device-pointer calls and nullptr for host-pointer calls, which run on the
@@ -301,8 +317,7 @@ int do_search(cphnsw_b200_index* h, const float* q, bool q_on_device, uint64_t n
                 dqc = static_cast<const unsigned char*>(q_codes) + q0 * rb;
             } else {
                 CPB_TRY(cx.d_qcodes.reserve(m * rb + 16));
-                CPB_CUDA(cudaMemcpyAsync(cx.d_qcodes.p, static_cast<const unsigned char*>(q_codes) + q0 * rb, m * rb,
-                                         cudaMemcpyHostToDevice, st));
+                CPB_TRY(copy_in(cx, cx.d_qcodes.p, static_cast<const unsigned char*>(q_codes) + q0 * rb, m * rb, st));
                 dqc = cx.d_qcodes.p;
             }
         } else {
@@ -310,7 +325,7 @@ int do_search(cphnsw_b200_index* h, const float* q, bool q_on_device, uint64_t n
                 dq = q + q0 * h->dim;
             } else {
                 CPB_TRY(cx.d_q.reserve(m * h->dim * 4));
-                CPB_CUDA(cudaMemcpyAsync(cx.d_q.p, q + q0 * h->dim, m * h->dim * 4, cudaMemcpyHostToDevice, st));
+                CPB_TRY(copy_in(cx, cx.d_q.p, q + q0 * h->dim, m * h->dim * 4, st));
                 dq = cx.d_q.as<float>();
             }
             CPB_TRY(cx.d_qcodes.reserve(m * rb + 16));
@@ -325,7 +340,14 @@ int do_search(cphnsw_b200_index* h, const float* q, bool q_on_device, uint64_t n
         }
         uint32_t *o_ids, *o_stats = nullptr;
         float* o_d;
-        if (out_on_device) {
+        const size_t out_bytes = m * k * 8 + (stats ? m * 8 : 0);
+        const bool staged = !out_on_device && out_bytes <= kStagedBytes;
+        if (staged) {
+            CPB_TRY(cx.h_out.reserve(kStagedBytes));
+            o_ids = static_cast<uint32_t*>(cx.h_out.p);
+            o_d = reinterpret_cast<float*>(o_ids + m * k);
+            if (stats) o_stats = o_ids + 2 * m * k;
+        } else if (out_on_device) {
             o_ids = ids + q0 * k;
             o_d = dists + q0 * k;
             if (stats) o_stats = stats + q0 * 2;
@@ -342,7 +364,13 @@ int do_search(cphnsw_b200_index* h, const float* q, bool q_on_device, uint64_t n
         CPB_TRY(launch_search(h, cx, dq, cx.d_qtables.as<float>(), m, k, beam, rerank_k, o_ids, o_d, o_stats, st, dqc,
                               scan_only));
         if (calibrated && rerank_k == 0) CPB_TRY(launch_affine(h, o_d, m * k, float(h->calib_alpha), float(h->calib_beta), st));
-        if (!out_on_device) {
+        if (staged) {
+            CPB_CUDA(cudaStreamSynchronize(st));
+            std::memcpy(ids + q0 * k, o_ids, m * k * 4);
+            std::memcpy(dists + q0 * k, o_d, m * k * 4);
+            if (stats) std::memcpy(stats + q0 * 2, o_stats, m * 8);
+            synced = true;
+        } else if (!out_on_device) {
             CPB_CUDA(cudaMemcpyAsync(ids + q0 * k, o_ids, m * k * 4, cudaMemcpyDeviceToHost, st));
             CPB_CUDA(cudaMemcpyAsync(dists + q0 * k, o_d, m * k * 4, cudaMemcpyDeviceToHost, st));
             if (stats) CPB_CUDA(cudaMemcpyAsync(stats + q0 * 2, o_stats, m * 8, cudaMemcpyDeviceToHost, st));
@@ -454,7 +482,7 @@ int do_multiprobe(cphnsw_b200_index* h, const float* q, uint64_t nq, uint32_t k,
     for (uint64_t q0 = 0; q0 < nq; q0 += chunk) {
         const uint64_t m = nq - q0 < chunk ? nq - q0 : chunk;
         CPB_TRY(cx.d_q.reserve(m * h->dim * 4));
-        CPB_CUDA(cudaMemcpyAsync(cx.d_q.p, q + q0 * h->dim, m * h->dim * 4, cudaMemcpyHostToDevice, st));
+        CPB_TRY(copy_in(cx, cx.d_q.p, q + q0 * h->dim, m * h->dim * 4, st));
         CPB_TRY(cx.d_qtables.reserve(m * table_floats * 4));
         CPB_TRY(cx.d_qcodes.reserve(m * rb + 16));
         CPB_TRY(launch_encode(h, cx.d_q.as<float>(), m, cx.d_qcodes.p, cx.d_qtables.as<float>(), nullptr, st));
@@ -466,14 +494,27 @@ int do_multiprobe(cphnsw_b200_index* h, const float* q, uint64_t nq, uint32_t k,
         if (search) {
             CPB_TRY(cx.d_probe_ids.reserve(m * T * k * 4));
             CPB_TRY(cx.d_probe_dist.reserve(m * T * k * 4));
-            CPB_TRY(cx.d_out_ids.reserve(m * k * 4));
-            CPB_TRY(cx.d_out_dist.reserve(m * k * 4));
+            const bool staged = m * k * 8 <= kStagedBytes;
+            if (staged) {
+                CPB_TRY(cx.h_out.reserve(kStagedBytes));
+            } else {
+                CPB_TRY(cx.d_out_ids.reserve(m * k * 4));
+                CPB_TRY(cx.d_out_dist.reserve(m * k * 4));
+            }
+            uint32_t* o_ids = staged ? static_cast<uint32_t*>(cx.h_out.p) : cx.d_out_ids.as<uint32_t>();
+            float* o_d = staged ? reinterpret_cast<float*>(o_ids + m * k) : cx.d_out_dist.as<float>();
             CPB_TRY(launch_search(h, cx, nullptr, nullptr, m * T, k, beam, 0, cx.d_probe_ids.as<uint32_t>(),
                                   cx.d_probe_dist.as<float>(), nullptr, st, cx.d_probe_codes.p));
             CPB_TRY(launch_merge_probes(h, cx.d_probe_ids.as<uint32_t>(), cx.d_probe_dist.as<float>(), m, T, k,
-                                        cx.d_out_ids.as<uint32_t>(), cx.d_out_dist.as<float>(), st));
-            CPB_CUDA(cudaMemcpyAsync(ids + q0 * k, cx.d_out_ids.p, m * k * 4, cudaMemcpyDeviceToHost, st));
-            CPB_CUDA(cudaMemcpyAsync(dists + q0 * k, cx.d_out_dist.p, m * k * 4, cudaMemcpyDeviceToHost, st));
+                                        o_ids, o_d, st));
+            if (staged) {
+                CPB_CUDA(cudaStreamSynchronize(st));
+                std::memcpy(ids + q0 * k, o_ids, m * k * 4);
+                std::memcpy(dists + q0 * k, o_d, m * k * 4);
+            } else {
+                CPB_CUDA(cudaMemcpyAsync(ids + q0 * k, o_ids, m * k * 4, cudaMemcpyDeviceToHost, st));
+                CPB_CUDA(cudaMemcpyAsync(dists + q0 * k, o_d, m * k * 4, cudaMemcpyDeviceToHost, st));
+            }
         }
         CPB_CUDA(cudaStreamSynchronize(st));
     }

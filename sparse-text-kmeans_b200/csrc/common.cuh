@@ -92,6 +92,27 @@ struct DevBuf {
     T* as() const { return reinterpret_cast<T*>(p); }
 };
 
+// Page-locked host memory, visible to the device; grow-only, contents are not preserved
+struct PinnedBuf {
+    void* p = nullptr;
+    size_t bytes = 0;
+    PinnedBuf() = default;
+    PinnedBuf(const PinnedBuf&) = delete;
+    PinnedBuf& operator=(const PinnedBuf&) = delete;
+    ~PinnedBuf() {
+        if (p) cudaFreeHost(p);
+    }
+    int reserve(size_t n) {
+        if (n <= bytes && p) return 0;
+        if (p) cudaFreeHost(p);
+        p = nullptr;
+        bytes = 0;
+        CPB_CUDA(cudaHostAlloc(&p, n, cudaHostAllocPortable | cudaHostAllocMapped));
+        bytes = n;
+        return 0;
+    }
+};
+
 // Everything one search call writes besides its outputs: a stream, the staging and result buffers, the
 // work counter and the visited slots of its launch.  A handle keeps a pool of these so that search calls from
 // several host threads run side by side (the reference's callers search from OpenMP loops,
@@ -113,6 +134,7 @@ struct SearchCtx {
     DevBuf d_qtables, d_qcodes, d_q, d_out_ids, d_out_dist, d_stats;
     DevBuf d_seeds, d_cand;  // entry scan -> walk: seed keys; walk -> rerank: ids
     DevBuf d_probe_codes, d_probe_ids, d_probe_dist;  // search_multiprobe
+    PinnedBuf h_in, h_out;  // staging of small host-pointer calls: queries; results, which the kernels write there
     ~SearchCtx() {
         if (done) cudaEventDestroy(done);
         if (stream) cudaStreamDestroy(stream);

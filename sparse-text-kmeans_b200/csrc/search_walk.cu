@@ -737,12 +737,269 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
     if (w.exact_visited && lane == 0) a.epochs[slot] = epoch;
 }
 
+// ---- few queries: a block per query ----------------------------------------------------------------------------------
+// With fewer queries than the chip has room for walks, what counts is the length of one walk: its steps in sequence,
+// some 5,000 cycles each for a warp alone.  Here eight warps share a query and a step takes the first sixteen unexpanded
+// members of W, two rows a warp; the prefix committed grows from 3.4 rows to about 8, and the rows' lookups and scores
+// run side by side.  Rows, candidates and the committed prefix are those of search_walk_kernel, so the results are too.
+//
+// A step meets at three barriers: the warps' candidates are listed with their ranks in W and the bound each puts on the
+// prefix; repeats (a node found by two rows) and candidates of rows that are not committed are struck out; W is rebuilt
+// in the other of its two arrays, every member moving up by the candidates that rank before it.
+constexpr int kSquadWarps = 8;
+constexpr int kSquadThreads = kSquadWarps * 32;
+constexpr int kSquadRows = 2;                            // per warp
+constexpr int kSquadFront = kSquadWarps * kSquadRows;    // members of W taken per step
+constexpr uint32_t kStruck = 0xffffffffu;
+
+template <bool U16, int METRIC>
+__global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w) {
+    extern __shared__ __align__(16) unsigned char walk_smem[];
+    __shared__ uint64_t list_key[kSquadThreads];
+    __shared__ uint32_t list_place[kSquadThreads];  // members of W below; kStruck: struck out
+    __shared__ uint32_t list_row[kSquadThreads];    // place of the row in the step's prefix
+    __shared__ uint32_t cids[kSquadWarps][32], fronts[kSquadWarps][2 * kSquadFront];
+    __shared__ uint32_t listed, prefix, seeded;
+    const SearchArgs& a = w.s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t tid = threadIdx.x, below = (1u << lane) - 1u;
+    const uint32_t q = blockIdx.x, n = uint32_t(a.n);
+    constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
+    const int row_bytes = a.K * (U16 ? 2 : 1);
+    uint64_t* W = reinterpret_cast<uint64_t*>(walk_smem);
+    uint64_t* W2 = W + w.wcap_slots;
+    uint2* tags = reinterpret_cast<uint2*>(W2 + w.wcap_slots);
+    unsigned char* qcode = reinterpret_cast<unsigned char*>(tags) + kTagBytes;
+    uint32_t* qpacked = reinterpret_cast<uint32_t*>(qcode);
+    uint32_t* cid = cids[warp];
+    uint32_t* front = fronts[warp];
+    const float* table = SYM ? nullptr : a.tables + size_t(q) * a.K * a.P;
+
+    for (uint32_t i = tid; i < kTagBytes / 16; i += kSquadThreads) reinterpret_cast<uint4*>(tags)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (SYM) {
+        const unsigned char* src = static_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes;
+        if (METRIC == kSymBytes) {
+            for (int i = tid; i < row_bytes; i += kSquadThreads) qcode[i] = src[i];
+        } else if (warp == 0) {
+            for (int i = 0; i < a.packed_words; ++i) {
+                const int r = 32 * i + lane;
+                const uint32_t word = __ballot_sync(kFull, r < a.K && (src[r * (U16 ? 2 : 1)] & 1u));
+                if (lane == 0) qpacked[i] = word;
+            }
+        }
+    }
+    if (tid == 0) listed = 0, prefix = kSquadFront;
+    __syncthreads();
+
+    auto score = [&](int total, uint32_t id) -> float {
+        if (METRIC == kSymPacked)
+            return lane < total ? packed_distance_lane(qpacked, a.packed, id, a.packed_words, a.resid_kp, a.resid_mul) : 0.0f;
+        if (METRIC == kSymBytes)
+            return lane < total ? sym_distance_lane<U16>(qcode, a.codes, id, a.K, a.resid_kp, a.resid_mul) : 0.0f;
+        return score_asym<U16, METRIC == kAsym128>(table, static_cast<const unsigned char*>(a.codes), a.K, a.P, cid, total, lane);
+    };
+
+    // entry nodes: the scan's best, or (up to 32 of them) all
+    if (warp == 0) {
+        uint64_t k = kFiller;
+        uint32_t most = a.beam;
+        if (w.seeds) {
+            if (lane < int(a.n_seed)) k = w.seeds[size_t(q) * kScanKeep + lane];
+            if (k != kFiller) tag_store(tags, key_id(k));
+        } else {
+            const uint32_t id = uint32_t(lane) < a.n_entry ? __ldg(a.entry + lane) : kInvalidNode;
+            const int total = int(min(a.n_entry, 32u));
+            cid[lane] = id;
+            __syncwarp();
+            const float d = score(total, id);
+            if (lane < total) {
+                k = make_key(d, id);
+                tag_store(tags, id);
+            }
+        }
+        uint32_t rank = 0;
+        for (int i = 0; i < 32; ++i) rank += __shfl_sync(kFull, k, i) < k;
+        const uint32_t have = __popc(__ballot_sync(kFull, k != kFiller));
+        if (k != kFiller && rank < most) W[rank] = k;
+        if (lane == 0) seeded = min(have, most);
+    }
+    __syncthreads();
+    uint32_t count = seeded, cur = 0;
+
+    uint32_t pre_node[kSquadRows], pre_row[kSquadRows];
+#pragma unroll
+    for (int b = 0; b < kSquadRows; ++b) pre_node[b] = kInvalidNode, pre_row[b] = kInvalidNode;
+    while (true) {
+        // the first unexpanded members of the first window of 32 that has any: every warp finds them for itself
+        uint32_t un = 0;
+        while (cur < count) {
+            uint32_t u[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t p = cur + 32 * i + lane;
+                u[i] = __ballot_sync(kFull, p < count && !(uint32_t(W[min(p, count - 1)]) & 1u));
+            }
+            if (u[0] | u[1] | u[2] | u[3]) {
+                const int i = u[0] ? 0 : (u[1] ? 1 : (u[2] ? 2 : 3));
+                un = u[0] ? u[0] : (u[1] ? u[1] : (u[2] ? u[2] : u[3]));
+                cur += 32 * i;
+                break;
+            }
+            cur += 128;
+        }
+        if (!un) break;
+        const uint32_t order = __popc(un & below);
+        const bool open = (un >> lane) & 1u;
+        const uint64_t ek = W[min(cur + lane, count - 1)];
+        if (open && order < 2 * kSquadFront) front[order] = uint32_t(ek) >> 1;
+        const uint32_t sel = __ballot_sync(kFull, open && order < kSquadFront);
+        const int have = __popc(un);
+        __syncwarp();
+        uint32_t row[kSquadRows], fresh[kSquadRows];
+#pragma unroll
+        for (int b = 0; b < kSquadRows; ++b) {
+            const int t = warp * kSquadRows + b;
+            const uint32_t node = t < have ? front[t] : kInvalidNode;
+            row[b] = pre_row[b];
+            // (a row that another warp asked for ahead comes from L1)
+            if (node != pre_node[b]) row[b] = (node != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(node) * a.M + lane) : kInvalidNode;
+        }
+#pragma unroll
+        for (int b = 0; b < kSquadRows; ++b) {
+            const int t = kSquadFront + warp * kSquadRows + b;
+            pre_node[b] = t < have ? front[t] : kInvalidNode;
+            pre_row[b] = (pre_node[b] != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(pre_node[b]) * a.M + lane) : kInvalidNode;
+        }
+#pragma unroll
+        for (int b = 0; b < kSquadRows; ++b) fresh[b] = __ballot_sync(kFull, row[b] < n && !tag_seen(tags, row[b]));
+        // as many of the warp's rows as bring at most 32 candidates
+        int total = 0, first_of[kSquadRows];
+        uint32_t bound = uint32_t(have < kSquadFront ? have : kSquadFront);
+        bool room = true;
+#pragma unroll
+        for (int b = 0; b < kSquadRows; ++b) {
+            const int nf = __popc(fresh[b]);
+            first_of[b] = total;
+            if (room && total + nf > 32) {
+                room = false;
+                bound = min(bound, uint32_t(warp * kSquadRows + b));
+            }
+            if (room) {
+                if ((fresh[b] >> lane) & 1u) cid[total + __popc(fresh[b] & below)] = row[b];
+                total += nf;
+            }
+        }
+        __syncwarp();
+        uint32_t id = kInvalidNode, my_row = 0;
+        bool own = false;
+        if (total) {
+            own = lane < total;
+            id = own ? cid[lane] : kInvalidNode;
+#pragma unroll
+            for (int b = 0; b < kSquadRows; ++b)
+                if (lane >= first_of[b]) my_row = warp * kSquadRows + b;
+            const float d = score(total, id);
+            const uint32_t grp = __match_any_sync(kFull, id);
+            own = own && (__ffs(grp) - 1) == lane;
+            const uint64_t key = make_key(d, id);
+            bool adm = own && (count < a.beam || key < W[count - 1]);
+            uint32_t p = 0;
+            if (adm) {
+                p = lower_bound(W, count, key);
+                if (p < count && (W[p] >> 1) == (key >> 1)) adm = false;  // a forgotten node that is a member of W
+            }
+            if (adm) {
+                const uint32_t rel = p - cur;  // cur <= position of every selected member
+                const uint32_t bl = p <= cur ? 0u : (rel >= 32u ? sel : sel & ((1u << rel) - 1u));
+                bound = min(bound, max(my_row + 1u, uint32_t(__popc(bl))));
+            }
+            const uint32_t am = __ballot_sync(kFull, adm);
+            if (am) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&listed, uint32_t(__popc(am)));
+                at = __shfl_sync(kFull, at, 0) + __popc(am & below);
+                if (adm) {
+                    list_key[at] = key;
+                    list_place[at] = p;
+                    list_row[at] = my_row;
+                }
+            }
+        }
+        bound = __reduce_min_sync(kFull, bound);
+        if (lane == 0) atomicMin(&prefix, bound);
+        __syncthreads();
+        const uint32_t commit = prefix, m = listed;
+        if (own && my_row < commit) tag_store(tags, id);
+        const bool listed_here = tid < m;
+        const uint64_t key = listed_here ? list_key[tid] : 0;
+        bool keep = listed_here && list_row[tid] < commit;
+        if (keep)
+            for (uint32_t i = 0; i < tid; ++i)
+                if (list_key[i] == key && list_row[i] < commit) keep = false;
+        if (listed_here && !keep) list_place[tid] = kStruck;
+        __syncthreads();
+        if (tid == 0) listed = 0, prefix = kSquadFront;
+        const uint64_t committed = commit;
+        uint32_t kept = 0, lowest = kStruck, rank = 0;
+        for (uint32_t i = 0; i < m; ++i) {
+            const uint32_t p = list_place[i];
+            lowest = min(lowest, p);
+            if (p != kStruck) {
+                ++kept;
+                rank += list_key[i] < key;
+            }
+        }
+        // the members of the committed rows carry their flag from now on
+        uint32_t last = 0;  // window positions up to this bit are the committed ones among sel
+        {
+            uint32_t s = sel;
+            for (uint32_t c = 1; c < committed; ++c) s &= s - 1;
+            last = committed ? __ffs(s) - 1 : 0u;
+        }
+        const uint32_t flag = committed ? sel & (last == 31 ? kFull : (2u << last) - 1u) : 0u;
+        if (kept) {
+            const uint32_t newcount = min(a.beam, count + kept);
+            for (uint32_t j = tid; j < count; j += kSquadThreads) {
+                uint64_t e = W[j];
+                const uint32_t rel = j - cur;
+                if (j >= cur && rel < 32u && ((flag >> rel) & 1u)) e |= 1u;
+                uint32_t up = 0;
+                for (uint32_t i = 0; i < m; ++i) up += list_place[i] <= j;
+                if (j + up < newcount) W2[j + up] = e;
+            }
+            if (keep) {
+                const uint32_t f = list_place[tid] + rank;
+                if (f < newcount) W2[f] = key;
+            }
+            uint64_t* t = W;
+            W = W2;
+            W2 = t;
+            count = newcount;
+        } else if (warp == 0 && ((flag >> lane) & 1u)) {
+            W[cur + lane] = ek | 1u;
+        }
+        cur = min(cur, lowest);
+        __syncthreads();
+    }
+
+    if (w.cand) {
+        uint32_t* out = w.cand + size_t(q) * a.rerank_k;
+        for (uint32_t p = tid; p < a.rerank_k; p += kSquadThreads) out[p] = p < count ? key_id(W[p]) : kInvalidNode;
+    } else {
+        for (uint32_t p = tid; p < a.k; p += kSquadThreads) {
+            const uint64_t e = p < count ? W[p] : 0;
+            a.out_ids[size_t(q) * a.k + p] = p < count ? key_id(e) : kInvalidNode;
+            a.out_dist[size_t(q) * a.k + p] = p < count ? float_unorder(uint32_t(e >> 32)) : INFINITY;
+        }
+    }
+}
+
 // ---- exact rerank: one block per query -------------------------------------------------------------------------
 // 8 lanes per candidate row (128-bit loads), 32 rows of a block in flight per pass; the dot product is accumulated
 // with fmaf per lane and folded 4, 2, 1, as the fused rerank of search_kernel does.  The keys are then sorted in
 // shared memory and the k best written out.
-constexpr int kRerankThreads = 256;
-
+// (256 threads a block; 1,024 when there are few queries: 28 against 11 us for one query with 500 candidates)
+template <int kRerankThreads>
 __global__ void __launch_bounds__(kRerankThreads)
 search_rerank_kernel(const float* __restrict__ vectors, const float* __restrict__ queries, const uint32_t* __restrict__ cand,
                      uint32_t rr, uint32_t slots /* power of two >= rr */, int dim, uint32_t k, uint32_t* __restrict__ out_ids,
@@ -897,6 +1154,23 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         w.seeds = sc.seeds;
         CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
     }
+    // few queries: a block each while two of them share an SM at most
+    const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes + row;
+    if (!w.exact_visited && a.nq <= uint32_t(2 * h->sm_count) && (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 32))) {
+#define CPB_SQUAD(U, X)                                                                           \
+    do {                                                                                          \
+        CPB_CUDA(allow_max_dynamic_smem(search_squad_kernel<U, X>));                              \
+        search_squad_kernel<U, X><<<a.nq, kSquadThreads, squad_smem, st>>>(w);                    \
+    } while (0)
+        if (metric == kAsym128) CPB_SQUAD(false, kAsym128);
+        else if (metric == kAsym && u16) CPB_SQUAD(true, kAsym);
+        else if (metric == kAsym) CPB_SQUAD(false, kAsym);
+        else if (metric == kSymBytes && u16) CPB_SQUAD(true, kSymBytes);
+        else if (metric == kSymBytes) CPB_SQUAD(false, kSymBytes);
+        else if (u16) CPB_SQUAD(true, kSymPacked);
+        else CPB_SQUAD(false, kSymPacked);
+#undef CPB_SQUAD
+    } else {
 #define CPB_WALK(X) (u16 ? launch_walk_t<true, X>(h, w, blocks, warps, st) : launch_walk_t<false, X>(h, w, blocks, warps, st))
     switch (metric) {
         case kAsym: CPB_TRY(CPB_WALK(kAsym)); break;
@@ -905,15 +1179,22 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         default: CPB_TRY(CPB_WALK(kSymPacked)); break;
     }
 #undef CPB_WALK
+    }
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     if (a.rerank_k) {
         uint32_t slots = 32;
         while (slots < a.rerank_k) slots <<= 1;
         const size_t smem = size_t(slots) * 8 + (size_t(a.dim) * 4 + 15) / 16 * 16;
-        CPB_CUDA(allow_max_dynamic_smem(search_rerank_kernel));
-        search_rerank_kernel<<<a.nq, kRerankThreads, smem, st>>>(a.vectors, a.queries, w.cand, a.rerank_k, slots, a.dim, a.k,
-                                                                a.out_ids, a.out_dist);
+        if (a.nq <= uint32_t(2 * h->sm_count)) {
+            CPB_CUDA(allow_max_dynamic_smem(search_rerank_kernel<1024>));
+            search_rerank_kernel<1024><<<a.nq, 1024, smem, st>>>(a.vectors, a.queries, w.cand, a.rerank_k, slots, a.dim, a.k, a.out_ids,
+                                                                a.out_dist);
+        } else {
+            CPB_CUDA(allow_max_dynamic_smem(search_rerank_kernel<256>));
+            search_rerank_kernel<256><<<a.nq, 256, smem, st>>>(a.vectors, a.queries, w.cand, a.rerank_k, slots, a.dim, a.k, a.out_ids,
+                                                              a.out_dist);
+        }
         h->launches++;
         CPB_CUDA(cudaGetLastError());
     }
