@@ -148,19 +148,10 @@ int host_codes_from_packed(const cphnsw_b200_index* h, uint64_t first, uint64_t 
 // grows a device buffer to new_bytes keeping its first keep_bytes
 int grow_keep(DevBuf& b, size_t keep_bytes, size_t new_bytes) {
     if (b.p && new_bytes <= b.bytes) return 0;
-    void* p = nullptr;
-    const size_t cap = new_bytes + new_bytes / 2;
-    CPB_CUDA(cudaMalloc(&p, cap));
-    if (b.p && keep_bytes) {
-        cudaError_t e = cudaMemcpy(p, b.p, keep_bytes, cudaMemcpyDeviceToDevice);
-        if (e != cudaSuccess) {
-            cudaFree(p);
-            CPB_CUDA(e);
-        }
-    }
-    b.release();
-    b.p = p;
-    b.bytes = cap;
+    DevBuf grown;
+    CPB_TRY(grown.reserve(new_bytes + new_bytes / 2));
+    if (b.p && keep_bytes) CPB_CUDA(cudaMemcpy(grown.p, b.p, keep_bytes, cudaMemcpyDeviceToDevice));
+    b.swap(grown);
     return 0;
 }
 
@@ -527,7 +518,18 @@ int do_multiprobe(cphnsw_b200_index* h, const float* q, uint64_t nq, uint32_t k,
 
 using namespace cpb;
 
+void cphnsw_b200_index::release_buffers() {
+    QuietDevice quiet;  // one wait for all of them
+    ctxs.clear();
+    for (DevBuf* b : {&d_signs, &d_signbits, &d_status, &d_vectors, &d_codes, &d_adj, &d_entry, &d_entry_codes, &d_entry_scan, &d_packed,
+                      &d_exact_base, &d_qtables, &d_qcodes, &d_q, &s_in, &s_in2, &s_out, &s_out2, &s_pad, &s_pad2, &s_sliced, &s_rank,
+                      &s_kept})
+        b->release();
+}
+
 cphnsw_b200_index::~cphnsw_b200_index() {
+    release_buffers();
+    if (sm_count) device_handle_destroyed(device);
     for (auto& pool : events)
         for (auto& e : pool) {
             if (e.start) cudaEventDestroy(e.start);
@@ -567,8 +569,8 @@ int cphnsw_b200_device_count(void) {
     }
     int ok = 0;
     for (int d = 0; d < n; ++d) {
-        cudaDeviceProp p;
-        if (cudaGetDeviceProperties(&p, d) == cudaSuccess && p.major == 10) ++ok;
+        int major = 0;
+        if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, d) == cudaSuccess && major == 10) ++ok;
     }
     return ok;
 }
@@ -615,10 +617,12 @@ static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint3
         return CPHNSW_B200_E_CUDA;
     }
     if (device < 0 || device >= ndev) { set_error("device %d out of range (%d devices)", device, ndev); return CPHNSW_B200_E_INVALID; }
-    cudaDeviceProp prop;
-    CPB_CUDA(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10) {
-        set_error("device %d is sm_%d%d; this library is built for sm_100a only", device, prop.major, prop.minor);
+    int major = 0, minor = 0, sms = 0;
+    CPB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+    CPB_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
+    CPB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (major != 10) {
+        set_error("device %d is sm_%d%d; this library is built for sm_100a only", device, major, minor);
         return CPHNSW_B200_E_CUDA;
     }
     CPB_CUDA(cudaSetDevice(device));
@@ -641,7 +645,7 @@ static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint3
     h->convention = fht_convention;
     h->device = device;
     h->binary_codes = binary ? 1 : 0;
-    h->sm_count = prop.multiProcessorCount;
+    h->sm_count = sms;
     // RotationChain: rotation r is seeded seed + r (include/cphnsw/encoder/rotation.hpp:173-178);
     // each table is drawn layer by layer from mt19937_64 through uniform_int_distribution<int>(0,1)
     // (rotation.hpp:134-144) — the standard library does the draw, as in the reference.
@@ -656,6 +660,7 @@ static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint3
     for (int kk = 1; kk < kKernelKinds; ++kk) h->events[kk].reserve(1024);
     if (rc == 0) rc = h->d_status.reserve(256);
     if (rc == 0 && cudaMemset(h->d_status.p, 0, 256) != cudaSuccess) rc = cuda_fail(cudaGetLastError(), "memset status");
+    device_handle_created(device);
     if (rc != 0) {
         delete h;
         return rc;

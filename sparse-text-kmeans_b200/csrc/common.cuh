@@ -42,16 +42,25 @@ int cuda_fail(cudaError_t e, const char* what);
 // function, not to the launch: concurrent callers that each set "what my launch needs" would lower it under one
 // another's feet, so every caller sets the same, largest value (the device's opt-in limit less the kernel's static
 // shared memory).
+// (Done once per kernel and device: the four runtime calls cost several microseconds a launch.)
+cudaError_t allow_max_dynamic_smem_of(const void* kernel);
 template <class F>
 inline cudaError_t allow_max_dynamic_smem(F* kernel) {
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
-    if (e != cudaSuccess) return e;
-    int dev = 0, optin = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - int(fa.sharedSizeBytes));
+    return allow_max_dynamic_smem_of(reinterpret_cast<const void*>(kernel));
 }
+
+// Device memory of the library.  Freed blocks are kept per device for later buffers of any handle: a small index built and
+// dropped spent most of its time in cudaMalloc and cudaFree.  What is kept is bounded (device_memory.cu), shrinks when the
+// device's last handle goes, and is returned to the driver as a whole when an allocation fails.  device_free waits for the
+// device like cudaFree does, unless the calling thread is inside a QuietDevice (which has waited already).
+int device_alloc(void** p, size_t* bytes, int* device);
+void device_free(void* p, size_t bytes, int device);
+void device_handle_created(int device);
+void device_handle_destroyed(int device);
+struct QuietDevice {
+    QuietDevice();
+    ~QuietDevice();
+};
 
 // kernel families whose launches can be timed
 enum KernelKind { kKernelEncode = 0, kKernelCodeDistance = 1, kKernelKnn = 2, kKernelSelect = 3, kKernelSearch = 4 };
@@ -64,12 +73,13 @@ struct EventPair {
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    int device = 0;
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        if (p) device_free(p, bytes, device);
         p = nullptr;
         bytes = 0;
     }
@@ -78,15 +88,16 @@ struct DevBuf {
         if (n <= bytes && p) return 0;
         release();
         if (n == 0) n = 16;
-        CPB_CUDA(cudaMalloc(&p, n));
+        CPB_TRY(device_alloc(&p, &n, &device));
         bytes = n;
         return 0;
     }
     void swap(DevBuf& o) {
         void* tp = p;
         size_t tb = bytes;
-        p = o.p, bytes = o.bytes;
-        o.p = tp, o.bytes = tb;
+        const int td = device;
+        p = o.p, bytes = o.bytes, device = o.device;
+        o.p = tp, o.bytes = tb, o.device = td;
     }
     template <class T>
     T* as() const { return reinterpret_cast<T*>(p); }
@@ -211,6 +222,7 @@ struct cphnsw_b200_index {
     std::mutex ev_mu;
     std::vector<cpb::EventPair> events[cpb::kKernelKinds];
     size_t events_used[cpb::kKernelKinds] = {0, 0, 0, 0, 0};
+    void release_buffers();
     ~cphnsw_b200_index();
 };
 

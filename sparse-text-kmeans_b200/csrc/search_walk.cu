@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
     if (w.exact_visited && lane == 0) a.epochs[slot] = epoch;
 }
 
-// ---- few queries: a block per query ----------------------------------------------------------------------------------
+// ---- few queries (asymmetric metric): a block per query ----------------------------------------------------------------------------------
 // With fewer queries than the chip has room for walks, what counts is the length of one walk: its steps in sequence,
 // some 5,000 cycles each for a warp alone.  Here eight warps share a query and a step takes the first sixteen unexpanded
 // members of W, two rows a warp; the prefix committed grows from 3.4 rows to about 8, and the rows' lookups and scores
@@ -746,11 +746,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
 // A step meets at three barriers: the warps' candidates are listed with their ranks in W and the bound each puts on the
 // prefix; repeats (a node found by two rows) and candidates of rows that are not committed are struck out; W is rebuilt
 // in the other of its two arrays, every member moving up by the candidates that rank before it.
+constexpr uint32_t kStruck = 0xffffffffu;
+
 constexpr int kSquadWarps = 8;
 constexpr int kSquadThreads = kSquadWarps * 32;
 constexpr int kSquadRows = 2;                            // per warp
 constexpr int kSquadFront = kSquadWarps * kSquadRows;    // members of W taken per step
-constexpr uint32_t kStruck = 0xffffffffu;
 
 template <bool U16, int METRIC>
 __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w) {
@@ -764,38 +765,18 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tid = threadIdx.x, below = (1u << lane) - 1u;
     const uint32_t q = blockIdx.x, n = uint32_t(a.n);
-    constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
-    const int row_bytes = a.K * (U16 ? 2 : 1);
     uint64_t* W = reinterpret_cast<uint64_t*>(walk_smem);
     uint64_t* W2 = W + w.wcap_slots;
     uint2* tags = reinterpret_cast<uint2*>(W2 + w.wcap_slots);
-    unsigned char* qcode = reinterpret_cast<unsigned char*>(tags) + kTagBytes;
-    uint32_t* qpacked = reinterpret_cast<uint32_t*>(qcode);
     uint32_t* cid = cids[warp];
     uint32_t* front = fronts[warp];
-    const float* table = SYM ? nullptr : a.tables + size_t(q) * a.K * a.P;
+    const float* table = a.tables + size_t(q) * a.K * a.P;
 
     for (uint32_t i = tid; i < kTagBytes / 16; i += kSquadThreads) reinterpret_cast<uint4*>(tags)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (SYM) {
-        const unsigned char* src = static_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes;
-        if (METRIC == kSymBytes) {
-            for (int i = tid; i < row_bytes; i += kSquadThreads) qcode[i] = src[i];
-        } else if (warp == 0) {
-            for (int i = 0; i < a.packed_words; ++i) {
-                const int r = 32 * i + lane;
-                const uint32_t word = __ballot_sync(kFull, r < a.K && (src[r * (U16 ? 2 : 1)] & 1u));
-                if (lane == 0) qpacked[i] = word;
-            }
-        }
-    }
     if (tid == 0) listed = 0, prefix = kSquadFront;
     __syncthreads();
 
-    auto score = [&](int total, uint32_t id) -> float {
-        if (METRIC == kSymPacked)
-            return lane < total ? packed_distance_lane(qpacked, a.packed, id, a.packed_words, a.resid_kp, a.resid_mul) : 0.0f;
-        if (METRIC == kSymBytes)
-            return lane < total ? sym_distance_lane<U16>(qcode, a.codes, id, a.K, a.resid_kp, a.resid_mul) : 0.0f;
+    auto score = [&](int total) -> float {
         return score_asym<U16, METRIC == kAsym128>(table, static_cast<const unsigned char*>(a.codes), a.K, a.P, cid, total, lane);
     };
 
@@ -811,7 +792,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
             const int total = int(min(a.n_entry, 32u));
             cid[lane] = id;
             __syncwarp();
-            const float d = score(total, id);
+            const float d = score(total);
             if (lane < total) {
                 k = make_key(d, id);
                 tag_store(tags, id);
@@ -898,7 +879,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
 #pragma unroll
             for (int b = 0; b < kSquadRows; ++b)
                 if (lane >= first_of[b]) my_row = warp * kSquadRows + b;
-            const float d = score(total, id);
+            const float d = score(total);
             const uint32_t grp = __match_any_sync(kFull, id);
             own = own && (__ffs(grp) - 1) == lane;
             const uint64_t key = make_key(d, id);
@@ -1096,6 +1077,13 @@ int launch_walk_t(cphnsw_b200_index* h, const WalkArgs& w, int blocks, int warps
     return go(search_walk_kernel<U16, METRIC, 4>);  // beams up to 4,096: four words of the merge's bit set per lane
 }
 
+template <bool U16, int METRIC>
+int launch_squad_t(const WalkArgs& w, size_t smem, cudaStream_t st) {
+    CPB_CUDA(allow_max_dynamic_smem(search_squad_kernel<U16, METRIC>));
+    search_squad_kernel<U16, METRIC><<<w.s.nq, kSquadThreads, smem, st>>>(w);
+    return 0;
+}
+
 }  // namespace
 
 // Fills in the launch shape and runs walk and rerank.  a.next_query is zero on entry.
@@ -1154,22 +1142,16 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         w.seeds = sc.seeds;
         CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
     }
-    // few queries: a block each while two of them share an SM at most
-    const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes + row;
-    if (!w.exact_visited && a.nq <= uint32_t(2 * h->sm_count) && (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 32))) {
-#define CPB_SQUAD(U, X)                                                                           \
-    do {                                                                                          \
-        CPB_CUDA(allow_max_dynamic_smem(search_squad_kernel<U, X>));                              \
-        search_squad_kernel<U, X><<<a.nq, kSquadThreads, squad_smem, st>>>(w);                    \
-    } while (0)
-        if (metric == kAsym128) CPB_SQUAD(false, kAsym128);
-        else if (metric == kAsym && u16) CPB_SQUAD(true, kAsym);
-        else if (metric == kAsym) CPB_SQUAD(false, kAsym);
-        else if (metric == kSymBytes && u16) CPB_SQUAD(true, kSymBytes);
-        else if (metric == kSymBytes) CPB_SQUAD(false, kSymBytes);
-        else if (u16) CPB_SQUAD(true, kSymPacked);
-        else CPB_SQUAD(false, kSymPacked);
-#undef CPB_SQUAD
+    // Few queries under the asymmetric metric: a block each.  Measured on 64 / 250 / 500 queries: 367 / 432 / 568 us against
+    // 473 / 513 / 536 with a warp each (100k x 128, beam 500), 250 / 500 / 1,000 of d = 960: 1.27 / 1.50 / 2.65 ms against
+    // 2.10 / 2.15 / 2.51; under the symmetric metrics, whose scores cost little and tie often, a warp was always faster.
+    const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 > 32 * 1024 ? 4 : 2;
+    const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes;
+    if (!sym && !w.exact_visited && a.nq <= squads_per_sm * uint32_t(h->sm_count) &&
+        (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 32))) {
+        if (metric == kAsym128) CPB_TRY((launch_squad_t<false, kAsym128>(w, squad_smem, st)));
+        else if (u16) CPB_TRY((launch_squad_t<true, kAsym>(w, squad_smem, st)));
+        else CPB_TRY((launch_squad_t<false, kAsym>(w, squad_smem, st)));
     } else {
 #define CPB_WALK(X) (u16 ? launch_walk_t<true, X>(h, w, blocks, warps, st) : launch_walk_t<false, X>(h, w, blocks, warps, st))
     switch (metric) {
