@@ -213,6 +213,7 @@ struct cphnsw_b200_index {
     cpb::DevBuf d_qtables, d_qcodes, d_q;
     // stage scratch for the host-pointer entry points
     cpb::DevBuf s_in, s_in2, s_out, s_out2, s_pad, s_pad2, s_sliced;
+    cpb::DevBuf s_flags;         // exact search: queries the tensor-core filter could not settle
     cpb::DevBuf s_rank, s_kept;  // rank-based pruning: reverse lists, kept rows
 
     std::atomic<uint64_t> launches{0};
@@ -279,6 +280,10 @@ int launch_pack_sign_bits(cphnsw_b200_index* h, const void* d_codes, uint64_t n,
 // exact inner-product top-k and rerank over fp32 vectors (exact.cu)
 int launch_exact_search(cphnsw_b200_index* h, const float* d_base, uint64_t n, const float* d_q, uint64_t nq, uint32_t k,
                         uint32_t* d_ids, float* d_dist, cudaStream_t st);
+// the same through the tensor cores (exact_mma.cu): settles all queries but the flagged ones
+bool exact_mma_supported(const cphnsw_b200_index* h, uint64_t n, uint64_t nq, uint32_t k);
+int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, const float* d_q, uint64_t nq, uint32_t k, uint32_t* d_ids,
+                     float* d_dist, uint8_t* d_flags, cudaStream_t st);
 int launch_rerank(cphnsw_b200_index* h, const float* d_base, uint64_t n, const float* d_q, uint64_t nq, const uint32_t* d_cand,
                   uint32_t num_cand, uint32_t k, uint32_t* d_ids, float* d_dist, cudaStream_t st);
 // multiprobe sequence of rotated queries [nq][K][P] -> probe codes [nq][T][K]; merge of per-probe results

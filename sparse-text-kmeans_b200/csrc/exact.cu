@@ -52,12 +52,18 @@ template <int SLOTS, int CPL>
 __global__ void __launch_bounds__(kExWarps * 32)
 exact_topk_kernel(const float* __restrict__ base, uint64_t n, int dim, const float* __restrict__ queries, uint64_t nq,
                   uint32_t k, int aligned16, uint32_t* __restrict__ out_ids, float* __restrict__ out_dist,
-                  uint32_t* __restrict__ part_key, uint32_t* __restrict__ part_id) {
+                  uint32_t* __restrict__ part_key, uint32_t* __restrict__ part_id,
+                  const uint8_t* __restrict__ wanted /* nullptr: every query */) {
     constexpr int TILE = 32 * CPL;
     constexpr int ROWS = TILE + kExWarps * kExQ;  // base rows, then query rows
     extern __shared__ __align__(16) float ex_smem[];  // [2][ROWS][kExRow]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t q_first = uint64_t(blockIdx.x) * kExWarps * kExQ;
+    if (wanted) {  // (the same answer in every warp: its lanes look at all of the block's queries)
+        const bool mine = lane < kExWarps * kExQ && q_first + lane < nq && wanted[q_first + lane];
+        static_assert(kExWarps * kExQ == 32, "a lane per query");
+        if (!__ballot_sync(kFull, mine)) return;
+    }
     const uint64_t tiles = (n + TILE - 1) / TILE;
     const uint64_t t_begin = tiles * blockIdx.y / gridDim.y, t_end = tiles * (blockIdx.y + 1) / gridDim.y;
     const int nch = (dim + kExChunk - 1) / kExChunk;
@@ -165,7 +171,7 @@ exact_topk_kernel(const float* __restrict__ base, uint64_t n, int dim, const flo
 #pragma unroll
     for (int q = 0; q < kExQ; ++q) {
         const uint64_t row = q_first + uint64_t(warp) * kExQ + q;
-        if (row >= nq) continue;
+        if (row >= nq || (wanted && !wanted[row])) continue;
 #pragma unroll
         for (int s = 0; s < SLOTS; ++s) {
             const uint32_t rank = s * 32 + lane;
@@ -185,10 +191,11 @@ exact_topk_kernel(const float* __restrict__ base, uint64_t n, int dim, const flo
 // One warp per query: the S partial lists (ascending id ranges, each sorted) merged into the final one.
 template <int SLOTS>
 __global__ void exact_merge_kernel(const uint32_t* __restrict__ part_key, const uint32_t* __restrict__ part_id, uint64_t nq,
-                                   int S, uint32_t k, uint32_t* __restrict__ out_ids, float* __restrict__ out_dist) {
+                                   int S, uint32_t k, uint32_t* __restrict__ out_ids, float* __restrict__ out_dist,
+                                   const uint8_t* __restrict__ wanted) {
     const int lane = threadIdx.x & 31;
     const uint64_t q = uint64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (q >= nq) return;
+    if (q >= nq || (wanted && !wanted[q])) return;
     uint32_t ld[SLOTS], li[SLOTS], tau = kFull;
 #pragma unroll
     for (int s = 0; s < SLOTS; ++s) ld[s] = kFull, li[s] = kInvalidNode;
@@ -275,7 +282,7 @@ __global__ void rerank_kernel(const float* __restrict__ base, uint64_t n, int di
 
 template <int SLOTS, int CPL>
 int launch_exact_t(cphnsw_b200_index* h, const float* d_base, uint64_t n, const float* d_q, uint64_t nq, uint32_t k,
-                   uint32_t* d_ids, float* d_dist, cudaStream_t st) {
+                   uint32_t* d_ids, float* d_dist, const uint8_t* d_wanted, cudaStream_t st) {
     constexpr int TILE = 32 * CPL;
     const int dim = int(h->dim);
     const size_t smem = size_t(2) * (TILE + kExWarps * kExQ) * kExRow * sizeof(float);
@@ -296,11 +303,11 @@ int launch_exact_t(cphnsw_b200_index* h, const float* d_base, uint64_t n, const 
         (dim & 3) == 0 && ((reinterpret_cast<uintptr_t>(d_base) | reinterpret_cast<uintptr_t>(d_q)) & 15) == 0 ? 1 : 0;
     CPB_CUDA(cudaFuncSetAttribute(exact_topk_kernel<SLOTS, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     exact_topk_kernel<SLOTS, CPL><<<dim3(unsigned(blocks), unsigned(S)), kExWarps * 32, smem, st>>>(
-        d_base, n, dim, d_q, nq, k, aligned16, d_ids, d_dist, pk, pi);
+        d_base, n, dim, d_q, nq, k, aligned16, d_ids, d_dist, pk, pi, d_wanted);
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     if (S > 1) {
-        exact_merge_kernel<SLOTS><<<unsigned((nq + 3) / 4), 128, 0, st>>>(pk, pi, nq, int(S), k, d_ids, d_dist);
+        exact_merge_kernel<SLOTS><<<unsigned((nq + 3) / 4), 128, 0, st>>>(pk, pi, nq, int(S), k, d_ids, d_dist, d_wanted);
         h->launches++;
         CPB_CUDA(cudaGetLastError());
     }
@@ -322,9 +329,15 @@ int launch_exact_search(cphnsw_b200_index* h, const float* d_base, uint64_t n, c
         set_error("exact_search: too many queries");
         return CPHNSW_B200_E_INVALID;
     }
-    if (k <= 32) return launch_exact_t<1, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, st);
-    if (k <= 64) return launch_exact_t<2, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, st);
-    return launch_exact_t<4, 2>(h, d_base, n, d_q, nq, k, d_ids, d_dist, st);
+    const uint8_t* wanted = nullptr;
+    if (exact_mma_supported(h, n, nq, k)) {
+        CPB_TRY(h->s_flags.reserve(nq));
+        CPB_TRY(launch_exact_mma(h, d_base, n, d_q, nq, k, d_ids, d_dist, h->s_flags.as<uint8_t>(), st));
+        wanted = h->s_flags.as<uint8_t>();  // what the filter could not settle
+    }
+    if (k <= 32) return launch_exact_t<1, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, wanted, st);
+    if (k <= 64) return launch_exact_t<2, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, wanted, st);
+    return launch_exact_t<4, 2>(h, d_base, n, d_q, nq, k, d_ids, d_dist, wanted, st);
 }
 
 // ids / dist as above from the candidates cand[nq][num_cand] (device)

@@ -25,7 +25,7 @@
 // that a tile comes from L2; only the rows left over by the last full wave are split between blocks along the candidates.
 #include <cuda_fp16.h>
 
-#include "knn_common.cuh"
+#include "mma_common.cuh"
 
 namespace cpb {
 namespace {
@@ -34,14 +34,13 @@ using knn::kFull;
 using knn::kWaitLimit;
 using knn::mbar_wait_bounded;
 using knn::smem_u32;
+using namespace mma;
 
-constexpr int kMmaRows = 256;             // rows per block and candidates per tile
 constexpr int kMmaCap = 384;              // entries of a buffer: at most 128 before a tile and 256 from it
 constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
 constexpr uint32_t kMmaKeep = 128;
 constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, every second tile
 constexpr int kMmaThreads = (kEpiWarps + 3) * 32;  // and one each for the operands' copies, the products, the codes' copies
-constexpr uint32_t kTmemCols = 512;
 constexpr int kMaxCodeStages = 4;
 constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 9 KB of static
 constexpr int kBoundOrders = 8;           // orders of likely neighbours
@@ -250,15 +249,6 @@ bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t*
 }
 
 // ---- tcgen05 pieces ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
-    // K-major, no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes apart along the rows (stride offset) and
-    // 256 * 16 bytes apart along K (leading offset); version 1
-    uint64_t d = (smem_addr >> 4) & 0x3fffu;
-    d |= uint64_t((kMmaRows * 16) >> 4) << 16;
-    d |= uint64_t(128 >> 4) << 32;
-    d |= uint64_t(1) << 46;
-    return d;
-}
 // D fp16, A and B e4m3, both K-major, M = 128, N = 256
 constexpr uint32_t kIdesc = (uint32_t(256 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
 
@@ -268,17 +258,6 @@ __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a, uint64_t b, 
         "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
         "l"(a), "l"(b), "r"(kIdesc), "r"(uint32_t(accumulate))
         : "memory");
-}
-__device__ __forceinline__ uint32_t elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // 16 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
 __device__ __forceinline__ void tmem_load16(uint32_t (&r)[8], uint32_t addr) {
@@ -294,39 +273,6 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[8]) {
                  :
                  : "memory");
 }
-// A bounded wait that also ends when another role of the block has given up.  A poll may sleep for a microsecond: warps
-// that spin take the issue slots of those that work.
-__device__ __forceinline__ bool mbar_try_wait_us(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, uint32_t limit, volatile int* aborted) {
-    for (uint32_t i = 0; i < limit; ++i) {
-        if (mbar_try_wait_us(bar, parity)) return true;
-        if ((i & 15) == 15 && *aborted) return false;
-    }
-    return false;
-}
-
-// ---- work split -----------------------------------------------------------------------------------------------------
-// A launch takes `rts` row tiles against all `cts` candidate tiles: rts * cts steps in row-major order, an equal run of
-// them for every block.  When rts is a multiple of the blocks a block takes whole row tiles, and all blocks read the same
-// candidate tiles at the same time; otherwise a row tile may be shared by blocks.  Along the runs block + row tile only
-// grows, so it names a segment (one block's part of one row tile) and its buffers.
-struct Split {
-    uint64_t steps;
-    uint32_t cts, blocks;
-    __host__ __device__ uint64_t first_step(uint32_t block) const { return uint64_t(block) * steps / blocks; }
-    __host__ __device__ uint32_t block_of(uint64_t step) const { return uint32_t(((step + 1) * blocks - 1) / steps); }
-};
-
 struct KnnMmaArgs {
     const uint4* operand;  // [tiles][chunks][256]
     const uint4* codes;    // padded rows

@@ -1,0 +1,80 @@
+"""Exact search through the tensor-core filter (csrc/exact_mma.cu) against the CPU loop and the plain kernel: ids and
+distances are those of fp32 sums in d order, so every comparison is exact."""
+import numpy as np
+import pytest
+
+from cphnsw_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cp():
+    import cphnsw_b200
+    return cphnsw_b200
+
+
+def exact(cp, base, q, k):
+    idx = cp.CPHNSWIndex(base.shape[1], K=8, M=4, ef_construction=8)
+    idx.set_exact_base(base)
+    return idx, idx.exact_search_batch(q, k)
+
+
+def plain(idx, q, k):
+    """Fewer than 64 queries a call: the plain kernel."""
+    out = [idx.exact_search_batch(q[i:i + 50], k) for i in range(0, q.shape[0], 50)]
+    return np.concatenate([o[0] for o in out]), np.concatenate([o[1] for o in out])
+
+
+# groups of 32 vectors, tiles of 256 vectors and 256 queries, dims padded to 16; the least sizes the filter takes
+@pytest.mark.parametrize("n,nq,dim,k", [(16384, 64, 128, 1), (16385, 257, 128, 10), (20011, 100, 96, 100), (33000, 300, 50, 32),
+                                        (16639, 64, 17, 64), (40000, 513, 3, 10), (70001, 200, 128, 128)])
+def test_filter_equals_plain_kernel(cp, n, nq, dim, k):
+    base, q = synthetic.gaussian_mixture(n, nq, dim, max(1, n // 1000), 0.3, n + k)
+    idx, (ids, dist) = exact(cp, base, q, k)
+    wi, wd = plain(idx, q, k)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
+@pytest.mark.parametrize("kind", ["scales", "equal", "near", "zeros", "inf", "nan", "tiny", "negative"])
+def test_awkward_values(cp, kind):
+    rng = np.random.default_rng(5)
+    n, nq, dim, k = 17000, 70, 64, 10
+    base = rng.standard_normal((n, dim)).astype(np.float32)
+    q = rng.standard_normal((nq, dim)).astype(np.float32)
+    if kind == "scales":  # rows and queries of very different lengths
+        base *= np.exp2(rng.integers(-12, 12, (n, 1))).astype(np.float32)
+        q *= np.exp2(rng.integers(-30, 30, (nq, 1))).astype(np.float32)
+    if kind == "equal":  # one vector n times: every product ties, far more candidates than the buffers hold
+        base[:] = base[0]
+    if kind == "near":  # products that differ by less than the bound on the error
+        base[:] = base[0] + np.float32(1e-5) * base
+    if kind == "zeros":
+        base[:] = 0
+        q[::2] = 0
+    if kind == "inf":
+        base[77, 3] = np.inf
+    if kind == "nan":  # a query that cannot be scaled goes the plain way, the others do not mind
+        q[5, 1] = np.inf
+    if kind == "tiny":
+        base *= np.float32(1e-30)
+        q *= np.float32(1e-25)
+    if kind == "negative":  # all products negative
+        base, q = -np.abs(base), np.abs(q)
+    with np.errstate(all="ignore"):
+        idx, (ids, dist) = exact(cp, base, q, k)
+        wi, wd = plain(idx, q, k)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd, equal_nan=True)
+
+
+def test_filter_equals_cpu_loop(cp):
+    import oracle
+    base, q = synthetic.gaussian_sphere(16500, 64, 40, 9)
+    _, (ids, dist) = exact(cp, base, q, 20)
+    dots = np.zeros((64, base.shape[0]), np.float32)
+    for d in range(40):
+        dots = dots + q[:, d:d + 1] * base[:, d][None, :]
+    order = np.lexsort((np.broadcast_to(np.arange(base.shape[0]), dots.shape), np.float32(0) - dots), axis=1)[:, :20]
+    assert np.array_equal(ids, order.astype(np.uint32))
+    assert np.array_equal(dist, np.take_along_axis(np.float32(0) - dots, order, 1))
+    assert np.array_equal(oracle.ground_truth(q, base, 20), ids)
