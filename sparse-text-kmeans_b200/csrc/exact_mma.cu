@@ -1,4 +1,4 @@
-// Exact inner-product search with the tensor cores as a filter (dimensions up to 128, 64 queries and more).
+// Exact inner-product search with the tensor cores as a filter (dimensions up to 128).
 //
 // Same result as exact_topk_kernel: the k smallest (-<q,x>, id), the dot product accumulated in fp32 in d order without
 // fused multiply-add.  Two fp32 operations per pair and dimension bound that kernel; here every pair costs a tensor
@@ -33,8 +33,8 @@ using namespace mma;
 constexpr int kXmEpiWarps = 16;
 constexpr int kXmThreads = (kXmEpiWarps + 2) * 32;
 constexpr uint32_t kXmGroup = 32;          // base vectors per maximum
-constexpr uint32_t kPickGroups = 1024;     // groups a query may have computed exactly
-constexpr uint32_t kPickKeys = 2048;       // candidates a query may sort
+constexpr uint32_t kPickGroups = 1024;     // groups a query may list
+constexpr uint32_t kPickKeys = 1024;       // candidates a query may sort
 constexpr int kPickThreads = 256;
 
 // ---- norms and largest coordinates: one warp per row -------------------------------------------------------------------
@@ -43,14 +43,25 @@ constexpr int kPickThreads = 256;
 __global__ void row_stats_kernel(const float* __restrict__ x, uint64_t n, int dim, uint32_t* __restrict__ stat, float2* __restrict__ per_row) {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
+    const bool vec4 = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // (dim <= 128: a load per lane)
     uint32_t top = 0, norm = 0;
+#pragma unroll 4
     for (uint64_t row = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < n; row += warps) {
         float sum = 0.0f;
         uint32_t big = 0;
-        for (int i = lane; i < dim; i += 32) {
-            const float v = __ldg(x + row * dim + i);
-            big = max(big, __float_as_uint(v) & 0x7fffffffu);
-            sum += v * v;
+        if (vec4) {
+            if (4 * lane < dim) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(x + row * dim) + lane);
+                big = max(max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu),
+                          max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
+                sum = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            }
+        } else {
+            for (int i = lane; i < dim; i += 32) {
+                const float v = __ldg(x + row * dim + i);
+                big = max(big, __float_as_uint(v) & 0x7fffffffu);
+                sum += v * v;
+            }
         }
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
@@ -309,7 +320,7 @@ struct PickArgs {
     const uint32_t* status;
     uint64_t n;
     uint32_t groups, k;
-    int dim, vec4;
+    int dim, vec4, vec8;
     uint32_t* ids;
     float* dist;
     uint8_t* flags;        // 1: left to exact_topk_kernel
@@ -322,12 +333,20 @@ __device__ __forceinline__ uint32_t order_of(float v) {
 }
 __device__ __forceinline__ float value_of(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
 
+// 32 bytes, 32-byte aligned, by one instruction
+__device__ __forceinline__ void load_sector(float* v, const float* p) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
 __global__ void __launch_bounds__(kPickThreads) exact_pick_kernel(PickArgs a) {
-    __shared__ uint32_t hist[2048];
     __shared__ uint64_t keys[kPickKeys];
+    __shared__ float list_max[kPickGroups], tops[kPickThreads];
     __shared__ uint32_t list[kPickGroups];
     __shared__ __align__(16) float qv[128];
-    __shared__ uint32_t sums[kPickThreads / 32], n_list, n_keys, bin_sm, rest_sm;
+    __shared__ uint32_t n_list, n_keys;
+    __shared__ float kth;
     const uint32_t tid = threadIdx.x, q = blockIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const float* mx = a.maxima + size_t(q) * a.groups;
@@ -339,72 +358,109 @@ __global__ void __launch_bounds__(kPickThreads) exact_pick_kernel(PickArgs a) {
     }
     for (int i = tid; i < 128; i += kPickThreads) qv[i] = i < a.dim ? __ldg(a.queries + size_t(q) * a.dim + i) : 0.0f;
     if (tid == 0) n_list = 0, n_keys = 0;
-    // A, from below: the k-th largest maximum to 22 bits, 11 at a time
-    uint32_t prefix = 0, want = a.k;
-    for (int round = 0; round < 2; ++round) {
-        for (int i = tid; i < 2048; i += kPickThreads) hist[i] = 0;
-        __syncthreads();
-        for (uint32_t g = tid; g < a.groups; g += kPickThreads) {
-            const uint32_t o = order_of(mx[g]);
-            if (round == 0) atomicAdd(hist + (o >> 21), 1u);
-            else if ((o >> 21) == prefix) atomicAdd(hist + ((o >> 10) & 2047u), 1u);
-        }
-        __syncthreads();
-        // thread t owns the bins 2047 - 8 t down to 2040 - 8 t
-        uint32_t own = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) own += hist[2047 - 8 * tid - i];
-        uint32_t x = own;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) sums[warp] = x;
-        __syncthreads();
-        uint32_t above = x - own;
-        for (int w = 0; w < warp; ++w) above += sums[w];
-        if (above < want && above + own >= want) {
-            uint32_t b = 2047 - 8 * tid;
-            while (above + hist[b] < want) above += hist[b--];
-            bin_sm = b;
-            rest_sm = want - above;
-        }
-        __syncthreads();
-        prefix = round == 0 ? bin_sm : (prefix << 11 | bin_sm);
-        want = rest_sm;
-        __syncthreads();
-    }
-    const float A = value_of(prefix << 10);
     const float X = __uint_as_float(a.stat[1]) * sx;
     const float m = pq.y * X * (1.0f / 1024 + 1.0f / 8192) + sqrtf(float(a.dim)) * (pq.y + X) * (1.0f / 16777216);
-    const float least = A - 2.0f * m, fine = A - m;
-    const uint32_t ragged = a.n % kXmGroup ? uint32_t(a.n / kXmGroup) : kFull;
-    for (uint32_t g = tid; g < a.groups; g += kPickThreads)
-        if (mx[g] >= least || g == ragged) {
-            const uint32_t at = atomicAdd(&n_list, 1u);
-            if (at < kPickGroups) list[at] = g;
-        }
-    __syncthreads();
-    const uint32_t groups = n_list;
-    if (groups > kPickGroups || !(A > -INFINITY)) {
-        if (tid == 0) a.flags[q] = 1;
-        return;
+    // The k-th largest of the threads' own maxima (256 of them, k <= 128) bounds A from below: A is found among the few
+    // maxima that reach it, and what reaches A - 2 m is listed.  (A radix selection over all maxima spent its time in
+    // atomics on few bins.)
+    const float4* mx4 = reinterpret_cast<const float4*>(mx);
+    float top = -INFINITY;
+#pragma unroll 4
+    for (uint32_t g = tid; g < a.groups / 4; g += kPickThreads) {
+        const float4 v = __ldg(mx4 + g);
+        top = fmaxf(fmaxf(top, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
     }
+    tops[tid] = top;
+    __syncthreads();
+    {
+        uint32_t above = 0;
+#pragma unroll 8
+        for (uint32_t i = 0; i < kPickThreads; ++i) above += tops[i] > top || (tops[i] == top && i < tid);
+        if (above == a.k - 1) kth = top;
+    }
+    __syncthreads();
+    // (the ragged group, whose maximum is -inf, joins the second list)
+    const uint32_t ragged = a.n % kXmGroup ? uint32_t(a.n / kXmGroup) : kFull;
+    float low = kth;
+    for (int round = 0; round < 2; ++round) {
+#pragma unroll 4
+        for (uint32_t g4 = tid; g4 < a.groups / 4; g4 += kPickThreads) {
+            const float4 v = __ldg(mx4 + g4);
+            const float w[4] = {v.x, v.y, v.z, v.w};
+            if (fmaxf(fmaxf(w[0], w[1]), fmaxf(w[2], w[3])) >= low || (round == 1 && g4 == ragged / 4)) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (w[i] >= low || (round == 1 && g4 * 4 + i == ragged)) {
+                        const uint32_t at = atomicAdd(&n_list, 1u);
+                        if (at < kPickGroups) {
+                            list[at] = g4 * 4 + i;
+                            list_max[at] = w[i];
+                        }
+                    }
+            }
+        }
+        __syncthreads();
+        const uint32_t listed = n_list;
+        if (listed > kPickGroups || !(low > -INFINITY)) {
+            if (tid == 0) a.flags[q] = 1;
+            return;
+        }
+        if (round == 0) {  // A: the k-th of them
+            for (uint32_t e = tid; e < listed; e += kPickThreads) {
+                const float v = list_max[e];
+                uint32_t above = 0;
+#pragma unroll 8
+                for (uint32_t i = 0; i < listed; ++i) above += list_max[i] > v || (list_max[i] == v && i < e);
+                if (above == a.k - 1) kth = v;
+            }
+            __syncthreads();
+            low = kth - 2.0f * m;
+            if (tid == 0) n_list = 0;
+            __syncthreads();
+        }
+    }
+    const uint32_t groups = n_list;
+    const float fine = kth - m;
     const float s = sx * pq.x;
     for (uint32_t i = warp; i < groups; i += kPickThreads / 32) {
         const uint64_t id = uint64_t(list[i]) * kXmGroup + lane;
         if (id < a.n) {
             const float* x = a.base + id * a.dim;
             float dot = 0.0f;
-            if (a.vec4) {
-#pragma unroll 8
-                for (int d = 0; d < a.dim; d += 4) {
-                    const float4 u = *reinterpret_cast<const float4*>(qv + d), v = __ldg(reinterpret_cast<const float4*>(x + d));
-                    dot = __fadd_rn(dot, __fmul_rn(u.x, v.x));
-                    dot = __fadd_rn(dot, __fmul_rn(u.y, v.y));
-                    dot = __fadd_rn(dot, __fmul_rn(u.z, v.z));
-                    dot = __fadd_rn(dot, __fmul_rn(u.w, v.w));
+            if (a.vec8) {  // whole sectors: half the requests of 16-byte loads, whose second halves mostly missed L1 again
+#pragma unroll 1
+                for (int d0 = 0; d0 < a.dim; d0 += 16) {
+                    float v[16];
+                    load_sector(v, x + d0);
+                    if (d0 + 8 < a.dim) load_sector(v + 8, x + d0 + 8);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 u = *reinterpret_cast<const float4*>(qv + d0 + 4 * c);
+                        if (c < 2 || d0 + 8 < a.dim) {
+                            dot = __fadd_rn(dot, __fmul_rn(u.x, v[4 * c]));
+                            dot = __fadd_rn(dot, __fmul_rn(u.y, v[4 * c + 1]));
+                            dot = __fadd_rn(dot, __fmul_rn(u.z, v[4 * c + 2]));
+                            dot = __fadd_rn(dot, __fmul_rn(u.w, v[4 * c + 3]));
+                        }
+                    }
+                }
+            } else if (a.vec4) {
+// a lane reads 64 bytes of its vector at once: a sector's two halves are then asked for together
+#pragma unroll 1
+                for (int d0 = 0; d0 < a.dim; d0 += 16) {
+                    float4 v[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[c] = d0 + 4 * c < a.dim ? __ldg(reinterpret_cast<const float4*>(x + d0) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float4 u = *reinterpret_cast<const float4*>(qv + d0 + 4 * c);  // (zeros past the last dimension)
+                        if (d0 + 4 * c < a.dim) {
+                            dot = __fadd_rn(dot, __fmul_rn(u.x, v[c].x));
+                            dot = __fadd_rn(dot, __fmul_rn(u.y, v[c].y));
+                            dot = __fadd_rn(dot, __fmul_rn(u.z, v[c].z));
+                            dot = __fadd_rn(dot, __fmul_rn(u.w, v[c].w));
+                        }
+                    }
                 }
             } else {
                 for (int d = 0; d < a.dim; ++d) dot = __fadd_rn(dot, __fmul_rn(qv[d], __ldg(x + d)));
@@ -437,10 +493,10 @@ __global__ void __launch_bounds__(kPickThreads) exact_pick_kernel(PickArgs a) {
 
 }  // namespace
 
-// The filter pays for its passes over the base (0.1 ms at 500k x 128) from some 64 queries on; it needs several groups per
-// result to bound the k-th best from.
+// Needs several groups per result to bound the k-th best from; below 16,384 vectors the launches cost more than the plain
+// kernel.  (4 queries on 20k / 300k x 128: 109 / 485 us on the plain kernel, 64 queries here: 75 / 167 us.)
 bool exact_mma_supported(const cphnsw_b200_index* h, uint64_t n, uint64_t nq, uint32_t k) {
-    return h->dim <= 128 && nq >= 64 && n >= 16384 && n < 0x80000000ull && n / kXmGroup >= 4ull * k && nq < 0x7fffffffull;
+    return h->dim <= 128 && n >= 16384 && n < 0x80000000ull && n / kXmGroup >= 4ull * k && nq < 0x7fffffffull;
 }
 
 // Writes the results of all queries but the flagged ones; flags uint8[nq] (device).
@@ -505,6 +561,7 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
         b.k = k;
         b.dim = dim;
         b.vec4 = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(d_base) & 15) == 0 ? 1 : 0;
+        b.vec8 = (dim & 7) == 0 && (reinterpret_cast<uintptr_t>(d_base) & 31) == 0 ? 1 : 0;
         b.ids = d_ids + q0 * k;
         b.dist = d_dist + q0 * k;
         b.flags = d_flags + q0;

@@ -20,19 +20,46 @@ def exact(cp, base, q, k):
     return idx, idx.exact_search_batch(q, k)
 
 
-def plain(idx, q, k):
-    """Fewer than 64 queries a call: the plain kernel."""
-    out = [idx.exact_search_batch(q[i:i + 50], k) for i in range(0, q.shape[0], 50)]
-    return np.concatenate([o[0] for o in out]), np.concatenate([o[1] for o in out])
+def cpu(base, q, k):
+    """The k smallest (0 - dot, id) of fp32 sums in d order."""
+    with np.errstate(all="ignore"):
+        dots = np.zeros((q.shape[0], base.shape[0]), np.float32)
+        for d in range(base.shape[1]):
+            dots += q[:, d:d + 1] * base[:, d][None, :]
+        dist = np.float32(0) - dots
+    part = np.argpartition(dist, k, axis=1)[:, :k]
+    worst = np.take_along_axis(dist, part, 1).max(axis=1)
+    ids = np.empty((q.shape[0], k), np.uint32)
+    for i in range(q.shape[0]):
+        c = np.flatnonzero(dist[i] <= worst[i])
+        ids[i] = c[np.argsort(dist[i][c], kind="stable")[:k]]
+    return ids, np.take_along_axis(dist, ids.astype(np.int64), 1)
+
+
+def plain(base, q, k):
+    """The plain kernel on pieces too small for the filter, joined."""
+    ids, dist = [], []
+    for r in range(0, base.shape[0], 16000):
+        _, (i, d) = exact(cp_module(), base[r:r + 16000], q, k)
+        ids.append(i.astype(np.int64) + r)
+        dist.append(d)
+    ids, dist = np.concatenate(ids, 1), np.concatenate(dist, 1)
+    order = np.lexsort((ids, dist), axis=1)[:, :k]
+    return np.take_along_axis(ids, order, 1).astype(np.uint32), np.take_along_axis(dist, order, 1)
+
+
+def cp_module():
+    import cphnsw_b200
+    return cphnsw_b200
 
 
 # groups of 32 vectors, tiles of 256 vectors and 256 queries, dims padded to 16; the least sizes the filter takes
-@pytest.mark.parametrize("n,nq,dim,k", [(16384, 64, 128, 1), (16385, 257, 128, 10), (20011, 100, 96, 100), (33000, 300, 50, 32),
+@pytest.mark.parametrize("n,nq,dim,k", [(16384, 1, 128, 1), (16385, 257, 128, 10), (20011, 100, 96, 100), (33000, 300, 50, 32),
                                         (16639, 64, 17, 64), (40000, 513, 3, 10), (70001, 200, 128, 128)])
-def test_filter_equals_plain_kernel(cp, n, nq, dim, k):
+def test_filter_equals_cpu_loop(cp, n, nq, dim, k):
     base, q = synthetic.gaussian_mixture(n, nq, dim, max(1, n // 1000), 0.3, n + k)
-    idx, (ids, dist) = exact(cp, base, q, k)
-    wi, wd = plain(idx, q, k)
+    _, (ids, dist) = exact(cp, base, q, k)
+    wi, wd = cpu(base, q, k)
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
 
 
@@ -62,19 +89,6 @@ def test_awkward_values(cp, kind):
     if kind == "negative":  # all products negative
         base, q = -np.abs(base), np.abs(q)
     with np.errstate(all="ignore"):
-        idx, (ids, dist) = exact(cp, base, q, k)
-        wi, wd = plain(idx, q, k)
+        _, (ids, dist) = exact(cp, base, q, k)
+        wi, wd = plain(base, q, k)
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd, equal_nan=True)
-
-
-def test_filter_equals_cpu_loop(cp):
-    import oracle
-    base, q = synthetic.gaussian_sphere(16500, 64, 40, 9)
-    _, (ids, dist) = exact(cp, base, q, 20)
-    dots = np.zeros((64, base.shape[0]), np.float32)
-    for d in range(40):
-        dots = dots + q[:, d:d + 1] * base[:, d][None, :]
-    order = np.lexsort((np.broadcast_to(np.arange(base.shape[0]), dots.shape), np.float32(0) - dots), axis=1)[:, :20]
-    assert np.array_equal(ids, order.astype(np.uint32))
-    assert np.array_equal(dist, np.take_along_axis(np.float32(0) - dots, order, 1))
-    assert np.array_equal(oracle.ground_truth(q, base, 20), ids)
