@@ -182,7 +182,7 @@ struct cphnsw_b200_index {
 
     std::vector<int8_t> signs;  // host [K][3][P]
     cpb::DevBuf d_signs;        // float [K][3][P], +-1 with the FHT convention folded into layers 1,2
-    cpb::DevBuf d_signbits;     // padded dim 1024 only: the same diagonals bit-packed, uint32 [K][3][32]
+    cpb::DevBuf d_signbits;     // padded dims 256, 512, 1024: the same diagonals bit-packed, uint32 [K][3][32]
     // uint32 words: 0 status of bounded device waits, 1 query counter of a search launch, 2 "an adjacency
     // row repeats an id", 4-5 frontier sizes of the connectivity BFS, 6-7 counters of the reverse-edge pass
     cpb::DevBuf d_status;

@@ -15,10 +15,10 @@
 //     (and the sign of the rotated output), applied here through `flip_mask` = W-1.
 //
 // Two kernels:
-//   encode_p128_kernel   padded dim 128 (d in 65..128): one thread owns one vector, the whole
-//                        128-point transform lives in registers (no shuffles, no barriers in the
+//   encode_thread_kernel padded dims 32, 64 and 128 (d in 17..128): one thread owns one vector, the whole
+//                        transform lives in registers (no shuffles, no barriers in the
 //                        inner loop); the bound is the fp32 add pipe.
-//   encode_warp_kernel   padded dims 32, 64, 256, 512: one warp per vector, P/32 consecutive elements per lane,
+//   encode_warp_kernel   padded dims 256 and 512: one warp per vector, P/32 consecutive elements per lane,
 //                        low stages in registers, high stages by shuffles.
 //   encode_generic_kernel any other power-of-two padded dim: one warp owns one vector in shared memory.
 #include "common.cuh"
@@ -26,12 +26,12 @@
 namespace cpb {
 namespace {
 
-constexpr int kP128 = 128;
 constexpr int kTileVecs = 128;          // vectors per block = threads per block
-// Padded row of the staged tile: 64-bit reads of 16 threads hit distinct banks.  (Measured and dropped with scalar
-// arithmetic: the diagonal applied as a sign-bit XOR on the integer pipe, 3.883 ms per 1M vectors against 3.835 ms; the
-// diagonal folded into every stage as block multipliers, 3.894 ms.)
-constexpr int kTileStride = kP128 + 2;
+// Padded row of the staged tile: 64-bit reads of 16 threads hit distinct banks.  (Measured and dropped at
+// P = 128: the diagonal applied as a sign-bit XOR on the integer pipe, which the argmax loads already, 3.81 ms per 1M
+// vectors against 3.56 ms; the diagonal folded into every stage as block multipliers, 2 % slower.)
+template <int P>
+constexpr int kTileStride = P + 2;
 
 // ---- packed fp32 pairs (two IEEE operations per instruction, each rounded as the scalar one) -----------------------
 // The transform is bound by fp32 adds; packing leaves the add pipe as busy but halves the issue slots they take, which
@@ -73,12 +73,21 @@ __device__ __forceinline__ void butterfly_pairs(f32x2 (&v)[N]) {
     }
 }
 
-// D then H on 128 values held as 64 pairs of neighbours.  `sg` points at 128 +-1 floats in shared memory, read by
+template <int H, int N>
+__device__ __forceinline__ void butterfly_stages(f32x2 (&v)[N]) {
+    if constexpr (H < N) {
+        butterfly_pairs<H>(v);
+        butterfly_stages<2 * H>(v);
+    }
+}
+
+// D then H on P values held as pairs of neighbours.  `sg` points at P +-1 floats in shared memory, read by
 // every thread at the same address (broadcast).  The products with +-1 are exact.
-__device__ __forceinline__ void diag_fht128(f32x2 (&v)[kP128 / 2], const float* __restrict__ sg) {
+template <int P>
+__device__ __forceinline__ void diag_fht(f32x2 (&v)[P / 2], const float* __restrict__ sg) {
     const ulonglong2* s2 = reinterpret_cast<const ulonglong2*>(sg);
 #pragma unroll
-    for (int c = 0; c < kP128 / 4; ++c) {
+    for (int c = 0; c < P / 4; ++c) {
         const ulonglong2 s = s2[c];
         float a, b;
         unpack2(mul2(v[2 * c], s.x), a, b);
@@ -86,22 +95,18 @@ __device__ __forceinline__ void diag_fht128(f32x2 (&v)[kP128 / 2], const float* 
         unpack2(mul2(v[2 * c + 1], s.y), a, b);
         v[2 * c + 1] = pack2(__fadd_rn(a, b), __fsub_rn(a, b));
     }
-    butterfly_pairs<1>(v);
-    butterfly_pairs<2>(v);
-    butterfly_pairs<4>(v);
-    butterfly_pairs<8>(v);
-    butterfly_pairs<16>(v);
-    butterfly_pairs<32>(v);
+    butterfly_stages<1>(v);
 }
 
 // Lowest-index argmax of |v| by a left-biased tournament: the right operand wins only when it is
 // strictly larger, so among equal magnitudes the lowest index survives every round
 // (same answer as the strict `>` scan of cp_encoder.hpp:82-88).
-__device__ __forceinline__ void argmax128(const f32x2 (&v)[kP128 / 2], float& win, int& idx) {
-    float w[64];
-    int id[64];
+template <int P>
+__device__ __forceinline__ void argmax_abs(const f32x2 (&v)[P / 2], float& win, int& idx) {
+    float w[P / 2];
+    int id[P / 2];
 #pragma unroll
-    for (int j = 0; j < 64; ++j) {
+    for (int j = 0; j < P / 2; ++j) {
         float a, b;
         unpack2(v[j], a, b);
         bool r = fabsf(b) > fabsf(a);
@@ -109,7 +114,7 @@ __device__ __forceinline__ void argmax128(const f32x2 (&v)[kP128 / 2], float& wi
         id[j] = r ? 2 * j + 1 : 2 * j;
     }
 #pragma unroll
-    for (int n = 32; n >= 1; n >>= 1) {
+    for (int n = P / 4; n >= 1; n >>= 1) {
 #pragma unroll
         for (int j = 0; j < n; ++j) {
             bool r = fabsf(w[2 * j + 1]) > fabsf(w[2 * j]);
@@ -129,16 +134,19 @@ __device__ __forceinline__ uint32_t component_of(float win, int idx, int flip_ma
     return (uint32_t(idx) << 1) | (neg ? 1u : 0u);
 }
 
-// QUERY = true additionally writes the rotated vectors and winning magnitudes (CPQuery).
-template <typename CompT, bool QUERY>
-__global__ void __launch_bounds__(kTileVecs, QUERY ? 2 : 3)
-encode_p128_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb /* rotations per block */,
-                   const float* __restrict__ signs /*[K][3][128]*/, int flip_mask,
+// QUERY = true additionally writes the rotated vectors and winning magnitudes (CPQuery).  A vector a thread at padded
+// dims 32 and 64 too: with a warp a vector the shuffles of the high stages (one an element) were the bound, 300k x 64 with
+// K = 32 took 2.09 ms and takes 0.50, 300k x 32 took 1.64 and takes 0.24.  (Measured and dropped at P = 128: the second
+// sign product in the fma of the first butterfly, 3.65 ms per 1M against 3.56.)
+template <typename CompT, bool QUERY, int P>
+__global__ void __launch_bounds__(kTileVecs, P == 128 ? (QUERY ? 2 : 3) : (P == 64 ? 5 : 8))
+encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb /* rotations per block */,
+                   const float* __restrict__ signs /*[K][3][P]*/, int flip_mask,
                    CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
     extern __shared__ float smem[];
-    float* tile = smem;                                                 // [kTileVecs][kTileStride]
-    float* sign_sm = tile + kTileVecs * kTileStride;                              // [2][3][128], double buffer
-    CompT* code_tile = reinterpret_cast<CompT*>(sign_sm + 2 * 3 * kP128);         // [kTileVecs][rotations of this block]
+    float* tile = smem;                                                 // [kTileVecs][kTileStride<P>]
+    float* sign_sm = tile + kTileVecs * kTileStride<P>;                              // [2][3][P], double buffer
+    CompT* code_tile = reinterpret_cast<CompT*>(sign_sm + 2 * 3 * P);         // [kTileVecs][rotations of this block]
     const int r0 = blockIdx.y * rpb, r1 = min(K, r0 + rpb), nr = r1 - r0;
 
     const uint64_t row0 = uint64_t(blockIdx.x) * kTileVecs;
@@ -148,56 +156,58 @@ encode_p128_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int 
     // stage the tile: coalesced 128-bit loads when rows are 16-byte aligned, else 32-bit loads
     const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     for (int r = warp; r < kTileVecs; r += kTileVecs / 32) {
-        float* dst = tile + r * kTileStride;
+        float* dst = tile + r * kTileStride<P>;
         if (r < rows) {
             const float* src = x + (row0 + r) * uint64_t(dim);
             if (vec4) {
-                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (4 * lane < dim) q = __ldg(reinterpret_cast<const float4*>(src) + lane);
-                dst[4 * lane] = q.x;
-                dst[4 * lane + 1] = q.y;
-                dst[4 * lane + 2] = q.z;
-                dst[4 * lane + 3] = q.w;
+                if (P == 128 || 4 * lane < P) {
+                    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (4 * lane < dim) q = __ldg(reinterpret_cast<const float4*>(src) + lane);
+                    dst[4 * lane] = q.x;
+                    dst[4 * lane + 1] = q.y;
+                    dst[4 * lane + 2] = q.z;
+                    dst[4 * lane + 3] = q.w;
+                }
             } else {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < P / 32; ++c) {
                     int i = lane + 32 * c;
                     dst[i] = i < dim ? __ldg(src + i) : 0.0f;
                 }
             }
         } else {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) dst[lane + 32 * c] = 0.0f;
+            for (int c = 0; c < P / 32; ++c) dst[lane + 32 * c] = 0.0f;
         }
     }
     // the three diagonals of one rotation are staged in shared memory one rotation ahead
     const int t = threadIdx.x;
-    if (t < 3 * kP128 / 4)
-        reinterpret_cast<float4*>(sign_sm)[t] = __ldg(reinterpret_cast<const float4*>(signs + size_t(r0) * 3 * kP128) + t);
+    if (t < 3 * P / 4)
+        reinterpret_cast<float4*>(sign_sm)[t] = __ldg(reinterpret_cast<const float4*>(signs + size_t(r0) * 3 * P) + t);
     __syncthreads();
 
-    const f32x2* mine = reinterpret_cast<const f32x2*>(tile + t * kTileStride);
+    const f32x2* mine = reinterpret_cast<const f32x2*>(tile + t * kTileStride<P>);
     const uint64_t row = row0 + t;
     for (int r = r0; r < r1; ++r) {
-        if (r + 1 < r1 && t < 3 * kP128 / 4)
-            reinterpret_cast<float4*>(sign_sm + ((r + 1 - r0) & 1) * 3 * kP128)[t] =
-                __ldg(reinterpret_cast<const float4*>(signs + size_t(r + 1) * 3 * kP128) + t);
-        f32x2 v[kP128 / 2];
+        if (r + 1 < r1 && t < 3 * P / 4)
+            reinterpret_cast<float4*>(sign_sm + ((r + 1 - r0) & 1) * 3 * P)[t] =
+                __ldg(reinterpret_cast<const float4*>(signs + size_t(r + 1) * 3 * P) + t);
+        f32x2 v[P / 2];
 #pragma unroll
-        for (int i = 0; i < kP128 / 2; ++i) v[i] = mine[i];
-        const float* sg = sign_sm + ((r - r0) & 1) * 3 * kP128;
+        for (int i = 0; i < P / 2; ++i) v[i] = mine[i];
+        const float* sg = sign_sm + ((r - r0) & 1) * 3 * P;
 #pragma unroll 1
-        for (int layer = 0; layer < 3; ++layer) diag_fht128(v, sg + layer * kP128);
+        for (int layer = 0; layer < 3; ++layer) diag_fht<P>(v, sg + layer * P);
         float win;
         int idx;
-        argmax128(v, win, idx);
+        argmax_abs<P>(v, win, idx);
         code_tile[t * nr + (r - r0)] = CompT(component_of(win, idx, flip_mask));
         if (QUERY && t < rows) {
             if (mags) mags[row * K + r] = fabsf(win);
             if (rotated) {
-                float4* out = reinterpret_cast<float4*>(rotated + (row * K + r) * kP128);
+                float4* out = reinterpret_cast<float4*>(rotated + (row * K + r) * P);
 #pragma unroll
-                for (int c = 0; c < kP128 / 4; ++c) {
+                for (int c = 0; c < P / 4; ++c) {
                     float a0, a1, a2, a3;
                     unpack2(v[2 * c], a0, a1);
                     unpack2(v[2 * c + 1], a2, a3);
@@ -346,14 +356,15 @@ encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int
     }
 }
 
-// ---- padded dims 32, 64, 256, 512: one warp per vector, E = P / 32 consecutive elements per lane -------------
+// ---- padded dims 256, 512: one warp per vector, E = P / 32 consecutive elements per lane ----------------------
 // Lane L holds elements E*L .. E*L + E - 1.  Stages h < E pair elements of one lane (registers), stages
 // h = E * 2^t pair lane L with lane L ^ 2^t (one shuffle per element): the lower index computes x + y, the upper
 // x - y with x the lower element, in ascending h like the reference's loop (fht.hpp:56-69), so the result is
-// bit-identical.  Nothing goes through shared memory.
+// bit-identical.  Nothing goes through shared memory.  The diagonals come bit-packed, a word per lane and layer (a set
+// bit negates): as floats they were E scattered loads a lane (100k x 500: 11.5 ms).
 template <typename CompT, bool QUERY, int E>
 __global__ void __launch_bounds__(128)
-encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb, const float* __restrict__ signs /*[K][3][P]*/,
+encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb, const uint32_t* __restrict__ signbits /*[K][3][32]*/,
                    int flip_mask, CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
     constexpr int P = 32 * E;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -367,11 +378,12 @@ encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int 
             float v[E];
 #pragma unroll
             for (int j = 0; j < E; ++j) v[j] = in[j];
-            const float* sg = signs + size_t(r) * 3 * P + first;
+            const uint32_t* sb = signbits + size_t(r) * 3 * 32 + lane;
 #pragma unroll 1
             for (int layer = 0; layer < 3; ++layer) {
+                const uint32_t word = __ldg(sb + layer * 32);
 #pragma unroll
-                for (int j = 0; j < E; ++j) v[j] = __fmul_rn(v[j], __ldg(sg + layer * P + j));
+                for (int j = 0; j < E; ++j) v[j] = __uint_as_float(__float_as_uint(v[j]) ^ ((word << (31 - j)) & 0x80000000u));
 #pragma unroll
                 for (int h = 1; h < E; h <<= 1) {
 #pragma unroll
@@ -529,28 +541,33 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     const float* signs = h->d_signs.as<float>();
     LaunchTimer timer(h, kKernelEncode, st);
 
-    if (P == kP128) {
-        size_t smem = size_t(kTileVecs) * kTileStride * sizeof(float) + size_t(2) * 3 * kP128 * sizeof(float) +
-                      size_t(kTileVecs) * K * h->comp_bytes;
+    if (P == 32 || P == 64 || P == 128) {
         const uint64_t tiles = (n + kTileVecs - 1) / kTileVecs;
-        const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * 6, K);
-        smem -= size_t(kTileVecs) * (K - rpb) * h->comp_bytes;
+        const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * (P == 128 ? 6 : 12), K);
+        const size_t smem = size_t(kTileVecs) * (P + 2) * sizeof(float) + size_t(2) * 3 * P * sizeof(float) + size_t(kTileVecs) * rpb * h->comp_bytes;
         const dim3 grid(unsigned(tiles), unsigned((K + rpb - 1) / rpb));
         const bool query = d_rot || d_mag;
-#define CPB_LAUNCH_P128(T, Q)                                                                              \
+#define CPB_LAUNCH_THREAD(T, Q, PP)                                                                        \
     do {                                                                                                   \
-        CPB_CUDA(allow_max_dynamic_smem(encode_p128_kernel<T, Q>));                                        \
-        encode_p128_kernel<T, Q><<<grid, kTileVecs, smem, st>>>(d_x, n, dim, K, rpb, signs, flip_mask,           \
-                                                               (T*)d_codes, d_rot, d_mag);                  \
+        CPB_CUDA(allow_max_dynamic_smem(encode_thread_kernel<T, Q, PP>));                                  \
+        encode_thread_kernel<T, Q, PP><<<grid, kTileVecs, smem, st>>>(d_x, n, dim, K, rpb, signs, flip_mask, \
+                                                                     (T*)d_codes, d_rot, d_mag);            \
+    } while (0)
+#define CPB_LAUNCH_THREAD_P(T, Q)                       \
+    do {                                                \
+        if (P == 32) CPB_LAUNCH_THREAD(T, Q, 32);       \
+        else if (P == 64) CPB_LAUNCH_THREAD(T, Q, 64);  \
+        else CPB_LAUNCH_THREAD(T, Q, 128);              \
     } while (0)
         if (h->comp_bytes == 1) {
-            if (query) CPB_LAUNCH_P128(uint8_t, true);
-            else CPB_LAUNCH_P128(uint8_t, false);
+            if (query) CPB_LAUNCH_THREAD_P(uint8_t, true);
+            else CPB_LAUNCH_THREAD_P(uint8_t, false);
         } else {
-            if (query) CPB_LAUNCH_P128(uint16_t, true);
-            else CPB_LAUNCH_P128(uint16_t, false);
+            if (query) CPB_LAUNCH_THREAD_P(uint16_t, true);
+            else CPB_LAUNCH_THREAD_P(uint16_t, false);
         }
-#undef CPB_LAUNCH_P128
+#undef CPB_LAUNCH_THREAD_P
+#undef CPB_LAUNCH_THREAD
     } else if (P == kP1024 && h->d_signbits.p) {
         const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + kWarps1024 - 1) / kWarps1024;
@@ -567,18 +584,17 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
             else CPB_LAUNCH_P1024(uint16_t, false);
         }
 #undef CPB_LAUNCH_P1024
-    } else if (P == 32 || P == 64 || P == 256 || P == 512) {
+    } else if (P == 256 || P == 512) {
+        const uint32_t* sb = h->d_signbits.as<uint32_t>();
         const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + 3) / 4;
         const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 32, K);
         const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 32 ? blocks : uint64_t(h->sm_count) * 32), unsigned((K + rpb - 1) / rpb));
 #define CPB_LAUNCH_WARP(T, Q, EE) \
-    encode_warp_kernel<T, Q, EE><<<grid, 128, 0, st>>>(d_x, n, dim, K, rpb, signs, flip_mask, (T*)d_codes, d_rot, d_mag)
+    encode_warp_kernel<T, Q, EE><<<grid, 128, 0, st>>>(d_x, n, dim, K, rpb, sb, flip_mask, (T*)d_codes, d_rot, d_mag)
 #define CPB_LAUNCH_WARP_E(T, Q)                      \
     do {                                             \
-        if (P == 32) CPB_LAUNCH_WARP(T, Q, 1);       \
-        else if (P == 64) CPB_LAUNCH_WARP(T, Q, 2);  \
-        else if (P == 256) CPB_LAUNCH_WARP(T, Q, 8); \
+        if (P == 256) CPB_LAUNCH_WARP(T, Q, 8);      \
         else CPB_LAUNCH_WARP(T, Q, 16);              \
     } while (0)
         if (h->comp_bytes == 1) {
