@@ -75,7 +75,7 @@ int upload_signs(cphnsw_b200_index* h) {
         // bit-packed copy for the kernels with a warp per vector (a set bit negates): word w, bit b <-> element
         // P/32 * w + b; at 1024 layers 1 and 2 in the column layout, word l, bit j <-> element 32*j + l
         const size_t E = P / 32;
-        std::vector<uint32_t> bits(K * 3 * 32, 0u);
+        std::vector<uint32_t> bits(K * (kWarpSignWords + (P < 1024 ? 3 * P / 32 : 0)), 0u);
         for (size_t r = 0; r < K; ++r)
             for (size_t l = 0; l < 3; ++l)
                 for (size_t i = 0; i < P; ++i)
@@ -83,6 +83,18 @@ int upload_signs(cphnsw_b200_index* h) {
                         if (l == 0 || P != 1024) bits[(r * 3 + l) * 32 + i / E] |= 1u << (i % E);
                         else bits[(r * 3 + l) * 32 + i % 32] |= 1u << (i / 32);
                     }
+        // behind it the copy for groups of P/128 lanes per vector, four words a lane and layer in the order of the lane's
+        // registers: the element of register e has e's low bits and, of the next bits and the top ones, the lane's index
+        // and the rest of e XOR the lane's index (layer 0: the lane's index on top)
+        const size_t G = P / 128, low = G == 2 ? 6 : 5;
+        uint32_t* group_bits = bits.data() + K * kWarpSignWords;
+        for (size_t row = 0; P < 1024 && row < K * 3; ++row)
+            for (size_t g = 0; g < G; ++g)
+                for (size_t e = 0; e < 128; ++e) {
+                    const size_t turned = (e >> low) ^ g, l = row % 3;
+                    const size_t i = (e & ((size_t(1) << low) - 1)) | (l ? g : turned) << low | (l ? turned : g) << 7;
+                    if (f[row * P + i] < 0.0f) group_bits[(row * G + g) * 4 + e / 32] |= 1u << (e % 32);
+                }
         CPB_TRY(h->d_signbits.reserve(bits.size() * 4));
         CPB_CUDA(cudaMemcpy(h->d_signbits.p, bits.data(), bits.size() * 4, cudaMemcpyHostToDevice));
     }

@@ -18,6 +18,7 @@
 namespace cpb {
 
 constexpr uint32_t kInvalidNode = 0xFFFFFFFFu;
+constexpr uint32_t kWarpSignWords = 96;  // bit-packed diagonals of a rotation, a word per lane and layer
 
 // Device-side status word values raised by kernels (read with cphnsw_b200_check_device_status).
 constexpr uint32_t kStatusOk = 0;
@@ -182,7 +183,7 @@ struct cphnsw_b200_index {
 
     std::vector<int8_t> signs;  // host [K][3][P]
     cpb::DevBuf d_signs;        // float [K][3][P], +-1 with the FHT convention folded into layers 1,2
-    cpb::DevBuf d_signbits;     // padded dims 256, 512, 1024: the same diagonals bit-packed, uint32 [K][3][32]
+    cpb::DevBuf d_signbits;     // padded dims 256, 512, 1024: the same diagonals bit-packed, uint32 [K][3][32]; then, below 1024, [K][3][P/128][4]
     // uint32 words: 0 status of bounded device waits, 1 query counter of a search launch, 2 "an adjacency
     // row repeats an id", 4-5 frontier sizes of the connectivity BFS, 6-7 counters of the reverse-edge pass
     cpb::DevBuf d_status;

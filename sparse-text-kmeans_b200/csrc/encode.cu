@@ -18,8 +18,10 @@
 //   encode_thread_kernel padded dims 32, 64 and 128 (d in 17..128): one thread owns one vector, the whole
 //                        transform lives in registers (no shuffles, no barriers in the
 //                        inner loop); the bound is the fp32 add pipe.
-//   encode_warp_kernel   padded dims 256 and 512: one warp per vector, P/32 consecutive elements per lane,
+//   encode_warp_kernel   padded dims 256 and 512, few vectors: one warp per vector, P/32 consecutive elements per lane,
 //                        low stages in registers, high stages by shuffles.
+//   encode_group_kernel  padded dims 256 and 512, many vectors: 2 or 4 lanes own one vector, 128 elements each; the stages
+//                        across lanes become register stages after an exchange.
 //   encode_generic_kernel any other power-of-two padded dim: one warp owns one vector in shared memory.
 #include "common.cuh"
 
@@ -58,6 +60,11 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
 // butterflies between pairs H apart (elements 2 * H apart)
 template <int H, int N>
@@ -73,11 +80,11 @@ __device__ __forceinline__ void butterfly_pairs(f32x2 (&v)[N]) {
     }
 }
 
-template <int H, int N>
+template <int H, int N, int END = N>
 __device__ __forceinline__ void butterfly_stages(f32x2 (&v)[N]) {
-    if constexpr (H < N) {
+    if constexpr (H < END) {
         butterfly_pairs<H>(v);
-        butterfly_stages<2 * H>(v);
+        butterfly_stages<2 * H, N, END>(v);
     }
 }
 
@@ -441,6 +448,184 @@ encode_warp_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int 
     }
 }
 
+// ---- padded dims 256, 512, many vectors: G = 2, 4 lanes per vector, 128 elements per lane ---------------------------
+// What bounds it is the add pipe, with the shuffles beside it.  With 128 elements a lane only g = log2(G) of the
+// log2(P) stages of a layer reach across lanes.  They become register stages too: a swap of an element bit that the
+// lanes carry with one that the registers carry moves half of the registers, one shuffle for each.
+//   The register of index r (7 bits) holds the element whose low 7 - g bits are r's and whose next g bits, or top g
+// bits, are r's top g bits XOR the lane's index in its group; the lane's index is the other of the two.  So every lane
+// sends the registers whose bit i is set to the lane whose bit i differs, and stores what it gets where it came from:
+// no selects.  In the butterflies over those bits a lane whose bit is set holds the operands the other way round,
+//     v[p] = s v[p] + v[q],  v[q] = v[p] - s v[q],  s = +-1 by lane,
+// which is x + y and x - y with one rounding each, as the reference has them.
+//   A layer starts with the top bits in the lanes (the first) or the middle ones (the later ones, as the layer before
+// left them).  Against a warp a vector with a shuffle for every element and stage across lanes: 100k x 500, K = 32, 4.26 ms
+// -> 2.46; 100k x 256, 2.08 -> 1.13.  (At 1024, eight lanes a vector, 5.9 ms against the transposes' 5.3.)
+template <int G>
+__device__ __forceinline__ void swap_bits(f32x2 (&v)[64]) {
+    constexpr int kSwap = G == 2 ? 1 : 2;
+#pragma unroll
+    for (int i = 0; i < kSwap; ++i) {
+#pragma unroll
+        for (int p = 0; p < 64; ++p)
+            if (p & (64 >> kSwap) << i) {
+                float a, b;
+                unpack2(v[p], a, b);
+                v[p] = pack2(__shfl_xor_sync(0xffffffffu, a, 1 << i), __shfl_xor_sync(0xffffffffu, b, 1 << i));
+            }
+    }
+}
+
+// the g stages over the registers' top bits
+template <int G>
+__device__ __forceinline__ void swapped_stages(f32x2 (&v)[64], int part) {
+    constexpr int kSwap = G == 2 ? 1 : 2;
+#pragma unroll
+    for (int i = 0; i < kSwap; ++i) {
+        const float s = (part >> i & 1) ? -1.0f : 1.0f;
+        const f32x2 plus = pack2(s, s), minus = pack2(-s, -s);
+        const int h = (64 >> kSwap) << i;
+#pragma unroll
+        for (int p = 0; p < 64; ++p)
+            if (!(p & h)) {
+                const f32x2 a = v[p], b = v[p + h];
+                v[p] = fma2(a, plus, b);
+                v[p + h] = fma2(b, minus, a);
+            }
+    }
+}
+
+template <typename CompT, bool QUERY, int G>
+__global__ void __launch_bounds__(kTileVecs, QUERY ? 2 : 3)
+encode_group_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb, const uint4* __restrict__ signbits /*[K][3][G]*/,
+                    int flip_mask, CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
+    constexpr int kSwap = G == 2 ? 1 : 2, kLow = 7 - kSwap, kVecs = kTileVecs / G, kStride = kTileStride<128>;
+    extern __shared__ float smem[];
+    float* tile = smem;                                                     // [kTileVecs][kStride], 128 elements a row
+    CompT* code_tile = reinterpret_cast<CompT*>(tile + kTileVecs * kStride);  // [kVecs][rotations of this block]
+    const int r0 = blockIdx.y * rpb, r1 = min(K, r0 + rpb), nr = r1 - r0;
+    const uint64_t row0 = uint64_t(blockIdx.x) * kVecs;
+    const int rows = int(min(uint64_t(kVecs), n - row0));
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, part = t % G;
+
+    const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
+    for (int r = warp; r < kTileVecs; r += kTileVecs / 32) {
+        float* dst = tile + r * kStride;
+        const int left = r / G < rows ? dim - 128 * (r % G) : 0;  // elements of the vector from this row on
+        const float* src = x + (row0 + r / G) * uint64_t(dim) + 128 * (r % G);
+        if (vec4) {
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (4 * lane < left) q = __ldg(reinterpret_cast<const float4*>(src) + lane);
+            dst[4 * lane] = q.x;
+            dst[4 * lane + 1] = q.y;
+            dst[4 * lane + 2] = q.z;
+            dst[4 * lane + 3] = q.w;
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) dst[lane + 32 * c] = lane + 32 * c < left ? __ldg(src + lane + 32 * c) : 0.0f;
+        }
+    }
+    __syncthreads();
+
+    const f32x2* mine = reinterpret_cast<const f32x2*>(tile + t * kStride);
+    const uint64_t row = row0 + t / G;
+    const uint4* sb = signbits + size_t(r0) * 3 * G + part;
+    uint4 next = __ldg(sb);
+    for (int r = r0; r < r1; ++r) {
+        f32x2 v[64];
+#pragma unroll
+        for (int p = 0; p < 64; ++p) v[p] = mine[p ^ part << (kLow - 1)];
+#pragma unroll 1
+        for (int layer = 0; layer < 3; ++layer) {
+            const uint4 sign = next;
+            sb += G;
+            if (r + 1 < r1 || layer < 2) next = __ldg(sb);
+#pragma unroll
+            for (int p = 0; p < 64; ++p) {
+                const uint32_t word = p < 16 ? sign.x : (p < 32 ? sign.y : (p < 48 ? sign.z : sign.w));
+                float a, b;
+                unpack2(v[p], a, b);
+                a = __uint_as_float(__float_as_uint(a) ^ ((word << (31 - 2 * (p & 15))) & 0x80000000u));
+                b = __uint_as_float(__float_as_uint(b) ^ ((word << (30 - 2 * (p & 15))) & 0x80000000u));
+                v[p] = pack2(__fadd_rn(a, b), __fsub_rn(a, b));
+            }
+            butterfly_stages<1, 64, 1 << (kLow - 1)>(v);
+            if (layer > 0) swap_bits<G>(v);
+            swapped_stages<G>(v, part);
+            swap_bits<G>(v);
+            swapped_stages<G>(v, part);
+        }
+        // the lowest index of the largest magnitude: a left-biased tournament in the order of the element bits, the
+        // sides of the top ones changed in the lanes that hold them the other way round; then across the lanes
+        float best, win;
+        int idx;
+        {
+            float w[64];
+            int id[64];
+#pragma unroll
+            for (int p = 0; p < 64; ++p) {
+                float a, b;
+                unpack2(v[p], a, b);
+                const bool right = fabsf(b) > fabsf(a);
+                w[p] = right ? b : a;
+                id[p] = right ? 2 * p + 1 : 2 * p;
+            }
+#pragma unroll
+            for (int m = 32; m >= 1; m >>= 1) {
+                const bool turned = m <= (64 >> kLow) && (part & (64 >> kLow) / m);
+#pragma unroll
+                for (int p = 0; p < m; ++p) {
+                    const float a = fabsf(w[2 * p]), b = fabsf(w[2 * p + 1]);
+                    const bool right = b > a || (turned && b == a);
+                    w[p] = right ? w[2 * p + 1] : w[2 * p];
+                    id[p] = right ? id[2 * p + 1] : id[2 * p];
+                }
+            }
+            win = w[0], best = fabsf(win);
+            idx = (id[0] & ((1 << kLow) - 1)) | part << kLow | ((id[0] >> kLow) ^ part) << 7;
+        }
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const float ow = __shfl_xor_sync(0xffffffffu, win, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+            if (fabsf(ow) > best || (fabsf(ow) == best && oi < idx)) {
+                best = fabsf(ow);
+                win = ow;
+                idx = oi;
+            }
+        }
+        if (part == 0) code_tile[t / G * nr + (r - r0)] = CompT(component_of(win, idx, flip_mask));
+        if (QUERY) {
+            if (mags && part == 0 && t / G < rows) mags[row * K + r] = best;
+            if (rotated) {
+                swap_bits<G>(v);  // back to 128 consecutive elements a lane
+                if (t / G < rows) {
+                    float4* out = reinterpret_cast<float4*>(rotated + (row * K + r) * uint64_t(128 * G)) + 32 * part;
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) {
+                        float a0, a1, a2, a3;
+                        unpack2(v[2 * c], a0, a1);
+                        unpack2(v[2 * c + 1], a2, a3);
+                        float4 o;
+                        o.x = (__popc((4 * c) & flip_mask) & 1) ? -a0 : a0;
+                        o.y = (__popc((4 * c + 1) & flip_mask) & 1) ? -a1 : a1;
+                        o.z = (__popc((4 * c + 2) & flip_mask) & 1) ? -a2 : a2;
+                        o.w = (__popc((4 * c + 3) & flip_mask) & 1) ? -a3 : a3;
+                        out[c ^ part << (kLow - 2)] = o;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    CompT* dst = codes + row0 * uint64_t(K);
+    if (nr == K) {
+        for (int i = t; i < rows * K; i += kTileVecs) dst[i] = code_tile[i];
+    } else {
+        for (int i = t; i < rows * nr; i += kTileVecs) dst[uint64_t(i / nr) * K + r0 + i % nr] = code_tile[i];
+    }
+}
+
 // ---- generic padded dim: one warp per vector, transform in shared memory ----------------------
 template <typename CompT>
 __global__ void encode_generic_kernel(const float* __restrict__ x, uint64_t n, int dim, int P, int K,
@@ -540,13 +725,17 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     const int flip_mask = w - 1;
     const float* signs = h->d_signs.as<float>();
     LaunchTimer timer(h, kKernelEncode, st);
+    const bool query = d_rot || d_mag;
+    // 256 and 512: lanes in groups from two to four blocks an SM on; fewer vectors leave most of a group's long chain of
+    // instructions exposed (one of 256: 10.7 us against 6.6; 1,000: 31 against 29; 500 of 512: 33 against 41).  Rotated
+    // vectors of 256 stay with the warp kernel, whose stores are whole lines (2,000: 58 us against 65).
+    const uint64_t group_tiles = P == 512 || (P == 256 && !query) ? (n * (P / 128) + kTileVecs - 1) / kTileVecs : 0;
 
     if (P == 32 || P == 64 || P == 128) {
         const uint64_t tiles = (n + kTileVecs - 1) / kTileVecs;
         const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * (P == 128 ? 6 : 12), K);
         const size_t smem = size_t(kTileVecs) * (P + 2) * sizeof(float) + size_t(2) * 3 * P * sizeof(float) + size_t(kTileVecs) * rpb * h->comp_bytes;
         const dim3 grid(unsigned(tiles), unsigned((K + rpb - 1) / rpb));
-        const bool query = d_rot || d_mag;
 #define CPB_LAUNCH_THREAD(T, Q, PP)                                                                        \
     do {                                                                                                   \
         CPB_CUDA(allow_max_dynamic_smem(encode_thread_kernel<T, Q, PP>));                                  \
@@ -569,7 +758,6 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
 #undef CPB_LAUNCH_THREAD_P
 #undef CPB_LAUNCH_THREAD
     } else if (P == kP1024 && h->d_signbits.p) {
-        const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + kWarps1024 - 1) / kWarps1024;
         const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 16, K);
         const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 16 ? blocks : uint64_t(h->sm_count) * 16), unsigned((K + rpb - 1) / rpb));
@@ -584,9 +772,31 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
             else CPB_LAUNCH_P1024(uint16_t, false);
         }
 #undef CPB_LAUNCH_P1024
+    } else if (group_tiles * K >= uint64_t(h->sm_count) * (P == 256 ? 4 : 2)) {
+        const int vecs = kTileVecs / (P / 128);
+        const uint64_t tiles = group_tiles;
+        const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * 6, K);
+        const size_t smem = size_t(kTileVecs) * kTileStride<128> * sizeof(float) + size_t(vecs) * rpb * h->comp_bytes;
+        const dim3 grid(unsigned(tiles), unsigned((K + rpb - 1) / rpb));
+        const uint4* sb = h->d_signbits.as<uint4>() + kWarpSignWords / 4 * K;
+#define CPB_LAUNCH_GROUP(T, Q, G)                                                                       \
+    do {                                                                                                \
+        CPB_CUDA(allow_max_dynamic_smem(encode_group_kernel<T, Q, G>));                                 \
+        encode_group_kernel<T, Q, G><<<grid, kTileVecs, smem, st>>>(d_x, n, dim, K, rpb, sb, flip_mask, \
+                                                                    (T*)d_codes, d_rot, d_mag);         \
+    } while (0)
+#define CPB_LAUNCH_GROUP_P(T)                       \
+    do {                                            \
+        if (P == 256) CPB_LAUNCH_GROUP(T, false, 2);  \
+        else if (query) CPB_LAUNCH_GROUP(T, true, 4); \
+        else CPB_LAUNCH_GROUP(T, false, 4);         \
+    } while (0)
+        if (h->comp_bytes == 1) CPB_LAUNCH_GROUP_P(uint8_t);  // binary codes keep the sign bits only
+        else CPB_LAUNCH_GROUP_P(uint16_t);
+#undef CPB_LAUNCH_GROUP_P
+#undef CPB_LAUNCH_GROUP
     } else if (P == 256 || P == 512) {
         const uint32_t* sb = h->d_signbits.as<uint32_t>();
-        const bool query = d_rot || d_mag;
         const uint64_t blocks = (n + 3) / 4;
         const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 32, K);
         const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 32 ? blocks : uint64_t(h->sm_count) * 32), unsigned((K + rpb - 1) / rpb));

@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dim,cb", [(17, 1), (32, 1), (33, 1), (64, 2), (65, 1), (129, 2), (256, 2), (257, 2), (510, 2), (512, 2), (513, 2),
                                     (1023, 2), (1024, 2)])
-@pytest.mark.parametrize("n,K,conv", [(1, 5, 1), (129, 8, 2), (2050, 3, 0)])
+@pytest.mark.parametrize("n,K,conv", [(1, 5, 1), (129, 8, 2), (2050, 19, 0)])
 def test_encode_tiles_match_oracle(oracle, dim, cb, n, K, conv):
     import cphnsw_b200 as cp
     rng = np.random.default_rng(dim + n)
