@@ -11,8 +11,11 @@
 // rotation j' to rank 1" for every j' > j, created in that order, so every rank combination has
 // exactly one derivation and the order is reproducible.
 //
-// One warp per query; the per-rotation ranking, the successor scores and the pool scan are spread
-// over the lanes.
+// One block per query.  What bounds it is a chain of warp-wide maxima: the ranks of a rotation come one after another.
+// The rotations are independent, so kProbeWarps warps rank them side by side, each maximum two warp reductions (all
+// rotations by one warp, five shuffles and compares a maximum, the
+// row read again for each: 1,024 queries, K = 32, 4 probes took 168 us; 24 us now).  The
+// successor scores and the pool scan are spread over the lanes of the first warp.
 #include <cmath>
 
 #include "common.cuh"
@@ -22,6 +25,7 @@ namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kNoParent = 0xffffffffu;
+constexpr int kProbeWarps = 8;
 
 struct ProbeArgs {
     const float* rotated;  // [nq][K][P]
@@ -31,12 +35,11 @@ struct ProbeArgs {
     void* out;             // [nq][T][K] components
 };
 
-template <bool U16>
-__global__ void probe_codes_kernel(ProbeArgs a) {
+template <bool U16, bool NARROW /* P <= 128: a rotation's magnitudes stay in registers */>
+__global__ void __launch_bounds__(kProbeWarps * 32) probe_codes_kernel(ProbeArgs a) {
     extern __shared__ __align__(16) unsigned char pr_smem[];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int K = a.K, P = a.P, T = a.T, V = a.V;
-    // per-block (one warp) shared arrays
     float* cost = reinterpret_cast<float*>(pr_smem);                  // [K][V]
     uint32_t* idx = reinterpret_cast<uint32_t*>(cost + K * V);        // [K][V]
     float* pscore = reinterpret_cast<float*>(idx + K * V);            // [pool_cap]
@@ -48,15 +51,29 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
 
     for (uint32_t q = blockIdx.x; q < a.nq; q += gridDim.x) {
         // ---- rank the coordinates of every rotation: V rounds of "next in (|x| desc, index asc) order"
-        for (int r = 0; r < K; ++r) {
+        for (int r = warp; r < K; r += kProbeWarps) {
             const float* x = a.rotated + (size_t(q) * K + r) * P;
             float prev_a = INFINITY;  // key of the previous winner: everything after it is still eligible
             int prev_i = -1;
             float top = 0.0f;
+            float held[4];
+            if (NARROW) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) held[j] = lane + 32 * j < P ? fabsf(__ldg(x + lane + 32 * j)) : -1.0f;
+            }
             for (int v = 0; v < V; ++v) {
                 float ba = -1.0f;
                 int bi = 0x7fffffff;
-                for (int i = lane; i < P; i += 32) {
+                if (NARROW) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        if (lane + 32 * j == prev_i) held[j] = -1.0f;
+                        if (held[j] > ba) {
+                            ba = held[j];
+                            bi = lane + 32 * j;
+                        }
+                    }
+                } else for (int i = lane; i < P; i += 32) {
                     const float av = fabsf(__ldg(x + i));
                     const bool after_prev = av < prev_a || (av == prev_a && i > prev_i);
                     if (after_prev && (av > ba || (av == ba && i < bi))) {
@@ -64,15 +81,10 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
                         bi = i;
                     }
                 }
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    const float oa = __shfl_xor_sync(kFull, ba, o);
-                    const int oi = __shfl_xor_sync(kFull, bi, o);
-                    if (oa > ba || (oa == ba && oi < bi)) {
-                        ba = oa;
-                        bi = oi;
-                    }
-                }
+                // magnitudes order as their bits; the lowest index among the lanes that hold the largest
+                const uint32_t most = __reduce_max_sync(kFull, ba >= 0.0f ? __float_as_uint(ba) : 0u);
+                bi = min(__reduce_min_sync(kFull, ba >= 0.0f && __float_as_uint(ba) == most ? bi : 0x7fffffff), P - 1);
+                ba = __uint_as_float(most);
                 if (v == 0) top = ba;
                 if (lane == 0) {
                     const float d = __fsub_rn(top, ba);
@@ -83,7 +95,11 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
                 prev_i = bi;
             }
         }
-        __syncwarp();
+        __syncthreads();
+        if (warp != 0) {
+            __syncthreads();  // the first warp is done with the ranks
+            continue;
+        }
 
         // ---- best-first enumeration of rank combinations
         int npool = 0, nprobe = 1;
@@ -99,6 +115,10 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
             const int first_set = primary ? 0 : j + 1;
             const int nset = V >= 2 ? K - first_set : 0;
             const int nchild = (can_raise ? 1 : 0) + nset;
+            uint32_t raised[8];  // the parent's rotations of rank above 0 (K <= 256): the only ones that cost
+#pragma unroll
+            for (int w = 0; w < 8; ++w)
+                raised[w] = 32 * w < K ? __ballot_sync(kFull, 32 * w + lane < K && rk[min(32 * w + lane, K - 1)] != 0) : 0u;
             for (int c = lane; c < nchild; c += 32) {
                 int rot, rank;
                 if (can_raise && c == 0) {
@@ -109,10 +129,12 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
                     rank = 1;
                 }
                 float s = 0.0f;
-                for (int r = 0; r < K; ++r) {
-                    const int rr = r == rot ? rank : int(rk[r]);
-                    if (rr) s = __fadd_rn(s, cost[r * V + rr]);
-                }
+#pragma unroll
+                for (int w = 0; w < 8; ++w)
+                    for (uint32_t m = raised[w] | (rot >> 5 == w ? 1u << (rot & 31) : 0u); m; m &= m - 1) {
+                        const int r = 32 * w + __ffs(m) - 1;
+                        s = __fadd_rn(s, cost[r * V + (r == rot ? rank : int(rk[r]))]);
+                    }
                 pscore[npool + c] = s;
                 pparent[npool + c] = uint32_t(parent);
                 prot[npool + c] = uint16_t(rot);
@@ -151,7 +173,7 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
                 pparent[bi] = kNoParent;
             }
             __syncwarp();
-            push_children(nprobe);
+            if (nprobe + 1 < T) push_children(nprobe);
             ++nprobe;
         }
 
@@ -167,7 +189,7 @@ __global__ void probe_codes_kernel(ProbeArgs a) {
                 else static_cast<uint8_t*>(a.out)[o] = uint8_t(comp);
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -205,19 +227,21 @@ __global__ void merge_probes_kernel(const uint32_t* __restrict__ ids, const floa
                 }
                 __syncwarp();
             }
+        // a lane an entry: the first of its id among the 32 and not among those already out
         int nout = 0;
-        for (int p = 0; p < n && nout < k; ++p) {
-            const uint32_t id = sid[p];
-            if (id == kInvalidNode) break;  // padding sorts last
-            bool dup = false;
-            for (int i = lane; i < nout; i += 32) dup |= oid[i] == id;
-            if (__any_sync(kFull, dup)) continue;
-            if (lane == 0) {
-                oid[nout] = id;
-                out_ids[size_t(q) * k + nout] = id;
-                out_dist[size_t(q) * k + nout] = sd[p];
+        for (int p0 = 0; p0 < n && nout < k; p0 += 32) {
+            const uint32_t id = sid[p0 + lane];
+            const uint32_t same = __match_any_sync(kFull, id);
+            bool fresh = id != kInvalidNode && (same & ((1u << lane) - 1)) == 0;  // padding sorts last
+            for (int i = 0; i < nout; ++i) fresh &= oid[i] != id;
+            const uint32_t m = __ballot_sync(kFull, fresh);
+            const int at = nout + __popc(m & ((1u << lane) - 1));
+            if (fresh && at < k) {
+                oid[at] = id;
+                out_ids[size_t(q) * k + at] = id;
+                out_dist[size_t(q) * k + at] = sd[p0 + lane];
             }
-            ++nout;
+            nout = min(k, nout + __popc(m));
             __syncwarp();
         }
         for (int i = nout + lane; i < k; i += 32) {
@@ -250,13 +274,13 @@ int launch_probe_codes(cphnsw_b200_index* h, const float* d_rotated, uint64_t nq
         return CPHNSW_B200_E_UNSUPPORTED;
     }
     const unsigned grid = unsigned(nq < uint64_t(h->sm_count) * 8 ? nq : uint64_t(h->sm_count) * 8);
-    if (h->comp_bytes == 2) {
-        CPB_CUDA(allow_max_dynamic_smem(probe_codes_kernel<true>));
-        probe_codes_kernel<true><<<grid, 32, smem, st>>>(a);
-    } else {
-        CPB_CUDA(allow_max_dynamic_smem(probe_codes_kernel<false>));
-        probe_codes_kernel<false><<<grid, 32, smem, st>>>(a);
-    }
+    auto go = [&](auto kernel) -> int {
+        CPB_CUDA(allow_max_dynamic_smem(kernel));
+        kernel<<<grid, kProbeWarps * 32, smem, st>>>(a);
+        return 0;
+    };
+    if (h->comp_bytes == 2) CPB_TRY(h->P <= 128 ? go(probe_codes_kernel<true, true>) : go(probe_codes_kernel<true, false>));
+    else CPB_TRY(h->P <= 128 ? go(probe_codes_kernel<false, true>) : go(probe_codes_kernel<false, false>));
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     return 0;
