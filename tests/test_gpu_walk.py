@@ -1,0 +1,37 @@
+"""The beam walk where its dispatch turns (csrc/search_walk.cu): a block or a warp per query, with and without the entry
+scan, the narrow and the wide rerank, beams at the edges of their steps.  Without statistics asked for the walk keeps a
+lossy filter of the nodes it has seen; ids and distances are those of the one-warp kernel and of the oracle all the same,
+bit for bit."""
+import numpy as np
+import pytest
+
+from cphnsw_b200 import synthetic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dim,K,cb,M,k,ef,rerank,entries,seeds", [
+    (128, 32, 1, 32, 10, 100, 500, 500, 32),   # K = 32, P = 128: the specialised scores
+    (96, 16, 1, 16, 1, 1, 0, 64, 1),           # a beam of one
+    (40, 33, 1, 24, 32, 33, 40, 100, 31),      # a second, ragged block of rotations
+    (300, 16, 2, 32, 10, 64, 64, 32, 32),      # two-byte components; every entry is a seed: no scan
+    (128, 32, 1, 32, 10, 65, 0, 100, 33),      # more seeds than the scan keeps
+    (960, 8, 2, 32, 10, 1000, 1024, 7, 32),    # a table of 32 KB; fewer entries than seeds; a full list to rerank
+])
+@pytest.mark.parametrize("nq", [1, 149, 297, 593])
+def test_walk_matches_one_warp_kernel_and_oracle(cp, oracle, dim, K, cb, M, k, ef, rerank, entries, seeds, nq):
+    n = 3001
+    base, q = synthetic.gaussian_mixture(n, nq, dim, 12, 0.3, dim + nq)
+    idx = cp.CPHNSWIndex(dim, M=M, ef_construction=max(200, M), K=K, component_bytes=cb, fht_convention=2)
+    idx.set_param("entry_scan", entries)
+    idx.set_param("k_entry", seeds)
+    idx.add_batch_parallel(base)
+    run = (lambda: idx.search_and_rerank_batch(q, k, ef, rerank)) if rerank else (lambda: idx.search_batch(q, k, ef))
+    ids, dist = run()
+    idx.set_param("search_kernel", 1)
+    wi, wd = run()
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+    if not rerank:
+        _, rot, _ = oracle.encode(q[:20], K, cb, oracle.sign_tables(dim, K, 42), 2, want_rotated=True)
+        oi, od = oracle.search(rot, idx.codes(), idx.adjacency(), idx.entry_ids(), max(ef, k), k, n_seed=seeds)
+        assert np.array_equal(ids[:20], oi) and np.array_equal(dist[:20], od)
