@@ -74,6 +74,22 @@ def test_many_clusters_against_the_bit_sliced_kernel(cp):
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
 
 
+@pytest.mark.parametrize("K,cb", [(32, 1), (32, 2)])
+def test_codes_off_a_sector_boundary(cp, oracle, K, cb):
+    # 16-byte aligned device codes are read by 16 bytes, 32-byte aligned ones by 32
+    import torch
+    n, k = 1500, 64
+    codes = np.random.default_rng(K + cb).integers(0, 16, (n, K)).astype(np.uint8 if cb == 1 else np.uint16)
+    wn, wd = oracle.knn_graph(codes, k, 0, n)
+    buf = torch.zeros(n * K * cb + 64, dtype=torch.uint8, device="cuda")
+    idx = index(cp, 128 if cb == 1 else 300, K, cb)
+    for offset in (0, 16):
+        buf[offset:offset + n * K * cb] = torch.from_numpy(codes.reshape(-1).view(np.uint8)).cuda()
+        nbrs = torch.zeros((n, k), dtype=torch.int32, device="cuda")
+        idx.knn_graph_dev(buf.data_ptr() + offset, n, k, 0, n, nbrs.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+        assert np.array_equal(nbrs.cpu().numpy().view(np.uint32), wn)
+
+
 def test_lost_wait_is_reported(cp, oracle):
     # the first wait gets no polls: every role of the block ends and the call reports it; the handle stays usable
     codes = np.random.default_rng(3).integers(0, 256, (3000, 32)).astype(np.uint8)
