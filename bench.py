@@ -29,10 +29,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, os.path.join(ROOT, "sparse-text-kmeans_b200"))
 
 METRIC = "batch-search QPS @ recall@10>=0.9 (search_and_rerank)"
-# DRAM bytes (read + written) per query of search_team_kernel, from the ncu capture summarised in
-# profiles/search_team_kernel_c2_quarter.md (C2 at 1/4 size, 2,500 queries: 1.281 GB + 0.080 GB per launch);
+# DRAM bytes (read + written) per query of the search kernels, from the ncu capture summarised in
+# profiles/search_walk_kernel_c2_quarter.md (C2 at 1/4 size, 2,500 queries);
 # the traffic per query does not depend on the number of queries, so a launch of nq queries moves nq times this
-NCU_SEARCH_DRAM_BYTES_PER_QUERY = 537e3
+NCU_SEARCH_DRAM_BYTES_PER_QUERY = 139e3
 # the same for the one-warp search_kernel (profiles/search_kernel_c2_quarter.md: 1.215 GB + 0.080 GB per launch)
 NCU_SEARCH_DRAM_BYTES_PER_QUERY_ONE_WARP = 518e3
 
@@ -52,7 +52,7 @@ def parse_args():
     ap.add_argument("--fvecs", nargs=2, metavar=("BASE", "QUERY"), default=None,
                     help="run on fvecs files (rows are normalised) instead of a synthetic workload")
     ap.add_argument("--search-kernel", type=int, default=0, choices=[0, 1, 2],
-                    help="0 = the library's choice, 1 = one warp per query, 2 = two warps per query")
+                    help="0 = the library's choice, 1 = the kernel that expands one node a step, 2 = the walk of several nodes a step")
     ap.add_argument("--K", type=int, default=None, help="code width (rotations); default: the workload's (32)")
     ap.add_argument("--exact-edges", action="store_true",
                     help="graph links chosen on the fp32 vectors (set_param exact_edges; single GPU builds)")
@@ -477,7 +477,7 @@ def run_b200(args):
     d_stats = torch.zeros((nq, 2), dtype=torch.int32, device=dev)
 
     def step_resident():
-        idx.search_dev(d_q.data_ptr(), nq, k, ef, rerank_k, d_ids.data_ptr(), d_dist.data_ptr(), d_stats.data_ptr())
+        idx.search_dev(d_q.data_ptr(), nq, k, ef, rerank_k, d_ids.data_ptr(), d_dist.data_ptr())
 
     # ---- timed region 1: inputs resident in HBM ----
     # the clock sampler starts before the warm-up (its own start-up then overlaps untimed work) and
@@ -525,6 +525,9 @@ def run_b200(args):
     value = world * nq / (ms_per_step * 1e-3)
 
     ids = d_ids.cpu().numpy().astype(np.uint32)
+    # expansions and distance evaluations per query, from a pass of their own (the counts need an exact visited set)
+    idx.search_dev(d_q.data_ptr(), nq, k, ef, rerank_k, d_ids.data_ptr(), d_dist.data_ptr(), d_stats.data_ptr())
+    torch.cuda.synchronize()
     stats = d_stats.cpu().numpy()
     recall = sharded.recall_at_k(ids[:n_gt], gt, k)
     if world > 1:
@@ -576,13 +579,11 @@ def run_b200(args):
     # a batch beyond the library's visited-slot budget is served by several launches: units per launch, not per step
     q_per_launch = nq * args.steps / max(1, search_launches)
     achieved = bytes_per_query * q_per_launch / (search_ms_per_launch * 1e-3) / 1e9
-    # the library takes the two-warp kernel when the query table fits shared memory and M <= 32
-    small_table = K * idx.padded_dim * 4 <= 32 * 1024
-    beam = max(ef, rerank_k, k)
-    team = args.search_kernel != 1 and M <= 32 and (beam <= 1024 or (beam <= 2048 and small_table)) and (small_table or K <= 32)
-    dram_per_query = NCU_SEARCH_DRAM_BYTES_PER_QUERY if team else NCU_SEARCH_DRAM_BYTES_PER_QUERY_ONE_WARP
+    # the library takes the walk of several nodes a step (with its entry scan and rerank kernels) when M <= 32
+    walk = args.search_kernel != 1 and M <= 32
+    dram_per_query = NCU_SEARCH_DRAM_BYTES_PER_QUERY if walk else NCU_SEARCH_DRAM_BYTES_PER_QUERY_ONE_WARP
     traffic = dram_per_query * q_per_launch if w["name"] == "C2" else None
-    roofline = {"kernel": "search_team_kernel" if team else "search_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roofline = {"kernel": "entry_scan_kernel + search_walk_kernel + search_rerank_kernel" if walk else "search_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": "of " + peak_kind,
                 "traffic": traffic,
                 # the same fraction on the DRAM bytes ncu measured instead of the algorithmic bytes: what the kernel
@@ -615,18 +616,15 @@ def run_b200(args):
                    "frac": build["encode_fp32_addsub_per_s"] / lanes,
                    "note": "K*3*P*log2(P) butterflies per vector over the measured stage time; peak = GPUs x SMs x 128 lanes x sampled SM clock"},
         "knn_graph": None, "select_neighbors": None}
-    planes = 8 if cb == 1 else (11 if idx.padded_dim == 1024 else 0)  # bit planes of a component in the bit-sliced kernel
-    if K == 32 and planes:
-        # bit-sliced kernel: one logic instruction per bit plane and rotation (256 at 8 planes, 352 at 11), 62 for the
-        # carry-save sum and ~12 for the threshold compare per (row, 32 candidates): 330 = 10.3 per pair (one-byte
-        # components), 426 = 13.3 per pair (two-byte components of padded dim 1024), on the ALU pipe, which issues 64
-        # lanes per SM and clock
-        per_group = planes * K + 62 + 12
-        alu = world * idx_sm_count * 64 * sm_mhz * 1e6
-        roofline_build["knn_graph"] = {"bound": "integer ALU pipe", "achieved": build["knn_pairs_per_s"] * per_group / 32.0, "peak": alu,
-                                       "unit": "instr/s", "frac": build["knn_pairs_per_s"] * per_group / 32.0 / alu,
-                                       "note": "%.1f integer instructions per pair (kernel source count); ncu sm__pipe_alu_cycles_active "
-                                               "67.5 %% on C2 at 1/4 size (profiles/knn_sliced_kernel_c2_quarter.md)" % (per_group / 32.0)}
+    if 2 <= K <= 64 and n >= 4096:
+        # tensor-core filter: a component is 7 values of +-1 at K <= 32 and 3 above, rows padded to a multiple of 32
+        # values; every pair costs two operations a value
+        values = (K * (7 if K <= 32 else 3) + 31) // 32 * 32
+        fp8 = 4.5e15 * world
+        roofline_build["knn_graph"] = {"bound": "fp8 tensor pipe and its epilogue", "achieved": build["knn_pairs_per_s"] * 2 * values, "peak": fp8,
+                                       "unit": "op/s", "frac": build["knn_pairs_per_s"] * 2 * values / fp8,
+                                       "note": "%d values per pair; peak is the nominal dense fp8 rate; ncu sm__pipe_tensor_cycles_active "
+                                               "62 %% of the sweep on C2 at 1/4 size (profiles/knn_mma_kernel_c2_quarter.md)" % values}
     sel_bytes = n * (knn_k * 4 + knn_k * code_row + M * 4.0)
     roofline_build["select_neighbors"] = {"bound": "hbm gather", "achieved": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9, "peak": peak * world,
                                           "unit": "GB/s", "frac": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9 / (peak * world),
