@@ -141,6 +141,50 @@ __device__ __forceinline__ uint32_t component_of(float win, int idx, int flip_ma
     return (uint32_t(idx) << 1) | (neg ? 1u : 0u);
 }
 
+// The block's vectors, zero-padded, a thread's part of one (128 elements, or all of it) a row: coalesced 128-bit loads
+// when rows are 16-byte aligned, else 32-bit loads, kStageRows rows in flight per warp (one at a time, the round trips of a
+// warp's 32 rows in sequence took as long as a rotation: 10k x 128, K = 32, 58 us against 50, with rotated vectors 113 against
+// 98; 2k x 256 47 against 37).
+constexpr int kStageRows = 8;
+template <int P>
+__device__ __forceinline__ void stage_tile(float* tile, const float* __restrict__ x, uint64_t row0, int rows, int dim, int lane, int warp) {
+    constexpr int W = P < 128 ? P : 128, G = P / W;  // elements of a row, rows per vector
+    constexpr int kStride = kTileStride<W>, C = W / 32;
+    const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
+    for (int r0 = warp * kStageRows; r0 < kTileVecs; r0 += kTileVecs / 32 * kStageRows) {
+        float4 q[kStageRows];
+#pragma unroll
+        for (int i = 0; i < kStageRows; ++i) {
+            const int r = r0 + i, left = r / G < rows ? dim - W * (r % G) : 0;  // elements of the vector from this row on
+            const float* src = x + (row0 + r / G) * uint64_t(dim) + W * (r % G);
+            q[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (vec4) {
+                if (4 * lane < left && 4 * lane < W) q[i] = __ldg(reinterpret_cast<const float4*>(src) + lane);
+            } else {
+                if (lane < left) q[i].x = __ldg(src + lane);
+                if (C > 1 && lane + 32 < left) q[i].y = __ldg(src + lane + 32);
+                if (C > 2 && lane + 64 < left) q[i].z = __ldg(src + lane + 64);
+                if (C > 2 && lane + 96 < left) q[i].w = __ldg(src + lane + 96);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kStageRows; ++i) {
+            float* dst = tile + (r0 + i) * kStride;
+            if (vec4) {
+                if (4 * lane < W) {
+                    f32x2* to = reinterpret_cast<f32x2*>(dst + 4 * lane);
+                    to[0] = pack2(q[i].x, q[i].y);
+                    to[1] = pack2(q[i].z, q[i].w);
+                }
+            } else {
+                dst[lane] = q[i].x;
+                if (C > 1) dst[lane + 32] = q[i].y;
+                if (C > 2) dst[lane + 64] = q[i].z, dst[lane + 96] = q[i].w;
+            }
+        }
+    }
+}
+
 // QUERY = true additionally writes the rotated vectors and winning magnitudes (CPQuery).  A vector a thread at padded
 // dims 32 and 64 too: with a warp a vector the shuffles of the high stages (one an element) were the bound, 300k x 64 with
 // K = 32 took 2.09 ms and takes 0.50, 300k x 32 took 1.64 and takes 0.24.  (Measured and dropped at P = 128: the second
@@ -160,33 +204,7 @@ encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, in
     const int rows = int(min(uint64_t(kTileVecs), n - row0));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // stage the tile: coalesced 128-bit loads when rows are 16-byte aligned, else 32-bit loads
-    const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    for (int r = warp; r < kTileVecs; r += kTileVecs / 32) {
-        float* dst = tile + r * kTileStride<P>;
-        if (r < rows) {
-            const float* src = x + (row0 + r) * uint64_t(dim);
-            if (vec4) {
-                if (P == 128 || 4 * lane < P) {
-                    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (4 * lane < dim) q = __ldg(reinterpret_cast<const float4*>(src) + lane);
-                    dst[4 * lane] = q.x;
-                    dst[4 * lane + 1] = q.y;
-                    dst[4 * lane + 2] = q.z;
-                    dst[4 * lane + 3] = q.w;
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < P / 32; ++c) {
-                    int i = lane + 32 * c;
-                    dst[i] = i < dim ? __ldg(src + i) : 0.0f;
-                }
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < P / 32; ++c) dst[lane + 32 * c] = 0.0f;
-        }
-    }
+    stage_tile<P>(tile, x, row0, rows, dim, lane, warp);
     // the three diagonals of one rotation are staged in shared memory one rotation ahead
     const int t = threadIdx.x;
     if (t < 3 * P / 4)
@@ -508,23 +526,7 @@ encode_group_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int
     const int rows = int(min(uint64_t(kVecs), n - row0));
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, part = t % G;
 
-    const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    for (int r = warp; r < kTileVecs; r += kTileVecs / 32) {
-        float* dst = tile + r * kStride;
-        const int left = r / G < rows ? dim - 128 * (r % G) : 0;  // elements of the vector from this row on
-        const float* src = x + (row0 + r / G) * uint64_t(dim) + 128 * (r % G);
-        if (vec4) {
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (4 * lane < left) q = __ldg(reinterpret_cast<const float4*>(src) + lane);
-            dst[4 * lane] = q.x;
-            dst[4 * lane + 1] = q.y;
-            dst[4 * lane + 2] = q.z;
-            dst[4 * lane + 3] = q.w;
-        } else {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) dst[lane + 32 * c] = lane + 32 * c < left ? __ldg(src + lane + 32 * c) : 0.0f;
-        }
-    }
+    stage_tile<128 * G>(tile, x, row0, rows, dim, lane, warp);
     __syncthreads();
 
     const f32x2* mine = reinterpret_cast<const f32x2*>(tile + t * kStride);
