@@ -419,7 +419,7 @@ __global__ void adjacency_dup_kernel(const uint32_t* __restrict__ adj, uint64_t 
 }
 
 // The entry nodes' codes as the entry scan of the asymmetric metric reads them: per block of 32 rotations, component
-// (j + e) & 31 of entry e at place j (zero for rotations past K)
+// j ^ e (their low five bits) of entry e at place j (zero for rotations past K)
 template <typename CompT>
 __global__ void rotate_entry_codes_kernel(const CompT* __restrict__ codes /* [n_entry][K] */, uint32_t n_entry, int K, int padded,
                                           CompT* __restrict__ out /* [n_entry][padded] */) {
@@ -427,7 +427,7 @@ __global__ void rotate_entry_codes_kernel(const CompT* __restrict__ codes /* [n_
     if (t >= uint64_t(n_entry) * padded) return;
     const uint32_t e = uint32_t(t / padded);
     const int j = int(t % padded);
-    const int r = (j & ~31) | ((j + int(e & 31u)) & 31);
+    const int r = j ^ int(e & 31u);
     out[t] = r < K ? codes[uint64_t(e) * K + r] : CompT(0);
 }
 
@@ -668,7 +668,7 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
         a.n_seed = k;
     }
     CPB_CUDA(cudaMemsetAsync(a.next_query, 0, 4, st));
-    // a narrow launch gives every query a block of its own (one warp or one team), so a handful of
+    // a narrow launch gives every query a block of its own (one warp or eight), so a handful of
     // queries spread over as many SMs and need as many visited slots
     const bool narrow = !cx.wide;
     const unsigned grid = narrow ? unsigned(nq) : unsigned(h->sm_count);

@@ -314,19 +314,28 @@ struct Vals {
     float v[QG];
 };
 
-// S(step, j) of the tree over rotations (j + lane) & 31; w: the entry's components in that order
+// two fp32 additions by one instruction, each rounded as the scalar one
+__device__ __forceinline__ void add_pair(float& a0, float& a1, float b0, float b1) {
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a0), "+f"(a1)
+        : "f"(b0), "f"(b1));
+}
+
+// S(step, j) of the tree over rotations j ^ lane; w: the entry's components in that order.  (The tree pairs rotations that
+// differ in one bit of their number, which the XOR leaves so.)  The scan is bound by its instructions: the address of a
+// value is one shift, one mask-and-or and the XOR of lane and j, the sums of two queries are one addition.
 template <bool U16, int QG, int STEP, int J>
 __device__ __forceinline__ Vals<QG> scan_tree(const unsigned char* table, const uint32_t (&w)[U16 ? 16 : 8], uint32_t lane_at,
-                                              uint32_t index2_mask) {
+                                              uint32_t row_mask) {
     Vals<QG> r;
     if constexpr (STEP == 32) {
         constexpr int PER = U16 ? 2 : 4, BITS = U16 ? 16 : 8;
-        constexpr int SH = (J % PER) * BITS;  // the component's position in its word
-        constexpr int ROW = 32 * QG * 4;      // bytes of one index of the table
+        constexpr int SH = (J % PER) * BITS;                      // the component's position in its word
+        constexpr int UP = QG == 4 ? 8 : (QG == 2 ? 7 : 6);       // twice an index to the bytes of its row of the table
         const uint32_t word = w[J / PER];
         const uint32_t sign = word << (31 - SH);
-        const uint32_t comp2 = (word >> SH) & index2_mask;  // twice the index, kept inside the table
-        const uint32_t at = comp2 * uint32_t(ROW / 2) + ((lane_at + uint32_t(J * QG * 4)) & uint32_t(ROW - 1));
+        const uint32_t row = UP >= SH ? word << (UP >= SH ? UP - SH : 0) : word >> (UP >= SH ? 0 : SH - UP);
+        const uint32_t at = (row & row_mask) | (lane_at ^ uint32_t(J * QG * 4));  // the mask keeps it inside the table
         float x[QG];
         if constexpr (QG == 4) {
             const float4 f = *reinterpret_cast<const float4*>(table + at);
@@ -340,10 +349,14 @@ __device__ __forceinline__ Vals<QG> scan_tree(const unsigned char* table, const 
 #pragma unroll
         for (int i = 0; i < QG; ++i) r.v[i] = __uint_as_float(__float_as_uint(x[i]) ^ (sign & 0x80000000u));
     } else {
-        const Vals<QG> a = scan_tree<U16, QG, STEP * 2, J>(table, w, lane_at, index2_mask);
-        const Vals<QG> b = scan_tree<U16, QG, STEP * 2, J + STEP>(table, w, lane_at, index2_mask);
+        r = scan_tree<U16, QG, STEP * 2, J>(table, w, lane_at, row_mask);
+        const Vals<QG> b = scan_tree<U16, QG, STEP * 2, J + STEP>(table, w, lane_at, row_mask);
+        if constexpr (QG == 1) {
+            r.v[0] = __fadd_rn(r.v[0], b.v[0]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < QG; ++i) r.v[i] = __fadd_rn(a.v[i], b.v[i]);
+            for (int i = 0; i < QG; i += 2) add_pair(r.v[i], r.v[i + 1], b.v[i], b.v[i + 1]);
+        }
     }
     return r;
 }
@@ -420,7 +433,7 @@ entry_scan_kernel(ScanArgs a) {
                     w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
                 }
                 const Vals<QG> s = scan_tree<U16, QG, 1, 0>(scan_smem + size_t(blk) * a.P * 32 * QG * 4, w, uint32_t(lane * QG * 4),
-                                                               uint32_t(2 * a.P - 2));
+                                                               uint32_t(2 * a.P - 2) << (QG == 4 ? 8 : (QG == 2 ? 7 : 6)));
 #pragma unroll
                 for (int g = 0; g < QG; ++g) d[g] = __fadd_rn(d[g], s.v[g]);
             }
