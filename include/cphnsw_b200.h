@@ -81,13 +81,12 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *   "prune" (0/1, default 1: the bulk build runs select_neighbors on the kNN candidates; 0 = the M nearest
  *            candidates are the links, build_with_gpu_knn(..., prune = false), evaluation/test_gpu_build.cpp:168-174),
  *   "knn_k" (candidates per node fed to select_neighbors, default min(2*M, 64)),
- *   "knn_kernel" (0 = pick, 1 = byte-wise distance, 2 = bit-sliced distance; K = 16/32/64 with uint8 codes or
+ *   "knn_kernel" (0 = pick; 3 = tensor-core filter in front of exact distances, plain codes of 2 to 64 components,
+ *                 what 0 picks from 4,096 nodes on; 1 = byte-wise distance, 2 = bit-sliced distance; K = 16/32/64 with uint8 codes or
  *                 in binary-code mode, K = 16/32 with uint16 codes of padded dim 1024, and one-byte binary codes of
  *                 any K <= 120 that is a multiple of 8, residual bits included when the primary part is one too),
- *   "search_kernel" (0 = pick: two warps per query whenever that kernel applies; 1 = one warp per query,
- *                    2 = two warps per query; the second needs
- *                    M <= 32, either K * padded_dim * 4 <= 32 KB or K <= 32, and a beam max(ef, k, rerank_k) of at most
- *                    1024 (2048 when K * padded_dim * 4 <= 32 KB); both return identical results),
+ *   "search_kernel" (0 = pick: the walk that expands several nodes a step whenever M <= 32; 1 = one node a step, any M;
+ *                    2 = the walk of several nodes, an error when M > 32; both return identical results),
  *   "binary_codes" (0/1, before any vector is added: 1 = the unified index's primary binary code
  *                   (include/cphnsw/core/codes.hpp:76-129 with R = 0): a component keeps only its sign bit, so
  *                   code distance = Hamming distance and the graph is built under it; search / search_and_rerank

@@ -711,7 +711,7 @@ int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double v) {
         return 0;
     }
     if (s == "search_kernel") {
-        if (v != 0 && v != 1 && v != 2) { set_error("search_kernel must be 0 (pick), 1 (one warp per query) or 2 (two warps per query)"); return CPHNSW_B200_E_INVALID; }
+        if (v != 0 && v != 1 && v != 2) { set_error("search_kernel must be 0 (pick), 1 (one node a step) or 2 (several nodes a step)"); return CPHNSW_B200_E_INVALID; }
         h->search_kernel = int(v);
         return 0;
     }

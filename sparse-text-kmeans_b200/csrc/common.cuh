@@ -132,7 +132,7 @@ struct PinnedBuf {
 // narrow ones for launches of up to kNarrowQueries queries, one block per query.
 constexpr uint32_t kNarrowQueries = 32;
 // widest beam of a search: the one-warp kernel keeps W as one sorted array of up to this many members in shared
-// memory (32 KB at 4,096); the two-warp kernel's tiered W holds 1,024 and is used up to that width
+// memory (32 KB at 4,096), and so does the walk of several nodes a step
 constexpr uint32_t kMaxBeam = 4096;
 struct SearchCtx {
     cudaStream_t stream = nullptr;
@@ -166,7 +166,7 @@ struct cphnsw_b200_index {
     int prune = 1;  // 0: the bulk build keeps the M nearest kNN candidates instead of running select_neighbors
     uint32_t k_entry = 4, knn_k = 0, entry_scan = 0;
     int knn_kernel = 0;  // 0 = pick, 1 = byte-wise distance, 2 = bit-sliced distance, 3 = tensor-core filter
-    int search_kernel = 0;  // 0 = pick, 1 = one warp per query, 2 = two warps per query
+    int search_kernel = 0;  // 0 = pick, 1 = one node a step, 2 = several nodes a step
     int search_table_smem = 1;  // 0: the query table is read in place even when it would fit shared memory
     int binary_codes = 0;  // 1: components keep only the sign bit (Hamming metric), search walks under the code distance
     // residual codes of the binary mode: the last residual_bits components are residual bits, a primary mismatch
