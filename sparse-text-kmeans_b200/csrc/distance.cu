@@ -398,10 +398,21 @@ __global__ void rev_count_kernel(const uint32_t* __restrict__ new_adj, uint64_t 
 // (counters[0] = entries used in the incoming list, counters[1] = affected nodes)
 __global__ void rev_alloc_kernel(const uint32_t* __restrict__ cnt, uint64_t n_old, uint32_t* __restrict__ seg,
                                  uint32_t* __restrict__ aff, uint32_t* __restrict__ counters) {
+    // one pair of device atomics a block: thousands of them on two words took 21 us
+    __shared__ uint32_t edges, rows, first_edge, first_row;
+    if (threadIdx.x == 0) edges = rows = 0;
+    __syncthreads();
     const uint64_t v = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (v >= n_old || cnt[v] == 0) return;
-    seg[v] = atomicAdd(counters, cnt[v]);
-    aff[atomicAdd(counters + 1, 1u)] = uint32_t(v);
+    const uint32_t c = v < n_old ? cnt[v] : 0u;
+    uint32_t edge = 0, row = 0;
+    if (c) edge = atomicAdd(&edges, c), row = atomicAdd(&rows, 1u);
+    __syncthreads();
+    if (threadIdx.x == 0 && rows) first_edge = atomicAdd(counters, edges), first_row = atomicAdd(counters + 1, rows);
+    __syncthreads();
+    if (c) {
+        seg[v] = first_edge + edge;
+        aff[first_row + row] = uint32_t(v);
+    }
 }
 __global__ void rev_fill_kernel(const uint32_t* __restrict__ new_adj, uint64_t m, int M, uint64_t n_old,
                                 const uint32_t* __restrict__ seg, uint32_t* __restrict__ fill, uint32_t* __restrict__ inc) {

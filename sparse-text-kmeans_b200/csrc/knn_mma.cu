@@ -160,39 +160,42 @@ __global__ void key_count_kernel(const CompT* __restrict__ codes, uint64_t n, in
     const uint64_t row = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (row < n) atomicAdd(hist + size_t(blockIdx.y) * kKeys + row_key(codes, K, row, blockIdx.y), 1u);
 }
-__global__ void __launch_bounds__(1024) key_scan_kernel(uint32_t* __restrict__ hist) {  // exclusive, one block per order
+// exclusive, one block per order; a warp takes 2,048 keys, 128 of them a step in one line of reads each (a thread with 64
+// keys of its own read a sector per key pair: 30 us)
+__global__ void __launch_bounds__(1024) key_scan_kernel(uint32_t* __restrict__ hist) {
     __shared__ uint32_t sums[32];
-    uint4* h = reinterpret_cast<uint4*>(hist + size_t(blockIdx.x) * kKeys + threadIdx.x * (kKeys / 1024));
+    constexpr int kSteps = int(kKeys / 4096);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* h = reinterpret_cast<uint4*>(hist + size_t(blockIdx.x) * kKeys) + warp * kSteps * 32 + lane;
+    auto scan = [&](uint32_t x) {  // inclusive, over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, d);
+            if (lane >= d) x += y;
+        }
+        return x;
+    };
     uint32_t own = 0;
-#pragma unroll 8
-    for (int i = 0; i < int(kKeys / 4096); ++i) {
-        const uint4 v = h[i];
+#pragma unroll
+    for (int i = 0; i < kSteps; ++i) {
+        const uint4 v = h[i * 32];
         own += v.x + v.y + v.z + v.w;
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = own;
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, x, d);
-        if (lane >= d) x += y;
-    }
-    if (lane == 31) sums[warp] = x;
+    own = __reduce_add_sync(kFull, own);
+    if (lane == 0) sums[warp] = own;
     __syncthreads();
     if (warp == 0) {
-        uint32_t s = sums[lane];
-        const uint32_t o = s;
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, s, d);
-            if (lane >= d) s += y;
-        }
-        sums[lane] = s - o;
+        const uint32_t o = sums[lane];
+        sums[lane] = scan(o) - o;
     }
     __syncthreads();
-    uint32_t at = sums[warp] + x - own;
+    uint32_t at = sums[warp];
 #pragma unroll 4
-    for (int i = 0; i < int(kKeys / 4096); ++i) {
-        const uint4 c = h[i];
-        h[i] = make_uint4(at, at + c.x, at + c.x + c.y, at + c.x + c.y + c.z);
-        at += c.x + c.y + c.z + c.w;
+    for (int i = 0; i < kSteps; ++i) {
+        const uint4 c = h[i * 32];
+        const uint32_t mine = c.x + c.y + c.z + c.w, upto = scan(mine), b = at + upto - mine;
+        h[i * 32] = make_uint4(b, b + c.x, b + c.x + c.y, b + c.x + c.y + c.z);
+        at += __shfl_sync(kFull, upto, 31);
     }
 }
 template <typename CompT>

@@ -407,15 +407,24 @@ __global__ void gather_rows_kernel(const unsigned char* __restrict__ src, int ro
     dst[i] = id < n ? src[uint64_t(id) * row_bytes + i % row_bytes] : 0;
 }
 
-// one warp per adjacency row (M <= 32): a valid id that appears twice raises the flag
+// adjacency rows (M <= 32): a valid id that appears twice raises the flag.  Every pair of lanes meets in 16 rotations of the
+// row, kDupRows rows in flight a warp (match.any took some 80 cycles of the SM a row: 100k rows 29 us).
+constexpr int kDupRows = 4;
 __global__ void adjacency_dup_kernel(const uint32_t* __restrict__ adj, uint64_t n, int M, uint32_t* __restrict__ flag) {
     const int lane = threadIdx.x & 31;
-    const uint64_t row = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= n) return;
-    const uint32_t id = lane < M ? adj[row * M + lane] : kInvalidNode;
-    const uint32_t grp = __match_any_sync(kFull, id);
-    const bool dup = id < n && (__ffs(grp) - 1) != lane;
-    if (__ballot_sync(kFull, dup) && lane == 0) atomicOr(flag, 1u);
+    const uint64_t row0 = ((uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5) * kDupRows;
+    uint32_t id[kDupRows];
+#pragma unroll
+    for (int i = 0; i < kDupRows; ++i) id[i] = lane < M && row0 + i < n ? adj[(row0 + i) * M + lane] : kInvalidNode;
+    bool dup = false;
+#pragma unroll
+    for (int i = 0; i < kDupRows; ++i) {
+        bool met = false;
+#pragma unroll
+        for (int d = 1; d <= 16; ++d) met |= __shfl_sync(kFull, id[i], lane + d) == id[i];
+        dup |= met && id[i] < n;
+    }
+    if (__any_sync(kFull, dup) && lane == 0) atomicOr(flag, 1u);
 }
 
 // The entry nodes' codes as the entry scan of the asymmetric metric reads them: per block of 32 rotations, component
@@ -572,7 +581,7 @@ int scan_adjacency_rows(cphnsw_b200_index* h, cudaStream_t st) {
     if (h->n == 0 || h->M > 32 || !h->d_adj.p) return 0;  // wider rows: the search dedupes each batch of 32
     uint32_t* flag = h->d_status.as<uint32_t>() + 2;
     CPB_CUDA(cudaMemsetAsync(flag, 0, 4, st));
-    const uint64_t threads = h->n * 32;
+    const uint64_t threads = (h->n + kDupRows - 1) / kDupRows * 32;
     adjacency_dup_kernel<<<unsigned((threads + 255) / 256), 256, 0, st>>>(h->d_adj.as<uint32_t>(), h->n, int(h->M), flag);
     h->launches++;
     CPB_CUDA(cudaGetLastError());

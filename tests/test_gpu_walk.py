@@ -35,3 +35,28 @@ def test_walk_matches_one_warp_kernel_and_oracle(cp, oracle, dim, K, cb, M, k, e
         _, rot, _ = oracle.encode(q[:20], K, cb, oracle.sign_tables(dim, K, 42), 2, want_rotated=True)
         oi, od = oracle.search(rot, idx.codes(), idx.adjacency(), idx.entry_ids(), max(ef, k), k, n_seed=seeds)
         assert np.array_equal(ids[:20], oi) and np.array_equal(dist[:20], od)
+
+
+@pytest.mark.parametrize("M", [24, 32])
+@pytest.mark.parametrize("row,a,b", [(0, 0, 1), (0, 0, 16), (0, 7, 23), (256, 3, 20)])
+def test_repeated_ids_in_a_row_count_once(cp, oracle, M, row, a, b):
+    # one row of the graph names a node twice, at places 1 to 17 apart; the last row is the last of a ragged group of rows
+    n, dim = 257, 128
+    base, q = synthetic.gaussian_mixture(n, 30, dim, 2, 0.5, M + b)
+    ref = cp.CPHNSWIndex(dim, M=M, ef_construction=64, K=32, component_bytes=1, fht_convention=2)
+    ref.add_batch_parallel(base)
+    codes, adj = ref.codes(), ref.adjacency()
+    rng = np.random.default_rng(b)
+    for r in {0, row}:
+        adj[r] = rng.choice(np.setdiff1d(np.arange(n), [r]), M, replace=False)
+    adj[row, b] = adj[row, a]
+    idx = cp.CPHNSWIndex(dim, M=M, ef_construction=64, K=32, component_bytes=1, fht_convention=2)
+    idx.set_param("k_entry", 4)
+    idx.set_param("entry_scan", 4)
+    idx.install(base, codes, adj)
+    _, rot, _ = oracle.encode(q, 32, 1, oracle.sign_tables(dim, 32, 42), 2, want_rotated=True)
+    for kernel in (0, 1):
+        idx.set_param("search_kernel", kernel)
+        ids, dist = idx.search_batch(q, 20, 200)
+        wi, wd = oracle.search(rot, codes, adj, idx.entry_ids(), 200, 20, n_seed=4)
+        assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
