@@ -51,10 +51,6 @@ __device__ __forceinline__ void prefetch_l1(const void* p) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 __device__ __forceinline__ bool key_less(float da, uint32_t ia, float db, uint32_t ib) {
     return da < db || (da == db && ia < ib);
 }
@@ -253,29 +249,6 @@ __device__ __forceinline__ void warp_select_smem(float* d, uint32_t* id, int n, 
             id[bp] = ti;
         }
         __syncwarp();
-    }
-}
-
-// bitonic sort of n (a power of two) pairs by (distance, id without the expanded flag); the flag travels with the id
-__device__ __forceinline__ void warp_sort_flagged(float* d, uint32_t* id, int n, int lane) {
-    for (int k2 = 2; k2 <= n; k2 <<= 1) {
-        for (int j = k2 >> 1; j > 0; j >>= 1) {
-            for (int t = lane; t < n / 2; t += 32) {
-                const int lo = ((t & ~(j - 1)) << 1) | (t & (j - 1));
-                const int hi = lo | j;
-                const bool asc = (lo & k2) == 0;
-                const float dl = d[lo], dh = d[hi];
-                const uint32_t il = id[lo], ih = id[hi];
-                const bool hi_less = key_less(dh, ih & kIdMask, dl, il & kIdMask);
-                if (hi_less == asc) {
-                    d[lo] = dh;
-                    id[lo] = ih;
-                    d[hi] = dl;
-                    id[hi] = il;
-                }
-            }
-            __syncwarp();
-        }
     }
 }
 
