@@ -853,6 +853,9 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         a.split.cts = uint32_t(tiles);
         a.split.steps = rts * tiles;
         a.split.blocks = uint32_t(a.split.steps < sms ? a.split.steps : sms);
+        // a block that gives up leaves its lengths unwritten; the rows it did not finish are then empty, not whatever the
+        // workspace held
+        CPB_CUDA(cudaMemsetAsync(a.counts, 0, size_t(a.split.blocks + rts) * kMmaRows * 2 * 4, st));
         knn_mma_kernel<U16, QUADS><<<a.split.blocks, kMmaThreads, 3 * operand_bytes + a.code_stages * code_bytes + own_bytes, st>>>(a);
         const uint32_t rows = uint32_t(rts) * kMmaRows;
         knn_finish_kernel<<<(rows + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, rows, d_nbrs, d_dist, uint32_t(row_begin));

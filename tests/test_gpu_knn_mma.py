@@ -102,6 +102,26 @@ def test_lost_wait_is_reported(cp, oracle):
     check(idx, oracle, codes, 16)
 
 
+def test_lost_wait_leaves_empty_rows(cp, oracle):
+    # the buffers' lengths of an earlier graph are still in the workspace: none of them may be read as this one's
+    import torch
+    codes = np.random.default_rng(4).integers(0, 256, (6000, 32)).astype(np.uint8)
+    idx = index(cp, 128, 32, 1)
+    d_codes = torch.from_numpy(codes).cuda()
+    nbrs = torch.zeros((6000, 64), dtype=torch.int32, device="cuda")
+    dist = torch.zeros((6000, 64), dtype=torch.int16, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    idx.knn_graph_dev(d_codes.data_ptr(), 6000, 64, 0, 6000, nbrs.data_ptr(), dist.data_ptr(), stream=st)
+    idx.set_param("first_wait_polls", 0)
+    idx.knn_graph_dev(d_codes.data_ptr(), 6000, 64, 0, 6000, nbrs.data_ptr(), dist.data_ptr(), stream=st)
+    torch.cuda.synchronize()
+    assert bool((nbrs == -1).all()) and bool((dist == -1).all())
+    with pytest.raises(cp.CPHNSWError):
+        idx.check_device_status()
+    idx.set_param("first_wait_polls", 1 << 22)
+    check(idx, oracle, codes, 64, (0, 300))
+
+
 def test_unsupported_codes_are_refused(cp):
     idx = index(cp, 128, 100, 1)
     with pytest.raises(cp.CPHNSWError):
