@@ -746,9 +746,9 @@ int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double v) {
         h->residual_bits = uint32_t(v);
         return 0;
     }
-    if (s == "first_wait_polls") {
-        if (v < 0 || v > 4194304.0) { set_error("first_wait_polls must be in 0..2^22"); return CPHNSW_B200_E_INVALID; }
-        h->first_wait_polls = uint32_t(v);
+    if (s == "first_wait_polls" || s == "handover_polls") {
+        if (v < 0 || v > 4194304.0) { set_error("%s must be in 0..2^22", name); return CPHNSW_B200_E_INVALID; }
+        (s == "first_wait_polls" ? h->first_wait_polls : h->handover_polls) = uint32_t(v);
         return 0;
     }
     if (s == "rank_prune") { h->rank_prune = v != 0.0; return 0; }
@@ -799,6 +799,7 @@ int cphnsw_b200_get_param(const cphnsw_b200_index* h, const char* name, double* 
     else if (s == "search_table_smem") *v = h->search_table_smem;
     else if (s == "build_seed") *v = h->build_seed;
     else if (s == "first_wait_polls") *v = h->first_wait_polls;
+    else if (s == "handover_polls") *v = h->handover_polls;
     else if (s == "rank_prune") *v = h->rank_prune;
     else if (s == "exact_edges") *v = h->exact_edges;
     else if (s == "rank_pruning_alpha") *v = h->rank_pruning_alpha;

@@ -330,8 +330,28 @@ struct KnnMmaArgs {
     uint8_t* dists;               // the same
     uint32_t* counts;             // [segments][256][2]
     uint32_t* status;
-    uint32_t first_wait_polls;
+    uint32_t first_wait_polls, handover_polls;
 };
+
+// A row tile's codes and limits pass between the two warps that share its rows: each stores, in shared memory, the number
+// of segments it is done with, and waits for the other's before it replaces them.  (A counter and not a barrier's phase:
+// a warp without a tile in a segment runs ahead of the other by several.)
+__device__ __forceinline__ void hand_over(uint32_t* done, uint32_t segments) {
+    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(done)), "r"(segments) : "memory");
+}
+__device__ __forceinline__ bool handed_over(const uint32_t* done, uint32_t segments, uint32_t limit, volatile int* aborted) {
+    if (segments == 0) return true;
+    for (uint32_t i = 0; i < limit; ++i) {
+        uint32_t have;
+        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(have) : "r"(smem_u32(done)) : "memory");
+        if (have >= segments) return true;
+        if ((i & 15) == 15) {
+            if (*aborted) return false;
+            __nanosleep(200);
+        }
+    }
+    return false;
+}
 
 // the dot product a pair at distance <= t reaches at least (t < 0: none does), twice
 __device__ __forceinline__ __half2 dot_of_distance(int symbols, int K, int t) {
@@ -542,9 +562,11 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                 if (!begun) {
                     // the rows' other warp has to be done with the segment before, whose codes and limits are replaced
                     begun = true;
-                    for (uint32_t polls = 0; *reinterpret_cast<volatile uint32_t*>(&finished[warp ^ 8]) < segment && polls < kWaitLimit && !*aborted;)
-                        ++polls;
-                    __syncwarp();
+                    ok = handed_over(&finished[warp ^ 8], segment, a.handover_polls, aborted);
+                    if (__ballot_sync(kFull, !ok)) {
+                        ok = false;
+                        break;
+                    }
                     const uint32_t row = row0 + lane;
                     const bool wanted = row >= a.row_begin && row < a.row_end;
                     limit[side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
@@ -653,7 +675,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                 begun = false;
                 __syncwarp();
                 ++segment;
-                if (lane == 0) *reinterpret_cast<volatile uint32_t*>(&finished[warp]) = segment;
+                if (lane == 0) hand_over(&finished[warp], segment);
             }
             if (++ct == a.split.cts) ct = 0, ++rt;
         }
@@ -828,6 +850,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.counts = reinterpret_cast<uint32_t*>(take(counts_b));
     a.status = h->d_status.as<uint32_t>();
     a.first_wait_polls = h->first_wait_polls;
+    a.handover_polls = h->handover_polls;
 
     LaunchTimer timer(h, kKernelKnn, st);
     const uint64_t cells = tiles * shape.chunks * kMmaRows;

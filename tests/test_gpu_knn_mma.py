@@ -122,6 +122,18 @@ def test_lost_wait_leaves_empty_rows(cp, oracle):
     check(idx, oracle, codes, 64, (0, 300))
 
 
+def test_lost_handover_is_reported(cp, oracle):
+    # 17 x 17 tiles over 148 blocks: some take steps of two row tiles, whose second waits for the end of the first
+    codes = np.random.default_rng(5).integers(0, 256, (4300, 32)).astype(np.uint8)
+    idx = index(cp, 128, 32, 1)
+    idx.set_param("handover_polls", 0)
+    with pytest.raises(cp.CPHNSWError) as err:
+        idx.knn_graph(codes, 16)
+    assert "[%d]" % cp.E_DEVICE_WAIT in str(err.value)
+    idx.set_param("handover_polls", idx.get_param("first_wait_polls"))
+    check(idx, oracle, codes, 16)
+
+
 def test_unsupported_codes_are_refused(cp):
     idx = index(cp, 128, 100, 1)
     with pytest.raises(cp.CPHNSWError):
