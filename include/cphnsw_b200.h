@@ -118,7 +118,8 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *                 every distance summed in fp32 in d order; O(n^2 d) build, search unchanged; with "prune" = 0 the M exact
  *                 nearest are the links; incremental add_batch keeps choosing by code distance),
  *   "first_wait_polls" (0..2^22, default 2^22: polls granted to the FIRST bounded wait of a kNN-graph launch; a test
- *                 sets 0 to make that wait give up, which the call reports as CPHNSW_B200_E_DEVICE_WAIT) and "handover_polls"
+ *                 sets 0 to make that wait give up, which the call reports as CPHNSW_B200_E_DEVICE_WAIT; the tensor-core
+ *                 sweep of an exact search has the same first wait, and one that is lost there costs time only) and "handover_polls"
  *                 (the same range and default, for the waits inside a tensor-core kNN launch for a row tile's end),
  *   "entry_scan" (evenly spaced nodes scored for every query before the walk; default = k_entry),
  *   "k_entry" (1..100, default 4: how many of the scored nodes, the best, seed the walk). */

@@ -169,7 +169,8 @@ struct SweepArgs {
     uint32_t nq, groups;   // groups: maxima per query (8 per tile)
     Split split;
     float* maxima;         // [nq][groups]
-    uint32_t* status;
+    uint32_t* status;      // this call's own: a lost wait sends the queries to exact_topk_kernel, no result is invalid
+    uint32_t first_wait_polls;
 };
 
 __global__ void __launch_bounds__(kXmThreads, 1) exact_sweep_kernel(SweepArgs a) {
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(kXmThreads, 1) exact_sweep_kernel(SweepArgs a)
         bool ok = true;
         for (uint32_t i = 0; i < steps && ok; ++i) {
             const uint32_t s = i & 1;
-            ok = __all_sync(kFull, wait_or_abort(&full_bar[s], (i >> 1) & 1, kWaitLimit, aborted) && !*aborted);
+            ok = __all_sync(kFull, wait_or_abort(&full_bar[s], (i >> 1) & 1, i == 0 ? a.first_wait_polls : kWaitLimit, aborted) && !*aborted);
             for (int h = 0; h < 2 && ok; ++h) {
                 if (i) ok = __all_sync(kFull, wait_or_abort(&tempty_bar[h][s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted));
                 if (!ok) break;
@@ -521,7 +522,8 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
     float* maxima = reinterpret_cast<float*>(p + 256 + base_b + q_b);
     float2* per_query = reinterpret_cast<float2*>(p + 256 + base_b + q_b + max_b);
 
-    CPB_CUDA(cudaMemsetAsync(stat, 0, 8, st));
+    uint32_t* status = stat + 2;
+    CPB_CUDA(cudaMemsetAsync(stat, 0, 12, st));
     const unsigned stat_blocks = unsigned(h->sm_count) * 8;
     row_stats_kernel<<<stat_blocks, 256, 0, st>>>(d_base, n, dim, stat, nullptr);
     const uint64_t cells = tiles * kMmaRows * chunks;
@@ -547,7 +549,8 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
         a.split.steps = rts * tiles;
         a.split.blocks = uint32_t(a.split.steps < uint64_t(h->sm_count) ? a.split.steps : uint64_t(h->sm_count));
         a.maxima = maxima;
-        a.status = h->d_status.as<uint32_t>();
+        a.status = status;
+        a.first_wait_polls = h->first_wait_polls;
         exact_sweep_kernel<<<a.split.blocks, kXmThreads, 3 * operand_bytes, st>>>(a);
         PickArgs b;
         b.maxima = maxima;
@@ -555,7 +558,7 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
         b.queries = qs;
         b.stat = stat;
         b.per_query = per_query;
-        b.status = h->d_status.as<uint32_t>();
+        b.status = status;
         b.n = n;
         b.groups = uint32_t(groups);
         b.k = k;

@@ -92,3 +92,19 @@ def test_awkward_values(cp, kind):
         _, (ids, dist) = exact(cp, base, q, k)
         wi, wd = plain(base, q, k)
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd, equal_nan=True)
+
+
+def test_lost_wait_costs_no_result(cp):
+    # the sweep's first wait gets no polls: every query is answered the plain way, and nothing is left behind that a later
+    # call on the handle would report as its own
+    base, q = synthetic.gaussian_mixture(17000, 300, 64, 17, 0.3, 9)
+    idx = cp.CPHNSWIndex(64, K=32, M=16)
+    idx.set_exact_base(base)
+    idx.set_param("first_wait_polls", 0)
+    ids, dist = idx.exact_search_batch(q, 10)
+    wi, wd = cpu(base, q, 10)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+    idx.check_device_status()
+    idx.set_param("first_wait_polls", 1 << 22)
+    idx.add_batch_parallel(base[:5000])
+    assert idx.size() == 5000
