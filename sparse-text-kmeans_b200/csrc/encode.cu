@@ -230,7 +230,10 @@ encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, in
         if (QUERY && t < rows) {
             if (mags) mags[row * K + r] = fabsf(win);
             if (rotated) {
-                float4* out = reinterpret_cast<float4*>(rotated + (row * K + r) * P);
+                float* out = rotated + (row * K + r) * P;
+                // (at 128 the code for both makes every small call 2 us longer, 10.7 us for 30 vectors against 8.8:
+                // launch_encode sends other addresses elsewhere)
+                const bool wide = P == 128 || (reinterpret_cast<uintptr_t>(rotated) & 15) == 0;
 #pragma unroll
                 for (int c = 0; c < P / 4; ++c) {
                     float a0, a1, a2, a3;
@@ -241,7 +244,8 @@ encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, in
                     o.y = (__popc((4 * c + 1) & flip_mask) & 1) ? -a1 : a1;
                     o.z = (__popc((4 * c + 2) & flip_mask) & 1) ? -a2 : a2;
                     o.w = (__popc((4 * c + 3) & flip_mask) & 1) ? -a3 : a3;
-                    out[c] = o;
+                    if (wide) reinterpret_cast<float4*>(out)[c] = o;
+                    else out[4 * c] = o.x, out[4 * c + 1] = o.y, out[4 * c + 2] = o.z, out[4 * c + 3] = o.w;
                 }
             }
         }
@@ -728,12 +732,14 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     const float* signs = h->d_signs.as<float>();
     LaunchTimer timer(h, kKernelEncode, st);
     const bool query = d_rot || d_mag;
+    // (a buffer for the rotated vectors off a 16-byte boundary: the kernels with scalar stores)
+    const bool wide = (reinterpret_cast<uintptr_t>(d_rot) & 15) == 0;
     // 256 and 512: lanes in groups from two to four blocks an SM on; fewer vectors leave most of a group's long chain of
     // instructions exposed (one of 256: 10.7 us against 6.6; 1,000: 31 against 29; 500 of 512: 33 against 41).  Rotated
     // vectors of 256 stay with the warp kernel, whose stores are whole lines (2,000: 58 us against 65).
-    const uint64_t group_tiles = P == 512 || (P == 256 && !query) ? (n * (P / 128) + kTileVecs - 1) / kTileVecs : 0;
+    const uint64_t group_tiles = (P == 512 && wide) || (P == 256 && !query) ? (n * (P / 128) + kTileVecs - 1) / kTileVecs : 0;
 
-    if (P == 32 || P == 64 || P == 128) {
+    if (P == 32 || P == 64 || (P == 128 && wide)) {
         const uint64_t tiles = (n + kTileVecs - 1) / kTileVecs;
         const int rpb = rotations_per_block(tiles, uint64_t(h->sm_count) * (P == 128 ? 6 : 12), K);
         const size_t smem = size_t(kTileVecs) * (P + 2) * sizeof(float) + size_t(2) * 3 * P * sizeof(float) + size_t(kTileVecs) * rpb * h->comp_bytes;

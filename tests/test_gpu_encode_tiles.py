@@ -24,3 +24,25 @@ def test_encode_tiles_match_oracle(oracle, dim, cb, n, K, conv):
     assert np.array_equal(codes, want)
     assert np.array_equal(mag, wmag)
     assert np.array_equal(rot, wrot)  # a zero's sign apart
+
+
+@pytest.mark.parametrize("dim,cb", [(20, 1), (64, 1), (100, 1), (256, 2), (500, 2), (700, 2)])
+@pytest.mark.parametrize("n", [1, 300])
+def test_rotated_vectors_to_any_float_address(dim, cb, n):
+    # the buffer for the rotated vectors starts one to three floats past a 16-byte boundary
+    import torch
+    import cphnsw_b200 as cp
+    K = 12
+    x = torch.randn((n, dim), device="cuda")
+    idx = cp.CPHNSWIndex(dim, M=8, ef_construction=8, K=K, component_bytes=cb)
+    P = 1 << (dim - 1).bit_length()
+    st = torch.cuda.current_stream().cuda_stream
+    codes = torch.empty(n * K * cb, dtype=torch.uint8, device="cuda")
+    want = None
+    for off in range(4):
+        buf = torch.full((n * K * P + 8,), 7.0, device="cuda")
+        idx.encode_dev(x.data_ptr(), n, codes.data_ptr(), buf.data_ptr() + 4 * off, stream=st)
+        assert bool((buf[:off] == 7).all()) and bool((buf[off + n * K * P:] == 7).all())
+        rot = buf[off:off + n * K * P].cpu().numpy()
+        want = rot if want is None else want
+        assert np.array_equal(rot, want)
