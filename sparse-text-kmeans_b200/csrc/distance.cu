@@ -636,14 +636,21 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
         set_error("knn_kernel=3 (tensor-core filter) needs plain codes of 2 to 64 components");
         return CPHNSW_B200_E_UNSUPPORTED;
     }
-    // (rows of whole 16-byte words are read in place and have to be aligned then)
-    const bool readable = (reinterpret_cast<uintptr_t>(d_codes) & 15) == 0 || size_t(h->K) * h->comp_bytes != size_t(WC) * 4;
+    // rows of whole 16-byte words are read in place and have to be aligned then; other rows are copied byte by byte, but the
+    // filter and the bit planes read components
+    const uintptr_t at = reinterpret_cast<uintptr_t>(d_codes);
+    const bool components = at % h->comp_bytes == 0;
+    const bool readable = components && ((at & 15) == 0 || size_t(h->K) * h->comp_bytes != size_t(WC) * 4);
+    if (h->knn_kernel >= 2 && !components) {
+        set_error("device code buffer must be aligned to its components");
+        return CPHNSW_B200_E_INVALID;
+    }
     if (h->knn_kernel == 3 || (h->knn_kernel == 0 && n >= kMmaMinNodes && readable && knn_mma_supported(h))) {
         const uint32_t* pc;
         CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
         return launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist, st);
     }
-    if (h->knn_kernel != 1 && knn_sliced_supported(h))
+    if (h->knn_kernel != 1 && components && knn_sliced_supported(h))
         return launch_knn_graph_sliced(h, d_codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
     const bool u16 = h->comp_bytes == 2;
     const uint32_t* pc;

@@ -90,6 +90,26 @@ def test_codes_off_a_sector_boundary(cp, oracle, K, cb):
         assert np.array_equal(nbrs.cpu().numpy().view(np.uint32), wn)
 
 
+def test_two_byte_codes_at_an_odd_address(cp, oracle):
+    # rows of 20 bytes are copied byte by byte into padded ones: any address will do
+    import torch
+    n, K, k = 4200, 10, 20
+    codes = np.random.default_rng(8).integers(0, 8, (n, K)).astype(np.uint16)
+    wn, _ = oracle.knn_graph(codes, k, 0, n)
+    idx = cp.CPHNSWIndex(300, K=K, component_bytes=2)
+    buf = torch.zeros(n * K * 2 + 16, dtype=torch.uint8, device="cuda")
+    nbrs = torch.zeros((n, k), dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    for offset in (0, 1, 2):
+        buf[offset:offset + n * K * 2] = torch.from_numpy(codes.reshape(-1).view(np.uint8)).cuda()
+        nbrs.zero_()
+        idx.knn_graph_dev(buf.data_ptr() + offset, n, k, 0, n, nbrs.data_ptr(), stream=st)
+        assert np.array_equal(nbrs.cpu().numpy().view(np.uint32), wn)
+    idx.set_param("knn_kernel", 3)
+    with pytest.raises(ValueError):
+        idx.knn_graph_dev(buf.data_ptr() + 1, n, k, 0, n, nbrs.data_ptr(), stream=st)
+
+
 def test_lost_wait_is_reported(cp, oracle):
     # the first wait gets no polls: every role of the block ends and the call reports it; the handle stays usable
     codes = np.random.default_rng(3).integers(0, 256, (3000, 32)).astype(np.uint8)
