@@ -86,7 +86,8 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *                 in binary-code mode, K = 16/32 with uint16 codes of padded dim 1024, and one-byte binary codes of
  *                 any K <= 120 that is a multiple of 8, residual bits included when the primary part is one too),
  *   "search_kernel" (0 = pick: the walk that expands several nodes a step whenever M <= 32; 1 = one node a step, any M;
- *                    2 = the walk of several nodes, an error when M > 32; both return identical results),
+ *                    2 = the walk of several nodes, an error when M > 32 (walks under the code distance - multiprobe, insertion,
+ *                    binary codes - take the other one then); both return identical results),
  *   "binary_codes" (0/1, before any vector is added: 1 = the unified index's primary binary code
  *                   (include/cphnsw/core/codes.hpp:76-129 with R = 0): a component keeps only its sign bit, so
  *                   code distance = Hamming distance and the graph is built under it; search / search_and_rerank

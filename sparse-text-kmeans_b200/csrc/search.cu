@@ -686,7 +686,7 @@ int launch_search(cphnsw_b200_index* h, SearchCtx& cx, const float* d_q, const f
 
     // several expansions per step: rows of up to 32 links, any metric and beam
     const bool walk_ok = !scan_only && h->M <= 32;
-    if (h->search_kernel == 2 && !walk_ok && !scan_only) {
+    if (h->search_kernel == 2 && !walk_ok && !scan_only && !sym) {
         set_error("search_kernel=2 needs M <= 32");
         return CPHNSW_B200_E_UNSUPPORTED;
     }

@@ -60,3 +60,21 @@ def test_repeated_ids_in_a_row_count_once(cp, oracle, M, row, a, b):
         ids, dist = idx.search_batch(q, 20, 200)
         wi, wd = oracle.search(rot, codes, adj, idx.entry_ids(), 200, 20, n_seed=4)
         assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
+def test_wide_rows_with_the_walk_asked_for(cp):
+    # M = 48: a search under the asymmetric score is refused, walks under the code distance take the one-warp kernel
+    base, q = synthetic.gaussian_mixture(1200, 20, 64, 4, 0.3, 3)
+    out = []
+    for kernel in (2, 1):
+        idx = cp.CPHNSWIndex(64, M=48, ef_construction=64, K=32)
+        idx.set_param("search_kernel", kernel)
+        idx.add_batch_parallel(base[:1000])
+        idx.add_batch(base[1000:])
+        ids, dist = idx.search_multiprobe_batch(q, 10, 100, 3)
+        out.append((idx.adjacency(), ids, dist))
+        if kernel == 2:
+            with pytest.raises(cp.CPHNSWError):
+                idx.search_batch(q, 10, 100)
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
