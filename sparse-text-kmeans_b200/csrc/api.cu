@@ -534,7 +534,7 @@ void cphnsw_b200_index::release_buffers() {
     QuietDevice quiet;  // one wait for all of them
     ctxs.clear();
     for (DevBuf* b : {&d_signs, &d_signbits, &d_status, &d_vectors, &d_codes, &d_adj, &d_entry, &d_entry_codes, &d_entry_scan, &d_packed,
-                      &d_exact_base, &d_qtables, &d_qcodes, &d_q, &s_in, &s_in2, &s_out, &s_out2, &s_pad, &s_pad2, &s_sliced, &s_flags, &s_rank,
+                      &d_exact_base, &d_qtables, &d_qcodes, &d_q, &s_in, &s_in2, &s_out, &s_out2, &s_pad, &s_pad2, &s_sliced, &s_exact, &s_flags, &s_rank,
                       &s_kept})
         b->release();
 }

@@ -215,7 +215,9 @@ struct cphnsw_b200_index {
     cpb::DevBuf d_qtables, d_qcodes, d_q;
     // stage scratch for the host-pointer entry points
     cpb::DevBuf s_in, s_in2, s_out, s_out2, s_pad, s_pad2, s_sliced;
-    cpb::DevBuf s_flags;         // exact search: queries the tensor-core filter could not settle
+    // exact search through the tensor cores: workspace, queries it could not settle (not shared with the graph stages, which
+    // may be in flight on another stream)
+    cpb::DevBuf s_exact, s_flags;
     cpb::DevBuf s_rank, s_kept;  // rank-based pruning: reverse lists, kept rows
 
     std::atomic<uint64_t> launches{0};

@@ -108,3 +108,34 @@ def test_lost_wait_costs_no_result(cp):
     idx.set_param("first_wait_polls", 1 << 22)
     idx.add_batch_parallel(base[:5000])
     assert idx.size() == 5000
+
+
+def test_beside_a_graph_on_another_stream(cp):
+    # a kNN graph and an exact search of one handle in flight on two streams: no workspace in common
+    import torch
+    n, nq, dim = 40000, 400, 128
+    base, q = synthetic.gaussian_mixture(n, nq, dim, 40, 0.3, 21)
+    idx = cp.CPHNSWIndex(dim, K=32)
+    d_base, d_q = torch.from_numpy(base).cuda(), torch.from_numpy(q).cuda()
+    codes = torch.from_numpy(idx.encode(base)).cuda()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def graph():
+        nbrs = torch.empty((n, 64), dtype=torch.int32, device="cuda")
+        idx.knn_graph_dev(codes.data_ptr(), n, 64, 0, n, nbrs.data_ptr(), stream=a.cuda_stream)
+        return nbrs
+
+    def search():
+        ids, dist = torch.empty((nq, 10), dtype=torch.int32, device="cuda"), torch.empty((nq, 10), device="cuda")
+        idx.exact_search_dev(d_base.data_ptr(), n, d_q.data_ptr(), nq, 10, ids.data_ptr(), dist.data_ptr(), stream=b.cuda_stream)
+        return ids
+
+    torch.cuda.synchronize()
+    g0 = graph()
+    torch.cuda.synchronize()
+    s0 = search()
+    torch.cuda.synchronize()
+    got = [(graph(), search()) for _ in range(4)]
+    torch.cuda.synchronize()
+    for g, s in got:
+        assert bool((g == g0).all()) and bool((s == s0).all())
