@@ -122,6 +122,10 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *                 sets 0 to make that wait give up, which the call reports as CPHNSW_B200_E_DEVICE_WAIT; the tensor-core
  *                 sweep of an exact search has the same first wait, and one that is lost there costs time only) and "handover_polls"
  *                 (the same range and default, for the waits inside a tensor-core kNN launch for a row tile's end),
+ *   "workspace_limit_mb" (default 0 = no limit: the most MiB of device memory a tensor-core filter's workspace may take.
+ *                 A kNN graph's is about 300 bytes a node plus 0.2 to 0.4 GB, an exact search's 2 bytes a base coordinate
+ *                 plus up to 0.5 GB; both stay with the handle.  Above the limit, and when the device has no memory for
+ *                 it, the kernels without a filter answer, with the same results),
  *   "entry_scan" (evenly spaced nodes scored for every query before the walk; default = k_entry),
  *   "k_entry" (1..100, default 4: how many of the scored nodes, the best, seed the walk). */
 int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double value);

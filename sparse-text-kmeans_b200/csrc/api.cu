@@ -751,6 +751,11 @@ int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double v) {
         (s == "first_wait_polls" ? h->first_wait_polls : h->handover_polls) = uint32_t(v);
         return 0;
     }
+    if (s == "workspace_limit_mb") {
+        if (!(v >= 0) || v > 1048576.0) { set_error("workspace_limit_mb must be in 0..2^20 (0 = no limit)"); return CPHNSW_B200_E_INVALID; }
+        h->workspace_limit = size_t(v * 1048576.0);
+        return 0;
+    }
     if (s == "rank_prune") { h->rank_prune = v != 0.0; return 0; }
     if (s == "exact_edges") { h->exact_edges = v != 0.0; return 0; }
     if (s == "rank_pruning_alpha") {
@@ -800,6 +805,7 @@ int cphnsw_b200_get_param(const cphnsw_b200_index* h, const char* name, double* 
     else if (s == "build_seed") *v = h->build_seed;
     else if (s == "first_wait_polls") *v = h->first_wait_polls;
     else if (s == "handover_polls") *v = h->handover_polls;
+    else if (s == "workspace_limit_mb") *v = double(h->workspace_limit) / 1048576.0;
     else if (s == "rank_prune") *v = h->rank_prune;
     else if (s == "exact_edges") *v = h->exact_edges;
     else if (s == "rank_pruning_alpha") *v = h->rank_pruning_alpha;

@@ -54,7 +54,8 @@ inline cudaError_t allow_max_dynamic_smem(F* kernel) {
 // dropped spent most of its time in cudaMalloc and cudaFree.  What is kept is bounded (device_memory.cu), shrinks when the
 // device's last handle goes, and is returned to the driver as a whole when an allocation fails.  device_free waits for the
 // device like cudaFree does, unless the calling thread is inside a QuietDevice (which has waited already).
-int device_alloc(void** p, size_t* bytes, int* device);
+// room (optional): set to false, and no error, when the device has no memory for the block.
+int device_alloc(void** p, size_t* bytes, int* device, bool* room = nullptr);
 void device_free(void* p, size_t bytes, int device);
 void device_handle_created(int device);
 void device_handle_destroyed(int device);
@@ -85,11 +86,11 @@ struct DevBuf {
         bytes = 0;
     }
     // grow-only; contents are not preserved
-    int reserve(size_t n) {
+    int reserve(size_t n, bool* room = nullptr) {
         if (n <= bytes && p) return 0;
         release();
         if (n == 0) n = 16;
-        CPB_TRY(device_alloc(&p, &n, &device));
+        CPB_TRY(device_alloc(&p, &n, &device, room));
         bytes = n;
         return 0;
     }
@@ -218,6 +219,7 @@ struct cphnsw_b200_index {
     // exact search through the tensor cores: workspace, queries it could not settle (not shared with the graph stages, which
     // may be in flight on another stream)
     cpb::DevBuf s_exact, s_flags;
+    size_t workspace_limit = 0;  // most bytes the workspace of a tensor-core filter may take (0: what the device has)
     cpb::DevBuf s_rank, s_kept;  // rank-based pruning: reverse lists, kept rows
 
     std::atomic<uint64_t> launches{0};
@@ -247,6 +249,11 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
 bool knn_sliced_supported(const cphnsw_b200_index* h);
 int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
                             uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
+// What the two tensor-core filters return instead of running when there is no room for their workspace: the kernels
+// without one, which need a fraction of it, answer then.
+constexpr int kNoRoom = 1;
+// `bytes` of workspace within the handle's limit and the device's memory, else kNoRoom
+int reserve_workspace(const cphnsw_b200_index* h, DevBuf& buf, size_t bytes);
 // tensor-core filter and exact distances of the pairs that pass (knn_mma.cu); padded: code rows of `words` 32-bit words
 bool knn_mma_supported(const cphnsw_b200_index* h);
 int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,

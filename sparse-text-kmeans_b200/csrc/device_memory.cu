@@ -38,7 +38,7 @@ thread_local int quiet_depth = 0;
 
 }  // namespace
 
-int device_alloc(void** p, size_t* bytes, int* device) {
+int device_alloc(void** p, size_t* bytes, int* device, bool* room) {
     CPB_CUDA(cudaGetDevice(device));
     const size_t n = (*bytes + 511) & ~size_t(511);
     if (*device < kMaxDevices) {
@@ -62,9 +62,23 @@ int device_alloc(void** p, size_t* bytes, int* device) {
         pool.trim(0);
         e = cudaMalloc(p, n);
     }
+    if (e == cudaErrorMemoryAllocation && room) {
+        cudaGetLastError();  // the caller goes on without
+        *room = false;
+        *p = nullptr;
+        *bytes = 0;
+        return 0;
+    }
     CPB_CUDA(e);
     *bytes = n;
     return 0;
+}
+
+int reserve_workspace(const cphnsw_b200_index* h, DevBuf& buf, size_t bytes) {
+    if (h->workspace_limit && bytes > h->workspace_limit) return kNoRoom;
+    bool room = true;
+    CPB_TRY(buf.reserve(bytes, &room));
+    return room ? 0 : kNoRoom;
 }
 
 void device_free(void* p, size_t bytes, int device) {

@@ -648,7 +648,12 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
     if (h->knn_kernel == 3 || (h->knn_kernel == 0 && n >= kMmaMinNodes && readable && knn_mma_supported(h))) {
         const uint32_t* pc;
         CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
-        return launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+        const int rc = launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+        if (rc != kNoRoom) return rc;
+        if (h->knn_kernel == 3) {
+            set_error("knn_kernel=3 (tensor-core filter): no device memory for its workspace");
+            return CPHNSW_B200_E_CUDA;
+        }
     }
     if (h->knn_kernel != 1 && components && knn_sliced_supported(h))
         return launch_knn_graph_sliced(h, d_codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);

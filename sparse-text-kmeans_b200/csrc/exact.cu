@@ -332,8 +332,11 @@ int launch_exact_search(cphnsw_b200_index* h, const float* d_base, uint64_t n, c
     const uint8_t* wanted = nullptr;
     if (exact_mma_supported(h, n, nq, k)) {
         CPB_TRY(h->s_flags.reserve(nq));
-        CPB_TRY(launch_exact_mma(h, d_base, n, d_q, nq, k, d_ids, d_dist, h->s_flags.as<uint8_t>(), st));
-        wanted = h->s_flags.as<uint8_t>();  // what the filter could not settle
+        const int rc = launch_exact_mma(h, d_base, n, d_q, nq, k, d_ids, d_dist, h->s_flags.as<uint8_t>(), st);
+        if (rc != kNoRoom) {
+            CPB_TRY(rc);
+            wanted = h->s_flags.as<uint8_t>();  // what the filter could not settle
+        }
     }
     if (k <= 32) return launch_exact_t<1, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, wanted, st);
     if (k <= 64) return launch_exact_t<2, 4>(h, d_base, n, d_q, nq, k, d_ids, d_dist, wanted, st);

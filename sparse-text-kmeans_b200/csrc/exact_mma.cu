@@ -514,7 +514,7 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t base_b = up(size_t(tiles) * operand_bytes), q_b = up(size_t(qtiles) * operand_bytes);
     const size_t max_b = up(size_t(batch) * groups * 4), row_b = up(size_t(batch) * 8);
-    CPB_TRY(h->s_exact.reserve(256 + base_b + q_b + max_b + row_b));
+    CPB_TRY(reserve_workspace(h, h->s_exact, 256 + base_b + q_b + max_b + row_b));
     unsigned char* p = h->s_exact.as<unsigned char>();
     uint32_t* stat = reinterpret_cast<uint32_t*>(p);
     uint4* base_op = reinterpret_cast<uint4*>(p + 256);

@@ -819,7 +819,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const size_t order_b = up(size_t(kBoundOrders) * n * 4), place_b = order_b, bound_b = up(size_t(n) * 4);
     const size_t slots = segments * kMmaRows * 2;
     const size_t ids_b = up(slots * kMmaCap * 4), dists_b = up(slots * kMmaCap), counts_b = up(slots * 4);
-    CPB_TRY(h->s_sliced.reserve(op_b + hist_b + order_b + place_b + bound_b + ids_b + dists_b + counts_b));
+    CPB_TRY(reserve_workspace(h, h->s_sliced, op_b + hist_b + order_b + place_b + bound_b + ids_b + dists_b + counts_b));
     unsigned char* p = h->s_sliced.as<unsigned char>();
     auto take = [&](size_t b) {
         unsigned char* r = p;

@@ -139,3 +139,27 @@ def test_beside_a_graph_on_another_stream(cp):
     torch.cuda.synchronize()
     for g, s in got:
         assert bool((g == g0).all()) and bool((s == s0).all())
+
+
+def test_no_room_for_the_filters(cp, oracle):
+    # the workspaces of both filters above the limit: the kernels without one answer
+    base, q = synthetic.gaussian_mixture(17000, 40, 64, 17, 0.3, 33)
+    idx = cp.CPHNSWIndex(64, K=32)
+    idx.set_param("workspace_limit_mb", 2)
+    idx.set_exact_base(base)
+    before = idx.launch_count()
+    ids, dist = idx.exact_search_batch(q, 10)
+    assert idx.launch_count() - before <= 2
+    wi, wd = cpu(base, q, 10)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+    codes = idx.encode(base[:5000])
+    before = idx.launch_count()
+    nbrs, d = idx.knn_graph(codes, 32)
+    assert idx.launch_count() - before <= 2
+    wn, wd = oracle.knn_graph(codes, 32, 0, 5000)
+    assert np.array_equal(nbrs, wn) and np.array_equal(d, wd)
+    idx.set_param("knn_kernel", 3)
+    with pytest.raises(cp.CPHNSWError):
+        idx.knn_graph(codes, 32)
+    idx.set_param("workspace_limit_mb", 0)
+    assert np.array_equal(idx.knn_graph(codes, 32)[0], wn)
