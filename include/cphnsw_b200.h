@@ -82,7 +82,8 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *            candidates are the links, build_with_gpu_knn(..., prune = false), evaluation/test_gpu_build.cpp:168-174),
  *   "knn_k" (candidates per node fed to select_neighbors, default min(2*M, 64)),
  *   "knn_kernel" (0 = pick; 3 = tensor-core filter in front of exact distances, plain codes of 2 to 64 components,
- *                 what 0 picks from 4,096 nodes on; 1 = byte-wise distance, 2 = bit-sliced distance; K = 16/32/64 with uint8 codes or
+ *                 what 0 picks from 4,096 nodes on unless a sample shows data without clusters, of which it would let
+ *                 most pairs through; 1 = byte-wise distance, 2 = bit-sliced distance; K = 16/32/64 with uint8 codes or
  *                 in binary-code mode, K = 16/32 with uint16 codes of padded dim 1024, and one-byte binary codes of
  *                 any K <= 120 that is a multiple of 8, residual bits included when the primary part is one too),
  *   "search_kernel" (0 = pick: the walk that expands several nodes a step whenever M <= 32; 1 = one node a step, any M;

@@ -246,18 +246,22 @@ int launch_code_distance(cphnsw_b200_index* h, const void* d_a, uint64_t na, con
 int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
                      uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
 // bit-sliced variant of the kNN kernel (uint8 components, K = 16 or 32)
+struct SweepChoice;  // knn_common.cuh
 bool knn_sliced_supported(const cphnsw_b200_index* h);
 int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
-                            uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
+                            uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, const SweepChoice& choice, cudaStream_t st);
 // What the two tensor-core filters return instead of running when there is no room for their workspace: the kernels
 // without one, which need a fraction of it, answer then.
 constexpr int kNoRoom = 1;
 // `bytes` of workspace within the handle's limit and the device's memory, else kNoRoom
 int reserve_workspace(const cphnsw_b200_index* h, DevBuf& buf, size_t bytes);
-// tensor-core filter and exact distances of the pairs that pass (knn_mma.cu); padded: code rows of `words` 32-bit words
+// tensor-core filter and exact distances of the pairs that pass (knn_mma.cu); padded: code rows of `words` 32-bit words;
+// other (optional): the choice to launch another kernel with, which then runs where a warp would
+// spend more than most_turns turns on the pairs of a tile that pass
 bool knn_mma_supported(const cphnsw_b200_index* h);
 int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,
-                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st);
+                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, double most_turns,
+                         SweepChoice* other, cudaStream_t st);
 int launch_select_neighbors(cphnsw_b200_index* h, const void* d_codes, uint64_t n, const uint32_t* d_cand,
                             uint32_t k, uint64_t row_begin, uint64_t row_end, uint32_t M, int keep_pruned,
                             uint32_t* d_adj, cudaStream_t st, const uint32_t* d_row_ids = nullptr);

@@ -142,7 +142,8 @@ template <int WC, bool U16, int SLOTS, int Q, bool WEIGHTED>
 __global__ void __launch_bounds__(kKnnThreads)
 knn_graph_kernel(const uint32_t* __restrict__ codes, uint64_t n, uint32_t k, uint64_t row_begin,
                  uint64_t row_end, uint32_t* __restrict__ nbrs, uint16_t* __restrict__ dists,
-                 uint32_t* __restrict__ status, uint32_t first_wait_polls, CodeWeights cwt) {
+                 uint32_t* __restrict__ status, uint32_t first_wait_polls, CodeWeights cwt, SweepChoice choice) {
+    if (choice.skip()) return;
     constexpr int CH = WC / 4;  // 16-byte chunks per code row
     constexpr int CHLOG = CH == 1 ? 0 : (CH == 2 ? 1 : (CH == 4 ? 2 : 3));
     constexpr int kKnnTile = KnnTile<WC>::value;
@@ -576,15 +577,14 @@ int launch_code_distance(cphnsw_b200_index* h, const void* d_a, uint64_t na, con
 
 template <int WC, bool U16, int SLOTS, int Q, bool WEIGHTED>
 static int launch_knn_w(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
-                        uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
+                        uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
     const size_t smem = size_t(2) * KnnTile<WC>::value * WC * 4;
     auto kernel = knn_graph_kernel<WC, U16, SLOTS, Q, WEIGHTED>;
     CPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const uint64_t rows = re - rb;
     const uint64_t blocks = (rows + kKnnWarps * Q - 1) / (kKnnWarps * Q);
-    LaunchTimer timer(h, kKernelKnn, st);
     kernel<<<unsigned(blocks), kKnnThreads, smem, st>>>(codes, n, k, rb, re, nbrs, dist, h->d_status.as<uint32_t>(), h->first_wait_polls,
-                                                       code_weights(h));
+                                                       code_weights(h), choice);
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     return 0;
@@ -593,23 +593,43 @@ static int launch_knn_w(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n,
 // the weighted (residual-code) distance is a separate instantiation: the plain count pays nothing for it
 template <int WC, bool U16, int SLOTS, int Q>
 static int launch_knn_t(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
-                        uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
-    if (h->residual_bits) return launch_knn_w<WC, U16, SLOTS, Q, true>(h, codes, n, k, rb, re, nbrs, dist, st);
-    return launch_knn_w<WC, U16, SLOTS, Q, false>(h, codes, n, k, rb, re, nbrs, dist, st);
+                        uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
+    if (h->residual_bits) return launch_knn_w<WC, U16, SLOTS, Q, true>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+    return launch_knn_w<WC, U16, SLOTS, Q, false>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
 }
 
 template <int WC, bool U16>
 static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
-                            uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
+                            uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
     constexpr int Q = WC == 32 ? 2 : (WC == 16 ? 4 : 8);
     const uint32_t need = k + 1;  // the row's own id may occupy one place
-    if (need <= 64) return launch_knn_t<WC, U16, 2, Q>(h, codes, n, k, rb, re, nbrs, dist, st);
-    if (need <= 96) return launch_knn_t<WC, U16, 3, Q>(h, codes, n, k, rb, re, nbrs, dist, st);
-    return launch_knn_t<WC, U16, 4, Q>(h, codes, n, k, rb, re, nbrs, dist, st);
+    if (need <= 64) return launch_knn_t<WC, U16, 2, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+    if (need <= 96) return launch_knn_t<WC, U16, 3, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+    return launch_knn_t<WC, U16, 4, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
 }
 
 // From this many nodes on the tensor-core kernel is taken; below it the launches around it cost more than the sweep.
 constexpr uint64_t kMmaMinNodes = 4096;
+// Where the data let too many pairs through its filter the bit-sliced or the byte-wise kernel is taken, which cost the same
+// whatever the data: most_turns is the load (see knn_mma.cu) up to which the filter is the faster, from measured picoseconds
+// a pair.  Filter: 1.2 and 0.01 to 0.02 a turn, by the bytes of a code.  Bit-sliced, K = 32: 1.1 at 400k rows, 1.9 at 100k,
+// 7.5 at 20k (a wave of blocks sweeps all nodes however few rows it has), in proportion to the planes; byte-wise 3 at
+// 32-byte codes, 9 at 64.  Unit sphere, 100k x 128, K = 32: 17.4 ms against 58 through the filter; mixtures of 1,000 points
+// a cluster: sigma 0.3 3.2 against 19.3, sigma 0.7 19.3 against 28.6.
+static double most_turns(const cphnsw_b200_index* h, uint64_t rows, bool sliced) {
+    const double bytes = double(h->K) * h->comp_bytes, planes = h->K * (h->comp_bytes == 2 ? 11.0 : 8.0);
+    const double other = sliced ? (0.8 + 113e3 / double(rows)) * (0.5 + planes / 512)
+                                : (bytes <= 16 ? 1.5 : bytes <= 32 ? 2.8 : 9.0) + 50e3 / double(rows);
+    const double turns = (other - 1.2) / (0.004 + 0.0002 * bytes);
+    return turns < 12 ? 12 : (turns > 300 ? 300 : turns);
+}
+// Below this many nodes the filter is the faster on any data (4,096 nodes of the unit sphere: 324 to 567 us against 607 to
+// 813 bit-sliced, K = 16 to 64), and the sample is not taken.
+constexpr uint64_t kMmaAlways = 8192;
+// Up to this many components in all the byte-wise kernel beats the bit-sliced one on one-byte codes (unit sphere, n = 16,384,
+// K = 16 / 32 / 64: 744 / 1,385 / 3,098 us against 1,547 / 1,704 / 3,393; n = 30,000: 1,952 / 3,404 / 9,143 against
+// 3,293 / 3,687 / 6,812).
+constexpr uint64_t kBytewiseComponents = 1 << 20;
 
 int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
                      uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
@@ -645,22 +665,28 @@ int launch_knn_graph(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint
         set_error("device code buffer must be aligned to its components");
         return CPHNSW_B200_E_INVALID;
     }
-    if (h->knn_kernel == 3 || (h->knn_kernel == 0 && n >= kMmaMinNodes && readable && knn_mma_supported(h))) {
-        const uint32_t* pc;
+    const bool filter = h->knn_kernel == 3 || (h->knn_kernel == 0 && n >= kMmaMinNodes && readable && knn_mma_supported(h));
+    const bool sliced = h->knn_kernel != 1 && components && knn_sliced_supported(h) &&
+                        !(filter && h->comp_bytes == 1 && n * h->K <= kBytewiseComponents);
+    SweepChoice choice;  // for the kernel without a filter
+    const uint32_t* pc = nullptr;
+    LaunchTimer timer(h, kKernelKnn, st);
+    if (filter) {
         CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
-        const int rc = launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist, st);
-        if (rc != kNoRoom) return rc;
-        if (h->knn_kernel == 3) {
+        const bool asked = h->knn_kernel == 3, always = asked || n < kMmaAlways;
+        const int rc = launch_knn_graph_mma(h, d_codes, pc, WC, n, k, row_begin, row_end, d_nbrs, d_dist,
+                                            most_turns(h, row_end - row_begin, sliced), always ? nullptr : &choice, st);
+        if (rc == kNoRoom && asked) {
             set_error("knn_kernel=3 (tensor-core filter): no device memory for its workspace");
             return CPHNSW_B200_E_CUDA;
         }
+        if (rc != 0 && rc != kNoRoom) return rc;
+        if (rc == 0 && always) return 0;
     }
-    if (h->knn_kernel != 1 && components && knn_sliced_supported(h))
-        return launch_knn_graph_sliced(h, d_codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+    if (sliced) return launch_knn_graph_sliced(h, d_codes, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st);
     const bool u16 = h->comp_bytes == 2;
-    const uint32_t* pc;
-    CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
-#define CALL(W, U) return launch_knn_slots<W, U>(h, pc, n, k, row_begin, row_end, d_nbrs, d_dist, st)
+    if (!pc) CPB_TRY(padded_view(h, d_codes, n, WC, h->s_pad, st, &pc));
+#define CALL(W, U) return launch_knn_slots<W, U>(h, pc, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st)
     CPB_DISPATCH_WC(WC, u16, CALL);
 #undef CALL
     return 0;

@@ -6,6 +6,16 @@
 #include "common.cuh"
 
 namespace cpb {
+
+// Of two sweeps launched one behind the other for the same rows the data decide which runs, on the device (knn_mma.cu):
+// a kernel with a choice ends at once when the measured load is on the other side of `most`.
+struct SweepChoice {
+    const unsigned long long* load = nullptr;  // (nullptr: it runs)
+    unsigned long long most = 0;
+    bool above = false;  // runs above `most` / up to it
+    __device__ __forceinline__ bool skip() const { return load != nullptr && (*load > most) != above; }
+};
+
 namespace knn {
 
 constexpr uint32_t kFull = 0xffffffffu;

@@ -14,7 +14,8 @@
 // orders, every row counted once, bounds its final t from above.  On clustered data t is mostly right or one too high, and
 // some 450 pairs per row pass, 140 of them truly within t.  The pairs found are kept in a buffer; when it runs full its k
 // best are kept and t falls below the worst of them for the pairs still to come, which have higher ids.  On data without
-// clusters the bound says nothing and t is lowered by this alone.
+// clusters the bound says nothing, t is lowered by this alone and most pairs pass: a sample of the data shows it, and the
+// sweep is then left to another kernel ("what the filter is worth" below).
 //
 // Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the candidates
 // in tiles of 256, two stages of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
@@ -66,7 +67,8 @@ __device__ __forceinline__ uint32_t symbol_of(uint32_t comp, uint32_t symbols) {
 // ---- operand: [tile of 256 rows][chunk][row][16 values] ------------------------------------------------------------
 template <typename CompT>
 __global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n, int K, int symbols, int chunks,
-                                    uint4* __restrict__ out, uint64_t tiles) {
+                                    uint4* __restrict__ out, uint64_t tiles, SweepChoice choice) {
+    if (choice.skip()) return;
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= tiles * chunks * kMmaRows) return;
     const int r = int(t % kMmaRows), c = int(t / kMmaRows % chunks);
@@ -233,14 +235,17 @@ constexpr uint32_t kSeenSlots = 1024;
 template <bool U16, int QUADS, bool SECTORS>
 __global__ void __launch_bounds__(kBoundWarps * 32)
 bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t* __restrict__ order, const uint32_t* __restrict__ place,
-             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound) {
+             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound, uint64_t apart /* of LoadArgs: its rows only; 0: all rows */,
+             SweepChoice choice) {
+    if (choice.skip()) return;
     constexpr int S = kBoundWindow / 32, N = kBoundOrders * S;
     __shared__ uint32_t seen_sm[kBoundWarps][kSeenSlots];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t at = uint64_t(blockIdx.x) * kBoundWarps + warp;
     if (at >= n) return;
-    const uint32_t row = order[at];
-    if (row < row_begin || row >= row_end) return;
+    const uint64_t wanted = apart ? row_begin + at / 32 * apart + at % 32 : order[at];
+    if (wanted < row_begin || wanted >= row_end) return;
+    const uint32_t row = uint32_t(wanted);
     uint32_t* seen = seen_sm[warp];
     for (uint32_t i = lane; i < kSeenSlots / 4; i += 32) reinterpret_cast<uint4*>(seen)[i] = make_uint4(kFull, kFull, kFull, kFull);
     const uint32_t where = lane < kBoundOrders ? place[uint64_t(row) * kBoundOrders + lane] : 0u;
@@ -290,6 +295,57 @@ bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t*
     if (lane == 0) bound[row] = T;
 }
 
+// ---- what the filter is worth ----------------------------------------------------------------------------------------
+// On clustered data next to nothing passes it, on data without clusters most pairs do (78 % at the final thresholds on
+// 100k points of the unit sphere, K = 32), and the epilogue's warps spend a turn on every pair of the row that has most of
+// them and one on every 32 of the 32 rows together.  Those turns are counted on a sample before anything else is done:
+// kLoadGroups groups of 32 rows against kLoadTiles candidate tiles each, at the rows' bounds.  Above the caller's limit
+// the sweep is left to another kernel.  (The share of pairs that would pass by chance at the bounds, which needs no pairs,
+// tells less: mixtures of 1,000, 5,000 and 100 points a cluster with shares of 0.4, 0.0 and 3 % took 13, 9 and 26 ms.)
+struct LoadArgs {
+    uint64_t apart;  // groups of rows are so many rows apart
+    uint32_t groups;
+};
+constexpr uint32_t kLoadGroups = 16, kLoadTiles = 16;
+
+// the symbols of a word's components, in their places
+template <bool U16>
+__device__ __forceinline__ uint32_t symbols_of(uint32_t w, uint32_t symbols) {
+    if (U16) return (w ^ (w >> 3 & 0x1fff1fffu) ^ (w >> 6 & 0x03ff03ffu) ^ (w >> 9 & 0x007f007fu)) & ((symbols - 1) * 0x00010001u);
+    return (w ^ (w >> 3 & 0x1f1f1f1fu) ^ (w >> 6 & 0x03030303u)) & ((symbols - 1) * 0x01010101u);
+}
+// a block: 32 rows (their symbols in shared memory) against a tile, a candidate per thread
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kMmaRows) load_kernel(const uint4* __restrict__ codes, uint64_t n, uint32_t symbols, uint32_t tiles,
+                                                        uint32_t row_begin, uint32_t row_end, const uint32_t* __restrict__ bound, LoadArgs a,
+                                                        unsigned long long* load) {
+    __shared__ uint4 rows_sm[32][QUADS];
+    __shared__ uint32_t bound_sm[32], passed[32];
+    const uint32_t g = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const uint64_t row0 = row_begin + g * a.apart;
+    const uint32_t have = uint32_t(row_end - row0 < 32 ? row_end - row0 : 32);
+    const uint32_t tile = uint32_t((uint64_t(blockIdx.y) * a.groups + g) * tiles / (uint64_t(a.groups) * kLoadTiles));
+    auto hashed = [&](uint4 v) {
+        return make_uint4(symbols_of<U16>(v.x, symbols), symbols_of<U16>(v.y, symbols), symbols_of<U16>(v.z, symbols), symbols_of<U16>(v.w, symbols));
+    };
+    for (uint32_t i = tid; i < have * QUADS; i += kMmaRows) rows_sm[i / QUADS][i % QUADS] = hashed(__ldg(codes + row0 * QUADS + i));
+    if (tid < 32) passed[tid] = 0, bound_sm[tid] = tid < have ? bound[row0 + tid] : 0u;
+    const uint64_t col = uint64_t(tile) * kMmaRows + tid;
+    uint4 own[QUADS];
+#pragma unroll
+    for (int w = 0; w < QUADS; ++w) own[w] = hashed(__ldg(codes + (col < n ? col : 0) * QUADS + w));
+    __syncthreads();
+    for (uint32_t r = 0; r < have; ++r) {
+        const uint32_t m = __ballot_sync(kFull, col < n && code_distance<U16, QUADS>(rows_sm[r], own) <= bound_sm[r]);
+        if (lane == 0 && m) atomicAdd(&passed[r], __popc(m));
+    }
+    __syncthreads();
+    if (tid < 32) {
+        const uint32_t most = __reduce_max_sync(kFull, passed[tid]), all = __reduce_add_sync(kFull, passed[tid]);
+        if (tid == 0) atomicAdd(load, (unsigned long long)(most + (all + 31) / 32));
+    }
+}
+
 // ---- tcgen05 pieces ------------------------------------------------------------------------------------------------
 // D fp16, A and B e4m3, both K-major, M = 128, N = 256
 constexpr uint32_t kIdesc = (uint32_t(256 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
@@ -331,6 +387,7 @@ struct KnnMmaArgs {
     uint32_t* counts;             // [segments][256][2]
     uint32_t* status;
     uint32_t first_wait_polls, handover_polls;
+    SweepChoice choice;
 };
 
 // A row tile's codes and limits pass between the two warps that share its rows: each stores, in shared memory, the number
@@ -407,6 +464,7 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
 
 template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
+    if (a.choice.skip()) return;
     extern __shared__ __align__(1024) unsigned char mma_smem[];
     __shared__ __align__(8) uint64_t full_bar[2][2], empty_bar[2][2];    // [stage][part of K]
     __shared__ __align__(8) uint64_t tfull_bar[2][2], tempty_bar[2][2];  // [half of the rows][side]
@@ -707,6 +765,7 @@ constexpr int kFinishKeys = 512;
 
 __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
                                                                        uint16_t* __restrict__ dists, uint32_t out_row0) {
+    if (a.choice.skip()) return;
     __shared__ uint64_t keys_sm[kFinishWarps][kFinishKeys];
     __shared__ uint32_t hist_sm[kFinishWarps][96];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -801,7 +860,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArg
 
 template <typename CompT, int QUADS>
 int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, uint64_t n, uint32_t k, uint64_t row_begin,
-                 uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
+                 uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, double most_turns, SweepChoice* other, cudaStream_t st) {
     constexpr bool U16 = sizeof(CompT) == 2;
     const CompT* codes = static_cast<const CompT*>(d_codes);
     const HashShape shape = hash_shape(int(h->K));
@@ -815,7 +874,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const size_t segments = size_t(most + sms);
 
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t op_b = up(size_t(tiles) * operand_bytes), hist_b = up(size_t(kBoundOrders) * kKeys * 4);
+    const size_t op_b = up(size_t(tiles) * operand_bytes), hist_b = up(size_t(kBoundOrders) * kKeys * 4 + 8);
     const size_t order_b = up(size_t(kBoundOrders) * n * 4), place_b = order_b, bound_b = up(size_t(n) * 4);
     const size_t slots = segments * kMmaRows * 2;
     const size_t ids_b = up(slots * kMmaCap * 4), dists_b = up(slots * kMmaCap), counts_b = up(slots * 4);
@@ -852,21 +911,43 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.first_wait_polls = h->first_wait_polls;
     a.handover_polls = h->handover_polls;
 
-    LaunchTimer timer(h, kKernelKnn, st);
-    const uint64_t cells = tiles * shape.chunks * kMmaRows;
-    expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(codes, n, int(h->K), shape.symbols, shape.chunks, operand, tiles);
-    CPB_CUDA(cudaMemsetAsync(hist, 0, size_t(kBoundOrders) * kKeys * 4, st));
+    unsigned long long* load = reinterpret_cast<unsigned long long*>(hist + kBoundOrders * kKeys);
+    const uint64_t rows_wanted = row_end - row_begin;
+    LoadArgs sample;
+    sample.groups = uint32_t((rows_wanted + 31) / 32 < kLoadGroups ? (rows_wanted + 31) / 32 : kLoadGroups);
+    sample.apart = rows_wanted / sample.groups < 32 ? 32 : rows_wanted / sample.groups;
+    a.choice = SweepChoice();
+    if (other) {
+        a.choice.load = load;
+        a.choice.most = (unsigned long long)(most_turns * sample.groups * kLoadTiles);
+        *other = a.choice;
+        other->above = true;
+    }
+    CPB_CUDA(cudaMemsetAsync(hist, 0, size_t(kBoundOrders) * kKeys * 4 + 8, st));
     const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
     key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
     key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
     key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order, place);
-    auto bounds = [&](auto kernel) {
-        kernel<<<unsigned((n + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(a.codes, a.K, n, order, place, k, a.row_begin,
-                                                                                          a.row_end, bound);
+    auto bounds = [&](uint64_t count, uint64_t apart, const SweepChoice& choice) {
+        auto go = [&](auto kernel) {
+            kernel<<<unsigned((count + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(a.codes, a.K, n, order, place, k, a.row_begin,
+                                                                                                  a.row_end, bound, apart, choice);
+        };
+        if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) go(bound_kernel<U16, QUADS, (QUADS > 1)>);
+        else go(bound_kernel<U16, QUADS, false>);
+        h->launches++;
     };
-    if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) bounds(bound_kernel<U16, QUADS, (QUADS > 1)>);
-    else bounds(bound_kernel<U16, QUADS, false>);
-    h->launches += 5;
+    if (other) {
+        bounds(uint64_t(sample.groups) * 32, sample.apart, SweepChoice());
+        load_kernel<U16, QUADS><<<dim3(sample.groups, kLoadTiles), kMmaRows, 0, st>>>(a.codes, n, uint32_t(shape.symbols), uint32_t(tiles),
+                                                                                     a.row_begin, a.row_end, bound, sample, load);
+        h->launches++;
+    }
+    bounds(n, 0, a.choice);
+    const uint64_t cells = tiles * shape.chunks * kMmaRows;
+    expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(codes, n, int(h->K), shape.symbols, shape.chunks, operand, tiles,
+                                                                             a.choice);
+    h->launches += 4;
     CPB_CUDA(cudaGetLastError());
     CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS>));
     for (uint64_t t0 = first_tile; t0 < end_tile;) {
@@ -897,8 +978,9 @@ bool knn_mma_supported(const cphnsw_b200_index* h) {
 }
 
 int launch_knn_graph_mma(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padded, int words, uint64_t n, uint32_t k,
-                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
-#define CPB_MMA(T, Q) return launch_mma_t<T, Q>(h, d_codes, padded, n, k, row_begin, row_end, d_nbrs, d_dist, st)
+                         uint64_t row_begin, uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, double most_turns,
+                         SweepChoice* other, cudaStream_t st) {
+#define CPB_MMA(T, Q) return launch_mma_t<T, Q>(h, d_codes, padded, n, k, row_begin, row_end, d_nbrs, d_dist, most_turns, other, st)
     const bool u16 = h->comp_bytes == 2;
     switch (words) {
         case 4: if (u16) CPB_MMA(uint16_t, 1); CPB_MMA(uint8_t, 1);

@@ -50,7 +50,8 @@ __device__ __forceinline__ void csa(uint32_t& carry, uint32_t& sum, uint32_t a, 
 // codes (masked out later)
 template <typename CompT>
 __global__ void slice_codes_kernel(const CompT* __restrict__ codes, uint64_t n, int K, int NB,
-                                   uint32_t* __restrict__ out, uint64_t n_groups) {
+                                   uint32_t* __restrict__ out, uint64_t n_groups, SweepChoice choice) {
+    if (choice.skip()) return;
     const int lane = threadIdx.x & 31;
     const uint64_t g = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (g >= n_groups) return;
@@ -73,7 +74,8 @@ template <typename CompT, int NB, int NBLK, int SLOTS, int WARPS>  // NB bit pla
 __global__ void __launch_bounds__(WARPS * 32)
 knn_sliced_kernel(const uint32_t* __restrict__ sliced, const CompT* __restrict__ codes, uint64_t n, uint32_t k,
                   uint64_t row_begin, uint64_t row_end, uint32_t* __restrict__ nbrs, uint16_t* __restrict__ dists,
-                  uint32_t* __restrict__ status, uint32_t first_wait_polls) {
+                  uint32_t* __restrict__ status, uint32_t first_wait_polls, SweepChoice choice) {
+    if (choice.skip()) return;
     constexpr int K = NBLK * 8;
     constexpr int CHUNKS = K * NB / 4;             // 16-byte chunks per group
     constexpr uint32_t TILE_BYTES = CHUNKS * 32 * 16;
@@ -479,7 +481,6 @@ int launch_sliced_binary_t(cphnsw_b200_index* h, const uint32_t* sliced, const u
     auto kernel = knn_sliced_binary_kernel<SLOTS>;
     CPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const uint64_t blocks = (re - rb + kSlWarps * kSlQ - 1) / (kSlWarps * kSlQ);
-    LaunchTimer timer(h, kKernelKnn, st);
     kernel<<<unsigned(blocks), kSlWarps * 32, smem, st>>>(sliced, codes, n, k, rb, re, nbrs, dist, h->d_status.as<uint32_t>(), h->first_wait_polls, nblk,
                                                          nblk_p, int(h->residual_bits ? h->residual_shift : 0));
     h->launches++;
@@ -489,15 +490,14 @@ int launch_sliced_binary_t(cphnsw_b200_index* h, const uint32_t* sliced, const u
 
 template <typename CompT, int NB, int NBLK, int SLOTS, int WARPS>
 int launch_sliced_t(cphnsw_b200_index* h, const uint32_t* sliced, const CompT* codes, uint64_t n, uint32_t k,
-                    uint64_t rb, uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
+                    uint64_t rb, uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
     constexpr int CHUNKS = NBLK * 8 * NB / 4;
     const size_t smem = size_t(2) * CHUNKS * 32 * 16 + size_t(WARPS) * kSlQ * CHUNKS * 16;
     auto kernel = knn_sliced_kernel<CompT, NB, NBLK, SLOTS, WARPS>;
     CPB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const uint64_t rows = re - rb;
     const uint64_t blocks = (rows + WARPS * kSlQ - 1) / (WARPS * kSlQ);
-    LaunchTimer timer(h, kKernelKnn, st);
-    kernel<<<unsigned(blocks), WARPS * 32, smem, st>>>(sliced, codes, n, k, rb, re, nbrs, dist, h->d_status.as<uint32_t>(), h->first_wait_polls);
+    kernel<<<unsigned(blocks), WARPS * 32, smem, st>>>(sliced, codes, n, k, rb, re, nbrs, dist, h->d_status.as<uint32_t>(), h->first_wait_polls, choice);
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     return 0;
@@ -505,11 +505,11 @@ int launch_sliced_t(cphnsw_b200_index* h, const uint32_t* sliced, const CompT* c
 
 template <typename CompT, int NB, int NBLK, int WARPS>
 int launch_sliced_slots(cphnsw_b200_index* h, const uint32_t* sliced, const CompT* codes, uint64_t n, uint32_t k,
-                        uint64_t rb, uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
+                        uint64_t rb, uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
     const uint32_t need = k + 1;
-    if (need <= 64) return launch_sliced_t<CompT, NB, NBLK, 2, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, st);
-    if (need <= 96) return launch_sliced_t<CompT, NB, NBLK, 3, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, st);
-    return launch_sliced_t<CompT, NB, NBLK, 4, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, st);
+    if (need <= 64) return launch_sliced_t<CompT, NB, NBLK, 2, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, choice, st);
+    if (need <= 96) return launch_sliced_t<CompT, NB, NBLK, 3, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, choice, st);
+    return launch_sliced_t<CompT, NB, NBLK, 4, WARPS>(h, sliced, codes, n, k, rb, re, nbrs, dist, choice, st);
 }
 
 }  // namespace
@@ -536,17 +536,17 @@ bool knn_sliced_supported(const cphnsw_b200_index* h) {
 namespace {
 template <typename CompT, int NB, int WARPS>
 int launch_sliced_k(cphnsw_b200_index* h, const uint32_t* sl, const CompT* codes, uint64_t n, uint32_t k, uint64_t rb,
-                    uint64_t re, uint32_t* nbrs, uint16_t* dist, cudaStream_t st) {
-    if (h->K == 16) return launch_sliced_slots<CompT, NB, 2, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, st);
-    if (h->K == 32) return launch_sliced_slots<CompT, NB, 4, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, st);
-    if constexpr (NB <= 8) return launch_sliced_slots<CompT, NB, 8, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, st);
+                    uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
+    if (h->K == 16) return launch_sliced_slots<CompT, NB, 2, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, choice, st);
+    if (h->K == 32) return launch_sliced_slots<CompT, NB, 4, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, choice, st);
+    if constexpr (NB <= 8) return launch_sliced_slots<CompT, NB, 8, WARPS>(h, sl, codes, n, k, rb, re, nbrs, dist, choice, st);
     set_error("bit-sliced kNN: K = 64 is not available with 11-plane components");
     return CPHNSW_B200_E_UNSUPPORTED;
 }
 }  // namespace
 
 int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t n, uint32_t k, uint64_t row_begin,
-                            uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, cudaStream_t st) {
+                            uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, const SweepChoice& choice, cudaStream_t st) {
     const int K = int(h->K);
     const bool u16 = h->comp_bytes == 2;
     const int NB = h->binary_codes ? 1 : (u16 ? 11 : 8);
@@ -559,18 +559,18 @@ int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t 
         const unsigned grid = unsigned((threads + 255) / 256);
         if (u16)
             slice_codes_kernel<uint16_t><<<grid, 256, 0, st>>>(static_cast<const uint16_t*>(d_codes), n, K, NB,
-                                                               h->s_sliced.as<uint32_t>(), n_groups);
+                                                               h->s_sliced.as<uint32_t>(), n_groups, choice);
         else
             slice_codes_kernel<uint8_t><<<grid, 256, 0, st>>>(static_cast<const uint8_t*>(d_codes), n, K, NB,
-                                                              h->s_sliced.as<uint32_t>(), n_groups);
+                                                              h->s_sliced.as<uint32_t>(), n_groups, choice);
         h->launches++;
         CPB_CUDA(cudaGetLastError());
     }
     const uint32_t* sl = h->s_sliced.as<uint32_t>();
     if (u16) {
         const uint16_t* codes = static_cast<const uint16_t*>(d_codes);
-        if (NB == 1) return launch_sliced_k<uint16_t, 1, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
-        return launch_sliced_k<uint16_t, 11, 8>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+        if (NB == 1) return launch_sliced_k<uint16_t, 1, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st);
+        return launch_sliced_k<uint16_t, 11, 8>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st);
     }
     const uint8_t* codes = static_cast<const uint8_t*>(d_codes);
     if (NB == 1 && knn_sliced_binary_general(h)) {
@@ -579,8 +579,8 @@ int launch_knn_graph_sliced(cphnsw_b200_index* h, const void* d_codes, uint64_t 
         if (need <= 96) return launch_sliced_binary_t<3>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
         return launch_sliced_binary_t<4>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
     }
-    if (NB == 1) return launch_sliced_k<uint8_t, 1, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
-    return launch_sliced_k<uint8_t, 8, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, st);
+    if (NB == 1) return launch_sliced_k<uint8_t, 1, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st);
+    return launch_sliced_k<uint8_t, 8, kSlWarps>(h, sl, codes, n, k, row_begin, row_end, d_nbrs, d_dist, choice, st);
 }
 
 }  // namespace cpb

@@ -154,6 +154,51 @@ def test_lost_handover_is_reported(cp, oracle):
     check(idx, oracle, codes, 16)
 
 
+# the data decide between the filter and a kernel without one: byte-wise (few components in all; widths the bit planes do
+# not serve) or bit-sliced; clustered and unclustered rows, all of them and a block
+@pytest.mark.parametrize("n,K,cb,dim", [(8192, 32, 1, 128), (9000, 64, 1, 128), (17000, 64, 1, 128), (8200, 24, 1, 96), (8500, 32, 2, 960),
+                                        (8300, 16, 2, 300)])
+@pytest.mark.parametrize("clustered", [True, False])
+def test_picked_kernel(cp, oracle, n, K, cb, dim, clustered):
+    rng = np.random.default_rng(n + K)
+    if clustered:
+        base, _ = synthetic.gaussian_mixture(n, 1, dim, n // 500, 0.2, n + K)
+        codes = oracle.encode(base, K, cb, oracle.sign_tables(dim, K, 42))
+    else:
+        codes = rng.integers(0, 2 * (1 << (dim - 1).bit_length()), (n, K)).astype(np.uint8 if cb == 1 else np.uint16)
+    idx = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
+    check(idx, oracle, codes, 40, (n // 3, n // 3 + 200))
+    nbrs, dist = idx.knn_graph(codes, 64)
+    idx.set_param("knn_kernel", 1)
+    wn, wd = idx.knn_graph(codes, 64)
+    assert np.array_equal(nbrs, wn) and np.array_equal(dist, wd)
+
+
+def test_unclustered_data_do_not_go_through_the_filter(cp):
+    # 20,000 points of the unit sphere: the filter takes 3.1 ms, the byte-wise kernel 1.75
+    import torch
+    n = 20000
+    x = torch.randn((n, 128), device="cuda")
+    idx = cp.CPHNSWIndex(128, K=32)
+    codes = torch.empty((n, 32), dtype=torch.uint8, device="cuda")
+    nbrs = torch.empty((n, 64), dtype=torch.int32, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    idx.encode_dev(x.data_ptr(), n, codes.data_ptr(), stream=st)
+    time = {}
+    for kernel in (0, 3):
+        idx.set_param("knn_kernel", kernel)
+        ms = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            idx.knn_graph_dev(codes.data_ptr(), n, 64, 0, n, nbrs.data_ptr(), stream=st)
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+        time[kernel] = min(ms[1:])
+    assert time[0] < 0.85 * time[3]
+
+
 def test_unsupported_codes_are_refused(cp):
     idx = index(cp, 128, 100, 1)
     with pytest.raises(cp.CPHNSWError):
