@@ -753,7 +753,8 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
 // ---- few queries (asymmetric metric): a block per query ----------------------------------------------------------------------------------
 // With fewer queries than the chip has room for walks, what counts is the length of one walk: its steps in sequence,
 // some 5,000 cycles each for a warp alone.  Here eight warps share a query and a step takes the first sixteen unexpanded
-// members of W, two rows a warp; the prefix committed grows from 3.4 rows to about 8, and the rows' lookups and scores
+// members of W, two rows a warp, dealt out in turn (where a row brings so many candidates that a warp has room for one only,
+// as on data without clusters, the step still has the first eight); the prefix committed grows from 3.4 rows to about 8, and the rows' lookups and scores
 // run side by side.  Rows, candidates and the committed prefix are those of search_walk_kernel, so the results are too.
 //
 // A step meets at three barriers: the warps' candidates are listed with their ranks in W and the bound each puts on the
@@ -852,7 +853,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
         uint32_t row[kSquadRows], fresh[kSquadRows];
 #pragma unroll
         for (int b = 0; b < kSquadRows; ++b) {
-            const int t = warp * kSquadRows + b;
+            const int t = b * kSquadWarps + warp;
             const uint32_t node = t < have ? front[t] : kInvalidNode;
             row[b] = pre_row[b];
             // (a row that another warp asked for ahead comes from L1)
@@ -860,7 +861,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
         }
 #pragma unroll
         for (int b = 0; b < kSquadRows; ++b) {
-            const int t = kSquadFront + warp * kSquadRows + b;
+            const int t = kSquadFront + b * kSquadWarps + warp;
             pre_node[b] = t < have ? front[t] : kInvalidNode;
             pre_row[b] = (pre_node[b] != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(pre_node[b]) * a.M + lane) : kInvalidNode;
         }
@@ -876,7 +877,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
             first_of[b] = total;
             if (room && total + nf > 32) {
                 room = false;
-                bound = min(bound, uint32_t(warp * kSquadRows + b));
+                bound = min(bound, uint32_t(b * kSquadWarps + warp));
             }
             if (room) {
                 if ((fresh[b] >> lane) & 1u) cid[total + __popc(fresh[b] & below)] = row[b];
@@ -891,7 +892,7 @@ __global__ void __launch_bounds__(kSquadThreads) search_squad_kernel(WalkArgs w)
             id = own ? cid[lane] : kInvalidNode;
 #pragma unroll
             for (int b = 0; b < kSquadRows; ++b)
-                if (lane >= first_of[b]) my_row = warp * kSquadRows + b;
+                if (lane >= first_of[b]) my_row = b * kSquadWarps + warp;
             const float d = score(total);
             const uint32_t grp = __match_any_sync(kFull, id);
             own = own && (__ffs(grp) - 1) == lane;
