@@ -78,3 +78,17 @@ def test_wide_rows_with_the_walk_asked_for(cp):
                 idx.search_batch(q, 10, 100)
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("dim,K,cb", [(128, 32, 1), (128, 64, 1), (100, 17, 1), (960, 32, 2), (300, 40, 2)])
+@pytest.mark.parametrize("nq", [2, 700])
+def test_rows_of_new_neighbours_match_one_warp_kernel(cp, dim, K, cb, nq):
+    # no clusters: nearly every link of a row is a candidate, and a lane scores one (up to eight share their lookups by four)
+    rng = np.random.default_rng(dim + K)
+    base, q = rng.standard_normal((4000, dim)).astype(np.float32), rng.standard_normal((nq, dim)).astype(np.float32)
+    idx = cp.CPHNSWIndex(dim, M=32, K=K, component_bytes=cb)
+    idx.add_batch_parallel(base)
+    got = idx.search_batch(q, 20, 150)
+    idx.set_param("search_kernel", 1)
+    for a, b in zip(got, idx.search_batch(q, 20, 150)):
+        assert np.array_equal(a, b)
