@@ -1163,7 +1163,7 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     // Few queries under the asymmetric metric: a block each.  Measured on 64 / 250 / 500 queries: 367 / 432 / 568 us against
     // 473 / 513 / 536 with a warp each (100k x 128, beam 500), 250 / 500 / 1,000 of d = 960: 1.27 / 1.50 / 2.65 ms against
     // 2.10 / 2.15 / 2.51; under the symmetric metrics, whose scores cost little and tie often, a warp was always faster.
-    const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 > 32 * 1024 ? 4 : 2;
+    const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 >= 32 * 1024 ? 4 : 2;
     const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes;
     if (!sym && !w.exact_visited && a.nq <= squads_per_sm * uint32_t(h->sm_count) &&
         (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 32))) {
