@@ -37,7 +37,7 @@ constexpr int kBucketLog2 = 9;    // tag filter: 512 buckets of 4 tags = 4 KB pe
 constexpr uint32_t kTagBytes = (1u << kBucketLog2) * 8;
 constexpr uint64_t kTagNodes = uint64_t(0xffff) << kBucketLog2;  // ids below this have exact tags
 constexpr uint64_t kFiller = ~0ull;
-constexpr int kScanKeep = 32;     // most seeds the entry-scan kernel keeps per query
+constexpr int kScanKeep = 128;    // most seeds the entry-scan kernel keeps per query: 32 in each of one or four registers a lane
 constexpr int kScanWarps = 8;
 // Warps (queries) per SM.  A step is about 900 instructions with a chain of memory and shuffle latencies between them,
 // so what counts is how many walks an SM has in flight: the query table (16 KB) is therefore read in place, through L1
@@ -52,7 +52,8 @@ enum { kAsym = 0, kAsym128 = 1, kSymBytes = 2, kSymPacked = 3 };
 
 struct WalkArgs {
     SearchArgs s;
-    const uint64_t* seeds;  // [nq][kScanKeep] keys of the entry scan's best, ascending (nullptr: scanned by the walk itself)
+    const uint64_t* seeds;  // [nq][seed_slots] keys of the entry scan's best, ascending (nullptr: scanned by the walk itself)
+    uint32_t seed_slots;
     uint32_t* cand;         // [nq][rerank_k] ids handed to the rerank kernel (nullptr: no rerank)
     uint32_t smem_per_warp;
     uint32_t wcap_slots;    // slots of W's array (multiple of 32)
@@ -276,7 +277,7 @@ __device__ __forceinline__ float score_asym(const float* table, const unsigned c
 }
 
 // ---- entry scan ------------------------------------------------------------------------------------------------
-// The n_seed best entry nodes of every query (n_seed <= 32), QG queries per block, the entries dealt to its warps in
+// The n_seed best entry nodes of every query (n_seed <= 128), QG queries per block, the entries dealt to its warps in
 // batches of 32, one entry per lane.  Every query reads every entry node, so the scan is bound by table lookups:
 // n_entry * K per query, 4 bytes of shared-memory bandwidth each.
 //   * The tables of the block's queries are interleaved [block of 32 rotations][index][rotation][query]: one address
@@ -285,7 +286,7 @@ __device__ __forceinline__ float score_asym(const float* table, const unsigned c
 //     entries' codes are stored with the components in that order (gather_entry_codes).  The balanced tree pairs
 //     rotations 16, 8, 4, 2, 1 apart, and pairing j with j + 16 (mod 32) pairs the same rotations whatever l is, so
 //     the sums keep their bits.
-//   * Each warp keeps its 32 best per query, one per lane.  A candidate has to beat the warp's own n_seed-th and the
+//   * Each warp keeps its 32 best per query, one per lane, or its 128 best, four per lane.  A candidate has to beat the warp's own n_seed-th and the
 //     largest of all warps' (n_seed / warps)-th distances, below which n_seed entries are known to lie, so the warps
 //     admit about as little as one list would.
 struct ScanArgs {
@@ -295,7 +296,7 @@ struct ScanArgs {
     const uint32_t* entry;
     uint32_t n_entry, n_seed, nq;
     int K, P, row_bytes, packed_words, resid_kp, resid_mul;
-    uint64_t* seeds;  // [nq][kScanKeep]
+    uint64_t* seeds;  // [nq][32 * KEEP]
 };
 
 // compare-exchange across lanes s apart: the lane keeps the smaller key when `low`
@@ -303,13 +304,33 @@ __device__ __forceinline__ uint64_t keep_order(uint64_t x, int s, bool low) {
     const uint64_t z = __shfl_xor_sync(kFull, x, s);
     return (z < x) == low ? z : x;
 }
-// the 32 smallest of two ascending lists, ascending: the smaller of (own, other reversed) is a bitonic sequence
-__device__ __forceinline__ uint64_t join_sorted(uint64_t x, uint64_t other, int lane) {
-    const uint64_t y = __shfl_sync(kFull, other, 31 - lane);
-    x = y < x ? y : x;
+// the smallest of an ascending list (32 a register) and of 32 ascending keys, ascending: the smaller and the larger of
+// (own, other reversed) are bitonic sequences, the larger go on to the next register
+template <int KEEP>
+__device__ __forceinline__ void join_sorted(uint64_t (&x)[KEEP], uint64_t other, int lane) {
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) x = keep_order(x, s, (lane & s) == 0);
-    return x;
+    for (int s = 0; s < KEEP; ++s) {
+        const uint64_t y = __shfl_sync(kFull, other, 31 - lane);
+        uint64_t lo = y < x[s] ? y : x[s], hi = y < x[s] ? x[s] : y;
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) {
+            lo = keep_order(lo, d, (lane & d) == 0);
+            if (s + 1 < KEEP) hi = keep_order(hi, d, (lane & d) == 0);
+        }
+        x[s] = lo;
+        other = hi;
+    }
+}
+// the key of rank r
+template <int KEEP>
+__device__ __forceinline__ uint64_t ranked(const uint64_t (&x)[KEEP], int r) {
+    uint64_t k = 0;
+#pragma unroll
+    for (int s = 0; s < KEEP; ++s) {
+        const uint64_t v = __shfl_sync(kFull, x[s], r & 31);
+        if (s == r >> 5) k = v;
+    }
+    return k;
 }
 constexpr int kSortAdmit = 8;  // from here on sorting a batch (120 instructions) costs less than inserting one by one (14 each)
 
@@ -365,11 +386,11 @@ __device__ __forceinline__ Vals<QG> scan_tree(const unsigned char* table, const 
     return r;
 }
 
-template <bool U16, int METRIC, int QG>
-__global__ void __launch_bounds__(kScanWarps * 32, 3)
+template <bool U16, int METRIC, int QG, int KEEP>
+__global__ void __launch_bounds__(kScanWarps * 32, KEEP == 1 ? 3 : 2)
 entry_scan_kernel(ScanArgs a) {
     extern __shared__ __align__(16) unsigned char scan_smem[];
-    __shared__ uint64_t lists[kScanWarps][QG][kScanKeep];
+    __shared__ uint64_t lists[kScanWarps][QG][32 * KEEP];
     __shared__ uint32_t bound[QG][kScanWarps];  // ordered distance of each warp's (n_seed / warps)-th best
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t q0 = blockIdx.x * QG;
@@ -413,10 +434,14 @@ entry_scan_kernel(ScanArgs a) {
     }
     __syncthreads();
 
-    uint64_t best[QG];
+    uint64_t best[QG][KEEP];
     uint32_t thr[QG];  // ordered distance a candidate must not exceed
 #pragma unroll
-    for (int g = 0; g < QG; ++g) best[g] = kFiller, thr[g] = 0xffffffffu;
+    for (int g = 0; g < QG; ++g) {
+        thr[g] = 0xffffffffu;
+#pragma unroll
+        for (int s = 0; s < KEEP; ++s) best[g][s] = kFiller;
+    }
     const int pub = (int(a.n_seed) + kScanWarps - 1) / kScanWarps - 1;
     for (uint32_t e0 = warp * 32; e0 < a.n_entry; e0 += kScanWarps * 32) {
         const uint32_t e = e0 + lane;
@@ -467,33 +492,50 @@ entry_scan_kernel(ScanArgs a) {
                 for (int k2 = 2; k2 <= 32; k2 <<= 1)
 #pragma unroll
                     for (int s = k2 >> 1; s >= 1; s >>= 1) x = keep_order(x, s, ((lane & s) == 0) == ((lane & k2) == 0 || k2 == 32));
-                best[g] = join_sorted(best[g], x, lane);
+                join_sorted(best[g], x, lane);
             } else {
                 while (m) {
                     const int src = __ffs(m) - 1;
                     m &= m - 1;
                     const uint64_t k = __shfl_sync(kFull, key, src);
-                    const int r = __popc(__ballot_sync(kFull, best[g] < k));
-                    const uint64_t up = __shfl_up_sync(kFull, best[g], 1);
-                    best[g] = lane < r ? best[g] : (lane == r ? k : up);
+                    int r = 0;
+#pragma unroll
+                    for (int s = 0; s < KEEP; ++s) r += __popc(__ballot_sync(kFull, best[g][s] < k));
+#pragma unroll
+                    for (int s = KEEP - 1; s >= 0; --s) {
+                        uint64_t up = __shfl_up_sync(kFull, best[g][s], 1);
+                        if (s > 0) {
+                            const uint64_t carry = __shfl_sync(kFull, best[g][s - 1], 31);
+                            if (lane == 0) up = carry;
+                        }
+                        const int at = 32 * s + lane;
+                        best[g][s] = at < r ? best[g][s] : (at == r ? k : up);
+                    }
                 }
             }
-            const uint32_t hi = uint32_t(best[g] >> 32);
-            thr[g] = __shfl_sync(kFull, hi, int(a.n_seed) - 1);
-            if (lane == pub) *reinterpret_cast<volatile uint32_t*>(&bound[g][warp]) = hi;
+            thr[g] = uint32_t(ranked(best[g], int(a.n_seed) - 1) >> 32);
+            if (lane == pub) *reinterpret_cast<volatile uint32_t*>(&bound[g][warp]) = uint32_t(best[g][0] >> 32);
         }
     }
 #pragma unroll
-    for (int g = 0; g < QG; ++g) lists[warp][g][lane] = best[g];
+    for (int g = 0; g < QG; ++g)
+#pragma unroll
+        for (int s = 0; s < KEEP; ++s) lists[warp][g][32 * s + lane] = best[g][s];
     __syncthreads();
     // one warp per query joins the sorted lists
     for (int g = warp; g < QG; g += kScanWarps) {
         if (q0 + g >= a.nq) continue;
-        uint64_t x = lists[0][g][lane];
+        uint64_t x[KEEP];
+#pragma unroll
+        for (int s = 0; s < KEEP; ++s) x[s] = lists[0][g][32 * s + lane];
         for (int o = 1; o < kScanWarps; ++o) {
-            x = join_sorted(x, lists[o][g][lane], lane);
+            for (int s = 0; s < KEEP; ++s) {
+                if (KEEP > 1 && lists[o][g][32 * s] >= ranked(x, 32 * KEEP - 1)) break;  // (and so are the ones behind it)
+                join_sorted(x, lists[o][g][32 * s + lane], lane);
+            }
         }
-        a.seeds[size_t(q0 + g) * kScanKeep + lane] = x;
+#pragma unroll
+        for (int s = 0; s < KEEP; ++s) a.seeds[size_t(q0 + g) * (32 * KEEP) + 32 * s + lane] = x[s];
     }
 }
 
@@ -568,9 +610,12 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
         const bool scan = a.n_seed < a.n_entry;
         const uint32_t cap0 = scan ? a.n_seed : a.beam;
         if (w.seeds) {
-            const uint64_t k = w.seeds[size_t(q) * kScanKeep + lane];
-            count = __popc(__ballot_sync(kFull, k != kFiller && uint32_t(lane) < cap0));
-            if (uint32_t(lane) < count) W[lane] = k;
+            for (uint32_t s = lane; s < w.seed_slots; s += 32) {
+                const uint64_t k = w.seeds[size_t(q) * w.seed_slots + s];
+                const bool have = k != kFiller && s < cap0;
+                if (have) W[s] = k;
+                count += __popc(__ballot_sync(kFull, have));
+            }
             nevals += a.n_entry;
             __syncwarp();
         }
@@ -798,16 +843,24 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
         return score_asym<U16, METRIC == kAsym128>(table, static_cast<const unsigned char*>(a.codes), a.K, a.P, cid, total, lane);
     };
 
-    // entry nodes: the scan's best, or (up to 32 of them) all
-    if (warp == 0) {
+    // entry nodes: the scan's best, in order; or all of them (up to 128), 32 a warp
+    if (w.seeds) {
+        if (warp == 0) {
+            uint32_t have = 0;
+            for (uint32_t s = lane; s < w.seed_slots; s += 32) {
+                const uint64_t k = w.seeds[size_t(q) * w.seed_slots + s];
+                const bool seed = k != kFiller && s < a.n_seed;
+                if (seed) tag_store(tags, key_id(k));
+                if (seed && s < a.beam) W[s] = k;
+                have += __popc(__ballot_sync(kFull, seed));
+            }
+            if (lane == 0) seeded = min(have, a.beam);
+        }
+    } else {
         uint64_t k = kFiller;
-        uint32_t most = a.beam;
-        if (w.seeds) {
-            if (lane < int(a.n_seed)) k = w.seeds[size_t(q) * kScanKeep + lane];
-            if (k != kFiller) tag_store(tags, key_id(k));
-        } else {
-            const uint32_t id = uint32_t(lane) < a.n_entry ? __ldg(a.entry + lane) : kInvalidNode;
-            const int total = int(min(a.n_entry, 32u));
+        if (warp * 32 < int(a.n_entry)) {
+            const int total = int(min(a.n_entry - warp * 32, 32u));
+            const uint32_t id = lane < total ? __ldg(a.entry + tid) : kInvalidNode;
             cid[lane] = id;
             __syncwarp();
             const float d = score(total);
@@ -816,11 +869,12 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
                 tag_store(tags, id);
             }
         }
+        list_key[tid] = k;
+        __syncthreads();
         uint32_t rank = 0;
-        for (int i = 0; i < 32; ++i) rank += __shfl_sync(kFull, k, i) < k;
-        const uint32_t have = __popc(__ballot_sync(kFull, k != kFiller));
-        if (k != kFiller && rank < most) W[rank] = k;
-        if (lane == 0) seeded = min(have, most);
+        for (uint32_t i = 0; i < a.n_entry; ++i) rank += list_key[i] < k;
+        if (k != kFiller && rank < a.beam) W[rank] = k;
+        if (tid == 0) seeded = min(a.n_entry, a.beam);
     }
     __syncthreads();
     uint32_t count = seeded, cur = 0;
@@ -1060,8 +1114,13 @@ search_rerank_kernel(const float* __restrict__ vectors, const float* __restrict_
 
 template <bool U16, int METRIC, int QG>
 int launch_scan_t(cphnsw_b200_index* h, const ScanArgs& a, size_t smem, cudaStream_t st) {
-    CPB_CUDA(allow_max_dynamic_smem(entry_scan_kernel<U16, METRIC, QG>));
-    entry_scan_kernel<U16, METRIC, QG><<<(a.nq + QG - 1) / QG, kScanWarps * 32, smem, st>>>(a);
+    auto go = [&](auto kernel) -> int {
+        CPB_CUDA(allow_max_dynamic_smem(kernel));
+        kernel<<<(a.nq + QG - 1) / QG, kScanWarps * 32, smem, st>>>(a);
+        return 0;
+    };
+    if (a.n_seed <= 32) CPB_TRY(go(entry_scan_kernel<U16, METRIC, QG, 1>));
+    else CPB_TRY(go(entry_scan_kernel<U16, METRIC, QG, 4>));
     h->launches++;
     CPB_CUDA(cudaGetLastError());
     return 0;
@@ -1139,6 +1198,7 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     const uint64_t want = (uint64_t(a.nq) + warps - 1) / warps;
     const int blocks = int(want < uint64_t(h->sm_count) ? want : uint64_t(h->sm_count));
     w.seeds = nullptr;
+    w.seed_slots = 0;
     const size_t scan_table = size_t((a.K + 31) / 32) * 32 * a.P * 4;
     if (a.n_seed < a.n_entry && a.n_seed <= uint32_t(kScanKeep) && (sym || (a.P >= 4 && scan_table <= 200 * 1024))) {
         ScanArgs sc;
@@ -1155,7 +1215,8 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         sc.packed_words = a.packed_words;
         sc.resid_kp = a.resid_kp;
         sc.resid_mul = a.resid_mul;
-        CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * kScanKeep * 8));
+        w.seed_slots = a.n_seed <= 32 ? 32 : kScanKeep;
+        CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * w.seed_slots * 8));
         sc.seeds = cx.d_seeds.as<uint64_t>();
         w.seeds = sc.seeds;
         CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
@@ -1166,7 +1227,7 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 >= 32 * 1024 ? 4 : 2;
     const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes;
     if (!sym && !w.exact_visited && a.nq <= squads_per_sm * uint32_t(h->sm_count) &&
-        (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 32))) {
+        (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 128))) {
         if (metric == kAsym128) CPB_TRY((launch_squad_t<false, kAsym128>(w, squad_smem, st)));
         else if (u16) CPB_TRY((launch_squad_t<true, kAsym>(w, squad_smem, st)));
         else CPB_TRY((launch_squad_t<false, kAsym>(w, squad_smem, st)));

@@ -80,6 +80,32 @@ def test_wide_rows_with_the_walk_asked_for(cp):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("dim,K,cb,M,k,ef,rerank,entries,seeds", [
+    (128, 32, 1, 32, 10, 100, 500, 700, 100),  # a list of 128 seeds per query
+    (128, 64, 1, 32, 10, 50, 0, 900, 64),      # a beam narrower than the seeds
+    (960, 16, 2, 24, 10, 300, 300, 333, 34),
+    (96, 16, 1, 16, 10, 20, 0, 100, 100),      # no scan: all entries are offered, more of them than the beam takes
+    (300, 40, 2, 32, 10, 64, 64, 33, 33),
+])
+@pytest.mark.parametrize("nq", [1, 150, 600])
+def test_many_seeds_match_one_warp_kernel(cp, dim, K, cb, M, k, ef, rerank, entries, seeds, nq):
+    base, q = synthetic.gaussian_mixture(3001, nq, dim, 12, 0.3, dim + nq)
+    idx = cp.CPHNSWIndex(dim, M=M, ef_construction=max(200, M), K=K, component_bytes=cb)
+    idx.set_param("entry_scan", entries)
+    idx.set_param("k_entry", seeds)
+    idx.add_batch_parallel(base)
+    runs = [lambda: idx.search_and_rerank_batch(q, k, ef, rerank) if rerank else idx.search_batch(q, k, ef),
+            lambda: idx.search_batch(q, k, ef, want_stats=True)]
+    if nq < 600:
+        runs.append(lambda: idx.search_multiprobe_batch(q, k, ef, 3))
+    for run in runs:
+        idx.set_param("search_kernel", 0)
+        got = run()
+        idx.set_param("search_kernel", 1)
+        for a, b in zip(got, run()):
+            assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("dim,K,cb", [(128, 32, 1), (128, 64, 1), (100, 17, 1), (960, 32, 2), (300, 40, 2)])
 @pytest.mark.parametrize("nq", [2, 700])
 def test_rows_of_new_neighbours_match_one_warp_kernel(cp, dim, K, cb, nq):
