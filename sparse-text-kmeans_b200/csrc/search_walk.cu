@@ -1189,7 +1189,13 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
     w.smem_per_warp = uint32_t((size_t(w.wcap_slots) * 8 + (w.exact_visited ? 0 : kTagBytes) + 256 + words * 256 + 128 + 32 +
                                 (sym ? row : 0) + 15) / 16 * 16);
     int warps = int((226 * 1024) / w.smem_per_warp);
-    const int most = w.exact_visited && warps > 16 ? 16 : kWalkWarps;  // visited arrays: 16 per SM
+    // Visited arrays: 16 per SM.  Query tables above 32 KB: with 24 walks an SM those in flight (227 MB at 64 KB) leave L2 where
+    // the walks read all of them, as on data without clusters (100k x 300, K = 32, 10,000 queries, beam 500: 58.7 ms with 24,
+    // 41.2 with 16; 960-d |N|: 59.2 and 39.5); clustered data, which read little of them, lose 3 to 12 % (4.40 and 4.94, 6.89 and
+    // 7.10 ms).  At 32 KB clustered data
+    // would lose 20 % (4.14 and 5.02 ms, K = 64), and the others keep up as they are (33.9 ms, 40.4 with two warps per query).
+    const bool wide_table = !sym && size_t(a.K) * a.P * 4 > 32 * 1024;
+    const int most = (w.exact_visited || wide_table) && warps > 16 ? 16 : kWalkWarps;
     if (warps > most) warps = most;
     const int per_sm = int((a.nq + h->sm_count - 1) / h->sm_count);  // a small batch spreads over all SMs
     if (warps > per_sm) warps = per_sm;
