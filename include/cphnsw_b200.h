@@ -60,6 +60,11 @@ const char* cphnsw_b200_last_error(void);
 /* Number of usable sm_100 devices (0 when none / no driver).  Never fails. */
 int cphnsw_b200_device_count(void);
 
+/* Device memory that handles have freed is kept for later buffers of any handle of the process: up to 1 GiB per device
+ * while the device has handles, up to 384 MiB after the last one is destroyed.  It goes back to the driver by itself when
+ * an allocation of this library fails; this call gives all of it back, for an allocator beside this one.  Any thread. */
+int cphnsw_b200_release_memory(int device);
+
 /* ---- lifetime -------------------------------------------------------------------------------
  * Replaces the constructors CPHNSWIndex(dim, M, ef_construction) / CPHNSWIndex(const CPHNSWParams&)
  * (use sites evaluation/eval_sift.cpp:228, evaluation/test_gpu_build.cpp:155-162) and

@@ -43,7 +43,7 @@ EXPORTS = [
     "cphnsw_b200_search_codes_batch", "cphnsw_b200_get_code", "cphnsw_b200_sharded_create", "cphnsw_b200_sharded_load",
     "cphnsw_b200_sharded_destroy", "cphnsw_b200_sharded_gpus", "cphnsw_b200_sharded_size", "cphnsw_b200_sharded_replica",
     "cphnsw_b200_sharded_set_param", "cphnsw_b200_sharded_add_batch_parallel", "cphnsw_b200_sharded_add_batch",
-    "cphnsw_b200_sharded_search", "cphnsw_b200_sharded_stage_times",
+    "cphnsw_b200_sharded_search", "cphnsw_b200_sharded_stage_times", "cphnsw_b200_release_memory",
 ]
 
 
@@ -74,6 +74,11 @@ def load_library():
 
 def device_count():
     return load_library().cphnsw_b200_device_count()
+
+
+def release_memory(device=0):
+    """Gives the device memory the library keeps between its handles' buffers back to the driver."""
+    _check(load_library().cphnsw_b200_release_memory(device))
 
 
 def _check(rc):

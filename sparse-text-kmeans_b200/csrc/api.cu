@@ -587,6 +587,17 @@ int cphnsw_b200_device_count(void) {
     return ok;
 }
 
+int cphnsw_b200_release_memory(int device) {
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+        cudaGetLastError();
+        set_error("no CUDA device available: this library has no CPU path");
+        return CPHNSW_B200_E_CUDA;
+    }
+    if (device < 0 || device >= ndev) { set_error("device %d out of range (%d devices)", device, ndev); return CPHNSW_B200_E_INVALID; }
+    return device_release_kept(device);
+}
+
 static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint32_t M, uint32_t ef_construction,
                        uint64_t seed, int fht_convention, int device, bool binary, cphnsw_b200_index** out) {
     if (!out) {

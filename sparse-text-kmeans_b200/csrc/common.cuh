@@ -57,6 +57,7 @@ inline cudaError_t allow_max_dynamic_smem(F* kernel) {
 // room (optional): set to false, and no error, when the device has no memory for the block.
 int device_alloc(void** p, size_t* bytes, int* device, bool* room = nullptr);
 void device_free(void* p, size_t bytes, int device);
+int device_release_kept(int device);  // all kept blocks of a device back to the driver
 void device_handle_created(int device);
 void device_handle_destroyed(int device);
 struct QuietDevice {

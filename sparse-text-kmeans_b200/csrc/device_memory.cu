@@ -117,6 +117,20 @@ void device_handle_destroyed(int device) {
     if (--pool.handles <= 0) pool.trim(kKeepIdle);
 }
 
+int device_release_kept(int device) {
+    if (device >= kMaxDevices) return 0;
+    int before = 0;
+    CPB_CUDA(cudaGetDevice(&before));
+    CPB_CUDA(cudaSetDevice(device));
+    {
+        Pool& pool = pools()[device];
+        std::lock_guard<std::mutex> lock(pool.mu);
+        pool.trim(0);  // (no kernel uses a kept block: they came in idle)
+    }
+    CPB_CUDA(cudaSetDevice(before));
+    return 0;
+}
+
 QuietDevice::QuietDevice() {
     // (a device that reports an error is not quiet: its blocks then go back to the driver)
     if (quiet_depth > 0 || cudaDeviceSynchronize() == cudaSuccess) ++quiet_depth;
