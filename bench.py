@@ -30,8 +30,9 @@ sys.path.insert(0, os.path.join(ROOT, "sparse-text-kmeans_b200"))
 
 METRIC = "batch-search QPS @ recall@10>=0.9 (search_and_rerank)"
 # DRAM bytes (read + written) per query of the search kernels, from the ncu capture summarised in
-# profiles/search_walk_kernel_c2_quarter.md (C2 at 1/4 size, 2,500 queries);
-# the traffic per query does not depend on the number of queries, so a launch of nq queries moves nq times this
+# profiles/search_walk_kernel_c2_quarter.md, for an index of the captured size only (C2 at 1/4 size, 2,500 queries): it does
+# not depend on the number of queries, but grows with the index, of which less fits L2
+NCU_SEARCH_BASE_POINTS = 250_000
 NCU_SEARCH_DRAM_BYTES_PER_QUERY = 139e3
 # the same for the one-warp search_kernel (profiles/search_kernel_c2_quarter.md: 1.215 GB + 0.080 GB per launch)
 NCU_SEARCH_DRAM_BYTES_PER_QUERY_ONE_WARP = 518e3
@@ -62,6 +63,15 @@ def parse_args():
     ap.add_argument("--search-table-smem", type=int, default=1, choices=[0, 1],
                     help="0 = the search kernels read the query table in place (global memory) even when it fits shared memory")
     return ap.parse_args()
+
+
+def measured_fp8_peak():
+    """Operations per second of the dense fp8 products: twice the measured bf16 rate (nominal where none was measured)."""
+    path = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    if os.path.exists(path):
+        with open(path) as f:
+            return 2e12 * float(json.load(f)["bf16_tflops"]), "twice the measured bf16 rate"
+    return 4.5e15, "the nominal dense fp8 rate"
 
 
 def measured_peaks():
@@ -582,14 +592,14 @@ def run_b200(args):
     # the library takes the walk of several nodes a step (with its entry scan and rerank kernels) when M <= 32
     walk = args.search_kernel != 1 and M <= 32
     dram_per_query = NCU_SEARCH_DRAM_BYTES_PER_QUERY if walk else NCU_SEARCH_DRAM_BYTES_PER_QUERY_ONE_WARP
-    traffic = dram_per_query * q_per_launch if w["name"] == "C2" else None
+    traffic = dram_per_query * q_per_launch if w["name"] == "C2" and n == NCU_SEARCH_BASE_POINTS else None
     roofline = {"kernel": "entry_scan_kernel + search_walk_kernel + search_rerank_kernel" if walk else "search_kernel", "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": "of " + peak_kind,
                 "traffic": traffic,
                 # the same fraction on the DRAM bytes ncu measured instead of the algorithmic bytes: what the kernel
                 # really asks of HBM (it is bound by dependent latencies, not by bandwidth)
                 "frac_measured_dram": (traffic / (search_ms_per_launch * 1e-3) / 1e9 / peak) if traffic else None,
-                "traffic_note": "bytes per launch, scaled by queries from the ncu capture of C2 at 1/4 size",
+                "traffic_note": "bytes per launch from the ncu capture of C2 at 1/4 size; null at other index sizes, where it was not measured",
                 "ms_per_launch": search_ms_per_launch, "queries_per_launch": q_per_launch, "algorithmic_bytes_per_query": bytes_per_query,
                 "expansions_per_query": exp_mean, "distance_evals_per_query": evals_mean,
                 "share_of_step": search_ms / (ms_total if ms_total else 1.0),
@@ -620,11 +630,12 @@ def run_b200(args):
         # tensor-core filter: a component is 7 values of +-1 at K <= 32 and 3 above, rows padded to a multiple of 32
         # values; every pair costs two operations a value
         values = (K * (7 if K <= 32 else 3) + 31) // 32 * 32
-        fp8 = 4.5e15 * world
+        fp8, fp8_kind = measured_fp8_peak()
+        fp8 *= world
         roofline_build["knn_graph"] = {"bound": "fp8 tensor pipe and its epilogue", "achieved": build["knn_pairs_per_s"] * 2 * values, "peak": fp8,
                                        "unit": "op/s", "frac": build["knn_pairs_per_s"] * 2 * values / fp8,
-                                       "note": "%d values per pair; peak is the nominal dense fp8 rate; ncu sm__pipe_tensor_cycles_active "
-                                               "62 %% of the sweep on C2 at 1/4 size (profiles/knn_mma_kernel_c2_quarter.md)" % values}
+                                       "note": "%d values per pair, every unordered pair twice; peak is %s; ncu sm__pipe_tensor_cycles_active "
+                                               "62 %% of the sweep on C2 at 1/4 size (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp8_kind)}
     sel_bytes = n * (knn_k * 4 + knn_k * code_row + M * 4.0)
     roofline_build["select_neighbors"] = {"bound": "hbm gather", "achieved": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9, "peak": peak * world,
                                           "unit": "GB/s", "frac": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9 / (peak * world),
