@@ -287,7 +287,7 @@ knn_graph_kernel(const uint32_t* __restrict__ codes, uint64_t n, uint32_t k, uin
 // two candidates per lane.  A candidate is kept unless a kept one is at least as close to it as the node is, so whenever
 // one is kept all later candidates are tested against it at once, and the next one still standing is the next kept: two
 // distances per kept member.  (Testing every candidate against all kept ones took three per candidate: 11.0 ms per 1M
-// nodes with 64 candidates of 32-byte codes, issue bound, against 0.36 ms.)
+// nodes with 64 candidates of 32-byte codes, issue bound, against 1.83 ms.)
 constexpr int kSelWarps = 4;
 constexpr int kSelMaxK = 64;
 

@@ -14,7 +14,7 @@
 //     the sign tables of layers 1 and 2; the last one only decides the sign bit of the code
 //     (and the sign of the rotated output), applied here through `flip_mask` = W-1.
 //
-// Two kernels:
+// Five kernels:
 //   encode_thread_kernel padded dims 32, 64 and 128 (d in 17..128): one thread owns one vector, the whole
 //                        transform lives in registers (no shuffles, no barriers in the
 //                        inner loop); the bound is the fp32 add pipe.
@@ -22,6 +22,7 @@
 //                        low stages in registers, high stages by shuffles.
 //   encode_group_kernel  padded dims 256 and 512, many vectors: 2 or 4 lanes own one vector, 128 elements each; the stages
 //                        across lanes become register stages after an exchange.
+//   encode_p1024_kernel  padded dim 1024: one warp per vector, transposes through shared memory between two layouts.
 //   encode_generic_kernel any other power-of-two padded dim: one warp owns one vector in shared memory.
 #include "common.cuh"
 

@@ -13,7 +13,7 @@
 // Visited nodes.  W itself decides what is admitted: a node seen before is either a member of W (found there by its
 // key when it is ranked) or was turned away or pushed out by members that are closer, and would be again, since the
 // worst member of a full W only gets closer.  Remembering visited nodes only saves the scoring, so a filter that may
-// forget is enough: 16-bit tags in shared memory, 8 to a bucket (one 128-bit read), the tag and the bucket together
+// forget is enough: 16-bit tags in shared memory, 4 to a bucket (one 64-bit read), the tag and the bucket together
 // being a bijection of the id, so that a hit is never wrong.  When the caller asks for statistics (the number of
 // distance evaluations counts every node once) or the index is too large for exact tags, the exact set is kept
 // instead: one byte per node and slot in global memory holding the number of the slot's last query that visited it.
@@ -282,10 +282,10 @@ __device__ __forceinline__ float score_asym(const float* table, const unsigned c
 // n_entry * K per query, 4 bytes of shared-memory bandwidth each.
 //   * The tables of the block's queries are interleaved [block of 32 rotations][index][rotation][query]: one address
 //     and one 16-byte read serve four queries.
-//   * At step j lane l looks up rotation (j + l) & 31 of its entry, so the lanes of a read sit in different banks; the
+//   * At step j lane l looks up rotation j XOR l of its entry, so the lanes of a read sit in different banks; the
 //     entries' codes are stored with the components in that order (gather_entry_codes).  The balanced tree pairs
-//     rotations 16, 8, 4, 2, 1 apart, and pairing j with j + 16 (mod 32) pairs the same rotations whatever l is, so
-//     the sums keep their bits.
+//     rotations 16, 8, 4, 2, 1 apart, which differ in one bit of their number, and the XOR leaves it so: the sums keep
+//     their bits.
 //   * Each warp keeps its 32 best per query, one per lane, or its 128 best, four per lane.  A candidate has to beat the warp's own n_seed-th and the
 //     largest of all warps' (n_seed / warps)-th distances, below which n_seed entries are known to lie, so the warps
 //     admit about as little as one list would.
@@ -1227,9 +1227,10 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         w.seeds = sc.seeds;
         CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
     }
-    // Few queries under the asymmetric metric: a block each.  Measured on 64 / 250 / 500 queries: 367 / 432 / 568 us against
-    // 473 / 513 / 536 with a warp each (100k x 128, beam 500), 250 / 500 / 1,000 of d = 960: 1.27 / 1.50 / 2.65 ms against
-    // 2.10 / 2.15 / 2.51; under the symmetric metrics, whose scores cost little and tie often, a warp was always faster.
+    // Few queries under the asymmetric metric: a block each.  Measured on 64 / 250 / 500 queries, beam 500, against a warp each:
+    // 100k x 128, K = 32, 352 / 390 / 544 us against 479 / 507 / 530, K = 64 (a table of 32 KB) 455 / 519 / 665 against
+    // 845 / 914 / 956, d = 960 581 / 722 / 908 against 851 / 963 / 995; under the symmetric metrics, whose scores cost little
+    // and tie often, a warp was always faster.
     const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 >= 32 * 1024 ? 4 : 2;
     const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes;
     if (!sym && !w.exact_visited && a.nq <= squads_per_sm * uint32_t(h->sm_count) &&
