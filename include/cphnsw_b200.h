@@ -127,11 +127,12 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *   "first_wait_polls" (0..2^22, default 2^22: polls granted to the FIRST bounded wait of a kNN-graph launch; a test
  *                 sets 0 to make that wait give up, which the call reports as CPHNSW_B200_E_DEVICE_WAIT; the tensor-core
  *                 sweep of an exact search has the same first wait, and one that is lost there costs time only) and "handover_polls"
- *                 (the same range and default, for the waits inside a tensor-core kNN launch for a row tile's end),
+ *                 (the same range and default, for the waits inside a tensor-core kNN launch for a stage to be handed back),
  *   "workspace_limit_mb" (default 0 = no limit: the most MiB of device memory a tensor-core filter's workspace may take.
- *                 A kNN graph's is about 300 bytes a node plus 0.2 to 0.4 GB, an exact search's 2 bytes a base coordinate
- *                 plus up to 0.5 GB; both stay with the handle.  Above the limit, and when the device has no memory for
- *                 it, the kernels without a filter answer, with the same results),
+ *                 A kNN graph's is about 300 bytes a node, 1.6 KB a row wanted and up to 64 MB - rows go in blocks where
+ *                 that is too much -, an exact search's 2 bytes a base coordinate plus up to 0.5 GB; both stay with the
+ *                 handle.  Above the limit, and when the device has no memory for it, the kernels without a filter answer,
+ *                 with the same results),
  *   "entry_scan" (evenly spaced nodes scored for every query before the walk; default = k_entry),
  *   "k_entry" (1..100, default 4: how many of the scored nodes, the best, seed the walk). */
 int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double value);

@@ -179,7 +179,7 @@ struct cphnsw_b200_index {
     // polls the kNN kernels and the exact sweep grant their FIRST tile wait ("first_wait_polls"; every other wait keeps the full
     // limit).  0 makes that wait give up at once: the way a test reaches the lost-wait path.
     uint32_t first_wait_polls = 1u << 22;
-    uint32_t handover_polls = 1u << 22;  // the same for the waits between the warps that share the rows of a kNN filter block
+    uint32_t handover_polls = 1u << 22;  // the same for a kNN filter block's waits for the stages that its products hand back
     int exact_edges = 0;              // bulk build picks candidates and links on the fp32 vectors (legacy hybrid construction)
     int rank_prune = 0;               // bulk build prunes by detourable-route count instead of select_neighbors
     float rank_pruning_alpha = 1.1f;  // CPHNSWParams::rank_pruning_alpha (include/cphnsw/core/types.hpp:399-400)

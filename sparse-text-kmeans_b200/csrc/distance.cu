@@ -612,15 +612,15 @@ static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_
 constexpr uint64_t kMmaMinNodes = 4096;
 // Where the data let too many pairs through its filter the bit-sliced or the byte-wise kernel is taken, which cost the same
 // whatever the data: most_turns is the load (see knn_mma.cu) up to which the filter is the faster, from measured picoseconds
-// a pair.  Filter: 1.2 and 0.01 to 0.02 a turn, by the bytes of a code.  Bit-sliced, K = 32: 1.1 at 400k rows, 1.9 at 100k,
+// a pair.  Filter: 0.25 and 0.006 to 0.05 a turn, by the bytes of a code.  Bit-sliced, K = 32: 1.1 at 400k rows, 1.9 at 100k,
 // 7.5 at 20k (a wave of blocks sweeps all nodes however few rows it has), in proportion to the planes; byte-wise 3 at
-// 32-byte codes, 9 at 64.  Unit sphere, 100k x 128, K = 32: 17.4 ms against 58 through the filter; mixtures of 1,000 points
-// a cluster: sigma 0.3 3.2 against 19.3, sigma 0.7 19.3 against 28.6.
+// 32-byte codes, 9 at 64.  Unit sphere, 100k x 128, K = 32: 17.4 ms against 77 through the filter; mixtures of 1,000 points
+// a cluster: sigma 0.3 2.1 against 19.3, sigma 0.6 17.3 against 19.3, sigma 0.7 24.9 against 19.3.
 static double most_turns(const cphnsw_b200_index* h, uint64_t rows, bool sliced) {
     const double bytes = double(h->K) * h->comp_bytes, planes = h->K * (h->comp_bytes == 2 ? 11.0 : 8.0);
     const double other = sliced ? (0.8 + 113e3 / double(rows)) * (0.5 + planes / 512)
                                 : (bytes <= 16 ? 1.5 : bytes <= 32 ? 2.8 : 9.0) + 50e3 / double(rows);
-    const double turns = (other - 1.2) / (0.004 + 0.0002 * bytes);
+    const double turns = (other - 0.25) / (h->comp_bytes == 2 ? 0.05 : bytes <= 16 ? 0.006 : 0.018);
     return turns < 12 ? 12 : (turns > 300 ? 300 : turns);
 }
 // Below this many nodes the filter is the faster on any data (4,096 nodes of the unit sphere: 324 to 567 us against 607 to

@@ -9,22 +9,39 @@
 // accumulators (+-1 and integers up to 224 are exact in both), so all n^2 pairs cost 2 * 224 tensor operations and one
 // instruction of the epilogue each; only pairs that reach the row's threshold t have their exact distance computed.
 //
-// Row thresholds.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie
+// Row limits.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie
 // beside rows that share both, and the k-th smallest exact distance in the windows of 128 around a row in eight such
-// orders, every row counted once, bounds its final t from above.  On clustered data t is mostly right or one too high, and
-// some 450 pairs per row pass, 140 of them truly within t.  The pairs found are kept in a buffer; when it runs full its k
-// best are kept and t falls below the worst of them for the pairs still to come, which have higher ids.  On data without
-// clusters the bound says nothing, t is lowered by this alone and most pairs pass: a sample of the data shows it, and the
-// sweep is then left to another kernel ("what the filter is worth" below).
+// orders, every row counted once, bounds its final k-th distance from above.  On clustered data it is mostly right or one
+// too high, and some 450 rows pass the filter for a row, 140 of them truly within the bound.
 //
-// Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the candidates
-// in tiles of 256, two stages of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
+// Each pair once.  The distance is symmetric, so a tile of pairs serves the rows of both sides: row tile r meets the column
+// tiles r, r + 1, .. r + half of them, cyclically, which gives every row tile the same work and every pair one product
+// (where only some rows are wanted, theirs are the first tiles and the other tiles are met by all of them).  A pair passes
+// at the larger of the row's limit and the largest of 32 columns', its exact distance is then held against both.  The sweep
+// lists 32 rows by 32 columns where one passes; a kernel of its own compares them and keeps the rows found for a row in a
+// buffer in global memory.
+//
+// Order.  Nodes are placed in an order in which neighbours lie together: the smallest node among the likely neighbours of a
+// node names its group, followed from node to node, and within 1,024 places rows are sorted by their limit.  The pairs that
+// pass are then met in a few tiles, and in all others the epilogue takes one maximum.  500k x 500k, K = 32, 64 neighbours:
+// 38.8 ms with every pair twice and in the order given, 17.6 so (15.0 of them the sweep, 2,200 cycles a tile whose products
+// take 1,792).  The near tiles go first: their k-th distances are mostly final, and limits and gates of the rest are tight.
+//
+// Full buffers.  Where the bounds say little the sweep goes by phases, every 16th (64th ..) column tile first, each of them
+// as much as all before it; between them the k-th distances found are the new limits.  A sample of the data shows whether
+// that is needed, and whether the filter is worth anything at all ("what the filter is worth" below).  A row whose buffer
+// runs over all the same starts anew at the k-th distance of what it held, and where that does not do either it is compared
+// with every node by a kernel without a buffer.
+//
+// Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the column tiles
+// of 256, halves of them in a ring of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
 // halves of tensor memory; while one half is computed the other is read.  A row has two epilogue threads, which take the
-// tiles in turn (a buffer and a limit each): one reads a tile while the other still deals with the pairs of the one before.
-// The operand is laid out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a
-// tile is one contiguous copy and no tensor map is needed.  Blocks that take whole rows of tiles sweep them in step, so
-// that a tile comes from L2; only the rows left over by the last full wave are split between blocks along the candidates.
+// tiles in turn.  The operand is laid out by
+// the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a tile is one contiguous copy
+// and no tensor map is needed.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "mma_common.cuh"
 
@@ -37,15 +54,27 @@ using knn::mbar_wait_bounded;
 using knn::smem_u32;
 using namespace mma;
 
-constexpr int kMmaCap = 384;              // entries of a buffer: at most 128 before a tile and 256 from it
+constexpr uint32_t kMmaCap = 384;         // entries of a row's buffer
 constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
-constexpr uint32_t kMmaKeep = 128;
+constexpr uint32_t kMmaKeep = 128;        // entries that are left of one that is cut
+constexpr uint32_t kMmaFull = 256;        // entries from which on it is cut between phases
+constexpr int kBatch = 4;                 // rows compared with 32 columns at a time
+constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in the list of hits
+constexpr uint64_t kLaunchSteps = 1u << 22;
+constexpr uint32_t kCheckBlocks = 4;      // blocks of the check an SM
+constexpr uint32_t kNearColumns = 8, kNearFrom = 64;  // column tiles that are swept first, of so many at least
 constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, every second tile
-constexpr int kMmaThreads = (kEpiWarps + 3) * 32;  // and one each for the operands' copies, the products, the codes' copies
-constexpr int kMaxCodeStages = 4;
-constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 9 KB of static
+constexpr int kMmaThreads = (kEpiWarps + 2) * 32;  // and one each for the operands' copies and the products
+constexpr int kMaxStages = 8;             // of half a tile each
+constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 5 KB of static
+constexpr int kSortRows = 1024;           // places sorted by limit together
+constexpr uint32_t kFirstColumns = 8;      // column tiles of the first phase, at most
+constexpr uint32_t kOnePhase = 64;         // up to so many (32,000 nodes) there is only one, and no second bound: what these would save
+                                           // costs less than their launches (16,000 x 128: 525 us with them, 392 without)
 constexpr int kBoundOrders = 8;           // orders of likely neighbours
 constexpr int kBoundWindow = 128;         // rows looked at per order
+constexpr int kNameOrders = 4, kNameWindow = 32;  // of them for the names of the groups
+constexpr uint64_t kOrderNodes = 4096;    // fewer are met in the order given (5,000 x 128: 225 us so, 210 in groups)
 constexpr uint32_t kKeys = 65536;
 
 // symbols and values of a code shape; 0 symbols: not served
@@ -65,18 +94,20 @@ __device__ __forceinline__ uint32_t symbol_of(uint32_t comp, uint32_t symbols) {
 }
 
 // ---- operand: [tile of 256 rows][chunk][row][16 values] ------------------------------------------------------------
+// codes: padded rows of `stride` components in their places
 template <typename CompT>
-__global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n, int K, int symbols, int chunks,
-                                    uint4* __restrict__ out, uint64_t tiles, SweepChoice choice) {
+__global__ void expand_codes_kernel(const CompT* __restrict__ codes, int stride, const uint2* __restrict__ place, int K, int symbols,
+                                    int chunks, uint4* __restrict__ out, uint64_t tiles, SweepChoice choice) {
     if (choice.skip()) return;
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= tiles * chunks * kMmaRows) return;
     const int r = int(t % kMmaRows), c = int(t / kMmaRows % chunks);
     const uint64_t row = t / (uint64_t(kMmaRows) * chunks) * kMmaRows + r;
     uint32_t w[4] = {0u, 0u, 0u, 0u};
-    if (row < n) {
+    if (place[row].x != kInvalidNode) {
+        const CompT* code = codes + row * stride;
         int comp = c * 16 / (symbols - 1), j = c * 16 % (symbols - 1) + 1;
-        uint32_t h = comp < K ? symbol_of(codes[row * K + comp], uint32_t(symbols)) : 0u;
+        uint32_t h = comp < K ? symbol_of(code[comp], uint32_t(symbols)) : 0u;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t e4m3 = (__popc(h & uint32_t(j)) & 1) ? 0xB8u : 0x38u;  // -1 : +1
@@ -84,7 +115,7 @@ __global__ void expand_codes_kernel(const CompT* __restrict__ codes, uint64_t n,
             if (++j == symbols) {
                 j = 1;
                 ++comp;
-                if (comp < K) h = symbol_of(codes[row * K + comp], uint32_t(symbols));
+                if (comp < K) h = symbol_of(code[comp], uint32_t(symbols));
             }
         }
     }
@@ -231,68 +262,128 @@ __device__ __forceinline__ void load_row(uint4 (&v)[QUADS], const uint4* p) {
 // (half the work of counting them, 24 registers less) and a 32-byte row is one load where it is aligned.  100k rows, K = 32:
 // 1.15 ms before, 0.85 now with one-byte components, 1.66 and 1.32 with two-byte ones.
 constexpr int kBoundWarps = 4;
-constexpr uint32_t kSeenSlots = 1024;
-template <bool U16, int QUADS, bool SECTORS>
+constexpr uint32_t kCloseRows = 12;
+template <bool U16, int QUADS, bool SECTORS, int ORDERS, int WINDOW>
 __global__ void __launch_bounds__(kBoundWarps * 32)
 bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t* __restrict__ order, const uint32_t* __restrict__ place,
-             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound, uint64_t apart /* of LoadArgs: its rows only; 0: all rows */,
+             uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound, uint32_t* __restrict__ group, uint32_t* __restrict__ mate,
+             uint64_t apart /* of LoadArgs: its rows only; 0: all rows */, const uint32_t* __restrict__ listed /* their number, rows: only these */,
              SweepChoice choice) {
     if (choice.skip()) return;
-    constexpr int S = kBoundWindow / 32, N = kBoundOrders * S;
+    constexpr int S = WINDOW / 32, N = ORDERS * S;
+    constexpr uint32_t kSeenSlots = N * 32 > 512 ? 1024 : 512;
     __shared__ uint32_t seen_sm[kBoundWarps][kSeenSlots];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t at = uint64_t(blockIdx.x) * kBoundWarps + warp;
-    if (at >= n) return;
-    const uint64_t wanted = apart ? row_begin + at / 32 * apart + at % 32 : order[at];
-    if (wanted < row_begin || wanted >= row_end) return;
-    const uint32_t row = uint32_t(wanted);
-    uint32_t* seen = seen_sm[warp];
-    for (uint32_t i = lane; i < kSeenSlots / 4; i += 32) reinterpret_cast<uint4*>(seen)[i] = make_uint4(kFull, kFull, kFull, kFull);
-    const uint32_t where = lane < kBoundOrders ? place[uint64_t(row) * kBoundOrders + lane] : 0u;
-    uint32_t id[N], dist[N / 4] = {};  // distances a byte each
+    const uint64_t warps = uint64_t(gridDim.x) * kBoundWarps, many = listed ? listed[0] : apart ? warps : n;
+    for (uint64_t at = uint64_t(blockIdx.x) * kBoundWarps + warp; at < many; at += warps) {
+        const uint64_t wanted = listed ? listed[1 + at] : apart ? row_begin + at / 32 * apart + at % 32 : order[at];
+        if (wanted < row_begin || wanted >= row_end) continue;
+        const uint32_t row = uint32_t(wanted);
+        uint32_t* seen = seen_sm[warp];
+        for (uint32_t i = lane; i < kSeenSlots / 4; i += 32) reinterpret_cast<uint4*>(seen)[i] = make_uint4(kFull, kFull, kFull, kFull);
+        const uint32_t where = lane < ORDERS ? place[uint64_t(row) * kBoundOrders + lane] : 0u;
+        uint32_t id[N], dist[N / 4] = {};  // distances a byte each
+        uint4 own[QUADS];
+#pragma unroll
+        for (int w = 0; w < QUADS; ++w) own[w] = __ldg(codes + size_t(row) * QUADS + w);
+#pragma unroll
+        for (int o = 0; o < ORDERS; ++o) {
+            const uint64_t pos = __shfl_sync(kFull, where, o);
+            uint64_t first = pos < WINDOW / 2 ? 0 : pos - WINDOW / 2;
+            if (first + WINDOW > n) first = n > WINDOW ? n - WINDOW : 0;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const uint64_t p = first + s * 32 + lane;
+                id[o * S + s] = p < n ? __ldg(order + size_t(o) * n + p) : row;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            uint4 theirs[QUADS];
+            load_row<SECTORS>(theirs, codes + size_t(id[i]) * QUADS);
+            dist[i / 4] |= (id[i] != row ? code_distance<U16, QUADS>(own, theirs) : 127u) << (8 * (i % 4));
+        }
+        // enough of the closest, repeats included, to hold k different rows in most cases; half the table at most
+        const uint32_t reach = kth_packed(dist, kSeenSlots / 2 < 4 * k ? kSeenSlots / 2 : 4 * k, K);
+        const bool all = count_upto(dist, reach) <= kSeenSlots * 3 / 4;  // else the farthest of them would crowd the table
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if ((dist[i / 4] >> (8 * (i % 4)) & 127u) < reach + (all ? 1u : 0u)) {
+                uint32_t slot = (id[i] * 0x9E3779B1u) >> (kSeenSlots == 1024 ? 22 : 23);
+                while (true) {
+                    const uint32_t was = atomicCAS(seen + slot, kFull, id[i]);
+                    if (was == kFull) break;
+                    if (was == id[i]) {
+                        dist[i / 4] |= 127u << (8 * (i % 4));  // a repeat
+                        break;
+                    }
+                    slot = (slot + 1) & (kSeenSlots - 1);
+                }
+            } else {
+                dist[i / 4] |= 127u << (8 * (i % 4));
+            }
+        }
+        const uint32_t T = kth_packed(dist, k, K);  // (K when fewer than k were found)
+        if (listed) {
+            if (lane == 0 && T < bound[row]) bound[row] = T;
+            __syncwarp();
+            continue;
+        }
+        // of the closest few, as far as they are likely in its cluster, the smallest wanted node names the row's group, the
+        // largest is a mate
+        const uint32_t close = min(kth_packed(dist, kCloseRows, K), uint32_t(K) * 5 / 8);
+        uint32_t least = row, most = row;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if ((dist[i / 4] >> (8 * (i % 4)) & 127u) <= close && id[i] >= row_begin && id[i] < row_end) least = min(least, id[i]), most = max(most, id[i]);
+        least = __reduce_min_sync(kFull, least);
+        most = __reduce_max_sync(kFull, most);
+        if (lane == 0) bound[row] = T, group[row] = least, mate[row] = most;
+        __syncwarp();
+    }
+}
+
+// Bounds from the rows that lie beside a row once its group lies together: 32 rows a block, the 512 places around them from
+// shared memory, a quarter of them for each warp, the k-th smallest of a row's distances.  (The windows of the orders alone,
+// eight of 128 for every row, took 8.3 us per 1,000 rows, gathers through the L1; the windows of four of 32 for the names of
+// the groups take 1.2, the order 0.7 and this 1.2.)
+constexpr int kBesideRows = 32, kBesideWarps = 4, kBesidePlaces = 512;
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kBesideWarps * 32) beside_kernel(const uint4* __restrict__ codes, const uint32_t* __restrict__ grouped, uint32_t rows,
+                                                                   int K, uint32_t k, uint32_t* __restrict__ bound,
+                                                                   uint32_t* __restrict__ far /* their number, rows */, SweepChoice choice) {
+    if (choice.skip()) return;
+    extern __shared__ __align__(16) unsigned char beside_smem[];
+    uint4* code = reinterpret_cast<uint4*>(beside_smem);                                   // [kBesidePlaces][QUADS]
+    uint16_t* count = reinterpret_cast<uint16_t*>(code + kBesidePlaces * QUADS);           // [distance][warp][row]
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row0 = blockIdx.x * kBesideRows, own_place = row0 + lane;
+    const uint32_t ahead = (kBesidePlaces - kBesideRows) / 2;
+    uint32_t from = row0 < ahead ? 0 : row0 - ahead;
+    if (from + kBesidePlaces > rows) from = rows > uint32_t(kBesidePlaces) ? rows - kBesidePlaces : 0;
+    const uint32_t have = min(rows - from, uint32_t(kBesidePlaces));
+    for (uint32_t i = tid; i < have * QUADS; i += kBesideWarps * 32) code[i] = __ldg(codes + size_t(grouped[from + i / QUADS]) * QUADS + i % QUADS);
+    for (int d = 0; d <= K; ++d) count[d * kBesideWarps * 32 + tid] = 0;
+    __syncthreads();
     uint4 own[QUADS];
 #pragma unroll
-    for (int w = 0; w < QUADS; ++w) own[w] = __ldg(codes + size_t(row) * QUADS + w);
-#pragma unroll
-    for (int o = 0; o < kBoundOrders; ++o) {
-        const uint64_t pos = __shfl_sync(kFull, where, o);
-        uint64_t first = pos < kBoundWindow / 2 ? 0 : pos - kBoundWindow / 2;
-        if (first + kBoundWindow > n) first = n > kBoundWindow ? n - kBoundWindow : 0;
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const uint64_t p = first + s * 32 + lane;
-            id[o * S + s] = p < n ? __ldg(order + size_t(o) * n + p) : row;
-        }
+    for (int w = 0; w < QUADS; ++w) own[w] = code[min(own_place, rows - 1) * QUADS - from * QUADS + w];
+    const uint32_t j1 = min(have, (warp + 1) * (kBesidePlaces / kBesideWarps));
+#pragma unroll 4
+    for (uint32_t j = warp * (kBesidePlaces / kBesideWarps); j < j1; ++j) {
+        const uint32_t d = code_distance<U16, QUADS>(own, code + j * QUADS);
+        count[d * kBesideWarps * 32 + tid] += from + j != own_place;
     }
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        uint4 theirs[QUADS];
-        load_row<SECTORS>(theirs, codes + size_t(id[i]) * QUADS);
-        dist[i / 4] |= (id[i] != row ? code_distance<U16, QUADS>(own, theirs) : 127u) << (8 * (i % 4));
+    __syncthreads();
+    if (warp != 0 || own_place >= rows) return;
+    const uint32_t node = grouped[own_place], before = bound[node];
+    uint32_t T = 0, upto = 0;
+    for (; T < uint32_t(K); ++T) {
+        for (int w = 0; w < kBesideWarps; ++w) upto += count[(T * kBesideWarps + w) * 32 + lane];
+        if (upto >= k) break;
     }
-    // enough of the closest, repeats included, to hold k different rows in most cases; half the table at most
-    const uint32_t reach = kth_packed(dist, kSeenSlots / 2 < 4 * k ? kSeenSlots / 2 : 4 * k, K);
-    const bool all = count_upto(dist, reach) <= kSeenSlots * 3 / 4;  // else the farthest of them would crowd the table
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        if ((dist[i / 4] >> (8 * (i % 4)) & 127u) < reach + (all ? 1u : 0u)) {
-            uint32_t slot = (id[i] * 0x9E3779B1u) >> 22;
-            while (true) {
-                const uint32_t was = atomicCAS(seen + slot, kFull, id[i]);
-                if (was == kFull) break;
-                if (was == id[i]) {
-                    dist[i / 4] |= 127u << (8 * (i % 4));  // a repeat
-                    break;
-                }
-                slot = (slot + 1) & (kSeenSlots - 1);
-            }
-        } else {
-            dist[i / 4] |= 127u << (8 * (i % 4));
-        }
-    }
-    const uint32_t T = kth_packed(dist, k, K);  // (K when fewer than k were found)
-    if (lane == 0) bound[row] = T;
+    if (T < before) bound[node] = T;
+    if (min(T, before) > uint32_t(K) * 5 / 8) far[1 + atomicAdd(far, 1u)] = node;
 }
 
 // ---- what the filter is worth ----------------------------------------------------------------------------------------
@@ -307,6 +398,20 @@ struct LoadArgs {
     uint32_t groups;
 };
 constexpr uint32_t kLoadGroups = 16, kLoadTiles = 16;
+// What the sample counts: turns, and the pairs that are truly within the rows' bounds.  Up to kCalmEntries of them a row
+// the buffers hold what the whole sweep finds, and up to kCalmTurns there is little to gain from limits that fall on the
+// way: it then goes in one phase (400k x 128, mixture sigma 0.5, 29 turns: 185 ms in one, 143 in seven).
+struct LoadCounts {
+    unsigned long long turns;
+    uint32_t within;
+};
+constexpr double kCalmEntries = 230, kCalmTurns = 20;
+struct Calm {
+    const LoadCounts* counts = nullptr;  // (nullptr: not known)
+    uint32_t most = 0;
+    unsigned long long most_turns = 0;
+    __device__ __forceinline__ bool yes() const { return counts && counts->within <= most && counts->turns <= most_turns; }
+};
 
 // the symbols of a word's components, in their places
 template <bool U16>
@@ -318,9 +423,9 @@ __device__ __forceinline__ uint32_t symbols_of(uint32_t w, uint32_t symbols) {
 template <bool U16, int QUADS>
 __global__ void __launch_bounds__(kMmaRows) load_kernel(const uint4* __restrict__ codes, uint64_t n, uint32_t symbols, uint32_t tiles,
                                                         uint32_t row_begin, uint32_t row_end, const uint32_t* __restrict__ bound, LoadArgs a,
-                                                        unsigned long long* load) {
-    __shared__ uint4 rows_sm[32][QUADS];
-    __shared__ uint32_t bound_sm[32], passed[32];
+                                                        LoadCounts* load) {
+    __shared__ uint4 rows_sm[32][QUADS], plain_sm[32][QUADS];
+    __shared__ uint32_t bound_sm[32], passed[32], within;
     const uint32_t g = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const uint64_t row0 = row_begin + g * a.apart;
     const uint32_t have = uint32_t(row_end - row0 < 32 ? row_end - row0 : 32);
@@ -328,21 +433,33 @@ __global__ void __launch_bounds__(kMmaRows) load_kernel(const uint4* __restrict_
     auto hashed = [&](uint4 v) {
         return make_uint4(symbols_of<U16>(v.x, symbols), symbols_of<U16>(v.y, symbols), symbols_of<U16>(v.z, symbols), symbols_of<U16>(v.w, symbols));
     };
-    for (uint32_t i = tid; i < have * QUADS; i += kMmaRows) rows_sm[i / QUADS][i % QUADS] = hashed(__ldg(codes + row0 * QUADS + i));
-    if (tid < 32) passed[tid] = 0, bound_sm[tid] = tid < have ? bound[row0 + tid] : 0u;
-    const uint64_t col = uint64_t(tile) * kMmaRows + tid;
-    uint4 own[QUADS];
-#pragma unroll
-    for (int w = 0; w < QUADS; ++w) own[w] = hashed(__ldg(codes + (col < n ? col : 0) * QUADS + w));
-    __syncthreads();
-    for (uint32_t r = 0; r < have; ++r) {
-        const uint32_t m = __ballot_sync(kFull, col < n && code_distance<U16, QUADS>(rows_sm[r], own) <= bound_sm[r]);
-        if (lane == 0 && m) atomicAdd(&passed[r], __popc(m));
+    for (uint32_t i = tid; i < have * QUADS; i += kMmaRows) {
+        const uint4 v = __ldg(codes + row0 * QUADS + i);
+        plain_sm[i / QUADS][i % QUADS] = v;
+        rows_sm[i / QUADS][i % QUADS] = hashed(v);
     }
+    if (tid < 32) passed[tid] = 0, bound_sm[tid] = tid < have ? bound[row0 + tid] : 0u;
+    if (tid == 0) within = 0;
+    const uint64_t col = uint64_t(tile) * kMmaRows + tid;
+    uint4 plain[QUADS], own[QUADS];
+#pragma unroll
+    for (int w = 0; w < QUADS; ++w) plain[w] = __ldg(codes + (col < n ? col : 0) * QUADS + w), own[w] = hashed(plain[w]);
+    __syncthreads();
+    uint32_t near = 0;
+    for (uint32_t r = 0; r < have; ++r) {
+        const bool pass = col < n && code_distance<U16, QUADS>(rows_sm[r], own) <= bound_sm[r];
+        const uint32_t m = __ballot_sync(kFull, pass);
+        if (lane == 0 && m) atomicAdd(&passed[r], __popc(m));
+        if (pass) near += code_distance<U16, QUADS>(plain_sm[r], plain) <= bound_sm[r];
+    }
+    if (near) atomicAdd(&within, near);
     __syncthreads();
     if (tid < 32) {
         const uint32_t most = __reduce_max_sync(kFull, passed[tid]), all = __reduce_add_sync(kFull, passed[tid]);
-        if (tid == 0) atomicAdd(load, (unsigned long long)(most + (all + 31) / 32));
+        if (tid == 0) {
+            atomicAdd(&load->turns, (unsigned long long)(most + (all + 31) / 32));
+            atomicAdd(&load->within, within);
+        }
     }
 }
 
@@ -357,72 +474,154 @@ __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a, uint64_t b, 
         "l"(a), "l"(b), "r"(kIdesc), "r"(uint32_t(accumulate))
         : "memory");
 }
-// 16 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
-__device__ __forceinline__ void tmem_load16(uint32_t (&r)[8], uint32_t addr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+// 32 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
+__device__ __forceinline__ void tmem_load32(uint32_t (&r)[16], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(addr)
                  : "memory");
 }
 // (the registers are operands so that no use of them moves in front of the wait)
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[8]) {
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
+                   "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
                  :
                  : "memory");
 }
+
+// ---- which tiles meet ------------------------------------------------------------------------------------------------
+// The first row_tiles tiles hold the rows wanted.  Row tile r meets the tiles r + j, j <= row_tiles / 2, of them, cyclically
+// (for an even number the farthest pair is met from both sides, each for its own rows), and all tiles behind them.
+struct Meet {
+    uint32_t tiles, row_tiles;
+    __host__ __device__ uint32_t columns() const { return row_tiles / 2 + 1 + (tiles - row_tiles); }
+    __device__ uint32_t column(uint32_t rt, uint32_t j) const {
+        if (j > row_tiles / 2) return row_tiles + (j - row_tiles / 2 - 1);
+        const uint32_t ct = rt + j;
+        return ct >= row_tiles ? ct - row_tiles : ct;
+    }
+    // the column's rows take part with limits of their own
+    __device__ bool both(uint32_t rt, uint32_t ct) const {
+        const uint32_t j = ct >= rt ? ct - rt : ct + row_tiles - rt;
+        return ct < row_tiles && j != 0 && 2 * j != row_tiles;
+    }
+};
+// The columns of one launch: from `base` on every stride-th, or the odd ones of those; `count` of them from the from-th on.
+struct Phase {
+    uint32_t base, stride;
+    bool odd;
+    uint32_t from, count;
+    __host__ __device__ uint32_t columns(uint32_t of) const {  // in all
+        const uint32_t c = (of - base + stride - 1) / stride;
+        return odd ? c / 2 : c;
+    }
+    __device__ uint32_t column(uint32_t i) const { return base + stride * (odd ? 2 * (from + i) + 1 : from + i); }
+};
+// What a block does: whole row tiles, a grid's width apart, so that the blocks meet the same column tiles at about the same
+// time and a tile comes from L2; then its part of the steps of the row tiles left over.
+struct Walk {
+    uint32_t len, whole, rt, at;  // steps of a row tile; whole row tiles to come; row tile and step
+    uint32_t steps, apart;        // of the block; rows between its whole row tiles
+    uint32_t rest_rt, rest_at;    // where its part of the rest begins
+    uint32_t hop;                 // the rest goes round a row tile's columns by this many: neighbouring columns are far apart
+    __device__ Walk(uint32_t row_tiles, uint32_t len_) {
+        const uint32_t blocks = gridDim.x, b = blockIdx.x;
+        len = len_;
+        apart = blocks;
+        whole = row_tiles / blocks;
+        const uint64_t rest = uint64_t(row_tiles % blocks) * len, r0 = b * rest / blocks, r1 = (b + 1) * rest / blocks;
+        rest_rt = whole * blocks + uint32_t(r0 / len), rest_at = uint32_t(r0 % len);
+        steps = whole * len + uint32_t(r1 - r0);
+        rt = whole ? b : rest_rt;
+        at = whole ? 0 : rest_at;
+        // in time, some 0.618 of the way round (hop is the inverse of that number without a common divisor with len)
+        hop = 1;
+        if (whole * blocks < row_tiles && len > 2) {
+            for (int apart_in_time = int(0.618f * float(len));; ++apart_in_time) {
+                int r0 = int(len), r1 = apart_in_time, t0 = 0, t1 = 1;
+                while (r1) {
+                    const int q = r0 / r1, r = r0 - q * r1, t = t0 - q * t1;
+                    r0 = r1, r1 = r, t0 = t1, t1 = t;
+                }
+                if (r0 == 1) {
+                    hop = uint32_t(t0 < 0 ? t0 + int(len) : t0);
+                    break;
+                }
+            }
+        }
+    }
+    __device__ bool last() const { return at + 1 == len; }
+    __device__ uint32_t step() const { return whole ? at : uint32_t(uint64_t(at) * hop % len); }
+    __device__ void next() {
+        if (++at < len) return;
+        at = 0;
+        if (whole && --whole) rt += apart;
+        else if (whole == 0 && rt >= rest_rt) ++rt;
+        else rt = rest_rt, at = rest_at;
+    }
+};
+
 struct KnnMmaArgs {
-    const uint4* operand;  // [tiles][chunks][256]
-    const uint4* codes;    // padded rows
-    int code_stages;       // candidate tiles whose codes are held in shared memory
-    int K, symbols, chunks;
-    uint64_t n;
+    const uint4* operand;   // [tiles][chunks][256], places in order
+    const uint4* codes;     // [tiles * 256] padded rows, places in order
+    uint2* place;           // [tiles * 256] the node at a place (kInvalidNode: none), largest distance of use to it (-1: none)
+    int16_t* gate;          // [row_tiles][8] what a product reaches at the largest limit of 32 places (gate_of)
+    int K, symbols, chunks, stages;
     uint32_t k;
-    Split split;
-    uint32_t tile0;               // first row tile of the launch
-    uint32_t row_begin, row_end;  // rows wanted
-    const uint32_t* bound;        // [n] bounds on the final thresholds
-    uint32_t* ids;                // [segments][256 rows][2 sides][kMmaCap]
-    uint8_t* dists;               // the same
-    uint32_t* counts;             // [segments][256][2]
+    Meet meet;
+    Phase phase;
+    enum { kAlways, kAllIfCalm, kNotIfCalm } when;  // calm data: the second takes all its columns at once, the third has nothing to do
+    bool wide;              // entries of two words
+    uint32_t* entries;      // [row_tiles * 256][kMmaCap]
+    uint32_t* counts;       // [row_tiles * 256] entries; above kMmaCap: some were lost
+    uint4* hits;            // 32 rows and 32 columns among which a product reaches its gate: first row, first column, rows, both
+    uint32_t* hit_count;
+    uint32_t hit_room;
     uint32_t* status;
     uint32_t first_wait_polls, handover_polls;
     SweepChoice choice;
+    Calm calm;
 };
 
-// A row tile's codes and limits pass between the two warps that share its rows: each stores, in shared memory, the number
-// of segments it is done with, and waits for the other's before it replaces them.  (A counter and not a barrier's phase:
-// a warp without a tile in a segment runs ahead of the other by several.)
-__device__ __forceinline__ void hand_over(uint32_t* done, uint32_t segments) {
-    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(done)), "r"(segments) : "memory");
-}
-__device__ __forceinline__ bool handed_over(const uint32_t* done, uint32_t segments, uint32_t limit, volatile int* aborted) {
-    if (segments == 0) return true;
-    for (uint32_t i = 0; i < limit; ++i) {
-        uint32_t have;
-        asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(have) : "r"(smem_u32(done)) : "memory");
-        if (have >= segments) return true;
-        if ((i & 15) == 15) {
-            if (*aborted) return false;
-            __nanosleep(200);
-        }
-    }
-    return false;
+// The dot product a pair at distance <= t reaches at least, as the bits of its half: above zero halves compare as their bits
+// do, and those below zero are below; where zero or less is enough every product will do.  t < 0: none does.
+__device__ __forceinline__ int gate_of(int symbols, int K, int t) {
+    const int dot = symbols * (K - t) - K;
+    return t < 0 ? 0x7fff : (dot > 0 ? int(__half_as_ushort(__float2half_rn(float(dot)))) : -0x8000);
 }
 
-// the dot product a pair at distance <= t reaches at least (t < 0: none does), twice
-__device__ __forceinline__ __half2 dot_of_distance(int symbols, int K, int t) {
-    return t < 0 ? __half2half2(__ushort_as_half(0x7c00)) : __float2half2_rn(float(symbols * (K - t) - K));
+// The entries of a row's buffer: (distance, node), packed in a word up to kPackedNodes nodes, in two above.
+constexpr uint32_t kPackedNodes = 1u << 25;
+constexpr uint32_t kNoDistance = 127;  // no entry
+struct Entry {
+    uint32_t d, node;
+};
+__device__ __forceinline__ Entry load_entry(const uint32_t* buf, bool wide, uint32_t e) {
+    if (wide) {
+        const uint2 v = reinterpret_cast<const uint2*>(buf)[e];
+        return Entry{v.x, v.y};
+    }
+    const uint32_t v = buf[e];
+    return Entry{v >> 25, v & (kPackedNodes - 1u)};
+}
+__device__ __forceinline__ void store_entry(uint32_t* buf, bool wide, uint32_t e, uint32_t d, uint32_t node) {
+    if (wide) reinterpret_cast<uint2*>(buf)[e] = make_uint2(d, node);
+    else buf[e] = d << 25 | node;
+}
+__device__ __forceinline__ uint32_t* buffer_of(uint32_t* entries, bool wide, uint32_t place) {
+    return entries + size_t(place) * (kMmaCap * (wide ? 2 : 1));
 }
 
 // The row's buffer shrinks to its k best (or all that are no worse than the k-th, up to kMmaKeep).  By the whole warp;
 // returns the k-th distance and the new count.
-__device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, uint32_t& count, uint32_t k, int K, int lane) {
+__device__ __forceinline__ uint32_t compact_row(uint32_t* buf, bool wide, uint32_t& count, uint32_t k, int K, int lane) {
     uint32_t dist[kMmaSlots];
 #pragma unroll
     for (int s = 0; s < kMmaSlots; ++s) {
         const uint32_t e = uint32_t(s * 32 + lane);
-        dist[s] = e < count ? dists[e] : kFull;
+        dist[s] = e < count ? load_entry(buf, wide, e).d : kFull;
     }
     const uint32_t T = kth_distance(dist, k, K);
     uint32_t below = 0, upto = 0;
@@ -437,7 +636,10 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
             const uint32_t mid = lo + ((hi - lo) >> 1);
             uint32_t c = 0;
 #pragma unroll 1
-            for (uint32_t e = lane; e < count; e += 32) c += dists[e] == T && ids[e] <= mid;
+            for (uint32_t e = lane; e < count; e += 32) {
+                const Entry x = load_entry(buf, wide, e);
+                c += x.d == T && x.node <= mid;
+            }
             if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
             else lo = mid + 1;
         }
@@ -447,14 +649,11 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
     uint32_t at = 0;
 #pragma unroll 1
     for (uint32_t e = lane; e < (count + 31u) / 32 * 32; e += 32) {  // (an entry moves down or stays)
-        const uint32_t d = e < count ? dists[e] : kFull, id = e < count ? ids[e] : kInvalidNode;
-        const bool keep = d < T || (d == T && id <= last);
+        const Entry x = e < count ? load_entry(buf, wide, e) : Entry{kFull, kInvalidNode};
+        const bool keep = x.d < T || (x.d == T && x.node <= last);
         const uint32_t m = __ballot_sync(kFull, keep);
-        if (keep) {
-            const uint32_t to = at + __popc(m & ((1u << lane) - 1u));
-            ids[to] = id;
-            dists[to] = uint8_t(d);
-        }
+        __syncwarp();
+        if (keep) store_entry(buf, wide, at + __popc(m & ((1u << lane) - 1u)), x.d, x.node);
         at += __popc(m);
         __syncwarp();
     }
@@ -462,46 +661,107 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* ids, uint8_t* dists, u
     return T;
 }
 
+// The exact distances of `rows` of the 32 places from row0 on to the 32 from col0 on, a column per lane and kBatch rows at a
+// time, and the rows found to the buffers they are of use to.  By the whole warp; row: the lane's place among the rows.
+template <bool U16, int QUADS>
+__device__ __forceinline__ void compare_rows(const KnnMmaArgs& a, uint32_t rows, uint32_t row0, uint2 row, uint32_t col0, bool both, int lane) {
+    if (rows == 0) return;
+    const uint32_t below = (1u << lane) - 1u, col = col0 + lane;
+    const uint2 p = __ldg(a.place + col);
+    uint4 own[QUADS];  // the lane's column
+#pragma unroll
+    for (int w = 0; w < QUADS; ++w) own[w] = __ldg(a.codes + size_t(col) * QUADS + w);
+    while (rows) {
+        uint32_t src[kBatch], here[kBatch], dist = 0, there = 0;  // columns of use to a row; rows of use to the column
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            src[b] = here[b] = 0;
+            if (rows) {
+                src[b] = __ffs(rows) - 1;
+                rows &= rows - 1;
+                uint4 theirs[QUADS];
+#pragma unroll
+                for (int w = 0; w < QUADS; ++w) theirs[w] = __ldg(a.codes + size_t(row0 + src[b]) * QUADS + w);
+                const uint32_t d = code_distance<U16, QUADS>(own, theirs);
+                const int row_limit = int(__shfl_sync(kFull, row.y, src[b]));
+                const uint32_t row_node = __shfl_sync(kFull, row.x, src[b]);
+                dist |= d << (8 * b);
+                here[b] = __ballot_sync(kFull, int(d) <= row_limit && p.x != kInvalidNode && col != row0 + src[b]);
+                there |= both && int(d) <= int(p.y) && row_node != kInvalidNode ? 1u << b : 0u;
+            }
+        }
+        uint32_t slot = 0, at = 0;
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+            if (here[b] && uint32_t(lane) == src[b]) slot = atomicAdd(a.counts + row0 + lane, uint32_t(__popc(here[b])));
+        if (there) at = atomicAdd(a.counts + col, uint32_t(__popc(there)));
+        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            const uint32_t d = dist >> (8 * b) & 255u;
+            const uint32_t to = __shfl_sync(kFull, slot, src[b]) + __popc(here[b] & below);
+            const uint32_t row_node = __shfl_sync(kFull, row.x, src[b]);
+            if ((here[b] >> lane & 1u) && to < kMmaCap) store_entry(buffer_of(a.entries, a.wide, row0 + src[b]), a.wide, to, d, p.x);
+            if (there >> b & 1u) {
+                if (at < kMmaCap) store_entry(buffer_of(a.entries, a.wide, col), a.wide, at, d, row_node);
+                ++at;
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// What the sweep has listed.  What bounds it is latency, of the rows and of the places in the buffers, some 1,500 cycles a
+// batch: 32 warps an SM.  (In the sweep's own epilogue, two warps a scheduler, the products wait for it: 100k x 128
+// clustered 3.2 ms in all, 2.1 with the list.)
+constexpr int kCheckWarps = 8;
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kCheckWarps * 32) knn_check_kernel(KnnMmaArgs a) {
+    if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = blockIdx.x * kCheckWarps + (threadIdx.x >> 5), warps = gridDim.x * kCheckWarps;
+    const uint32_t many = min(*a.hit_count, a.hit_room);
+    const uint32_t parts = many < 8 * warps ? 4 : 1;  // few: eight rows a warp
+    for (uint32_t i = warp; i < many * parts; i += warps) {
+        const uint4 h = __ldg(a.hits + i / parts);
+        const uint32_t rows = parts == 1 ? h.z : h.z & (0xffu << (8 * (i % parts)));
+        compare_rows<U16, QUADS>(a, rows, h.x, __ldg(a.place + h.x + lane), h.y, h.w != 0, lane);
+    }
+}
+
 template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     if (a.choice.skip()) return;
     extern __shared__ __align__(1024) unsigned char mma_smem[];
-    __shared__ __align__(8) uint64_t full_bar[2][2], empty_bar[2][2];    // [stage][part of K]
+    __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages];
     __shared__ __align__(8) uint64_t tfull_bar[2][2], tempty_bar[2][2];  // [half of the rows][side]
-    __shared__ __align__(8) uint64_t cfull_bar[kMaxCodeStages], cempty_bar[kMaxCodeStages], drain_bar;
-    __shared__ uint16_t queue[kEpiWarps][64];       // pairs a warp has collected: column | lane of the row << 8
-    __shared__ uint32_t filled[2][kMmaRows];        // [side][row]: entries of the buffer
-    __shared__ int limit[2][kMmaRows];              // [side][row]: largest distance still of use
-    __shared__ uint32_t finished[kEpiWarps];        // segments the epilogue warps are done with
+    __shared__ __align__(8) uint64_t drain_bar;
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
+    const bool calm = a.calm.yes();
+    if (calm && a.when == KnnMmaArgs::kNotIfCalm) return;
+    const Phase phase = calm && a.when == KnnMmaArgs::kAllIfCalm ? Phase{a.phase.base, 1u, false, 0u, a.meet.columns() - a.phase.base} : a.phase;
     const int lane = threadIdx.x & 31, warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
     const uint32_t operand_bytes = uint32_t(a.chunks) * kMmaRows * 16;
     const int ksteps = a.chunks / 2, split_k = (ksteps + 1) / 2;  // 32 values of K a step: two 16-byte chunks
-    unsigned char* a_sm = mma_smem;
-    unsigned char* b_sm = mma_smem + operand_bytes;      // two stages
-    unsigned char* c_sm = mma_smem + 3 * operand_bytes;  // the candidates' codes, code_stages of them
-    constexpr uint32_t kCodeBytes = kMmaRows * QUADS * 16;
     constexpr uint32_t kStepBytes = 2 * kMmaRows * 16;
-    constexpr bool kOwnInSmem = QUADS <= 4;  // the rows' own codes (wider ones: read from L2)
-    const uint64_t s0 = a.split.first_step(blockIdx.x);
-    const uint32_t steps = uint32_t(a.split.first_step(blockIdx.x + 1) - s0);
-    const uint32_t rt0 = uint32_t(s0 / a.split.cts), ct0 = uint32_t(s0 % a.split.cts);  // first row and candidate tile
+    const uint32_t stage_bytes = uint32_t(split_k) * kStepBytes;  // half of a tile along K: part 0, and part 1 at most as long
+    unsigned char* a_sm = mma_smem;
+    unsigned char* b_sm = mma_smem + operand_bytes;
+    Walk walk(a.meet.row_tiles, phase.count);
+    const uint32_t steps = walk.steps;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i)
             for (int j = 0; j < 2; ++j) {
-                knn::mbar_init(&full_bar[i][j], 1);
-                knn::mbar_init(&empty_bar[i][j], 1);
                 knn::mbar_init(&tfull_bar[i][j], 1);
                 knn::mbar_init(&tempty_bar[i][j], 4);
             }
-        for (int i = 0; i < kMaxCodeStages; ++i) {
-            knn::mbar_init(&cfull_bar[i], 1);
-            knn::mbar_init(&cempty_bar[i], kEpiWarps / 2);
+        for (int i = 0; i < kMaxStages; ++i) {
+            knn::mbar_init(&full_bar[i], 1);
+            knn::mbar_init(&empty_bar[i], 1);
         }
         knn::mbar_init(&drain_bar, 1);
-        for (int i = 0; i < kEpiWarps; ++i) finished[i] = 0;
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -515,82 +775,73 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     const uint32_t tmem = tmem_base_sm;
     volatile int* aborted = &abort_flag;
 
-    uint32_t loads = 0;  // copies issued by this warp: parts of operands, or code tiles
+    uint32_t loads = 0;  // parts whose copies this warp has issued
     if (warp == kEpiWarps) {
         if (lane == 0) {
-            uint32_t rt = rt0, ct = ct0;
-            bool fresh = true, ok = true;  // fresh: the row tile's own operand has to come too
+            uint32_t stage = 0, parity = 0;                      // parity: of the stage's next filling
+            bool fresh = true, ok = true;                       // fresh: the row tile's own operand has to come too
             const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
             for (uint32_t i = 0; i < steps && ok && !*aborted; ++i) {
-                const uint32_t s = i & 1;
-                // a new row operand replaces the one that the step before still reads
-                if (fresh && i) ok = wait_or_abort(&empty_bar[s ^ 1][1], ((i - 1) >> 1) & 1, kWaitLimit, aborted);
+                const uint32_t ct = a.meet.column(walk.rt, phase.column(walk.step()));
+                // a new row operand replaces the one that the products of the step before still read
+                if (fresh && i) {
+                    const uint32_t before = stage ? stage - 1 : uint32_t(a.stages) - 1;
+                    ok = wait_or_abort(&empty_bar[before], stage ? parity : parity ^ 1, kWaitLimit, aborted);
+                }
                 for (int part = 0; part < 2 && ok; ++part) {
-                    const uint32_t from = part ? split_k * kStepBytes : 0u;
-                    const uint32_t bytes = (part ? ksteps - split_k : split_k) * kStepBytes;
-                    ok = wait_or_abort(&empty_bar[s][part], ((i >> 1) & 1) ^ 1, kWaitLimit, aborted);
+                    const uint32_t from = part ? stage_bytes : 0u;
+                    const uint32_t bytes = part ? operand_bytes - stage_bytes : stage_bytes;
+                    ok = wait_or_abort(&empty_bar[stage], parity ^ 1, a.handover_polls, aborted);  // handed back by the products
                     if (!ok) break;
                     const uint32_t own = fresh && part == 0 ? operand_bytes : 0u;
-                    knn::mbar_expect_tx(&full_bar[s][part], bytes + own);
-                    if (own) knn::bulk_g2s(a_sm, op + size_t(a.tile0 + rt) * operand_bytes, own, &full_bar[s][part]);
-                    if (bytes) knn::bulk_g2s(b_sm + s * operand_bytes + from, op + size_t(ct) * operand_bytes + from, bytes, &full_bar[s][part]);
+                    knn::mbar_expect_tx(&full_bar[stage], bytes + own);
+                    if (own) knn::bulk_g2s(a_sm, op + size_t(walk.rt) * operand_bytes, own, &full_bar[stage]);
+                    if (bytes) knn::bulk_g2s(b_sm + stage * stage_bytes, op + size_t(ct) * operand_bytes + from, bytes, &full_bar[stage]);
                     ++loads;
+                    if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
                 }
-                fresh = ++ct == a.split.cts;
-                if (fresh) ct = 0, ++rt;
+                const uint32_t rt = walk.rt;
+                walk.next();
+                fresh = walk.rt != rt;
             }
             if (!ok) *aborted = 1;
-        }
-    } else if (warp == kEpiWarps + 2) {
-        if (lane == 0) {
-            uint32_t ct = ct0, cs = 0, parity = 1;
-            for (uint32_t i = 0; i < steps && !*aborted; ++i) {
-                if (!wait_or_abort(&cempty_bar[cs], parity, kWaitLimit, aborted)) {
-                    *aborted = 1;
-                    break;
-                }
-                const uint64_t left = a.n - uint64_t(ct) * kMmaRows;
-                const uint32_t bytes = uint32_t(left < kMmaRows ? left : kMmaRows) * QUADS * 16;
-                knn::mbar_expect_tx(&cfull_bar[cs], bytes);
-                knn::bulk_g2s(c_sm + cs * kCodeBytes, a.codes + size_t(ct) * kMmaRows * QUADS, bytes, &cfull_bar[cs]);
-                ++loads;
-                if (++cs == uint32_t(a.code_stages)) cs = 0, parity ^= 1;
-                if (++ct == a.split.cts) ct = 0;
-            }
         }
     } else if (warp == kEpiWarps + 1) {
         // The whole warp goes along and one lane issues: descriptors then stay in uniform registers.  (One thread in a
         // branch of its own took 270 cycles a product, twice what the product does.)
         const uint32_t elected = elect_one();
-        const uint64_t a_desc = operand_desc(smem_u32(a_sm));
-        const uint64_t b_desc[2] = {operand_desc(smem_u32(b_sm)), operand_desc(smem_u32(b_sm + operand_bytes))};
+        const uint64_t a_desc = operand_desc(smem_u32(a_sm)), b_desc = operand_desc(smem_u32(b_sm));
         constexpr uint64_t kStep = kStepBytes >> 4;
+        uint32_t stage = 0, parity = 0;
         bool ok = true;
         for (uint32_t i = 0; i < steps && ok; ++i) {
-            const uint32_t s = i & 1;
-            ok = __all_sync(kFull, wait_or_abort(&full_bar[s][0], (i >> 1) & 1, i == 0 ? a.first_wait_polls : kWaitLimit, aborted) && !*aborted);
+            const uint32_t side = i & 1, st0 = stage, par0 = parity;
+            if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
+            const uint32_t st1 = stage, par1 = parity;
+            if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
+            ok = __all_sync(kFull, wait_or_abort(&full_bar[st0], par0, i == 0 ? a.first_wait_polls : kWaitLimit, aborted) && !*aborted);
             for (int h = 0; h < 2 && ok; ++h) {
                 // the half was read for the step before by the other side
-                if (i) ok = __all_sync(kFull, wait_or_abort(&tempty_bar[h][s ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted));
+                if (i) ok = __all_sync(kFull, wait_or_abort(&tempty_bar[h][side ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted));
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d = tmem + h * 256;
-                uint64_t ad = a_desc + h * ((128 * 16) >> 4), bd = b_desc[s];
+                uint64_t ad = a_desc + h * ((128 * 16) >> 4), bd = b_desc + (st0 * stage_bytes >> 4);
                 if (elected) {
 #pragma unroll 4
                     for (int ks = 0; ks < split_k; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, ks != 0);
-                    if (h == 1) mma_commit(&empty_bar[s][0]);
+                    if (h == 1) mma_commit(&empty_bar[st0]);
                 }
                 if (h == 0) {
-                    ok = __all_sync(kFull, wait_or_abort(&full_bar[s][1], (i >> 1) & 1, kWaitLimit, aborted));
+                    ok = __all_sync(kFull, wait_or_abort(&full_bar[st1], par1, kWaitLimit, aborted));
                     if (!ok) break;
                 }
-                ad = a_desc + h * ((128 * 16) >> 4) + split_k * kStep, bd = b_desc[s] + split_k * kStep;
+                ad = a_desc + h * ((128 * 16) >> 4) + split_k * kStep, bd = b_desc + (st1 * stage_bytes >> 4);
                 if (elected) {
 #pragma unroll 4
                     for (int ks = split_k; ks < ksteps; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, true);
-                    mma_commit(&tfull_bar[h][s]);
-                    if (h == 1) mma_commit(&empty_bar[s][1]);
+                    mma_commit(&tfull_bar[h][side]);
+                    if (h == 1) mma_commit(&empty_bar[st1]);
                 }
             }
         }
@@ -598,157 +849,76 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         if (elected) mma_commit(&drain_bar);  // everything issued above has finished when this completes
     } else {
         const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
-        const uint32_t base = uint32_t(half * 128 + quarter * 32), local = base + lane;  // rows of the warp, of the lane
-        const uint32_t n = uint32_t(a.n);
-        const uint32_t below = (1u << lane) - 1u;
+        const uint32_t base = uint32_t(half * 128 + quarter * 32);  // the warp's rows in the tile
         const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256;
-        uint16_t* mine = queue[warp];
-        uint4* own = reinterpret_cast<uint4*>(c_sm + size_t(a.code_stages) * kCodeBytes) + base * QUADS;  // the rows' codes
-        uint32_t rt = rt0, ct = ct0, segment = 0;
-        bool ok = true, begun = false;  // begun: this side has had a tile of the segment
+        uint32_t row0 = 0;  // the warp's first row
+        uint2 row = make_uint2(kInvalidNode, ~0u);
+        bool ok = true, begun = false;  // begun: this side has had a step of the row tile
         for (uint32_t i = 0; i < steps; ++i) {
-            const uint32_t row0 = (a.tile0 + rt) * kMmaRows + base;  // the warp's first row
-            const bool last = ct + 1 == a.split.cts || i + 1 == steps;  // of the segment
+            const uint32_t rt = walk.rt, ct = a.meet.column(rt, phase.column(walk.step()));
+            const bool last = walk.last() || i + 1 == steps;  // of the row tile
+            walk.next();
             if ((i & 1) == uint32_t(side)) {
-                const size_t buf0 = ((size_t(blockIdx.x + rt) * kMmaRows + base) * 2 + side) * kMmaCap;
+                if (!begun) {
+                    begun = true;
+                    row0 = rt * kMmaRows + base;
+                    row = __ldg(a.place + row0 + lane);
+                }
+                // a pair is of use at the row's limit or at its column's, of which the largest of 32 stands for all at first
+                const bool both = a.meet.both(rt, ct);
+                const int least = gate_of(a.symbols, a.K, int(row.y));
+                uint4 gates = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+                if (both) gates = __ldg(reinterpret_cast<const uint4*>(a.gate) + ct);
                 ok = wait_or_abort(&tfull_bar[half][side], (i >> 1) & 1, kWaitLimit, aborted);
                 if (__ballot_sync(kFull, !ok || *aborted)) {
                     ok = false;
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (!begun) {
-                    // the rows' other warp has to be done with the segment before, whose codes and limits are replaced
-                    begun = true;
-                    ok = handed_over(&finished[warp ^ 8], segment, a.handover_polls, aborted);
-                    if (__ballot_sync(kFull, !ok)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t row = row0 + lane;
-                    const bool wanted = row >= a.row_begin && row < a.row_end;
-                    limit[side][local] = wanted ? int(min(a.bound[row], uint32_t(a.K))) : -1;
-                    filled[side][local] = 0;
-                    if (kOwnInSmem && wanted)
+                // the largest product of every 32 columns; one load is in flight while the columns of the one before are looked at
+                uint32_t r[2][16], hit = 0;
+                tmem_load32(r[0], addr);
 #pragma unroll
-                        for (int w = 0; w < QUADS; ++w) own[lane * QUADS + w] = __ldg(a.codes + size_t(row) * QUADS + w);
-                    __syncwarp();
-                }
-                const __half2 thr = dot_of_distance(a.symbols, a.K, *reinterpret_cast<volatile int*>(&limit[side][local]));
-                // pairs that pass, bit j of a word: column 2 j for j < 16, else column 2 (j - 16) + 1; one load is in flight
-                // while the columns of the one before are compared
-                uint32_t pass[8], r[2][8];
-                tmem_load16(r[0], addr);
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    tmem_wait(r[c & 1]);
-                    if (c < 15) tmem_load16(r[(c + 1) & 1], addr + (c + 1) * 16);
-                    uint32_t m = c & 1 ? pass[c >> 1] : 0u;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        m |= __hge2_mask(*reinterpret_cast<const __half2*>(&r[c & 1][j]), thr) & (0x00010001u << (j + (c & 1) * 8));
-                    pass[c >> 1] = m;
+                for (int g = 0; g < 8; ++g) {
+                    uint32_t (&v)[16] = r[g & 1];
+                    tmem_wait(v);
+                    if (g < 7) tmem_load32(r[(g + 1) & 1], addr + (g + 1) * 32);
+                    const uint32_t m0 = __vimax3_s16x2(v[0], v[1], v[2]), m1 = __vimax3_s16x2(v[3], v[4], v[5]);
+                    const uint32_t m2 = __vimax3_s16x2(v[6], v[7], v[8]), m3 = __vimax3_s16x2(v[9], v[10], v[11]);
+                    const uint32_t m4 = __vimax3_s16x2(v[12], v[13], v[14]);
+                    const uint32_t m = __vimax3_s16x2(__vimax3_s16x2(m0, m1, m2), __vimax3_s16x2(m3, m4, v[15]), 0x80008000u);
+                    const uint32_t pair = g < 4 ? (g < 2 ? gates.x : gates.y) : (g < 6 ? gates.z : gates.w);
+                    const int gate = min(least, g & 1 ? int(pair) >> 16 : int(int16_t(pair)));
+                    hit |= max(int(int16_t(m)), int(m) >> 16) >= gate ? 1u << g : 0u;
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&tempty_bar[half][side]);
 
-                // their exact distances, 32 pairs at a time, a lane each
-                const uint32_t cs = i % uint32_t(a.code_stages);
-                ok = wait_or_abort(&cfull_bar[cs], (i / uint32_t(a.code_stages)) & 1, kWaitLimit, aborted);
-                if (__ballot_sync(kFull, !ok)) {
-                    ok = false;
-                    break;
-                }
-                const uint4* cand = reinterpret_cast<const uint4*>(c_sm + cs * kCodeBytes);
-                const uint32_t col0 = ct * kMmaRows;
-                uint32_t queued = 0;
-                auto drain = [&](uint32_t m) {
-                    __syncwarp();
-                    queued -= m;
-                    const bool act = uint32_t(lane) < m;
-                    const uint32_t e = act ? mine[queued + lane] : 0u;
-                    const uint32_t col = e & 255u, src = e >> 8;
-                    const uint4* theirs = kOwnInSmem ? own + src * QUADS : a.codes + size_t(min(row0 + src, n - 1)) * QUADS;
-                    const int d = int(code_distance<U16, QUADS>(theirs, cand + col * QUADS));
-                    const uint32_t id = col0 + col;
-                    if (act && id != row0 + src && d <= *reinterpret_cast<volatile int*>(&limit[side][base + src])) {
-                        const size_t to = buf0 + size_t(src) * (2 * kMmaCap) + atomicAdd(&filled[side][base + src], 1u);
-                        a.ids[to] = id;
-                        a.dists[to] = uint8_t(d);
-                    }
-                    __syncwarp();
-                };
-                if (col0 + kMmaRows > n) {  // columns past the last node
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const uint32_t from = col0 + c * 32, have = from >= n ? 0u : (n - from < 32 ? n - from : 32u);
-                        pass[c] &= ((1u << ((have + 1) / 2)) - 1u) | ((1u << (have / 2)) - 1u) << 16;
-                    }
-                }
-                uint32_t words = 0;  // the words that have a pair left, beside the current one
-#pragma unroll
-                for (int c = 0; c < 8; ++c) words |= pass[c] ? 1u << c : 0u;
-                uint32_t word = 0, at = 0;
-                while (true) {
-                    if (word == 0 && words) {
-                        at = __ffs(words) - 1;
-                        words &= words - 1;
-                        const uint32_t w0 = at & 1 ? pass[1] : pass[0], w1 = at & 1 ? pass[3] : pass[2];
-                        const uint32_t w2 = at & 1 ? pass[5] : pass[4], w3 = at & 1 ? pass[7] : pass[6];
-                        const uint32_t lo = at & 2 ? w1 : w0, hi = at & 2 ? w3 : w2;
-                        word = at & 4 ? hi : lo;
-                    }
-                    const uint32_t any = __ballot_sync(kFull, word != 0);
-                    if (any == 0) break;
-                    const uint32_t b = __ffs(word) - 1;
-                    if (word) mine[queued + __popc(any & below)] = uint16_t(at * 32 + 2 * (b & 15) + (b >> 4) + (lane << 8));
-                    word &= word - 1;
-                    queued += __popc(any);
-                    if (queued >= 32) drain(32);
-                }
-                if (queued) drain(queued);
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&cempty_bar[cs]);
-
-                // rows whose buffer could overflow in the next tile
-                uint32_t full = __ballot_sync(kFull, filled[side][local] > kMmaKeep);
-                while (full) {
-                    const int src = __ffs(full) - 1;
-                    full &= full - 1;
-                    uint32_t count = filled[side][base + src];
-                    const size_t at = buf0 + size_t(src) * (2 * kMmaCap);
-                    const uint32_t T = compact_row(a.ids + at, a.dists + at, count, a.k, a.K, lane);
-                    if (lane == 0) {
-                        filled[side][base + src] = count;
-                        // this side's later candidates have higher ids and must be strictly closer
-                        atomicMin(&limit[side][base + src], int(T) - 1);
-                        atomicMin(&limit[side ^ 1][base + src], int(T));
+                uint32_t any_hit = __reduce_or_sync(kFull, hit);
+                if (any_hit) {  // listed; where there is no room, compared at once
+                    uint32_t at = 0;
+                    if (lane == 0) at = atomicAdd(a.hit_count, uint32_t(__popc(any_hit)));
+                    at = __shfl_sync(kFull, at, 0);
+                    for (; any_hit; any_hit &= any_hit - 1, ++at) {
+                        const int g = __ffs(any_hit) - 1;
+                        const uint32_t rows = __ballot_sync(kFull, hit >> g & 1u), col0 = ct * kMmaRows + g * 32;
+                        if (at >= a.hit_room) compare_rows<U16, QUADS>(a, rows, row0, row, col0, both, lane);
+                        else if (lane == 0) a.hits[at] = make_uint4(row0, col0, rows, both ? 1u : 0u);
                     }
                     __syncwarp();
                 }
             }
-            if (last) {
-                a.counts[(size_t(blockIdx.x + rt) * kMmaRows + local) * 2 + side] = begun ? filled[side][local] : 0u;
-                begun = false;
-                __syncwarp();
-                ++segment;
-                if (lane == 0) hand_over(&finished[warp], segment);
-            }
-            if (++ct == a.split.cts) ct = 0, ++rt;
+            if (last) begun = false;
         }
         if (!ok) *aborted = 1;
     }
     __syncthreads();
     // copies and products in flight after a lost wait end before the block's memory goes away
-    if (*aborted && lane == 0) {
-        if (warp == kEpiWarps) {
-            atomicExch(a.status, kStatusWaitTimeout);
-            for (uint32_t l = loads > 4 ? loads - 4 : 0; l < loads; ++l) mbar_wait_bounded(&full_bar[(l >> 1) & 1][l & 1], (l >> 2) & 1, kWaitLimit);
-        } else if (warp == kEpiWarps + 2) {
-            const uint32_t stages = uint32_t(a.code_stages);
-            for (uint32_t l = loads > stages ? loads - stages : 0; l < loads; ++l) mbar_wait_bounded(&cfull_bar[l % stages], (l / stages) & 1, kWaitLimit);
-        }
+    if (*aborted && warp == kEpiWarps && lane == 0) {
+        atomicExch(a.status, kStatusWaitTimeout);
+        const uint32_t stages = uint32_t(a.stages);
+        for (uint32_t l = loads > stages ? loads - stages : 0; l < loads; ++l) mbar_wait_bounded(&full_bar[l % stages], (l / stages) & 1, kWaitLimit);
     }
     if (warp == kEpiWarps + 1) {
         if (lane == 0) mbar_wait_bounded(&drain_bar, 0, kWaitLimit);
@@ -759,102 +929,378 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     __syncthreads();
 }
 
-// ---- results: the k best of a row's buffers by (distance, id) ---------------------------------------------------------
+// ---- order of the nodes ----------------------------------------------------------------------------------------------
+// A node's group is named by the smallest node among its likely neighbours, whose group is named the same way, followed to
+// the end (nodes only get smaller; where it takes long, not to the end).  A cluster has a few such names; a node and its
+// mate join theirs.
+__device__ __forceinline__ uint32_t name_of(uint32_t* group, uint32_t node) {
+    for (int i = 0; i < 64; ++i) {
+        const uint32_t up = *reinterpret_cast<volatile uint32_t*>(group + node);
+        if (up == node) break;
+        node = up;
+    }
+    return node;
+}
+__global__ void group_join_kernel(uint32_t* __restrict__ group, const uint32_t* __restrict__ mate, uint32_t row_begin, uint32_t row_end,
+                                  SweepChoice choice) {
+    if (choice.skip()) return;
+    const uint32_t row = row_begin + blockIdx.x * blockDim.x + threadIdx.x;
+    if (row >= row_end) return;
+    const uint32_t a = name_of(group, row), b = name_of(group, mate[row]);
+    if (a != b) atomicMin(group + max(a, b), min(a, b));  // (one of several for the same name stays: the next round has the others)
+}
+__global__ void group_count_kernel(uint32_t* __restrict__ group, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ count, SweepChoice choice) {
+    if (choice.skip()) return;
+    const uint32_t row = row_begin + blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t g = row < row_end ? name_of(group, row) : kInvalidNode;
+    const uint32_t same = __match_any_sync(kFull, g);
+    if (row >= row_end) return;
+    group[row] = g;  // (a name on the same path: who reads it meanwhile gets there as well)
+    if ((threadIdx.x & 31) == uint32_t(__ffs(same) - 1)) atomicAdd(count + g, uint32_t(__popc(same)));
+}
+// the places of the groups, in any order
+__global__ void group_place_kernel(const uint32_t* __restrict__ count, uint32_t n, uint32_t* __restrict__ place, uint32_t* __restrict__ used,
+                                   SweepChoice choice) {
+    if (choice.skip()) return;
+    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t c = g < n ? count[g] : 0u;
+    uint32_t upto = c;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, upto, d);
+        if (lane >= uint32_t(d)) upto += y;
+    }
+    uint32_t at = 0;
+    if (lane == 31 && upto) at = atomicAdd(used, upto);
+    at = __shfl_sync(kFull, at, 31) + upto - c;
+    if (c) place[g] = at;
+}
+__global__ void group_scatter_kernel(const uint32_t* __restrict__ group, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ place,
+                                     uint32_t* __restrict__ node, SweepChoice choice) {
+    if (choice.skip()) return;
+    const uint32_t row = row_begin + blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const uint32_t g = row < row_end ? group[row] : kInvalidNode;
+    const uint32_t same = __match_any_sync(kFull, g), first = __ffs(same) - 1;
+    uint32_t at = 0;
+    if (row < row_end && lane == first) at = atomicAdd(place + g, uint32_t(__popc(same)));
+    at = __shfl_sync(kFull, at, first);
+    if (row < row_end) node[at + __popc(same & ((1u << lane) - 1u))] = row;
+}
+// A block of 1,024 places: wanted rows, which come first (in their groups' order, or without one), a group's sorted by their limits; the other nodes behind the row
+// tiles as they are; codes, limits and gates.
+template <int QUADS>
+__global__ void __launch_bounds__(kSortRows) layout_kernel(const uint4* __restrict__ codes, uint32_t n, uint32_t row_begin, uint32_t row_end,
+                                                           const uint32_t* __restrict__ bound, const uint32_t* __restrict__ group, int K, int symbols, Meet meet,
+                                                           const uint32_t* __restrict__ node, uint4* __restrict__ out, uint2* __restrict__ places,
+                                                           int16_t* __restrict__ gate, SweepChoice choice) {
+    if (choice.skip()) return;
+    constexpr int kGates = kSortRows / 32, kGroups = 8, kLimits = 72;  // (groups from the eighth on are sorted together)
+    __shared__ uint32_t cursor[kGroups * kLimits], begun[32];
+    __shared__ int largest[kGates];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, chunk = blockIdx.x * kSortRows, place = chunk + tid;
+    const uint32_t wanted = row_end - row_begin, behind = meet.row_tiles * kMmaRows;
+    if (tid < kGroups * kLimits) cursor[tid] = 0;
+    if (tid < kGates) largest[tid] = -1;
+    uint32_t id = kInvalidNode, to = place, bin = 0;
+    int lim = -1;
+    bool begins = false;
+    if (place < wanted) {
+        id = node ? node[place] : row_begin + place;
+        lim = int(min(bound[id], uint32_t(K)));
+        begins = node && tid > 0 && group[id] != group[node[place - 1]];
+    } else if (place >= behind && place - behind < n - wanted) {
+        id = place - behind;
+        if (id >= row_begin) id += wanted;
+    }
+    const uint32_t starts = __ballot_sync(kFull, begins);
+    if (lane == 0) begun[warp] = __popc(starts);
+    __syncthreads();
+    if (lim >= 0) {
+        uint32_t g = __popc(starts & (0xffffffffu >> (31 - lane)));
+        for (uint32_t w = 0; w < warp; ++w) g += begun[w];
+        bin = min(g, uint32_t(kGroups - 1)) * kLimits + uint32_t(lim);
+        atomicAdd(&cursor[bin], 1u);
+    }
+    __syncthreads();
+    if (warp == 0) {  // exclusive
+        constexpr int kEach = kGroups * kLimits / 32;
+        uint32_t x = 0;
+        for (int i = 0; i < kEach; ++i) x += cursor[lane * kEach + i];
+        const uint32_t own = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, o);
+            if (lane >= uint32_t(o)) x += y;
+        }
+        x -= own;
+        for (int i = 0; i < kEach; ++i) {
+            const uint32_t c = cursor[lane * kEach + i];
+            cursor[lane * kEach + i] = x;
+            x += c;
+        }
+    }
+    __syncthreads();
+    if (lim >= 0) {
+        const uint32_t rank = atomicAdd(&cursor[bin], 1u);
+        to = chunk + rank;
+        atomicMax(&largest[rank / 32], lim);
+    }
+    __syncthreads();
+    if (to < meet.tiles * kMmaRows) {
+        places[to] = make_uint2(id, uint32_t(lim));
+#pragma unroll
+        for (int w = 0; w < QUADS; ++w) out[size_t(to) * QUADS + w] = id != kInvalidNode ? __ldg(codes + size_t(id) * QUADS + w) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (tid < kGates && chunk + tid * 32 < meet.row_tiles * kMmaRows) gate[chunk / 32 + tid] = int16_t(gate_of(symbols, K, largest[tid]));
+}
+
+// ---- between two phases: room in the buffers, limits of the k best so far ---------------------------------
+// Where a buffer ran over the k-th distance of what it holds is a limit that few nodes are within: with a list the buffer
+// starts anew and the row is listed for knn_again_kernel (without one nothing more is of use to the row for now).
+__global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool only_lost, uint32_t* __restrict__ again /* their number, places */) {
+    if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
+    const int lane = threadIdx.x & 31;
+    const uint32_t row0 = blockIdx.x * kMmaRows + (threadIdx.x & ~31u), own = row0 + lane;
+    uint32_t count = a.counts[own];
+    int limit = int(a.place[own].y);
+    const bool lost = count > kMmaCap, anew = lost && again;
+    uint32_t todo = __ballot_sync(kFull, anew || (!lost && !only_lost && count >= a.k && limit >= 0));
+    const uint32_t anews = __ballot_sync(kFull, anew);
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        uint32_t c = min(__shfl_sync(kFull, count, src), kMmaCap);
+        uint32_t* buf = buffer_of(a.entries, a.wide, row0 + src);
+        uint32_t T;
+        auto kth = [&](auto slots) {
+            uint32_t dist[decltype(slots)::value];
+#pragma unroll
+            for (int s = 0; s < decltype(slots)::value; ++s) dist[s] = uint32_t(s * 32 + lane) < c ? load_entry(buf, a.wide, s * 32 + lane).d : kFull;
+            return kth_distance(dist, a.k, a.K);
+        };
+        if (!(anews >> src & 1u) && c > kMmaFull) T = compact_row(buf, a.wide, c, a.k, a.K, lane);
+        else if (c > kMmaFull) T = kth(std::integral_constant<int, kMmaSlots>());
+        else if (c > kMmaKeep) T = kth(std::integral_constant<int, kMmaFull / 32>());
+        else T = kth(std::integral_constant<int, kMmaKeep / 32>());
+        if (anews >> src & 1u) c = 0;
+        if (lane == src) count = c, limit = limit < 0 || limit > int(T) ? int(T) : limit;
+    }
+    if (anew) again[1 + atomicAdd(again, 1u)] = own;
+    if (lost && !again) limit = -1;
+    if (only_lost && !anews) return;
+    a.counts[own] = count;
+    a.place[own].y = uint32_t(limit);
+    const int most = __reduce_max_sync(kFull, limit);
+    if (lane == 0) a.gate[row0 / 32] = int16_t(gate_of(a.symbols, a.K, most));
+}
+
+// The listed rows against the nodes of all tiles, or of the row tiles less than `near` tiles away, at their new limits; grid
+// y deals the rows, grid x the nodes.
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint32_t* __restrict__ again, uint32_t near) {
+    if (a.choice.skip()) return;
+    const uint32_t many = again[0], places = (near ? 2 * near - 1 : a.meet.tiles) * kMmaRows;
+    for (uint32_t b = blockIdx.y; b < many; b += gridDim.y) {
+        const uint32_t row = again[1 + b], tile = row / kMmaRows;
+        const uint32_t from = near ? (tile >= near - 1 ? tile - (near - 1) : tile + a.meet.row_tiles - (near - 1)) * kMmaRows : 0;
+        const int limit = int(a.place[row].y);
+        uint4 own[QUADS];
+#pragma unroll
+        for (int w = 0; w < QUADS; ++w) own[w] = __ldg(a.codes + size_t(row) * QUADS + w);
+#pragma unroll 4
+        for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < places; i += gridDim.x * 256) {
+            uint32_t j = from + i;
+            if (near && j >= a.meet.row_tiles * kMmaRows) j -= a.meet.row_tiles * kMmaRows;
+            uint4 v[QUADS];
+#pragma unroll
+            for (int w = 0; w < QUADS; ++w) v[w] = __ldg(a.codes + size_t(j) * QUADS + w);
+            const int d = int(code_distance<U16, QUADS>(own, v));
+            if (d > limit || j == row) continue;
+            const uint32_t node = a.place[j].x;
+            if (node == kInvalidNode) continue;
+            const uint32_t at = atomicAdd(a.counts + row, 1u);
+            if (at < kMmaCap) store_entry(buffer_of(a.entries, a.wide, row), a.wide, at, uint32_t(d), node);
+        }
+    }
+}
+
+// ---- results: the k best of a row's buffer by (distance, id) -----------------------------------------------------------
+// A warp a row.  The entries up to the k-th distance, k and a few ties, are sorted in registers as the words they are; where
+// they are wide or many, a row's rank is the number of entries before it.
 constexpr int kFinishWarps = 4;
-constexpr int kFinishKeys = 512;
+constexpr int kFinishSort = 128;
 
 __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
-                                                                       uint16_t* __restrict__ dists, uint32_t out_row0) {
+                                                                       uint16_t* __restrict__ dists, uint32_t out_row0,
+                                                                       uint32_t* __restrict__ redo /* their number, rows */) {
     if (a.choice.skip()) return;
-    __shared__ uint64_t keys_sm[kFinishWarps][kFinishKeys];
-    __shared__ uint32_t hist_sm[kFinishWarps][96];
+    __shared__ uint64_t keys_sm[kFinishWarps][kMmaCap];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t local = blockIdx.x * kFinishWarps + warp;
-    if (local >= rows) return;
-    const uint32_t row = a.tile0 * kMmaRows + local;
-    if (row < a.row_begin || row >= a.row_end) return;
-    uint64_t* keys = keys_sm[warp];
-    uint32_t* hist = hist_sm[warp];
-    const uint32_t rt = local / kMmaRows, in_tile = local % kMmaRows;
-    const uint32_t seg0 = a.split.block_of(uint64_t(rt) * a.split.cts) + rt;
-    const uint32_t seg1 = a.split.block_of(uint64_t(rt + 1) * a.split.cts - 1) + rt;
-    // every buffer of the row, 32 entries at a time
-    auto each = [&](auto&& f) {
-        for (uint32_t b = seg0 * 2; b <= seg1 * 2 + 1; ++b) {
-            const size_t slot = (size_t(b >> 1) * kMmaRows + in_tile) * 2 + (b & 1);
-            const uint32_t count = a.counts[slot];
-            for (uint32_t e = 0; e < count; e += 32) {
-                const bool have = e + lane < count;
-                f(have ? uint32_t(a.dists[slot * kMmaCap + e + lane]) : kFull, slot * kMmaCap + e + lane);
-            }
-        }
-    };
-    for (int i = lane; i < 96; i += 32) hist[i] = 0;
-    __syncwarp();
-    each([&](uint32_t d, size_t) {
-        if (d != kFull) atomicAdd(hist + d, 1u);
-    });
-    __syncwarp();
-    // T: the k-th distance (K when there are fewer); lane l owns bins 3 l .. 3 l + 2
-    const uint32_t h0 = hist[3 * lane], h1 = hist[3 * lane + 1], h2 = hist[3 * lane + 2];
-    uint32_t x = h0 + h1 + h2;
+    const uint32_t place = blockIdx.x * kFinishWarps + warp;
+    if (place >= rows) return;
+    const uint32_t row = a.place[place].x, count = a.counts[place];
+    if (row == kInvalidNode) return;
+    if (count > kMmaCap) {
+        if (lane == 0) redo[1 + atomicAdd(redo, 1u)] = row;
+        return;
+    }
+    const uint32_t* buf = buffer_of(a.entries, a.wide, place);
+    Entry x[kMmaSlots];
+    uint32_t dist[kMmaSlots];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
+    for (int s = 0; s < kMmaSlots; ++s) {
+        x[s] = Entry{kFull, 0u};
+        if (s * 32u < count && uint32_t(s * 32 + lane) < count) x[s] = load_entry(buf, a.wide, s * 32 + lane);
+        dist[s] = x[s].d;
     }
-    const uint32_t total = __shfl_sync(kFull, x, 31), lower = x - h0 - h1 - h2;  // entries in the bins of earlier lanes
-    uint32_t T = kFull, below = 0;
-    if (lower < a.k && x >= a.k) {
-        T = 3 * lane, below = lower;
-        if (below + h0 < a.k) {
-            ++T, below += h0;
-            if (below + h1 < a.k) ++T, below += h1;
-        }
+    uint32_t T = uint32_t(a.K);
+    if (count > a.k) {
+        if (count <= kMmaKeep) T = kth_distance(reinterpret_cast<const uint32_t (&)[kMmaKeep / 32]>(dist), a.k, a.K);
+        else T = kth_distance(dist, a.k, a.K);
     }
-    const uint32_t owner = __ballot_sync(kFull, T != kFull);
-    uint32_t last = kInvalidNode, kept = total;  // largest id of use at distance T; entries collected
-    if (owner) {
-        const int src = __ffs(owner) - 1;
-        T = __shfl_sync(kFull, T, src);
-        below = __shfl_sync(kFull, below, src);
-        kept = below + hist[T];
-        if (kept > uint32_t(kFinishKeys)) {  // a great many ties: the id that bounds the ones wanted
-            uint32_t lo = 0, hi = kInvalidNode;
-            while (lo < hi) {
-                const uint32_t mid = lo + ((hi - lo) >> 1);
-                uint32_t c = 0;
-                each([&](uint32_t d, size_t at) { c += d == T && a.ids[at] <= mid; });
-                if (__reduce_add_sync(kFull, c) >= a.k - below) hi = mid;
-                else lo = mid + 1;
-            }
-            last = lo;
-        }
-    }
-    uint32_t m = 0;
-    each([&](uint32_t d, size_t at) {
-        const uint32_t id = d <= T && d != kFull ? a.ids[at] : kInvalidNode;
-        const bool take = id != kInvalidNode && (d < T || id <= last);
-        const uint32_t b = __ballot_sync(kFull, take);
-        if (take) keys[m + __popc(b & ((1u << lane) - 1u))] = (uint64_t(d) << 32) | id;
-        m += __popc(b);
-    });
-    __syncwarp();
     uint32_t* out_n = nbrs + size_t(row - out_row0) * a.k;
     uint16_t* out_d = dists ? dists + size_t(row - out_row0) * a.k : nullptr;
-    for (uint32_t e = lane; e < m; e += 32) {  // rank by counting: keys are distinct
-        const uint64_t key = keys[e];
-        uint32_t rank = 0;
-#pragma unroll 4
-        for (uint32_t i = 0; i < m; ++i) rank += keys[i] < key;
-        if (rank < a.k) {
-            out_n[rank] = uint32_t(key);
-            if (out_d) out_d[rank] = uint16_t(key >> 32);
+    uint64_t* keys = keys_sm[warp];
+    uint32_t* words = reinterpret_cast<uint32_t*>(keys);
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t m = 0;
+#pragma unroll
+    for (int s = 0; s < kMmaSlots; ++s) {
+        if (s * 32u >= count) break;
+        const bool take = x[s].d <= T;
+        const uint32_t b = __ballot_sync(kFull, take), at = m + __popc(b & below);
+        if (take && a.wide) keys[at] = (uint64_t(x[s].d) << 32) | x[s].node;
+        else if (take) words[at] = x[s].d << 25 | x[s].node;
+        m += __popc(b);
+    }
+    __syncwarp();
+    const uint32_t kept = min(m, a.k);
+    if (!a.wide && m <= uint32_t(kFinishSort)) {
+        uint32_t v[kFinishSort / 32];  // element s * 32 + lane
+#pragma unroll
+        for (int s = 0; s < kFinishSort / 32; ++s) v[s] = uint32_t(s * 32 + lane) < m ? words[s * 32 + lane] : kFull;
+#pragma unroll
+        for (int size = 2; size <= kFinishSort; size *= 2) {
+#pragma unroll
+            for (int d = size / 2; d >= 1; d /= 2) {
+                if (d >= 32) {
+#pragma unroll
+                    for (int s = 0; s < kFinishSort / 32; ++s) {
+                        if (s & (d / 32)) continue;
+                        const bool up = ((s * 32) & size) == 0;  // (the whole is ascending: no bit at its size)
+                        const uint32_t lo = min(v[s], v[s | (d / 32)]), hi = max(v[s], v[s | (d / 32)]);
+                        v[s] = up ? lo : hi, v[s | (d / 32)] = up ? hi : lo;
+                    }
+                } else {
+#pragma unroll
+                    for (int s = 0; s < kFinishSort / 32; ++s) {
+                        const uint32_t y = __shfl_xor_sync(kFull, v[s], d);
+                        const bool low = ((lane & d) == 0) == (((s * 32 + lane) & size) == 0);
+                        v[s] = low ? min(v[s], y) : max(v[s], y);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < kFinishSort / 32; ++s) {
+            const uint32_t rank = s * 32 + lane;
+            if (rank >= kept) continue;
+            out_n[rank] = v[s] & (kPackedNodes - 1u);
+            if (out_d) out_d[rank] = uint16_t(v[s] >> 25);
+        }
+    } else {
+        for (uint32_t e = lane; e < m; e += 32) {
+            auto key = [&](uint32_t i) { return a.wide ? keys[i] : (uint64_t(words[i] >> 25) << 32) | (words[i] & (kPackedNodes - 1u)); };
+            const uint64_t own = key(e);
+            uint32_t rank = 0;
+            for (uint32_t i = 0; i < m; ++i) rank += key(i) < own;
+            if (rank >= kept) continue;
+            out_n[rank] = uint32_t(own);
+            if (out_d) out_d[rank] = uint16_t(own >> 32);
         }
     }
-    for (uint32_t o = m + lane; o < a.k; o += 32) {
+    for (uint32_t o = kept + lane; o < a.k; o += 32) {
         out_n[o] = kInvalidNode;
         if (out_d) out_d[o] = 0xFFFF;
+    }
+}
+
+// ---- rows whose buffer ran over: compared with every node ---------------------------------------------------------------
+// A block a row, twice over the nodes: the distances up to the row's bound are counted, then the nodes below the k-th are
+// collected, and the smallest ids at it, which every warp finds first in its own range of the nodes.
+constexpr int kRedoWarps = 32;
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kRedoWarps * 32) knn_redo_kernel(const uint4* __restrict__ codes, uint32_t n, uint32_t k, int K,
+                                                                   const uint32_t* __restrict__ bound, const uint32_t* __restrict__ redo,
+                                                                   uint32_t* __restrict__ nbrs, uint16_t* __restrict__ dists, uint32_t out_row0,
+                                                                   SweepChoice choice) {
+    if (choice.skip()) return;
+    __shared__ uint32_t hist[96], ties[kRedoWarps][128], tie_count[kRedoWarps], below_sm, T_sm, found;
+    __shared__ uint64_t keys[128];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, many = redo[0];
+    const uint32_t from = uint32_t(uint64_t(n) * warp / kRedoWarps), to = uint32_t(uint64_t(n) * (warp + 1) / kRedoWarps);
+    for (uint32_t b = blockIdx.x; b < many; b += gridDim.x) {
+        const uint32_t row = redo[1 + b], most = min(bound[row], uint32_t(K));
+        uint4 own[QUADS];
+#pragma unroll
+        for (int w = 0; w < QUADS; ++w) own[w] = __ldg(codes + size_t(row) * QUADS + w);
+        auto distance = [&](uint32_t j) {
+            uint4 v[QUADS];
+#pragma unroll
+            for (int w = 0; w < QUADS; ++w) v[w] = __ldg(codes + size_t(j) * QUADS + w);
+            return code_distance<U16, QUADS>(own, v);
+        };
+        if (tid < 96) hist[tid] = 0;
+        if (tid == 0) found = 0;
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t j0 = from; j0 < to; j0 += 32) {
+            const uint32_t j = j0 + lane, d = j < to && j != row ? distance(j) : kFull;
+            // one addition for the lanes at the lowest distance of the step, one each for the others
+            const uint32_t low = __reduce_min_sync(kFull, d), same = __ballot_sync(kFull, d == low);
+            if (low > most) continue;
+            if (d == low ? lane == uint32_t(__ffs(same) - 1) : d <= most) atomicAdd(hist + d, d == low ? uint32_t(__popc(same)) : 1u);
+        }
+        __syncthreads();
+        if (tid == 0) {
+            uint32_t T = 0, below = 0;
+            while (T < most && below + hist[T] < k) below += hist[T++];
+            T_sm = T, below_sm = below;
+        }
+        __syncthreads();
+        const uint32_t T = T_sm, below = below_sm, need = k - below;  // need >= 1 of those at T (or all there are)
+        uint32_t have = 0;
+#pragma unroll 4
+        for (uint32_t j0 = from; j0 < to; j0 += 32) {
+            const uint32_t j = j0 + lane, d = j < to && j != row ? distance(j) : kFull;
+            if (d < T) keys[atomicAdd(&found, 1u)] = (uint64_t(d) << 32) | j;
+            const uint32_t m = __ballot_sync(kFull, d == T);
+            const uint32_t at = have + __popc(m & ((1u << lane) - 1u));
+            if (d == T && at < need) ties[warp][at] = j;
+            have = min(need, have + uint32_t(__popc(m)));
+        }
+        if (lane == 0) tie_count[warp] = have;
+        __syncthreads();
+        uint32_t skip = 0;  // ties of the warps before
+        for (uint32_t w = 0; w < warp; ++w) skip += tie_count[w];
+        for (uint32_t i = lane; i < have && skip + i < need; i += 32) keys[below + skip + i] = (uint64_t(T) << 32) | ties[warp][i];
+        uint32_t total = 0;
+        for (uint32_t w = 0; w < kRedoWarps; ++w) total += tie_count[w];
+        total = below + min(need, total);
+        __syncthreads();
+        uint32_t* out_n = nbrs + size_t(row - out_row0) * k;
+        uint16_t* out_d = dists ? dists + size_t(row - out_row0) * k : nullptr;
+        if (tid < k) {
+            uint32_t rank = tid, id = kInvalidNode, d = 0xFFFF;
+            if (tid < total) {
+                const uint64_t key = keys[tid];
+                rank = 0, id = uint32_t(key), d = uint32_t(key >> 32);
+                for (uint32_t i = 0; i < total; ++i) rank += keys[i] < key;
+            }
+            out_n[rank] = id;
+            if (out_d) out_d[rank] = uint16_t(d);
+        }
+        __syncthreads();
     }
 }
 
@@ -863,22 +1309,35 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
                  uint64_t row_end, uint32_t* d_nbrs, uint16_t* d_dist, double most_turns, SweepChoice* other, cudaStream_t st) {
     constexpr bool U16 = sizeof(CompT) == 2;
     const CompT* codes = static_cast<const CompT*>(d_codes);
+    const uint4* rows = reinterpret_cast<const uint4*>(padded);
     const HashShape shape = hash_shape(int(h->K));
-    const uint64_t tiles = (n + kMmaRows - 1) / kMmaRows;
-    const size_t operand_bytes = size_t(shape.chunks) * kMmaRows * 16;
-    const uint64_t sms = uint64_t(h->sm_count);
-    // row tiles go in launches of whole waves (the buffers of a segment take 960 KB) and a last one that splits the rest
-    constexpr uint64_t kWaves = 2;
-    const uint64_t first_tile = row_begin / kMmaRows, end_tile = (row_end - 1) / kMmaRows + 1;
-    const uint64_t most = end_tile - first_tile < kWaves * sms ? end_tile - first_tile : kWaves * sms;
-    const size_t segments = size_t(most + sms);
+    const uint32_t operand_bytes = uint32_t(shape.chunks) * kMmaRows * 16;
+    const uint32_t sms = uint32_t(h->sm_count);
+    const uint64_t wanted = row_end - row_begin;
+    if (n > (1u << 27) - 2 * kMmaRows) return kNoRoom;  // (a collected pair has 27 bits for a place)
 
+    // Workspace.  The buffers of the rows found take 1.9 KB a wanted row: where they do not fit, the rows go in blocks.
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t op_b = up(size_t(tiles) * operand_bytes), hist_b = up(size_t(kBoundOrders) * kKeys * 4 + 8);
-    const size_t order_b = up(size_t(kBoundOrders) * n * 4), place_b = order_b, bound_b = up(size_t(n) * 4);
-    const size_t slots = segments * kMmaRows * 2;
-    const size_t ids_b = up(slots * kMmaCap * 4), dists_b = up(slots * kMmaCap), counts_b = up(slots * 4);
-    CPB_TRY(reserve_workspace(h, h->s_sliced, op_b + hist_b + order_b + place_b + bound_b + ids_b + dists_b + counts_b));
+    const uint64_t most_tiles = (n + kMmaRows - 1) / kMmaRows + 1;  // row tiles and the others are rounded up apart
+    const size_t op_b = up(size_t(most_tiles) * operand_bytes), codes_b = up(size_t(most_tiles) * kMmaRows * QUADS * 16);
+    const size_t places_b = up(size_t(most_tiles) * kMmaRows * 8), gates_b = up(size_t(most_tiles) * 16), n_b = up(size_t(n) * 4);
+    const size_t hist_b = up(size_t(kBoundOrders) * kKeys * 4), order_b = up(size_t(kBoundOrders) * n * 4);
+    const size_t before_b = hist_b + 2 * order_b;  // of use until the sweep begins, in the buffers' place
+    uint64_t block = wanted;
+    const bool wide = n > kPackedNodes - 1;  // (the last packed node stands for none)
+    const uint64_t most_hits = most_tiles * (most_tiles + 1) * 64;
+    const uint32_t hit_room = uint32_t(most_hits < kHitRoom ? most_hits : kHitRoom);
+    const size_t hits_b = size_t(hit_room) * 16;
+    size_t entries_b, counts_b, list_b;
+    while (true) {
+        const size_t slots = size_t((block + kMmaRows - 1) / kMmaRows) * kMmaRows;
+        entries_b = up(slots * kMmaCap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up((slots + 1) * 4);
+        const size_t buffers_b = entries_b > before_b ? entries_b : before_b;
+        const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + 256);
+        if (rc == 0) break;
+        if (rc != kNoRoom || entries_b <= before_b || block <= uint64_t(sms) * kMmaRows) return rc;
+        block = (block + 1) / 2;
+    }
     unsigned char* p = h->s_sliced.as<unsigned char>();
     auto take = [&](size_t b) {
         unsigned char* r = p;
@@ -886,93 +1345,183 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         return r;
     };
     uint4* operand = reinterpret_cast<uint4*>(take(op_b));
+    uint4* placed = reinterpret_cast<uint4*>(take(codes_b));
+    uint2* places = reinterpret_cast<uint2*>(take(places_b));
+    int16_t* gate = reinterpret_cast<int16_t*>(take(gates_b));
+    uint32_t* bound = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* group = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* mate = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* grouped = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* group_count = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* group_place = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* counts = reinterpret_cast<uint32_t*>(take(counts_b));
+    uint32_t* again = reinterpret_cast<uint32_t*>(take(list_b));
+    uint32_t* redo = reinterpret_cast<uint32_t*>(take(list_b));
+    uint4* hits = reinterpret_cast<uint4*>(take(hits_b));
+    struct Counters {
+        LoadCounts load;
+        uint32_t used, hits;
+    };
+    static_assert(sizeof(Counters) <= 256, "counters take 256 bytes");
+    Counters* counters = reinterpret_cast<Counters*>(take(256));
+    uint32_t* entries = reinterpret_cast<uint32_t*>(p);
     uint32_t* hist = reinterpret_cast<uint32_t*>(take(hist_b));
     uint32_t* order = reinterpret_cast<uint32_t*>(take(order_b));
-    uint32_t* place = reinterpret_cast<uint32_t*>(take(place_b));
-    uint32_t* bound = reinterpret_cast<uint32_t*>(take(bound_b));
+    uint32_t* place = reinterpret_cast<uint32_t*>(take(order_b));
 
     KnnMmaArgs a;
     a.operand = operand;
-    a.codes = reinterpret_cast<const uint4*>(padded);
-    const size_t code_bytes = size_t(kMmaRows) * QUADS * 16, own_bytes = QUADS <= 4 ? code_bytes : 0;
-    a.code_stages = 3 * operand_bytes + 4 * code_bytes + own_bytes <= kMmaSmem ? 4 : 2;  // even: a stage serves one side
+    a.codes = placed;
+    a.place = places;
+    a.gate = gate;
+    a.wide = wide;
     a.K = int(h->K);
     a.symbols = shape.symbols;
     a.chunks = shape.chunks;
-    a.n = n;
+    const uint32_t stage_bytes = uint32_t(shape.chunks / 2 + 1) / 2 * 2 * kMmaRows * 16;
+    a.stages = int((kMmaSmem - operand_bytes) / stage_bytes);
+    if (a.stages > kMaxStages) a.stages = kMaxStages;
     a.k = k;
-    a.row_begin = uint32_t(row_begin);
-    a.row_end = uint32_t(row_end);
-    a.bound = bound;
-    a.ids = reinterpret_cast<uint32_t*>(take(ids_b));
-    a.dists = reinterpret_cast<uint8_t*>(take(dists_b));
-    a.counts = reinterpret_cast<uint32_t*>(take(counts_b));
+    a.entries = entries;
+    a.counts = counts;
+    a.hits = hits;
+    a.hit_count = &counters->hits;
+    a.hit_room = hit_room;
     a.status = h->d_status.as<uint32_t>();
     a.first_wait_polls = h->first_wait_polls;
     a.handover_polls = h->handover_polls;
 
-    unsigned long long* load = reinterpret_cast<unsigned long long*>(hist + kBoundOrders * kKeys);
-    const uint64_t rows_wanted = row_end - row_begin;
     LoadArgs sample;
-    sample.groups = uint32_t((rows_wanted + 31) / 32 < kLoadGroups ? (rows_wanted + 31) / 32 : kLoadGroups);
-    sample.apart = rows_wanted / sample.groups < 32 ? 32 : rows_wanted / sample.groups;
-    a.choice = SweepChoice();
+    sample.groups = uint32_t((wanted + 31) / 32 < kLoadGroups ? (wanted + 31) / 32 : kLoadGroups);
+    sample.apart = wanted / sample.groups < 32 ? 32 : wanted / sample.groups;
+    const uint64_t node_tiles = (n + kMmaRows - 1) / kMmaRows;
     if (other) {
-        a.choice.load = load;
+        a.choice.load = &counters->load.turns;
         a.choice.most = (unsigned long long)(most_turns * sample.groups * kLoadTiles);
         *other = a.choice;
         other->above = true;
+        a.calm.counts = &counters->load;
+        a.calm.most_turns = (unsigned long long)(kCalmTurns * sample.groups * kLoadTiles);
+        a.calm.most = uint32_t(kCalmEntries * 32 * kLoadTiles * sample.groups / double(node_tiles));
     }
-    CPB_CUDA(cudaMemsetAsync(hist, 0, size_t(kBoundOrders) * kKeys * 4 + 8, st));
+    CPB_CUDA(cudaMemsetAsync(hist, 0, hist_b, st));
+    CPB_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), st));
     const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
     key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
     key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
     key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order, place);
-    auto bounds = [&](uint64_t count, uint64_t apart, const SweepChoice& choice) {
+    auto bounds = [&](uint64_t count, uint64_t apart, auto orders, auto window, const uint32_t* listed, const SweepChoice& choice) {
         auto go = [&](auto kernel) {
-            kernel<<<unsigned((count + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(a.codes, a.K, n, order, place, k, a.row_begin,
-                                                                                                  a.row_end, bound, apart, choice);
+            kernel<<<unsigned((count + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(rows, a.K, n, order, place, k, uint32_t(row_begin),
+                                                                                                  uint32_t(row_end), bound, group, mate, apart, listed, choice);
         };
-        if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) go(bound_kernel<U16, QUADS, (QUADS > 1)>);
-        else go(bound_kernel<U16, QUADS, false>);
+        constexpr int O = decltype(orders)::value, W = decltype(window)::value;
+        if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) go(bound_kernel<U16, QUADS, (QUADS > 1), O, W>);
+        else go(bound_kernel<U16, QUADS, false, O, W>);
         h->launches++;
     };
+    using All = std::integral_constant<int, kBoundOrders>;
+    using Full = std::integral_constant<int, kBoundWindow>;
     if (other) {
-        bounds(uint64_t(sample.groups) * 32, sample.apart, SweepChoice());
-        load_kernel<U16, QUADS><<<dim3(sample.groups, kLoadTiles), kMmaRows, 0, st>>>(a.codes, n, uint32_t(shape.symbols), uint32_t(tiles),
-                                                                                     a.row_begin, a.row_end, bound, sample, load);
+        bounds(uint64_t(sample.groups) * 32, sample.apart, All(), Full(), nullptr, SweepChoice());
+        load_kernel<U16, QUADS><<<dim3(sample.groups, kLoadTiles), kMmaRows, 0, st>>>(rows, n, uint32_t(shape.symbols), uint32_t(node_tiles),
+                                                                                     uint32_t(row_begin), uint32_t(row_end), bound, sample,
+                                                                                     &counters->load);
         h->launches++;
     }
-    bounds(n, 0, a.choice);
-    const uint64_t cells = tiles * shape.chunks * kMmaRows;
-    expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(codes, n, int(h->K), shape.symbols, shape.chunks, operand, tiles,
-                                                                             a.choice);
-    h->launches += 4;
+    const bool ordered = n >= kOrderNodes;
+    if (ordered) bounds(n, 0, std::integral_constant<int, kNameOrders>(), std::integral_constant<int, kNameWindow>(), nullptr, a.choice);
+    else bounds(n, 0, All(), std::integral_constant<int, kBoundWindow / 2>(), nullptr, a.choice);
+    const unsigned row_blocks = unsigned((wanted + 255) / 256);
+    for (int i = 0; i < (n > kOnePhase * 2 * kMmaRows ? 3 : 2) && ordered; ++i) group_join_kernel<<<row_blocks, 256, 0, st>>>(group, mate, uint32_t(row_begin), uint32_t(row_end), a.choice);
+    h->launches += ordered ? 6 : 3;
     CPB_CUDA(cudaGetLastError());
+    CPB_CUDA(allow_max_dynamic_smem(beside_kernel<U16, QUADS>));
     CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS>));
-    for (uint64_t t0 = first_tile; t0 < end_tile;) {
-        const uint64_t left = end_tile - t0;
-        const uint64_t rts = left >= kWaves * sms ? kWaves * sms : (left >= sms ? left / sms * sms : left);
-        a.tile0 = uint32_t(t0);
-        a.split.cts = uint32_t(tiles);
-        a.split.steps = rts * tiles;
-        a.split.blocks = uint32_t(a.split.steps < sms ? a.split.steps : sms);
-        // a block that gives up leaves its lengths unwritten; the rows it did not finish are then empty, not whatever the
-        // workspace held
-        CPB_CUDA(cudaMemsetAsync(a.counts, 0, size_t(a.split.blocks + rts) * kMmaRows * 2 * 4, st));
-        knn_mma_kernel<U16, QUADS><<<a.split.blocks, kMmaThreads, 3 * operand_bytes + a.code_stages * code_bytes + own_bytes, st>>>(a);
-        const uint32_t rows = uint32_t(rts) * kMmaRows;
-        knn_finish_kernel<<<(rows + kFinishWarps - 1) / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, rows, d_nbrs, d_dist, uint32_t(row_begin));
+    for (uint64_t begin = row_begin; begin < row_end; begin += block) {
+        const uint32_t rb = uint32_t(begin), re = uint32_t(row_end - begin < block ? row_end : begin + block), m = re - rb;
+        a.meet.row_tiles = (m + kMmaRows - 1) / kMmaRows;
+        a.meet.tiles = a.meet.row_tiles + uint32_t((n - m + kMmaRows - 1) / kMmaRows);
+        CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
+        CPB_CUDA(cudaMemsetAsync(redo, 0, 4, st));
+        // a block that gives up leaves rows without entries: they are then empty, not whatever the workspace held
+        CPB_CUDA(cudaMemsetAsync(counts, 0, size_t(a.meet.row_tiles) * kMmaRows * 4, st));
+        if (ordered) {
+            CPB_CUDA(cudaMemsetAsync(group_count, 0, size_t(n) * 4, st));
+            CPB_CUDA(cudaMemsetAsync(&counters->used, 0, 4, st));
+            group_count_kernel<<<(m + 255) / 256, 256, 0, st>>>(group, rb, re, group_count, a.choice);
+            group_place_kernel<<<unsigned((n + 255) / 256), 256, 0, st>>>(group_count, uint32_t(n), group_place, &counters->used, a.choice);
+            group_scatter_kernel<<<(m + 255) / 256, 256, 0, st>>>(group, rb, re, group_place, grouped, a.choice);
+            beside_kernel<U16, QUADS><<<(m + kBesideRows - 1) / kBesideRows, kBesideWarps * 32,
+                                        kBesidePlaces * QUADS * 16 + (a.K + 1) * kBesideWarps * 64, st>>>(rows, grouped, m, a.K, k, bound, again, a.choice);
+            // (the orders are still there for the first block of rows only)
+            if (rb == row_begin && n > kOnePhase * 2 * kMmaRows) bounds(uint64_t(sms) * 64, 0, All(), Full(), again, a.choice);
+            CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
+            h->launches += 4;
+        }
+        layout_kernel<QUADS><<<(a.meet.tiles * kMmaRows + kSortRows - 1) / kSortRows, kSortRows, 0, st>>>(
+            rows, uint32_t(n), rb, re, bound, group, a.K, a.symbols, a.meet, ordered ? grouped : nullptr, placed, places, gate, a.choice);
+        const uint64_t cells = uint64_t(a.meet.tiles) * shape.chunks * kMmaRows;
+        expand_codes_kernel<CompT><<<unsigned((cells + 255) / 256), 256, 0, st>>>(reinterpret_cast<const CompT*>(placed), QUADS * 16 / int(sizeof(CompT)),
+                                                                                 places, int(h->K), shape.symbols, shape.chunks, operand,
+                                                                                 a.meet.tiles, a.choice);
         h->launches += 2;
+        const uint32_t columns = a.meet.columns();
+        // a launch takes so many steps that its hits have room in the list
+        const uint32_t range = uint32_t(kLaunchSteps / a.meet.row_tiles) + 1;
+        auto sweep = [&](uint32_t count) {
+            const uint64_t steps = uint64_t(a.meet.row_tiles) * count;
+            CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
+            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, operand_bytes + a.stages * stage_bytes, st>>>(a);
+            knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
+            h->launches += 2;
+            return 0;
+        };
+        // near columns, among which a group's rows are
+        uint32_t near = 0;
+        if (a.meet.row_tiles / 2 + 1 >= kNearFrom) {
+            near = kNearColumns;
+            a.when = KnnMmaArgs::kAlways;
+            a.phase = Phase{0u, 1u, false, 0u, near};
+            CPB_TRY(sweep(near));
+            tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, again);
+            knn_again_kernel<U16, QUADS><<<dim3(2, 4 * sms), 256, 0, st>>>(a, again, near);
+            CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
+            h->launches += 2;
+        }
+        uint32_t stride = 1;
+        while (columns > kOnePhase && columns - near > kFirstColumns * stride) stride *= 2;
+        const bool one = a.calm.counts && columns - near <= range;  // (does on calm data)
+        for (bool whole = true; stride; stride /= 2, whole = false) {
+            a.phase = Phase{near, stride, !whole, 0u, 0u};
+            const uint32_t all = a.phase.columns(columns);
+            for (uint32_t from = 0; from < all; from += range) {
+                a.when = one ? (whole && from == 0 ? KnnMmaArgs::kAllIfCalm : KnnMmaArgs::kNotIfCalm) : KnnMmaArgs::kAlways;
+                a.phase.from = from, a.phase.count = all - from < range ? all - from : range;
+                CPB_TRY(sweep(a.when == KnnMmaArgs::kAllIfCalm ? columns - near : a.phase.count));
+            }
+            if (stride > 1) {
+                if (one) a.when = KnnMmaArgs::kNotIfCalm;
+                tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, nullptr);
+                h->launches++;
+            }
+        }
+        a.when = KnnMmaArgs::kAlways;
+        tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, true, again);
+        knn_again_kernel<U16, QUADS><<<dim3(16, sms), 256, 0, st>>>(a, again, 0u);
+        const uint32_t slots = a.meet.row_tiles * kMmaRows;
+        knn_finish_kernel<<<slots / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, slots, d_nbrs, d_dist, uint32_t(row_begin), redo);
+        knn_redo_kernel<U16, QUADS><<<sms, kRedoWarps * 32, 0, st>>>(rows, uint32_t(n), k, a.K, bound, redo, d_nbrs, d_dist, uint32_t(row_begin),
+                                                                        a.choice);
+        h->launches += 4;
         CPB_CUDA(cudaGetLastError());
-        t0 += rts;
     }
     return 0;
 }
 
 }  // namespace
 
-// Plain K-component codes of up to 64 components (the operand of 256 rows has to fit shared memory three times).
+// Plain K-component codes of up to 64 components (the operand of 256 rows has to fit shared memory twice).
 bool knn_mma_supported(const cphnsw_b200_index* h) {
     return !h->binary_codes && !h->residual_bits && h->K >= 2 && hash_shape(int(h->K)).symbols != 0;
 }

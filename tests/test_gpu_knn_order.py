@@ -1,0 +1,82 @@
+"""The kNN graph's tensor-core sweep that takes every pair once, in an order of groups, by phases (csrc/knn_mma.cu): sizes where
+its routes turn, against the byte-wise kernel, which knows none of them.  Both are exact, ties by id, so they agree in every entry."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cp():
+    import cphnsw_b200
+    return cphnsw_b200
+
+
+def mixture_codes(idx, n, dim, per, sigma, K, cb, seed):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    c = torch.randn((max(1, n // per), dim), generator=g, device="cuda")
+    x = c[torch.randint(0, len(c), (n,), generator=g, device="cuda")] + sigma * torch.randn((n, dim), generator=g, device="cuda")
+    x /= x.norm(dim=1, keepdim=True)
+    codes = torch.empty((n, K), dtype=torch.uint8 if cb == 1 else torch.int16, device="cuda")
+    idx.encode_dev(x.data_ptr(), n, codes.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    return codes
+
+
+def graph(idx, codes, k, rb, re):
+    import torch
+    nbrs = torch.empty((re - rb, k), dtype=torch.int32, device="cuda")
+    dist = torch.empty((re - rb, k), dtype=torch.int16, device="cuda")
+    idx.knn_graph_dev(codes.data_ptr(), codes.shape[0], k, rb, re, nbrs.data_ptr(), dist.data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    idx.check_device_status()
+    return nbrs, dist
+
+
+def agree(cp, idx, dim, K, cb, codes, k, rb, re):
+    import torch
+    plain = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
+    plain.set_param("knn_kernel", 1)
+    a, b = graph(idx, codes, k, rb, re), graph(plain, codes, k, rb, re)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+
+
+# 10,240 nodes: from here on in an order; 64 columns of tiles (32,512 nodes): near ones first; 296 row tiles: two whole waves and
+# none left over, an even number; 297: odd, one left over; a block of rows against all nodes; clusters far larger than what
+# lies beside a row (several phases); two-byte and four-symbol codes; no clusters at all, every buffer runs over
+@pytest.mark.parametrize("n,k,dim,K,cb,per,sigma,rows", [
+    (10239, 64, 128, 32, 1, 1000, 0.3, None), (10240, 64, 128, 32, 1, 1000, 0.3, None), (10241, 1, 128, 32, 1, 1000, 0.3, None),
+    (32256, 64, 96, 32, 1, 1000, 0.3, None), (32512, 127, 128, 32, 1, 1000, 0.3, None), (75776, 64, 128, 16, 1, 1000, 0.3, None),
+    (75777, 32, 64, 32, 1, 1000, 0.3, None), (40001, 64, 128, 32, 1, 1000, 0.3, (5003, 29007)), (36000, 64, 128, 32, 1, 18000, 0.3, None),
+    (20001, 64, 300, 32, 2, 1000, 0.4, None), (33001, 64, 128, 64, 1, 500, 0.4, (0, 33000)), (12000, 64, 128, 32, 1, 1, 0.3, None),
+    (34000, 20, 64, 10, 1, 1000, 0.3, None)])
+@pytest.mark.parametrize("kernel", [0, 3])
+def test_routes(cp, n, k, dim, K, cb, per, sigma, rows, kernel):
+    idx = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
+    codes = mixture_codes(idx, n, dim, per, sigma, K, cb, n + k)
+    idx.set_param("knn_kernel", kernel)
+    agree(cp, idx, dim, K, cb, codes, k, *(rows or (0, n)))
+
+
+# thousands of equal codes: their rows' buffers run over twice, and the row is compared with every node
+@pytest.mark.parametrize("n,equal", [(11000, 700), (34000, 3000)])
+def test_equal_codes(cp, n, equal):
+    import torch
+    idx = cp.CPHNSWIndex(128, K=32)
+    codes = mixture_codes(idx, n, 128, 1000, 0.3, 32, 1, n)
+    codes[torch.randperm(n, device="cuda")[:equal]] = codes[0].clone()
+    idx.set_param("knn_kernel", 3)
+    agree(cp, idx, 128, 32, 1, codes, 64, 0, n)
+
+
+def test_rows_in_blocks_where_the_workspace_is_small(cp):
+    # 60,000 rows: 169 MB with all rows' buffers at once, 122 in two blocks
+    idx = cp.CPHNSWIndex(128, K=32)
+    codes = mixture_codes(idx, 60000, 128, 1000, 0.3, 32, 1, 5)
+    idx.set_param("knn_kernel", 3)
+    idx.set_param("workspace_limit_mb", 130)
+    agree(cp, idx, 128, 32, 1, codes, 64, 0, 60000)
+    idx.set_param("workspace_limit_mb", 20)
+    with pytest.raises(cp.CPHNSWError):
+        graph(idx, codes, 64, 0, 60000)
