@@ -3,8 +3,8 @@
 // Same result as exact_topk_kernel: the k smallest (-<q,x>, id), the dot product accumulated in fp32 in d order without
 // fused multiply-add.  Two fp32 operations per pair and dimension bound that kernel; here every pair costs a tensor
 // product in fp16 and only a few hundred candidates per query are computed exactly:
-//   * base and queries are scaled by powers of two (the base as a whole, every query by itself) so that no coordinate
-//     exceeds 1 and rounded to fp16;
+//   * base and queries are scaled by powers of two (the base by tiles of 256 vectors, every query by itself) so that no
+//     coordinate exceeds 1 and rounded to fp16; the sweep brings the products of a tile to the scale of the whole base;
 //   * a sweep over all pairs keeps, per query, the largest product of every group of 32 base vectors;
 //     (the last group, when the base ends inside it, is computed exactly in any case)
 //   * with A the k-th largest of a query's group maxima and m a bound on the error of a product, k vectors have an exact
@@ -37,14 +37,21 @@ constexpr uint32_t kPickGroups = 1024;     // groups a query may list
 constexpr uint32_t kPickKeys = 1024;       // candidates a query may sort
 constexpr int kPickThreads = 256;
 
+// A power of two that brings the largest coordinate, given by its bits, to at most 1; 0: not to be searched here.
+__device__ __forceinline__ float scale_of(uint32_t big) {
+    const int e = int(big >> 23);
+    if (big == 0) return 1.0f;
+    return e >= 64 && e <= 190 ? __uint_as_float(uint32_t(253 - e) << 23) : 0.0f;
+}
+// the base's scale, from its largest coordinate in stat[0]
+__device__ __forceinline__ float base_scale(const uint32_t* stat) { return scale_of(stat[0]); }
+
 // ---- norms and largest coordinates: one warp per row -------------------------------------------------------------------
-// stat[0]: bits of the largest |coordinate|, stat[1]: bits of the largest norm (both non-negative floats, which order as
-// integers; a number that is not finite shows as 0x7f800000 and above).  per_row: {scale, scaled norm} of every row.
-__global__ void row_stats_kernel(const float* __restrict__ x, uint64_t n, int dim, uint32_t* __restrict__ stat, float2* __restrict__ per_row) {
+// per_row: {scale, scaled norm} of every query.
+__global__ void row_stats_kernel(const float* __restrict__ x, uint64_t n, int dim, float2* __restrict__ per_row) {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = uint64_t(gridDim.x) * (blockDim.x >> 5);
     const bool vec4 = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;  // (dim <= 128: a load per lane)
-    uint32_t top = 0, norm = 0;
 #pragma unroll 4
     for (uint64_t row = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; row < n; row += warps) {
         float sum = 0.0f;
@@ -67,39 +74,23 @@ __global__ void row_stats_kernel(const float* __restrict__ x, uint64_t n, int di
         for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
         big = __reduce_max_sync(kFull, big);
         const float len = sqrtf(sum) * 1.0001f;
-        top = max(top, big);
-        norm = max(norm, __float_as_uint(len) & 0x7fffffffu);
-        if (per_row && lane == 0) {
-            // a power of two that brings the largest coordinate to at most 1 (0: not to be searched here)
-            const int e = int(big >> 23);
-            const bool fine = big == 0 || (e >= 64 && e <= 190);
-            const float scale = big == 0 ? 1.0f : __uint_as_float(uint32_t(253 - e) << 23);
-            per_row[row] = make_float2(fine ? scale : 0.0f, len * scale);
+        if (lane == 0) {
+            const float scale = scale_of(big);
+            per_row[row] = make_float2(scale, len * scale);
         }
     }
-    if (stat && lane == 0) {
-        atomicMax(stat, top);
-        atomicMax(stat + 1, norm);
-    }
-}
-// the base's scale: 0 when it cannot be searched here
-__device__ __forceinline__ float base_scale(const uint32_t* stat) {
-    const uint32_t big = stat[0];
-    const int e = int(big >> 23);
-    if (big == 0) return 1.0f;
-    return e >= 64 && e <= 190 ? __uint_as_float(uint32_t(253 - e) << 23) : 0.0f;
 }
 
 // ---- operand: [tile of 256 rows][chunk][row][8 halves] ------------------------------------------------------------------
-__global__ void to_half_kernel(const float* __restrict__ x, uint64_t n, int dim, int chunks, const uint32_t* __restrict__ stat,
-                               const float2* __restrict__ per_row, uint4* __restrict__ out, uint64_t tiles) {
+__global__ void to_half_kernel(const float* __restrict__ x, uint64_t n, int dim, int chunks, const float2* __restrict__ per_row,
+                               uint4* __restrict__ out, uint64_t tiles) {
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t row = t / chunks;
     const int c = int(t % chunks);
     if (row >= tiles * kMmaRows) return;
     uint4 w = make_uint4(0u, 0u, 0u, 0u);
     if (row < n) {
-        const float s = per_row ? per_row[row].x : base_scale(stat);
+        const float s = per_row[row].x;
         __half2 h[4];
         const float* src = x + row * dim + c * 8;
         if ((dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
@@ -121,6 +112,80 @@ __global__ void to_half_kernel(const float* __restrict__ x, uint64_t n, int dim,
                        *reinterpret_cast<uint32_t*>(&h[3]));
     }
     out[(row / kMmaRows * chunks + c) * kMmaRows + row % kMmaRows] = w;
+}
+
+// A tile of the base in one pass: its vectors in registers, 16 to a warp and four coordinates to a lane, their largest
+// coordinate and norm, then the halves at the tile's own scale, chunk by chunk through shared memory (a chunk's rows 16
+// bytes further apart in the banks than 4 KB) as contiguous copies.  What bounds it is the base's bytes: 500k x 128 are read
+// once, 77 us (5.0 TB/s); with a pass for the statistics before the conversion 121.
+// stat[0]: bits of the base's largest |coordinate|, stat[1]: bits of its largest norm (both non-negative floats, which order
+// as integers; a number that is not finite shows as 0x7f800000 and above).
+constexpr int kTileWarps = 16, kTileRows = kMmaRows / kTileWarps;
+constexpr uint32_t kChunkStride = kMmaRows * 16 + 16;
+__global__ void __launch_bounds__(kTileWarps * 32) base_tile_kernel(const float* __restrict__ x, uint64_t n, int dim, int chunks,
+                                                                    uint32_t* __restrict__ stat, float* __restrict__ tile_scale,
+                                                                    unsigned char* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char tile_smem[];
+    __shared__ uint32_t top, longest;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t row0 = uint64_t(blockIdx.x) * kMmaRows + warp * kTileRows;
+    const bool vec4 = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    if (threadIdx.x == 0) top = longest = 0;
+    __syncthreads();
+    float4 v[kTileRows];
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) {
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + i < n) {
+            const float* src = x + (row0 + i) * dim + 4 * lane;
+            if (vec4) {
+                if (4 * lane < dim) v[i] = __ldg(reinterpret_cast<const float4*>(src));
+            } else {
+                if (4 * lane < dim) v[i].x = __ldg(src);
+                if (4 * lane + 1 < dim) v[i].y = __ldg(src + 1);
+                if (4 * lane + 2 < dim) v[i].z = __ldg(src + 2);
+                if (4 * lane + 3 < dim) v[i].w = __ldg(src + 3);
+            }
+        }
+    }
+    uint32_t big = 0;
+    float most = 0.0f;  // of the squared norms
+    bool odd = false;   // one of them is not a number
+#pragma unroll
+    for (int i = 0; i < kTileRows; ++i) {
+        big = max(big, max(max(__float_as_uint(v[i].x) & 0x7fffffffu, __float_as_uint(v[i].y) & 0x7fffffffu),
+                           max(__float_as_uint(v[i].z) & 0x7fffffffu, __float_as_uint(v[i].w) & 0x7fffffffu)));
+        float sum = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+        odd = odd || !(sum >= 0.0f);
+        most = fmaxf(most, sum);
+    }
+    big = __reduce_max_sync(kFull, big);
+    if (lane == 0) {
+        atomicMax(&top, big);
+        atomicMax(&longest, odd ? 0x7fffffffu : __float_as_uint(sqrtf(most) * 1.0001f));
+    }
+    __syncthreads();
+    // (a tile that cannot be searched keeps the others from it too, by stat)
+    const float s = scale_of(top);
+    if (threadIdx.x == 0) {
+        atomicMax(stat, top);
+        atomicMax(stat + 1, longest);
+        tile_scale[blockIdx.x] = s;
+    }
+    if (lane < chunks * 2) {
+#pragma unroll
+        for (int i = 0; i < kTileRows; ++i) {
+            const __half2 a = __floats2half2_rn(v[i].x * s, v[i].y * s), b = __floats2half2_rn(v[i].z * s, v[i].w * s);
+            *reinterpret_cast<uint2*>(tile_smem + (lane >> 1) * kChunkStride + (warp * kTileRows + i) * 16 + (lane & 1) * 8) =
+                make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        }
+    }
+    __syncthreads();
+    uint4* dst = reinterpret_cast<uint4*>(out + size_t(blockIdx.x) * chunks * kMmaRows * 16);
+    for (int i = threadIdx.x; i < chunks * kMmaRows; i += kTileWarps * 32)
+        dst[i] = *reinterpret_cast<const uint4*>(tile_smem + (i / kMmaRows) * kChunkStride + (i % kMmaRows) * 16);
 }
 
 // ---- sweep ----------------------------------------------------------------------------------------------------------------
@@ -164,6 +229,8 @@ __device__ __forceinline__ float max16(const float (&r)[16]) {
 struct SweepArgs {
     const uint4* queries;  // [tiles of 256 queries][chunks][256]
     const uint4* base;     // [tiles][chunks][256]
+    const float* tile_scale;
+    const uint32_t* stat;
     int chunks;
     uint64_t n;
     uint32_t nq, groups;   // groups: maxima per query (8 per tile)
@@ -259,10 +326,12 @@ __global__ void __launch_bounds__(kXmThreads, 1) exact_sweep_kernel(SweepArgs a)
         const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
         const uint32_t local = uint32_t(half * 128 + quarter * 32 + lane), n = uint32_t(a.n);
         const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256;
+        const float whole = base_scale(a.stat);
         bool ok = true;
         for (uint32_t i = side; i < steps; i += 2) {
             const uint64_t step = s0 + i;
             const uint32_t q = uint32_t(step / a.split.cts) * kMmaRows + local, ct = uint32_t(step % a.split.cts);
+            const float tile = __ldg(a.tile_scale + ct), to_whole = tile > 0.0f ? whole / tile : 0.0f;  // (powers of two)
             ok = wait_or_abort(&tfull_bar[half][side], (i >> 1) & 1, kWaitLimit, aborted);
             if (__ballot_sync(kFull, !ok || *aborted)) {
                 ok = false;
@@ -278,7 +347,7 @@ __global__ void __launch_bounds__(kXmThreads, 1) exact_sweep_kernel(SweepArgs a)
                 float m = max16(r0);
                 tmem_waitf(r1);
                 if (g < 7) tmem_load16f(r0, addr + g * 32 + 32);
-                out[g] = fmaxf(m, max16(r1));
+                out[g] = fmaxf(m, max16(r1)) * to_whole;
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -513,34 +582,37 @@ int launch_exact_mma(cphnsw_b200_index* h, const float* d_base, uint64_t n, cons
     const uint64_t qtiles = (batch + kMmaRows - 1) / kMmaRows;
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t base_b = up(size_t(tiles) * operand_bytes), q_b = up(size_t(qtiles) * operand_bytes);
-    const size_t max_b = up(size_t(batch) * groups * 4), row_b = up(size_t(batch) * 8);
-    CPB_TRY(reserve_workspace(h, h->s_exact, 256 + base_b + q_b + max_b + row_b));
+    const size_t max_b = up(size_t(batch) * groups * 4), row_b = up(size_t(batch) * 8), scale_b = up(size_t(tiles) * 4);
+    CPB_TRY(reserve_workspace(h, h->s_exact, 256 + base_b + q_b + max_b + row_b + scale_b));
     unsigned char* p = h->s_exact.as<unsigned char>();
     uint32_t* stat = reinterpret_cast<uint32_t*>(p);
     uint4* base_op = reinterpret_cast<uint4*>(p + 256);
     uint4* q_op = reinterpret_cast<uint4*>(p + 256 + base_b);
     float* maxima = reinterpret_cast<float*>(p + 256 + base_b + q_b);
     float2* per_query = reinterpret_cast<float2*>(p + 256 + base_b + q_b + max_b);
+    float* tile_scale = reinterpret_cast<float*>(p + 256 + base_b + q_b + max_b + row_b);
 
     uint32_t* status = stat + 2;
     CPB_CUDA(cudaMemsetAsync(stat, 0, 12, st));
     const unsigned stat_blocks = unsigned(h->sm_count) * 8;
-    row_stats_kernel<<<stat_blocks, 256, 0, st>>>(d_base, n, dim, stat, nullptr);
-    const uint64_t cells = tiles * kMmaRows * chunks;
-    to_half_kernel<<<unsigned((cells + 255) / 256), 256, 0, st>>>(d_base, n, dim, chunks, stat, nullptr, base_op, tiles);
-    h->launches += 2;
+    CPB_CUDA(allow_max_dynamic_smem(base_tile_kernel));
+    base_tile_kernel<<<unsigned(tiles), kTileWarps * 32, chunks * kChunkStride, st>>>(d_base, n, dim, chunks, stat, tile_scale,
+                                                                                     reinterpret_cast<unsigned char*>(base_op));
+    h->launches++;
     CPB_CUDA(cudaGetLastError());
     CPB_CUDA(allow_max_dynamic_smem(exact_sweep_kernel));
     for (uint64_t q0 = 0; q0 < nq; q0 += batch) {
         const uint64_t m = nq - q0 < batch ? nq - q0 : batch;
         const uint64_t rts = (m + kMmaRows - 1) / kMmaRows;
         const float* qs = d_q + q0 * dim;
-        row_stats_kernel<<<unsigned((m + 7) / 8 < stat_blocks ? (m + 7) / 8 : stat_blocks), 256, 0, st>>>(qs, m, dim, nullptr, per_query);
+        row_stats_kernel<<<unsigned((m + 7) / 8 < stat_blocks ? (m + 7) / 8 : stat_blocks), 256, 0, st>>>(qs, m, dim, per_query);
         const uint64_t q_cells = rts * kMmaRows * chunks;
-        to_half_kernel<<<unsigned((q_cells + 255) / 256), 256, 0, st>>>(qs, m, dim, chunks, nullptr, per_query, q_op, rts);
+        to_half_kernel<<<unsigned((q_cells + 255) / 256), 256, 0, st>>>(qs, m, dim, chunks, per_query, q_op, rts);
         SweepArgs a;
         a.queries = q_op;
         a.base = base_op;
+        a.tile_scale = tile_scale;
+        a.stat = stat;
         a.chunks = chunks;
         a.n = n;
         a.nq = uint32_t(m);
