@@ -628,14 +628,15 @@ def run_b200(args):
         "knn_graph": None, "select_neighbors": None}
     if 2 <= K <= 64 and n >= 4096:
         # tensor-core filter: a component is 7 values of +-1 at K <= 32 and 3 above, rows padded to a multiple of 32
-        # values; every pair costs two operations a value
+        # values; a pair costs two operations a value, once where both its rows are of one GPU
         values = (K * (7 if K <= 32 else 3) + 31) // 32 * 32
         fp8, fp8_kind = measured_fp8_peak()
         fp8 *= world
-        roofline_build["knn_graph"] = {"bound": "fp8 tensor pipe and its epilogue", "achieved": build["knn_pairs_per_s"] * 2 * values, "peak": fp8,
-                                       "unit": "op/s", "frac": build["knn_pairs_per_s"] * 2 * values / fp8,
-                                       "note": "%d values per pair, every unordered pair twice; peak is %s; ncu sm__pipe_tensor_cycles_active "
-                                               "62 %% of the sweep on C2 at 1/4 size (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp8_kind)}
+        products = build["knn_pairs_per_s"] * (1.0 - 0.5 / world) * 2 * values
+        roofline_build["knn_graph"] = {"bound": "fp8 tensor pipe and its epilogue", "achieved": products, "peak": fp8,
+                                       "unit": "op/s", "frac": products / fp8,
+                                       "note": "%d values per pair, an unordered pair once on a GPU that has both rows; peak is %s; the whole stage, "
+                                               "bounds and order included (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp8_kind)}
     sel_bytes = n * (knn_k * 4 + knn_k * code_row + M * 4.0)
     roofline_build["select_neighbors"] = {"bound": "hbm gather", "achieved": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9, "peak": peak * world,
                                           "unit": "GB/s", "frac": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9 / (peak * world),
