@@ -112,6 +112,18 @@ __device__ __forceinline__ float asym_distance_lane(const float* table, const vo
     return -acc;
 }
 
+// Differing components among 16 bytes of two codes: a flag in the top bit of every component that differs, the flags of the
+// four words side by side for one population count (which issues at a quarter of the rate of the rest).  Read by words, 32
+// rows of 32 bytes took 64 wavefronts of the L1; 4,096 probes of multiprobe search on 200k x 128: 500 us, 464 so.
+template <bool U16>
+__device__ __forceinline__ uint32_t quad_mismatches(uint4 x, uint32_t q0, uint32_t q1, uint32_t q2, uint32_t q3) {
+    constexpr uint32_t LO = U16 ? 0x7fff7fffu : 0x7f7f7f7fu;
+    x.x ^= q0, x.y ^= q1, x.z ^= q2, x.w ^= q3;
+    const uint32_t f0 = (((x.x & LO) + LO) | x.x) & ~LO, f1 = (((x.y & LO) + LO) | x.y) & ~LO;
+    const uint32_t f2 = (((x.z & LO) + LO) | x.z) & ~LO, f3 = (((x.w & LO) + LO) | x.w) & ~LO;
+    return __popc(f0 | f1 >> 1 | f2 >> 2 | f3 >> 3);
+}
+
 // Symmetric metric (search_multiprobe): number of components in which the node's code differs
 // from the query code staged in shared memory, as a float.
 template <bool U16>
@@ -124,7 +136,11 @@ __device__ __forceinline__ float sym_distance_lane(const unsigned char* qcode, c
         constexpr uint32_t LO = U16 ? 0x7fff7fffu : 0x7f7f7f7fu;
         const uint32_t* r32 = reinterpret_cast<const uint32_t*>(row);
         const uint32_t* q32 = reinterpret_cast<const uint32_t*>(qcode);
-        if (!mul) {
+        if (!mul && (row_bytes & 15) == 0) {  // (rows lie on 16 bytes then, as score_asym takes them)
+            const uint4* r4 = reinterpret_cast<const uint4*>(row);
+            for (int w = 0; w < row_bytes / 16; ++w)
+                d += quad_mismatches<U16>(__ldg(r4 + w), q32[4 * w], q32[4 * w + 1], q32[4 * w + 2], q32[4 * w + 3]);
+        } else if (!mul) {
             for (int w = 0; w < row_bytes / 4; ++w) {
                 const uint32_t x = q32[w] ^ __ldg(r32 + w);
                 d += __popc((((x & LO) + LO) | x) & ~LO);  // one flag per differing byte / halfword

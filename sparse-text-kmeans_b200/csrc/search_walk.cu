@@ -468,6 +468,23 @@ entry_scan_kernel(ScanArgs a) {
             }
 #pragma unroll
             for (int g = 0; g < QG; ++g) d[g] = -d[g];
+        } else if (METRIC == kSymBytes && (a.row_bytes & 15) == 0 && !a.resid_mul) {
+            // an entry's code is read once for all queries of the block
+            uint32_t differ[QG];
+#pragma unroll
+            for (int g = 0; g < QG; ++g) differ[g] = 0;
+            const uint4* row = reinterpret_cast<const uint4*>(a.entry_scan + size_t(ee) * a.row_bytes);
+            const uint4* codes = reinterpret_cast<const uint4*>(scan_smem);  // a row apart
+            for (int w = 0; w < a.row_bytes / 16; ++w) {
+                const uint4 x = __ldg(row + w);
+#pragma unroll
+                for (int g = 0; g < QG; ++g) {
+                    const uint4 c = codes[g * (a.row_bytes / 16) + w];
+                    differ[g] += quad_mismatches<U16>(x, c.x, c.y, c.z, c.w);
+                }
+            }
+#pragma unroll
+            for (int g = 0; g < QG; ++g) d[g] = float(differ[g]);
         } else {
 #pragma unroll
             for (int g = 0; g < QG; ++g) {
