@@ -45,6 +45,9 @@ __device__ __forceinline__ float scale_of(uint32_t big) {
 }
 // the base's scale, from its largest coordinate in stat[0]
 __device__ __forceinline__ float base_scale(const uint32_t* stat) { return scale_of(stat[0]); }
+// A tile's scale: 2^62, that of the smallest base that is searched, where all its coordinates are smaller still or zero (they
+// stay below 1/2, and products at 2^62 are brought to the base's scale, 2^62 or less, like any others').
+__device__ __forceinline__ float tile_scale_of(uint32_t big) { return scale_of(max(big, 64u << 23)); }
 
 // ---- norms and largest coordinates: one warp per row -------------------------------------------------------------------
 // per_row: {scale, scaled norm} of every query.
@@ -167,8 +170,8 @@ __global__ void __launch_bounds__(kTileWarps * 32) base_tile_kernel(const float*
         atomicMax(&longest, odd ? 0x7fffffffu : __float_as_uint(sqrtf(most) * 1.0001f));
     }
     __syncthreads();
-    // (a tile that cannot be searched keeps the others from it too, by stat)
-    const float s = scale_of(top);
+    // (a tile whose coordinates are too large has scale 0 and keeps the whole base from being searched here, by stat)
+    const float s = tile_scale_of(top);
     if (threadIdx.x == 0) {
         atomicMax(stat, top);
         atomicMax(stat + 1, longest);

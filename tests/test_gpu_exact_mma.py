@@ -94,6 +94,22 @@ def test_awkward_values(cp, kind):
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd, equal_nan=True)
 
 
+# tiles of 256 vectors below the smallest coordinate that is searched (2^-63) in a base that is: the larger vectors, one in every
+# second tile, are far from the queries, so all neighbours are in coordinates that count as much as theirs
+@pytest.mark.parametrize("k", [1, 10])
+@pytest.mark.parametrize("tops", [(-62.0,), (-62.0, -64.0, -70.0), (-60.0, -63.5)])
+def test_tiles_on_both_sides_of_the_smallest_coordinate(cp, k, tops):
+    rng = np.random.default_rng(11)
+    n, nq, dim = 20000, 70, 32
+    base = (rng.uniform(-1, 1, (n, dim)) * 2.0 ** -63.2).astype(np.float32)
+    q = np.abs(rng.standard_normal((nq, dim))).astype(np.float32)
+    for i, row in enumerate(range(100, n, 512)):
+        base[row, i % dim] = -2.0 ** tops[i % len(tops)]
+    _, (ids, dist) = exact(cp, base, q, k)
+    wi, wd = cpu(base, q, k)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
 def test_lost_wait_costs_no_result(cp):
     # the sweep's first wait gets no polls: every query is answered the plain way, and nothing is left behind that a later
     # call on the handle would report as its own
