@@ -1314,7 +1314,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const uint32_t operand_bytes = uint32_t(shape.chunks) * kMmaRows * 16;
     const uint32_t sms = uint32_t(h->sm_count);
     const uint64_t wanted = row_end - row_begin;
-    if (n > (1u << 27) - 2 * kMmaRows) return kNoRoom;  // (a collected pair has 27 bits for a place)
+    // (places are words of 32 bits, rounded up by tiles; at 144 bytes a node and more no GPU this runs on has room for as many)
+    if (n > uint64_t(1) << 31) return kNoRoom;
 
     // Workspace.  The buffers of the rows found take 1.9 KB a wanted row: where they do not fit, the rows go in blocks.
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };

@@ -80,3 +80,29 @@ def test_rows_in_blocks_where_the_workspace_is_small(cp):
     idx.set_param("workspace_limit_mb", 20)
     with pytest.raises(cp.CPHNSWError):
         graph(idx, codes, 64, 0, 60000)
+
+
+# entries of a row's buffer are one word up to 2^25 - 1 nodes and two above; nodes behind 2^27 are served like the others.  The wanted
+# rows are the last 600, in six clusters whose other members lie anywhere, and 30 of them in none
+@pytest.mark.parametrize("n", [(1 << 25) - 1, 1 << 25, (1 << 27) + 301])
+def test_many_nodes(cp, n):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    K, rows, k = 16, 600, 20
+    codes = torch.empty((n, K), dtype=torch.uint8, device="cuda")
+    for i in range(0, n, 1 << 24):
+        codes[i:i + (1 << 24)] = torch.randint(0, 256, (min(n - i, 1 << 24), K), generator=g, device="cuda", dtype=torch.uint8)
+    centres = torch.randint(0, 256, (6, K), generator=g, device="cuda", dtype=torch.uint8)
+
+    def member(c, m):
+        own = torch.rand((m, K), generator=g, device="cuda") < 0.25
+        return torch.where(own, torch.randint(0, 256, (m, K), generator=g, device="cuda", dtype=torch.uint8), centres[c])
+
+    for c in range(6):
+        codes[n - rows + 100 * c:n - rows + 100 * c + 95] = member(c, 95)
+        codes[torch.randint(0, n - rows, (40,), generator=g, device="cuda")] = member(c, 40)
+    idx = cp.CPHNSWIndex(64, K=K)
+    idx.set_param("knn_kernel", 3)
+    agree(cp, idx, 64, K, 1, codes, k, n - rows, n)
+    idx.close()
