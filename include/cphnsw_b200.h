@@ -130,9 +130,10 @@ int cphnsw_b200_destroy(cphnsw_b200_index* h);
  *                 (the same range and default, for the waits inside a tensor-core kNN launch for a stage to be handed back),
  *   "workspace_limit_mb" (default 0 = no limit: the most MiB of device memory a tensor-core filter's workspace may take.
  *                 A kNN graph's is about 300 bytes a node, 1.6 KB a row wanted and up to 64 MB - rows go in blocks where
- *                 that is too much -, an exact search's 2 bytes a base coordinate plus up to 0.5 GB; both stay with the
- *                 handle.  Above the limit, and when the device has no memory for it, the kernels without a filter answer,
- *                 with the same results),
+ *                 that is too much -, an exact search's 2 bytes a base coordinate plus up to 0.5 GB.  Both stay with the
+ *                 handle, a graph's above 2 GiB only until the build or the knn_graph call ends, or, after knn_graph_dev,
+ *                 until the next build or install.  Above the limit, and when the device has no memory for it, the kernels
+ *                 without a filter answer, with the same results),
  *   "entry_scan" (evenly spaced nodes scored for every query before the walk; default = k_entry),
  *   "k_entry" (1..100, default 4: how many of the scored nodes, the best, seed the walk). */
 int cphnsw_b200_set_param(cphnsw_b200_index* h, const char* name, double value);

@@ -123,7 +123,17 @@ int check_status(cphnsw_b200_index* h) {
 
 size_t code_row_bytes(const cphnsw_b200_index* h) { return size_t(h->K) * h->comp_bytes; }
 
+// A kNN graph's workspace (1.8 KB a node) does not stay with the handle above this size: a search has no use for it, and an
+// index of 10M nodes would hold 18 GB.  Giving back 2 GiB and asking again takes 1.4 and 0.8 ms, 16 GiB 10 and 2.6; the graph
+// that fills 2 GiB 90 ms, and a graph's time grows with the square.  (Waits for the device; graphs enqueued by
+// knn_graph_dev, which must not wait, leave theirs to the next call that installs or builds.)
+constexpr size_t kGraphKept = size_t(2) << 30;
+void give_back_graph_workspace(cphnsw_b200_index* h) {
+    if (h->s_sliced.bytes > kGraphKept) h->s_sliced.release();
+}
+
 int set_entry_ids(cphnsw_b200_index* h) {
+    give_back_graph_workspace(h);
     uint64_t s = h->entry_scan ? h->entry_scan : h->k_entry;
     if (s > h->n) s = h->n;
     std::vector<uint32_t> ids(s);
@@ -193,6 +203,7 @@ int build_graph(cphnsw_b200_index* h, uint64_t n, DevBuf& adj, cudaStream_t st) 
     }
     CPB_TRY(h->s_out.reserve(size_t(n) * k * 4 + 16));
     CPB_TRY(launch_knn_graph(h, h->d_codes.p, n, k, 0, n, h->s_out.as<uint32_t>(), nullptr, st));
+    give_back_graph_workspace(h);  // (before the memory that pruning and the entry tables need)
     if (h->rank_prune)
         CPB_TRY(launch_rank_prune(h, n, h->s_out.as<uint32_t>(), k, h->M, h->rank_pruning_alpha, adj.as<uint32_t>(), st));
     else
@@ -1313,6 +1324,7 @@ int cphnsw_b200_knn_graph(cphnsw_b200_index* h, const void* codes, uint64_t n, u
                              dist_out ? h->s_out2.as<uint16_t>() : nullptr, 0));
     CPB_CUDA(cudaMemcpy(nbrs_out, h->s_out.p, rows * k * 4, cudaMemcpyDeviceToHost));
     if (dist_out) CPB_CUDA(cudaMemcpy(dist_out, h->s_out2.p, rows * k * 2, cudaMemcpyDeviceToHost));
+    give_back_graph_workspace(h);
     return check_status(h);
 }
 

@@ -60,3 +60,35 @@ def test_handles_of_several_threads(cp):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors
+
+
+def test_a_large_graph_workspace_does_not_stay_with_the_index(cp):
+    # 1.3M nodes: 2.2 GB of buffers for the kNN graph, which the index has no use for once it is searched
+    import torch
+    use(cp, 1000).close()
+    cp.release_memory()
+    rng = np.random.default_rng(3)
+    n, dim = 1_300_000, 32
+    base = (rng.standard_normal((1300, dim)).repeat(1000, 0) + 0.1 * rng.standard_normal((n, dim))).astype(np.float32)
+    before = free_mb()
+    idx = cp.CPHNSWIndex(dim, M=8, K=16)
+    idx.add_batch_parallel(base)
+    held = before - free_mb()  # vectors 160, links 40, candidates 80, codes 20; 1,024 at most are kept for other buffers
+    assert held <= 1024 + 512
+    # by the stages on device arrays: they enqueue only, so the workspace goes when the index is installed
+    x = torch.from_numpy(base).cuda()
+    codes = torch.empty((n, 16), dtype=torch.uint8, device="cuda")
+    cand = torch.empty((n, 16), dtype=torch.int32, device="cuda")
+    idx.close()
+    cp.release_memory()
+    before = free_mb()
+    idx = cp.CPHNSWIndex(dim, M=8, K=16)
+    st = torch.cuda.current_stream().cuda_stream
+    idx.encode_dev(x.data_ptr(), n, codes.data_ptr(), stream=st)
+    idx.knn_graph_dev(codes.data_ptr(), n, 16, 0, n, cand.data_ptr(), stream=st)
+    assert before - free_mb() > 2000
+    adj = cand[:, :8].contiguous()
+    idx.install_dev(x.data_ptr(), codes.data_ptr(), adj.data_ptr(), n, stream=st)
+    assert before - free_mb() <= 1024 + 512
+    idx.close()
+    cp.release_memory()
