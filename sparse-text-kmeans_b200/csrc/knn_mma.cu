@@ -54,10 +54,11 @@ using knn::mbar_wait_bounded;
 using knn::smem_u32;
 using namespace mma;
 
-constexpr uint32_t kMmaCap = 384;         // entries of a row's buffer
+constexpr uint32_t kMmaCap = 384;         // entries of a row's buffer, where there is more than one phase
 constexpr int kMmaSlots = kMmaCap / 32;   // of them per lane
 constexpr uint32_t kMmaKeep = 128;        // entries that are left of one that is cut
 constexpr uint32_t kMmaFull = 256;        // entries from which on it is cut between phases
+constexpr size_t kLongBuffers = size_t(128) << 20;  // bytes of the buffers of a graph of one phase, at most, if they are longer
 constexpr int kBatch = 4;                 // rows compared with 32 columns at a time
 constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in the list of hits
 constexpr uint64_t kLaunchSteps = 1u << 22;
@@ -574,8 +575,9 @@ struct KnnMmaArgs {
     Phase phase;
     enum { kAlways, kAllIfCalm, kNotIfCalm } when;  // calm data: the second takes all its columns at once, the third has nothing to do
     bool wide;              // entries of two words
-    uint32_t* entries;      // [row_tiles * 256][kMmaCap]
-    uint32_t* counts;       // [row_tiles * 256] entries; above kMmaCap: some were lost
+    uint32_t cap;           // entries of a row's buffer: kMmaCap, or more (of one word each) in a graph of one phase
+    uint32_t* entries;      // [row_tiles * 256][cap]
+    uint32_t* counts;       // [row_tiles * 256] entries; above cap: some were lost
     uint4* hits;            // 32 rows and 32 columns among which a product reaches its gate: first row, first column, rows, both
     uint32_t* hit_count;
     uint32_t hit_room;
@@ -610,8 +612,8 @@ __device__ __forceinline__ void store_entry(uint32_t* buf, bool wide, uint32_t e
     if (wide) reinterpret_cast<uint2*>(buf)[e] = make_uint2(d, node);
     else buf[e] = d << 25 | node;
 }
-__device__ __forceinline__ uint32_t* buffer_of(uint32_t* entries, bool wide, uint32_t place) {
-    return entries + size_t(place) * (kMmaCap * (wide ? 2 : 1));
+__device__ __forceinline__ uint32_t* buffer_of(const KnnMmaArgs& a, uint32_t place) {
+    return a.entries + size_t(place) * (a.cap * (a.wide ? 2 : 1));
 }
 
 // The row's buffer shrinks to its k best (or all that are no worse than the k-th, up to kMmaKeep).  By the whole warp;
@@ -701,9 +703,9 @@ __device__ __forceinline__ void compare_rows(const KnnMmaArgs& a, uint32_t rows,
             const uint32_t d = dist >> (8 * b) & 255u;
             const uint32_t to = __shfl_sync(kFull, slot, src[b]) + __popc(here[b] & below);
             const uint32_t row_node = __shfl_sync(kFull, row.x, src[b]);
-            if ((here[b] >> lane & 1u) && to < kMmaCap) store_entry(buffer_of(a.entries, a.wide, row0 + src[b]), a.wide, to, d, p.x);
+            if ((here[b] >> lane & 1u) && to < a.cap) store_entry(buffer_of(a, row0 + src[b]), a.wide, to, d, p.x);
             if (there >> b & 1u) {
-                if (at < kMmaCap) store_entry(buffer_of(a.entries, a.wide, col), a.wide, at, d, row_node);
+                if (at < a.cap) store_entry(buffer_of(a, col), a.wide, at, d, row_node);
                 ++at;
             }
         }
@@ -1063,14 +1065,14 @@ __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool on
     const uint32_t row0 = blockIdx.x * kMmaRows + (threadIdx.x & ~31u), own = row0 + lane;
     uint32_t count = a.counts[own];
     int limit = int(a.place[own].y);
-    const bool lost = count > kMmaCap, anew = lost && again;
+    const bool lost = count > a.cap, anew = lost && again;
     uint32_t todo = __ballot_sync(kFull, anew || (!lost && !only_lost && count >= a.k && limit >= 0));
     const uint32_t anews = __ballot_sync(kFull, anew);
     while (todo) {
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;
-        uint32_t c = min(__shfl_sync(kFull, count, src), kMmaCap);
-        uint32_t* buf = buffer_of(a.entries, a.wide, row0 + src);
+        uint32_t c = min(__shfl_sync(kFull, count, src), kMmaCap);  // (of a longer buffer the first)
+        uint32_t* buf = buffer_of(a, row0 + src);
         uint32_t T;
         auto kth = [&](auto slots) {
             uint32_t dist[decltype(slots)::value];
@@ -1119,7 +1121,7 @@ __global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint
             const uint32_t node = a.place[j].x;
             if (node == kInvalidNode) continue;
             const uint32_t at = atomicAdd(a.counts + row, 1u);
-            if (at < kMmaCap) store_entry(buffer_of(a.entries, a.wide, row), a.wide, at, uint32_t(d), node);
+            if (at < a.cap) store_entry(buffer_of(a, row), a.wide, at, uint32_t(d), node);
         }
     }
 }
@@ -1129,49 +1131,104 @@ __global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint
 // they are wide or many, a row's rank is the number of entries before it.
 constexpr int kFinishWarps = 4;
 constexpr int kFinishSort = 128;
+constexpr int kFinishBins = 96;  // distances are 64 at most
+
+// A longer buffer: its entries up to the k-th distance, or the k first by id where too many are at it, by the whole warp;
+// returns their number.
+__device__ __forceinline__ uint32_t best_of_long(const uint32_t* buf, uint32_t count, uint32_t k, uint32_t nodes, uint32_t* bins, uint32_t* words, int lane) {
+    for (int i = lane; i < kFinishBins; i += 32) bins[i] = 0;
+    __syncwarp();
+#pragma unroll 4
+    for (uint32_t e = lane; e < count; e += 32) atomicAdd(bins + load_entry(buf, false, e).d, 1u);
+    __syncwarp();
+    const uint32_t c0 = bins[3 * lane], c1 = bins[3 * lane + 1], c2 = bins[3 * lane + 2];
+    uint32_t upto = c0 + c1 + c2;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, upto, o);
+        if (lane >= o) upto += y;
+    }
+    const int at = __ffs(__ballot_sync(kFull, upto >= k)) - 1;  // (count > k: there is one)
+    uint32_t below = upto - c0 - c1 - c2, T = 3 * lane, same = c0;
+    if (below + same < k) below += c0, same = c1, ++T;
+    if (below + same < k) below += c1, same = c2, ++T;
+    T = __shfl_sync(kFull, T, at), below = __shfl_sync(kFull, below, at), same = __shfl_sync(kFull, same, at);
+    uint32_t last = kInvalidNode;  // largest id taken at distance T
+    if (below + same > kMmaCap) {
+        uint32_t lo = 0, hi = nodes;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            uint32_t c = 0;
+#pragma unroll 4
+            for (uint32_t e = lane; e < count; e += 32) {
+                const Entry x = load_entry(buf, false, e);
+                c += x.d == T && x.node <= mid;
+            }
+            if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
+            else lo = mid + 1;
+        }
+        last = lo;
+    }
+    uint32_t m = 0;
+#pragma unroll 4
+    for (uint32_t e0 = 0; e0 < count; e0 += 32) {
+        const uint32_t e = e0 + lane;
+        const Entry x = e < count ? load_entry(buf, false, e) : Entry{kFull, 0u};
+        const bool take = x.d < T || (x.d == T && x.node <= last);
+        const uint32_t b = __ballot_sync(kFull, take);
+        if (take) words[m + __popc(b & ((1u << lane) - 1u))] = x.d << 25 | x.node;
+        m += __popc(b);
+    }
+    return m;
+}
 
 __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
                                                                        uint16_t* __restrict__ dists, uint32_t out_row0,
                                                                        uint32_t* __restrict__ redo /* their number, rows */) {
     if (a.choice.skip()) return;
     __shared__ uint64_t keys_sm[kFinishWarps][kMmaCap];
+    __shared__ uint32_t bins_sm[kFinishWarps][kFinishBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t place = blockIdx.x * kFinishWarps + warp;
     if (place >= rows) return;
     const uint32_t row = a.place[place].x, count = a.counts[place];
     if (row == kInvalidNode) return;
-    if (count > kMmaCap) {
+    if (count > a.cap) {
         if (lane == 0) redo[1 + atomicAdd(redo, 1u)] = row;
         return;
     }
-    const uint32_t* buf = buffer_of(a.entries, a.wide, place);
-    Entry x[kMmaSlots];
-    uint32_t dist[kMmaSlots];
-#pragma unroll
-    for (int s = 0; s < kMmaSlots; ++s) {
-        x[s] = Entry{kFull, 0u};
-        if (s * 32u < count && uint32_t(s * 32 + lane) < count) x[s] = load_entry(buf, a.wide, s * 32 + lane);
-        dist[s] = x[s].d;
-    }
-    uint32_t T = uint32_t(a.K);
-    if (count > a.k) {
-        if (count <= kMmaKeep) T = kth_distance(reinterpret_cast<const uint32_t (&)[kMmaKeep / 32]>(dist), a.k, a.K);
-        else T = kth_distance(dist, a.k, a.K);
-    }
+    const uint32_t* buf = buffer_of(a, place);
     uint32_t* out_n = nbrs + size_t(row - out_row0) * a.k;
     uint16_t* out_d = dists ? dists + size_t(row - out_row0) * a.k : nullptr;
     uint64_t* keys = keys_sm[warp];
     uint32_t* words = reinterpret_cast<uint32_t*>(keys);
     const uint32_t below = (1u << lane) - 1u;
     uint32_t m = 0;
+    if (count > kMmaCap) {
+        m = best_of_long(buf, count, a.k, a.meet.tiles * kMmaRows, bins_sm[warp], words, lane);
+    } else {
+        Entry x[kMmaSlots];
+        uint32_t dist[kMmaSlots];
 #pragma unroll
-    for (int s = 0; s < kMmaSlots; ++s) {
-        if (s * 32u >= count) break;
-        const bool take = x[s].d <= T;
-        const uint32_t b = __ballot_sync(kFull, take), at = m + __popc(b & below);
-        if (take && a.wide) keys[at] = (uint64_t(x[s].d) << 32) | x[s].node;
-        else if (take) words[at] = x[s].d << 25 | x[s].node;
-        m += __popc(b);
+        for (int s = 0; s < kMmaSlots; ++s) {
+            x[s] = Entry{kFull, 0u};
+            if (s * 32u < count && uint32_t(s * 32 + lane) < count) x[s] = load_entry(buf, a.wide, s * 32 + lane);
+            dist[s] = x[s].d;
+        }
+        uint32_t T = uint32_t(a.K);
+        if (count > a.k) {
+            if (count <= kMmaKeep) T = kth_distance(reinterpret_cast<const uint32_t (&)[kMmaKeep / 32]>(dist), a.k, a.K);
+            else T = kth_distance(dist, a.k, a.K);
+        }
+#pragma unroll
+        for (int s = 0; s < kMmaSlots; ++s) {
+            if (s * 32u >= count) break;
+            const bool take = x[s].d <= T;
+            const uint32_t b = __ballot_sync(kFull, take), at = m + __popc(b & below);
+            if (take && a.wide) keys[at] = (uint64_t(x[s].d) << 32) | x[s].node;
+            else if (take) words[at] = x[s].d << 25 | x[s].node;
+            m += __popc(b);
+        }
     }
     __syncwarp();
     const uint32_t kept = min(m, a.k);
@@ -1330,12 +1387,28 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const uint32_t hit_room = uint32_t(most_hits < kHitRoom ? most_hits : kHitRoom);
     const size_t hits_b = size_t(hit_room) * 16;
     size_t entries_b, counts_b, list_b;
+    // In one phase a row's limit stays what the places beside it say, the k-th of 512 distances: on data without clusters a
+    // share of k / 512 of the nodes is within it, which twice as long a buffer holds with the ties.  (With 384 entries nearly
+    // every row ran over and was compared with all nodes up to three times more; K = 32, unit sphere, 5,000 nodes: 716 us so,
+    // 319 now; K = 64, 8,191 nodes: 2,048 and 715; mixture of sigma 0.6, 14,000 x 960, two bytes: 2,598 and 1,378.  Clustered
+    // data do not touch what they do not fill.)
+    const Meet whole{uint32_t((wanted + kMmaRows - 1) / kMmaRows + (n - wanted + kMmaRows - 1) / kMmaRows), uint32_t((wanted + kMmaRows - 1) / kMmaRows)};
+    uint64_t cap = kMmaCap;
+    if (whole.columns() <= kOnePhase && whole.row_tiles / 2 + 1 < kNearFrom) {
+        const uint64_t longest = kLongBuffers / (uint64_t(whole.row_tiles) * kMmaRows * 4), of_use = n * k / 256;
+        cap = (of_use < longest ? of_use : longest) / 32 * 32;
+        if (cap < kMmaCap) cap = kMmaCap;
+    }
     while (true) {
         const size_t slots = size_t((block + kMmaRows - 1) / kMmaRows) * kMmaRows;
-        entries_b = up(slots * kMmaCap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up((slots + 1) * 4);
+        entries_b = up(slots * cap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up((slots + 1) * 4);
         const size_t buffers_b = entries_b > before_b ? entries_b : before_b;
         const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + 256);
         if (rc == 0) break;
+        if (rc == kNoRoom && cap > kMmaCap) {
+            cap = kMmaCap;
+            continue;
+        }
         if (rc != kNoRoom || entries_b <= before_b || block <= uint64_t(sms) * kMmaRows) return rc;
         block = (block + 1) / 2;
     }
@@ -1376,6 +1449,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.place = places;
     a.gate = gate;
     a.wide = wide;
+    a.cap = uint32_t(cap);
     a.K = int(h->K);
     a.symbols = shape.symbols;
     a.chunks = shape.chunks;

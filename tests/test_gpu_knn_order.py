@@ -59,8 +59,9 @@ def test_routes(cp, n, k, dim, K, cb, per, sigma, rows, kernel):
     agree(cp, idx, dim, K, cb, codes, k, *(rows or (0, n)))
 
 
-# thousands of equal codes: their rows' buffers run over twice, and the row is compared with every node
-@pytest.mark.parametrize("n,equal", [(11000, 700), (34000, 3000)])
+# hundreds to thousands of equal codes: more ties than a row's neighbours are taken from by id (in one phase a buffer holds n k / 256
+# entries), or their rows' buffers run over twice and the row is compared with every node
+@pytest.mark.parametrize("n,equal", [(5000, 390), (11000, 700), (11000, 2740), (11000, 5000), (34000, 3000)])
 def test_equal_codes(cp, n, equal):
     import torch
     idx = cp.CPHNSWIndex(128, K=32)
