@@ -268,16 +268,16 @@ template <bool U16, int QUADS, bool SECTORS, int ORDERS, int WINDOW>
 __global__ void __launch_bounds__(kBoundWarps * 32)
 bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t* __restrict__ order, const uint32_t* __restrict__ place,
              uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound, uint32_t* __restrict__ group, uint32_t* __restrict__ mate,
-             uint64_t apart /* of LoadArgs: its rows only; 0: all rows */, const uint32_t* __restrict__ listed /* their number, rows: only these */,
-             SweepChoice choice) {
+             uint64_t apart /* of LoadArgs: its rows only; 0: all rows */, const uint32_t* __restrict__ listed /* only these rows */,
+             const uint32_t* __restrict__ listed_count, SweepChoice choice) {
     if (choice.skip()) return;
     constexpr int S = WINDOW / 32, N = ORDERS * S;
     constexpr uint32_t kSeenSlots = N * 32 > 512 ? 1024 : 512;
     __shared__ uint32_t seen_sm[kBoundWarps][kSeenSlots];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t warps = uint64_t(gridDim.x) * kBoundWarps, many = listed ? listed[0] : apart ? warps : n;
+    const uint64_t warps = uint64_t(gridDim.x) * kBoundWarps, many = listed ? *listed_count : apart ? warps : n;
     for (uint64_t at = uint64_t(blockIdx.x) * kBoundWarps + warp; at < many; at += warps) {
-        const uint64_t wanted = listed ? listed[1 + at] : apart ? row_begin + at / 32 * apart + at % 32 : order[at];
+        const uint64_t wanted = listed ? listed[at] : apart ? row_begin + at / 32 * apart + at % 32 : order[at];
         if (wanted < row_begin || wanted >= row_end) continue;
         const uint32_t row = uint32_t(wanted);
         uint32_t* seen = seen_sm[warp];
@@ -353,7 +353,7 @@ constexpr int kBesideRows = 32, kBesideWarps = 4, kBesidePlaces = 512;
 template <bool U16, int QUADS>
 __global__ void __launch_bounds__(kBesideWarps * 32) beside_kernel(const uint4* __restrict__ codes, const uint32_t* __restrict__ grouped, uint32_t rows,
                                                                    int K, uint32_t k, uint32_t* __restrict__ bound,
-                                                                   uint32_t* __restrict__ far /* their number, rows */, SweepChoice choice) {
+                                                                   uint32_t* __restrict__ far, uint32_t* __restrict__ far_count, SweepChoice choice) {
     if (choice.skip()) return;
     extern __shared__ __align__(16) unsigned char beside_smem[];
     uint4* code = reinterpret_cast<uint4*>(beside_smem);                                   // [kBesidePlaces][QUADS]
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(kBesideWarps * 32) beside_kernel(const uint4* 
         if (upto >= k) break;
     }
     if (T < before) bound[node] = T;
-    if (min(T, before) > uint32_t(K) * 5 / 8) far[1 + atomicAdd(far, 1u)] = node;
+    if (min(T, before) > uint32_t(K) * 5 / 8) far[atomicAdd(far_count, 1u)] = node;
 }
 
 // ---- what the filter is worth ----------------------------------------------------------------------------------------
@@ -1059,7 +1059,8 @@ __global__ void __launch_bounds__(kSortRows) layout_kernel(const uint4* __restri
 // ---- between two phases: room in the buffers, limits of the k best so far ---------------------------------
 // Where a buffer ran over the k-th distance of what it holds is a limit that few nodes are within: with a list the buffer
 // starts anew and the row is listed for knn_again_kernel (without one nothing more is of use to the row for now).
-__global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool only_lost, uint32_t* __restrict__ again /* their number, places */) {
+__global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool only_lost, uint32_t* __restrict__ again /* places */,
+                                                           uint32_t* __restrict__ again_count) {
     if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
     const int lane = threadIdx.x & 31;
     const uint32_t row0 = blockIdx.x * kMmaRows + (threadIdx.x & ~31u), own = row0 + lane;
@@ -1087,7 +1088,7 @@ __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool on
         if (anews >> src & 1u) c = 0;
         if (lane == src) count = c, limit = limit < 0 || limit > int(T) ? int(T) : limit;
     }
-    if (anew) again[1 + atomicAdd(again, 1u)] = own;
+    if (anew) again[atomicAdd(again_count, 1u)] = own;
     if (lost && !again) limit = -1;
     if (only_lost && !anews) return;
     a.counts[own] = count;
@@ -1099,11 +1100,12 @@ __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool on
 // The listed rows against the nodes of all tiles, or of the row tiles less than `near` tiles away, at their new limits; grid
 // y deals the rows, grid x the nodes.
 template <bool U16, int QUADS>
-__global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint32_t* __restrict__ again, uint32_t near) {
+__global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint32_t* __restrict__ again, const uint32_t* __restrict__ again_count,
+                                                        uint32_t near) {
     if (a.choice.skip()) return;
-    const uint32_t many = again[0], places = (near ? 2 * near - 1 : a.meet.tiles) * kMmaRows;
+    const uint32_t many = *again_count, places = (near ? 2 * near - 1 : a.meet.tiles) * kMmaRows;
     for (uint32_t b = blockIdx.y; b < many; b += gridDim.y) {
-        const uint32_t row = again[1 + b], tile = row / kMmaRows;
+        const uint32_t row = again[b], tile = row / kMmaRows;
         const uint32_t from = near ? (tile >= near - 1 ? tile - (near - 1) : tile + a.meet.row_tiles - (near - 1)) * kMmaRows : 0;
         const int limit = int(a.place[row].y);
         uint4 own[QUADS];
@@ -1184,7 +1186,7 @@ __device__ __forceinline__ uint32_t best_of_long(const uint32_t* buf, uint32_t c
 
 __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
                                                                        uint16_t* __restrict__ dists, uint32_t out_row0,
-                                                                       uint32_t* __restrict__ redo /* their number, rows */) {
+                                                                       uint32_t* __restrict__ redo /* rows */, uint32_t* __restrict__ redo_count) {
     if (a.choice.skip()) return;
     __shared__ uint64_t keys_sm[kFinishWarps][kMmaCap];
     __shared__ uint32_t bins_sm[kFinishWarps][kFinishBins];
@@ -1194,7 +1196,7 @@ __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArg
     const uint32_t row = a.place[place].x, count = a.counts[place];
     if (row == kInvalidNode) return;
     if (count > a.cap) {
-        if (lane == 0) redo[1 + atomicAdd(redo, 1u)] = row;
+        if (lane == 0) redo[atomicAdd(redo_count, 1u)] = row;
         return;
     }
     const uint32_t* buf = buffer_of(a, place);
@@ -1289,15 +1291,16 @@ constexpr int kRedoWarps = 32;
 template <bool U16, int QUADS>
 __global__ void __launch_bounds__(kRedoWarps * 32) knn_redo_kernel(const uint4* __restrict__ codes, uint32_t n, uint32_t k, int K,
                                                                    const uint32_t* __restrict__ bound, const uint32_t* __restrict__ redo,
+                                                                   const uint32_t* __restrict__ redo_count,
                                                                    uint32_t* __restrict__ nbrs, uint16_t* __restrict__ dists, uint32_t out_row0,
                                                                    SweepChoice choice) {
     if (choice.skip()) return;
     __shared__ uint32_t hist[96], ties[kRedoWarps][128], tie_count[kRedoWarps], below_sm, T_sm, found;
     __shared__ uint64_t keys[128];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, many = redo[0];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, many = *redo_count;
     const uint32_t from = uint32_t(uint64_t(n) * warp / kRedoWarps), to = uint32_t(uint64_t(n) * (warp + 1) / kRedoWarps);
     for (uint32_t b = blockIdx.x; b < many; b += gridDim.x) {
-        const uint32_t row = redo[1 + b], most = min(bound[row], uint32_t(K));
+        const uint32_t row = redo[b], most = min(bound[row], uint32_t(K));
         uint4 own[QUADS];
 #pragma unroll
         for (int w = 0; w < QUADS; ++w) own[w] = __ldg(codes + size_t(row) * QUADS + w);
@@ -1401,9 +1404,9 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     }
     while (true) {
         const size_t slots = size_t((block + kMmaRows - 1) / kMmaRows) * kMmaRows;
-        entries_b = up(slots * cap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up((slots + 1) * 4);
+        entries_b = up(slots * cap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up(slots * 4);
         const size_t buffers_b = entries_b > before_b ? entries_b : before_b;
-        const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + 256);
+        const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + 512);
         if (rc == 0) break;
         if (rc == kNoRoom && cap > kMmaCap) {
             cap = kMmaCap;
@@ -1425,19 +1428,22 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     uint32_t* bound = reinterpret_cast<uint32_t*>(take(n_b));
     uint32_t* group = reinterpret_cast<uint32_t*>(take(n_b));
     uint32_t* mate = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* far = mate;  // rows whose bound says little (the mates have joined their groups by then)
     uint32_t* grouped = reinterpret_cast<uint32_t*>(take(n_b));
-    uint32_t* group_count = reinterpret_cast<uint32_t*>(take(n_b));
     uint32_t* group_place = reinterpret_cast<uint32_t*>(take(n_b));
-    uint32_t* counts = reinterpret_cast<uint32_t*>(take(counts_b));
     uint32_t* again = reinterpret_cast<uint32_t*>(take(list_b));
     uint32_t* redo = reinterpret_cast<uint32_t*>(take(list_b));
     uint4* hits = reinterpret_cast<uint4*>(take(hits_b));
+    // cleared for every block of rows, in one go (as clears of their own: a graph of 4,096 nodes 177 us, 167 so)
     struct Counters {
-        LoadCounts load;
-        uint32_t used, hits;
+        uint32_t used, hits, far, again, redo;
     };
-    static_assert(sizeof(Counters) <= 256, "counters take 256 bytes");
+    static_assert(sizeof(Counters) <= 256 && sizeof(LoadCounts) <= 256, "counters take 256 bytes");
+    unsigned char* cleared = p;
     Counters* counters = reinterpret_cast<Counters*>(take(256));
+    uint32_t* group_count = reinterpret_cast<uint32_t*>(take(n_b));
+    uint32_t* counts = reinterpret_cast<uint32_t*>(take(counts_b));
+    LoadCounts* load = reinterpret_cast<LoadCounts*>(take(256));
     uint32_t* entries = reinterpret_cast<uint32_t*>(p);
     uint32_t* hist = reinterpret_cast<uint32_t*>(take(hist_b));
     uint32_t* order = reinterpret_cast<uint32_t*>(take(order_b));
@@ -1471,16 +1477,15 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     sample.apart = wanted / sample.groups < 32 ? 32 : wanted / sample.groups;
     const uint64_t node_tiles = (n + kMmaRows - 1) / kMmaRows;
     if (other) {
-        a.choice.load = &counters->load.turns;
+        a.choice.load = &load->turns;
         a.choice.most = (unsigned long long)(most_turns * sample.groups * kLoadTiles);
         *other = a.choice;
         other->above = true;
-        a.calm.counts = &counters->load;
+        a.calm.counts = load;
         a.calm.most_turns = (unsigned long long)(kCalmTurns * sample.groups * kLoadTiles);
         a.calm.most = uint32_t(kCalmEntries * 32 * kLoadTiles * sample.groups / double(node_tiles));
     }
-    CPB_CUDA(cudaMemsetAsync(hist, 0, hist_b, st));
-    CPB_CUDA(cudaMemsetAsync(counters, 0, sizeof(Counters), st));
+    CPB_CUDA(cudaMemsetAsync(load, 0, 256 + hist_b, st));
     const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
     key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
     key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
@@ -1488,7 +1493,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     auto bounds = [&](uint64_t count, uint64_t apart, auto orders, auto window, const uint32_t* listed, const SweepChoice& choice) {
         auto go = [&](auto kernel) {
             kernel<<<unsigned((count + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(rows, a.K, n, order, place, k, uint32_t(row_begin),
-                                                                                                  uint32_t(row_end), bound, group, mate, apart, listed, choice);
+                                                                                                  uint32_t(row_end), bound, group, mate, apart, listed, &counters->far, choice);
         };
         constexpr int O = decltype(orders)::value, W = decltype(window)::value;
         if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) go(bound_kernel<U16, QUADS, (QUADS > 1), O, W>);
@@ -1501,7 +1506,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         bounds(uint64_t(sample.groups) * 32, sample.apart, All(), Full(), nullptr, SweepChoice());
         load_kernel<U16, QUADS><<<dim3(sample.groups, kLoadTiles), kMmaRows, 0, st>>>(rows, n, uint32_t(shape.symbols), uint32_t(node_tiles),
                                                                                      uint32_t(row_begin), uint32_t(row_end), bound, sample,
-                                                                                     &counters->load);
+                                                                                     load);
         h->launches++;
     }
     const bool ordered = n >= kOrderNodes;
@@ -1517,21 +1522,16 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         const uint32_t rb = uint32_t(begin), re = uint32_t(row_end - begin < block ? row_end : begin + block), m = re - rb;
         a.meet.row_tiles = (m + kMmaRows - 1) / kMmaRows;
         a.meet.tiles = a.meet.row_tiles + uint32_t((n - m + kMmaRows - 1) / kMmaRows);
-        CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
-        CPB_CUDA(cudaMemsetAsync(redo, 0, 4, st));
-        // a block that gives up leaves rows without entries: they are then empty, not whatever the workspace held
-        CPB_CUDA(cudaMemsetAsync(counts, 0, size_t(a.meet.row_tiles) * kMmaRows * 4, st));
+        // (a block that gives up leaves rows without entries: they are then empty, not whatever the workspace held)
+        CPB_CUDA(cudaMemsetAsync(cleared, 0, 256 + n_b + size_t(a.meet.row_tiles) * kMmaRows * 4, st));
         if (ordered) {
-            CPB_CUDA(cudaMemsetAsync(group_count, 0, size_t(n) * 4, st));
-            CPB_CUDA(cudaMemsetAsync(&counters->used, 0, 4, st));
             group_count_kernel<<<(m + 255) / 256, 256, 0, st>>>(group, rb, re, group_count, a.choice);
             group_place_kernel<<<unsigned((n + 255) / 256), 256, 0, st>>>(group_count, uint32_t(n), group_place, &counters->used, a.choice);
             group_scatter_kernel<<<(m + 255) / 256, 256, 0, st>>>(group, rb, re, group_place, grouped, a.choice);
             beside_kernel<U16, QUADS><<<(m + kBesideRows - 1) / kBesideRows, kBesideWarps * 32,
-                                        kBesidePlaces * QUADS * 16 + (a.K + 1) * kBesideWarps * 64, st>>>(rows, grouped, m, a.K, k, bound, again, a.choice);
+                                        kBesidePlaces * QUADS * 16 + (a.K + 1) * kBesideWarps * 64, st>>>(rows, grouped, m, a.K, k, bound, far, &counters->far, a.choice);
             // (the orders are still there for the first block of rows only)
-            if (rb == row_begin && n > kOnePhase * 2 * kMmaRows) bounds(uint64_t(sms) * 64, 0, All(), Full(), again, a.choice);
-            CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
+            if (rb == row_begin && n > kOnePhase * 2 * kMmaRows) bounds(uint64_t(sms) * 64, 0, All(), Full(), far, a.choice);
             h->launches += 4;
         }
         layout_kernel<QUADS><<<(a.meet.tiles * kMmaRows + kSortRows - 1) / kSortRows, kSortRows, 0, st>>>(
@@ -1544,9 +1544,11 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         const uint32_t columns = a.meet.columns();
         // a launch takes so many steps that its hits have room in the list
         const uint32_t range = uint32_t(kLaunchSteps / a.meet.row_tiles) + 1;
+        bool first = true;
         auto sweep = [&](uint32_t count) {
             const uint64_t steps = uint64_t(a.meet.row_tiles) * count;
-            CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
+            if (!first) CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
+            first = false;
             knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, operand_bytes + a.stages * stage_bytes, st>>>(a);
             knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
             h->launches += 2;
@@ -1559,9 +1561,9 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             a.when = KnnMmaArgs::kAlways;
             a.phase = Phase{0u, 1u, false, 0u, near};
             CPB_TRY(sweep(near));
-            tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, again);
-            knn_again_kernel<U16, QUADS><<<dim3(2, 4 * sms), 256, 0, st>>>(a, again, near);
-            CPB_CUDA(cudaMemsetAsync(again, 0, 4, st));
+            tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, again, &counters->again);
+            knn_again_kernel<U16, QUADS><<<dim3(2, 4 * sms), 256, 0, st>>>(a, again, &counters->again, near);
+            CPB_CUDA(cudaMemsetAsync(&counters->again, 0, 4, st));
             h->launches += 2;
         }
         uint32_t stride = 1;
@@ -1577,16 +1579,17 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             }
             if (stride > 1) {
                 if (one) a.when = KnnMmaArgs::kNotIfCalm;
-                tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, nullptr);
+                tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, nullptr, nullptr);
                 h->launches++;
             }
         }
         a.when = KnnMmaArgs::kAlways;
-        tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, true, again);
-        knn_again_kernel<U16, QUADS><<<dim3(16, sms), 256, 0, st>>>(a, again, 0u);
+        tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, true, again, &counters->again);
+        knn_again_kernel<U16, QUADS><<<dim3(16, sms), 256, 0, st>>>(a, again, &counters->again, 0u);
         const uint32_t slots = a.meet.row_tiles * kMmaRows;
-        knn_finish_kernel<<<slots / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, slots, d_nbrs, d_dist, uint32_t(row_begin), redo);
-        knn_redo_kernel<U16, QUADS><<<sms, kRedoWarps * 32, 0, st>>>(rows, uint32_t(n), k, a.K, bound, redo, d_nbrs, d_dist, uint32_t(row_begin),
+        knn_finish_kernel<<<slots / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, slots, d_nbrs, d_dist, uint32_t(row_begin), redo,
+                                                                          &counters->redo);
+        knn_redo_kernel<U16, QUADS><<<sms, kRedoWarps * 32, 0, st>>>(rows, uint32_t(n), k, a.K, bound, redo, &counters->redo, d_nbrs, d_dist, uint32_t(row_begin),
                                                                         a.choice);
         h->launches += 4;
         CPB_CUDA(cudaGetLastError());
