@@ -72,6 +72,9 @@ constexpr int kSortRows = 1024;           // places sorted by limit together
 constexpr uint32_t kFirstColumns = 8;      // column tiles of the first phase, at most
 constexpr uint32_t kOnePhase = 64;         // up to so many (32,000 nodes) there is only one, and no second bound: what these would save
                                            // costs less than their launches (16,000 x 128: 525 us with them, 392 without)
+constexpr uint32_t kOnePhaseBounds = 48;   // from here on (24,600 nodes) data that are not calm get the second bounds all the same
+                                           // (300-d, two bytes, sigma 0.6: 30,000 5,994 us without, 4,056 with; K = 64, sigma 0.5,
+                                           // 20,000: 1,662 and 1,881)
 constexpr int kBoundOrders = 8;           // orders of likely neighbours
 constexpr int kBoundWindow = 128;         // rows looked at per order
 constexpr int kNameOrders = 4, kNameWindow = 32;  // of them for the names of the groups
@@ -183,6 +186,24 @@ __device__ __forceinline__ uint32_t kth_packed(const uint32_t (&dist)[WORDS], ui
     return lo;
 }
 
+// What the sample counts: turns, and the pairs that are truly within the rows' bounds.  Up to kCalmEntries of them a row
+// the buffers hold what the whole sweep finds, and up to kCalmTurns there is little to gain from limits that fall on the
+// way: it then goes in one phase (400k x 128, mixture sigma 0.5, 29 turns: 185 ms in one, 143 in seven).  Graphs of one phase
+// take the near columns by themselves from kSmallCalm turns in all on, where the launches around them, 60 us, are made up for:
+// K = 32, sigma 0.6, 20,000 x 128 (77 turns) 1,256 us in one, 1,177 so, 10,000 (106) 544 and 591; in 64-byte codes from
+// 0.56 of that (300-d, two bytes, 30,000, 151 turns: 7,982 and 4,056; 14,000, 61 turns: 921 and 951).
+struct LoadCounts {
+    unsigned long long turns;
+    uint32_t within;
+};
+constexpr double kCalmEntries = 230, kCalmTurns = 20, kSmallCalm = 25e9;
+struct Calm {
+    const LoadCounts* counts = nullptr;  // (nullptr: not known)
+    uint32_t most = 0;
+    unsigned long long most_turns = 0;
+    __device__ __forceinline__ bool yes() const { return counts && counts->within <= most && counts->turns <= most_turns; }
+};
+
 // ---- bounds from likely neighbours ---------------------------------------------------------------------------------
 // the low 8 bits of two components (the sign and the low index bits; all of a one-byte component)
 template <typename CompT>
@@ -269,8 +290,8 @@ __global__ void __launch_bounds__(kBoundWarps * 32)
 bound_kernel(const uint4* __restrict__ codes, int K, uint64_t n, const uint32_t* __restrict__ order, const uint32_t* __restrict__ place,
              uint32_t k, uint32_t row_begin, uint32_t row_end, uint32_t* __restrict__ bound, uint32_t* __restrict__ group, uint32_t* __restrict__ mate,
              uint64_t apart /* of LoadArgs: its rows only; 0: all rows */, const uint32_t* __restrict__ listed /* only these rows */,
-             const uint32_t* __restrict__ listed_count, SweepChoice choice) {
-    if (choice.skip()) return;
+             const uint32_t* __restrict__ listed_count, SweepChoice choice, Calm calm) {
+    if (choice.skip() || calm.yes()) return;
     constexpr int S = WINDOW / 32, N = ORDERS * S;
     constexpr uint32_t kSeenSlots = N * 32 > 512 ? 1024 : 512;
     __shared__ uint32_t seen_sm[kBoundWarps][kSeenSlots];
@@ -399,21 +420,6 @@ struct LoadArgs {
     uint32_t groups;
 };
 constexpr uint32_t kLoadGroups = 16, kLoadTiles = 16;
-// What the sample counts: turns, and the pairs that are truly within the rows' bounds.  Up to kCalmEntries of them a row
-// the buffers hold what the whole sweep finds, and up to kCalmTurns there is little to gain from limits that fall on the
-// way: it then goes in one phase (400k x 128, mixture sigma 0.5, 29 turns: 185 ms in one, 143 in seven).
-struct LoadCounts {
-    unsigned long long turns;
-    uint32_t within;
-};
-constexpr double kCalmEntries = 230, kCalmTurns = 20;
-struct Calm {
-    const LoadCounts* counts = nullptr;  // (nullptr: not known)
-    uint32_t most = 0;
-    unsigned long long most_turns = 0;
-    __device__ __forceinline__ bool yes() const { return counts && counts->within <= most && counts->turns <= most_turns; }
-};
-
 // the symbols of a word's components, in their places
 template <bool U16>
 __device__ __forceinline__ uint32_t symbols_of(uint32_t w, uint32_t symbols) {
@@ -616,6 +622,23 @@ __device__ __forceinline__ uint32_t* buffer_of(const KnnMmaArgs& a, uint32_t pla
     return a.entries + size_t(place) * (a.cap * (a.wide ? 2 : 1));
 }
 
+// What is nearer than T, and at T up to node `last`, moves to the front of the buffer; returns their number.  By the whole warp.
+__device__ __forceinline__ uint32_t keep_entries(uint32_t* buf, bool wide, uint32_t count, uint32_t T, uint32_t last, int lane) {
+    __syncwarp();
+    uint32_t at = 0;
+#pragma unroll 1
+    for (uint32_t e = lane; e < (count + 31u) / 32 * 32; e += 32) {  // (an entry moves down or stays)
+        const Entry x = e < count ? load_entry(buf, wide, e) : Entry{kFull, kInvalidNode};
+        const bool keep = x.d < T || (x.d == T && x.node <= last);
+        const uint32_t m = __ballot_sync(kFull, keep);
+        __syncwarp();
+        if (keep) store_entry(buf, wide, at + __popc(m & ((1u << lane) - 1u)), x.d, x.node);
+        at += __popc(m);
+        __syncwarp();
+    }
+    return at;
+}
+
 // The row's buffer shrinks to its k best (or all that are no worse than the k-th, up to kMmaKeep).  By the whole warp;
 // returns the k-th distance and the new count.
 __device__ __forceinline__ uint32_t compact_row(uint32_t* buf, bool wide, uint32_t& count, uint32_t k, int K, int lane) {
@@ -647,19 +670,7 @@ __device__ __forceinline__ uint32_t compact_row(uint32_t* buf, bool wide, uint32
         }
         last = lo;
     }
-    __syncwarp();
-    uint32_t at = 0;
-#pragma unroll 1
-    for (uint32_t e = lane; e < (count + 31u) / 32 * 32; e += 32) {  // (an entry moves down or stays)
-        const Entry x = e < count ? load_entry(buf, wide, e) : Entry{kFull, kInvalidNode};
-        const bool keep = x.d < T || (x.d == T && x.node <= last);
-        const uint32_t m = __ballot_sync(kFull, keep);
-        __syncwarp();
-        if (keep) store_entry(buf, wide, at + __popc(m & ((1u << lane) - 1u)), x.d, x.node);
-        at += __popc(m);
-        __syncwarp();
-    }
-    count = at;
+    count = keep_entries(buf, wide, count, T, last, lane);
     return T;
 }
 
@@ -1056,23 +1067,77 @@ __global__ void __launch_bounds__(kSortRows) layout_kernel(const uint4* __restri
     if (tid < kGates && chunk + tid * 32 < meet.row_tiles * kMmaRows) gate[chunk / 32 + tid] = int16_t(gate_of(symbols, K, largest[tid]));
 }
 
+// ---- buffers of more than kMmaCap entries, of one word each -----------------------------------------------------------
+constexpr int kBins = 96;  // distances are 64 at most
+struct Best {
+    uint32_t T, last;  // the k-th distance; the largest node to take at it
+};
+// The k best of a buffer of more than k entries, or all up to the k-th distance where those are kMmaCap at most.  By the
+// whole warp; bins: [kBins] of its own.
+__device__ __forceinline__ Best best_of_long(const uint32_t* buf, uint32_t count, uint32_t k, uint32_t nodes, uint32_t* bins, int lane) {
+    for (int i = lane; i < kBins; i += 32) bins[i] = 0;
+    __syncwarp();
+#pragma unroll 4
+    for (uint32_t e = lane; e < count; e += 32) atomicAdd(bins + load_entry(buf, false, e).d, 1u);
+    __syncwarp();
+    const uint32_t c0 = bins[3 * lane], c1 = bins[3 * lane + 1], c2 = bins[3 * lane + 2];
+    uint32_t upto = c0 + c1 + c2;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, upto, o);
+        if (lane >= o) upto += y;
+    }
+    const int at = __ffs(__ballot_sync(kFull, upto >= k)) - 1;  // (count > k: there is one)
+    uint32_t below = upto - c0 - c1 - c2, T = 3 * lane, same = c0;
+    if (below + same < k) below += c0, same = c1, ++T;
+    if (below + same < k) below += c1, same = c2, ++T;
+    T = __shfl_sync(kFull, T, at), below = __shfl_sync(kFull, below, at), same = __shfl_sync(kFull, same, at);
+    __syncwarp();
+    if (below + same <= kMmaCap) return Best{T, kInvalidNode};
+    uint32_t lo = 0, hi = nodes;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        uint32_t c = 0;
+#pragma unroll 4
+        for (uint32_t e = lane; e < count; e += 32) {
+            const Entry x = load_entry(buf, false, e);
+            c += x.d == T && x.node <= mid;
+        }
+        if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
+        else lo = mid + 1;
+    }
+    return Best{T, lo};
+}
+
 // ---- between two phases: room in the buffers, limits of the k best so far ---------------------------------
 // Where a buffer ran over the k-th distance of what it holds is a limit that few nodes are within: with a list the buffer
 // starts anew and the row is listed for knn_again_kernel (without one nothing more is of use to the row for now).
+// SHARE warps deal 32 rows among them: eight where the warps that took all 32 would be waited for (64 neighbours, sigma 0.3,
+// 40,000 x 128: 1,057 us with one, 881 with eight), one in large graphs, whose warps are many and mostly have nothing to do.
+template <int SHARE>
 __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool only_lost, uint32_t* __restrict__ again /* places */,
                                                            uint32_t* __restrict__ again_count) {
+    static_assert(SHARE == 1 || SHARE * 32 == kMmaRows, "a block has the rows of one gate, or a warp has");
     if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
-    const int lane = threadIdx.x & 31;
-    const uint32_t row0 = blockIdx.x * kMmaRows + (threadIdx.x & ~31u), own = row0 + lane;
+    __shared__ uint32_t bins_sm[kMmaRows / 32][kBins];
+    __shared__ int largest;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t row0 = (blockIdx.x * (kMmaRows / 32) + warp) / SHARE * 32, own = row0 + lane;
     uint32_t count = a.counts[own];
     int limit = int(a.place[own].y);
+    if constexpr (SHARE > 1) {
+        if (threadIdx.x == 0) largest = -1;
+        __syncthreads();  // (a row's own warp writes what the others have read)
+    }
+    const bool mine = SHARE == 1 || lane % SHARE == warp;
     const bool lost = count > a.cap, anew = lost && again;
-    uint32_t todo = __ballot_sync(kFull, anew || (!lost && !only_lost && count >= a.k && limit >= 0));
+    if (only_lost && !__any_sync(kFull, anew)) return;
+    uint32_t todo = __ballot_sync(kFull, mine && (anew || (!lost && !only_lost && count >= a.k && limit >= 0)));
     const uint32_t anews = __ballot_sync(kFull, anew);
     while (todo) {
         const int src = __ffs(todo) - 1;
         todo &= todo - 1;
-        uint32_t c = min(__shfl_sync(kFull, count, src), kMmaCap);  // (of a longer buffer the first)
+        uint32_t c = min(__shfl_sync(kFull, count, src), a.cap);
         uint32_t* buf = buffer_of(a, row0 + src);
         uint32_t T;
         auto kth = [&](auto slots) {
@@ -1081,20 +1146,30 @@ __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool on
             for (int s = 0; s < decltype(slots)::value; ++s) dist[s] = uint32_t(s * 32 + lane) < c ? load_entry(buf, a.wide, s * 32 + lane).d : kFull;
             return kth_distance(dist, a.k, a.K);
         };
-        if (!(anews >> src & 1u) && c > kMmaFull) T = compact_row(buf, a.wide, c, a.k, a.K, lane);
+        if (c > kMmaCap) {
+            const Best best = best_of_long(buf, c, a.k, a.meet.tiles * kMmaRows, bins_sm[warp], lane);
+            T = best.T;
+            if (!(anews >> src & 1u)) c = keep_entries(buf, false, c, T, best.last, lane);
+        } else if (!(anews >> src & 1u) && c > kMmaFull) T = compact_row(buf, a.wide, c, a.k, a.K, lane);
         else if (c > kMmaFull) T = kth(std::integral_constant<int, kMmaSlots>());
         else if (c > kMmaKeep) T = kth(std::integral_constant<int, kMmaFull / 32>());
         else T = kth(std::integral_constant<int, kMmaKeep / 32>());
         if (anews >> src & 1u) c = 0;
         if (lane == src) count = c, limit = limit < 0 || limit > int(T) ? int(T) : limit;
     }
-    if (anew) again[atomicAdd(again_count, 1u)] = own;
-    if (lost && !again) limit = -1;
-    if (only_lost && !anews) return;
-    a.counts[own] = count;
-    a.place[own].y = uint32_t(limit);
-    const int most = __reduce_max_sync(kFull, limit);
-    if (lane == 0) a.gate[row0 / 32] = int16_t(gate_of(a.symbols, a.K, most));
+    if (mine) {
+        if (anew) again[atomicAdd(again_count, 1u)] = own;
+        if (lost && !again) limit = -1;
+        a.counts[own] = count;
+        a.place[own].y = uint32_t(limit);
+    }
+    int most = __reduce_max_sync(kFull, mine ? limit : -1);
+    if constexpr (SHARE > 1) {
+        if (lane == 0) atomicMax(&largest, most);
+        __syncthreads();
+        most = largest;
+    }
+    if (SHARE == 1 ? lane == 0 : threadIdx.x == 0) a.gate[row0 / 32] = int16_t(gate_of(a.symbols, a.K, most));
 }
 
 // The listed rows against the nodes of all tiles, or of the row tiles less than `near` tiles away, at their new limits; grid
@@ -1133,63 +1208,12 @@ __global__ void __launch_bounds__(256) knn_again_kernel(KnnMmaArgs a, const uint
 // they are wide or many, a row's rank is the number of entries before it.
 constexpr int kFinishWarps = 4;
 constexpr int kFinishSort = 128;
-constexpr int kFinishBins = 96;  // distances are 64 at most
-
-// A longer buffer: its entries up to the k-th distance, or the k first by id where too many are at it, by the whole warp;
-// returns their number.
-__device__ __forceinline__ uint32_t best_of_long(const uint32_t* buf, uint32_t count, uint32_t k, uint32_t nodes, uint32_t* bins, uint32_t* words, int lane) {
-    for (int i = lane; i < kFinishBins; i += 32) bins[i] = 0;
-    __syncwarp();
-#pragma unroll 4
-    for (uint32_t e = lane; e < count; e += 32) atomicAdd(bins + load_entry(buf, false, e).d, 1u);
-    __syncwarp();
-    const uint32_t c0 = bins[3 * lane], c1 = bins[3 * lane + 1], c2 = bins[3 * lane + 2];
-    uint32_t upto = c0 + c1 + c2;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(kFull, upto, o);
-        if (lane >= o) upto += y;
-    }
-    const int at = __ffs(__ballot_sync(kFull, upto >= k)) - 1;  // (count > k: there is one)
-    uint32_t below = upto - c0 - c1 - c2, T = 3 * lane, same = c0;
-    if (below + same < k) below += c0, same = c1, ++T;
-    if (below + same < k) below += c1, same = c2, ++T;
-    T = __shfl_sync(kFull, T, at), below = __shfl_sync(kFull, below, at), same = __shfl_sync(kFull, same, at);
-    uint32_t last = kInvalidNode;  // largest id taken at distance T
-    if (below + same > kMmaCap) {
-        uint32_t lo = 0, hi = nodes;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            uint32_t c = 0;
-#pragma unroll 4
-            for (uint32_t e = lane; e < count; e += 32) {
-                const Entry x = load_entry(buf, false, e);
-                c += x.d == T && x.node <= mid;
-            }
-            if (__reduce_add_sync(kFull, c) >= k - below) hi = mid;
-            else lo = mid + 1;
-        }
-        last = lo;
-    }
-    uint32_t m = 0;
-#pragma unroll 4
-    for (uint32_t e0 = 0; e0 < count; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        const Entry x = e < count ? load_entry(buf, false, e) : Entry{kFull, 0u};
-        const bool take = x.d < T || (x.d == T && x.node <= last);
-        const uint32_t b = __ballot_sync(kFull, take);
-        if (take) words[m + __popc(b & ((1u << lane) - 1u))] = x.d << 25 | x.node;
-        m += __popc(b);
-    }
-    return m;
-}
-
 __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArgs a, uint32_t rows, uint32_t* __restrict__ nbrs,
                                                                        uint16_t* __restrict__ dists, uint32_t out_row0,
                                                                        uint32_t* __restrict__ redo /* rows */, uint32_t* __restrict__ redo_count) {
     if (a.choice.skip()) return;
     __shared__ uint64_t keys_sm[kFinishWarps][kMmaCap];
-    __shared__ uint32_t bins_sm[kFinishWarps][kFinishBins];
+    __shared__ uint32_t bins_sm[kFinishWarps][kBins];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t place = blockIdx.x * kFinishWarps + warp;
     if (place >= rows) return;
@@ -1207,7 +1231,15 @@ __global__ void __launch_bounds__(kFinishWarps * 32) knn_finish_kernel(KnnMmaArg
     const uint32_t below = (1u << lane) - 1u;
     uint32_t m = 0;
     if (count > kMmaCap) {
-        m = best_of_long(buf, count, a.k, a.meet.tiles * kMmaRows, bins_sm[warp], words, lane);
+        const Best best = best_of_long(buf, count, a.k, a.meet.tiles * kMmaRows, bins_sm[warp], lane);
+#pragma unroll 4
+        for (uint32_t e0 = 0; e0 < count; e0 += 32) {
+            const Entry x = e0 + lane < count ? load_entry(buf, false, e0 + lane) : Entry{kFull, 0u};
+            const bool take = x.d < best.T || (x.d == best.T && x.node <= best.last);
+            const uint32_t b = __ballot_sync(kFull, take);
+            if (take) words[m + __popc(b & below)] = x.d << 25 | x.node;
+            m += __popc(b);
+        }
     } else {
         Entry x[kMmaSlots];
         uint32_t dist[kMmaSlots];
@@ -1397,7 +1429,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     // data do not touch what they do not fill.)
     const Meet whole{uint32_t((wanted + kMmaRows - 1) / kMmaRows + (n - wanted + kMmaRows - 1) / kMmaRows), uint32_t((wanted + kMmaRows - 1) / kMmaRows)};
     uint64_t cap = kMmaCap;
-    if (whole.columns() <= kOnePhase && whole.row_tiles / 2 + 1 < kNearFrom) {
+    const bool small = whole.columns() <= kOnePhase && whole.row_tiles / 2 + 1 < kNearFrom;
+    if (small) {
         const uint64_t longest = kLongBuffers / (uint64_t(whole.row_tiles) * kMmaRows * 4), of_use = n * k / 256;
         cap = (of_use < longest ? of_use : longest) / 32 * 32;
         if (cap < kMmaCap) cap = kMmaCap;
@@ -1449,6 +1482,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     uint32_t* order = reinterpret_cast<uint32_t*>(take(order_b));
     uint32_t* place = reinterpret_cast<uint32_t*>(take(order_b));
 
+    // data that are not calm, in small graphs: bounds and near columns as in larger ones
+    const bool two = small && other && whole.row_tiles / 2 + 1 >= 2 * kNearColumns;
     KnnMmaArgs a;
     a.operand = operand;
     a.codes = placed;
@@ -1482,18 +1517,18 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         *other = a.choice;
         other->above = true;
         a.calm.counts = load;
-        a.calm.most_turns = (unsigned long long)(kCalmTurns * sample.groups * kLoadTiles);
-        a.calm.most = uint32_t(kCalmEntries * 32 * kLoadTiles * sample.groups / double(node_tiles));
+        a.calm.most_turns = (unsigned long long)((two ? kSmallCalm / (double(n) * n) * (QUADS > 2 ? 0.56 : 1.0) : kCalmTurns) * sample.groups * kLoadTiles);
+        a.calm.most = two ? kFull : uint32_t(kCalmEntries * 32 * kLoadTiles * sample.groups / double(node_tiles));
     }
     CPB_CUDA(cudaMemsetAsync(load, 0, 256 + hist_b, st));
     const dim3 by_row(unsigned((n + 255) / 256), kBoundOrders);
     key_count_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist);
     key_scan_kernel<<<kBoundOrders, 1024, 0, st>>>(hist);
     key_scatter_kernel<CompT><<<by_row, 256, 0, st>>>(codes, n, int(h->K), hist, order, place);
-    auto bounds = [&](uint64_t count, uint64_t apart, auto orders, auto window, const uint32_t* listed, const SweepChoice& choice) {
+    auto bounds = [&](uint64_t count, uint64_t apart, auto orders, auto window, const uint32_t* listed, const SweepChoice& choice, const Calm& calm = Calm()) {
         auto go = [&](auto kernel) {
             kernel<<<unsigned((count + kBoundWarps - 1) / kBoundWarps), kBoundWarps * 32, 0, st>>>(rows, a.K, n, order, place, k, uint32_t(row_begin),
-                                                                                                  uint32_t(row_end), bound, group, mate, apart, listed, &counters->far, choice);
+                                                                                                  uint32_t(row_end), bound, group, mate, apart, listed, &counters->far, choice, calm);
         };
         constexpr int O = decltype(orders)::value, W = decltype(window)::value;
         if (QUADS > 1 && reinterpret_cast<uintptr_t>(padded) % 32 == 0) go(bound_kernel<U16, QUADS, (QUADS > 1), O, W>);
@@ -1532,6 +1567,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
                                         kBesidePlaces * QUADS * 16 + (a.K + 1) * kBesideWarps * 64, st>>>(rows, grouped, m, a.K, k, bound, far, &counters->far, a.choice);
             // (the orders are still there for the first block of rows only)
             if (rb == row_begin && n > kOnePhase * 2 * kMmaRows) bounds(uint64_t(sms) * 64, 0, All(), Full(), far, a.choice);
+            else if (rb == row_begin && two && whole.columns() > kOnePhaseBounds) bounds(uint64_t(sms) * 64, 0, All(), Full(), far, a.choice, a.calm);
             h->launches += 4;
         }
         layout_kernel<QUADS><<<(a.meet.tiles * kMmaRows + kSortRows - 1) / kSortRows, kSortRows, 0, st>>>(
@@ -1554,6 +1590,11 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             h->launches += 2;
             return 0;
         };
+        auto tighten = [&](bool only_lost, uint32_t* list) {
+            if (a.meet.row_tiles < 8 * sms) tighten_kernel<8><<<a.meet.row_tiles * 8, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
+            else tighten_kernel<1><<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
+            h->launches++;
+        };
         // near columns, among which a group's rows are
         uint32_t near = 0;
         if (a.meet.row_tiles / 2 + 1 >= kNearFrom) {
@@ -1561,10 +1602,21 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             a.when = KnnMmaArgs::kAlways;
             a.phase = Phase{0u, 1u, false, 0u, near};
             CPB_TRY(sweep(near));
-            tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, again, &counters->again);
+            tighten(false, again);
             knn_again_kernel<U16, QUADS><<<dim3(2, 4 * sms), 256, 0, st>>>(a, again, &counters->again, near);
             CPB_CUDA(cudaMemsetAsync(&counters->again, 0, 4, st));
-            h->launches += 2;
+            h->launches++;
+        }
+        if (two) {  // the same where data are not calm; the others take all columns at once
+            near = kNearColumns;
+            a.when = KnnMmaArgs::kAllIfCalm;
+            a.phase = Phase{0u, 1u, false, 0u, near};
+            CPB_TRY(sweep(columns));
+            a.when = KnnMmaArgs::kNotIfCalm;
+            tighten(false, again);
+            knn_again_kernel<U16, QUADS><<<dim3(2, 4 * sms), 256, 0, st>>>(a, again, &counters->again, near);
+            CPB_CUDA(cudaMemsetAsync(&counters->again, 0, 4, st));
+            h->launches++;
         }
         uint32_t stride = 1;
         while (columns > kOnePhase && columns - near > kFirstColumns * stride) stride *= 2;
@@ -1573,25 +1625,24 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             a.phase = Phase{near, stride, !whole, 0u, 0u};
             const uint32_t all = a.phase.columns(columns);
             for (uint32_t from = 0; from < all; from += range) {
-                a.when = one ? (whole && from == 0 ? KnnMmaArgs::kAllIfCalm : KnnMmaArgs::kNotIfCalm) : KnnMmaArgs::kAlways;
+                a.when = one ? (whole && from == 0 && !two ? KnnMmaArgs::kAllIfCalm : KnnMmaArgs::kNotIfCalm) : KnnMmaArgs::kAlways;
                 a.phase.from = from, a.phase.count = all - from < range ? all - from : range;
                 CPB_TRY(sweep(a.when == KnnMmaArgs::kAllIfCalm ? columns - near : a.phase.count));
             }
             if (stride > 1) {
                 if (one) a.when = KnnMmaArgs::kNotIfCalm;
-                tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, false, nullptr, nullptr);
-                h->launches++;
+                tighten(false, nullptr);
             }
         }
         a.when = KnnMmaArgs::kAlways;
-        tighten_kernel<<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, true, again, &counters->again);
+        tighten(true, again);
         knn_again_kernel<U16, QUADS><<<dim3(16, sms), 256, 0, st>>>(a, again, &counters->again, 0u);
         const uint32_t slots = a.meet.row_tiles * kMmaRows;
         knn_finish_kernel<<<slots / kFinishWarps, kFinishWarps * 32, 0, st>>>(a, slots, d_nbrs, d_dist, uint32_t(row_begin), redo,
                                                                           &counters->redo);
         knn_redo_kernel<U16, QUADS><<<sms, kRedoWarps * 32, 0, st>>>(rows, uint32_t(n), k, a.K, bound, redo, &counters->redo, d_nbrs, d_dist, uint32_t(row_begin),
                                                                         a.choice);
-        h->launches += 4;
+        h->launches += 3;
         CPB_CUDA(cudaGetLastError());
     }
     return 0;
