@@ -1114,12 +1114,13 @@ __device__ __forceinline__ Best best_of_long(const uint32_t* buf, uint32_t count
 // starts anew and the row is listed for knn_again_kernel (without one nothing more is of use to the row for now).
 // SHARE warps deal 32 rows among them: eight where the warps that took all 32 would be waited for (64 neighbours, sigma 0.3,
 // 40,000 x 128: 1,057 us with one, 881 with eight), one in large graphs, whose warps are many and mostly have nothing to do.
-template <int SHARE>
+// LONG: there are buffers of more than kMmaCap entries (the code for them costs those without it: 500,000 x 128 0.42 and 0.52 ms).
+template <int SHARE, bool LONG>
 __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool only_lost, uint32_t* __restrict__ again /* places */,
                                                            uint32_t* __restrict__ again_count) {
     static_assert(SHARE == 1 || SHARE * 32 == kMmaRows, "a block has the rows of one gate, or a warp has");
     if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
-    __shared__ uint32_t bins_sm[kMmaRows / 32][kBins];
+    __shared__ uint32_t bins_sm[LONG ? kMmaRows / 32 : 1][kBins];
     __shared__ int largest;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t row0 = (blockIdx.x * (kMmaRows / 32) + warp) / SHARE * 32, own = row0 + lane;
@@ -1146,7 +1147,7 @@ __global__ void __launch_bounds__(kMmaRows) tighten_kernel(KnnMmaArgs a, bool on
             for (int s = 0; s < decltype(slots)::value; ++s) dist[s] = uint32_t(s * 32 + lane) < c ? load_entry(buf, a.wide, s * 32 + lane).d : kFull;
             return kth_distance(dist, a.k, a.K);
         };
-        if (c > kMmaCap) {
+        if (LONG && c > kMmaCap) {
             const Best best = best_of_long(buf, c, a.k, a.meet.tiles * kMmaRows, bins_sm[warp], lane);
             T = best.T;
             if (!(anews >> src & 1u)) c = keep_entries(buf, false, c, T, best.last, lane);
@@ -1591,8 +1592,10 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             return 0;
         };
         auto tighten = [&](bool only_lost, uint32_t* list) {
-            if (a.meet.row_tiles < 8 * sms) tighten_kernel<8><<<a.meet.row_tiles * 8, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
-            else tighten_kernel<1><<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
+            const unsigned shared = a.meet.row_tiles * 8;
+            if (cap > kMmaCap) tighten_kernel<8, true><<<shared, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
+            else if (a.meet.row_tiles < 8 * sms) tighten_kernel<8, false><<<shared, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
+            else tighten_kernel<1, false><<<a.meet.row_tiles, kMmaRows, 0, st>>>(a, only_lost, list, &counters->again);
             h->launches++;
         };
         // near columns, among which a group's rows are
