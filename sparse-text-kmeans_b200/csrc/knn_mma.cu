@@ -1427,12 +1427,14 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     // share of k / 512 of the nodes is within it, which twice as long a buffer holds with the ties.  (With 384 entries nearly
     // every row ran over and was compared with all nodes up to three times more; K = 32, unit sphere, 5,000 nodes: 716 us so,
     // 319 now; K = 64, 8,191 nodes: 2,048 and 715; mixture of sigma 0.6, 14,000 x 960, two bytes: 2,598 and 1,378.  Clustered
-    // data do not touch what they do not fill.)
+    // data do not touch what they do not fill.  Components of two bytes have so many values that without
+    // clusters nearly all distances are K: buffers twice as long hold enough of those that are not; 300-d, unit sphere, 8,191
+    // nodes 2,696 us and 1,388, 7,000 2,058 and 1,086.)
     const Meet whole{uint32_t((wanted + kMmaRows - 1) / kMmaRows + (n - wanted + kMmaRows - 1) / kMmaRows), uint32_t((wanted + kMmaRows - 1) / kMmaRows)};
     uint64_t cap = kMmaCap;
     const bool small = whole.columns() <= kOnePhase && whole.row_tiles / 2 + 1 < kNearFrom;
     if (small) {
-        const uint64_t longest = kLongBuffers / (uint64_t(whole.row_tiles) * kMmaRows * 4), of_use = n * k / 256;
+        const uint64_t longest = kLongBuffers / (uint64_t(whole.row_tiles) * kMmaRows * 4), of_use = n * k / (U16 ? 128 : 256);
         cap = (of_use < longest ? of_use : longest) / 32 * 32;
         if (cap < kMmaCap) cap = kMmaCap;
     }

@@ -49,7 +49,7 @@ def agree(cp, idx, dim, K, cb, codes, k, rb, re):
     (10239, 64, 128, 32, 1, 1000, 0.3, None), (10240, 64, 128, 32, 1, 1000, 0.3, None), (10241, 1, 128, 32, 1, 1000, 0.3, None),
     (32256, 64, 96, 32, 1, 1000, 0.3, None), (32512, 127, 128, 32, 1, 1000, 0.3, None), (75776, 64, 128, 16, 1, 1000, 0.3, None),
     (75777, 32, 64, 32, 1, 1000, 0.3, None), (40001, 64, 128, 32, 1, 1000, 0.3, (5003, 29007)), (36000, 64, 128, 32, 1, 18000, 0.3, None),
-    (20001, 64, 300, 32, 2, 1000, 0.4, None), (33001, 64, 128, 64, 1, 500, 0.4, (0, 33000)), (12000, 64, 128, 32, 1, 1, 0.3, None),
+    (20001, 64, 300, 32, 2, 1000, 0.4, None), (7001, 64, 300, 32, 2, 1, 0.3, None), (33001, 64, 128, 64, 1, 500, 0.4, (0, 33000)), (12000, 64, 128, 32, 1, 1, 0.3, None),
     (34000, 20, 64, 10, 1, 1000, 0.3, None)])
 @pytest.mark.parametrize("kernel", [0, 3])
 def test_routes(cp, n, k, dim, K, cb, per, sigma, rows, kernel):
