@@ -614,19 +614,29 @@ static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_
 constexpr uint64_t kMmaMinNodes = 4096;
 // Where the data let too many pairs through its filter the bit-sliced or the byte-wise kernel is taken, which cost the same
 // whatever the data: most_turns is the load (see knn_mma.cu) up to which the filter is the faster, from measured picoseconds
-// a pair.  Filter: 0.25 and 0.006 to 0.05 a turn, by the bytes of a code.  Bit-sliced, K = 32: 1.1 at 400k rows, 1.9 at 100k,
-// 7.5 at 20k (a wave of blocks sweeps all nodes however few rows it has), in proportion to the planes; byte-wise 3 at
-// 32-byte codes, 9 at 64.  Unit sphere, 100k x 128, K = 32: 17.4 ms against 77 through the filter; mixtures of 1,000 points
-// a cluster: sigma 0.3 2.1 against 19.3, sigma 0.6 17.3 against 19.3, sigma 0.7 24.9 against 19.3.
+// a pair.  Bit-sliced, K = 32: 1.1 at 400k rows, 1.9 at 100k, 7.5 at 20k (a wave of blocks sweeps all nodes however few rows
+// it has), in proportion to the planes; byte-wise 3 at 32-byte codes, 9 at 64.  Filter: 0.25 and so much a turn that the
+// following fall on their sides.  The windows see too few of a cluster of 100, whose turns then are as many as those of
+// mixtures that the filter is slow on, and data without clusters have the most: hence the least of all the limits.  ms,
+// filter / other kernels, turns: K = 32, 100k x 128, sigma 0.6 15.8 / 19.2, 67; sigma 0.7 24.2 / 19.1, 166; clusters of 100
+// 3.3 / 18.3, 129, 30k 0.5 / 3.4, 254; unit sphere 77 / 17.3, 481, 20k 3.1 / 1.5, 476.  K = 16, 100k x 64, sigma 0.6 13.3 /
+// 14.8, 89, 0.7 18.4 / 14.6, 142; 400k, sigma 0.5 198 / 110, 40; 20k, clusters of 100 0.5 / 1.4, 278, unit sphere 2.4 / 1.2,
+// 326.  K = 64, 100k, sigma 0.6 38.0 / 38.3, 344; 40k, 0.7 7.1 / 11.0, 433, unit sphere 11.9 / 9.6, 510.  Two bytes, 300-d,
+// 100k, sigma 0.6 37 / 92, 208, 0.7 40 / 91, 320, clusters of 100 8.1 / 89.8, 219, unit sphere 256 / 88, 509; 960-d, 100k,
+// sigma 0.5 30.4 / 23.1, 165, 40k 5.7 / 7.0, 143, 0.6 7.5 / 6.9, 230, 10k, 0.7 0.8 / 1.8, 284.
 static double most_turns(const cphnsw_b200_index* h, uint64_t rows, bool sliced) {
     const double bytes = double(h->K) * h->comp_bytes, planes = h->K * (h->comp_bytes == 2 ? 11.0 : 8.0);
-    const double other = sliced ? (0.8 + 113e3 / double(rows)) * (0.5 + planes / 512)
+    const double other = sliced ? (planes <= 128 ? 0.57 + 140e3 / double(rows) : 0.8 + 113e3 / double(rows)) * (0.5 + planes / 512)
                                 : (bytes <= 16 ? 1.5 : bytes <= 32 ? 2.8 : 9.0) + 50e3 / double(rows);
-    const double turns = (other - 0.25) / (h->comp_bytes == 2 ? 0.05 : bytes <= 16 ? 0.006 : 0.018);
-    return turns < 12 ? 12 : (turns > 300 ? 300 : turns);
+    const double turn = h->comp_bytes == 2 ? 0.0185 : bytes <= 16 ? (sliced ? 0.0145 : 0.0095) : bytes <= 32 ? 0.0115 : 0.0077;
+    const double turns = (other - 0.25) / turn;
+    const double most = h->comp_bytes == 2 ? 330 : bytes <= 32 ? 310 : 480;
+    return turns < 12 ? 12 : (turns > most ? most : turns);
 }
-// Below this many nodes the filter is the faster on any data (4,096 nodes of the unit sphere: 324 to 567 us against 607 to
-// 813 bit-sliced, K = 16 to 64), and the sample is not taken.
+// Below this many nodes the sample is not taken, which costs 55 us: the filter is the faster wherever there are clusters and
+// about as fast without (us, filter / the best other: 8,191 x 128, sigma 0.3 237 / 542, 0.7 403 / 543, unit sphere 402 / 447,
+// 5,000 185 / 352 and 316 / 269; 5,000 x 64, K = 16, unit sphere 229 / 303, K = 64 355 / 596; 960-d 481 / 687), but for codes
+// whose distances are nearly all K (300-d, two bytes, unit sphere, 8,191: 1,388 / 947).
 constexpr uint64_t kMmaAlways = 8192;
 // Up to this many components in all the byte-wise kernel beats the bit-sliced one on one-byte codes (unit sphere, n = 16,384,
 // K = 16 / 32 / 64: 744 / 1,385 / 3,098 us against 1,547 / 1,704 / 3,393; n = 30,000: 1,952 / 3,404 / 9,143 against
