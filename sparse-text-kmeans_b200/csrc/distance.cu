@@ -598,16 +598,29 @@ static int launch_knn_t(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n,
     return launch_knn_w<WC, U16, SLOTS, Q, false>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
 }
 
-template <int WC, bool U16>
-static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
-                            uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
-    // Rows a warp: what its registers hold beside their lists.  Six of 32 bytes leave room for a fourth block an SM and end
-    // more evenly (20,000 rows, K = 32, byte-wise: 1.74 ms with eight, 1.53 with six; 10,000 0.65 and 0.51; 100,000 27.5 and 27.0).
-    constexpr int Q = WC == 32 ? 2 : (WC == 16 ? 4 : (WC == 8 ? 6 : 8));
+template <int WC, bool U16, int Q>
+static int launch_knn_rows(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
+                           uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
     const uint32_t need = k + 1;  // the row's own id may occupy one place
     if (need <= 64) return launch_knn_t<WC, U16, 2, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
     if (need <= 96) return launch_knn_t<WC, U16, 3, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
     return launch_knn_t<WC, U16, 4, Q>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+}
+
+template <int WC, bool U16>
+static int launch_knn_slots(cphnsw_b200_index* h, const uint32_t* codes, uint64_t n, uint32_t k, uint64_t rb,
+                            uint64_t re, uint32_t* nbrs, uint16_t* dist, const SweepChoice& choice, cudaStream_t st) {
+    // Rows a warp: what its registers hold beside their lists.  Of 32 bytes six or eight: shared memory has room for three
+    // blocks an SM whatever their rows, so the number with fewer rows in all the waves one behind the other is taken (K = 32,
+    // byte-wise, six / eight: 10,000 rows, a wave of either, 500 / 647 us; 14,000, two and one, 926 / 804; 20,000, two of
+    // either, 1,548 / 1,748; 100,000 27.7 / 28.2 ms).
+    if constexpr (WC == 8) {
+        auto rows = [&](uint64_t q) { return (re - rb + kKnnWarps * q * 3 * h->sm_count - 1) / (kKnnWarps * q * 3 * h->sm_count) * q; };
+        if (rows(8) < rows(6)) return launch_knn_rows<WC, U16, 8>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+        return launch_knn_rows<WC, U16, 6>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+    } else {
+        return launch_knn_rows<WC, U16, WC == 32 ? 2 : (WC == 16 ? 4 : 8)>(h, codes, n, k, rb, re, nbrs, dist, choice, st);
+    }
 }
 
 // From this many nodes on the tensor-core kernel is taken; below it the launches around it cost more than the sweep.

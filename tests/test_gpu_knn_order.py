@@ -107,3 +107,14 @@ def test_many_nodes(cp, n):
     idx.set_param("knn_kernel", 3)
     agree(cp, idx, 64, K, 1, codes, k, n - rows, n)
     idx.close()
+
+
+# the byte-wise kernel's rows a warp, six or eight of 32 bytes: 10,656 rows are a wave of sixes, 14,208 one of eights (three blocks
+# on each of 148 SMs)
+@pytest.mark.parametrize("rows", [10656, 10657, 14208, 14209])
+@pytest.mark.parametrize("k", [20, 64, 127])
+def test_rows_a_warp(cp, rows, k):
+    idx = cp.CPHNSWIndex(128, K=32)
+    codes = mixture_codes(idx, 15000, 128, 1000, 0.3, 32, 1, rows)
+    idx.set_param("knn_kernel", 2)
+    agree(cp, idx, 128, 32, 1, codes, k, 500, 500 + rows)
