@@ -9,10 +9,11 @@
 // accumulators (+-1 and integers up to 224 are exact in both), so all n^2 pairs cost 2 * 224 tensor operations and one
 // instruction of the epilogue each; only pairs that reach the row's threshold t have their exact distance computed.
 //
-// Row limits.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie
-// beside rows that share both, and the k-th smallest exact distance in the windows of 128 around a row in eight such
-// orders, every row counted once, bounds its final k-th distance from above.  On clustered data it is mostly right or one
-// too high, and some 450 rows pass the filter for a row, 140 of them truly within the bound.
+// Row limits.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie beside
+// rows that share both, so windows of 32 in four such orders name groups of nodes, and once a group's rows lie together the
+// k-th smallest exact distance among the 512 places beside a row bounds its final k-th distance from above.  In larger
+// graphs rows that this says little about get the windows of 128 in eight orders, every row counted once.  On clustered data
+// the bound is mostly right or one too high: of 100,000 x 128, K = 32, sigma 0.3, 200 rows are within it for 64 neighbours.
 //
 // Each pair once.  The distance is symmetric, so a tile of pairs serves the rows of both sides: row tile r meets the column
 // tiles r, r + 1, .. r + half of them, cyclically, which gives every row tile the same work and every pair one product
@@ -27,11 +28,12 @@
 // 38.8 ms with every pair twice and in the order given, 17.6 so (15.0 of them the sweep, 2,200 cycles a tile whose products
 // take 1,792).  The near tiles go first: their k-th distances are mostly final, and limits and gates of the rest are tight.
 //
-// Full buffers.  Where the bounds say little the sweep goes by phases, every 16th (64th ..) column tile first, each of them
-// as much as all before it; between them the k-th distances found are the new limits.  A sample of the data shows whether
-// that is needed, and whether the filter is worth anything at all ("what the filter is worth" below).  A row whose buffer
-// runs over all the same starts anew at the k-th distance of what it held, and where that does not do either it is compared
-// with every node by a kernel without a buffer.
+// Full buffers.  Up to 32,000 nodes the sweep goes in one phase, with buffers for what the bounds let through, or, where
+// clusters overlap, the near columns first.  Above, where the bounds say little, it goes by phases, every 16th (64th ..)
+// column tile first, each of them as much as all before it; between them the k-th distances found are the new limits.  A
+// sample of the data shows whether that is needed, and whether the filter is worth anything at all ("what the filter is
+// worth" below).  A row whose buffer runs over all the same starts anew at the k-th distance of what it held, and where that
+// does not do either it is compared with every node by a kernel without a buffer.
 //
 // Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the column tiles
 // of 256, halves of them in a ring of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
@@ -70,8 +72,9 @@ constexpr int kMaxStages = 8;             // of half a tile each
 constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 5 KB of static
 constexpr int kSortRows = 1024;           // places sorted by limit together
 constexpr uint32_t kFirstColumns = 8;      // column tiles of the first phase, at most
-constexpr uint32_t kOnePhase = 64;         // up to so many (32,000 nodes) there is only one, and no second bound: what these would save
-                                           // costs less than their launches (16,000 x 128: 525 us with them, 392 without)
+constexpr uint32_t kOnePhase = 64;         // up to so many (32,000 nodes) there is one, or the near columns and the rest, and calm
+                                           // data have no second bounds: what these would save costs less than their launches
+                                           // (16,000 x 128, sigma 0.3: 525 us with phases and second bounds, 392 without)
 constexpr uint32_t kOnePhaseBounds = 48;   // from here on (24,600 nodes) data that are not calm get the second bounds all the same
                                            // (300-d, two bytes, sigma 0.6: 30,000 5,994 us without, 4,056 with; K = 64, sigma 0.5,
                                            // 20,000: 1,662 and 1,881)
@@ -602,7 +605,6 @@ __device__ __forceinline__ int gate_of(int symbols, int K, int t) {
 
 // The entries of a row's buffer: (distance, node), packed in a word up to kPackedNodes nodes, in two above.
 constexpr uint32_t kPackedNodes = 1u << 25;
-constexpr uint32_t kNoDistance = 127;  // no entry
 struct Entry {
     uint32_t d, node;
 };
@@ -1410,7 +1412,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     // (places are words of 32 bits, rounded up by tiles; at 144 bytes a node and more no GPU this runs on has room for as many)
     if (n > uint64_t(1) << 31) return kNoRoom;
 
-    // Workspace.  The buffers of the rows found take 1.9 KB a wanted row: where they do not fit, the rows go in blocks.
+    // Workspace.  The buffers take 1.5 KB a wanted row, 3 KB with entries of two words: where they do not fit, the rows go in
+    // blocks.
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const uint64_t most_tiles = (n + kMmaRows - 1) / kMmaRows + 1;  // row tiles and the others are rounded up apart
     const size_t op_b = up(size_t(most_tiles) * operand_bytes), codes_b = up(size_t(most_tiles) * kMmaRows * QUADS * 16);
@@ -1581,7 +1584,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
                                                                                  a.meet.tiles, a.choice);
         h->launches += 2;
         const uint32_t columns = a.meet.columns();
-        // a launch takes so many steps that its hits have room in the list
+        // A launch takes 4M steps: on clustered data, where nearly all of them have no hit, those there are have room in the list.
+        // (Of as many as 64 a step, the sweep compares itself what finds none.)
         const uint32_t range = uint32_t(kLaunchSteps / a.meet.row_tiles) + 1;
         bool first = true;
         auto sweep = [&](uint32_t count) {

@@ -1,5 +1,5 @@
 // Pieces of the two kernels that sweep operand tiles through the tensor cores (knn_mma.cu, exact_mma.cu): shared-memory
-// descriptors, issue and commit, waits, and the split of the tiles between blocks.
+// descriptors, issue and commit, waits; and the split of the exact search's tiles between blocks.
 #pragma once
 
 #include "knn_common.cuh"
@@ -57,13 +57,11 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, ui
 // ---- work split -----------------------------------------------------------------------------------------------------
 // A launch takes `rts` row tiles against all `cts` candidate tiles: rts * cts steps in row-major order, an equal run of
 // them for every block.  When rts is a multiple of the blocks a block takes whole row tiles, and all blocks read the same
-// candidate tiles at the same time; otherwise a row tile may be shared by blocks.  Along the runs block + row tile only
-// grows, so it names a segment (one block's part of one row tile) and its buffers.
+// candidate tiles at the same time; otherwise a row tile may be shared by blocks.
 struct Split {
     uint64_t steps;
     uint32_t cts, blocks;
     __host__ __device__ uint64_t first_step(uint32_t block) const { return uint64_t(block) * steps / blocks; }
-    __host__ __device__ uint32_t block_of(uint64_t step) const { return uint32_t(((step + 1) * blocks - 1) / steps); }
 };
 
 }  // namespace mma

@@ -42,15 +42,25 @@ def agree(cp, idx, dim, K, cb, codes, k, rb, re):
     assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
 
 
-# 10,240 nodes: from here on in an order; 64 columns of tiles (32,512 nodes): near ones first; 296 row tiles: two whole waves and
-# none left over, an even number; 297: odd, one left over; a block of rows against all nodes; clusters far larger than what
-# lies beside a row (several phases); two-byte and four-symbol codes; no clusters at all, every buffer runs over
+# 4,096 nodes: by default through the filter and in an order from here on; 8,192: the sample is taken, and data that are not calm
+# (sigma 0.5 and above) take the near columns first, 24,321 nodes and more with second bounds; 32,001: near columns first on any
+# data; 32,513: phases; 32,769: a third joining of groups, second bounds on any data; 1 and 256 nodes: a tile or less; 296 row
+# tiles: two whole waves and none left over, an even number; 297: odd, one left over; blocks of rows against all nodes, one of
+# them on either side of the near columns; clusters far larger than what lies beside a row (several phases); two-byte and
+# four-symbol codes; no clusters at all
 @pytest.mark.parametrize("n,k,dim,K,cb,per,sigma,rows", [
     (10239, 64, 128, 32, 1, 1000, 0.3, None), (10240, 64, 128, 32, 1, 1000, 0.3, None), (10241, 1, 128, 32, 1, 1000, 0.3, None),
     (32256, 64, 96, 32, 1, 1000, 0.3, None), (32512, 127, 128, 32, 1, 1000, 0.3, None), (75776, 64, 128, 16, 1, 1000, 0.3, None),
     (75777, 32, 64, 32, 1, 1000, 0.3, None), (40001, 64, 128, 32, 1, 1000, 0.3, (5003, 29007)), (36000, 64, 128, 32, 1, 18000, 0.3, None),
     (20001, 64, 300, 32, 2, 1000, 0.4, None), (7001, 64, 300, 32, 2, 1, 0.3, None), (33001, 64, 128, 64, 1, 500, 0.4, (0, 33000)), (12000, 64, 128, 32, 1, 1, 0.3, None),
-    (34000, 20, 64, 10, 1, 1000, 0.3, None)])
+    (34000, 20, 64, 10, 1, 1000, 0.3, None),
+    (1, 5, 64, 32, 1, 1, 0.3, None), (256, 127, 64, 32, 1, 100, 0.3, None), (257, 64, 64, 32, 1, 100, 0.3, None),
+    (4095, 64, 128, 32, 1, 1000, 0.3, None), (4096, 64, 128, 32, 1, 1000, 0.3, None), (4097, 64, 300, 32, 2, 500, 0.4, None),
+    (8191, 64, 128, 32, 1, 1000, 0.7, None), (8192, 64, 128, 64, 1, 1000, 0.7, None), (14001, 32, 300, 32, 2, 1000, 0.6, None),
+    (24320, 64, 128, 32, 1, 1000, 0.7, None), (24321, 64, 128, 32, 1, 1000, 0.7, None), (24577, 127, 300, 32, 2, 1000, 0.6, None),
+    (32000, 64, 128, 32, 1, 1000, 0.3, None), (32001, 64, 128, 32, 1, 1000, 0.6, None), (32513, 64, 128, 32, 1, 1000, 0.5, None),
+    (32768, 64, 128, 16, 1, 1000, 0.6, None), (32769, 64, 128, 16, 1, 1000, 0.6, None),
+    (40001, 64, 128, 32, 1, 1000, 0.5, (1000, 33000)), (40001, 64, 128, 32, 1, 1000, 0.5, (1000, 33001))])
 @pytest.mark.parametrize("kernel", [0, 3])
 def test_routes(cp, n, k, dim, K, cb, per, sigma, rows, kernel):
     idx = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
@@ -118,3 +128,12 @@ def test_rows_a_warp(cp, rows, k):
     codes = mixture_codes(idx, 15000, 128, 1000, 0.3, 32, 1, rows)
     idx.set_param("knn_kernel", 2)
     agree(cp, idx, 128, 32, 1, codes, k, 500, 500 + rows)
+
+
+# 150,000 points without clusters: the last phase lists up to 143 x 586 x 64 groups of 32 rows and 32 columns, 1.2M more than the list
+# has room for, which are compared in the sweep
+def test_more_hits_than_the_list_has_room_for(cp):
+    idx = cp.CPHNSWIndex(128, K=32)
+    codes = mixture_codes(idx, 150000, 128, 1, 1.0, 32, 1, 9)
+    idx.set_param("knn_kernel", 3)
+    agree(cp, idx, 128, 32, 1, codes, 64, 0, 150000)
