@@ -5,9 +5,10 @@
 // symbol is written as a row of the S-point Hadamard matrix without its constant column: S - 1 values of +-1 whose dot
 // product is S - 1 for equal symbols and -1 for different ones.  The dot product of two such rows of (S - 1) K values is
 // S m - K, m the number of components with equal symbols, and m is at least the number of equal components: a pair whose
-// dot product is below S (K - t) - K differs in more than t components.  The products run on tcgen05 in fp8 with fp16
-// accumulators (+-1 and integers up to 224 are exact in both), so all n^2 pairs cost 2 * 224 tensor operations and one
-// instruction of the epilogue each; only pairs that reach the row's threshold t have their exact distance computed.
+// dot product is below S (K - t) - K differs in more than t components.  The products run on tcgen05 in 4-bit floats with fp32
+// accumulators (+-1 and integers up to 224 are exact in both), so a pair costs 2 * 256 tensor operations, at twice the rate of
+// 8-bit ones, and half an instruction of the epilogue; only pairs that reach the row's threshold t have their exact distance
+// computed.
 //
 // Row limits.  Before the sweep a bound is taken from likely neighbours: rows sorted by two of their components lie beside
 // rows that share both, so windows of 32 in four such orders name groups of nodes, and once a group's rows lie together the
@@ -25,8 +26,8 @@
 // Order.  Nodes are placed in an order in which neighbours lie together: the smallest node among the likely neighbours of a
 // node names its group, followed from node to node, and within 1,024 places rows are sorted by their limit.  The pairs that
 // pass are then met in a few tiles, and in all others the epilogue takes one maximum.  500k x 500k, K = 32, 64 neighbours:
-// 38.8 ms with every pair twice and in the order given, 17.6 so (15.0 of them the sweep, 2,200 cycles a tile whose products
-// take 1,792).  The near tiles go first: their k-th distances are mostly final, and limits and gates of the rest are tight.
+// 38.8 ms with every pair twice and in the order given, 17.6 so, with 8-bit operands.  The near tiles go first: their k-th
+// distances are mostly final, and limits and gates of the rest are tight.
 //
 // Full buffers.  Up to 32,000 nodes the sweep goes in one phase, with buffers for what the bounds let through, or, where
 // clusters overlap, the near columns first.  Above, where the bounds say little, it goes by phases, every 16th (64th ..)
@@ -35,14 +36,19 @@
 // worth" below).  A row whose buffer runs over all the same starts anew at the k-th distance of what it held, and where that
 // does not do either it is compared with every node by a kernel without a buffer.
 //
-// Shape.  A block owns 256 rows, their operand resident in shared memory (56 KB at 224 values), and sweeps the column tiles
-// of 256, halves of them in a ring of bulk copies.  A tile is two groups of tcgen05.mma with M = 128, N = 256 into the two
-// halves of tensor memory; while one half is computed the other is read.  A row has two epilogue threads, which take the
-// tiles in turn.  The operand is laid out by
-// the expansion kernel in the form the tensor core reads (8-row by 16-byte core matrices), so a tile is one contiguous copy
-// and no tensor map is needed.
-#include <cuda_fp16.h>
-
+// Shape.  A block owns 256 rows and sweeps the column tiles of 256, a ring of whole tiles in shared memory (32 KB each at 224
+// values) filled by bulk copies.  The rows' operand stays in tensor memory, so the products read only the columns' from shared
+// memory.  A tile is eight units of four products, M = 128, N = 64, into seven accumulators: small units, because some 700 cycles
+// lie between the issue of a unit and the reuse of its accumulator, and what is in flight has to cover them.  Two warps issue;
+// sixteen read, a quarter of the columns and of either half's rows each, and hand an accumulator back as soon as it is in
+// registers.  The operand is laid out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core
+// matrices), so a tile is one contiguous copy and no tensor map is needed.
+// 500k x 500k, K = 32: the sweep takes 9.5 ms, some 1,420 cycles a tile whose products take 1,024 (with 8-bit operands and fp16
+// accumulators 15.1 ms, 2,200 of 1,792), the whole graph 14.7 against 20.4; 1M x 1M 50.2 against 72.9.  On the way, the whole graph:
+// units of N = 128 and three accumulators with one warp issuing 21.0; descriptors known to be uniform and polls before waits 18.3;
+// readers that hand back before they look 17.5; units of 64, a second issuing warp, columns and gates of 32 steps at a time 15.5;
+// polls ahead of the products before 15.2; a step's hits listed a step later and by one atomic 14.7.  Waits that spin instead of
+// sleeping: 15.6 to 16.2.
 #include <type_traits>
 
 #include "mma_common.cuh"
@@ -66,9 +72,10 @@ constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in
 constexpr uint64_t kLaunchSteps = 1u << 22;
 constexpr uint32_t kCheckBlocks = 4;      // blocks of the check an SM
 constexpr uint32_t kNearColumns = 8, kNearFrom = 64;  // column tiles that are swept first, of so many at least
-constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, every second tile
-constexpr int kMmaThreads = (kEpiWarps + 2) * 32;  // and one each for the operands' copies and the products
-constexpr int kMaxStages = 8;             // of half a tile each
+constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, a half of the columns
+constexpr int kMmaWarps = 2;              // warps that issue products, see there
+constexpr int kMmaThreads = (kEpiWarps + 1 + kMmaWarps) * 32;  // and one for the operands' copies
+constexpr int kMaxStages = 8;             // of a tile each
 constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 5 KB of static
 constexpr int kSortRows = 1024;           // places sorted by limit together
 constexpr uint32_t kFirstColumns = 8;      // column tiles of the first phase, at most
@@ -86,13 +93,13 @@ constexpr uint32_t kKeys = 65536;
 
 // symbols and values of a code shape; 0 symbols: not served
 struct HashShape {
-    int symbols, chunks;  // chunks: 16-byte pieces of a row's operand, an even number
+    int symbols, chunks;  // chunks: 16-byte pieces of a row's operand, 32 values each, an even number
 };
 __host__ __device__ inline HashShape hash_shape(int K) {
     HashShape s;
     s.symbols = K <= 32 ? 8 : (K <= 64 ? 4 : 0);
     const int values = K * (s.symbols - 1);
-    s.chunks = (values + 31) / 32 * 2;
+    s.chunks = (values + 63) / 64 * 2;
     return s;
 }
 
@@ -100,7 +107,7 @@ __device__ __forceinline__ uint32_t symbol_of(uint32_t comp, uint32_t symbols) {
     return (comp ^ (comp >> 3) ^ (comp >> 6) ^ (comp >> 9)) & (symbols - 1);
 }
 
-// ---- operand: [tile of 256 rows][chunk][row][16 values] ------------------------------------------------------------
+// ---- operand: [tile of 256 rows][chunk][row][32 values of 4 bits] ---------------------------------------------------
 // codes: padded rows of `stride` components in their places
 template <typename CompT>
 __global__ void expand_codes_kernel(const CompT* __restrict__ codes, int stride, const uint2* __restrict__ place, int K, int symbols,
@@ -113,12 +120,12 @@ __global__ void expand_codes_kernel(const CompT* __restrict__ codes, int stride,
     uint32_t w[4] = {0u, 0u, 0u, 0u};
     if (place[row].x != kInvalidNode) {
         const CompT* code = codes + row * stride;
-        int comp = c * 16 / (symbols - 1), j = c * 16 % (symbols - 1) + 1;
+        int comp = c * 32 / (symbols - 1), j = c * 32 % (symbols - 1) + 1;
         uint32_t h = comp < K ? symbol_of(code[comp], uint32_t(symbols)) : 0u;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const uint32_t e4m3 = (__popc(h & uint32_t(j)) & 1) ? 0xB8u : 0x38u;  // -1 : +1
-            if (comp < K) w[i / 4] |= e4m3 << (8 * (i % 4));
+        for (int i = 0; i < 32; ++i) {
+            const uint32_t e2m1 = (__popc(h & uint32_t(j)) & 1) ? 0xAu : 0x2u;  // -1 : +1
+            if (comp < K) w[i / 8] |= e2m1 << (4 * (i % 8));
             if (++j == symbols) {
                 j = 1;
                 ++comp;
@@ -474,31 +481,52 @@ __global__ void __launch_bounds__(kMmaRows) load_kernel(const uint4* __restrict_
 }
 
 // ---- tcgen05 pieces ------------------------------------------------------------------------------------------------
-// D fp16, A and B e4m3, both K-major, M = 128, N = 256
-constexpr uint32_t kIdesc = (uint32_t(256 >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+// D fp32, A and B e2m1 with a scale of ue8m0 for every 32 values, both K-major, M = 128, N = 64.  Tensor memory: accumulators
+// of 64 columns each, and the block's rows, a half of them in 32 columns, 8 values a word.  The scales, all of them one, lie in
+// the last four columns of the halves, for A in the first and for B in the second: where a row has as many values these columns
+// meet zeros of the other operand (28 to 32 components of 7 values are 196 to 224 of 256).
+constexpr uint32_t kUnitCols = 64, kUnits = 7, kUnitsStep = 8;  // columns of an accumulator; accumulators; units of a step
+constexpr uint32_t kRowsAt = kUnits * kUnitCols, kRowsCols = 32, kScaleCols = 4;
+constexpr uint32_t kScalesAt = kRowsAt + kRowsCols - kScaleCols;
+constexpr uint32_t kScaleOne = 0x7f7f7f7fu;
+static_assert(kRowsAt + 2 * kRowsCols == kTmemCols, "tensor memory");
+constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kUnitCols >> 3) << 17) | (1u << 23) | (uint32_t(128 >> 7) << 27);
 
-__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a, uint64_t b, bool accumulate) {
+__device__ __forceinline__ void mma_f4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t scales, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(kIdesc), "r"(uint32_t(accumulate))
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b), "r"(kIdesc), "r"(scales), "r"(scales + kRowsCols), "r"(uint32_t(accumulate))
         : "memory");
 }
-// 32 fp16 columns of the warp's 32 lanes of tensor memory, two neighbours per register: asked for, and waited for
-__device__ __forceinline__ void tmem_load32(uint32_t (&r)[16], uint32_t addr) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.pack::16b.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(addr)
-                 : "memory");
+// 32 columns of the warp's 32 lanes of tensor memory: asked for, and waited for
+__device__ __forceinline__ void tmem_load32(uint32_t (&r)[32], uint32_t addr) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
+        "%21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(addr)
+        : "memory");
 }
 // (the registers are operands so that no use of them moves in front of the wait)
-__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]),
-                   "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-                 :
-                 : "memory");
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[32], uint32_t (&q)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(r[i]), "+r"(q[i]));
+}
+__device__ __forceinline__ void tmem_store4(uint32_t addr, const uint4& v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ int largest(const uint32_t (&v)[32]) {
+    int m[12];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) m[i] = __vimax3_s32(int(v[3 * i]), int(v[3 * i + 1]), int(v[3 * i + 2]));
+    m[10] = int(v[30]), m[11] = int(v[31]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m[i] = __vimax3_s32(m[3 * i], m[3 * i + 1], m[3 * i + 2]);
+    return __vimax3_s32(m[0], m[1], max(m[2], m[3]));
 }
 
 // ---- which tiles meet ------------------------------------------------------------------------------------------------
@@ -533,6 +561,7 @@ struct Phase {
 // time and a tile comes from L2; then its part of the steps of the row tiles left over.
 struct Walk {
     uint32_t len, whole, rt, at;  // steps of a row tile; whole row tiles to come; row tile and step
+    uint32_t col;                 // the step's column (at, or at * hop % len)
     uint32_t steps, apart;        // of the block; rows between its whole row tiles
     uint32_t rest_rt, rest_at;    // where its part of the rest begins
     uint32_t hop;                 // the rest goes round a row tile's columns by this many: neighbouring columns are far apart
@@ -561,15 +590,25 @@ struct Walk {
                 }
             }
         }
+        col = column(0);
     }
-    __device__ bool last() const { return at + 1 == len; }
-    __device__ uint32_t step() const { return whole ? at : uint32_t(uint64_t(at) * hop % len); }
     __device__ void next() {
-        if (++at < len) return;
+        if (++at < len) {
+            col += whole ? 1 : hop;
+            if (col >= len) col -= len;
+        } else {
+            next_rows();
+        }
+    }
+    // by row tiles: the steps until it changes, their columns, and the change
+    __device__ uint32_t run() const { return len - at; }
+    __device__ uint32_t column(uint32_t ahead) const { return whole ? at + ahead : uint32_t(uint64_t(at + ahead) * hop % len); }
+    __device__ void next_rows() {
         at = 0;
         if (whole && --whole) rt += apart;
         else if (whole == 0 && rt >= rest_rt) ++rt;
         else rt = rest_rt, at = rest_at;
+        col = column(0);
     }
 };
 
@@ -596,11 +635,12 @@ struct KnnMmaArgs {
     Calm calm;
 };
 
-// The dot product a pair at distance <= t reaches at least, as the bits of its half: above zero halves compare as their bits
-// do, and those below zero are below; where zero or less is enough every product will do.  t < 0: none does.
+// The dot product a pair at distance <= t reaches at least, as the upper half of its float's bits (the lower is zero, dot
+// products are 224 at most): above zero floats compare as their bits do, and those below zero are below; where zero or less
+// is enough every product will do.  t < 0: none does.
 __device__ __forceinline__ int gate_of(int symbols, int K, int t) {
     const int dot = symbols * (K - t) - K;
-    return t < 0 ? 0x7fff : (dot > 0 ? int(__half_as_ushort(__float2half_rn(float(dot)))) : -0x8000);
+    return t < 0 ? 0x7fff : (dot > 0 ? int(__float_as_uint(float(dot)) >> 16) : -0x8000);
 }
 
 // The entries of a row's buffer: (distance, node), packed in a word up to kPackedNodes nodes, in two above.
@@ -744,12 +784,95 @@ __global__ void __launch_bounds__(kCheckWarps * 32) knn_check_kernel(KnnMmaArgs 
     }
 }
 
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// The products of a block's steps, KSTEPS of 64 values of K each, by two warps: the first has the even units and four of the
+// accumulators, the second the odd units and three.  (A warp only waits for units of its own: the other's barriers could be two
+// phases on.)  The whole warp goes along and one lane issues: descriptors then stay in uniform registers.  (One thread in a
+// branch of its own took 270 cycles a product, which takes 32.)  A unit of four products takes 128 cycles, so what lies between
+// them counts: a wait that is over is one poll and a vote.
+template <int KSTEPS>
+__device__ __forceinline__ bool issue_products(const KnnMmaArgs& a, Walk walk, uint32_t steps, uint32_t first, uint32_t tmem, uint32_t smem,
+                                               uint32_t operand_bytes, uint32_t elected, uint64_t* full_bar, uint64_t* empty_bar, uint64_t* tfull_bar,
+                                               uint64_t* tempty_bar, uint64_t* rows_bar, uint64_t* done_bar, volatile int* aborted) {
+    auto wait = [&](bool over, uint64_t* bar, uint32_t parity, uint32_t limit) {
+        return __all_sync(kFull, over) || __all_sync(kFull, wait_or_abort(bar, parity, limit, aborted));
+    };
+    // the unit that had the accumulator of unit 2 v + first of step i was read: the same of the step before, or the second warp's
+    // third before
+    auto emptied = [&](uint32_t v, uint32_t i, uint64_t*& bar, uint32_t& parity) {
+        bar = &tempty_bar[first ? (v == 3 ? 1 : 2 * v + 3) : 2 * v];
+        parity = (first && v == 3 ? i : i + 1) & 1;
+    };
+    constexpr uint64_t kStep = (2 * kMmaRows * 16) >> 4;  // two 16-byte chunks of 256 rows
+    const uint64_t b_desc = operand_desc(smem);
+    const uint32_t stages = uint32_t(a.stages);
+    uint32_t stage = 0, parity = 0, rows_parity = 0, turn = 0;  // turn: among the second warp's accumulators
+    uint32_t left = walk.run();
+    bool fresh = true;  // of a new row tile
+    bool full = false, empty = true;  // what the polls said (a step's first waits, of a barrier that nothing has used, are over)
+    uint64_t* bar;
+    uint32_t of;
+    for (uint32_t i = 0; i < steps; ++i) {
+        if (!wait(full, &full_bar[stage], parity, i == 0 ? a.first_wait_polls : kWaitLimit)) return false;
+        if (fresh) {
+            if (!wait(false, rows_bar, rows_parity, kWaitLimit)) return false;
+            rows_parity ^= 1;
+        }
+        fresh = --left == 0;
+        if (fresh) {
+            walk.next_rows();
+            left = walk.run();
+        }
+        const uint64_t tile = b_desc + (stage * operand_bytes >> 4);
+        uint64_t* const done_with = &empty_bar[stage];
+        if (++stage == stages) stage = 0, parity ^= 1;
+#pragma unroll
+        for (uint32_t v = 0; v < 4; ++v) {  // halves of the rows by quarters of the columns
+            const uint32_t u = 2 * v + first;
+            emptied(v, i, bar, of);
+            if (!wait(empty, bar, of, kWaitLimit)) return false;
+            // the next waits are polled before this unit's products are issued, which hides their latency
+            if (v == 3) full = mbar_test(&full_bar[stage], parity);
+            emptied((v + 1) & 3, v == 3 ? i + 1 : i, bar, of);
+            empty = mbar_test(bar, of);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elected) {
+                const uint32_t at = first ? 4 + turn : v;
+#pragma unroll
+                for (int ks = 0; ks < KSTEPS; ++ks)
+                    mma_f4(tmem + at * kUnitCols, tmem + kRowsAt + (v >> 1) * kRowsCols + ks * 8, tile + (u & 3) * ((kUnitCols * 16) >> 4) + ks * kStep,
+                           tmem + kScalesAt, ks != 0);
+                mma_commit(&tfull_bar[u]);
+                if (v == 3) {
+                    mma_commit(done_with);
+                    if (fresh) mma_commit(done_bar);
+                }
+            }
+            __syncwarp();
+            if (++turn == 3) turn = 0;
+        }
+    }
+    return true;
+}
+
 template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     if (a.choice.skip()) return;
     extern __shared__ __align__(1024) unsigned char mma_smem[];
     __shared__ __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages];
-    __shared__ __align__(8) uint64_t tfull_bar[2][2], tempty_bar[2][2];  // [half of the rows][side]
+    // of a step's units, not of the accumulators: who waits is then a phase behind at most
+    __shared__ __align__(8) uint64_t tfull_bar[kUnitsStep], tempty_bar[kUnitsStep];
+    __shared__ __align__(8) uint64_t rows_bar, done_bar;  // a row tile's rows are in tensor memory; its last products are through
     __shared__ __align__(8) uint64_t drain_bar;
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
@@ -758,25 +881,21 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     const Phase phase = calm && a.when == KnnMmaArgs::kAllIfCalm ? Phase{a.phase.base, 1u, false, 0u, a.meet.columns() - a.phase.base} : a.phase;
     const int lane = threadIdx.x & 31, warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
     const uint32_t operand_bytes = uint32_t(a.chunks) * kMmaRows * 16;
-    const int ksteps = a.chunks / 2, split_k = (ksteps + 1) / 2;  // 32 values of K a step: two 16-byte chunks
-    constexpr uint32_t kStepBytes = 2 * kMmaRows * 16;
-    const uint32_t stage_bytes = uint32_t(split_k) * kStepBytes;  // half of a tile along K: part 0, and part 1 at most as long
-    unsigned char* a_sm = mma_smem;
-    unsigned char* b_sm = mma_smem + operand_bytes;
     Walk walk(a.meet.row_tiles, phase.count);
     const uint32_t steps = walk.steps;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i)
-            for (int j = 0; j < 2; ++j) {
-                knn::mbar_init(&tfull_bar[i][j], 1);
-                knn::mbar_init(&tempty_bar[i][j], 4);
-            }
+        for (uint32_t i = 0; i < kUnitsStep; ++i) {
+            knn::mbar_init(&tfull_bar[i], 1);
+            knn::mbar_init(&tempty_bar[i], 4);
+        }
         for (int i = 0; i < kMaxStages; ++i) {
             knn::mbar_init(&full_bar[i], 1);
-            knn::mbar_init(&empty_bar[i], 1);
+            knn::mbar_init(&empty_bar[i], kMmaWarps);
         }
-        knn::mbar_init(&drain_bar, 1);
+        knn::mbar_init(&rows_bar, kEpiWarps);
+        knn::mbar_init(&done_bar, kMmaWarps);
+        knn::mbar_init(&drain_bar, kMmaWarps);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -790,142 +909,142 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     const uint32_t tmem = tmem_base_sm;
     volatile int* aborted = &abort_flag;
 
-    uint32_t loads = 0;  // parts whose copies this warp has issued
+    uint32_t loads = 0;  // tiles whose copies this warp has issued
     if (warp == kEpiWarps) {
         if (lane == 0) {
-            uint32_t stage = 0, parity = 0;                      // parity: of the stage's next filling
-            bool fresh = true, ok = true;                       // fresh: the row tile's own operand has to come too
+            uint32_t stage = 0, parity = 0;  // parity: of the stage's next filling
+            bool ok = true;
             const unsigned char* op = reinterpret_cast<const unsigned char*>(a.operand);
-            for (uint32_t i = 0; i < steps && ok && !*aborted; ++i) {
-                const uint32_t ct = a.meet.column(walk.rt, phase.column(walk.step()));
-                // a new row operand replaces the one that the products of the step before still read
-                if (fresh && i) {
-                    const uint32_t before = stage ? stage - 1 : uint32_t(a.stages) - 1;
-                    ok = wait_or_abort(&empty_bar[before], stage ? parity : parity ^ 1, kWaitLimit, aborted);
-                }
-                for (int part = 0; part < 2 && ok; ++part) {
-                    const uint32_t from = part ? stage_bytes : 0u;
-                    const uint32_t bytes = part ? operand_bytes - stage_bytes : stage_bytes;
-                    ok = wait_or_abort(&empty_bar[stage], parity ^ 1, a.handover_polls, aborted);  // handed back by the products
-                    if (!ok) break;
-                    const uint32_t own = fresh && part == 0 ? operand_bytes : 0u;
-                    knn::mbar_expect_tx(&full_bar[stage], bytes + own);
-                    if (own) knn::bulk_g2s(a_sm, op + size_t(walk.rt) * operand_bytes, own, &full_bar[stage]);
-                    if (bytes) knn::bulk_g2s(b_sm + stage * stage_bytes, op + size_t(ct) * operand_bytes + from, bytes, &full_bar[stage]);
-                    ++loads;
-                    if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
-                }
-                const uint32_t rt = walk.rt;
+            for (uint32_t i = 0; i < steps && !*aborted; ++i) {
+                const uint32_t ct = a.meet.column(walk.rt, phase.column(walk.col));
+                ok = wait_or_abort(&empty_bar[stage], parity ^ 1, a.handover_polls, aborted);  // handed back by the products
+                if (!ok) break;
+                knn::mbar_expect_tx(&full_bar[stage], operand_bytes);
+                knn::bulk_g2s(mma_smem + stage * operand_bytes, op + size_t(ct) * operand_bytes, operand_bytes, &full_bar[stage]);
+                ++loads;
+                if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
                 walk.next();
-                fresh = walk.rt != rt;
             }
             if (!ok) *aborted = 1;
         }
-    } else if (warp == kEpiWarps + 1) {
-        // The whole warp goes along and one lane issues: descriptors then stay in uniform registers.  (One thread in a
-        // branch of its own took 270 cycles a product, twice what the product does.)
+    } else if (warp > kEpiWarps) {
         const uint32_t elected = elect_one();
-        const uint64_t a_desc = operand_desc(smem_u32(a_sm)), b_desc = operand_desc(smem_u32(b_sm));
-        constexpr uint64_t kStep = kStepBytes >> 4;
-        uint32_t stage = 0, parity = 0;
-        bool ok = true;
-        for (uint32_t i = 0; i < steps && ok; ++i) {
-            const uint32_t side = i & 1, st0 = stage, par0 = parity;
-            if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
-            const uint32_t st1 = stage, par1 = parity;
-            if (++stage == uint32_t(a.stages)) stage = 0, parity ^= 1;
-            ok = __all_sync(kFull, wait_or_abort(&full_bar[st0], par0, i == 0 ? a.first_wait_polls : kWaitLimit, aborted) && !*aborted);
-            for (int h = 0; h < 2 && ok; ++h) {
-                // the half was read for the step before by the other side
-                if (i) ok = __all_sync(kFull, wait_or_abort(&tempty_bar[h][side ^ 1], ((i - 1) >> 1) & 1, kWaitLimit, aborted));
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + h * 256;
-                uint64_t ad = a_desc + h * ((128 * 16) >> 4), bd = b_desc + (st0 * stage_bytes >> 4);
-                if (elected) {
-#pragma unroll 4
-                    for (int ks = 0; ks < split_k; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, ks != 0);
-                    if (h == 1) mma_commit(&empty_bar[st0]);
-                }
-                if (h == 0) {
-                    ok = __all_sync(kFull, wait_or_abort(&full_bar[st1], par1, kWaitLimit, aborted));
-                    if (!ok) break;
-                }
-                ad = a_desc + h * ((128 * 16) >> 4) + split_k * kStep, bd = b_desc + (st1 * stage_bytes >> 4);
-                if (elected) {
-#pragma unroll 4
-                    for (int ks = split_k; ks < ksteps; ++ks, ad += kStep, bd += kStep) mma_f8(d, ad, bd, true);
-                    mma_commit(&tfull_bar[h][side]);
-                    if (h == 1) mma_commit(&empty_bar[st1]);
-                }
-            }
+        auto issue = [&](auto ksteps) {
+            return issue_products<decltype(ksteps)::value>(a, walk, steps, uint32_t(warp - kEpiWarps - 1), tmem, smem_u32(mma_smem), operand_bytes, elected, full_bar, empty_bar, tfull_bar,
+                                                           tempty_bar, &rows_bar, &done_bar, aborted);
+        };
+        bool ok = false;
+        switch (a.chunks) {
+            case 2: ok = issue(std::integral_constant<int, 1>()); break;
+            case 4: ok = issue(std::integral_constant<int, 2>()); break;
+            case 6: ok = issue(std::integral_constant<int, 3>()); break;
+            default: ok = issue(std::integral_constant<int, 4>()); break;
         }
         if (!ok) *aborted = 1;
         if (elected) mma_commit(&drain_bar);  // everything issued above has finished when this completes
     } else {
-        const int quarter = warp & 3, half = (warp >> 2) & 1, side = warp >> 3;
-        const uint32_t base = uint32_t(half * 128 + quarter * 32);  // the warp's rows in the tile
-        const uint32_t addr = tmem + (uint32_t(quarter * 32) << 16) + half * 256;
-        uint32_t row0 = 0;  // the warp's first row
-        uint2 row = make_uint2(kInvalidNode, ~0u);
-        bool ok = true, begun = false;  // begun: this side has had a step of the row tile
-        for (uint32_t i = 0; i < steps; ++i) {
-            const uint32_t rt = walk.rt, ct = a.meet.column(rt, phase.column(walk.step()));
-            const bool last = walk.last() || i + 1 == steps;  // of the row tile
-            walk.next();
-            if ((i & 1) == uint32_t(side)) {
-                if (!begun) {
-                    begun = true;
-                    row0 = rt * kMmaRows + base;
-                    row = __ldg(a.place + row0 + lane);
-                }
-                // a pair is of use at the row's limit or at its column's, of which the largest of 32 stands for all at first
-                const bool both = a.meet.both(rt, ct);
-                const int least = gate_of(a.symbols, a.K, int(row.y));
-                uint4 gates = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
-                if (both) gates = __ldg(reinterpret_cast<const uint4*>(a.gate) + ct);
-                ok = wait_or_abort(&tfull_bar[half][side], (i >> 1) & 1, kWaitLimit, aborted);
-                if (__ballot_sync(kFull, !ok || *aborted)) {
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                // the largest product of every 32 columns; one load is in flight while the columns of the one before are looked at
-                uint32_t r[2][16], hit = 0;
-                tmem_load32(r[0], addr);
+        const uint32_t quarter = warp & 3, cols = warp >> 2;  // of the lanes, of the columns
+        const uint32_t addr = tmem + ((quarter * 32) << 16);
+        // a part of a row tile's rows to tensor memory: the quarter of the first or second half, half of their chunks
+        const uint32_t each = uint32_t(a.chunks) / 2, from = (cols >> 1) * each;
+        auto put_rows = [&](uint32_t rt, bool again, uint32_t done_parity) {
+            const uint4* src = a.operand + (size_t(rt) * a.chunks + from) * kMmaRows + (cols & 1) * 128 + quarter * 32 + lane;
+            uint4 v[kRowsCols / 8];
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
-                    uint32_t (&v)[16] = r[g & 1];
-                    tmem_wait(v);
-                    if (g < 7) tmem_load32(r[(g + 1) & 1], addr + (g + 1) * 32);
-                    const uint32_t m0 = __vimax3_s16x2(v[0], v[1], v[2]), m1 = __vimax3_s16x2(v[3], v[4], v[5]);
-                    const uint32_t m2 = __vimax3_s16x2(v[6], v[7], v[8]), m3 = __vimax3_s16x2(v[9], v[10], v[11]);
-                    const uint32_t m4 = __vimax3_s16x2(v[12], v[13], v[14]);
-                    const uint32_t m = __vimax3_s16x2(__vimax3_s16x2(m0, m1, m2), __vimax3_s16x2(m3, m4, v[15]), 0x80008000u);
-                    const uint32_t pair = g < 4 ? (g < 2 ? gates.x : gates.y) : (g < 6 ? gates.z : gates.w);
-                    const int gate = min(least, g & 1 ? int(pair) >> 16 : int(int16_t(pair)));
-                    hit |= max(int(int16_t(m)), int(m) >> 16) >= gate ? 1u << g : 0u;
-                }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty_bar[half][side]);
-
-                uint32_t any_hit = __reduce_or_sync(kFull, hit);
-                if (any_hit) {  // listed; where there is no room, compared at once
-                    uint32_t at = 0;
-                    if (lane == 0) at = atomicAdd(a.hit_count, uint32_t(__popc(any_hit)));
-                    at = __shfl_sync(kFull, at, 0);
-                    for (; any_hit; any_hit &= any_hit - 1, ++at) {
-                        const int g = __ffs(any_hit) - 1;
-                        const uint32_t rows = __ballot_sync(kFull, hit >> g & 1u), col0 = ct * kMmaRows + g * 32;
-                        if (at >= a.hit_room) compare_rows<U16, QUADS>(a, rows, row0, row, col0, both, lane);
-                        else if (lane == 0) a.hits[at] = make_uint4(row0, col0, rows, both ? 1u : 0u);
-                    }
-                    __syncwarp();
-                }
+            for (uint32_t c = 0; c < kRowsCols / 8; ++c)
+                if (c < each) v[c] = __ldg(src + c * kMmaRows);
+            if (again && !__all_sync(kFull, wait_or_abort(&done_bar, done_parity, kWaitLimit, aborted))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (uint32_t c = 0; c < kRowsCols / 8; ++c)
+                if (c < each && from + c < (kRowsCols - kScaleCols) / 4) tmem_store4(addr + kRowsAt + (cols & 1) * kRowsCols + (from + c) * 4, v[c]);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&rows_bar);
+            return true;
+        };
+        if (cols < 2 && steps) tmem_store4(addr + kScalesAt + cols * kRowsCols, make_uint4(kScaleOne, kScaleOne, kScaleOne, kScaleOne));
+        // the accumulators of the step's two units: two of the first warp's four, or those whose turn it is of the second's three
+        uint32_t at0 = cols / 2, at1 = cols / 2 + 2, done_parity = 0;
+        if (cols & 1) at0 += 4, at1 = at0 == 4 ? 6 : at0 - 1;
+        // The last hits found: of the rows from `first` on and from 128 places on, with 32 columns from `col` on (its lowest bit:
+        // both) and the 32 after them.  They are listed when the next are found, or at the end: the place in the list then has come
+        // (waiting for it took as long as a step), and a step's take one atomic (100k x 960, two bytes: two a step 643 us, 539 so).
+        uint32_t found[4] = {0u, 0u, 0u, 0u}, first = 0, col = 0, to = 0;
+        auto list_hits = [&]() {
+            to = __shfl_sync(kFull, to, 0);
+#pragma unroll 1
+            for (uint32_t g = 0; g < 4; ++g) {
+                const uint32_t rows = g < 2 ? (g ? found[1] : found[0]) : (g == 2 ? found[2] : found[3]);
+                if (rows == 0) continue;
+                const uint32_t from_row = first + (g >> 1) * 128, from_col = (col & ~1u) + (g & 1) * 32;
+                if (lane == 0 && to < a.hit_room) a.hits[to] = make_uint4(from_row, from_col, rows, col & 1u);
+                if (to >= a.hit_room) compare_rows<U16, QUADS>(a, rows, from_row, __ldg(a.place + from_row + lane), from_col, col & 1u, lane);
+                ++to;
             }
-            if (last) begun = false;
+            __syncwarp();
+        };
+        bool ok = true;
+        for (uint32_t i = 0; i < steps && ok; walk.next_rows()) {
+            const uint32_t rt = walk.rt, row0 = rt * kMmaRows + quarter * 32, run = min(walk.run(), steps - i);
+            ok = put_rows(rt, i != 0, done_parity);
+            if (i) done_parity ^= 1;
+            // what a product reaches at the limit of the lane's row of either half, in the upper half
+            const int least0 = gate_of(a.symbols, a.K, int(__ldg(a.place + row0 + lane).y)) << 16;
+            const int least1 = gate_of(a.symbols, a.K, int(__ldg(a.place + row0 + 128 + lane).y)) << 16;
+            // 32 steps' column tiles and what reaches the largest limit of their columns, a step a lane and asked for 32 ahead: a
+            // pair is of use at the row's limit or at its column's, of which the largest of 32 stands for all at first
+            uint32_t tile = 0, gates = 0, next_tile, next_gates;
+            auto look_ahead = [&](uint32_t b) {
+                next_tile = a.meet.column(rt, phase.column(walk.column(min(b + lane, run - 1))));
+                next_gates = a.meet.both(rt, next_tile) ? __ldg(reinterpret_cast<const uint32_t*>(a.gate) + next_tile * 4 + cols) : 0x7fff7fffu;
+            };
+            look_ahead(0);
+            for (uint32_t s = 0; s < run && ok; ++s, ++i) {
+                if (s % 32 == 0) {
+                    tile = next_tile, gates = next_gates;
+                    if (s + 32 < run) look_ahead(s + 32);
+                }
+                const uint32_t pair = __shfl_sync(kFull, gates, s % 32);
+                const int gate0 = int(pair << 16), gate1 = int(pair & 0xffff0000u);
+                uint32_t rows[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    const uint32_t u = 4 * h + cols;
+                    if (!__all_sync(kFull, knn::mbar_try_wait(&tfull_bar[u], i & 1)) &&
+                        !__all_sync(kFull, wait_or_abort(&tfull_bar[u], i & 1, kWaitLimit, aborted))) {
+                        ok = false;
+                        break;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    uint32_t r[2][32];
+                    const uint32_t from_col = addr + (h ? at1 : at0) * kUnitCols;
+                    tmem_load32(r[0], from_col);
+                    tmem_load32(r[1], from_col + 32);
+                    tmem_wait(r[0], r[1]);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty_bar[u]);
+                    // the largest product of every 32 columns
+                    const int least = h ? least1 : least0;
+                    const bool hit0 = largest(r[0]) >= min(least, gate0), hit1 = largest(r[1]) >= min(least, gate1);
+                    rows[2 * h] = __ballot_sync(kFull, hit0);
+                    rows[2 * h + 1] = __ballot_sync(kFull, hit1);
+                }
+                if (rows[0] | rows[1] | rows[2] | rows[3]) {
+                    list_hits();
+                    uint32_t many = 0;
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) found[g] = rows[g], many += rows[g] != 0;
+                    const uint32_t ct = __shfl_sync(kFull, tile, s % 32);
+                    first = row0, col = (ct * kMmaRows + cols * kUnitCols) | (a.meet.both(rt, ct) ? 1u : 0u);
+                    if (lane == 0) to = atomicAdd(a.hit_count, many);
+                }
+                if (cols & 1) at1 = at0, at0 = at0 == 6 ? 4 : at0 + 1;
+            }
         }
+        list_hits();
         if (!ok) *aborted = 1;
     }
     __syncthreads();
@@ -1500,8 +1619,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.K = int(h->K);
     a.symbols = shape.symbols;
     a.chunks = shape.chunks;
-    const uint32_t stage_bytes = uint32_t(shape.chunks / 2 + 1) / 2 * 2 * kMmaRows * 16;
-    a.stages = int((kMmaSmem - operand_bytes) / stage_bytes);
+    a.stages = int(kMmaSmem / operand_bytes);
     if (a.stages > kMaxStages) a.stages = kMaxStages;
     a.k = k;
     a.entries = entries;
@@ -1592,7 +1710,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             const uint64_t steps = uint64_t(a.meet.row_tiles) * count;
             if (!first) CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
             first = false;
-            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, operand_bytes + a.stages * stage_bytes, st>>>(a);
+            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, a.stages * operand_bytes, st>>>(a);
             knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
             h->launches += 2;
             return 0;
@@ -1659,7 +1777,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
 
 }  // namespace
 
-// Plain K-component codes of up to 64 components (the operand of 256 rows has to fit shared memory twice).
+// Plain K-component codes of up to 64 components (four steps of 64 values: a half of the rows has 32 columns of tensor memory).
 bool knn_mma_supported(const cphnsw_b200_index* h) {
     return !h->binary_codes && !h->residual_bits && h->K >= 2 && hash_shape(int(h->K)).symbols != 0;
 }

@@ -74,6 +74,19 @@ def test_many_clusters_against_the_bit_sliced_kernel(cp):
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
 
 
+# the operand's length turns (64 values a step; 28 components are the first whose rows share tensor memory with the scales), in
+# 149 row tiles: a full wave of blocks, and one row tile that all of them share
+@pytest.mark.parametrize("K", [9, 10, 18, 19, 27, 28, 31, 42, 43, 64])
+def test_operand_lengths(cp, K):
+    base, _ = synthetic.gaussian_mixture(38_100, 1, 96, 38, 0.3, K)
+    idx = index(cp, 96, K, 1)
+    codes = idx.encode(base)
+    a = idx.knn_graph(codes, 40)
+    idx.set_param("knn_kernel", 1)
+    b = idx.knn_graph(codes, 40)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
 @pytest.mark.parametrize("K,cb", [(32, 1), (32, 2)])
 def test_codes_off_a_sector_boundary(cp, oracle, K, cb):
     # 16-byte aligned device codes are read by 16 bytes, 32-byte aligned ones by 32
