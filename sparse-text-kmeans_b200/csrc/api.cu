@@ -73,16 +73,16 @@ int upload_signs(cphnsw_b200_index* h) {
     CPB_CUDA(cudaMemcpy(h->d_signs.p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
     if (P == 256 || P == 512 || P == 1024) {
         // bit-packed copy for the kernels with a warp per vector (a set bit negates): word w, bit b <-> element
-        // P/32 * w + b; at 1024 layers 1 and 2 in the column layout, word l, bit j <-> element 32*j + l
+        // P/32 * w + b; at 1024 word w, bit b <-> the element that lane w has in register b where the layer begins
         const size_t E = P / 32;
         std::vector<uint32_t> bits(K * (kWarpSignWords + (P < 1024 ? 3 * P / 32 : 0)), 0u);
+        std::vector<uint32_t> element(3 * P);  // of a layer's (word, bit)
+        for (size_t l = 0; l < 3; ++l)
+            for (size_t i = 0; i < P; ++i) element[l * P + i] = P == 1024 ? p1024_element(int(l), int(i / E), int(i % E)) : uint32_t(i);
         for (size_t r = 0; r < K; ++r)
             for (size_t l = 0; l < 3; ++l)
                 for (size_t i = 0; i < P; ++i)
-                    if (f[(r * 3 + l) * P + i] < 0.0f) {
-                        if (l == 0 || P != 1024) bits[(r * 3 + l) * 32 + i / E] |= 1u << (i % E);
-                        else bits[(r * 3 + l) * 32 + i % 32] |= 1u << (i / 32);
-                    }
+                    if (f[(r * 3 + l) * P + element[l * P + i]] < 0.0f) bits[(r * 3 + l) * 32 + i / E] |= 1u << (i % E);
         // behind it the copy for groups of P/128 lanes per vector, four words a lane and layer in the order of the lane's
         // registers: the element of register e has e's low bits and, of the next bits and the top ones, the lane's index
         // and the rest of e XOR the lane's index (layer 0: the lane's index on top)

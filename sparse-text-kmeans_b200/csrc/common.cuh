@@ -240,6 +240,8 @@ namespace cpb {
 int code_row_words(uint32_t K, uint32_t comp_bytes);
 
 // ---- launchers (each returns 0 or a negative status and counts its launches in h) ----
+// padded dim 1024: the element that a lane has in a register where a layer of the transform begins
+uint32_t p1024_element(int layer, int lane, int reg);
 int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_codes, float* d_rot,
                   float* d_mag, cudaStream_t st);
 int launch_code_distance(cphnsw_b200_index* h, const void* d_a, uint64_t na, const void* d_b,

@@ -22,7 +22,7 @@
 //                        low stages in registers, high stages by shuffles.
 //   encode_group_kernel  padded dims 256 and 512, many vectors: 2 or 4 lanes own one vector, 128 elements each; the stages
 //                        across lanes become register stages after an exchange.
-//   encode_p1024_kernel  padded dim 1024: one warp per vector, transposes through shared memory between two layouts.
+//   encode_p1024_kernel  padded dim 1024: one warp per vector, register and lane bits change places through tensor memory.
 //   encode_generic_kernel any other power-of-two padded dim: one warp owns one vector in shared memory.
 #include "common.cuh"
 
@@ -262,128 +262,186 @@ encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, in
 }
 
 // ---- padded dim 1024 (d in 513..1024): one warp per vector, 32 elements per lane -------------------
-// The 10 stages of a 1024-point transform are done as two register passes of a 32-point transform:
-// stages h = 1..16 with the lane holding 32 consecutive elements (i = 32*lane + j), stages
-// h = 32..512 with the lane holding a stride-32 column (i = 32*j + lane), and a transpose through a
-// padded 32x33 shared-memory tile between the two layouts.  The stage order h = 1, 2, 4, ... and
-// the butterfly (lo = x + y, hi = x - y, x the lower index) are the reference's, so the result is
-// bit-identical.  The diagonals come bit-packed in the layout they are applied in (a set bit
-// negates), one word per lane and layer.
+// Five of an element's ten index bits are the register's, five the lane's, and a stage pairs registers, so bits have to
+// change places as the stages go up.  They do by way of tensor memory: what a warp stores in one shape (16 lanes by 128 bits,
+// eight such side by side, twice) it loads in another (32 lanes by 32 bits).  The lane that stores register r = R4 .. R0 (bits)
+// with p4 .. p0 its own index puts it at lane R4 R0 p4 p3 p2 and column R3 R2 R1 p1 p0, and the one that loads has lane and
+// column for lane and register: two of the lane's bits come to the registers, two of the registers' go to the lanes.
+//   The vector starts with bits 0 1 8 5 2 as R0 .. R4 and 3 4 6 7 9 as p0 .. p4.  Stages 0, 1, 2 are those of R0, R1, R4; a
+// change leaves bits 3 4 1 8 5 and 6 7 9 0 2, so the next three are again those of R0, R1, R4, and so on (all bits three up,
+// modulo ten): 30 stages of three layers take nine changes.  Stage order and butterfly (lo = x + y, hi = x - y, x the lower
+// index) are the reference's, so the result is bit-identical.  The diagonals come bit-packed in the order a layer finds the
+// elements in (a set bit negates), one word per lane and layer.
+//   What bounds it is the add pipe (0.61 of it) and the instructions beside: without the changes of places it would take 0.84 of
+// its time, without two of the three diagonals 0.9, without the search for the argmax 0.93.  With transposes through shared
+// memory, five of 64 wavefronts each a vector and rotation, these were the bound: 100k x 960, K = 32, 5,340 us; 4,390 now.
 constexpr int kP1024 = 1024;
 constexpr int kWarps1024 = 4;
+constexpr int kBlocks1024 = 4;  // resident on an SM (five of 96 registers spill: 4,480 us)
+constexpr uint32_t kTmemCols1024 = 32;
 
-__device__ __forceinline__ void fht32_regs(float (&v)[32]) {
-    f32x2 p[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-        const float x = v[2 * j], y = v[2 * j + 1];
-        p[j] = pack2(__fadd_rn(x, y), __fsub_rn(x, y));
-    }
-    butterfly_pairs<1>(p);
-    butterfly_pairs<2>(p);
-    butterfly_pairs<4>(p);
-    butterfly_pairs<8>(p);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) unpack2(p[j], v[2 * j], v[2 * j + 1]);
+// the bit of an element's index that position `at` (R0 .. R4, p0 .. p4) holds after `changes` changes of places
+__host__ __device__ constexpr int index_bit(int at, int changes) {
+    const int first[10] = {0, 1, 8, 5, 2, 3, 4, 6, 7, 9};
+    return (first[at] + 3 * changes) % 10;
+}
+__host__ __device__ constexpr int index_part(int value, int from, int changes) {  // of a register's number (from = 0), of a lane's (5)
+    int i = 0;
+    for (int b = 0; b < 5; ++b)
+        if (value >> b & 1) i |= 1 << index_bit(from + b, changes);
+    return i;
 }
 
-__device__ __forceinline__ void flip_signs32(float (&v)[32], uint32_t word) {
+__device__ __forceinline__ void change_places(f32x2 (&p)[16], uint32_t tmem) {
+    float v[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-        v[j] = __int_as_float(__float_as_int(v[j]) ^ int((word << (31 - j)) & 0x80000000u));
+    for (int j = 0; j < 16; ++j) unpack2(p[j], v[2 * j], v[2 * j + 1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        asm volatile("tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(
+                         tmem + (uint32_t(h * 16) << 16)),
+                     "f"(v[16 * h]), "f"(v[16 * h + 1]), "f"(v[16 * h + 2]), "f"(v[16 * h + 3]), "f"(v[16 * h + 4]), "f"(v[16 * h + 5]), "f"(v[16 * h + 6]),
+                     "f"(v[16 * h + 7]), "f"(v[16 * h + 8]), "f"(v[16 * h + 9]), "f"(v[16 * h + 10]), "f"(v[16 * h + 11]), "f"(v[16 * h + 12]),
+                     "f"(v[16 * h + 13]), "f"(v[16 * h + 14]), "f"(v[16 * h + 15])
+                     : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, "
+        "%21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]),
+          "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]),
+          "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(tmem)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {  // (no use of them moves in front of the wait)
+        asm volatile("" : "+f"(v[2 * j]), "+f"(v[2 * j + 1]));
+        p[j] = pack2(v[2 * j], v[2 * j + 1]);
+    }
+}
+// the stage of R0, the halves of a pair
+__device__ __forceinline__ void butterfly_halves(f32x2 (&p)[16]) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        float a, b;
+        unpack2(p[j], a, b);
+        p[j] = pack2(__fadd_rn(a, b), __fsub_rn(a, b));
+    }
+}
+__device__ __forceinline__ void flip_signs32(f32x2 (&p)[16], uint32_t word) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        float a, b;
+        unpack2(p[j], a, b);
+        a = __int_as_float(__float_as_int(a) ^ int((word << (31 - 2 * j)) & 0x80000000u));
+        b = __int_as_float(__float_as_int(b) ^ int((word << (30 - 2 * j)) & 0x80000000u));
+        p[j] = pack2(a, b);
+    }
 }
 
 template <typename CompT, bool QUERY>
-__global__ void __launch_bounds__(kWarps1024 * 32)
+__global__ void __launch_bounds__(kWarps1024 * 32, kBlocks1024)
 encode_p1024_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, int rpb,
                     const uint32_t* __restrict__ signbits /*[K][3][32]*/, int flip_mask,
                     CompT* __restrict__ codes, float* __restrict__ rotated, float* __restrict__ mags) {
-    __shared__ float tiles[kWarps1024][32 * 33];
+    __shared__ uint32_t tmem_base_sm;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* buf = tiles[warp];
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(uint32_t(__cvta_generic_to_shared(&tmem_base_sm))),
+                     "r"(kTmemCols1024)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_base_sm + (uint32_t(warp * 32) << 16);
     const bool vec4 = (dim % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
+    const int begins = index_part(lane, 5, 0);  // of the lane's elements, at first
     for (uint64_t row = uint64_t(blockIdx.x) * kWarps1024 + warp; row < n; row += uint64_t(gridDim.x) * kWarps1024) {
-        // the vector, zero-padded, in the consecutive layout: xin[j] = x[32*lane + j]
-        float xin[32];
+        // the vector, zero-padded; registers 4 c .. 4 c + 3 of a lane are neighbours (bits 0 and 1 of the index, and bits 8, 5, 2)
+        f32x2 in[16];
         const float* src = x + row * uint64_t(dim);
-        if (vec4) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                const int i = 32 * lane + 4 * c;
-                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c = 0; c < 8; ++c) {
+            const int i = begins + index_part(4 * c, 0, 0);
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (vec4) {
                 if (i < dim) q = __ldg(reinterpret_cast<const float4*>(src + i));
-                xin[4 * c] = q.x, xin[4 * c + 1] = q.y, xin[4 * c + 2] = q.z, xin[4 * c + 3] = q.w;
+            } else {
+                if (i < dim) q.x = __ldg(src + i);
+                if (i + 1 < dim) q.y = __ldg(src + i + 1);
+                if (i + 2 < dim) q.z = __ldg(src + i + 2);
+                if (i + 3 < dim) q.w = __ldg(src + i + 3);
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int i = 32 * lane + j;
-                xin[j] = i < dim ? __ldg(src + i) : 0.0f;
-            }
+            in[2 * c] = pack2(q.x, q.y), in[2 * c + 1] = pack2(q.z, q.w);
         }
         for (int r = blockIdx.y * rpb; r < min(K, int(blockIdx.y + 1) * rpb); ++r) {
-            const uint32_t* sb = signbits + size_t(r) * 3 * 32;
-            float v[32];
+            const uint32_t* sb = signbits + size_t(r) * 3 * 32 + lane;
+            const uint32_t word0 = __ldg(sb), word1 = __ldg(sb + 32), word2 = __ldg(sb + 64);
+            f32x2 v[16];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = xin[j];
-#pragma unroll 1
-            for (int layer = 0; layer < 3; ++layer) {
-                const uint32_t word = __ldg(sb + layer * 32 + lane);
-                flip_signs32(v, word);  // layer 0: consecutive layout; layers 1, 2: column layout
-                if (layer > 0) {        // column -> consecutive
-                    __syncwarp();
+            for (int j = 0; j < 16; ++j) v[j] = in[j];
+            flip_signs32(v, word0);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) buf[j * 33 + lane] = v[j];
-                    __syncwarp();
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = buf[lane * 33 + j];
-                }
-                fht32_regs(v);  // stages h = 1..16
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) buf[lane * 33 + j] = v[j];  // consecutive -> column
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = buf[j * 33 + lane];
-                fht32_regs(v);  // stages h = 32..512
+            for (int c = 0; c < 10; ++c) {  // stages 3 c, 3 c + 1, 3 c + 2 of 30; layers begin with the 10th and the 20th
+                if (c) change_places(v, tmem);
+                butterfly_halves(v);
+                if (c == 3) flip_signs32(v, word1);
+                butterfly_pairs<1>(v);
+                if (c == 6) flip_signs32(v, word2);
+                butterfly_pairs<8>(v);
             }
-            // column layout: v[j] is element 32*j + lane.  Lowest-index argmax of |v|.
+            // lowest-index argmax of |v|: the largest magnitude, then the first element that has it (from the last one down)
             float best = -1.0f, win = 0.0f;
             int idx = 0x7fffffff;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const float av = fabsf(v[j]);
-                if (av > best) {
-                    best = av;
-                    win = v[j];
-                    idx = 32 * j + lane;
-                }
+            for (int j = 0; j < 16; ++j) {
+                float a, b;
+                unpack2(v[j], a, b);
+                best = fmaxf(best, fmaxf(fabsf(a), fabsf(b)));
             }
+            best = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(best)));  // (none of them is above zero only where all are NaN)
 #pragma unroll
-            for (int o = 16; o >= 1; o >>= 1) {
-                const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const float ow = __shfl_xor_sync(0xffffffffu, win, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-                if (ob > best || (ob == best && oi < idx)) {
-                    best = ob;
-                    win = ow;
-                    idx = oi;
-                }
+            for (int e = 31; e >= 0; --e) {  // R3 R2 R0 R1 R4 hold bits 2 5 7 8 9
+                const int reg = (e >> 2 & 3) | (e >> 1 & 1) << 2 | (e & 1) << 3 | (e >> 4) << 4;
+                float a, b;
+                unpack2(v[reg / 2], a, b);
+                const float y = reg & 1 ? b : a;
+                if (fabsf(y) == best) idx = index_part(reg, 0, 9), win = y;
             }
+            if (idx != 0x7fffffff) idx += index_part(lane, 5, 9);
+            const int least = __reduce_min_sync(0xffffffffu, idx);
+            win = __shfl_sync(0xffffffffu, win, __ffs(__ballot_sync(0xffffffffu, idx == least)) - 1);
             if (lane == 0) {
-                codes[row * K + r] = CompT(component_of(win, idx, flip_mask));
+                codes[row * K + r] = CompT(component_of(win, least, flip_mask));
                 if (QUERY && mags) mags[row * K + r] = best;
             }
             if (QUERY && rotated) {
+                change_places(v, tmem);  // back to where they began
                 float* out = rotated + (row * K + r) * uint64_t(kP1024);
+                const bool wide = (reinterpret_cast<uintptr_t>(rotated) & 15) == 0;
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const int i = 32 * j + lane;
-                    out[i] = (__popc(i & flip_mask) & 1) ? -v[j] : v[j];
+                for (int c = 0; c < 8; ++c) {
+                    const int i = begins + index_part(4 * c, 0, 0);
+                    float4 o;
+                    unpack2(v[2 * c], o.x, o.y);
+                    unpack2(v[2 * c + 1], o.z, o.w);
+                    if (__popc(i & flip_mask) & 1) o.x = -o.x;
+                    if (__popc((i + 1) & flip_mask) & 1) o.y = -o.y;
+                    if (__popc((i + 2) & flip_mask) & 1) o.z = -o.z;
+                    if (__popc((i + 3) & flip_mask) & 1) o.w = -o.w;
+                    if (wide) *reinterpret_cast<float4*>(out + i) = o;
+                    else out[i] = o.x, out[i + 1] = o.y, out[i + 2] = o.z, out[i + 3] = o.w;
                 }
             }
         }
     }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_sm), "r"(kTmemCols1024) : "memory");
 }
 
 // ---- padded dims 256, 512: one warp per vector, E = P / 32 consecutive elements per lane ----------------------
@@ -720,6 +778,10 @@ static int rotations_per_block(uint64_t blocks, uint64_t want, int K) {
     return int((K + split - 1) / split);
 }
 
+uint32_t p1024_element(int layer, int lane, int reg) {
+    return uint32_t(index_part(reg, 0, 3 * layer) | index_part(lane, 5, 3 * layer));
+}
+
 int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_codes, float* d_rot,
                   float* d_mag, cudaStream_t st) {
     if (n == 0) return 0;
@@ -769,7 +831,9 @@ int launch_encode(cphnsw_b200_index* h, const float* d_x, uint64_t n, void* d_co
     } else if (P == kP1024 && h->d_signbits.p) {
         const uint64_t blocks = (n + kWarps1024 - 1) / kWarps1024;
         const int rpb = rotations_per_block(blocks, uint64_t(h->sm_count) * 16, K);
-        const dim3 grid(unsigned(blocks < uint64_t(h->sm_count) * 16 ? blocks : uint64_t(h->sm_count) * 16), unsigned((K + rpb - 1) / rpb));
+        // (many vectors: as many blocks as are resident)
+        const uint64_t most = uint64_t(h->sm_count) * kBlocks1024;
+        const dim3 grid(unsigned(blocks < most ? blocks : most), unsigned((K + rpb - 1) / rpb));
         const uint32_t* sb = h->d_signbits.as<uint32_t>();
 #define CPB_LAUNCH_P1024(T, Q)                                                                              \
     encode_p1024_kernel<T, Q><<<grid, kWarps1024 * 32, 0, st>>>(d_x, n, dim, K, rpb, sb, flip_mask, (T*)d_codes, d_rot, d_mag)
