@@ -37,6 +37,21 @@ def test_walk_matches_one_warp_kernel_and_oracle(cp, oracle, dim, K, cb, M, k, e
         assert np.array_equal(ids[:20], oi) and np.array_equal(dist[:20], od)
 
 
+# a base beyond L2 that is read many times over: the queries are taken by their nearest entry nodes (more queries than one pass of
+# the block that orders them, fewer seeds than it looks at)
+@pytest.mark.parametrize("n,dim,nq,rerank,seeds", [(40_003, 960, 601, 1000, 32), (70_001, 512, 2_500, 500, 3)])
+def test_queries_in_order_of_their_entry_nodes(cp, n, dim, nq, rerank, seeds):
+    base, q = synthetic.gaussian_mixture(n, nq, dim, 40, 0.3, nq)
+    idx = cp.CPHNSWIndex(dim, M=32, ef_construction=200, K=16, component_bytes=2)
+    idx.set_param("entry_scan", 300)
+    idx.set_param("k_entry", seeds)
+    idx.add_batch_parallel(base)
+    ids, dist = idx.search_and_rerank_batch(q, 10, 100, rerank)
+    idx.set_param("search_kernel", 1)
+    wi, wd = idx.search_and_rerank_batch(q, 10, 100, rerank)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
 @pytest.mark.parametrize("M", [24, 32])
 @pytest.mark.parametrize("row,a,b", [(0, 0, 1), (0, 0, 16), (0, 7, 23), (256, 3, 20)])
 def test_repeated_ids_in_a_row_count_once(cp, oracle, M, row, a, b):
