@@ -869,47 +869,71 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
     if (w.exact_visited && lane == 0) a.epochs[slot] = epoch;
 }
 
-// ---- few queries (asymmetric metric): a block per query ----------------------------------------------------------------------------------
+// ---- few queries: a block per query ----------------------------------------------------------------------------------
 // With fewer queries than the chip has room for walks, what counts is the length of one walk: its steps in sequence,
-// some 5,000 cycles each for a warp alone.  Here eight warps share a query and a step takes the first sixteen unexpanded
-// members of W, two rows a warp, dealt out in turn (where a row brings so many candidates that a warp has room for one only,
-// as on data without clusters, the step still has the first eight); the prefix committed grows from 3.4 rows to about 8, and the rows' lookups and scores
-// run side by side.  Rows, candidates and the committed prefix are those of search_walk_kernel, so the results are too.
+// some 5,000 cycles each for a warp alone.  Here eight warps share a query and a step takes the first 32 unexpanded members of W
+// (those of a window of 32), four rows a warp, dealt out in turn (where a row brings so many candidates that a warp has room for
+// one only, as on data without clusters, the step still has the first eight); the prefix committed grows from 3.4 rows to 32 where
+// the beam is nearly settled, and the rows' lookups and scores run side by side.  Rows, candidates and the committed prefix are
+// those of search_walk_kernel, so the results are too.
 //
-// A step meets at three barriers: the warps' candidates are listed with their ranks in W and the bound each puts on the
-// prefix; repeats (a node found by two rows) and candidates of rows that are not committed are struck out; W is rebuilt
-// in the other of its two arrays, every member moving up by the candidates that rank before it.
-constexpr uint32_t kStruck = 0xffffffffu;
+// A step meets at barriers: every warp says which bound its candidates put on the prefix; the candidates of the rows within it
+// are listed with their ranks in W; repeats (a node found by two rows) are struck out; those left are ranked among each other and
+// go to their places in the other of W's two arrays; and every member moves there by the number of them that rank before it,
+// found by bisection.  What bounds it is the chain of round trips, some 6,400 cycles a step: rows, codes and tables from L2, the
+// bisection of W, barriers.  One query on 100k x 128, beam 500, all kernels: 302 us with the candidates of all rows listed before
+// the prefix was known (a query's first ten or so steps find 100 to 250 and commit one row), ranked by a thread an entry and every
+// member held against every entry; 224 with 16 rows a step, 213 with 24, 191 with 32.  Codes of the rows expected next loaded
+// ahead, W known to be shared memory: no faster.
+constexpr uint32_t kStruck = 0xffffffffu;  // no place
 
 constexpr int kSquadWarps = 8;
 constexpr int kSquadThreads = kSquadWarps * 32;
-constexpr int kSquadRows = 2;                            // per warp
+constexpr int kSquadRows = 4;                            // per warp
 constexpr int kSquadFront = kSquadWarps * kSquadRows;    // members of W taken per step
 
 template <bool U16, int METRIC>
 __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs w) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     __shared__ uint64_t list_key[kSquadThreads];
-    __shared__ uint32_t list_place[kSquadThreads];  // members of W below; kStruck: struck out
-    __shared__ uint32_t list_row[kSquadThreads];    // place of the row in the step's prefix
+    __shared__ uint32_t list_place[kSquadThreads];  // members of W below
     __shared__ uint32_t cids[kSquadWarps][32], fronts[kSquadWarps][2 * kSquadFront];
-    __shared__ uint32_t listed, prefix, seeded;
+    __shared__ uint32_t sorted_place[kSquadThreads];  // of the entries kept, in order
+    __shared__ uint32_t listed, prefix, seeded, kept_all;
     const SearchArgs& a = w.s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tid = threadIdx.x, below = (1u << lane) - 1u;
     const uint32_t q = blockIdx.x, n = uint32_t(a.n);
+    unsigned char* qcode = walk_smem + size_t(w.wcap_slots) * 16 + kTagBytes;  // symmetric metrics
     uint64_t* W = reinterpret_cast<uint64_t*>(walk_smem);
     uint64_t* W2 = W + w.wcap_slots;
     uint2* tags = reinterpret_cast<uint2*>(W2 + w.wcap_slots);
     uint32_t* cid = cids[warp];
     uint32_t* front = fronts[warp];
-    const float* table = a.tables + size_t(q) * a.K * a.P;
+    constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
+    const float* table = SYM ? nullptr : a.tables + size_t(q) * a.K * a.P;
+    if (SYM && warp == 0) {  // the query's code, as bytes or packed sign bits
+        const int row_bytes = a.K * (U16 ? 2 : 1);
+        const unsigned char* src = static_cast<const unsigned char*>(a.qcodes) + size_t(q) * row_bytes;
+        if (METRIC == kSymBytes) {
+            for (int i = lane; i < row_bytes; i += 32) qcode[i] = src[i];
+        } else {
+            for (int i = 0; i < a.packed_words; ++i) {
+                const int r = 32 * i + lane;
+                const uint32_t word = __ballot_sync(kFull, r < a.K && (src[r * (U16 ? 2 : 1)] & 1u));
+                if (lane == 0) reinterpret_cast<uint32_t*>(qcode)[i] = word;
+            }
+        }
+    }
 
     for (uint32_t i = tid; i < kTagBytes / 16; i += kSquadThreads) reinterpret_cast<uint4*>(tags)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (tid == 0) listed = 0, prefix = kSquadFront;
     __syncthreads();
 
-    auto score = [&](int total) -> float {
+    auto score = [&](int total, uint32_t id) -> float {
+        if (METRIC == kSymPacked)
+            return lane < total ? packed_distance_lane(reinterpret_cast<const uint32_t*>(qcode), a.packed, id, a.packed_words, a.resid_kp, a.resid_mul) : 0.0f;
+        if (METRIC == kSymBytes) return lane < total ? sym_distance_lane<U16>(qcode, a.codes, id, a.K, a.resid_kp, a.resid_mul) : 0.0f;
         return score_asym<U16, METRIC == kAsym128>(table, static_cast<const unsigned char*>(a.codes), a.K, a.P, cid, total, lane);
     };
 
@@ -933,7 +957,7 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
             const uint32_t id = lane < total ? __ldg(a.entry + tid) : kInvalidNode;
             cid[lane] = id;
             __syncwarp();
-            const float d = score(total);
+            const float d = score(total, id);
             if (lane < total) {
                 k = make_key(d, id);
                 tag_store(tags, id);
@@ -1013,20 +1037,20 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
             }
         }
         __syncwarp();
-        uint32_t id = kInvalidNode, my_row = 0;
-        bool own = false;
+        uint32_t id = kInvalidNode, my_row = 0, p = 0;
+        uint64_t key = kFiller;
+        bool own = false, adm = false;
         if (total) {
             own = lane < total;
             id = own ? cid[lane] : kInvalidNode;
 #pragma unroll
             for (int b = 0; b < kSquadRows; ++b)
                 if (lane >= first_of[b]) my_row = b * kSquadWarps + warp;
-            const float d = score(total);
+            const float d = score(total, id);
             const uint32_t grp = __match_any_sync(kFull, id);
             own = own && (__ffs(grp) - 1) == lane;
-            const uint64_t key = make_key(d, id);
-            bool adm = own && (count < a.beam || key < W[count - 1]);
-            uint32_t p = 0;
+            key = make_key(d, id);
+            adm = own && (count < a.beam || key < W[count - 1]);
             if (adm) {
                 p = lower_bound(W, count, key);
                 if (p < count && (W[p] >> 1) == (key >> 1)) adm = false;  // a forgotten node that is a member of W
@@ -1036,63 +1060,76 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
                 const uint32_t bl = p <= cur ? 0u : (rel >= 32u ? sel : sel & ((1u << rel) - 1u));
                 bound = min(bound, max(my_row + 1u, uint32_t(__popc(bl))));
             }
-            const uint32_t am = __ballot_sync(kFull, adm);
-            if (am) {
-                uint32_t at = 0;
-                if (lane == 0) at = atomicAdd(&listed, uint32_t(__popc(am)));
-                at = __shfl_sync(kFull, at, 0) + __popc(am & below);
-                if (adm) {
-                    list_key[at] = key;
-                    list_place[at] = p;
-                    list_row[at] = my_row;
-                }
-            }
         }
         bound = __reduce_min_sync(kFull, bound);
         if (lane == 0) atomicMin(&prefix, bound);
         __syncthreads();
-        const uint32_t commit = prefix, m = listed;
+        const uint32_t commit = prefix;
         if (own && my_row < commit) tag_store(tags, id);
-        const bool listed_here = tid < m;
-        const uint64_t key = listed_here ? list_key[tid] : 0;
-        bool keep = listed_here && list_row[tid] < commit;
-        if (keep)
-            for (uint32_t i = 0; i < tid; ++i)
-                if (list_key[i] == key && list_row[i] < commit) keep = false;
-        if (listed_here && !keep) list_place[tid] = kStruck;
-        __syncthreads();
-        if (tid == 0) listed = 0, prefix = kSquadFront;
-        const uint64_t committed = commit;
-        uint32_t kept = 0, lowest = kStruck, rank = 0;
-        for (uint32_t i = 0; i < m; ++i) {
-            const uint32_t p = list_place[i];
-            lowest = min(lowest, p);
-            if (p != kStruck) {
-                ++kept;
-                rank += list_key[i] < key;
+        adm = adm && my_row < commit;
+        const uint32_t am = __ballot_sync(kFull, adm);
+        if (am) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&listed, uint32_t(__popc(am)));
+            at = __shfl_sync(kFull, at, 0) + __popc(am & below);
+            if (adm) {
+                list_key[at] = key;
+                list_place[at] = p;
             }
         }
-        // the members of the committed rows carry their flag from now on
-        uint32_t last = 0;  // window positions up to this bit are the committed ones among sel
-        {
-            uint32_t s = sel;
-            for (uint32_t c = 1; c < committed; ++c) s &= s - 1;
-            last = committed ? __ffs(s) - 1 : 0u;
+        __syncthreads();
+        const uint32_t m = listed;
+        uint32_t kept = 0, lowest = kStruck;
+        if (tid == 0) prefix = kSquadFront, kept_all = 0;
+        if (m) {
+            // several threads an entry, as many as there are; they share the loop over the others
+            const int share = m <= 32 ? 3 : (m <= 64 ? 2 : (m <= 128 ? 1 : 0));
+            const uint32_t threads = 1u << share, entry = tid >> share, part = tid & (threads - 1);
+            const uint32_t mates = (kFull >> (32 - threads)) << (lane & ~(threads - 1));
+            const bool have_entry = entry < m;
+            const uint64_t mine = have_entry ? list_key[entry] : 0;
+            bool twice = false;
+            if (have_entry) {
+#pragma unroll 4
+                for (uint32_t i = part; i < entry; i += threads) twice |= list_key[i] == mine;
+            }
+            const uint32_t repeats = __ballot_sync(kFull, twice);
+            const bool keep = have_entry && !(repeats & mates);
+            const uint32_t place = keep ? list_place[entry] : kStruck;
+            if (have_entry && (repeats & mates) && part == 0) list_key[entry] = kFiller;  // (ranks above all)
+            __syncthreads();
+            if (tid == 0) listed = 0;
+            uint32_t rank = 0;
+            if (keep) {
+#pragma unroll 4
+                for (uint32_t i = part; i < m; i += threads) rank += list_key[i] < mine;
+            }
+            for (uint32_t d = 1; d < threads; d <<= 1) rank += __shfl_xor_sync(kFull, rank, d);
+            const bool first = keep && part == 0;
+            const uint32_t kept_here = __popc(__ballot_sync(kFull, first));
+            if (lane == 0 && kept_here) atomicAdd(&kept_all, kept_here);
+            if (first) {
+                sorted_place[rank] = place;
+                if (place + rank < a.beam) W2[place + rank] = mine;
+            }
+            __syncthreads();
+            kept = kept_all, lowest = sorted_place[0];
         }
-        const uint32_t flag = committed ? sel & (last == 31 ? kFull : (2u << last) - 1u) : 0u;
+        // the members of the committed rows carry their flag from now on
+        const uint32_t flag = __ballot_sync(kFull, open && order < commit);
         if (kept) {
             const uint32_t newcount = min(a.beam, count + kept);
             for (uint32_t j = tid; j < count; j += kSquadThreads) {
                 uint64_t e = W[j];
                 const uint32_t rel = j - cur;
                 if (j >= cur && rel < 32u && ((flag >> rel) & 1u)) e |= 1u;
-                uint32_t up = 0;
-                for (uint32_t i = 0; i < m; ++i) up += list_place[i] <= j;
+                uint32_t up = 0, end = j < lowest ? 0u : kept;  // the entries placed at j or before
+                while (up < end) {
+                    const uint32_t mid = (up + end) >> 1;
+                    if (sorted_place[mid] <= j) up = mid + 1;
+                    else end = mid;
+                }
                 if (j + up < newcount) W2[j + up] = e;
-            }
-            if (keep) {
-                const uint32_t f = list_place[tid] + rank;
-                if (f < newcount) W2[f] = key;
             }
             uint64_t* t = W;
             W = W2;
@@ -1313,17 +1350,23 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
             w.order = sc.near + a.nq;
         }
     }
-    // Few queries under the asymmetric metric: a block each.  Measured on 64 / 250 / 500 queries, beam 500, against a warp each:
-    // 100k x 128, K = 32, 352 / 390 / 544 us against 479 / 507 / 530, K = 64 (a table of 32 KB) 455 / 519 / 665 against
-    // 845 / 914 / 956, d = 960 581 / 722 / 908 against 851 / 963 / 995; under the symmetric metrics, whose scores cost little
-    // and tie often, a warp was always faster.
-    const uint32_t squads_per_sm = size_t(a.K) * a.P * 4 >= 32 * 1024 ? 4 : 2;
-    const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes;
-    if (!sym && !w.exact_visited && a.nq <= squads_per_sm * uint32_t(h->sm_count) &&
-        (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 128))) {
-        if (metric == kAsym128) CPB_TRY((launch_squad_t<false, kAsym128>(w, squad_smem, st)));
-        else if (u16) CPB_TRY((launch_squad_t<true, kAsym>(w, squad_smem, st)));
-        else CPB_TRY((launch_squad_t<false, kAsym>(w, squad_smem, st)));
+    // Few queries: a block each, as many as run at once.  Against a warp each, us for 1 / 148 / 296 / 592 queries: 100k x 128,
+    // beam 500, K = 32 166 / 212 / 284 / 341 against 475 / 507 / 530 / 563; K = 64, a table of 32 KB, 237 / 309 / 364 / 509 against
+    // 845 / 914 / 956 / 980; 60k points of the sphere, K = 32 1,139 / 1,308 / 1,453 / 1,875 against 1,815 at 592, so the line is at
+    // 555 there; sign-bit codes, K = 64, beam 200, 164 / 203 / 233 / 278 against 244 / 289 / 350 / 359, of the sphere 339 / 453 /
+    // 497 / 592 against 565 / 604 / 629 / 640; code distance, K = 32, of the sphere 425 / 530 / 575 / 704 against 601 / 698 / 709 /
+    // 758.  Beyond, blocks go in waves: 800 queries 486 against 613 on clusters, but 2,945 against 1,897 of the sphere.
+    const uint32_t squads = uint32_t(h->sm_count) * (size_t(a.K) * a.P * 4 >= 32 * 1024 || sym ? 16 : 15) / 4;
+    const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes + (sym ? row : 0);
+    if (!w.exact_visited && a.nq <= squads && (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 128))) {
+#define CPB_SQUAD(X) (u16 ? launch_squad_t<true, X>(w, squad_smem, st) : launch_squad_t<false, X>(w, squad_smem, st))
+        switch (metric) {
+            case kAsym: CPB_TRY(CPB_SQUAD(kAsym)); break;
+            case kAsym128: CPB_TRY((launch_squad_t<false, kAsym128>(w, squad_smem, st))); break;
+            case kSymBytes: CPB_TRY(CPB_SQUAD(kSymBytes)); break;
+            default: CPB_TRY(CPB_SQUAD(kSymPacked)); break;
+        }
+#undef CPB_SQUAD
     } else {
 #define CPB_WALK(X) (u16 ? launch_walk_t<true, X>(h, w, blocks, warps, st) : launch_walk_t<false, X>(h, w, blocks, warps, st))
     switch (metric) {

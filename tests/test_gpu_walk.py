@@ -37,6 +37,30 @@ def test_walk_matches_one_warp_kernel_and_oracle(cp, oracle, dim, K, cb, M, k, e
         assert np.array_equal(ids[:20], oi) and np.array_equal(dist[:20], od)
 
 
+# a block or a warp per query under the symmetric metrics: one-byte and two-byte components, sign bits with and without residual
+# bits; a fifth of the vectors are copies of one (their distances tie, by id) and the beam is wider than the cluster
+@pytest.mark.parametrize("kind,dim,K,ef", [("bytes", 100, 33, 40), ("bytes", 300, 16, 300), ("binary", 128, 64, 200), ("residual", 64, 32, 65)])
+@pytest.mark.parametrize("nq", [1, 592, 593])
+def test_few_queries_under_the_symmetric_metrics(cp, kind, dim, K, ef, nq):
+    n = 3001
+    base, q = synthetic.gaussian_mixture(n, nq, dim, 12, 0.3, dim + nq)
+    base[::5] = base[0]
+    if kind == "bytes":
+        idx = cp.CPHNSWIndex(dim, M=24, ef_construction=200, K=K, component_bytes=2 if dim > 128 else 1)
+    else:
+        idx = cp.CPHNSWIndex.binary(dim, M=32, ef_construction=200, K=K)
+    if kind == "residual":
+        idx.set_param("residual_bits", 16)
+    idx.set_param("entry_scan", 200)
+    idx.set_param("k_entry", 32)
+    idx.add_batch_parallel(base)
+    run = (lambda: idx.search_multiprobe_batch(q, 10, ef, 1)) if kind == "bytes" else (lambda: idx.search_batch(q, 10, ef))
+    ids, dist = run()
+    idx.set_param("search_kernel", 1)
+    wi, wd = run()
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
 # a base beyond L2 that is read many times over: the queries are taken by their nearest entry nodes (more queries than one pass of
 # the block that orders them, fewer seeds than it looks at)
 @pytest.mark.parametrize("n,dim,nq,rerank,seeds", [(40_003, 960, 601, 1000, 32), (70_001, 512, 2_500, 500, 3)])
