@@ -883,21 +883,23 @@ __global__ void __launch_bounds__(kWalkWarps * 32) search_walk_kernel(WalkArgs w
 // found by bisection.  What bounds it is the chain of round trips, some 6,400 cycles a step: rows, codes and tables from L2, the
 // bisection of W, barriers.  One query on 100k x 128, beam 500, all kernels: 302 us with the candidates of all rows listed before
 // the prefix was known (a query's first ten or so steps find 100 to 250 and commit one row), ranked by a thread an entry and every
-// member held against every entry; 224 with 16 rows a step, 213 with 24, 191 with 32.  Codes of the rows expected next loaded
-// ahead, W known to be shared memory: no faster.
+// member held against every entry; 224 with 16 rows a step, 213 with 24, 191 with 32.  Two windows
+// and 64 rows: 186, but of the sphere 3 % slower than with 32.  Codes of the rows expected next loaded ahead, W known to be shared
+// memory: no faster.
 constexpr uint32_t kStruck = 0xffffffffu;  // no place
 
 constexpr int kSquadWarps = 8;
 constexpr int kSquadThreads = kSquadWarps * 32;
 constexpr int kSquadRows = 4;                            // per warp
 constexpr int kSquadFront = kSquadWarps * kSquadRows;    // members of W taken per step
+static_assert(kSquadFront == 32, "the unexpanded members of a window");
 
 template <bool U16, int METRIC>
 __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs w) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     __shared__ uint64_t list_key[kSquadThreads];
     __shared__ uint32_t list_place[kSquadThreads];  // members of W below
-    __shared__ uint32_t cids[kSquadWarps][32], fronts[kSquadWarps][2 * kSquadFront];
+    __shared__ uint32_t cids[kSquadWarps][32], fronts[kSquadWarps][kSquadFront];
     __shared__ uint32_t sorted_place[kSquadThreads];  // of the entries kept, in order
     __shared__ uint32_t listed, prefix, seeded, kept_all;
     const SearchArgs& a = w.s;
@@ -973,9 +975,6 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
     __syncthreads();
     uint32_t count = seeded, cur = 0;
 
-    uint32_t pre_node[kSquadRows], pre_row[kSquadRows];
-#pragma unroll
-    for (int b = 0; b < kSquadRows; ++b) pre_node[b] = kInvalidNode, pre_row[b] = kInvalidNode;
     while (true) {
         // the first unexpanded members of the first window of 32 that has any: every warp finds them for itself
         uint32_t un = 0;
@@ -998,30 +997,20 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
         const uint32_t order = __popc(un & below);
         const bool open = (un >> lane) & 1u;
         const uint64_t ek = W[min(cur + lane, count - 1)];
-        if (open && order < 2 * kSquadFront) front[order] = uint32_t(ek) >> 1;
-        const uint32_t sel = __ballot_sync(kFull, open && order < kSquadFront);
+        if (open) front[order] = uint32_t(ek) >> 1;
         const int have = __popc(un);
         __syncwarp();
         uint32_t row[kSquadRows], fresh[kSquadRows];
 #pragma unroll
         for (int b = 0; b < kSquadRows; ++b) {
             const int t = b * kSquadWarps + warp;
-            const uint32_t node = t < have ? front[t] : kInvalidNode;
-            row[b] = pre_row[b];
-            // (a row that another warp asked for ahead comes from L1)
-            if (node != pre_node[b]) row[b] = (node != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(node) * a.M + lane) : kInvalidNode;
-        }
-#pragma unroll
-        for (int b = 0; b < kSquadRows; ++b) {
-            const int t = kSquadFront + b * kSquadWarps + warp;
-            pre_node[b] = t < have ? front[t] : kInvalidNode;
-            pre_row[b] = (pre_node[b] != kInvalidNode && lane < a.M) ? __ldg(a.adj + size_t(pre_node[b]) * a.M + lane) : kInvalidNode;
+            row[b] = t < have && lane < a.M ? __ldg(a.adj + size_t(front[t]) * a.M + lane) : kInvalidNode;
         }
 #pragma unroll
         for (int b = 0; b < kSquadRows; ++b) fresh[b] = __ballot_sync(kFull, row[b] < n && !tag_seen(tags, row[b]));
         // as many of the warp's rows as bring at most 32 candidates
         int total = 0, first_of[kSquadRows];
-        uint32_t bound = uint32_t(have < kSquadFront ? have : kSquadFront);
+        uint32_t bound = uint32_t(have);
         bool room = true;
 #pragma unroll
         for (int b = 0; b < kSquadRows; ++b) {
@@ -1057,7 +1046,7 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
             }
             if (adm) {
                 const uint32_t rel = p - cur;  // cur <= position of every selected member
-                const uint32_t bl = p <= cur ? 0u : (rel >= 32u ? sel : sel & ((1u << rel) - 1u));
+                const uint32_t bl = p <= cur ? 0u : (rel >= 32u ? un : un & ((1u << rel) - 1u));
                 bound = min(bound, max(my_row + 1u, uint32_t(__popc(bl))));
             }
         }
