@@ -65,13 +65,13 @@ def parse_args():
     return ap.parse_args()
 
 
-def measured_fp8_peak():
-    """Operations per second of the dense fp8 products: twice the measured bf16 rate (nominal where none was measured)."""
+def measured_fp4_peak():
+    """Operations per second of the dense fp4 products: four times the measured bf16 rate (nominal where none was measured)."""
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
         with open(path) as f:
-            return 2e12 * float(json.load(f)["bf16_tflops"]), "twice the measured bf16 rate"
-    return 4.5e15, "the nominal dense fp8 rate"
+            return 4e12 * float(json.load(f)["bf16_tflops"]), "four times the measured bf16 rate"
+    return 9e15, "the nominal dense fp4 rate"
 
 
 def measured_peaks():
@@ -630,13 +630,13 @@ def run_b200(args):
         # tensor-core filter: a component is 7 values of +-1 at K <= 32 and 3 above, rows padded to a multiple of 32
         # values; a pair costs two operations a value, once where both its rows are of one GPU
         values = (K * (7 if K <= 32 else 3) + 31) // 32 * 32
-        fp8, fp8_kind = measured_fp8_peak()
-        fp8 *= world
+        fp4, fp4_kind = measured_fp4_peak()
+        fp4 *= world
         products = build["knn_pairs_per_s"] * (1.0 - 0.5 / world) * 2 * values
-        roofline_build["knn_graph"] = {"bound": "fp8 tensor pipe and its epilogue", "achieved": products, "peak": fp8,
-                                       "unit": "op/s", "frac": products / fp8,
+        roofline_build["knn_graph"] = {"bound": "fp4 tensor pipe and its epilogue", "achieved": products, "peak": fp4,
+                                       "unit": "op/s", "frac": products / fp4,
                                        "note": "%d values per pair, an unordered pair once on a GPU that has both rows; peak is %s; the whole stage, "
-                                               "bounds and order included (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp8_kind)}
+                                               "bounds and order included (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp4_kind)}
     sel_bytes = n * (knn_k * 4 + knn_k * code_row + M * 4.0)
     roofline_build["select_neighbors"] = {"bound": "hbm gather", "achieved": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9, "peak": peak * world,
                                           "unit": "GB/s", "frac": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9 / (peak * world),

@@ -146,8 +146,7 @@ struct SearchCtx {
     uint64_t vis_stride = 0;
     size_t vis_slots = 0;
     DevBuf d_qtables, d_qcodes, d_q, d_out_ids, d_out_dist, d_stats;
-    DevBuf d_seeds, d_cand;  // entry scan -> walk: seed keys; walk -> rerank: ids
-    DevBuf d_order;          // the queries' nearest entry nodes, and the order in which they are taken
+    DevBuf d_seeds, d_cand;  // entry scan -> walk: seed keys, and behind them the queries' nearest entry nodes and their order; walk -> rerank: ids
     DevBuf d_probe_codes, d_probe_ids, d_probe_dist;  // search_multiprobe
     PinnedBuf h_in, h_out;  // staging of small host-pointer calls: queries; results, which the kernels write there
     ~SearchCtx() {

@@ -1319,7 +1319,7 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         sc.resid_kp = a.resid_kp;
         sc.resid_mul = a.resid_mul;
         w.seed_slots = a.n_seed <= 32 ? 32 : kScanKeep;
-        CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * w.seed_slots * 8));
+        CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * (w.seed_slots * 8 + 8)));
         sc.seeds = cx.d_seeds.as<uint64_t>();
         w.seeds = sc.seeds;
         // The order costs 10 us.  It is of use where links, codes and vectors do not fit L2 (126 MB), and made up for where the
@@ -1329,8 +1329,7 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         const double node_bytes = double(a.M) * 4 + double(row), vector_bytes = a.rerank_k ? double(a.dim) * 4 : 0.0;
         if (a.nq > 2 * uint32_t(h->sm_count) && double(a.n) * (node_bytes + vector_bytes) > kOrderBase &&
             double(a.nq) * (a.beam * node_bytes + a.rerank_k * vector_bytes) > kOrderReads) {
-            CPB_TRY(cx.d_order.reserve(size_t(a.nq) * 8));
-            sc.near = cx.d_order.as<uint32_t>();
+            sc.near = reinterpret_cast<uint32_t*>(sc.seeds + size_t(a.nq) * w.seed_slots);
         }
         CPB_TRY(a.comp_bytes == 2 ? launch_scan<true>(h, sc, metric, st) : launch_scan<false>(h, sc, metric, st));
         if (sc.near) {
