@@ -43,11 +43,12 @@
 // sixteen read, a quarter of the columns and of either half's rows each, and hand an accumulator back as soon as it is in
 // registers.  The operand is laid out by the expansion kernel in the form the tensor core reads (8-row by 16-byte core
 // matrices), so a tile is one contiguous copy and no tensor map is needed.
-// 500k x 500k, K = 32: the sweep takes 9.5 ms, some 1,420 cycles a tile whose products take 1,024 (with 8-bit operands and fp16
-// accumulators 15.1 ms, 2,200 of 1,792), the whole graph 14.7 against 20.4; 1M x 1M 50.2 against 72.9.  On the way, the whole graph:
+// 500k x 500k, K = 32: the sweep takes 9.7 ms, 1,300 to 1,450 cycles a tile whose products take 1,024 (with 8-bit operands and fp16
+// accumulators 15.1 ms, 2,200 of 1,792), the whole graph 14.9 against 20.4; 1M x 1M 50.9 against 72.9.  On the way, the whole graph:
 // units of N = 128 and three accumulators with one warp issuing 21.0; descriptors known to be uniform and polls before waits 18.3;
 // readers that hand back before they look 17.5; units of 64, a second issuing warp, columns and gates of 32 steps at a time 15.5;
-// polls ahead of the products before 15.2; a step's hits listed a step later and by one atomic 14.7.  Waits that spin instead of
+// polls ahead of the products before 15.2; a step's hits listed a step later and by one atomic 14.7.  Hits
+// kept in shared memory until there are five are listed by half as many atomics: 14.9 here, but 2 to 6 % less where clusters overlap.  Waits that spin instead of
 // sleeping: 15.6 to 16.2.
 #include <type_traits>
 
@@ -874,6 +875,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     __shared__ __align__(8) uint64_t tfull_bar[kUnitsStep], tempty_bar[kUnitsStep];
     __shared__ __align__(8) uint64_t rows_bar, done_bar;  // a row tile's rows are in tensor memory; its last products are through
     __shared__ __align__(8) uint64_t drain_bar;
+    __shared__ __align__(16) uint4 hits_sm[kEpiWarps][8];
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
     const bool calm = a.calm.yes();
@@ -968,22 +970,26 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         // the accumulators of the step's two units: two of the first warp's four, or those whose turn it is of the second's three
         uint32_t at0 = cols / 2, at1 = cols / 2 + 2, done_parity = 0;
         if (cols & 1) at0 += 4, at1 = at0 == 4 ? 6 : at0 - 1;
-        // The last hits found: of the rows from `first` on and from 128 places on, with 32 columns from `col` on (its lowest bit:
-        // both) and the 32 after them.  They are listed when the next are found, or at the end: the place in the list then has come
-        // (waiting for it took as long as a step), and a step's take one atomic (100k x 960, two bytes: two a step 643 us, 539 so).
-        uint32_t found[4] = {0u, 0u, 0u, 0u}, first = 0, col = 0, to = 0;
+        // Hits wait in shared memory for a place in the list, asked for when more than four are there and used when the next come, or
+        // at the end: the place then has come (waiting for it took as long as a step), and where hits are dense two steps' take one
+        // atomic on the list's length, which would be the bound there (100k x 960, two bytes: two atomics a step 643 us, one 539;
+        // 100k x 64, K = 16, clusters of 100, the last phase: one 429, with five to eight hits an atomic 272).
+        uint4* const waiting = hits_sm[warp];
+        uint32_t have = 0, asked = 0, to = 0;
+        auto ask = [&]() {
+            if (lane == 0) to = atomicAdd(a.hit_count, have);
+            asked = have;
+        };
         auto list_hits = [&]() {
             to = __shfl_sync(kFull, to, 0);
+            if (uint32_t(lane) < asked && to + lane < a.hit_room) a.hits[to + lane] = waiting[lane];
 #pragma unroll 1
-            for (uint32_t g = 0; g < 4; ++g) {
-                const uint32_t rows = g < 2 ? (g ? found[1] : found[0]) : (g == 2 ? found[2] : found[3]);
-                if (rows == 0) continue;
-                const uint32_t from_row = first + (g >> 1) * 128, from_col = (col & ~1u) + (g & 1) * 32;
-                if (lane == 0 && to < a.hit_room) a.hits[to] = make_uint4(from_row, from_col, rows, col & 1u);
-                if (to >= a.hit_room) compare_rows<U16, QUADS>(a, rows, from_row, __ldg(a.place + from_row + lane), from_col, col & 1u, lane);
-                ++to;
+            for (uint32_t e = to < a.hit_room ? a.hit_room - to : 0u; e < asked; ++e) {  // no room: compared at once
+                const uint4 h = waiting[e];
+                compare_rows<U16, QUADS>(a, h.z, h.x, __ldg(a.place + h.x + lane), h.y, h.w != 0, lane);
             }
             __syncwarp();
+            have = asked = 0;
         };
         bool ok = true;
         for (uint32_t i = 0; i < steps && ok; walk.next_rows()) {
@@ -1033,18 +1039,23 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                     rows[2 * h + 1] = __ballot_sync(kFull, hit1);
                 }
                 if (rows[0] | rows[1] | rows[2] | rows[3]) {
-                    list_hits();
-                    uint32_t many = 0;
-#pragma unroll
-                    for (int g = 0; g < 4; ++g) found[g] = rows[g], many += rows[g] != 0;
+                    if (asked) list_hits();
+                    const uint32_t some = (rows[0] != 0) | (rows[1] != 0) << 1 | (rows[2] != 0) << 2 | (rows[3] != 0) << 3;
                     const uint32_t ct = __shfl_sync(kFull, tile, s % 32);
-                    first = row0, col = (ct * kMmaRows + cols * kUnitCols) | (a.meet.both(rt, ct) ? 1u : 0u);
-                    if (lane == 0) to = atomicAdd(a.hit_count, many);
+                    if (some >> lane & 1u) {
+                        const uint32_t mine = lane < 2 ? (lane ? rows[1] : rows[0]) : (lane == 2 ? rows[2] : rows[3]);
+                        waiting[have + __popc(some & ((1u << lane) - 1u))] =
+                            make_uint4(row0 + (lane >> 1) * 128, ct * kMmaRows + cols * kUnitCols + (lane & 1) * 32, mine, a.meet.both(rt, ct) ? 1u : 0u);
+                    }
+                    have += __popc(some);
+                    __syncwarp();
+                    if (have > 4) ask();
                 }
                 if (cols & 1) at1 = at0, at0 = at0 == 6 ? 4 : at0 + 1;
             }
         }
-        list_hits();
+        if (have && !asked) ask();
+        if (asked) list_hits();
         if (!ok) *aborted = 1;
     }
     __syncthreads();
@@ -1621,6 +1632,8 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.chunks = shape.chunks;
     a.stages = int(kMmaSmem / operand_bytes);
     if (a.stages > kMaxStages) a.stages = kMaxStages;
+    // (never two blocks on an SM, of which the second would wait for the first one's tensor memory)
+    const size_t ring = size_t(a.stages) * operand_bytes, sweep_smem = ring > (size_t(120) << 10) ? ring : size_t(120) << 10;
     a.k = k;
     a.entries = entries;
     a.counts = counts;
@@ -1710,7 +1723,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
             const uint64_t steps = uint64_t(a.meet.row_tiles) * count;
             if (!first) CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
             first = false;
-            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, a.stages * operand_bytes, st>>>(a);
+            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, sweep_smem, st>>>(a);
             knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
             h->launches += 2;
             return 0;
