@@ -73,7 +73,7 @@ constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in
 constexpr uint64_t kLaunchSteps = 1u << 22;
 constexpr uint32_t kCheckBlocks = 4;      // blocks of the check an SM
 constexpr uint32_t kNearColumns = 8, kNearFrom = 64;  // column tiles that are swept first, of so many at least
-constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes, a half of the rows, a half of the columns
+constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the lanes and of the columns, of both halves of the rows
 constexpr int kMmaWarps = 2;              // warps that issue products, see there
 constexpr int kMmaThreads = (kEpiWarps + 1 + kMmaWarps) * 32;  // and one for the operands' copies
 constexpr int kMaxStages = 8;             // of a tile each
