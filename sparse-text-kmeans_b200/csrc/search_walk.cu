@@ -899,7 +899,9 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
     extern __shared__ __align__(16) unsigned char walk_smem[];
     __shared__ uint64_t list_key[kSquadThreads];
     __shared__ uint32_t list_place[kSquadThreads];  // members of W below
-    __shared__ uint32_t cids[kSquadWarps][32], fronts[kSquadWarps][kSquadFront];
+    // a warp's candidates and front until the step's prefix is known; then, until it ends, the listed keys that are kept
+    __shared__ uint64_t kept_key[kSquadThreads];
+    static_assert(sizeof(kept_key) == kSquadWarps * (32 + kSquadFront) * 4, "32 candidates and kSquadFront members a warp");
     __shared__ uint32_t sorted_place[kSquadThreads];  // of the entries kept, in order
     __shared__ uint32_t listed, prefix, seeded, kept_all;
     const SearchArgs& a = w.s;
@@ -910,8 +912,8 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
     uint64_t* W = reinterpret_cast<uint64_t*>(walk_smem);
     uint64_t* W2 = W + w.wcap_slots;
     uint2* tags = reinterpret_cast<uint2*>(W2 + w.wcap_slots);
-    uint32_t* cid = cids[warp];
-    uint32_t* front = fronts[warp];
+    uint32_t* cid = reinterpret_cast<uint32_t*>(kept_key) + warp * (32 + kSquadFront);
+    uint32_t* front = cid + 32;
     constexpr bool SYM = METRIC == kSymBytes || METRIC == kSymPacked;
     const float* table = SYM ? nullptr : a.tables + size_t(q) * a.K * a.P;
     if (SYM && warp == 0) {  // the query's code, as bytes or packed sign bits
@@ -1085,13 +1087,13 @@ __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs
             const uint32_t repeats = __ballot_sync(kFull, twice);
             const bool keep = have_entry && !(repeats & mates);
             const uint32_t place = keep ? list_place[entry] : kStruck;
-            if (have_entry && (repeats & mates) && part == 0) list_key[entry] = kFiller;  // (ranks above all)
+            if (have_entry && part == 0) kept_key[entry] = keep ? mine : kFiller;  // (ranks above all; list_key is still being read)
             __syncthreads();
             if (tid == 0) listed = 0;
             uint32_t rank = 0;
             if (keep) {
 #pragma unroll 4
-                for (uint32_t i = part; i < m; i += threads) rank += list_key[i] < mine;
+                for (uint32_t i = part; i < m; i += threads) rank += kept_key[i] < mine;
             }
             for (uint32_t d = 1; d < threads; d <<= 1) rank += __shfl_xor_sync(kFull, rank, d);
             const bool first = keep && part == 0;

@@ -101,6 +101,31 @@ def test_repeated_ids_in_a_row_count_once(cp, oracle, M, row, a, b):
         assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
 
 
+# nodes by eights with the same links in another order each: what one warp of a block finds in a step, the others find as well, and
+# of the keys listed up to seven are struck out while other warps still compare theirs
+@pytest.mark.parametrize("M,nq", [(16, 1), (32, 40), (32, 149)])
+def test_ids_found_by_many_rows_of_a_step_count_once(cp, oracle, M, nq):
+    n, dim = 2000, 128
+    base, q = synthetic.gaussian_mixture(n, nq, dim, 4, 0.5, M + nq)
+    rng = np.random.default_rng(M)
+    ref = cp.CPHNSWIndex(dim, M=M, ef_construction=64, K=32, component_bytes=1, fht_convention=2)
+    codes = ref.encode(base)
+    adj = np.empty((n, M), np.uint32)
+    for i in range(0, n, 8):
+        links = rng.choice(n, M, replace=False)
+        for r in range(i, i + 8):
+            adj[r] = rng.permutation(np.where(links == r, (r + 8) % n, links))
+    idx = cp.CPHNSWIndex(dim, M=M, ef_construction=64, K=32, component_bytes=1, fht_convention=2)
+    idx.set_param("k_entry", 32)
+    idx.set_param("entry_scan", 32)
+    idx.install(base, codes, adj)
+    _, rot, _ = oracle.encode(q, 32, 1, oracle.sign_tables(dim, 32, 42), 2, want_rotated=True)
+    for ef in (40, 300):
+        ids, dist = idx.search_batch(q, 20, ef)
+        wi, wd = oracle.search(rot, codes, adj, idx.entry_ids(), ef, 20, n_seed=32)
+        assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+
+
 def test_wide_rows_with_the_walk_asked_for(cp):
     # M = 48: a search under the asymmetric score is refused, walks under the code distance take the one-warp kernel
     base, q = synthetic.gaussian_mixture(1200, 20, 64, 4, 0.3, 3)
