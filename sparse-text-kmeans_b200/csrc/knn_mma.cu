@@ -69,7 +69,12 @@ constexpr uint32_t kMmaKeep = 128;        // entries that are left of one that i
 constexpr uint32_t kMmaFull = 256;        // entries from which on it is cut between phases
 constexpr size_t kLongBuffers = size_t(128) << 20;  // bytes of the buffers of a graph of one phase, at most, if they are longer
 constexpr int kBatch = 4;                 // rows compared with 32 columns at a time
-constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in the list of hits
+constexpr uint32_t kHitRoom = 1u << 22;   // groups of 32 rows and 32 columns in the list of hits, where there are no more in all
+constexpr uint32_t kStepHits = 64;        // such groups in a step
+constexpr uint32_t kSection = 8192, kSections = 672;  // else: entries of a section of the list, and sections (63 MB in all)
+constexpr uint32_t kDrain = 2048;         // hits of a section that its block compares itself, at a time, when there are no others
+constexpr uint32_t kLeastRoom = 512;      // room that a section has to have for its block to go on with it
+static_assert(kLeastRoom >= kStepHits && kSection - kLeastRoom >= kDrain, "a section has room for a step, or hits to compare");
 constexpr uint64_t kLaunchSteps = 1u << 22;
 constexpr uint32_t kCheckBlocks = 4;      // blocks of the check an SM
 constexpr uint32_t kNearColumns = 8, kNearFrom = 64;  // column tiles that are swept first, of so many at least
@@ -77,7 +82,7 @@ constexpr int kEpiWarps = 16;             // epilogue warps: a quarter of the la
 constexpr int kMmaWarps = 2;              // warps that issue products, see there
 constexpr int kMmaThreads = (kEpiWarps + 1 + kMmaWarps) * 32;  // and one for the operands' copies
 constexpr int kMaxStages = 8;             // of a tile each
-constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 5 KB of static
+constexpr size_t kMmaSmem = 216 * 1024;   // dynamic shared memory a block may use beside its 3 KB of static
 constexpr int kSortRows = 1024;           // places sorted by limit together
 constexpr uint32_t kFirstColumns = 8;      // column tiles of the first phase, at most
 constexpr uint32_t kOnePhase = 64;         // up to so many (32,000 nodes) there is one, or the near columns and the rest, and calm
@@ -627,9 +632,14 @@ struct KnnMmaArgs {
     uint32_t cap;           // entries of a row's buffer: kMmaCap, or more (of one word each) in a graph of one phase
     uint32_t* entries;      // [row_tiles * 256][cap]
     uint32_t* counts;       // [row_tiles * 256] entries; above cap: some were lost
-    uint4* hits;            // 32 rows and 32 columns among which a product reaches its gate: first row, first column, rows, both
+    // 32 rows and 32 columns among which a product reaches its gate, in one list or in sections
+    uint4* hits;             // first row, first column, rows, both
     uint32_t* hit_count;
-    uint32_t hit_room;
+    uint2* places;           // [kSections][kSection] first row | both, first column
+    uint32_t* rows;          // [kSections][kSection]
+    uint32_t* section_hits;  // [kSections]
+    uint32_t* taken;         // sections that blocks have taken behind their first ones, of which there is one a block
+    uint32_t blocks;         // of the sweep
     uint32_t* status;
     uint32_t first_wait_polls, handover_polls;
     SweepChoice choice;
@@ -767,21 +777,83 @@ __device__ __forceinline__ void compare_rows(const KnnMmaArgs& a, uint32_t rows,
     }
 }
 
+struct SectionHits {
+    uint32_t of[kSections], upto[kSections], groups[kSections / 32];  // hits of a section; of its group of 32 up to it; up to a group
+};
+// The place of the e-th hit.  (A call, and the kernel has the registers that comparing takes and no more.)
+__device__ __noinline__ uint32_t place_of_hit(const SectionHits& hits, uint32_t e) {
+    const int lane = threadIdx.x & 31;
+    constexpr int kGroups = int(kSections / 32);
+    const int g = __popc(__ballot_sync(kFull, lane < kGroups && hits.groups[min(lane, kGroups - 1)] <= e));
+    const uint32_t in_group = e - (g ? hits.groups[g - 1] : 0u);
+    const int s = __popc(__ballot_sync(kFull, hits.upto[32 * g + lane] <= in_group));
+    return uint32_t(32 * g + s) * kSection + in_group - (s ? hits.upto[32 * g + s - 1] : 0u);
+}
+
 // What the sweep has listed.  What bounds it is latency, of the rows and of the places in the buffers, some 1,500 cycles a
-// batch: 32 warps an SM.  (In the sweep's own epilogue, two warps a scheduler, the products wait for it: 100k x 128
-// clustered 3.2 ms in all, 2.1 with the list.)
+// batch, and from 64 bytes on the comparing: 32 warps an SM, of 128 bytes 16 with registers enough for a batch in flight
+// (60,000 x 300, two bytes, K = 64: 24.9 ms with 24 warps, 23.6 so).  (In the sweep's own epilogue, two warps a scheduler, the
+// products wait for it: 100k x 128 clustered 3.2 ms in all, 2.1 with the list.)
 constexpr int kCheckWarps = 8;
 template <bool U16, int QUADS>
-__global__ void __launch_bounds__(kCheckWarps * 32) knn_check_kernel(KnnMmaArgs a) {
+__global__ void __launch_bounds__(kCheckWarps * 32, (QUADS > 4 ? 2 : 0)) knn_check_kernel(KnnMmaArgs a) {
     if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
     const int lane = threadIdx.x & 31;
     const uint32_t warp = blockIdx.x * kCheckWarps + (threadIdx.x >> 5), warps = gridDim.x * kCheckWarps;
-    const uint32_t many = min(*a.hit_count, a.hit_room);
+    const uint32_t many = *a.hit_count;
     const uint32_t parts = many < 8 * warps ? 4 : 1;  // few: eight rows a warp
     for (uint32_t i = warp; i < many * parts; i += warps) {
         const uint4 h = __ldg(a.hits + i / parts);
         const uint32_t rows = parts == 1 ? h.z : h.z & (0xffu << (8 * (i % parts)));
         compare_rows<U16, QUADS>(a, rows, h.x, __ldg(a.place + h.x + lane), h.y, h.w != 0, lane);
+    }
+}
+template <bool U16, int QUADS>
+__device__ __forceinline__ void compare_hit(const KnnMmaArgs& a, uint2 at, uint32_t rows, int lane) {
+    const uint32_t row0 = at.x & ~31u;
+    compare_rows<U16, QUADS>(a, rows, row0, __ldg(a.place + row0 + lane), at.y, at.x & 1u, lane);
+}
+
+// The same for hits in sections: few are taken one by one, many place by place, those behind a section's hits too, which costs less
+// than to look for each.
+template <bool U16, int QUADS>
+__global__ void __launch_bounds__(kCheckWarps * 32, (QUADS > 4 ? 2 : 0)) knn_check_sections_kernel(KnnMmaArgs a) {
+    if (a.choice.skip() || (a.when == KnnMmaArgs::kNotIfCalm && a.calm.yes())) return;
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp = blockIdx.x * kCheckWarps + (threadIdx.x >> 5), warps = gridDim.x * kCheckWarps;
+    constexpr int kGroups = int(kSections / 32);
+    __shared__ SectionHits hits;
+    const uint32_t used = min(a.blocks + *a.taken, kSections);
+    auto scan = [&](uint32_t x) {  // inclusive, over the lanes
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(kFull, x, d);
+            if (lane >= d) x += y;
+        }
+        return x;
+    };
+#pragma unroll
+    for (int g = int(threadIdx.x >> 5); g < kGroups; g += kCheckWarps) {
+        const uint32_t s = uint32_t(32 * g + lane), own = s < used ? __ldg(a.section_hits + s) : 0u, x = scan(own);
+        hits.of[s] = own, hits.upto[s] = x;
+        if (lane == 31) hits.groups[g] = x;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t x = scan(lane < kGroups ? hits.groups[lane] : 0u);
+        if (lane < kGroups) hits.groups[lane] = x;
+    }
+    __syncthreads();
+    const uint32_t many = hits.groups[kGroups - 1];
+    if (many >= 64 * warps && many > used * (kSection / 4)) {
+        for (uint32_t at = warp; at < used * kSection; at += warps)
+            if (at % kSection < hits.of[at / kSection]) compare_hit<U16, QUADS>(a, __ldg(a.places + at), __ldg(a.rows + at), lane);
+        return;
+    }
+    const uint32_t parts = many < 8 * warps ? 4 : 1;  // few: eight rows a warp
+    for (uint32_t i = warp; i < many * parts; i += warps) {
+        const uint32_t at = place_of_hit(hits, i / parts), rows = __ldg(a.rows + at);
+        compare_hit<U16, QUADS>(a, __ldg(a.places + at), parts == 1 ? rows : rows & (0xffu << (8 * (i % parts))), lane);
     }
 }
 
@@ -866,7 +938,8 @@ __device__ __forceinline__ bool issue_products(const KnnMmaArgs& a, Walk walk, u
     return true;
 }
 
-template <bool U16, int QUADS>  // QUADS: 16-byte words of a padded code row
+// QUADS: 16-byte words of a padded code row.  SECTIONS: there may be more hits than a list has room for
+template <bool U16, int QUADS, bool SECTIONS>
 __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     if (a.choice.skip()) return;
     extern __shared__ __align__(1024) unsigned char mma_smem[];
@@ -875,7 +948,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
     __shared__ __align__(8) uint64_t tfull_bar[kUnitsStep], tempty_bar[kUnitsStep];
     __shared__ __align__(8) uint64_t rows_bar, done_bar;  // a row tile's rows are in tensor memory; its last products are through
     __shared__ __align__(8) uint64_t drain_bar;
-    __shared__ __align__(16) uint4 hits_sm[kEpiWarps][8];
+    __shared__ __align__(16) uint4 hits_sm[SECTIONS ? 1 : kEpiWarps][8];
+    __shared__ __align__(8) uint64_t met_bar, go_bar;
+    __shared__ uint32_t listed, section, room;  // in the block's section, its number, and its room when the readers last met
     __shared__ uint32_t tmem_base_sm;
     __shared__ int abort_flag;
     const bool calm = a.calm.yes();
@@ -898,6 +973,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         knn::mbar_init(&rows_bar, kEpiWarps);
         knn::mbar_init(&done_bar, kMmaWarps);
         knn::mbar_init(&drain_bar, kMmaWarps);
+        knn::mbar_init(&met_bar, kEpiWarps);
+        knn::mbar_init(&go_bar, 1);
+        listed = 0, section = blockIdx.x;
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -970,11 +1048,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         // the accumulators of the step's two units: two of the first warp's four, or those whose turn it is of the second's three
         uint32_t at0 = cols / 2, at1 = cols / 2 + 2, done_parity = 0;
         if (cols & 1) at0 += 4, at1 = at0 == 4 ? 6 : at0 - 1;
-        // Hits wait in shared memory for a place in the list, asked for when more than four are there and used when the next come, or
-        // at the end: the place then has come (waiting for it took as long as a step), and where hits are dense two steps' take one
-        // atomic on the list's length, which would be the bound there (100k x 960, two bytes: two atomics a step 643 us, one 539;
-        // 100k x 64, K = 16, clusters of 100, the last phase: one 429, with five to eight hits an atomic 272).
-        uint4* const waiting = hits_sm[warp];
+        // Hits are listed, and compared by a kernel behind the sweep.  One list: they wait in shared memory for a place in it, asked for
+        // when more than four are there and used when the next come, or at the end: the place then has come (waiting for it took as
+        // long as a step), and where hits are dense two steps' take one atomic on the list's length, which would be the bound there
+        // (100k x 960, two bytes: two atomics a step 643 us, one 539; 100k x 64, K = 16, clusters of 100, the last phase: one 429,
+        // with five to eight hits an atomic 272).
+        uint4* const waiting = hits_sm[SECTIONS ? 0 : warp];
         uint32_t have = 0, asked = 0, to = 0;
         auto ask = [&]() {
             if (lane == 0) to = atomicAdd(a.hit_count, have);
@@ -982,14 +1061,50 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
         };
         auto list_hits = [&]() {
             to = __shfl_sync(kFull, to, 0);
-            if (uint32_t(lane) < asked && to + lane < a.hit_room) a.hits[to + lane] = waiting[lane];
-#pragma unroll 1
-            for (uint32_t e = to < a.hit_room ? a.hit_room - to : 0u; e < asked; ++e) {  // no room: compared at once
-                const uint4 h = waiting[e];
-                compare_rows<U16, QUADS>(a, h.z, h.x, __ldg(a.place + h.x + lane), h.y, h.w != 0, lane);
-            }
+            if (uint32_t(lane) < asked) a.hits[to + lane] = waiting[lane];
             __syncwarp();
             have = asked = 0;
+        };
+        // Sections: a block fills one, with an atomic in shared memory for the place.  By the time that the section can be full the warps
+        // meet, and the block goes on with it if it has room, with another one, or, when there are no others, after all its warps have
+        // compared a part of what is in it.  (A warp that compares by itself what has no room holds up the others, which read the same
+        // accumulators, and most warps have nothing to compare at that time.  Groups that overlap, sigma 0.45, K = 32, 64 neighbours:
+        // 1M x 128 455 ms like that, 263 so; sigma 0.4, 16 neighbours, 2M 369 and 242.  Where hits are few the meetings are too: 1M,
+        // sigma 0.3, 51.2 and 49.7.)  Up to 65,024 nodes every group has room in one list, which is quicker to go through (a check of
+        // 14,000 x 300, two bytes, sigma 0.6: 676 us, 722 with sections).
+        uint32_t next_look = SECTIONS ? kSection / kStepHits : ~0u, meetings = 0;
+        auto meet = [&](auto then) {  // all of them, and what the first one does before any goes on
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&met_bar);
+            if (warp == 0) {
+                if (!__all_sync(kFull, wait_or_abort(&met_bar, meetings & 1, kWaitLimit, aborted))) return false;
+                if (lane == 0) {
+                    then();
+                    mbar_arrive(&go_bar);
+                }
+                __syncwarp();
+            }
+            return bool(__all_sync(kFull, wait_or_abort(&go_bar, meetings++ & 1, kWaitLimit, aborted)));
+        };
+        auto look = [&](uint32_t i) {
+            const bool met = meet([&]() {
+                room = kSection - listed;
+                if (room >= kLeastRoom) return;
+                const uint32_t other = a.blocks + atomicAdd(a.taken, 1u);
+                room = 0;
+                if (other >= kSections) return;
+                a.section_hits[section] = listed;
+                section = other, listed = 0, room = kSection;
+            });
+            if (!met) return false;
+            if (room == 0) {
+                const size_t first = size_t(section) * kSection;
+#pragma unroll 1
+                for (uint32_t e = listed - kDrain + warp; e < listed; e += kEpiWarps) compare_hit<U16, QUADS>(a, a.places[first + e], a.rows[first + e], lane);
+                if (!meet([&]() { listed -= kDrain, room = kSection - listed; })) return false;
+            }
+            next_look = i + room / kStepHits;
+            return true;
         };
         bool ok = true;
         for (uint32_t i = 0; i < steps && ok; walk.next_rows()) {
@@ -1008,6 +1123,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
             };
             look_ahead(0);
             for (uint32_t s = 0; s < run && ok; ++s, ++i) {
+                if (SECTIONS && i == next_look && !look(i)) {
+                    ok = false;
+                    break;
+                }
                 if (s % 32 == 0) {
                     tile = next_tile, gates = next_gates;
                     if (s + 32 < run) look_ahead(s + 32);
@@ -1039,26 +1158,41 @@ __global__ void __launch_bounds__(kMmaThreads, 1) knn_mma_kernel(KnnMmaArgs a) {
                     rows[2 * h + 1] = __ballot_sync(kFull, hit1);
                 }
                 if (rows[0] | rows[1] | rows[2] | rows[3]) {
-                    if (asked) list_hits();
+                    if (!SECTIONS && asked) list_hits();
                     const uint32_t some = (rows[0] != 0) | (rows[1] != 0) << 1 | (rows[2] != 0) << 2 | (rows[3] != 0) << 3;
                     const uint32_t ct = __shfl_sync(kFull, tile, s % 32);
+                    if (SECTIONS) {
+                        if (lane == 0) to = atomicAdd(&listed, uint32_t(__popc(some)));
+                        to = __shfl_sync(kFull, to, 0);
+                    }
                     if (some >> lane & 1u) {
                         const uint32_t mine = lane < 2 ? (lane ? rows[1] : rows[0]) : (lane == 2 ? rows[2] : rows[3]);
-                        waiting[have + __popc(some & ((1u << lane) - 1u))] =
-                            make_uint4(row0 + (lane >> 1) * 128, ct * kMmaRows + cols * kUnitCols + (lane & 1) * 32, mine, a.meet.both(rt, ct) ? 1u : 0u);
+                        const uint32_t before = __popc(some & ((1u << lane) - 1u));
+                        const uint32_t first_row = row0 + (lane >> 1) * 128, first_col = ct * kMmaRows + cols * kUnitCols + (lane & 1) * 32;
+                        const uint32_t both = a.meet.both(rt, ct) ? 1u : 0u;
+                        if (SECTIONS) {
+                            const size_t at = size_t(section) * kSection + to + before;
+                            a.places[at] = make_uint2(first_row | both, first_col);
+                            a.rows[at] = mine;
+                        } else {
+                            waiting[have + before] = make_uint4(first_row, first_col, mine, both);
+                        }
                     }
-                    have += __popc(some);
-                    __syncwarp();
-                    if (have > 4) ask();
+                    if (!SECTIONS) {
+                        have += __popc(some);
+                        __syncwarp();
+                        if (have > 4) ask();
+                    }
                 }
                 if (cols & 1) at1 = at0, at0 = at0 == 6 ? 4 : at0 + 1;
             }
         }
-        if (have && !asked) ask();
-        if (asked) list_hits();
+        if (!SECTIONS && have && !asked) ask();
+        if (!SECTIONS && asked) list_hits();
         if (!ok) *aborted = 1;
     }
     __syncthreads();
+    if (SECTIONS && threadIdx.x == 0) a.section_hits[section] = listed;
     // copies and products in flight after a lost wait end before the block's memory goes away
     if (*aborted && warp == kEpiWarps && lane == 0) {
         atomicExch(a.status, kStatusWaitTimeout);
@@ -1552,9 +1686,10 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     const size_t before_b = hist_b + 2 * order_b;  // of use until the sweep begins, in the buffers' place
     uint64_t block = wanted;
     const bool wide = n > kPackedNodes - 1;  // (the last packed node stands for none)
-    const uint64_t most_hits = most_tiles * (most_tiles + 1) * 64;
-    const uint32_t hit_room = uint32_t(most_hits < kHitRoom ? most_hits : kHitRoom);
-    const size_t hits_b = size_t(hit_room) * 16;
+    const uint64_t most_hits = most_tiles * (most_tiles + 1) * kStepHits;  // (a launch has no more steps)
+    const bool sections = most_hits > kHitRoom;
+    const size_t hits_b = up(sections ? size_t(kSections) * kSection * 8 : size_t(most_hits) * 16);
+    const size_t rows_b = sections ? up(size_t(kSections) * kSection * 4) : 0, section_hits_b = up(kSections * 4);
     size_t entries_b, counts_b, list_b;
     // In one phase a row's limit stays what the places beside it say, the k-th of 512 distances: on data without clusters a
     // share of k / 512 of the nodes is within it, which twice as long a buffer holds with the ties.  (With 384 entries nearly
@@ -1575,7 +1710,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         const size_t slots = size_t((block + kMmaRows - 1) / kMmaRows) * kMmaRows;
         entries_b = up(slots * cap * (wide ? 8 : 4)), counts_b = up(slots * 4), list_b = up(slots * 4);
         const size_t buffers_b = entries_b > before_b ? entries_b : before_b;
-        const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + 512);
+        const int rc = reserve_workspace(h, h->s_sliced, op_b + codes_b + places_b + gates_b + 6 * n_b + buffers_b + counts_b + 2 * list_b + hits_b + rows_b + section_hits_b + 512);
         if (rc == 0) break;
         if (rc == kNoRoom && cap > kMmaCap) {
             cap = kMmaCap;
@@ -1584,6 +1719,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
         if (rc != kNoRoom || entries_b <= before_b || block <= uint64_t(sms) * kMmaRows) return rc;
         block = (block + 1) / 2;
     }
+    KnnMmaArgs a;
     unsigned char* p = h->s_sliced.as<unsigned char>();
     auto take = [&](size_t b) {
         unsigned char* r = p;
@@ -1602,10 +1738,13 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     uint32_t* group_place = reinterpret_cast<uint32_t*>(take(n_b));
     uint32_t* again = reinterpret_cast<uint32_t*>(take(list_b));
     uint32_t* redo = reinterpret_cast<uint32_t*>(take(list_b));
-    uint4* hits = reinterpret_cast<uint4*>(take(hits_b));
+    a.hits = reinterpret_cast<uint4*>(p);
+    a.places = reinterpret_cast<uint2*>(take(hits_b));
+    a.rows = reinterpret_cast<uint32_t*>(take(rows_b));
+    a.section_hits = reinterpret_cast<uint32_t*>(take(section_hits_b));
     // cleared for every block of rows, in one go (as clears of their own: a graph of 4,096 nodes 177 us, 167 so)
     struct Counters {
-        uint32_t used, hits, far, again, redo;
+        uint32_t used, hits, far, again, redo;  // hits: or sections taken
     };
     static_assert(sizeof(Counters) <= 256 && sizeof(LoadCounts) <= 256, "counters take 256 bytes");
     unsigned char* cleared = p;
@@ -1620,7 +1759,6 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
 
     // data that are not calm, in small graphs: bounds and near columns as in larger ones
     const bool two = small && other && whole.row_tiles / 2 + 1 >= 2 * kNearColumns;
-    KnnMmaArgs a;
     a.operand = operand;
     a.codes = placed;
     a.place = places;
@@ -1637,9 +1775,7 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     a.k = k;
     a.entries = entries;
     a.counts = counts;
-    a.hits = hits;
-    a.hit_count = &counters->hits;
-    a.hit_room = hit_room;
+    a.hit_count = a.taken = &counters->hits;
     a.status = h->d_status.as<uint32_t>();
     a.first_wait_polls = h->first_wait_polls;
     a.handover_polls = h->handover_polls;
@@ -1689,7 +1825,9 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
     h->launches += ordered ? 6 : 3;
     CPB_CUDA(cudaGetLastError());
     CPB_CUDA(allow_max_dynamic_smem(beside_kernel<U16, QUADS>));
-    CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS>));
+    if (sections) CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS, true>));
+    else CPB_CUDA(allow_max_dynamic_smem(knn_mma_kernel<U16, QUADS, false>));
+    const uint32_t most_blocks = sms < kSections ? sms : kSections;
     for (uint64_t begin = row_begin; begin < row_end; begin += block) {
         const uint32_t rb = uint32_t(begin), re = uint32_t(row_end - begin < block ? row_end : begin + block), m = re - rb;
         a.meet.row_tiles = (m + kMmaRows - 1) / kMmaRows;
@@ -1715,16 +1853,21 @@ int launch_mma_t(cphnsw_b200_index* h, const void* d_codes, const uint32_t* padd
                                                                                  a.meet.tiles, a.choice);
         h->launches += 2;
         const uint32_t columns = a.meet.columns();
-        // A launch takes 4M steps: on clustered data, where nearly all of them have no hit, those there are have room in the list.
-        // (Of as many as 64 a step, the sweep compares itself what finds none.)
+        // A launch takes 4M steps: on clustered data, where nearly all of them have no hit, those there are have room in the sections.
         const uint32_t range = uint32_t(kLaunchSteps / a.meet.row_tiles) + 1;
         bool first = true;
         auto sweep = [&](uint32_t count) {
             const uint64_t steps = uint64_t(a.meet.row_tiles) * count;
             if (!first) CPB_CUDA(cudaMemsetAsync(a.hit_count, 0, 4, st));
             first = false;
-            knn_mma_kernel<U16, QUADS><<<unsigned(steps < sms ? steps : sms), kMmaThreads, sweep_smem, st>>>(a);
-            knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
+            a.blocks = uint32_t(steps < most_blocks ? steps : most_blocks);
+            if (sections) {
+                knn_mma_kernel<U16, QUADS, true><<<a.blocks, kMmaThreads, sweep_smem, st>>>(a);
+                knn_check_sections_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
+            } else {
+                knn_mma_kernel<U16, QUADS, false><<<a.blocks, kMmaThreads, sweep_smem, st>>>(a);
+                knn_check_kernel<U16, QUADS><<<sms * kCheckBlocks, kCheckWarps * 32, 0, st>>>(a);
+            }
             h->launches += 2;
             return 0;
         };

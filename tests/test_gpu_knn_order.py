@@ -130,10 +130,14 @@ def test_rows_a_warp(cp, rows, k):
     agree(cp, idx, 128, 32, 1, codes, k, 500, 500 + rows)
 
 
-# 150,000 points without clusters: the last phase lists up to 143 x 586 x 64 groups of 32 rows and 32 columns, 1.2M more than the list
-# has room for, which are compared in the sweep
-def test_more_hits_than_the_list_has_room_for(cp):
-    idx = cp.CPHNSWIndex(128, K=32)
-    codes = mixture_codes(idx, 150000, 128, 1, 1.0, 32, 1, 9)
+# points without clusters, whose sweep finds nearly all groups of 32 rows and 32 columns: up to 65,024 nodes they have room in one list,
+# above in sections of one, of which there are enough at 80,000 (the last phase has 3.2M groups, the sections room for 5.5M).  At
+# 200,000 (9.8M) blocks compare what has no room
+@pytest.mark.parametrize("n,dim,K,cb,rows", [
+    (65024, 128, 32, 1, None), (65025, 128, 32, 1, None), (80000, 64, 16, 1, None), (200000, 128, 32, 1, None), (200000, 300, 64, 2, None),
+    (200000, 300, 32, 2, (20001, 180000))])
+def test_more_hits_than_the_list_has_room_for(cp, n, dim, K, cb, rows):
+    idx = cp.CPHNSWIndex(dim, K=K, component_bytes=cb)
+    codes = mixture_codes(idx, n, dim, 1, 1.0, K, cb, 9)
     idx.set_param("knn_kernel", 3)
-    agree(cp, idx, 128, 32, 1, codes, 64, 0, 150000)
+    agree(cp, idx, dim, K, cb, codes, 64, *(rows or (0, n)))
