@@ -893,6 +893,7 @@ constexpr int kSquadThreads = kSquadWarps * 32;
 constexpr int kSquadRows = 4;                            // per warp
 constexpr int kSquadFront = kSquadWarps * kSquadRows;    // members of W taken per step
 static_assert(kSquadFront == 32, "the unexpanded members of a window");
+constexpr size_t kSquadStatic = 6160;                    // its static shared memory
 
 template <bool U16, int METRIC>
 __global__ void __launch_bounds__(kSquadThreads, 4) search_squad_kernel(WalkArgs w) {
@@ -1340,14 +1341,25 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
             w.order = sc.near + a.nq;
         }
     }
-    // Few queries: a block each, as many as run at once.  Against a warp each, us for 1 / 148 / 296 / 592 queries: 100k x 128,
-    // beam 500, K = 32 166 / 212 / 284 / 341 against 475 / 507 / 530 / 563; K = 64, a table of 32 KB, 237 / 309 / 364 / 509 against
-    // 845 / 914 / 956 / 980; 60k points of the sphere, K = 32 1,139 / 1,308 / 1,453 / 1,875 against 1,815 at 592, so the line is at
-    // 555 there; sign-bit codes, K = 64, beam 200, 164 / 203 / 233 / 278 against 244 / 289 / 350 / 359, of the sphere 339 / 453 /
-    // 497 / 592 against 565 / 604 / 629 / 640; code distance, K = 32, of the sphere 425 / 530 / 575 / 704 against 601 / 698 / 709 /
-    // 758.  Beyond, blocks go in waves: 800 queries 486 against 613 on clusters, but 2,945 against 1,897 of the sphere.
-    const uint32_t squads = uint32_t(h->sm_count) * (size_t(a.K) * a.P * 4 >= 32 * 1024 || sym ? 16 : 15) / 4;
+    // Few queries: a block each.  Against a warp each, us for 1 / 148 / 296 / 592 queries: 100k x 128, beam 500, K = 32 166 / 212 /
+    // 284 / 341 against 475 / 507 / 530 / 563; K = 64, a table of 32 KB, 237 / 309 / 364 / 509 against 845 / 914 / 956 / 980; 60k
+    // points of the sphere, K = 32 1,139 / 1,308 / 1,453 / 1,875 against 1,815 at 592; sign-bit codes, K = 64, beam 200, 164 / 203 /
+    // 233 / 278 against 244 / 289 / 350 / 359, of the sphere 339 / 453 / 497 / 592 against 565 / 604 / 629 / 640; code distance, K =
+    // 32, of the sphere 425 / 530 / 575 / 704 against 601 / 698 / 709 / 758.
+    //   How many an SM: four run at once where shared memory has room for their beams, to some 2,950, else three, and the others go in
+    // a second wave.  Query tables of 32 KB and more: four, in waves or not (beam 4,096, 592 queries: 0.78 of a warp each).  Symmetric
+    // metrics: four, in waves up to 499 queries (sign bits, K = 64, beam 4,096: 0.98 of a warp each at 500, 1.10 at 592).  Small
+    // tables, whose warps are nearly as fast, 445 and 555 queries, of a warp each: K = 32, M = 32, beam 100 0.86 and 0.96, beam 40
+    // 0.93 and 1.04, up to 444 0.76 to 0.94; M = 24, beam 64 0.94 and 0.98; beam 4,096 1.13 and 1.36, of the sphere 1.27 and 1.34, up
+    // to 444 0.51 to 0.81.  Rows of 16 links bring few candidates a step: beam 40 1.06 at 333, 1.17 at 555, of the sphere 1.03 and
+    // 1.13; beam 200 0.79 and 0.94, of the sphere 1.04 and 1.25.  More than four an SM: 800 queries 486 us against 613 on clusters,
+    // but 2,945 against 1,897 of the sphere.
     const size_t squad_smem = size_t(w.wcap_slots) * 16 + kTagBytes + (sym ? row : 0);
+    const bool four = size_t(228 * 1024) / (squad_smem + kSquadStatic + 1024) >= 4;
+    uint32_t eighths = 32;  // of a query an SM
+    if (sym) eighths = four ? 32 : 27;
+    else if (size_t(a.K) * a.P * 4 < 32 * 1024) eighths = a.M <= 16 ? (a.beam < 200 ? 16 : 24) : (a.beam < 64 || !four ? 24 : 30);
+    const uint32_t squads = uint32_t(h->sm_count) * eighths / 8;
     if (!w.exact_visited && a.nq <= squads && (w.seeds || (a.n_seed >= a.n_entry && a.n_entry <= 128))) {
 #define CPB_SQUAD(X) (u16 ? launch_squad_t<true, X>(w, squad_smem, st) : launch_squad_t<false, X>(w, squad_smem, st))
         switch (metric) {

@@ -61,6 +61,32 @@ def test_few_queries_under_the_symmetric_metrics(cp, kind, dim, K, ef, nq):
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
 
 
+# as many queries as go a block each, and one more: in eighths of a query an SM by links, beam, the size of the query table and the
+# blocks that fit an SM (a beam of 4,096: three)
+@pytest.mark.parametrize("kind,dim,K,M,ef,eighths", [
+    ("bytes", 64, 16, 16, 199, 16), ("bytes", 64, 16, 16, 200, 24), ("bytes", 128, 32, 17, 63, 24), ("bytes", 128, 32, 32, 64, 30),
+    ("bytes", 64, 16, 32, 4096, 24),
+    ("wide", 300, 16, 32, 40, 32), ("wide", 300, 16, 32, 4096, 32), ("binary", 128, 64, 32, 40, 32), ("binary", 128, 64, 32, 4096, 27)])
+def test_as_many_queries_as_go_a_block_each(cp, kind, dim, K, M, ef, eighths):
+    import torch
+    most = torch.cuda.get_device_properties(0).multi_processor_count * eighths // 8
+    n = 4500
+    base, q = synthetic.gaussian_mixture(n, most + 1, dim, 12, 0.3, dim + ef)
+    if kind == "binary":
+        idx = cp.CPHNSWIndex.binary(dim, M=M, ef_construction=200, K=K)
+    else:
+        idx = cp.CPHNSWIndex(dim, M=M, ef_construction=200, K=K, component_bytes=2 if dim > 128 else 1)
+    idx.set_param("entry_scan", 200)
+    idx.set_param("k_entry", 32)
+    idx.add_batch_parallel(base)
+    ids, dist = idx.search_batch(q, 10, ef)
+    fewer = idx.search_batch(q[:most], 10, ef)
+    idx.set_param("search_kernel", 1)
+    wi, wd = idx.search_batch(q, 10, ef)
+    assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
+    assert np.array_equal(fewer[0], wi[:most]) and np.array_equal(fewer[1], wd[:most])
+
+
 # a base beyond L2 that is read many times over: the queries are taken by their nearest entry nodes (more queries than one pass of
 # the block that orders them, fewer seeds than it looks at)
 @pytest.mark.parametrize("n,dim,nq,rerank,seeds", [(40_003, 960, 601, 1000, 32), (70_001, 512, 2_500, 500, 3)])
