@@ -74,6 +74,13 @@ def measured_fp4_peak():
     return 9e15, "the nominal dense fp4 rate"
 
 
+def filter_values(K):
+    """Values of a code's row in the tensor-core filter: a component is 7 of +-1 at K <= 32 and 3 above; and with the padding
+    to a multiple of 64, which the products take too."""
+    own = K * (7 if K <= 32 else 3)
+    return own, (own + 63) // 64 * 64
+
+
 def measured_peaks():
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(path):
@@ -627,16 +634,16 @@ def run_b200(args):
                    "note": "K*3*P*log2(P) butterflies per vector over the measured stage time; peak = GPUs x SMs x 128 lanes x sampled SM clock"},
         "knn_graph": None, "select_neighbors": None}
     if 2 <= K <= 64 and n >= 4096:
-        # tensor-core filter: a component is 7 values of +-1 at K <= 32 and 3 above, rows padded to a multiple of 32
-        # values; a pair costs two operations a value, once where both its rows are of one GPU
-        values = (K * (7 if K <= 32 else 3) + 31) // 32 * 32
+        # the operations issued: two a value and pair, once where both its rows are of one GPU
+        own_values, values = filter_values(K)
         fp4, fp4_kind = measured_fp4_peak()
         fp4 *= world
         products = build["knn_pairs_per_s"] * (1.0 - 0.5 / world) * 2 * values
         roofline_build["knn_graph"] = {"bound": "fp4 tensor pipe and its epilogue", "achieved": products, "peak": fp4,
                                        "unit": "op/s", "frac": products / fp4,
-                                       "note": "%d values per pair, an unordered pair once on a GPU that has both rows; peak is %s; the whole stage, "
-                                               "bounds and order included (profiles/knn_mma_kernel_c2_quarter.md)" % (values, fp4_kind)}
+                                       "note": "operations issued: %d values per pair, %d of them padding, an unordered pair once on a GPU that has both "
+                                               "rows; peak is %s; the whole stage, bounds and order included "
+                                               "(profiles/knn_mma_kernel_c2_quarter.md)" % (values, values - own_values, fp4_kind)}
     sel_bytes = n * (knn_k * 4 + knn_k * code_row + M * 4.0)
     roofline_build["select_neighbors"] = {"bound": "hbm gather", "achieved": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9, "peak": peak * world,
                                           "unit": "GB/s", "frac": sel_bytes / (stage_ms["select_neighbors"] * 1e-3) / 1e9 / (peak * world),

@@ -70,3 +70,15 @@ def test_reference_arm_other_ranks_print_nothing():
     out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--gpus", "2"], capture_output=True,
                          text=True, timeout=120, env=env)
     assert out.returncode == 0 and out.stdout.strip() == ""
+
+
+def test_filter_values_are_those_the_kernel_lays_out():
+    """The operations of the kNN filter that bench.py counts: rows of 64 values, of which a row's chunk of 16 bytes holds 32."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("bench_filter_values", os.path.join(ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(bench)
+    for K, own, issued in ((2, 14, 64), (9, 63, 64), (10, 70, 128), (19, 133, 192), (32, 224, 256), (33, 99, 128), (48, 144, 192), (64, 192, 192)):
+        assert bench.filter_values(K) == (own, issued)
+    with open(os.path.join(ROOT, "sparse-text-kmeans_b200", "csrc", "knn_mma.cu")) as f:
+        assert "s.chunks = (values + 63) / 64 * 2;" in f.read()
