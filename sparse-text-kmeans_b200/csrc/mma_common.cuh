@@ -11,7 +11,7 @@ using knn::kFull;
 using knn::smem_u32;
 
 constexpr int kMmaRows = 256;         // rows per block and candidates per tile
-constexpr uint32_t kTmemCols = 512;   // two accumulators of 128 rows by 256 columns
+constexpr uint32_t kTmemCols = 512;   // all of an SM's; each kernel says what lies where
 
 __device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
     // K-major, no swizzle: core matrices of 8 rows x 16 bytes, 128 bytes apart along the rows (stride offset) and
