@@ -651,10 +651,11 @@ static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint3
         return CPHNSW_B200_E_CUDA;
     }
     if (device < 0 || device >= ndev) { set_error("device %d out of range (%d devices)", device, ndev); return CPHNSW_B200_E_INVALID; }
-    int major = 0, minor = 0, sms = 0;
+    int major = 0, minor = 0, sms = 0, l2 = 0;
     CPB_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
     CPB_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device));
     CPB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CPB_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, device));
     if (major != 10) {
         set_error("device %d is sm_%d%d; this library is built for sm_100a only", device, major, minor);
         return CPHNSW_B200_E_CUDA;
@@ -680,6 +681,7 @@ static int create_impl(uint64_t dim, uint32_t K, uint32_t component_bytes, uint3
     h->device = device;
     h->binary_codes = binary ? 1 : 0;
     h->sm_count = sms;
+    h->l2_bytes = l2;
     // RotationChain: rotation r is seeded seed + r (include/cphnsw/encoder/rotation.hpp:173-178);
     // each table is drawn layer by layer from mt19937_64 through uniform_int_distribution<int>(0,1)
     // (rotation.hpp:134-144) — the standard library does the draw, as in the reference.

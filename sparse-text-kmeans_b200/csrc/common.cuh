@@ -175,7 +175,7 @@ struct cphnsw_b200_index {
     // counts 2^residual_shift (combined distance (h_p << shift) + h_r, include/cphnsw/core/types.hpp:284-302)
     uint32_t residual_bits = 0, residual_shift = 0;
     uint32_t build_seed = 0;  // 0: add_batch_parallel builds the exact kNN graph; else only of this many nodes, the rest inserted
-    int sm_count = 0;
+    int sm_count = 0, l2_bytes = 0;
     // polls the kNN kernels and the exact sweep grant their FIRST tile wait ("first_wait_polls"; every other wait keeps the full
     // limit).  0 makes that wait give up at once: the way a test reaches the lost-wait path.
     uint32_t first_wait_polls = 1u << 22;

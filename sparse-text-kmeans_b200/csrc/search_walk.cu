@@ -37,7 +37,7 @@ constexpr int kBucketLog2 = 9;    // tag filter: 512 buckets of 4 tags = 4 KB pe
 constexpr uint32_t kTagBytes = (1u << kBucketLog2) * 8;
 constexpr uint64_t kTagNodes = uint64_t(0xffff) << kBucketLog2;  // ids below this have exact tags
 constexpr uint64_t kFiller = ~0ull;
-constexpr double kOrderBase = 128e6, kOrderReads = 2e9;
+constexpr double kOrderReads = 2e9;
 constexpr int kOrderSeeds = 8, kOrderLog2 = 12, kOrderBins = 1 << kOrderLog2;
 constexpr int kScanKeep = 128;    // most seeds the entry-scan kernel keeps per query: 32 in each of one or four registers a lane
 constexpr int kScanWarps = 8;
@@ -568,9 +568,9 @@ entry_scan_kernel(ScanArgs a) {
 // Queries of one cluster rerank much the same vectors.  Taken one after the other they find them in L2; as given, a base that
 // does not fit L2 is read from HBM once for each.  Queries with the same nearest entry node, of whose kOrderSeeds nearest the
 // smallest stands for all, go together, in any order otherwise.  One block: a count, a scan and a scatter over kOrderBins bins
-// that such nodes are hashed to.  10,000 queries, 1M x 128, 500 reranked: walk 2,550 -> 2,060 us (links, codes and tables come from
-// L2 as well), rerank 460 -> 437, for 10 us; 2,000 of 960 dimensions, 100k, 1,000 reranked: rerank 939 -> 847.  (The nearest of one
-// or two seeds alone: walk and rerank together 270 us slower; sorted by their true clusters: 3,343 us in all, 3,145 so.)
+// that such nodes are hashed to.  All kernels of a search, with the 10 us of this one, on four seeds in turn: 10,000 queries, 1M x 128,
+// 500 reranked 3,002 to 3,011 us as given, 2,895 to 2,917 in order; 2,000 of 960 dimensions, 100k, 1,000 reranked 2,811 to 2,850
+// and 2,620 to 2,684.  (By the nearest of one seed 2,954 to 2,990 and 2,723 to 2,757, of two 2,943 to 2,980 and 2,724 to 2,743.)
 __global__ void __launch_bounds__(1024) order_queries_kernel(const uint32_t* __restrict__ near, uint32_t nq, uint32_t* __restrict__ order) {
     constexpr int kEach = kOrderBins / 1024;
     __shared__ uint32_t bins[kOrderBins], sums[32];
@@ -1325,12 +1325,13 @@ int launch_search_walk(cphnsw_b200_index* h, SearchCtx& cx, SearchArgs a, bool s
         CPB_TRY(cx.d_seeds.reserve(size_t(a.nq) * (w.seed_slots * 8 + 8)));
         sc.seeds = cx.d_seeds.as<uint64_t>();
         w.seeds = sc.seeds;
-        // The order costs 10 us.  It is of use where links, codes and vectors do not fit L2 (126 MB), and made up for where the
-        // queries read them many times: 10,000 queries on 1M x 128, 3.4 GB, 3,680 us as given and 3,145 in order; 2,000 on 100k x 960,
-        // 8 GB, 3,364 and 3,112; on 100k x 512, 2.2 GB, 1,167 and 1,156; 400 on 100k x 960, 0.8 GB, 698 and 706.
+        // The order costs 10 us.  It is of use where links, codes and vectors do not fit L2, and made up for where the queries read them
+        // many times.  Four seeds, us as given and in order: 10,000 queries on 1M x 128, 3.4 GB, 3,002 to 3,011 and 2,895 to 2,917; on
+        // 300k x 128 2,515 to 2,543 and 2,468 to 2,493; 2,000 on 100k x 960, 8 GB, 2,811 to 2,850 and 2,620 to 2,684; on 100k x 512,
+        // 2.2 GB, 1,168 to 1,174 and 1,131 to 1,140; 600 on 100k x 960, 2.4 GB, 1,787 to 1,834 and 1,791 to 1,818, where it breaks even.
         sc.near = nullptr;
         const double node_bytes = double(a.M) * 4 + double(row), vector_bytes = a.rerank_k ? double(a.dim) * 4 : 0.0;
-        if (a.nq > 2 * uint32_t(h->sm_count) && double(a.n) * (node_bytes + vector_bytes) > kOrderBase &&
+        if (a.nq > 2 * uint32_t(h->sm_count) && double(a.n) * (node_bytes + vector_bytes) > double(h->l2_bytes) &&
             double(a.nq) * (a.beam * node_bytes + a.rerank_k * vector_bytes) > kOrderReads) {
             sc.near = reinterpret_cast<uint32_t*>(sc.seeds + size_t(a.nq) * w.seed_slots);
         }

@@ -102,6 +102,32 @@ def test_queries_in_order_of_their_entry_nodes(cp, n, dim, nq, rerank, seeds):
     assert np.array_equal(ids, wi) and np.array_equal(dist, wd)
 
 
+# the order is taken, a launch more, from a node beyond L2 and a query beyond 2 GB of reads on; a node is 32 links, a code row of 32 bytes
+# and its vector, and 1,000 are read for a query
+def test_where_the_order_of_queries_begins(cp):
+    import torch
+    dim, node = 960, 32 * 4 + 32 + 960 * 4
+    most_nodes = torch.cuda.get_device_properties(0).L2_cache_size // node
+    most = int(2e9 // (1000 * node))
+    base, q = synthetic.gaussian_mixture(most_nodes + 1, most + 1, dim, 40, 0.3, 17)
+    launches = {}
+    for n in (most_nodes, most_nodes + 1):
+        idx = cp.CPHNSWIndex(dim, M=32, ef_construction=200, K=16, component_bytes=2)
+        idx.set_param("entry_scan", 300)
+        idx.set_param("k_entry", 32)
+        idx.add_batch_parallel(base[:n])
+        found = {}
+        for nq in (most, most + 1):
+            before = idx.launch_count()
+            found[nq] = idx.search_and_rerank_batch(q[:nq], 10, 100, 1000)
+            launches[n, nq] = idx.launch_count() - before
+        for a, b in zip(found[most], found[most + 1]):
+            assert np.array_equal(a, b[:most])
+    few = launches[most_nodes, most]
+    assert launches[most_nodes, most + 1] == few and launches[most_nodes + 1, most] == few
+    assert launches[most_nodes + 1, most + 1] == few + 1
+
+
 @pytest.mark.parametrize("M", [24, 32])
 @pytest.mark.parametrize("row,a,b", [(0, 0, 1), (0, 0, 16), (0, 7, 23), (256, 3, 20)])
 def test_repeated_ids_in_a_row_count_once(cp, oracle, M, row, a, b):
