@@ -153,7 +153,10 @@ int cphnsw_b200_set_sign_tables(cphnsw_b200_index* h, const int8_t* signs);
 
 /* Replaces legacy CPEncoder<ComponentT,K>::encode / encode_batch
  * (include/cphnsw/encoder/cp_encoder.hpp:161-184,244-260) and GPUEncoder::encode_batch
- * (src/cuda/gpu_encoder.cu:430-471).  x float[n][dim] -> codes ComponentT[n][K]. */
+ * (src/cuda/gpu_encoder.cu:430-471).  x float[n][dim] -> codes ComponentT[n][K].
+ * Vectors of 513 to 1,024 dimensions are encoded by way of tensor memory (32 of an SM's 512 columns a block),
+ * in every call that encodes.  Beside kernels that hold all of an SM's tensor memory, on another stream, blocks
+ * that share an SM with one wait until it gives columns back: such a kernel must not wait for an encode. */
 int cphnsw_b200_encode(cphnsw_b200_index* h, const float* x, uint64_t n, void* codes_out);
 
 /* Replaces legacy encode_query / GPUEncoder::encode_queries_batch (src/cuda/gpu_encoder.cu:473-513):

@@ -275,6 +275,9 @@ encode_thread_kernel(const float* __restrict__ x, uint64_t n, int dim, int K, in
 //   What bounds it is the add pipe (0.61 of it) and the instructions beside: without the changes of places it would take 0.84 of
 // its time, without two of the three diagonals 0.9, without the search for the argmax 0.93.  With transposes through shared
 // memory, five of 64 wavefronts each a vector and rotation, these were the bound: 100k x 960, K = 32, 5,340 us; 4,390 now.
+// Rotated vectors wanted, 2,000 of 960: 153 us with transposes, 118 now, although a lane then spills 10 to 18 registers.
+//   Tensor memory is an SM's own: a block that finds all of it taken, by a kernel on another stream, stands until some is given
+// back.  (Beside a block of the sweeps of this library, which take all, none has the registers to start.)
 constexpr int kP1024 = 1024;
 constexpr int kWarps1024 = 4;
 constexpr int kBlocks1024 = 4;  // resident on an SM (five of 96 registers spill: 4,480 us)
